@@ -358,7 +358,12 @@ def work(case):
 
 
 def tolerance(case):
-    return {"rel": 1e-2}
+    """about four times what the results of one precision are from 64 bits: the Llama family and the encoder keep keys, values (and the
+    encoder its activations) in bf16, which shows in the logits as 3e-3 to 5e-3; the layered models' norms behind every sublayer leave
+    1e-5 to 1e-3 of it; the exact mode is at 2e-7 to 3e-7"""
+    if case["work"] != "step":
+        return {"rel": 2e-2}
+    return {"rel": 1.2e-6 if case["dtype"] == "f32" else 4e-3}
 
 
 # ---- the same results in 64 bits ----------------------------------------------------------------------------------------------------
