@@ -838,6 +838,8 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
         FL_CUDA(cudaStreamSynchronize(c.stream));
         drop_graphs(c);
         const size_t R = std::max<size_t>(T, 2 * y.rows), W = m.W, P = R * std::max(m.max_top, 1);
+        // rows of the experts' runs in a step of many rows (whole 128-row tiles per expert that any row picked)
+        const size_t run_rows = R > 128 && m.max_experts > 0 ? 128 * (P / 128 + std::min<size_t>(P, m.max_experts)) : 0;
         y.x.alloc(R * W); y.h.alloc(R * W); y.y.alloc(R * W);
         y.proj.alloc(R * m.max_in); y.u.alloc(R * std::max(m.max_u, 1)); y.go.alloc(R * std::max(m.max_hv, 1));
         y.la.alloc(R * std::max(m.max_hd, 1));
@@ -857,10 +859,10 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
             y.qp_hi.alloc(R * m.max_hp); y.qp_lo.alloc(R * m.max_hp); y.qo_hi.alloc(R * m.max_hq); y.qo_lo.alloc(R * m.max_hq);
             y.ol_hi.alloc(R * m.max_hc); y.ol_lo.alloc(R * m.max_hc);
         }
-        y.gu.alloc(P * 2 * std::max(m.max_ff, 1)); y.act.alloc(P * std::max(m.max_ff, 1)); y.eo.alloc(P * W);
+        y.gu.alloc(P * 2 * std::max(m.max_ff, 1)); y.act.alloc(P * std::max(m.max_ff, 1)); y.eo.alloc(std::max(P, run_rows) * W);
         y.sh_gu.alloc(R * 2 * std::max(m.max_ff, 1)); y.sh_act.alloc(R * std::max(m.max_ff, 1)); y.sh_o.alloc(R * W);
         y.route_w.alloc(P); y.route_sel.alloc(P); y.sgate.alloc(R);
-        y.pair_row.alloc(P); y.pair_of.alloc(P); y.grp_off.alloc((size_t)m.max_experts + 2);
+        y.pair_row.alloc(P); y.pair_of.alloc(P); y.grp_off.alloc((size_t)m.max_experts + 2); y.tile_off.alloc((size_t)m.max_experts + 2);
         if (!m.f32) {
             y.h_hi.alloc(R * W); y.h_lo.alloc(R * W);
             if (m.max_qr > 0) { y.cq_hi.alloc(R * m.max_qr); y.cq_lo.alloc(R * m.max_qr); }
@@ -881,7 +883,8 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
                 }
             }
             if (y.gemm_out.n < need) y.gemm_out.alloc(need);
-            if (gx_rows > 0 && y.gx_hi.n == 0) {
+            if (gx_rows > 0) gx_rows = std::max(gx_rows, run_rows);
+            if (y.gx_hi.n < gx_rows * W) {
                 y.gx_hi.alloc(gx_rows * W, true); y.gx_lo.alloc(gx_rows * W, true);
                 y.ga_hi.alloc(gx_rows * std::max(m.max_ff, 1), true); y.ga_lo.alloc(gx_rows * std::max(m.max_ff, 1), true);
                 y.grp_cnt.alloc((size_t)m.max_experts + 1, true);
@@ -948,6 +951,15 @@ static void launch_glu(LaunchCtx& lc, const Slices& gu, int rows, int F, float l
         launch(lc, "glu", 0, ly_glu_kernel<4>, dim3(rows, (F + 1023) / 1024), dim3(256), 0, gu, ldg, ldo, F, limit, act, bias, out, hi, lo);
     else
         launch(lc, "glu", 0, ly_glu_kernel<1>, dim3(rows, (F + 255) / 256), dim3(256), 0, gu, ldg, ldo, F, limit, act, bias, out, hi, lo);
+}
+
+// The first matrix of a gated feed-forward and its activation, as the hi | lo halves the second one reads.  More than 128 rows whose
+// tiles fill the chip take the activation in the GEMM's epilogue: the [rows, 2 F] f32 result (235 MB at 2048 rows of F = 14336) is neither
+// written nor read back (three such layers of width 4096, whole prefill: 8.29 -> 8.07 ms).  Few tiles keep the GEMM that cuts K; the
+// epilogue cannot see a sum in slices.
+static bool ff_in_fused(int R, int F, int K, int act, bool tc_in, bool tc_out, const uint16_t* hhi) {
+    const int tiles = (R + 127) / 128 * ((F + 127) / 128);
+    return tc_in && tc_out && hhi != nullptr && R > 128 && act != FL_ACT_RELU2 && F % 8 == 0 && (2 * tiles > kNumSMs || (K + 63) / 64 < 16);
 }
 
 static void gemm_groups(LaunchCtx& lc, const char* tag, const LyGemm& g, int groups, int max_rows) {
@@ -1627,24 +1639,35 @@ static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const in
         const float* sh = nullptr;
         if (d.shared_ff > 0 && !par) {  // the always-on expert first (parallel sublayers hold it in the mixer's matrices): its split-K scratch is free again before the routed experts run
             const int Fs = d.shared_ff;
-            const Slices gu = gemm_slices(c, lc, "gemm_shared_in", sub_in, hhi, hlo, lw.s_gu, lw.tm_sgu, lw.tc_sgu, 2 * Fs, W, y.sh_gu.p, Ti);
-            launch_glu(lc, gu, Ti, Fs, d.shared_limit, act, nullptr, lw.tc_sdown ? (float*)nullptr : y.sh_act.p, lw.tc_sdown ? ahi : (uint16_t*)nullptr, alo);
+            if (ff_in_fused(Ti, Fs, W, act, lw.tc_sgu, lw.tc_sdown, hhi)) {
+                dense_gemm_glu(c, lc, "gemm_shared_in", Ti, Fs, W, lw.tm_sgu, hhi, hlo, nullptr, act, d.shared_limit, ahi, alo);
+            } else {
+                const Slices gu = gemm_slices(c, lc, "gemm_shared_in", sub_in, hhi, hlo, lw.s_gu, lw.tm_sgu, lw.tc_sgu, 2 * Fs, W, y.sh_gu.p, Ti);
+                launch_glu(lc, gu, Ti, Fs, d.shared_limit, act, nullptr, lw.tc_sdown ? (float*)nullptr : y.sh_act.p, lw.tc_sdown ? ahi : (uint16_t*)nullptr, alo);
+            }
             gemm_tc_or_exact(c, lc, "gemm_shared_out", y.sh_act.p, ahi, alo, lw.s_down, lw.tm_sdown, lw.tc_sdown, W, Fs, y.sh_o.p, Ti);
             sh = y.sh_o.p;
         }
         const dim3 gw((W + 255) / 256, Ti);
         if (lw.tc_moe && Ti > 128) {
-            // many rows: every expert over all rows on the tensor cores, kept where the row picked it (ascending expert order)
-            for (int e = 0; e < E; ++e) {
-                dense_gemm(c, lc, "gemm_tc_moe_in", Ti, GF, W, lw.tm_egu[e], y.gu.p, hhi, hlo);
-                launch_glu(lc, Slices{y.gu.p, 1, 0}, Ti, F, d.limit, act, nullptr, nullptr, ahi, alo);
-                dense_gemm(c, lc, "gemm_tc_moe_out", Ti, W, F, lw.tm_edown[e], y.eo.p, ahi, alo);
-                launch(lc, "moe_accum", 0, ly_moe_accum_kernel, gw, dim3(256), 0, (const float*)y.eo.p, (const int*)y.route_sel.p,
-                       (const float*)y.route_w.p, top, e, (const float*)nullptr, e == 0 ? 1 : 0, W, out);
+            // many rows: each expert's rows gathered into a run of whole 128-row tiles, ONE grouped GEMM pair over all runs.  (Every expert over
+            // all rows, kept where picked, did E / top times the work: 1531 tokens, 8 experts of 5632, top 2, two layers: 5.43 -> 3.02 ms for the
+            // whole prefill; 340 rows of 2816-wide experts: 2.37 -> 1.41 ms.)
+            const size_t cap = 128 * ((size_t)P / 128 + std::min(P, E));
+            const RowRuns runs{E, y.tile_off.p};
+            launch(lc, "moe_lists", 0, ly_moe_lists_kernel, dim3(E), dim3(32), 0, (const int*)y.route_sel.p, Ti, top, E, y.grp_off.p, y.pair_row.p,
+                   y.pair_of.p);
+            launch(lc, "moe_gather", 0, ly_moe_gather_runs_kernel, dim3(P), dim3(256), 0, (const uint16_t*)hhi, (const uint16_t*)hlo, W, (const int*)y.route_sel.p, top, E,
+                   (const int*)y.grp_off.p, y.pair_of.p, y.gx_hi.p, y.gx_lo.p, y.tile_off.p);
+            if (act != FL_ACT_RELU2) {
+                dense_gemm_glu(c, lc, "gemm_tc_moe_in", (int)cap, F, W, lw.tm_gu, y.gx_hi.p, y.gx_lo.p, nullptr, act, d.limit, y.ga_hi.p, y.ga_lo.p, &runs);
+            } else {
+                dense_gemm_runs(c, lc, "gemm_tc_moe_in", (int)cap, F, W, lw.tm_gu, y.gu.p, y.gx_hi.p, y.gx_lo.p, runs);
+                launch(lc, "glu", 0, ly_relu2_runs_kernel, dim3((F + 1023) / 1024, (unsigned)(cap / 128)), dim3(256), 0, (const float*)y.gu.p, F, E, (const int*)y.tile_off.p,
+                       y.ga_hi.p, y.ga_lo.p);
             }
-            if (sh != nullptr)
-                launch(lc, "moe_accum", 0, ly_moe_accum_kernel, gw, dim3(256), 0, sh, (const int*)nullptr, (const float*)nullptr, 0, -1,
-                       sg, 0, W, out);
+            dense_gemm_runs(c, lc, "gemm_tc_moe_out", (int)cap, W, F, lw.tm_down, y.eo.p, y.ga_hi.p, y.ga_lo.p, runs);
+            launch(lc, "moe_combine", 0, ly_moe_combine_kernel, gw, dim3(256), 0, (const float*)y.eo.p, (const int*)y.pair_of.p, (const float*)y.route_w.p, top, sh, sg, W, out);
         } else {
             launch(lc, "moe_lists", 0, ly_moe_lists_kernel, dim3(E), dim3(32), 0, (const int*)y.route_sel.p, Ti, top, E, y.grp_off.p, y.pair_row.p,
                    y.pair_of.p);
@@ -1747,8 +1770,12 @@ static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const in
         sublayer_front(lw, run, 1);
         const int F = d.ff, act = d.ffn_act, GF = act == FL_ACT_RELU2 ? F : 2 * F;
         if (d.ffn == FL_FFN_DENSE) {
-            const Slices gu = gemm_slices(c, lc, "gemm_ff_in", sub_in, hhi, hlo, lw.w_gu, lw.tm_gu, lw.tc_gu, GF, W, y.gu.p, Ti);
-            launch_glu(lc, gu, Ti, F, d.limit, act, lw.b_gu, lw.tc_down ? (float*)nullptr : y.act.p, lw.tc_down ? ahi : (uint16_t*)nullptr, alo);
+            if (ff_in_fused(Ti, F, W, act, lw.tc_gu, lw.tc_down, hhi)) {
+                dense_gemm_glu(c, lc, "gemm_ff_in", Ti, F, W, lw.tm_gu, hhi, hlo, lw.b_gu, act, d.limit, ahi, alo);
+            } else {
+                const Slices gu = gemm_slices(c, lc, "gemm_ff_in", sub_in, hhi, hlo, lw.w_gu, lw.tm_gu, lw.tc_gu, GF, W, y.gu.p, Ti);
+                launch_glu(lc, gu, Ti, F, d.limit, act, lw.b_gu, lw.tc_down ? (float*)nullptr : y.act.p, lw.tc_down ? ahi : (uint16_t*)nullptr, alo);
+            }
             ff = gemm_slices(c, lc, "gemm_ff_out", y.act.p, ahi, alo, lw.w_down, lw.tm_down, lw.tc_down, W, F, y.y.p, Ti);
             if (sum_norm) fold(ff);
         } else {

@@ -1168,6 +1168,45 @@ int dense_gemm(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int N, int K,
     return ks;
 }
 
+// More than 128 rows: the gated feed-forward's first GEMM with the activation in its epilogue (see GemmArgs.act), and -- with tile_off --
+// GEMMs over runs of rows, each with its own matrix (see GemmArgs.groups).  The weight map has 128-row boxes.
+static void launch_rows_gemm(fl_cache& c, LaunchCtx& lc, const char* tag, const GemmArgs& g, int tiles, int weight_rows, const CUtensorMap& tmW, const uint16_t* xhi,
+                             const uint16_t* xlo, bool glu) {
+    const bool prof = g_prof.on && !lc.capturing;
+    const bool pdl = lc.pdl && !prof;
+    ProfEntry pe;
+    if (prof) {
+        pe.tag = tag;
+        pe.bytes = (uint64_t)weight_rows * g.K * 2;
+        FL_CUDA(cudaEventCreate(&pe.e0));
+        FL_CUDA(cudaEventCreate(&pe.e1));
+        FL_CUDA(cudaEventRecord(pe.e0, lc.stream));
+    }
+    const CUtensorMap hi = make_tmap_bf16(xhi, g.M, g.K, g.K, kGemmBM), lo = make_tmap_bf16(xlo, g.M, g.K, g.K, kGemmBM);
+    if (glu) launch_gemm_tc<256, GEPI_GLU_HL, DUAL_A>(lc.stream, pdl, tiles, hi, lo, tmW, g);
+    else launch_gemm_tc<256, GEPI_F32, DUAL_A>(lc.stream, pdl, tiles, hi, lo, tmW, g);
+    if (prof) {
+        FL_CUDA(cudaEventRecord(pe.e1, lc.stream));
+        g_prof.entries.push_back(pe);
+    }
+    if (lc.capturing) lc.captured++; else g_launches.fetch_add(1, std::memory_order_relaxed);
+}
+void dense_gemm_glu(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int F, int K, const CUtensorMap& tmW, const uint16_t* xhi, const uint16_t* xlo,
+                    const float* bias, int act, float limit, uint16_t* ohi, uint16_t* olo, const RowRuns* runs) {
+    FL_CHECK(R > 128 && F % 8 == 0 && K % 8 == 0 && act != FL_ACT_RELU2, FL_ERR_STATE, "internal: gated GEMM shape");
+    GemmArgs g{R, F, K, bias, nullptr, 0, ohi, F, 1, 0, olo};
+    g.act = act; g.act_limit = limit; g.raster_m = kGemmRasterRows;
+    int mats = 1;
+    if (runs != nullptr) { g.groups = mats = runs->groups; g.tile_off = runs->tile_off; g.grp_m = 2 * F; }
+    launch_rows_gemm(c, lc, tag, g, (R + kGemmBM - 1) / kGemmBM * ((F + 127) / 128), mats * 2 * F, tmW, xhi, xlo, true);
+}
+void dense_gemm_runs(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int N, int K, const CUtensorMap& tmW, float* out, const uint16_t* xhi,
+                     const uint16_t* xlo, const RowRuns& runs) {
+    GemmArgs g{R, N, K, nullptr, nullptr, 0, out, N, 1, 0};
+    g.groups = runs.groups; g.tile_off = runs.tile_off; g.grp_m = N;
+    launch_rows_gemm(c, lc, tag, g, (R + kGemmBM - 1) / kGemmBM * ((N + 255) / 256), runs.groups * N, tmW, xhi, xlo, false);
+}
+
 // Block-diagonal GEMM with hi | lo output (see GemmArgs.blocks): tokens are the M dimension above 128 rows, else the weights are
 // (swap-AB, never split over K: the halves are those of the finished sum).
 void dense_gemm_blocks(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int blocks, int N, int K, const CUtensorMap& tmW, const uint16_t* xhi,

@@ -15,10 +15,11 @@
 #include <algorithm>
 
 #include "common.cuh"
+#include "glu.cuh"
 
 namespace fl {
 
-enum : int { GEPI_BIAS_BF16 = 0, GEPI_BIAS_GELU_BF16 = 1, GEPI_BIAS_RESID_F32 = 2, GEPI_F32 = 3, GEPI_ATOMIC_F32 = 4, GEPI_F32_T = 5, GEPI_SILU_HL = 6, GEPI_HL = 7, GEPI_HL_T = 8 };
+enum : int { GEPI_BIAS_BF16 = 0, GEPI_BIAS_GELU_BF16 = 1, GEPI_BIAS_RESID_F32 = 2, GEPI_F32 = 3, GEPI_ATOMIC_F32 = 4, GEPI_F32_T = 5, GEPI_SILU_HL = 6, GEPI_HL = 7, GEPI_HL_T = 8, GEPI_GLU_HL = 9 };
 enum : int { DUAL_NONE = 0, DUAL_A = 1, DUAL_B = 2 };
 
 constexpr int kGemmBM = 128;
@@ -64,6 +65,16 @@ struct GemmArgs {
     // DUAL_A with plain tiles: the tile walk takes raster_m row tiles against one weight tile before the next weight tile (0: every
     // weight tile of a row tile first).
     int raster_m = 0;
+    // Gated feed-forward (GEPI_GLU_HL with DUAL_A): the weight matrix stacks N gate rows and N up rows; a tile's 256 weight rows are 128 of
+    // each and the epilogue writes glu(gate, up) [M, N] as bf16 hi (out) and lo (out2).  bias [2 N] or null.
+    int act = 0;
+    float act_limit = 0.f;
+    // ROW GROUPS (DUAL_A; the experts of a step with many rows): the rows of A come in `groups` runs of whole 128-row tiles, run e in
+    // tiles [tile_off[e], tile_off[e + 1]) (device memory, written by the gather kernel); run e multiplies the e-th of the stacked
+    // weight matrices of grp_m rows.  M is the row capacity; rows of a run's last tile past its count hold whatever was there, and so
+    // do their results, which nobody reads.
+    int groups = 0;
+    const int* tile_off = nullptr;
 };
 
 // ---- PTX wrappers ------------------------------------------------------------------------------------------------------
@@ -227,7 +238,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     const int mt_e = grouped ? (g.grp_m + kGemmBM - 1) / kGemmBM : 0;      // m tiles per group
     constexpr bool kBlocks = EPI == GEPI_HL || EPI == GEPI_HL_T;           // block-diagonal forms
     const int nblk = kBlocks && g.blocks > 1 ? g.blocks : 1;
-    const int mt_b = (g.M + kGemmBM - 1) / kGemmBM, nt_b = (g.N + BN - 1) / BN;
+    constexpr int kBNOut = EPI == GEPI_GLU_HL ? BN / 2 : BN;               // output columns of a tile
+    static_assert(EPI != GEPI_GLU_HL || (BN == 256 && DUAL == DUAL_A), "the gated epilogue pairs two 128-row weight boxes");
+    const int mt_b = (g.M + kGemmBM - 1) / kGemmBM, nt_b = (g.N + kBNOut - 1) / kBNOut;
+    const bool runs = DUAL == DUAL_A && (EPI == GEPI_F32 || EPI == GEPI_GLU_HL) && g.groups > 0;
+    int cur_e = 0;                                        // the run a thread's walk has reached (items only grow)
     const int mt = grouped ? (g.M / g.grp_m) * mt_e : (EPI == GEPI_HL_T ? nblk * mt_b : mt_b), nt = grouped ? 1 : (EPI == GEPI_HL ? nblk * nt_b : nt_b);
     const int ksplit = g.ksplit > 1 ? g.ksplit : 1;
     // tile -> (first row of the A box, first row of the B box, group, first row inside the group)
@@ -248,19 +263,26 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             mrow0 = (bm % mt_b) * kGemmBM;
             m0 = grp * g.M + mrow0;
             n0 = (tile % nt) * BN;
+        } else if (runs) {              // the row tiles of a run against one weight tile, then the next weight tile
+            int t0 = g.tile_off[cur_e], t1 = g.tile_off[cur_e + 1];
+            while (tile >= t1 * nt) { t0 = t1; t1 = g.tile_off[++cur_e + 1]; }
+            grp = cur_e;
+            const int local = tile - t0 * nt, cnt = t1 - t0;
+            m0 = mrow0 = (t0 + local % cnt) * kGemmBM;
+            n0 = grp * g.grp_m + (local / cnt) * kBNOut;
         } else if (DUAL == DUAL_A && g.raster_m > 0) {
             grp = 0;
             const int per = g.raster_m * nt, first = tile / per * g.raster_m, local = tile % per, cnt = min(g.raster_m, mt - first);
             m0 = mrow0 = (first + local % cnt) * kGemmBM;
-            n0 = (local / cnt) * BN;
+            n0 = (local / cnt) * kBNOut;
         } else {
             grp = 0;
             m0 = mrow0 = (tile / nt) * kGemmBM;
-            n0 = (tile % nt) * BN;
+            n0 = (tile % nt) * kBNOut;
         }
     };
     const int nkps = (nk + ksplit - 1) / ksplit;          // k-blocks per split
-    const int ntiles = mt * nt * ksplit;                  // work items: (m tile, n tile, k split), k split fastest
+    int ntiles = mt * nt * ksplit;                        // work items: (m tile, n tile, k split), k split fastest
 
     // programmatic dependent launch: the next kernel's prologue may start now; our own prologue (barriers, TMEM, descriptor
     // fetch) overlaps the previous kernel's tail.  Everything that touches dependent memory is ordered behind the producer's
@@ -309,6 +331,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             pdl_wait();
             asm volatile("fence.proxy.async;" ::: "memory");      // the previous kernel's generic-proxy stores -> TMA reads
+            if (runs) ntiles = g.tile_off[g.groups] * nt;
             uint32_t c = 0;
             for (int item = blockIdx.x; item < ntiles; item += gridDim.x) {
                 const int tile = item / ksplit, ks = item % ksplit;
@@ -337,7 +360,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         tma_load_2d(sa + kBOff, &tmB, kb * kGemmBK, n0, &full[st]);
                         // DUAL_A with a 256-row weight tile: the weight descriptors carry a 128-row box (the swap-AB decode GEMMs'
                         // A operand), so the tile arrives as two boxes; rows past the matrix are zero-filled by the TMA engine
-                        if (DUAL == DUAL_A && BN == 256) tma_load_2d(sa + kBOff + kBBytes / 2, &tmB, kb * kGemmBK, n0 + 128, &full[st]);
+                        if (DUAL == DUAL_A && BN == 256)
+                            tma_load_2d(sa + kBOff + kBBytes / 2, &tmB, kb * kGemmBK, n0 + (EPI == GEPI_GLU_HL ? g.N : 128), &full[st]);
                     }
                 }
             }
@@ -347,7 +371,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         if (lane == 0) {
             constexpr uint32_t idesc = umma_idesc_bf16(kGemmBM, kMmaN);
             uint32_t c = 0, ti = 0;
-            if (grouped) pdl_wait();      // grp_cnt is written by the preceding kernel
+            if (grouped || runs) pdl_wait();      // grp_cnt / tile_off is written by a preceding kernel
+            if (runs) ntiles = g.tile_off[g.groups] * nt;
             for (int item = blockIdx.x; item < ntiles; item += gridDim.x) {
                 if (grouped && g.grp_cnt[(item / ksplit) / mt_e] == 0) continue;
                 const uint32_t ti_now = ti++;
@@ -381,7 +406,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int q = warp & 3;
         const int cslice = (warp - 2) >> 2;
         uint32_t ti = 0;
-        if (grouped) pdl_wait();          // grp_cnt is written by the preceding kernel
+        if (grouped || runs) pdl_wait();          // grp_cnt / tile_off is written by a preceding kernel
+        if (runs) ntiles = g.tile_off[g.groups] * nt;
         for (int item = blockIdx.x; item < ntiles; item += gridDim.x) {
             const int tile = item / ksplit, ksi = item % ksplit;
             int m0, n0, grp, mrow0;
@@ -395,10 +421,54 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             const int row_lim = grouped ? g.grp_m : g.M, col_lim = grouped ? gcnt : g.N;
             if (grouped) n0 = 0;
             if (EPI == GEPI_HL) n0 -= grp * g.N;       // columns count inside the block
+            if (runs) n0 -= grp * g.grp_m;             // ... inside the run's matrix
             mbar_wait(&acc_full[as], (ti_now >> 1) & 1);
             tc_fence_after();
 #pragma unroll 1
-            for (int c0 = cslice * 32; c0 < BN; c0 += 128) {      // 32-column chunks dealt round-robin to the 4 warps of a lane quarter
+            for (int c0 = cslice * 32; c0 < kBNOut; c0 += 128) {  // 32-column chunks dealt round-robin to the 4 warps of a lane quarter
+                if (EPI == GEPI_GLU_HL) {
+                    // 16 columns at a time: accumulator columns [0, 128) hold gate rows, [128, 256) the up rows of the same outputs
+#pragma unroll 1
+                    for (int h = 0; h < 32; h += 16) {
+                        uint32_t rg[16], ru[16];
+                        const uint32_t at = tmem_base + as * kAccCols + ((uint32_t)(q * 32) << 16) + (uint32_t)(c0 + h);
+                        tmem_ld16(at, rg);
+                        tmem_ld16(at + 128u, ru);
+                        const int col = n0 + c0 + h;
+                        if (row < row_lim && col < g.N) {
+                            const bool second = col + 8 < g.N;             // N is a multiple of 8
+                            uint32_t ph[8], pl[8];
+#pragma unroll
+                            for (int e = 0; e < 8; ++e) {
+                                float a[2];
+#pragma unroll
+                                for (int i = 0; i < 2; ++i) {
+                                    const int j = 2 * e + i;
+                                    float gv = __uint_as_float(rg[j]), uv = __uint_as_float(ru[j]);
+                                    if (g.bias != nullptr && (e < 4 || second)) { gv += g.bias[col + j]; uv += g.bias[g.N + col + j]; }
+                                    a[i] = glu_value(gv, uv, g.act, g.act_limit);
+                                }
+                                ph[e] = pack_bf16x2(a[0], a[1]);
+                                pl[e] = pack_bf16x2(a[0] - bf16lo(ph[e]), a[1] - bf16hi(ph[e]));
+                            }
+                            uint16_t* oh = reinterpret_cast<uint16_t*>(g.out) + (size_t)row * g.ldo + col;
+                            uint16_t* ol = reinterpret_cast<uint16_t*>(g.out2) + (size_t)row * g.ldo + col;
+                            if (((g.ldo | g.N) & 15) == 0) {
+                                st_global_32b(oh, ph);
+                                st_global_32b(ol, pl);
+                            } else {
+                                *reinterpret_cast<uint4*>(oh) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+                                *reinterpret_cast<uint4*>(ol) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+                                if (second) {
+                                    *reinterpret_cast<uint4*>(oh + 8) = make_uint4(ph[4], ph[5], ph[6], ph[7]);
+                                    *reinterpret_cast<uint4*>(ol + 8) = make_uint4(pl[4], pl[5], pl[6], pl[7]);
+                                }
+                            }
+                        }
+                        __syncwarp();
+                    }
+                    continue;
+                }
                 uint32_t r[32];
                 tmem_ld32(tmem_base + as * kAccCols + ((uint32_t)(q * 32) << 16) + (uint32_t)c0, r);
                 if (DUAL == DUAL_B) {       // accumulator columns [0, BN) = W . hi, [BN, 2 BN) = W . lo

@@ -13,6 +13,7 @@
 #include <math.h>
 
 #include "common.cuh"
+#include "glu.cuh"
 #include "mma.cuh"
 
 namespace fl {
@@ -66,7 +67,6 @@ __device__ __forceinline__ float2 block_sum2(float2 v, float2* red) {     // two
     return red[32];
 }
 
-__device__ __forceinline__ float sigmoidf_(float z) { return 1.f / (1.f + expf(-z)); }
 
 // The tensor-core GEMMs take an f32 activation as two bf16 halves, v = hi + lo (about 16 mantissa bits): written by the kernel
 // that produces the activation, beside the f32 copy.  hi == nullptr: the exact path, nothing to write.
@@ -2076,16 +2076,6 @@ static __global__ void ly_gated_group_norm_kernel(const float* __restrict__ y, c
 // act 1: act[p, f] = gelu_tanh(g) * u,  gelu_tanh(z) = z/2 (1 + tanh(sqrt(2/pi) (z + 0.044715 z^3))).  bias [2F] (optional) is added
 // to gate | up first.  act 2: act[p, f] = relu(gu[p, f])^2 -- no gate matrix, gu has F columns.  act 3: act[p, f] = relu(g) * u.
 // act 4: act[p, f] = silu(g) * u.
-__device__ __forceinline__ float gelu_tanhf_(float g) { return 0.5f * g * (1.f + tanhf(0.7978845608028654f * (g + 0.044715f * g * g * g))); }
-__device__ __forceinline__ float glu_value(float g, float u, int act, float limit) {
-    if (act == 2) { g = fmaxf(g, 0.f); return g * g; }
-    if (act == 3) return fmaxf(g, 0.f) * u;
-    if (act == 4) return g * sigmoidf_(g) * u;
-    if (act == 1) return gelu_tanhf_(g) * u;
-    g = fminf(g, limit);
-    u = fminf(fmaxf(u, -limit), limit);
-    return g * sigmoidf_(1.702f * g) * (u + 1.f);
-}
 // One block per (row p, chunk of 256 V channels); V consecutive channels per thread (V = 4: F, the row strides ldg of gu and ldo of the
 // output, and the addresses in multiples of 4).
 template <int V>
@@ -2365,21 +2355,51 @@ static __global__ void ly_moe_combine_grouped_kernel(const float* __restrict__ e
         y[(size_t)row * W + c] = t;
     }
 }
-// Many rows: every expert runs over ALL rows on the tensor cores and a row keeps expert e's output times its routing weight (zero
-// when it did not pick e).  y (+)= w_e[row] * ye[row];  e < 0: the shared expert, weight sgate[row].  Experts in ascending order.
-static __global__ void ly_moe_accum_kernel(const float* __restrict__ ye, const int* __restrict__ sel, const float* __restrict__ wt, int top, int e,
-                                           const float* __restrict__ sgate, int first, int W, float* __restrict__ y) {
-    const int row = blockIdx.y;
-    float w = 0.f;
-    if (e < 0) w = sgate ? sgate[row] : 1.f;
-    else
-        for (int k = 0; k < top; ++k) w += sel[row * top + k] == e ? wt[row * top + k] : 0.f;
-    if (w == 0.f && !first) return;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < W; c += gridDim.x * blockDim.x) {
-        const size_t i = (size_t)row * W + c;
-        const float add = w != 0.f ? w * ye[i] : 0.f;
-        y[i] = first ? add : y[i] + add;
+// Many rows: the rows of expert e (list order) become a run of whole 128-row tiles, tiles [tile_off[e], tile_off[e + 1]) of gx_hi / gx_lo.
+// One block per (row, pick): copies the row's halves to its place and leaves that place (a row of gx) in pair_of; block 0 also writes
+// tile_off[E + 1].  grp_off: as ly_moe_lists_kernel left it.  Rows of a run's last tile behind its list are not written: their products
+// are computed and never read.
+static __global__ void __launch_bounds__(256) ly_moe_gather_runs_kernel(const uint16_t* __restrict__ hhi, const uint16_t* __restrict__ hlo, int W, const int* __restrict__ sel,
+                                                                        int top, int E, const int* __restrict__ grp_off, int* __restrict__ pair_of,
+                                                                        uint16_t* __restrict__ gx_hi, uint16_t* __restrict__ gx_lo, int* __restrict__ tile_off) {
+    __shared__ float red[33];
+    __shared__ int before[256];
+    const int i = blockIdx.x, e = sel[i], tid = threadIdx.x;
+    auto tiles = [&](int x) { return (grp_off[x + 1] - grp_off[x] + 127) / 128; };
+    int t = 0;
+    for (int x = tid; x < e; x += 256) t += tiles(x);
+    const int first = (int)block_sum((float)t, red);            // (whole numbers far below 2^24)
+    const size_t dst = (size_t)first * 128 + (pair_of[i] - grp_off[e]);
+    const size_t src = (size_t)(i / top) * W;
+    if (W % 8 == 0) {
+        for (int c = tid * 8; c < W; c += 256 * 8) {
+            *reinterpret_cast<uint4*>(gx_hi + dst * W + c) = *reinterpret_cast<const uint4*>(hhi + src + c);
+            *reinterpret_cast<uint4*>(gx_lo + dst * W + c) = *reinterpret_cast<const uint4*>(hlo + src + c);
+        }
+    } else {
+        for (int c = tid; c < W; c += 256) { gx_hi[dst * W + c] = hhi[src + c]; gx_lo[dst * W + c] = hlo[src + c]; }
     }
+    __syncthreads();
+    if (tid == 0) pair_of[i] = (int)dst;
+    if (i != 0) return;
+    // block 0: an exclusive prefix sum over the experts, each thread a stretch of them
+    const int per = (E + 255) / 256, x0 = min(E, tid * per), x1 = min(E, x0 + per);
+    int mine = 0;
+    for (int x = x0; x < x1; ++x) mine += tiles(x);
+    before[tid] = mine;
+    __syncthreads();
+    int at = 0;
+    for (int k = 0; k < tid; ++k) at += before[k];
+    for (int x = x0; x < x1; ++x) { tile_off[x] = at; at += tiles(x); }
+    if (tid == 255) tile_off[E] = at;
+}
+// relu(x)^2 over the runs' rows (a feed-forward without a gate): hi | lo halves.  grid (column chunks, row tiles of the capacity)
+static __global__ void __launch_bounds__(256) ly_relu2_runs_kernel(const float* __restrict__ x, int F, int E, const int* __restrict__ tile_off, uint16_t* __restrict__ ahi,
+                                                                   uint16_t* __restrict__ alo) {
+    if ((int)blockIdx.y >= tile_off[E]) return;
+    for (int r = blockIdx.y * 128; r < (int)blockIdx.y * 128 + 128; ++r)
+        for (int c = blockIdx.x * 1024 + threadIdx.x; c < min(F, (int)blockIdx.x * 1024 + 1024); c += 256)
+            split_store(ahi, alo, (size_t)r * F + c, glu_value(x[(size_t)r * F + c], 0.f, 2, 0.f));
 }
 
 // y[row, c] = sum_k wt[row, k] * eo[pair_of[row, k], c]  (pick order)  + sgate[row] * sh[row, c]
