@@ -5,6 +5,7 @@
 
 #include "layered_model.cuh"
 #include "layered_ops.cuh"
+#include "chunk_scan.cuh"
 #include "model.cuh"
 #include "synth.cuh"
 
@@ -1075,6 +1076,80 @@ static void launch_rec_scan(LaunchCtx& lc, const RecArgs& a, int n) {
     else go(ly_rec_scan_kernel<64, DELTA>, 64);
 }
 
+enum class Recurrence { scalar, gla, delta };
+// Portions of kCsMinTokens tokens and more take the chunked kernels (chunk_scan.cuh), in the serving precision: the exact mode's sums must
+// not depend on how a prompt was cut.  The chunked kernels read 16 bytes at a time and hold at most 128 state rows.
+static bool chunks_fit(const ChunkArgs& a, bool f32, const int* counts, int n) {
+    if (f32 || a.D > 128 || ((a.D | a.Dv | a.ld | a.off_q | a.off_k | a.off_v) & 3) != 0) return false;
+    for (int i = 0; i < n; ++i)
+        if (counts[i] >= kCsMinTokens) return true;
+    return false;
+}
+template <int DP>
+static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurrence kind, const int* counts, int n, cudaStream_t stream) {
+    constexpr size_t row = DP + kCsPad, tile = kCsC * row, sq = kCsC * kCsLdA;
+    constexpr size_t sm_in = (2 * tile + sq) * 4, sm_gla = (3 * tile + sq + kCsC / 16 * DP) * 4, sm_delta = (2 * tile + 2 * sq) * 4;
+    constexpr size_t sm_dstate = (DP * (kCsCols + kCsPad) + 2 * (2 * tile + kCsC * (kCsCols + kCsPad) + kCsC)) * 4;
+    constexpr size_t sm_out = (tile + DP * kCsLdA) * 4, sm_out2 = sm_out + 2 * sq * 4;
+    static bool attr_set = false;
+    if (!attr_set) {
+        auto room = [](auto kern, size_t smem) { FL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); };
+        room(ly_chunk_in_kernel<DP>, sm_in); room(ly_chunk_gla_kernel<DP>, sm_gla); room(ly_chunk_delta_kernel<DP>, sm_delta);
+        room(ly_chunk_delta_state_kernel<DP>, sm_dstate);
+        room(ly_chunk_out_kernel<DP, 0>, sm_out); room(ly_chunk_out_kernel<DP, 1>, sm_out); room(ly_chunk_out_kernel<DP, 2>, sm_out2);
+        attr_set = true;
+    }
+    int longs = 0, most = 0;
+    for (int i = 0; i < n; ++i)
+        if (counts[i] >= kCsMinTokens) { ++longs; most = std::max(most, (counts[i] + kCsC - 1) / kCsC); }
+    a.span = std::max(1, kCsChunks / longs);
+    const size_t held = (size_t)std::min(a.span, most) * longs, per = (size_t)a.H * a.D * a.Dv;
+    auto need = [&](auto& buf, size_t k) { if (buf.n < k) { FL_CUDA(cudaStreamSynchronize(stream)); buf.alloc(k); } };
+    need(y.cs_us, held * per); need(y.cs_dec, held * a.H * (kind == Recurrence::gla ? a.D : 1));
+    a.us = y.cs_us.p; a.dec = y.cs_dec.p;
+    if (kind == Recurrence::gla) { need(y.cs_qd, y.rows * a.H * a.D); a.qd = y.cs_qd.p; }
+    if (kind == Recurrence::delta) { need(y.cs_aq, held * a.H * kCsC * kCsC); need(y.cs_wk, held * a.H * kCsC * a.D); a.aq = y.cs_aq.p; a.wk = y.cs_wk.p; }
+    for (a.span0 = 0; a.span0 < most; a.span0 += a.span) {
+        int chunks = 0;
+        for (int i = 0; i < n; ++i)
+            if (counts[i] >= kCsMinTokens) chunks += std::max(0, std::min(a.span, (counts[i] + kCsC - 1) / kCsC - a.span0));
+        const dim3 grid(chunks, a.H), b(256);
+        if (kind == Recurrence::delta) {
+            launch(lc, "delta_chunks", 0, ly_chunk_delta_kernel<DP>, grid, b, sm_delta, a);
+            launch(lc, "delta_states", 0, ly_chunk_delta_state_kernel<DP>, dim3((a.Dv + kCsCols - 1) / kCsCols, a.H, n), b, sm_dstate, a);
+            launch(lc, "delta_chunks_out", 0, ly_chunk_out_kernel<DP, 2>, grid, b, sm_out2, a);
+            continue;
+        }
+        const bool gla = kind == Recurrence::gla;
+        if (gla) launch(lc, "gla_chunks", 0, ly_chunk_gla_kernel<DP>, grid, b, sm_gla, a);
+        else launch(lc, "ssm_chunks", 0, ly_chunk_in_kernel<DP>, grid, b, sm_in, a);
+        launch(lc, gla ? "gla_states" : "ssm_states", 0, ly_chunk_state_kernel, dim3((unsigned)((per / 4 + 255) / 256), n), b, 0, a, gla ? 1 : 0);
+        if (gla) launch(lc, "gla_chunks_out", 0, ly_chunk_out_kernel<DP, 1>, grid, b, sm_out, a);
+        else launch(lc, "ssm_chunks_out", 0, ly_chunk_out_kernel<DP, 0>, grid, b, sm_out, a);
+    }
+}
+// -> whether the token-serial kernel has sequences left
+static bool launch_chunks(fl_cache& c, LaunchCtx& lc, const ChunkArgs& a, Recurrence kind, const int* counts, int n) {
+    if (a.D <= 64) launch_chunks_dp<64>(*c.ly, lc, a, kind, counts, n, c.stream);
+    else launch_chunks_dp<128>(*c.ly, lc, a, kind, counts, n, c.stream);
+    for (int i = 0; i < n; ++i)
+        if (counts[i] < kCsMinTokens) return true;
+    return false;
+}
+// a recurrence with one decay per head and token
+template <bool DELTA>
+static void run_recurrence(fl_cache& c, LaunchCtx& lc, RecArgs ra, bool f32, const int* counts, int n) {
+    ChunkArgs ca{};
+    ca.src = ra.cv; ca.ld = ra.ldc; ca.off_q = ra.off_q; ca.off_k = ra.off_k; ca.off_v = ra.off_v; ca.ab = ra.ab; ca.dskip = ra.dskip;
+    ca.o = ra.o; ca.state = ra.state; ca.seq_row0 = ra.seq_row0; ca.seq_slot = ra.seq_slot; ca.seq_pos0 = ra.seq_pos0;
+    ca.n = n; ca.H = ra.H; ca.G = ra.G; ca.D = ra.D; ca.Dv = ra.Dv;
+    if (chunks_fit(ca, f32, counts, n)) {
+        ra.skip_from = kCsMinTokens;
+        if (!launch_chunks(c, lc, ca, DELTA ? Recurrence::delta : Recurrence::scalar, counts, n)) return;
+    }
+    launch_rec_scan<DELTA>(lc, ra, n);
+}
+
 // P = softmax of the score block's rows (see ly_attn_softmax_kernel)
 static void launch_attn_softmax(LayeredCache& y, LaunchCtx& lc, const int* row_pos, int row0, int H, int rows, int k_lo, int n_first, int nk, int nkp, int window,
                                 int keep_first, int chunk, float softcap, int sink, const float* sinkv) {
@@ -1401,11 +1476,11 @@ static void run_mixer(fl_cache& c, LaunchCtx& lc, const StepTab& st, const Layer
                    delta ? (const float*)nullptr : (const float*)lw.dskip, y.go.p, y.gla_state[gla_index].p, st.seq_row0, st.seq_slot, st.seq_pos0,
                    H, G, rows, Dv};
         if (delta) {
-            launch_rec_scan<true>(lc, ra, n);
+            run_recurrence<true>(c, lc, ra, m.f32, counts, n);
             launch(lc, "gla_out", 0, ly_gla_out_kernel, dim3((Ti * H + 7) / 8), dim3(256), 0, (const float*)y.go.p, (const float*)y.proj.p, lw.n_in, lw.off_g,
                    (const float*)lw.hnorm, eps, Ti, H, Dv, ldu, y.u.p, lw.tc_o ? uhi : (uint16_t*)nullptr, ulo);
         } else {
-            launch_rec_scan<false>(lc, ra, n);
+            run_recurrence<false>(c, lc, ra, m.f32, counts, n);
             const int inner = H * Dv, part = inner / d.norm_groups;
             launch(lc, "gated_group_norm", 0, ly_gated_group_norm_kernel, dim3(Ti, d.norm_groups), dim3(std::min(1024, std::max(64, (part + 31) / 32 * 32))), 0,
                    (const float*)y.go.p, (const float*)y.proj.p, lw.n_in, lw.off_g, (const float*)lw.hnorm, eps, inner, d.norm_groups, 0, ldu, y.u.p,
@@ -1417,7 +1492,7 @@ static void run_mixer(fl_cache& c, LaunchCtx& lc, const StepTab& st, const Layer
                (const float*)lw.decay, H, y.cv.p, y.rs.p);
         RecArgs ra{y.cv.p, lw.conv_ch, lw.off_q - lw.conv_off, lw.off_k - lw.conv_off, lw.off_v - lw.conv_off, y.rs.p, (const float*)nullptr, y.go.p,
                    y.gla_state[gla_index].p, st.seq_row0, st.seq_slot, st.seq_pos0, H, H, D, Dv};
-        launch_rec_scan<false>(lc, ra, n);
+        run_recurrence<false>(c, lc, ra, m.f32, counts, n);
         const bool v4 = ((inner | lw.n_in | lw.off_g | ldu) & 3) == 0;       // four channels per thread
         launch(lc, "gated_group_norm", 0, ly_gated_group_norm_kernel, dim3(Ti, 1), dim3(std::min(v4 ? 256 : 1024, std::max(64, ((v4 ? inner / 4 : inner) + 31) / 32 * 32))), 0,
                (const float*)y.go.p, (const float*)y.proj.p, lw.n_in, lw.off_g, (const float*)lw.hnorm, eps, inner, 1, 1, ldu, y.u.p,
@@ -1427,7 +1502,16 @@ static void run_mixer(fl_cache& c, LaunchCtx& lc, const StepTab& st, const Layer
         gemm(lc, "gemm_gla_decay", y.proj.p + lw.off_a, lw.n_in, lw.a2, H * D, d.decay_rank, y.la.p, H * D, Ti);
         GlaArgs ga{y.proj.p, lw.n_in, lw.off_q, lw.off_k, lw.off_v, y.la.p, lw.a2b, 1.f / d.tau, y.go.p, y.gla_state[gla_index].p, st.seq_row0,
                    st.seq_slot, st.seq_pos0, H, D, Dv, (float)(1.0 / std::sqrt((double)D))};
-        launch_gla_scan(lc, ga, n);
+        ChunkArgs gc{};
+        gc.src = ga.proj; gc.ld = ga.ldp; gc.off_q = ga.off_q; gc.off_k = ga.off_k; gc.off_v = ga.off_v; gc.z = ga.z; gc.zb = ga.zb; gc.inv_tau = ga.inv_tau;
+        gc.qscale = ga.qscale; gc.o = ga.o; gc.state = ga.state; gc.seq_row0 = ga.seq_row0; gc.seq_slot = ga.seq_slot; gc.seq_pos0 = ga.seq_pos0;
+        gc.n = n; gc.H = gc.G = H; gc.D = D; gc.Dv = Dv;
+        bool rest = true;
+        if (chunks_fit(gc, m.f32, counts, n)) {
+            ga.skip_from = kCsMinTokens;
+            rest = launch_chunks(c, lc, gc, Recurrence::gla, counts, n);
+        }
+        if (rest) launch_gla_scan(lc, ga, n);
         launch(lc, "gla_out", 0, ly_gla_out_kernel, dim3((Ti * H + 7) / 8), dim3(256), 0, (const float*)ga.o, (const float*)y.proj.p, lw.n_in, lw.off_g,
                (const float*)lw.hnorm, eps, Ti, H, Dv, ldu, y.u.p, lw.tc_o ? uhi : (uint16_t*)nullptr, ulo);
     } else {

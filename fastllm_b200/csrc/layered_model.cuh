@@ -167,6 +167,7 @@ struct LayeredCache {
     // serving precision: hi/lo halves of the activations that feed tensor-core GEMMs, and the split-K slices of their outputs
     DevBuf<uint16_t> h_hi, h_lo, cq_hi, cq_lo, qp_hi, qp_lo, qo_hi, qo_lo, ol_hi, ol_lo, u_hi, u_lo, act_hi, act_lo, hf_hi, hf_lo;
     DevBuf<float> gemm_out;
+    DevBuf<float> cs_us, cs_dec, cs_qd, cs_aq, cs_wk;   // chunked recurrences (chunk_scan.cuh)
     DevBuf<uint16_t> gx_hi, gx_lo, ga_hi, ga_lo;        // grouped expert GEMMs: gathered inputs / activations, [experts * cap] rows
     DevBuf<int> grp_cnt;
     // tensor-core latent attention of long portions: gathered keys, their transpose, Q / P operand halves, the score block

@@ -533,6 +533,7 @@ struct GlaArgs {
     const int *seq_row0, *seq_slot, *seq_pos0;
     int H, D, Dv;
     float qscale;
+    int skip_from = 0;          // > 0: sequences that bring at least this many tokens are left to the chunked kernels
 };
 constexpr int kGlaVS = 32, kGlaDG = 8;        // value columns per block, key-channel groups per block
 
@@ -551,6 +552,7 @@ static __global__ void __launch_bounds__(kGlaVS * kGlaDG) ly_gla_scan_kernel(Gla
     const int seq = blockIdx.x, hd = blockIdx.y, v0 = blockIdx.z * kGlaVS;
     const int tid = threadIdx.x, vc = tid & 31, dg = tid >> 5;
     const int r0 = a.seq_row0[seq], r1 = a.seq_row0[seq + 1];
+    if (a.skip_from > 0 && r1 - r0 >= a.skip_from) return;
     const bool vok = v0 + vc < Dv;
     float* st = a.state + (((size_t)a.seq_slot[seq] * a.H + hd) * D) * Dv + v0 + vc;
     float s[RPT];
@@ -1915,6 +1917,7 @@ struct RecArgs {
     float* state;               // [slots][H][D][Dv]
     const int *seq_row0, *seq_slot, *seq_pos0;
     int H, G, D, Dv;
+    int skip_from = 0;          // as for the gated linear attention
 };
 constexpr int kRecCols = 32, kRecParts = 4;       // value columns per block; threads that share a column's rows
 // Token by token, per head:  S <- a S;  u = b v   (DELTA: u = b (v - S^T k));  S <- S + k u^T;  o = S^T q (+ dskip v).
@@ -1938,6 +1941,7 @@ static __global__ void __launch_bounds__(128) ly_rec_scan_kernel(RecArgs a) {
     const bool vok = col < Dv;
     float* wsm = sm + wid * (NST * SLOT);
     const int r0 = a.seq_row0[seq], r1 = a.seq_row0[seq + 1];
+    if (a.skip_from > 0 && r1 - r0 >= a.skip_from) return;
     float* st = a.state + (((size_t)a.seq_slot[seq] * a.H + hd) * D) * Dv + col;
     float s[RPT];
     const bool fresh = a.seq_pos0[seq] == 0;

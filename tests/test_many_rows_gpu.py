@@ -5,6 +5,7 @@ elements that land on the other side of a rounding boundary, and a near-tied rou
 import numpy as np
 import pytest
 
+import test_medulorn_gpu as M
 import test_nifunex_gpu as N
 import test_rofetar_gpu as R
 import test_tozarax_gpu as T
@@ -39,3 +40,57 @@ def test_expert_runs_without_a_gate(n, ff):
 def test_gated_epilogue(n, ff, width):
     cfg = R.config([R.att(mlp=R.dense(ff=ff))], vocab=64, width=width)
     check(R, cfg, n, 35, 0.0)
+
+
+# ---- recurrences in chunks of 64 tokens (portions of at least 128) against the same model fed in portions that stay token by token ------
+# No cache is rounded in these models, so what is left between the two is the order of f32 sums in the recurrence and in the GEMMs around
+# it: a few 1e-7 per sum, some tens of sums and norms behind one another.
+CHUNK_TOL = 3e-5
+
+
+def recurrent(kind, dim, vdim, heads=2):
+    if kind == "gla":
+        return N, N.config([N.gla(heads=heads, dim=dim, vdim=vdim, tau=2.0, rank=4)], width=64)
+    if kind == "gla_fast_decay":
+        return N, N.config([N.gla(heads=heads, dim=dim, vdim=vdim, tau=0.05, rank=4)], width=64)
+    if kind == "mamba":
+        return R, R.config([R.mamba(heads=2 * heads, vdim=vdim, state=dim, groups=heads)], width=64)
+    return R, R.config([R.delta(heads=2 * heads, kv_heads=heads, dim=dim, vdim=vdim)], width=64)
+
+
+@pytest.mark.parametrize("kind", ["gla", "gla_fast_decay", "mamba", "delta"])
+@pytest.mark.parametrize("dim,vdim,n", [(16, 16, 128), (64, 64, 191), (68, 36, 129), (128, 68, 192), (100, 128, 321), (4, 132, 200)])
+def test_chunks_equal_token_by_token(kind, dim, vdim, n):
+    mod, cfg = recurrent(kind, dim, vdim)
+    _, model = mod.build(cfg, seed=41, dtype="bf16")
+    toks = mod.tokens(cfg, n, seed=42)
+    serial = mod.run_cut(model, toks, [100] * 4, cache=model.new_device_cache(2, 512))
+    whole = mod.run_whole(model, toks, cache=model.new_device_cache(2, 512))
+    assert mod.relerr(whole, np.asarray(serial, dtype=np.float64)) < CHUNK_TOL
+    # a portion of chunks behind a short one, and a short one behind it: the state passes both borders
+    cut = mod.run_cut(model, toks, [30, n - 40] if n >= 168 else [n], cache=model.new_device_cache(2, 512))
+    assert mod.relerr(cut, np.asarray(serial, dtype=np.float64)) < CHUNK_TOL
+
+
+@pytest.mark.parametrize("kind", ["gla", "mamba", "delta"])
+def test_chunks_of_several_sequences(kind):
+    """two prompts of more chunks than are held at a time beside a short one and a decoded token; a reused slot starts from zero"""
+    mod, cfg = recurrent(kind, 32, 32)
+    _, model = mod.build(cfg, seed=43, dtype="bf16")
+    lens = (1100, 3, 1090, 1)
+    reqs = [mod.tokens(cfg, k, seed=50 + i) for i, k in enumerate(lens)]
+    cache = model.new_device_cache(4, 1536)
+    for round_ in range(2):
+        got = cache.forward_ragged([2, 0, 3, 1], reqs, [list(range(k)) for k in lens])
+        at = 0
+        for r, k in zip(reqs, lens):
+            alone = mod.run_cut(model, r, [120] * 10, cache=model.new_device_cache(1, 1536))
+            assert mod.relerr(got[at:at + k], np.asarray(alone, dtype=np.float64)) < CHUNK_TOL
+            at += k
+        for s in range(4):
+            cache.slot_reset(s)
+
+
+@pytest.mark.parametrize("dim,vdim,n", [(16, 24, 128), (128, 128, 200), (64, 72, 333)])
+def test_lightning_chunks(dim, vdim, n):
+    check(M, M.config([M.par_layer(b=M.lightning(heads=2, dim=dim, vdim=vdim))], width=64), n, 45, 0.0)
