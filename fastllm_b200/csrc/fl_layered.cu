@@ -6,6 +6,7 @@
 #include "layered_model.cuh"
 #include "layered_ops.cuh"
 #include "chunk_scan.cuh"
+#include "gqa_attn_tc.cuh"
 #include "model.cuh"
 #include "synth.cuh"
 
@@ -1231,6 +1232,43 @@ static void latent_attn_tc(fl_cache& c, LaunchCtx& lc, const LatentAttnArgs& a, 
     }
 }
 
+// Grouped-query attention of rows [r0, r0 + Ts) -- one sequence's portion, positions pos0.. -- in one kernel (gqa_attn_tc.cuh): heads of up
+// to 128 channels whose results go to the output projection as halves.  -> false: this shape is gqa_attn_tc's
+template <int DK, int DV>
+static void launch_gqa_tc(LayeredCache& y, LaunchCtx& lc, const GqaAttnArgs& a, GqaTcArgs t, const int* page_row) {
+    static bool attr_set = false;
+    if (!attr_set) {
+        FL_CUDA(cudaFuncSetAttribute(ly_gqa_tc_kernel<DK, DV>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)gqa_tc_smem(DK, DV)));
+        attr_set = true;
+    }
+    const uint64_t nkp = (uint64_t)t.pg.pages * kKvPage;
+    launch(lc, "gqa_pages", 0, ly_gqa_pages_kernel<DK, DV>, dim3(t.pg.pages, a.G), dim3(256), 0, (const uint16_t*)a.pool, page_row, t.pg, t.pos0 + t.Ts, a.kv, a.D, a.Dv,
+           y.at_kc.p, y.at_kct.p);
+    const CUtensorMap tk = make_tmap_bf16(y.at_kc.p, a.G * nkp, DK, DK, kKvPage), tv = make_tmap_bf16(y.at_kct.p, (uint64_t)a.G * DV, nkp, nkp, DV);
+    launch(lc, "gqa_attn_tc", 0, ly_gqa_tc_kernel<DK, DV>, dim3((t.Ts + kGtQ - 1) / kGtQ, a.H), dim3(kGtThreads), gqa_tc_smem(DK, DV), tk, tv, t);
+}
+static bool gqa_attn_fused(fl_cache& c, LaunchCtx& lc, const GqaAttnArgs& a, int r0, int Ts, int pos0, int slot) {
+    if (a.D > 128 || a.Dv > 128 || ((a.D | a.Dv | a.ldo) & 7) != 0 || ((a.ldp | a.off_q) & 3) != 0 || a.ohi == nullptr) return false;
+    LayeredCache& y = *c.ly;
+    const int lo = std::max(a.window > 0 ? std::max(pos0 - a.window + 1, 0) : 0, a.chunk > 0 ? pos0 / a.chunk * a.chunk : 0);
+    GqaPages pg;
+    pg.base = lo / kKvPage;
+    pg.first = (a.window > 0 && a.keep_first > 0) ? std::min((a.keep_first + kKvPage - 1) / kKvPage, pg.base) : 0;
+    pg.pages = pg.first + (pos0 + Ts - 1) / kKvPage - pg.base + 1;
+    const int dk = a.D <= 64 ? 64 : 128, dv = a.Dv <= 64 ? 64 : 128;
+    const size_t keys = (size_t)a.G * pg.pages * kKvPage;
+    auto need = [&](auto& buf, size_t n) { if (buf.n < n) { FL_CUDA(cudaStreamSynchronize(c.stream)); buf.alloc(n + n / 4); } };
+    need(y.at_kc, keys * dk); need(y.at_kct, keys * dv);
+    const GqaTcArgs t{a.proj, a.ldp, a.off_q, r0, Ts, pos0, a.H, a.G, a.D, a.Dv, pg, a.window, a.keep_first, a.chunk, a.scale, a.softcap, a.sink, a.sinkv,
+                      a.ohi, a.olo, a.ldo, a.gate, 8.f};
+    const int* page_row = y.page_table.p + (size_t)slot * c.pages_per_seq;
+    if (dk == 64 && dv == 64) launch_gqa_tc<64, 64>(y, lc, a, t, page_row);
+    else if (dk == 64) launch_gqa_tc<64, 128>(y, lc, a, t, page_row);
+    else if (dv == 64) launch_gqa_tc<128, 64>(y, lc, a, t, page_row);
+    else launch_gqa_tc<128, 128>(y, lc, a, t, page_row);
+    return true;
+}
+
 // Grouped-query attention of rows [r0, r0 + Ts) -- one sequence's portion, positions pos0.. -- on the tensor-core GEMM: per block of
 // query rows and per key/value head a score GEMM whose rows are (token, query head of the group) pairs, an f32 softmax (score cap,
 // sink, causal mask) and a value GEMM; the block size keeps a score block within a fixed scratch budget.
@@ -1449,7 +1487,7 @@ static void run_mixer(fl_cache& c, LaunchCtx& lc, const StepTab& st, const Layer
                 at.row_base = done;
                 launch_gqa_attn<uint16_t>(lc, at, r0 - done, max_keys, true);
             }
-            gqa_attn_tc(c, lc, at, r0, Ts, h_pos0[si], slots[si]);
+            if (!gqa_attn_fused(c, lc, at, r0, Ts, h_pos0[si], slots[si])) gqa_attn_tc(c, lc, at, r0, Ts, h_pos0[si], slots[si]);
             done = r0 + Ts;
         }
         if (done < Ti) {

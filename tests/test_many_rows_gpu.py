@@ -9,6 +9,7 @@ import test_medulorn_gpu as M
 import test_nifunex_gpu as N
 import test_rofetar_gpu as R
 import test_tozarax_gpu as T
+import test_tufazen_gpu as U
 
 pytestmark = pytest.mark.gpu
 
@@ -94,3 +95,41 @@ def test_chunks_of_several_sequences(kind):
 @pytest.mark.parametrize("dim,vdim,n", [(16, 24, 128), (128, 128, 200), (64, 72, 333)])
 def test_lightning_chunks(dim, vdim, n):
     check(M, M.config([M.par_layer(b=M.lightning(heads=2, dim=dim, vdim=vdim))], width=64), n, 45, 0.0)
+
+
+# ---- grouped-query attention of a portion in one kernel ----------------------------------------------------------------------------------
+def both_ways(mod, cfg, n, cuts, seed):
+    oracle, model = mod.build(cfg, seed=seed, dtype="bf16")
+    toks = mod.tokens(cfg, n, seed=seed + 1)
+    ref = oracle.run(toks)
+    assert mod.relerr(mod.run_whole(model, toks, cache=model.new_device_cache(2, 1024)), ref) < mod.TOL["bf16"]
+    assert mod.relerr(mod.run_cut(model, toks, cuts, cache=model.new_device_cache(2, 1024)), ref) < mod.TOL["bf16"]
+
+
+# head sizes on both sides of 64 and up to 128, keys and values alike or not; portions of one page, a page and a row, a query tile and a row;
+# portions that start inside a page
+@pytest.mark.parametrize("dim,vdim,n", [(8, 8, 64), (16, 72, 65), (64, 64, 129), (72, 24, 200), (128, 128, 300), (120, 64, 257)])
+def test_attention_of_a_portion(dim, vdim, n):
+    cfg = R.config([R.att(heads=4, kv_heads=2, dim=dim, vdim=vdim, rot_dims=8), R.att(heads=2, kv_heads=2, dim=dim, vdim=vdim, rot_dims=4, kv_from=0)], width=64)
+    both_ways(R, cfg, n, [30, n - 31] if n >= 95 else [n - 1], 61)
+
+
+# windows with kept first keys (inside the window's first page, over two pages, none) and chunks, each longer than the 256 keys up to which
+# the per-row kernel is taken
+@pytest.mark.parametrize("window,keep,n", [(257, 2, 400), (300, 70, 520), (321, 0, 450)])
+def test_attention_windows_of_a_portion(window, keep, n):
+    both_ways(M, M.config([M.par_layer(M.windowed(dim=16, vdim=16, window=window, keep=keep), M.lightning(heads=2, dim=8, vdim=8))], width=64), n, [70, 201, 100], 63)
+
+
+def test_attention_chunks_of_a_portion():
+    both_ways(M, M.config([M.attn_layer(M.chunked(dim=16, vdim=16, chunk=270), mlp=None)], width=64), 600, [100, 300], 65)
+
+
+@pytest.mark.parametrize("dim,dims", [(16, 8), (24, 24), (128, 40)])
+def test_attention_with_gates_and_shared_values(dim, dims):
+    both_ways(U, U.bare([U.alayer(U.grouped(dim=dim, dims=dims))], width=64), 200, [77, 100], 67)
+
+
+def test_attention_sharp_scores():
+    """scores far apart: the running maximum moves and the accumulator is rescaled"""
+    both_ways(R, R.config([R.att(heads=2, kv_heads=1, dim=32, vdim=32, rot_dims=8, scale=6.0, softcap=None)], width=64), 300, [130, 100], 69)
