@@ -906,12 +906,27 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
 
 // The FMA-chain GEMM: f32 accumulators where it stands in for the tensor-core GEMM on shapes outside its tiles (serving precision),
 // f64 accumulators in the exact mode.
+static void launch_ly_gemm(LaunchCtx& lc, const char* tag, const LyGemm& g, int groups, int max_rows) {
+    const uint64_t bytes = (uint64_t)groups * g.N * g.K * 2;
+    if (!lc.exact) {
+        launch(lc, tag, bytes, ly_gemm_kernel, dim3((g.N + kLyBN - 1) / kLyBN, (max_rows + kLyBM - 1) / kLyBM, groups), dim3(256), 0, g);
+        return;
+    }
+    static bool attr_set = false;
+    if (!attr_set) {
+        FL_CUDA(cudaFuncSetAttribute(ly_gemm64_kernel<32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ly_gemm64_smem<32, 32>()));
+        FL_CUDA(cudaFuncSetAttribute(ly_gemm64_kernel<8, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ly_gemm64_smem<8, 64>()));
+        attr_set = true;
+    }
+    // up to 16 rows a tile of 32 would mostly multiply nothing (two tiles of eight: half the f64 work)
+    if (max_rows <= 16)
+        launch(lc, tag, bytes, ly_gemm64_kernel<8, 64>, dim3((g.N + 63) / 64, (max_rows + 7) / 8, groups), dim3(256), ly_gemm64_smem<8, 64>(), g);
+    else
+        launch(lc, tag, bytes, ly_gemm64_kernel<32, 32>, dim3((g.N + 31) / 32, (max_rows + 31) / 32, groups), dim3(256), ly_gemm64_smem<32, 32>(), g);
+}
 static void gemm(LaunchCtx& lc, const char* tag, const float* A, int lda, const uint16_t* Wt, int N, int K, float* Y, int ldy, int R) {
     if (R <= 0) return;
-    LyGemm g{A, 0, lda, nullptr, Wt, 0, N, K, Y, 0, ldy, nullptr, R};
-    const dim3 grid((N + kLyBN - 1) / kLyBN, (R + kLyBM - 1) / kLyBM, 1);
-    if (lc.exact) launch(lc, tag, (uint64_t)N * K * 2, ly_gemm_kernel<double>, grid, dim3(256), 0, g);
-    else launch(lc, tag, (uint64_t)N * K * 2, ly_gemm_kernel<float>, grid, dim3(256), 0, g);
+    launch_ly_gemm(lc, tag, LyGemm{A, 0, lda, nullptr, Wt, 0, N, K, Y, 0, ldy, nullptr, R}, 1, R);
 }
 // Y[R, N] = A[R, K] . Wt[N, K]^T on the tensor cores when the matrix has a descriptor (serving precision; A as hi | lo halves),
 // else on the exact kernel.  A tensor-core GEMM of few rows may leave split-K slices in the shared scratch: the caller hands them to
@@ -965,10 +980,7 @@ static bool ff_in_fused(int R, int F, int K, int act, bool tc_in, bool tc_out, c
 }
 
 static void gemm_groups(LaunchCtx& lc, const char* tag, const LyGemm& g, int groups, int max_rows) {
-    if (max_rows <= 0) return;
-    const dim3 grid((g.N + kLyBN - 1) / kLyBN, (max_rows + kLyBM - 1) / kLyBM, groups);
-    if (lc.exact) launch(lc, tag, (uint64_t)groups * g.N * g.K * 2, ly_gemm_kernel<double>, grid, dim3(256), 0, g);
-    else launch(lc, tag, (uint64_t)groups * g.N * g.K * 2, ly_gemm_kernel<float>, grid, dim3(256), 0, g);
+    if (max_rows > 0) launch_ly_gemm(lc, tag, g, groups, max_rows);
 }
 
 template <typename CT>

@@ -133,3 +133,16 @@ def test_attention_with_gates_and_shared_values(dim, dims):
 def test_attention_sharp_scores():
     """scores far apart: the running maximum moves and the accumulator is rescaled"""
     both_ways(R, R.config([R.att(heads=2, kv_heads=1, dim=32, vdim=32, rot_dims=8, scale=6.0, softcap=None)], width=64), 300, [130, 100], 69)
+
+
+# ---- the exact mode's GEMM -----------------------------------------------------------------------------------------------------------------
+@pytest.mark.parametrize("width,ff", [(64, 72), (50, 34), (36, 130)])
+def test_exact_gemm_rows_stand_alone(width, ff):
+    """f64 sums whose order depends on K alone: bitwise the same logits whether a token's row shares its tile with 7, 15, 16, 31, 32 others or
+    with none, aligned rows or not"""
+    cfg = R.config([R.delta(heads=4, kv_heads=2, dim=6, vdim=10, mlp=R.dense(ff=ff)), R.att(heads=4, kv_heads=2, dim=8, vdim=12, mlp=R.dense(ff=ff))], vocab=101, width=width)
+    oracle, model = R.build(cfg, seed=71)
+    toks = R.tokens(cfg, 110, seed=72)
+    whole = R.run_whole(model, toks, cache=model.new_device_cache(2, 128))
+    assert R.relerr(whole, oracle.run(toks)) < R.TOL["f32"]
+    assert np.array_equal(whole, R.run_cut(model, toks, [1, 8, 9, 16, 17, 32, 2], cache=model.new_device_cache(2, 128)))
