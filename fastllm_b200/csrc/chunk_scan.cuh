@@ -186,6 +186,7 @@ __device__ __forceinline__ void cs_decay_columns(float* sA, const float* sa, flo
 // ---- lightning attention, Mamba-2: one decay per head and token ---------------------------------------------------------------------
 template <int DP>
 static __global__ void __launch_bounds__(256, 2) ly_chunk_in_kernel(ChunkArgs a) {
+    pdl_chain();
     extern __shared__ __align__(16) float sm[];
     constexpr int LD = DP + kCsPad;
     float *sQ = sm, *sK = sQ + kCsC * LD, *sA = sK + kCsC * LD;        // the value slab takes the queries' place once they are used
@@ -229,6 +230,7 @@ static __global__ void __launch_bounds__(256, 2) ly_chunk_in_kernel(ChunkArgs a)
 // decayed from its block's start, the key to the end of the block before that, so every factor stays <= 1.
 template <int DP>
 static __global__ void __launch_bounds__(256) ly_chunk_gla_kernel(ChunkArgs a) {
+    pdl_chain();
     extern __shared__ __align__(16) float sm[];
     constexpr int LD = DP + kCsPad, B = 16, NB = kCsC / B;
     float *sQ = sm, *sK = sQ + kCsC * LD, *sF = sK + kCsC * LD, *sA = sF + kCsC * LD, *sB = sA + kCsC * kCsLdA;    // sF: the tokens' decays, then value slabs
@@ -330,6 +332,7 @@ static __global__ void __launch_bounds__(256) ly_chunk_gla_kernel(ChunkArgs a) {
 // us[chunk] <- S at the chunk's start; S <- dec[chunk] S + (what us[chunk] held).  Four state elements per thread, the next chunk's
 // addition on its way.  grid (H D Dv / 1024, sequences)
 static __global__ void __launch_bounds__(256) ly_chunk_state_kernel(ChunkArgs a, int dec_rows) {
+    pdl_chain();
     const int seq = blockIdx.y;
     int r0 = a.seq_row0[0], c0 = 0, cnt = 0, tokens = 0;
     for (int s = 0; s <= seq; ++s) {
@@ -365,6 +368,7 @@ static __global__ void __launch_bounds__(256) ly_chunk_state_kernel(ChunkArgs a,
 // o = A u + (decayed q) S with A from aq.
 template <int DP, int MODE>
 static __global__ void __launch_bounds__(256, 2) ly_chunk_out_kernel(ChunkArgs a) {
+    pdl_chain();
     extern __shared__ __align__(16) float sm[];
     constexpr int LD = DP + kCsPad;
     float *sQ = sm, *sS = sQ + kCsC * LD, *sA = sS + DP * kCsLdA, *sU = sA + kCsC * kCsLdA;      // sA, sU: MODE 2 alone
@@ -434,6 +438,7 @@ static __global__ void __launch_bounds__(256, 2) ly_chunk_out_kernel(ChunkArgs a
 // matrix in front of S_0 in wk, and the decayed (q_i . k_j) in aq.  T is built from its 16 x 16 diagonal blocks, by substitution.
 template <int DP>
 static __global__ void __launch_bounds__(256) ly_chunk_delta_kernel(ChunkArgs a) {
+    pdl_chain();
     extern __shared__ __align__(16) float sm[];
     constexpr int LD = DP + kCsPad, B = 16, NB = kCsC / B;
     float *sQ = sm, *sK = sQ + kCsC * LD, *sM = sK + kCsC * LD, *sT = sM + kCsC * kCsLdA;       // the value slab takes the queries' place
@@ -555,6 +560,7 @@ static __global__ void __launch_bounds__(256) ly_chunk_delta_kernel(ChunkArgs a)
 constexpr int kCsCols = 32;
 template <int DP>
 static __global__ void __launch_bounds__(256) ly_chunk_delta_state_kernel(ChunkArgs a) {
+    pdl_chain();
     extern __shared__ __align__(16) float sm[];
     constexpr int LD = DP + kCsPad, LC = kCsCols + kCsPad, STAGE = 2 * kCsC * LD + kCsC * LC + kCsC;
     float* sS = sm;                                 // [DP][LC]

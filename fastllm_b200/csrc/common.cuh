@@ -77,6 +77,9 @@ __device__ __forceinline__ float warp_max(float v) {
 // issue their first weight loads BEFORE pdl_wait() and overlap them with the producer's tail.
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// First statement of a kernel in a chain under programmatic dependent launch: the next kernel's blocks may be set up now, this one's work
+// starts when everything before it is complete and visible.  Every thread passes it, so a kernel never completes before its predecessor.
+__device__ __forceinline__ void pdl_chain() { pdl_launch_dependents(); pdl_wait(); }
 
 // ---- mbarrier / bulk-copy (TMA engine, 1-D) helpers ------------------------------------------------------
 

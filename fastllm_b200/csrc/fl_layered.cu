@@ -1401,7 +1401,11 @@ void layered_forward(fl_cache& c, const int* slots, const int* counts, int n, co
     // ---- device: layer by layer over all rows of the step ----
     LaunchCtx lc;
     lc.stream = c.stream;
-    lc.pdl = false;
+    // Programmatic dependent launch where the kernels are short enough for their set-up to count: a mixed step of 340 rows of width 2048 runs
+    // in 0.87 instead of 0.99 ms, 1531 rows in 2.14 instead of 2.17 ms.  Where a kernel fills the chip for long, the next one's waiting blocks
+    // only take its room: 2048 rows of width 4096 lose 1.5 %, the exact mode (two blocks of 70 KB per SM) 5 %.
+    static const bool no_pdl = env_flag("FL_NO_PDL");
+    lc.pdl = !no_pdl && !m.f32 && (size_t)T * m.W <= ((size_t)4 << 20);
     lc.exact = m.f32;
     // A step in which every sequence brings ONE token has a launch geometry that depends on (sequences, wanted rows) alone --
     // positions, slots and pages are read from the device tables -- so it is captured into a CUDA graph the second time the pair is

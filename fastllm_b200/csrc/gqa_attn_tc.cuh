@@ -65,6 +65,7 @@ struct GqaTcArgs {
 template <int DK, int DV>
 static __global__ void __launch_bounds__(256) ly_gqa_pages_kernel(const uint16_t* __restrict__ pool, const int* __restrict__ page_row, GqaPages pg, int end, KvLayout kv, int D,
                                                                   int Dv, uint16_t* __restrict__ kc, uint16_t* __restrict__ vt) {
+    pdl_chain();
     __shared__ uint16_t tile[DV][kKvPage + 2];
     const int b = blockIdx.x, g = blockIdx.y, page = pg.page(b), nkp = pg.pages * kKvPage, tid = threadIdx.x;
     const int keys = min(kKvPage, end - page * kKvPage);

@@ -77,6 +77,7 @@ __device__ __forceinline__ void split_store(uint16_t* hi, uint16_t* lo, size_t i
     lo[i] = f32_to_bf16_rne(v - __uint_as_float((uint32_t)h << 16));
 }
 static __global__ void ly_split_kernel(const float* __restrict__ x, size_t n, uint16_t* __restrict__ hi, uint16_t* __restrict__ lo) {
+    pdl_chain();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) split_store(hi, lo, i, x[i]);
 }
 // V consecutive floats at once (V = 4: one 16-byte access; the address must be 16-byte aligned) and their hi | lo halves
@@ -131,6 +132,7 @@ __device__ __forceinline__ void ld_slices(const Slices& s, size_t i, float (&o)[
 }
 // out[i] = sum over the split-K slices of a tensor-core GEMM, in slice order
 static __global__ void ly_sum_slices_kernel(const float* __restrict__ y, int nsl, size_t stride, size_t n, float* __restrict__ out) {
+    pdl_chain();
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         float t = 0.f;
         for (int k = 0; k < nsl; ++k) t += y[(size_t)k * stride + i];
@@ -166,6 +168,7 @@ static __global__ void ly_embed_norm_kernel(const uint16_t* __restrict__ embed, 
                                             const uint16_t* __restrict__ pos_tab, const int* __restrict__ row_pos, float escale,
                                             const float* __restrict__ en, BigramTab bg, const float* __restrict__ step, float* __restrict__ x,
                                             float* __restrict__ x0, float* __restrict__ h, uint16_t* __restrict__ hhi, uint16_t* __restrict__ hlo) {
+    pdl_chain();
     __shared__ float red[33];
     const int row = blockIdx.x;
     const uint16_t* be = nullptr;
@@ -230,6 +233,7 @@ template <int V>
 static __global__ void __launch_bounds__(1024) ly_post_norm_kernel(float* __restrict__ x, Slices y, const float* __restrict__ yb, const float* __restrict__ wb,
                                            NormW next, const float* __restrict__ ls, const float* __restrict__ x0, const float* __restrict__ step,
                                            float eps, int W, int plain, int split_x, float* __restrict__ h, uint16_t* __restrict__ hhi, uint16_t* __restrict__ hlo) {
+    pdl_chain();
     extern __shared__ __align__(16) float srow[];
     __shared__ float red[33];
     const size_t rb = (size_t)blockIdx.x * W;
@@ -304,6 +308,7 @@ static __global__ void __launch_bounds__(1024) ly_join_kernel(float* __restrict_
                                       float* __restrict__ hist, size_t hist_stride, int slot, const float* __restrict__ dw,
                                       const float* __restrict__ x0, const float* __restrict__ pstep, NormW next, float eps, int W, int split_x,
                                       float* __restrict__ h, uint16_t* __restrict__ hhi, uint16_t* __restrict__ hlo) {
+    pdl_chain();
     __shared__ float red[33];
     const int row = blockIdx.x;
     const size_t rb = (size_t)row * W;
@@ -397,6 +402,7 @@ template <int V>
 static __global__ void ly_sum_norm_kernel(float* __restrict__ x, const float* __restrict__ y, const float* __restrict__ yb, const float* __restrict__ y2,
                                           float alpha, float sa, float sb, const float* __restrict__ w, float eps, int W, int plain, int split_x,
                                           uint16_t* __restrict__ hhi, uint16_t* __restrict__ hlo) {
+    pdl_chain();
     extern __shared__ __align__(16) float srow[];
     __shared__ float red[33];
     const size_t rb = (size_t)blockIdx.x * W;
@@ -436,6 +442,7 @@ static __global__ void ly_sum_norm_kernel(float* __restrict__ x, const float* __
 
 // logits <- cap tanh(logits / cap)
 static __global__ void ly_softcap_kernel(float* __restrict__ z, size_t n, float cap) {
+    pdl_chain();
     const float inv = 1.f / cap;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) z[i] = cap * tanhf(z[i] * inv);
 }
@@ -443,6 +450,7 @@ static __global__ void ly_softcap_kernel(float* __restrict__ z, size_t n, float 
 // hf[i] = norm(x[want[i]]; w) * scale: the rows that go on to the vocabulary projection (scale: what the logits are multiplied by)
 static __global__ void ly_final_norm_kernel(const float* __restrict__ x, const int* __restrict__ want, NormW nw, float eps, int W,
                                             float scale, float* __restrict__ hf, uint16_t* __restrict__ hhi, uint16_t* __restrict__ hlo) {
+    pdl_chain();
     __shared__ float red[33];
     const float* xr = x + (size_t)want[blockIdx.x] * W;
     float ss = 0.f;
@@ -471,6 +479,7 @@ constexpr int kLyBM = 64, kLyBN = 64, kLyBK = 16;
 
 // (f32 accumulators: the serving precision's shapes outside the tensor-core tiles; the exact mode has ly_gemm64_kernel)
 static __global__ void __launch_bounds__(256) ly_gemm_kernel(LyGemm g) {
+    pdl_chain();
     __shared__ float As[kLyBK][kLyBM + 4];
     __shared__ float Ws[kLyBK][kLyBN + 4];
     const int grp = blockIdx.z;
@@ -535,6 +544,7 @@ __device__ __forceinline__ void mma_f64_884(double (&d)[2], double a, double b) 
 }
 template <int BM, int BN>
 static __global__ void __launch_bounds__(256, 2) ly_gemm64_kernel(LyGemm g) {
+    pdl_chain();
     constexpr int KT = 64, LD = KT + 4, STAGE = (BM + BN) * LD, MT = BM / 8, NT = BN / 8;
     constexpr int PA = BM * KT / 4, PW = BN * KT / 4, NA = (PA + 255) / 256, NWT = (PW + 255) / 256;      // 4-element pieces per stage / per thread
     extern __shared__ __align__(16) double sm64[];           // two stages of [BM][LD] | [BN][LD], then the warps' sums
@@ -671,6 +681,7 @@ constexpr int kGlaVS = 32, kGlaDG = 8;        // value columns per block, key-ch
 // dg, dg + 8, ... of its column in registers.  The order of operations per token does not depend on how a prompt was cut.
 template <int RPT>
 static __global__ void __launch_bounds__(kGlaVS * kGlaDG) ly_gla_scan_kernel(GlaArgs a) {
+    pdl_chain();
     extern __shared__ float sm[];
     const int D = a.D, Dv = a.Dv;
     float* sq = sm;                     // [2][D]
@@ -757,6 +768,7 @@ static __global__ void __launch_bounds__(kGlaVS * kGlaDG) ly_gla_scan_kernel(Gla
 // u[row, h, :] = o[row, h, :] / sqrt(mean o^2 + eps) * w[:] * silu(g[row, h, :])     (one warp per (row, head))
 static __global__ void ly_gla_out_kernel(const float* __restrict__ o, const float* __restrict__ proj, int ldp, int off_g, const float* __restrict__ w,
                                          float eps, int T, int H, int Dv, int ldo, float* __restrict__ u, uint16_t* __restrict__ uhi, uint16_t* __restrict__ ulo) {
+    pdl_chain();
     const int item = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (item >= T * H) return;
     const int row = item / H, hd = item % H;
@@ -787,6 +799,7 @@ __device__ __forceinline__ void turn_pair(float* q0, int D, int R, int half, int
 // The rotated parts of a row's queries [H][D + R] (expanded from a query latent) turn in place.
 static __global__ void ly_rotate_q_kernel(float* __restrict__ q, int ldq, const int* __restrict__ row_pos, const float* __restrict__ cosb,
                                           const float* __restrict__ sinb, int H, int D, int R, int rdims) {
+    pdl_chain();
     const int half = rdims / 2;
     const size_t at = (size_t)row_pos[blockIdx.x] * half;
     for (int i = threadIdx.x; i < H * half; i += blockDim.x) turn_pair(q + (size_t)blockIdx.x * ldq, D, R, half, i, cosb + at, sinb + at);
@@ -810,6 +823,7 @@ struct LatentAppendArgs {
 // they are folded as the columns are read, and the gate's columns are folded into proj for the kernel that reads them later.
 template <typename CT>
 static __global__ void __launch_bounds__(1024) ly_latent_append_kernel(LatentAppendArgs a) {
+    pdl_chain();
     __shared__ float2 red[33];
     const int row = blockIdx.x, pos = a.row_pos[row], tid = threadIdx.x, nt = blockDim.x;
     const size_t rb = (size_t)row * a.ldp;
@@ -935,6 +949,7 @@ constexpr int kLatWarps = 8;
 // channels); the eight partial results are merged at the end.  Which warp takes which key depends on the position alone.
 template <typename CT, int CPL>
 static __global__ void __launch_bounds__(kLatWarps * 32) ly_latent_attn_kernel(LatentAttnArgs a) {
+    pdl_chain();
     extern __shared__ float sm[];               // [kLatWarps][C] accumulators, then [kLatWarps][2] (max, sum)
     constexpr int RPL = 4;                      // rotated channels per lane (R <= 128)
     const int row = a.row_base + blockIdx.x, hd = blockIdx.y, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1017,6 +1032,7 @@ static __global__ void ly_latent_split_q_kernel(Slices q, int ldq, const int* __
                                                 const float* __restrict__ sinb, int H, int D, int R, int rdims, int C, int Ep, float scale,
                                                 uint16_t* __restrict__ phi, uint16_t* __restrict__ plo, uint16_t* __restrict__ qhi,
                                                 uint16_t* __restrict__ qlo) {
+    pdl_chain();
     // grid (rows, chunks): the chunks of a row share its heads' channels
     const int row = blockIdx.x, t0 = blockIdx.y * blockDim.x + threadIdx.x, nt = gridDim.y * blockDim.x;
     const size_t rb = (size_t)row * ldq;
@@ -1082,6 +1098,7 @@ inline size_t lat_mma_smem(int Ep, int MT) {
 }
 template <int MT, int NT>
 static __global__ void __launch_bounds__(256) ly_latent_mma_kernel(LatMmaArgs a) {
+    pdl_chain();
     constexpr int KPW = NT == 8 ? 5 : (NT == 4 ? 3 : 2);        // 16-channel steps per warp: 8 KPW >= (C + R) / 16, R <= 128
     constexpr int MR = MT * 16, TPR = 256 / MR, CPT = kLatTile / TPR;
     extern __shared__ __align__(16) uint8_t lsm[];
@@ -1304,6 +1321,7 @@ static __global__ void __launch_bounds__(256) ly_latent_mma_kernel(LatMmaArgs a)
 // One block per 64 keys x 64 columns: the tile passes through shared memory so that both copies are written in runs.
 static __global__ void __launch_bounds__(256) ly_attn_gather_keys_kernel(const uint16_t* __restrict__ pool, const int* __restrict__ page_row, int k_lo, int nk, int nkp,
                                                                          int C, int E, int Ep, uint16_t* __restrict__ kc, uint16_t* __restrict__ kct) {
+    pdl_chain();
     __shared__ uint16_t tile[64][66];
     const int r0 = blockIdx.x * 64, c0 = blockIdx.y * 64;
     for (int i = threadIdx.x; i < 64 * 64; i += 256) {
@@ -1325,6 +1343,7 @@ static __global__ void __launch_bounds__(256) ly_attn_gather_keys_kernel(const u
 // Q operand rows (token, head): [q~ * scale | rotated query part * scale | 0] as hi | lo halves
 static __global__ void ly_attn_build_q_kernel(const float* __restrict__ qa, const float* __restrict__ proj, int ldp, int off_q, int row0, int H, int D,
                                               int R, int C, int Ep, float scale, uint16_t* __restrict__ qhi, uint16_t* __restrict__ qlo) {
+    pdl_chain();
     const int t = blockIdx.x, hd = blockIdx.y, row = row0 + t;
     const float* qap = qa + ((size_t)row * H + hd) * C;
     const float* qrp = proj + (size_t)row * ldp + off_q + hd * (D + R) + D;
@@ -1356,6 +1375,7 @@ __device__ __forceinline__ KeySpan key_span(int pos, int window, int keep_first,
 static __global__ void ly_attn_softmax_kernel(const float* __restrict__ S, const int* __restrict__ row_pos, int row0, int H, int k_lo, int n_first, int nk,
                                               int nkp, int window, int keep_first, int chunk, float softcap, int sink, const float* __restrict__ sinkv,
                                               int keep, uint16_t* __restrict__ phi, uint16_t* __restrict__ plo) {
+    pdl_chain();
     extern __shared__ float srow[];
     __shared__ float red[33];
     const size_t r = blockIdx.x;
@@ -1459,6 +1479,7 @@ struct OutGate {
 // u[row, hd * Dv + c] *= gate (rows of u are ldo apart), with the hi | lo halves of the product
 static __global__ void ly_out_gate_kernel(float* __restrict__ u, int ldo, OutGate gate, int H, int Dv, int T, uint16_t* __restrict__ uhi,
                                           uint16_t* __restrict__ ulo) {
+    pdl_chain();
     const int n = H * Dv;
     const size_t total = (size_t)T * n;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -1477,6 +1498,7 @@ template <int NG>
 static __global__ void __launch_bounds__(256) ly_attn_softmax_warp_kernel(const float* __restrict__ S, const int* __restrict__ row_pos, int row0, int H, int rows,
                                                                           int k_lo, int nk, int nkp, int window, int chunk, float softcap, int sink,
                                                                           const float* __restrict__ sinkv, uint16_t* __restrict__ phi, uint16_t* __restrict__ plo) {
+    pdl_chain();
     const int r = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (r >= rows) return;
     const int pos = row_pos[row0 + r / H];
@@ -1547,6 +1569,7 @@ struct AttnPrepArgs {
 // the channel inside the whole projection.
 template <typename CT>
 static __global__ void __launch_bounds__(256) ly_attn_prep_kernel(AttnPrepArgs a) {
+    pdl_chain();
     extern __shared__ float sm[];               // [warps][D]
     __shared__ float red[33];
     const int row = blockIdx.x, pos = a.row_pos[row], lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
@@ -1671,6 +1694,7 @@ __device__ __forceinline__ float warp_sum_scatter(float (&v)[N], int lane) {
 // loaded without a branch between them (lanes behind the head's end read its last chunk; their query is zero and their sums are not used).
 template <typename CT, int CPL, int RB, bool VEC>
 static __global__ void __launch_bounds__(kGqaWarps * 32) ly_gqa_attn_kernel(GqaAttnArgs a) {
+    pdl_chain();
     extern __shared__ float sm[];               // [warps][RB][Dv] accumulators, then [warps][RB][2] (max, sum)
     const int row = a.row_base + blockIdx.x, hd0 = blockIdx.y * RB, split = blockIdx.z, S = gridDim.z;
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -1795,6 +1819,7 @@ static __global__ void __launch_bounds__(kGqaWarps * 32) ly_gqa_attn_kernel(GqaA
 // out == nullptr: only the halves are wanted.  roll: element i of a partial is channel (i + roll) mod Dv (see KvLayout).
 static __global__ void ly_gqa_merge_kernel(const float* __restrict__ part, int S, int H, int Dv, int sink, const float* __restrict__ sinkv, int row_base,
                                            int ldo, int roll, OutGate gate, float* __restrict__ out, uint16_t* __restrict__ ohi, uint16_t* __restrict__ olo) {
+    pdl_chain();
     const int row = row_base + blockIdx.x, hd = blockIdx.y;
     const float* pp = part + ((size_t)blockIdx.x * H + hd) * S * (Dv + 2);
     const float sv = sinkv ? sinkv[hd] : 0.f;
@@ -1828,6 +1853,7 @@ static __global__ void ly_gqa_merge_kernel(const float* __restrict__ part, int S
 // Rows r < n_first hold keys 0 .. n_first - 1 (kept first keys before k_lo), rows n_first + i key k_lo + i, i < nk.
 static __global__ void ly_gqa_gather_kv_kernel(const uint16_t* __restrict__ pool, const int* __restrict__ page_row, int k_lo, int n_first, int nk, int nkp,
                                                int E, int koff, int D, int Dp, int voff, int Dv, int roll, uint16_t* __restrict__ kc, uint16_t* __restrict__ vt) {
+    pdl_chain();
     const int r = blockIdx.x;
     const uint16_t* src = nullptr;
     if (r < n_first + nk) {
@@ -1843,6 +1869,7 @@ static __global__ void ly_gqa_gather_kv_kernel(const uint16_t* __restrict__ pool
 // Q operand rows (token t, head hq of group g): the prepared query times `scale`, zero padded to Dp, as hi | lo halves.  grid (nq, rep)
 static __global__ void ly_gqa_build_q_kernel(const float* __restrict__ proj, int ldp, int off_q, int row0, int rep, int g, int D, int Dp, float scale,
                                              uint16_t* __restrict__ qhi, uint16_t* __restrict__ qlo) {
+    pdl_chain();
     const int t = blockIdx.x, hq = blockIdx.y;
     const float* qp = proj + (size_t)(row0 + t) * ldp + off_q + (size_t)(g * rep + hq) * D;
     const size_t base = ((size_t)t * rep + hq) * Dp;
@@ -1852,6 +1879,7 @@ static __global__ void ly_gqa_build_q_kernel(const float* __restrict__ proj, int
 // apart, times the gate) and its hi | lo halves
 static __global__ void ly_gqa_scatter_kernel(const float* __restrict__ o, int nq, int G, int rep, int Dv, int row0, int ldo, OutGate gate, float* __restrict__ u,
                                              uint16_t* __restrict__ uhi, uint16_t* __restrict__ ulo) {
+    pdl_chain();
     const size_t total = (size_t)nq * G * rep * Dv;
     const int H = G * rep;
     for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
@@ -1893,6 +1921,7 @@ __device__ __forceinline__ float conv_silu(const ConvArgs& a, int row, int row0,
 }
 // After the rows of a step were convolved: the slot keeps the last taps - 1 inputs of each sequence.  grid (sequences, channel blocks).
 static __global__ void ly_conv_state_kernel(ConvArgs a) {
+    pdl_chain();
     const int seq = blockIdx.x, c = blockIdx.y * blockDim.x + threadIdx.x;
     if (c >= a.ch) return;
     const int r0 = a.seq_row0[seq], n = a.seq_row0[seq + 1] - r0, pos0 = a.seq_pos0[seq], slot = a.seq_slot[seq];
@@ -1908,6 +1937,7 @@ static __global__ void ly_conv_state_kernel(ConvArgs a) {
 template <int V>
 static __global__ void __launch_bounds__(128) ly_token_shift_kernel(ConvArgs a, const float* __restrict__ mu, float* __restrict__ out,
                                                                       uint16_t* __restrict__ ohi, uint16_t* __restrict__ olo) {
+    pdl_chain();
     const int row = blockIdx.x, c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
     if (c >= a.ch) return;
     const int seq = a.row_seq[row], pos = a.row_pos[row];
@@ -1930,6 +1960,7 @@ static __global__ void __launch_bounds__(128) ly_token_shift_kernel(ConvArgs a, 
 // ab[row, h] = (decay[h], 1): the scan's fixed fade and a write strength of one.  grid (rows, channel chunks of `chunk`).
 static __global__ void ly_lightning_prep_kernel(const float* __restrict__ proj, int ldp, int off, int ch, int chunk, const float* __restrict__ decay, int H,
                                                 float* __restrict__ cv, float* __restrict__ ab) {
+    pdl_chain();
     const int row = blockIdx.x, c0 = blockIdx.y * chunk, c1 = min(ch, c0 + chunk);
     const float* pr = proj + (size_t)row * ldp + off;
     if (((ldp | off | ch | chunk) & 3) == 0) {          // 16-byte rows: four channels per thread
@@ -1957,6 +1988,7 @@ static __global__ void ly_lightning_prep_kernel(const float* __restrict__ proj, 
 template <int V>
 static __global__ void __launch_bounds__(128) ly_input_conv_kernel(ConvArgs a, int rpb, int T, float* __restrict__ out, uint16_t* __restrict__ ohi,
                                                                      uint16_t* __restrict__ olo) {
+    pdl_chain();
     extern __shared__ __align__(16) float wsm[];
     const int c = (blockIdx.y * blockDim.x + threadIdx.x) * V;
     if (c >= a.ch) return;
@@ -1997,6 +2029,7 @@ static __global__ void __launch_bounds__(128) ly_input_conv_kernel(ConvArgs a, i
 // grid (rows, channel chunks of `chunk`): the first chunk's block also computes the per-head scalars.
 static __global__ void ly_mamba_prep_kernel(ConvArgs a, int chunk, int off_dt, const float* __restrict__ dt_bias, const float* __restrict__ a_log, int H,
                                             float* __restrict__ ab) {
+    pdl_chain();
     const int row = blockIdx.x, seq = a.row_seq[row], pos = a.row_pos[row];
     const int row0 = a.seq_row0[seq], pos0 = a.seq_pos0[seq], slot = a.seq_slot[seq];
     const int c0 = blockIdx.y * chunk, c1 = min(a.ch, c0 + chunk);
@@ -2014,6 +2047,7 @@ static __global__ void ly_mamba_prep_kernel(ConvArgs a, int chunk, int off_dt, c
 // grid (rows, channel chunks of `chunk`, a multiple of D: a q or k head never straddles two blocks).
 static __global__ void ly_delta_prep_kernel(ConvArgs a, int chunk, int off_b, int off_a, const float* __restrict__ dt_bias, const float* __restrict__ a_log,
                                             int H, int G, int D, float qscale, float* __restrict__ ab) {
+    pdl_chain();
     const int row = blockIdx.x, seq = a.row_seq[row], pos = a.row_pos[row];
     const int row0 = a.seq_row0[seq], pos0 = a.seq_pos0[seq], slot = a.seq_slot[seq];
     const int c0 = blockIdx.y * chunk, c1 = min(a.ch, c0 + chunk);
@@ -2057,6 +2091,7 @@ constexpr int kRecCols = 32, kRecParts = 4;       // value columns per block; th
 // so a token's step waits for no global load.  The order of operations per token does not depend on how a prompt was cut.
 template <int RPT, bool DELTA>
 static __global__ void __launch_bounds__(128) ly_rec_scan_kernel(RecArgs a) {
+    pdl_chain();
     extern __shared__ __align__(16) float sm[]; // [4 warps][NST tokens][k | q: 4 parts x (RPT + 4) each (the pad keeps the parts on different banks) | v x 8 | a | b | pad]
     constexpr int DP = RPT * kRecParts;         // rows, padded (rows >= D hold zeros and never change)
     constexpr int PS = RPT + 4, DPS = kRecParts * PS;      // floats per part / per vector in shared memory
@@ -2165,6 +2200,7 @@ static __global__ void __launch_bounds__(128) ly_rec_scan_kernel(RecArgs a) {
 static __global__ void ly_gated_group_norm_kernel(const float* __restrict__ y, const float* __restrict__ proj, int ldp, int off_z,
                                                   const float* __restrict__ w, float eps, int inner, int parts, int sig_after, int ldo, float* __restrict__ u,
                                                   uint16_t* __restrict__ uhi, uint16_t* __restrict__ ulo) {
+    pdl_chain();
     __shared__ float red[33];
     const int row = blockIdx.x, n = inner / parts, c0 = blockIdx.y * n;
     const float* yr = y + (size_t)row * inner + c0;
@@ -2214,6 +2250,7 @@ static __global__ void ly_gated_group_norm_kernel(const float* __restrict__ y, c
 template <int V>
 static __global__ void __launch_bounds__(256) ly_glu_kernel(Slices gu, int ldg, int ldo, int F, float limit, int act_kind, const float* __restrict__ bias, float* __restrict__ act,
                                                             uint16_t* __restrict__ ahi, uint16_t* __restrict__ alo) {
+    pdl_chain();
     const int f = (blockIdx.y * 256 + threadIdx.x) * V;
     if (f >= F) return;
     const size_t p = blockIdx.x, base = p * (size_t)ldg + f;
@@ -2240,6 +2277,7 @@ static __global__ void __launch_bounds__(256) ly_glu_kernel(Slices gu, int ldg, 
 // layer's columns first), z [rows, D] perhaps still in split-K slices.  a == nullptr: only the halves are read.
 static __global__ void ly_token_side_kernel(Slices z, const int* __restrict__ tok, const uint16_t* __restrict__ e, size_t lde, int D, float* __restrict__ a,
                                             uint16_t* __restrict__ ahi, uint16_t* __restrict__ alo) {
+    pdl_chain();
     const int row = blockIdx.x;
     const uint16_t* er = e + (size_t)tok[row] * lde;
     for (int j = threadIdx.x; j < D; j += blockDim.x) {
@@ -2256,6 +2294,7 @@ static __global__ void ly_token_side_kernel(Slices z, const int* __restrict__ to
 // rb (optional): a bias [E] added to the logits.  (Softmax over all, then renormalised over the chosen = softmax over the chosen alone.)
 static __global__ void ly_router_kernel(const float* __restrict__ h, int W, const float* __restrict__ wr, const float* __restrict__ rb, int E, int top,
                                         const float* __restrict__ wsg, int* __restrict__ sel, float* __restrict__ wt, float* __restrict__ sgate) {
+    pdl_chain();
     extern __shared__ float z[];                 // [E]
     const int row = blockIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const float* hr = h + (size_t)row * W;
@@ -2312,6 +2351,7 @@ template <int RB>
 static __global__ void __launch_bounds__(256) ly_router_groups_kernel(const float* __restrict__ h, int W, const float* __restrict__ wr, int E, int top, int softmax,
                                                const float* __restrict__ corr, int groups, int keep, int mark2, int renorm, int T, int* __restrict__ sel,
                                                float* __restrict__ wt) {
+    pdl_chain();
     extern __shared__ float zs[];                // per row: [E] scores s, [E] choice scores c, [groups] marks
     const int row0 = blockIdx.x * RB, lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5, per_row = 2 * E + groups;
     const int nr = min(RB, T - row0);
@@ -2413,6 +2453,7 @@ static __global__ void __launch_bounds__(256) ly_router_groups_kernel(const floa
 // its own, a second places its picks by ballot compaction -- stable, so the lists do not depend on timing.
 static __global__ void ly_moe_lists_kernel(const int* __restrict__ sel, int T, int top, int E, int* __restrict__ grp_off, int* __restrict__ pair_row,
                                            int* __restrict__ pair_of) {
+    pdl_chain();
     const int e = blockIdx.x, lane = threadIdx.x, n = T * top;
     int less = 0, mine = 0;
     for (int i = lane; i < n; i += 32) {
@@ -2446,6 +2487,7 @@ static __global__ void ly_moe_lists_kernel(const int* __restrict__ sel, int T, i
 static __global__ void ly_moe_gather_kernel(const uint16_t* __restrict__ hhi, const uint16_t* __restrict__ hlo, int W, const int* __restrict__ grp_off,
                                             const int* __restrict__ pair_row, int cap, uint16_t* __restrict__ gx_hi, uint16_t* __restrict__ gx_lo,
                                             int* __restrict__ cnt) {
+    pdl_chain();
     const int e = blockIdx.x, lo = grp_off[e], n = grp_off[e + 1] - lo;
     if (blockIdx.y == 0 && threadIdx.x == 0) cnt[e] = n;
     for (int i = blockIdx.y; i < n; i += gridDim.y) {
@@ -2457,6 +2499,7 @@ static __global__ void ly_moe_gather_kernel(const uint16_t* __restrict__ hhi, co
 // i < cnt[e] only -> hi | lo.
 static __global__ void ly_glu_grouped_kernel(const float* __restrict__ gu, int nsl, size_t sl_stride, int F, float limit, int act_kind,
                                              const int* __restrict__ cnt, int cap, uint16_t* __restrict__ ahi, uint16_t* __restrict__ alo) {
+    pdl_chain();
     const int r = blockIdx.y;                   // row e * cap + i
     if (r % cap >= cnt[r / cap]) return;
     for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < F; f += gridDim.x * blockDim.x) {
@@ -2474,6 +2517,7 @@ static __global__ void ly_moe_combine_grouped_kernel(const float* __restrict__ e
                                                      const int* __restrict__ pair_of, const int* __restrict__ grp_off, int cap,
                                                      const float* __restrict__ wt, int top, const float* __restrict__ sh, const float* __restrict__ sgate,
                                                      int W, float* __restrict__ y) {
+    pdl_chain();
     const int row = blockIdx.y;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < W; c += gridDim.x * blockDim.x) {
         float t = 0.f;
@@ -2495,6 +2539,7 @@ static __global__ void ly_moe_combine_grouped_kernel(const float* __restrict__ e
 static __global__ void __launch_bounds__(256) ly_moe_gather_runs_kernel(const uint16_t* __restrict__ hhi, const uint16_t* __restrict__ hlo, int W, const int* __restrict__ sel,
                                                                         int top, int E, const int* __restrict__ grp_off, int* __restrict__ pair_of,
                                                                         uint16_t* __restrict__ gx_hi, uint16_t* __restrict__ gx_lo, int* __restrict__ tile_off) {
+    pdl_chain();
     __shared__ float red[33];
     __shared__ int before[256];
     const int i = blockIdx.x, e = sel[i], tid = threadIdx.x;
@@ -2529,6 +2574,7 @@ static __global__ void __launch_bounds__(256) ly_moe_gather_runs_kernel(const ui
 // relu(x)^2 over the runs' rows (a feed-forward without a gate): hi | lo halves.  grid (column chunks, row tiles of the capacity)
 static __global__ void __launch_bounds__(256) ly_relu2_runs_kernel(const float* __restrict__ x, int F, int E, const int* __restrict__ tile_off, uint16_t* __restrict__ ahi,
                                                                    uint16_t* __restrict__ alo) {
+    pdl_chain();
     if ((int)blockIdx.y >= tile_off[E]) return;
     for (int r = blockIdx.y * 128; r < (int)blockIdx.y * 128 + 128; ++r)
         for (int c = blockIdx.x * 1024 + threadIdx.x; c < min(F, (int)blockIdx.x * 1024 + 1024); c += 256)
@@ -2538,6 +2584,7 @@ static __global__ void __launch_bounds__(256) ly_relu2_runs_kernel(const float* 
 // y[row, c] = sum_k wt[row, k] * eo[pair_of[row, k], c]  (pick order)  + sgate[row] * sh[row, c]
 static __global__ void ly_moe_combine_kernel(const float* __restrict__ eo, const int* __restrict__ pair_of, const float* __restrict__ wt, int top,
                                              const float* __restrict__ sh, const float* __restrict__ sgate, int W, float* __restrict__ y) {
+    pdl_chain();
     const int row = blockIdx.y;
     for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < W; c += gridDim.x * blockDim.x) {
         float t = 0.f;
