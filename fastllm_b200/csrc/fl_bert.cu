@@ -4,6 +4,7 @@
 #include <memory>
 
 #include "bert.cuh"
+#include "bert_small.cuh"
 #include "bert_model.cuh"
 #include "gemm_tc.cuh"
 #include "synth.cuh"
@@ -264,6 +265,12 @@ void bert_finalize(BertModel& m) {
         w.tm_wi = make_tmap_bf16(w.wi, m.I, m.H, m.H, kBertBN);
         w.tm_wo2 = make_tmap_bf16(w.wo2, m.H, m.I, m.I, kBertBN);
     }
+    if (m.H == kBsH && m.I == kBsI && m.nh == kBsHeads) {
+        std::vector<BertSmallLayer> tab;
+        for (const BertLayerW& w : m.layers) tab.push_back({w.wqkv, w.wo, w.wi, w.wo2, w.bqkv, w.bo, w.bi, w.bo2, w.ln1w, w.ln1b, w.ln2w, w.ln2b});
+        m.small_layers.alloc(tab.size() * sizeof(BertSmallLayer));
+        FL_CUDA(cudaMemcpy(m.small_layers.p, tab.data(), tab.size() * sizeof(BertSmallLayer), cudaMemcpyHostToDevice));
+    }
     m.finalized = true;
 }
 
@@ -279,8 +286,60 @@ static void bert_reserve(BertModel& m, int b, int t) {
     m.h_ids.alloc(2 * Tc); m.h_out.alloc(m.cap_batch * H);
 }
 
+// Few short sentences: the whole encoder in one launch of clusters (bert_small.cuh).  -> false: the launch chain takes the call.
+// The line lies where the clusters (about nine of 16 blocks) are all resident and none has more than 64 tokens: a second wave would cost what
+// the chain does (0.26 ms, whatever it has below some hundred tokens).
+constexpr int kBsCluster = 16;
+template <int MT>
+static bool bert_small_launch(BertModel& m, const BertSmallArgs& a, int clusters, bool ask) {
+    auto kern = bert_small_kernel<MT, kBsCluster>;
+    static bool attr_set = false;
+    if (!attr_set) {
+        FL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bert_small_smem<MT, kBsCluster>()));
+        FL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+        attr_set = true;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(clusters * kBsCluster);
+    cfg.blockDim = dim3(kBsThreads);
+    cfg.dynamicSmemBytes = bert_small_smem<MT, kBsCluster>();
+    cfg.stream = m.stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = kBsCluster;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    if (ask) {
+        int n = 0;
+        if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
+        m.small_clusters = n;
+        return true;
+    }
+    FL_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
+    g_launches.fetch_add(1, std::memory_order_relaxed);
+    return true;
+}
+static bool bert_enqueue_small(BertModel& m, int b, int t, bool has_mask) {
+    if (m.small_layers.n == 0 || t > kBsTokens) return false;
+    if (m.small_clusters < 0) bert_small_launch<kBsTokens / 16>(m, BertSmallArgs{}, 1, true);
+    if (m.small_clusters < 1) return false;
+    // as many clusters as fit at a time, each with as few sentences as that leaves: up to 64 tokens per cluster
+    const int spc = (b + m.small_clusters - 1) / m.small_clusters, clusters = (b + spc - 1) / spc, rows = spc * t;
+    if (rows > kBsTokens) return false;
+    const BertSmallArgs a{reinterpret_cast<const BertSmallLayer*>(m.small_layers.p), m.wemb, m.pemb, m.lnw, m.lnb, m.ids.p, has_mask ? m.mask.p : nullptr,
+                          m.L, b, t, m.V, m.maxpos, spc, m.cfg.norm_eps, (float)(1.0 / std::sqrt((double)m.d)), m.qkv.p, m.ctx.p, m.hbuf.p, m.pre.p, m.out.p};
+    switch ((rows + 15) / 16) {
+        case 1: return bert_small_launch<1>(m, a, clusters, false);
+        case 2: return bert_small_launch<2>(m, a, clusters, false);
+        case 3: return bert_small_launch<3>(m, a, clusters, false);
+        default: return bert_small_launch<4>(m, a, clusters, false);
+    }
+}
+
 // Enqueue the encoder on m.stream: B1 -> 6 x (B2..B7) -> B8
 static void bert_enqueue(BertModel& m, int b, int t, bool has_mask) {
+    if (bert_enqueue_small(m, b, t, has_mask)) return;
     const int T = b * t, H = m.H, I = m.I;
     cudaStream_t st = m.stream;
     const int rows_per_cta = 8;

@@ -1,0 +1,28 @@
+"""The encoder's one-launch kernel (up to 64 tokens per cluster of blocks) against the oracle, at the edges of its row tiles and clusters."""
+import numpy as np
+import pytest
+
+from oracle import bert as obert
+from oracle import synth
+
+import test_bert_gpu as B
+
+pytestmark = pytest.mark.gpu
+
+
+# one token; a row tile and a row on both sides of it; the most tokens of a cluster; several sentences per cluster with a last one that holds
+# fewer; more sentences than clusters; one token or one sentence too many (the launch chain)
+@pytest.mark.parametrize("b,t", [(1, 1), (1, 16), (1, 17), (1, 33), (1, 64), (3, 21), (8, 64), (9, 30), (20, 5), (37, 7), (256, 2), (1, 65), (40, 40)])
+def test_short_sentences(b, t):
+    cfg = obert.MINILM_L6
+    w = obert.synth_weights(cfg, 0, 0.02)
+    m = B._product(cfg, w)
+    ids = synth.token_ids(500 + t, cfg.vocab_size, (b, t))
+    mask = np.ones((b, t), dtype=np.uint32)
+    mask[1:, -(t // 3):] = 0 if t >= 3 else 1
+    for k in (None, mask):
+        want, got = obert.MiniLM(cfg, w).embed_ids(ids, k), m.embed_ids(ids, k)
+        assert B._cos(got, want).min() >= B.COS_TOL and np.abs(got - want).max() <= 2e-2
+    # a sentence's embedding is that of the sentence alone, beyond the order of sums
+    alone = m.embed_ids(ids[-1:])
+    assert B._cos(alone, m.embed_ids(ids)[-1:]).min() >= B.COS_TOL
