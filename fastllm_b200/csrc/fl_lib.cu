@@ -1909,6 +1909,37 @@ FL_EXPORT int fl_cache_destroy(fl_cache* c) {
     FL_API_END
 }
 
+// A step's logits to the caller's buffer, through the pinned one; returns when they are there.  From 4 MB on the caller's pages are touched
+// while the device still computes (new ones cost a fault each) and the transfer goes in parts, each copied on while the next arrives.
+// 64 rows of 32000 logits behind a device step of 0.6 ms, whole call: 1.25 -> 1.15 ms (copying with helper threads: no faster here, they wake up late).
+static void deliver_logits(cudaStream_t stream, const float* dev, float* pinned, float* host, size_t n) {
+    constexpr size_t kPart = 512 * 1024;                // floats
+    constexpr int kMaxParts = 16;
+    const int parts = (int)std::min<size_t>(kMaxParts, n / kPart);
+    if (parts < 2) {
+        FL_CUDA(cudaMemcpyAsync(pinned, dev, n * 4, cudaMemcpyDeviceToHost, stream));
+        FL_CUDA(cudaStreamSynchronize(stream));
+        std::memcpy(host, pinned, n * 4);
+        return;
+    }
+    struct Events {
+        cudaEvent_t e[kMaxParts] = {};
+        ~Events() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
+    } ev;
+    auto at = [&](int p) { return n * (size_t)p / parts; };
+    for (int p = 0; p < parts; ++p) {
+        FL_CUDA(cudaMemcpyAsync(pinned + at(p), dev + at(p), (at(p + 1) - at(p)) * 4, cudaMemcpyDeviceToHost, stream));
+        FL_CUDA(cudaEventCreateWithFlags(&ev.e[p], cudaEventDisableTiming));
+        FL_CUDA(cudaEventRecord(ev.e[p], stream));
+    }
+    volatile char* page = reinterpret_cast<volatile char*>(host);
+    for (size_t i = 0; i < n * 4; i += 4096) page[i] = 0;
+    for (int p = 0; p < parts; ++p) {
+        FL_CUDA(cudaEventSynchronize(ev.e[p]));
+        std::memcpy(host + at(p), pinned + at(p), (at(p + 1) - at(p)) * 4);
+    }
+}
+
 FL_EXPORT int fl_forward(fl_model* m, fl_cache* c, const uint32_t* ids, int b, int t, size_t rope_offset, float* logits_host) {
     FL_API_BEGIN
     FL_CHECK(m && c && logits_host, FL_ERR_INVALID, "NULL argument");
@@ -1928,10 +1959,8 @@ FL_EXPORT int fl_forward(fl_model* m, fl_cache* c, const uint32_t* ids, int b, i
     try {
         run_forward(*c, ids, b, t, rope_offset);
         const size_t n = (size_t)b * c->w->Vfull;
-        FL_CUDA(cudaMemcpyAsync(c->h_logits.p, c->logits.p, n * 4, cudaMemcpyDeviceToHost, c->stream));
-        FL_CUDA(cudaStreamSynchronize(c->stream));
+        deliver_logits(c->stream, c->logits.p, c->h_logits.p, logits_host, n);
         check_peer_error();
-        std::memcpy(logits_host, c->h_logits.p, n * 4);
     } catch (const fl::Error& e) {
         if (e.code == FL_ERR_CUDA || e.code == FL_ERR_NCCL) c->poisoned = true;   // a missed peer leaves kv_len / exchange epochs out of step
         throw;
@@ -2127,10 +2156,8 @@ FL_EXPORT int fl_forward_slots(fl_model* m, fl_cache* c, const int* slots, const
     try {
         run_forward_slots(*c, slots, ids, n, t, rope_offsets);
         const size_t cnt = (size_t)n * c->w->Vfull;
-        FL_CUDA(cudaMemcpyAsync(c->h_logits.p, c->logits.p, cnt * 4, cudaMemcpyDeviceToHost, c->stream));
-        FL_CUDA(cudaStreamSynchronize(c->stream));
+        deliver_logits(c->stream, c->logits.p, c->h_logits.p, logits_host, cnt);
         check_peer_error();
-        std::memcpy(logits_host, c->h_logits.p, cnt * 4);
     } catch (const fl::Error& e) {
         if (e.code == FL_ERR_CUDA || e.code == FL_ERR_NCCL) c->poisoned = true;
         throw;
