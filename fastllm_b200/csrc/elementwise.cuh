@@ -58,6 +58,35 @@ static __global__ void argmax_finalize_kernel(const float* __restrict__ val, con
     }
 }
 
+// The same for the dense path: val / idx [row][parts] -> next_ids[row].  One block of 64 threads per row.
+constexpr int kArgmaxParts = 320;
+static __global__ void __launch_bounds__(64) argmax_rows_kernel(const float* __restrict__ val, const int* __restrict__ idx, int parts, uint32_t* __restrict__ next_ids) {
+    pdl_launch_dependents();
+    pdl_wait();
+    __shared__ float sv[2];
+    __shared__ int si[2];
+    const size_t row = (size_t)blockIdx.x * parts;
+    float v = -INFINITY;
+    int i = -1;
+    for (int p = threadIdx.x; p < parts; p += 64) {
+        const float ov = val[row + p];
+        const int oi = idx[row + p];
+        if (ov > v || (ov == v && oi > i)) { v = ov; i = oi; }
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xFFFFFFFFu, v, o);
+        const int oi = __shfl_xor_sync(0xFFFFFFFFu, i, o);
+        if (ov > v || (ov == v && oi > i)) { v = ov; i = oi; }
+    }
+    if ((threadIdx.x & 31) == 0) { sv[threadIdx.x >> 5] = v; si[threadIdx.x >> 5] = i; }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        if (sv[1] > v || (sv[1] == v && si[1] > i)) i = si[1];
+        next_ids[blockIdx.x] = (uint32_t)i;
+    }
+}
+
 // End of a forward call: kv_base[seq] += t.  In the device-resident greedy loop also rope_pos += 1 and ids <- next_ids.
 static __global__ void advance_state_kernel(StepState* st, int b, int t, int rope_inc, uint32_t* ids, const uint32_t* next_ids, int feedback,
                                      uint32_t* trace, int* trace_pos) {

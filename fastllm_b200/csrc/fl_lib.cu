@@ -839,6 +839,7 @@ static void cache_create(fl_cache& c, int max_batch, int max_seq) {
     c.amax_parts = kNumSMs * 4;
     c.amax_val.alloc((size_t)kPassRows * c.amax_parts);
     c.amax_idx.alloc((size_t)kPassRows * c.amax_parts);
+    c.am_val.alloc((size_t)max_batch * kArgmaxParts); c.am_idx.alloc((size_t)max_batch * kArgmaxParts);
     c.h_ids.alloc((size_t)max_batch * max_seq);
     c.h_logits.alloc((size_t)max_batch * w.Vfull);
     c.slot_len.assign(max_batch, 0);
@@ -872,6 +873,13 @@ static void cache_destroy_graphs(fl_cache& c) {
 // pass-major / layer-minor: a token's layer-l attention only needs the layer-l K/V of EARLIER tokens, which earlier
 // passes already appended, so the order is causal-correct.
 static void enqueue_forward_dense(fl_cache& c, LaunchCtx& lc, int b, int t, bool loop_mode);
+
+// logits of b rows from the slices of the lm_head's output, and their arg-max: parts of at least 512 logits, about four blocks per SM in all
+static void launch_argmax(fl_cache& c, LaunchCtx& lc, const float* y, int nsl, long long stride, int V, int b) {
+    const int parts = std::max(1, std::min(std::min((V + 511) / 512, kArgmaxParts), 4 * kNumSMs / b));
+    launch(lc, "dense_argmax", 0, dense_argmax_kernel, dim3(parts, b), dim3(256), 0, y, nsl, stride, V, c.logits.p, c.am_val.p, c.am_idx.p);
+    launch(lc, "argmax_finalize", 0, argmax_rows_kernel, dim3(b), dim3(64), 0, (const float*)c.am_val.p, (const int*)c.am_idx.p, parts, c.next_ids.p);
+}
 
 static void enqueue_forward(fl_cache& c, LaunchCtx& lc, int b, int t, bool loop_mode) {
     const Weights& w = *c.w;
@@ -986,8 +994,7 @@ static void enqueue_forward(fl_cache& c, LaunchCtx& lc, int b, int t, bool loop_
     if (w.tp > 1) {   // gather the vocab slices of every rank, lay them out as [b, Vfull], arg-max (last index wins ties)
         tp_allgather(lc, c.tp_local.p, c.tp_gather.p, (size_t)b * w.V);
         launch(lc, "tp_logits", 0, tp_logits_kernel, dim3(kNumSMs), dim3(256), 0, (const float*)c.tp_gather.p, w.tp, b, w.V, c.logits.p);
-        launch(lc, "dense_argmax", 0, dense_argmax_kernel, dim3(b), dim3(1024), 0, (const float*)c.logits.p, 1, (long long)0, w.Vfull,
-               c.logits.p, c.next_ids.p);
+        launch_argmax(c, lc, c.logits.p, 1, 0, w.Vfull, b);
     }
     launch(lc, "advance_state", 0, advance_state_kernel, dim3(1), dim3(kMaxBatch), 0, c.state.p, b, t, loop_mode ? 1 : 0, c.ids.p,
            (const uint32_t*)c.next_ids.p, loop_mode ? 1 : 0, loop_mode ? c.trace.p : (uint32_t*)nullptr,
@@ -1461,11 +1468,9 @@ static void enqueue_forward_dense(fl_cache& c, LaunchCtx& lc, int b, int t, bool
                c.tp_local.p);
         tp_allgather(lc, c.tp_local.p, c.tp_gather.p, (size_t)b * w.V);
         launch(lc, "tp_logits", 0, tp_logits_kernel, dim3(kNumSMs), dim3(256), 0, (const float*)c.tp_gather.p, w.tp, b, w.V, c.logits.p);
-        launch(lc, "dense_argmax", 0, dense_argmax_kernel, dim3(b), dim3(1024), 0, (const float*)c.logits.p, 1, (long long)0, w.Vfull, c.logits.p,
-               c.next_ids.p);
+        launch_argmax(c, lc, c.logits.p, 1, 0, w.Vfull, b);
     } else {
-        launch(lc, "dense_argmax", 0, dense_argmax_kernel, dim3(b), dim3(1024), 0, (const float*)d.y.p, ksh, (long long)b * w.V, w.V, c.logits.p,
-               c.next_ids.p);
+        launch_argmax(c, lc, d.y.p, ksh, (long long)b * w.V, w.V, b);
     }
     launch(lc, "advance_state", 0, advance_state_kernel, dim3(1), dim3(kMaxBatch), 0, c.state.p, b, t, loop_mode ? 1 : 0, c.ids.p,
            (const uint32_t*)c.next_ids.p, loop_mode ? 1 : 0, loop_mode ? c.trace.p : (uint32_t*)nullptr,

@@ -147,6 +147,8 @@ struct fl_cache {
     fl::DevBuf<int> trace_pos;
     fl::DevBuf<float> resid, q, attn_out, act, logits, part_acc, part_ml, amax_val;
     fl::DevBuf<int> amax_idx, counters;
+    fl::DevBuf<float> am_val;             // arg-max partials of the dense path [row][kArgmaxParts]
+    fl::DevBuf<int> am_idx;
     fl::PinnedBuf<uint32_t> h_ids;
     fl::PinnedBuf<float> h_logits;
     size_t trace_cap = 0;
