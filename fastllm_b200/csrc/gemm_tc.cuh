@@ -50,8 +50,8 @@ struct GemmArgs {
     // by the gather kernel) is the number of valid rows: a group without rows is skipped entirely (no weight traffic), columns
     // past the count are not stored.
     int grp_m = 0;
-    int grp_cap = 0;
-    const int* grp_cnt = nullptr;
+    union { int grp_cap = 0; int groups; };                              // (the second name: row runs, below)
+    union { const int* grp_cnt = nullptr; const int* tile_off; };
     // BLOCK-DIAGONAL GEMM (GEPI_HL with DUAL_A, GEPI_HL_T with DUAL_B): `blocks` stacked weight matrices, block b multiplies columns
     // [b K, (b + 1) K) of the activations [tokens, blocks K]; the weight rows per block (N with DUAL_A, M with DUAL_B) and K are per
     // block.  Where a block's K ends inside a k-block the weights are zero-filled (their map is K wide), so the neighbour's
@@ -60,21 +60,19 @@ struct GemmArgs {
     int blocks = 0;
     int o_bs = 0;
     const float* gate = nullptr;
-    int ldg = 0;
-    int gate_blk = 0;
+    union { int ldg = 0; float act_limit; };                             // (the second name: gated feed-forward, below)
+    union { int gate_blk = 0; int act; };
     // DUAL_A with plain tiles: the tile walk takes raster_m row tiles against one weight tile before the next weight tile (0: every
     // weight tile of a row tile first).
     int raster_m = 0;
     // Gated feed-forward (GEPI_GLU_HL with DUAL_A): the weight matrix stacks N gate rows and N up rows; a tile's 256 weight rows are 128 of
     // each and the epilogue writes glu(gate, up) [M, N] as bf16 hi (out) and lo (out2).  bias [2 N] or null.
-    int act = 0;
-    float act_limit = 0.f;
+    // act and act_limit: as glu_value takes them.
     // ROW GROUPS (DUAL_A; the experts of a step with many rows): the rows of A come in `groups` runs of whole 128-row tiles, run e in
     // tiles [tile_off[e], tile_off[e + 1]) (device memory, written by the gather kernel); run e multiplies the e-th of the stacked
     // weight matrices of grp_m rows.  M is the row capacity; rows of a run's last tile past its count hold whatever was there, and so
-    // do their results, which nobody reads.
-    int groups = 0;
-    const int* tile_off = nullptr;
+    // do their results, which nobody reads.  (This and the gated form share places with fields that they do not use: the struct is a kernel
+    // parameter, and growing it cost the encoder's q|k|v GEMM 4 %.)
 };
 
 // ---- PTX wrappers ------------------------------------------------------------------------------------------------------
@@ -241,7 +239,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     constexpr int kBNOut = EPI == GEPI_GLU_HL ? BN / 2 : BN;               // output columns of a tile
     static_assert(EPI != GEPI_GLU_HL || (BN == 256 && DUAL == DUAL_A), "the gated epilogue pairs two 128-row weight boxes");
     const int mt_b = (g.M + kGemmBM - 1) / kGemmBM, nt_b = (g.N + kBNOut - 1) / kBNOut;
-    const bool runs = DUAL == DUAL_A && (EPI == GEPI_F32 || EPI == GEPI_GLU_HL) && g.groups > 0;
+    constexpr bool kRuns = DUAL == DUAL_A && (EPI == GEPI_F32 || EPI == GEPI_GLU_HL);
+    const bool runs = kRuns && g.groups > 0;
     int cur_e = 0;                                        // the run a thread's walk has reached (items only grow)
     const int mt = grouped ? (g.M / g.grp_m) * mt_e : (EPI == GEPI_HL_T ? nblk * mt_b : mt_b), nt = grouped ? 1 : (EPI == GEPI_HL ? nblk * nt_b : nt_b);
     const int ksplit = g.ksplit > 1 ? g.ksplit : 1;
@@ -282,7 +281,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
     };
     const int nkps = (nk + ksplit - 1) / ksplit;          // k-blocks per split
-    int ntiles = mt * nt * ksplit;                        // work items: (m tile, n tile, k split), k split fastest
+    const int nitems = mt * nt * ksplit;                  // work items: (m tile, n tile, k split), k split fastest (runs: as tile_off says)
 
     // programmatic dependent launch: the next kernel's prologue may start now; our own prologue (barriers, TMEM, descriptor
     // fetch) overlaps the previous kernel's tail.  Everything that touches dependent memory is ordered behind the producer's
@@ -319,7 +318,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             // requested after the wait.  (The first pass over the ring needs no empty-slot wait: the slots have never been used.)
             uint32_t pre = 0;
             if (DUAL == DUAL_B && g.w_prefetch) {
-                for (int item = blockIdx.x; item < ntiles && pre < (uint32_t)kStages; item += gridDim.x) {
+                for (int item = blockIdx.x; item < nitems && pre < (uint32_t)kStages; item += gridDim.x) {
                     const int tile = item / ksplit, ks = item % ksplit;
                     const int m0 = (tile / nt) * kGemmBM;
                     const int kb1 = min((ks + 1) * nkps, nk);
@@ -331,7 +330,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             pdl_wait();
             asm volatile("fence.proxy.async;" ::: "memory");      // the previous kernel's generic-proxy stores -> TMA reads
-            if (runs) ntiles = g.tile_off[g.groups] * nt;
+            const int ntiles = runs ? g.tile_off[g.groups] * nt : nitems;
             uint32_t c = 0;
             for (int item = blockIdx.x; item < ntiles; item += gridDim.x) {
                 const int tile = item / ksplit, ks = item % ksplit;
@@ -372,7 +371,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             constexpr uint32_t idesc = umma_idesc_bf16(kGemmBM, kMmaN);
             uint32_t c = 0, ti = 0;
             if (grouped || runs) pdl_wait();      // grp_cnt / tile_off is written by a preceding kernel
-            if (runs) ntiles = g.tile_off[g.groups] * nt;
+            const int ntiles = runs ? g.tile_off[g.groups] * nt : nitems;
             for (int item = blockIdx.x; item < ntiles; item += gridDim.x) {
                 if (grouped && g.grp_cnt[(item / ksplit) / mt_e] == 0) continue;
                 const uint32_t ti_now = ti++;
@@ -407,7 +406,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int cslice = (warp - 2) >> 2;
         uint32_t ti = 0;
         if (grouped || runs) pdl_wait();          // grp_cnt / tile_off is written by a preceding kernel
-        if (runs) ntiles = g.tile_off[g.groups] * nt;
+        const int ntiles = runs ? g.tile_off[g.groups] * nt : nitems;
         for (int item = blockIdx.x; item < ntiles; item += gridDim.x) {
             const int tile = item / ksplit, ksi = item % ksplit;
             int m0, n0, grp, mrow0;
@@ -426,7 +425,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             tc_fence_after();
 #pragma unroll 1
             for (int c0 = cslice * 32; c0 < kBNOut; c0 += 128) {  // 32-column chunks dealt round-robin to the 4 warps of a lane quarter
-                if (EPI == GEPI_GLU_HL) {
+                if constexpr (EPI == GEPI_GLU_HL) {
                     // 16 columns at a time: accumulator columns [0, 128) hold gate rows, [128, 256) the up rows of the same outputs
 #pragma unroll 1
                     for (int h = 0; h < 32; h += 16) {
