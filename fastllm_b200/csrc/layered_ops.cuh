@@ -2072,6 +2072,77 @@ static __global__ void ly_delta_prep_kernel(ConvArgs a, int chunk, int off_b, in
     }
 }
 
+// The two preparations above for steps of many rows, convolutions of four taps: a thread takes four neighbouring channels of kConvRows rows
+// in turn with their last three inputs in registers, so an input is read once (16 bytes at a time) instead of once per tap.  A q or k head of
+// 32, 64 or 128 channels lies in 8, 16 or 32 neighbouring lanes, which sum its squares among themselves.
+// delta: channels [0, nq) are q heads, [nq, 2 nq) k heads of D channels (nq = 0: nothing is normed); per row and head, as above,
+// a = exp(-exp(A_log) softplus(proj[off_a + h] + dt_bias)) and b = sigmoid(proj[off_b + h]) or (off_b < 0) the softplus itself.
+// grid (rows / kConvRows, channels / 1024)
+constexpr int kConvRows = 16;
+struct ConvHeads { int nq, D; float qscale; int off_a, off_b; const float *dt_bias, *a_log; int H; float* ab; };
+static __global__ void __launch_bounds__(256) ly_conv4_rows_kernel(ConvArgs a, ConvHeads hd, int T) {
+    pdl_chain();
+    const int r0 = blockIdx.x * kConvRows, r1 = min(T, r0 + kConvRows), c = (blockIdx.y * 256 + threadIdx.x) * 4;
+    if (blockIdx.y == 0) {
+        for (int i = threadIdx.x; i < (r1 - r0) * hd.H; i += 256) {
+            const int row = r0 + i / hd.H, h = i % hd.H;
+            const float* pr = a.proj + (size_t)row * a.ldp;
+            const float dt = softplusf_(pr[hd.off_a + h] + hd.dt_bias[h]);
+            hd.ab[((size_t)row * hd.H + h) * 2] = expf(-expf(hd.a_log[h]) * dt);
+            hd.ab[((size_t)row * hd.H + h) * 2 + 1] = hd.off_b >= 0 ? sigmoidf_(pr[hd.off_b + h]) : dt;
+        }
+    }
+    const bool on = c < a.ch;                   // (lanes past the channels take part in the sums)
+    float w[4][4], b[4] = {}, x[4][4];          // [channel][tap], [tap][channel]
+    if (on) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+            const float4 v = *reinterpret_cast<const float4*>(a.w + (size_t)(c + i) * 4);
+            w[i][0] = v.x; w[i][1] = v.y; w[i][2] = v.z; w[i][3] = v.w;
+            if (a.b) b[i] = a.b[c + i];
+        }
+    }
+    const bool norm = c < 2 * hd.nq;
+    const float scale = c < hd.nq ? hd.qscale : 1.f;
+    int seq = -1;
+    for (int row = r0; row < r1; ++row) {
+        const int s = a.row_seq[row];
+        if (s != seq && on) {                   // a sequence begins (or the block does): its last three inputs
+            seq = s;
+            const int row0 = a.seq_row0[s], pos = a.row_pos[row], pos0 = a.seq_pos0[s], slot = a.seq_slot[s];
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) x[k][i] = conv_input(a, row, row0, pos, pos0, slot, 3 - k, c + i);
+        }
+        float y[4] = {};
+        if (on) {
+            ld_vec<4>(a.proj + (size_t)row * a.ldp + a.off + c, x[3]);
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                float t = b[i];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) t = fmaf(w[i][k], x[k][i], t);
+                y[i] = siluf_(t);
+            }
+#pragma unroll
+            for (int k = 0; k < 3; ++k)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) x[k][i] = x[k + 1][i];
+        }
+        if (hd.nq > 0) {
+            float ss = y[0] * y[0] + y[1] * y[1] + y[2] * y[2] + y[3] * y[3];
+            for (int o = hd.D / 8; o > 0; o >>= 1) ss += __shfl_xor_sync(0xFFFFFFFFu, ss, o);
+            if (norm) {
+                const float r = scale / sqrtf(ss + 1e-6f);
+#pragma unroll
+                for (int i = 0; i < 4; ++i) y[i] *= r;
+            }
+        }
+        if (on) st_vec<4>(a.cv + (size_t)row * a.ch + c, y);
+    }
+}
+
 struct RecArgs {
     const float* cv; int ldc, off_q, off_k, off_v;      // read-out vector q[g], write vector k[g] (D channels each), value v[h] (Dv channels)
     const float* ab;            // [T, H, 2]: decay a, strength b
@@ -2449,35 +2520,47 @@ static __global__ void __launch_bounds__(256) ly_router_groups_kernel(const floa
 }
 
 // Row lists per expert, in ascending (row, pick) order: grp_off[E + 1], pair_row[p] = source row, pair_of[row * top + k] = p.
-// One warp per expert (grid = E blocks of 32 threads): a first sweep counts the picks of lower experts (the list's offset) and
-// its own, a second places its picks by ballot compaction -- stable, so the lists do not depend on timing.
-static __global__ void ly_moe_lists_kernel(const int* __restrict__ sel, int T, int top, int E, int* __restrict__ grp_off, int* __restrict__ pair_row,
-                                           int* __restrict__ pair_of) {
+// One block per expert: a first sweep counts the picks of lower experts (the list's offset) and its own, a second places its picks, 256 at a
+// time, by ballot compaction -- stable, so the lists do not depend on timing.
+static __global__ void __launch_bounds__(256) ly_moe_lists_kernel(const int* __restrict__ sel, int T, int top, int E, int* __restrict__ grp_off, int* __restrict__ pair_row,
+                                                                  int* __restrict__ pair_of) {
     pdl_chain();
-    const int e = blockIdx.x, lane = threadIdx.x, n = T * top;
+    __shared__ int cnt[2][8];
+    const int e = blockIdx.x, tid = threadIdx.x, lane = tid & 31, w = tid >> 5, n = T * top;
     int less = 0, mine = 0;
-    for (int i = lane; i < n; i += 32) {
+    for (int i = tid; i < n; i += 256) {
         const int s = sel[i];
         less += s < e;
         mine += s == e;
     }
+    less = __reduce_add_sync(0xFFFFFFFFu, less);
+    mine = __reduce_add_sync(0xFFFFFFFFu, mine);
+    if (lane == 0) { cnt[0][w] = less; cnt[1][w] = mine; }
+    __syncthreads();
+    less = mine = 0;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) { less += __shfl_xor_sync(0xFFFFFFFFu, less, o); mine += __shfl_xor_sync(0xFFFFFFFFu, mine, o); }
-    if (lane == 0) {
+    for (int k = 0; k < 8; ++k) { less += cnt[0][k]; mine += cnt[1][k]; }
+    if (tid == 0) {
         grp_off[e] = less;
         if (e == E - 1) grp_off[E] = less + mine;
     }
     int p = less;
-    for (int i0 = 0; i0 < n; i0 += 32) {
-        const int i = i0 + lane;
+    for (int i0 = 0; i0 < n; i0 += 256) {
+        const int i = i0 + tid;
         const bool hit = i < n && sel[i] == e;
         const unsigned m = __ballot_sync(0xFFFFFFFFu, hit);
+        __syncthreads();                        // everybody has read the counts of the round before
+        if (lane == 0) cnt[0][w] = __popc(m);
+        __syncthreads();
+        int before = 0, all = 0;
+#pragma unroll
+        for (int k = 0; k < 8; ++k) { before += k < w ? cnt[0][k] : 0; all += cnt[0][k]; }
         if (hit) {
-            const int q = p + __popc(m & ((1u << lane) - 1u));
+            const int q = p + before + __popc(m & ((1u << lane) - 1u));
             pair_row[q] = i / top;
             pair_of[i] = q;
         }
-        p += __popc(m);
+        p += all;
     }
 }
 
@@ -2581,17 +2664,28 @@ static __global__ void __launch_bounds__(256) ly_relu2_runs_kernel(const float* 
             split_store(ahi, alo, (size_t)r * F + c, glu_value(x[(size_t)r * F + c], 0.f, 2, 0.f));
 }
 
-// y[row, c] = sum_k wt[row, k] * eo[pair_of[row, k], c]  (pick order)  + sgate[row] * sh[row, c]
-static __global__ void ly_moe_combine_kernel(const float* __restrict__ eo, const int* __restrict__ pair_of, const float* __restrict__ wt, int top,
-                                             const float* __restrict__ sh, const float* __restrict__ sgate, int W, float* __restrict__ y) {
+// y[row, c] = sum_k wt[row, k] * eo[pair_of[row, k], c]  (pick order)  + sgate[row] * sh[row, c];  V channels per thread (V = 4: W a multiple
+// of 4).  grid (channel blocks of 256 V, rows)
+template <int V>
+static __global__ void __launch_bounds__(256) ly_moe_combine_kernel(const float* __restrict__ eo, const int* __restrict__ pair_of, const float* __restrict__ wt, int top,
+                                                                    const float* __restrict__ sh, const float* __restrict__ sgate, int W, float* __restrict__ y) {
     pdl_chain();
-    const int row = blockIdx.y;
-    for (int c = blockIdx.x * blockDim.x + threadIdx.x; c < W; c += gridDim.x * blockDim.x) {
-        float t = 0.f;
-        for (int k = 0; k < top; ++k) t = fmaf(wt[row * top + k], eo[(size_t)pair_of[row * top + k] * W + c], t);
-        if (sh != nullptr) t = fmaf(sgate ? sgate[row] : 1.f, sh[(size_t)row * W + c], t);
-        y[(size_t)row * W + c] = t;
+    const int row = blockIdx.y, c = (blockIdx.x * 256 + threadIdx.x) * V;
+    if (c >= W) return;
+    float t[V] = {}, v[V];
+    for (int k = 0; k < top; ++k) {
+        const float wk = wt[row * top + k];
+        ld_vec<V>(eo + (size_t)pair_of[row * top + k] * W + c, v);
+#pragma unroll
+        for (int i = 0; i < V; ++i) t[i] = fmaf(wk, v[i], t[i]);
     }
+    if (sh != nullptr) {
+        const float g = sgate ? sgate[row] : 1.f;
+        ld_vec<V>(sh + (size_t)row * W + c, v);
+#pragma unroll
+        for (int i = 0; i < V; ++i) t[i] = fmaf(g, v[i], t[i]);
+    }
+    st_vec<V>(y + (size_t)row * W + c, t);
 }
 
 }  // namespace fl
