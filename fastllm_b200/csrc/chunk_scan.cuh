@@ -14,7 +14,7 @@
 //   3. ly_chunk_out_kernel                                                 one block per (chunk, head): what the starting state adds
 // Bound: f32 FMA issue in 1 and 3 (operands in shared memory, 4 x 4 results per thread: 64 FMA per 8 16-byte loads), HBM in 2.
 // Measured per layer, token by token -> chunks: gated linear attention, 1531 tokens, 16 heads of 128 x 128: 1160 -> 260 us; Mamba-2, 2048
-// tokens, 128 heads of 128 x 64: 1186 -> 726 us; delta rule, 2048 tokens, 32 heads of 128 x 128: 1022 -> 617 us; lightning attention, 333
+// tokens, 128 heads of 128 x 64: 1186 -> 668 us (four heads per block: their scores are multiplied once); delta rule, 2048 tokens, 32 heads of 128 x 128: 1022 -> 626 us; lightning attention, 333
 // tokens, 16 heads: 246 -> 65 us.  Same model, same tokens: the logits agree to 1e-5 .. 4e-5, their error against 64 bits is unchanged.
 #pragma once
 #include "layered_ops.cuh"
@@ -139,10 +139,10 @@ __device__ __forceinline__ void cs_load_slab(float* dst, const float* src, int l
         *reinterpret_cast<float4*>(dst + r * kCsLdA + c) = v;
     }
 }
-// o (rows [0, len) of the head, columns [v0, v0 + 64)) = A V (+ dskip v);  us [D][Dv] = K^T V
+// o (rows [0, len) of the head, columns [v0, v0 + 64)) = A V (+ dskip v);  us [D][Dv] = K^T V, V's rows times `rows` first (nullptr: as they are)
 template <int DP>
-__device__ __forceinline__ void cs_slab_products(const ChunkArgs& a, const float* sA, const float* sK, int ldk, const float* sV, int row, int len, int hd, int v0, float dsk,
-                                                 float* us, int ty, int tx) {
+__device__ __forceinline__ void cs_slab_products(const ChunkArgs& a, const float* sA, const float* sK, int ldk, float* sV, int row, int len, int hd, int v0, float dsk,
+                                                 float* us, int ty, int tx, const float* rows) {
     float acc[4][4];
     cs_zero(acc);
     cs_mm_nn<kCsC>(acc, sA, kCsLdA, sV, kCsLdA, ty, tx);
@@ -160,6 +160,11 @@ __device__ __forceinline__ void cs_slab_products(const ChunkArgs& a, const float
             *reinterpret_cast<float4*>(a.o + (size_t)(row + i) * a.H * a.Dv + hd * a.Dv + col) = v;
         }
     }
+    if (rows != nullptr) {
+        __syncthreads();
+        for (int i = threadIdx.x; i < kCsC * kCsSlab; i += 256) sV[i / kCsSlab * kCsLdA + i % kCsSlab] *= rows[i / kCsSlab];
+        __syncthreads();
+    }
 #pragma unroll 1
     for (int m0 = 0; m0 < DP; m0 += 64) {
         cs_zero(acc);
@@ -171,57 +176,100 @@ __device__ __forceinline__ void cs_slab_products(const ChunkArgs& a, const float
         }
     }
 }
-// One decay per head and token: sa[t] = decay of token t (1 behind the portion).  sA <- sA * (decay from j to i), zero above the
-// diagonal; to_end[j] = decay from j to the chunk's end.  Threads 0..63, one column each.
-__device__ __forceinline__ void cs_decay_columns(float* sA, const float* sa, float* to_end, bool keep_diagonal) {
-    const int j = threadIdx.x;
-    if (j >= kCsC) return;
-    for (int i = 0; i < j; ++i) sA[i * kCsLdA + j] = 0.f;
-    if (!keep_diagonal) sA[j * kCsLdA + j] = 0.f;
-    float p = 1.f;
-    for (int i = j + 1; i < kCsC; ++i) { p *= sa[i]; sA[i * kCsLdA + j] *= p; }
-    to_end[j] = p;
+// One decay per head and token: sa[t] = decay of token t (1 behind the portion).  The decay from token j to token i of a thread's results
+// (i = ty + 16 r, j = tx + 16 c: block row r, block column c) is (start of i's 16-token block to i) x (the blocks between) x (j to its block's
+// end), inside a block the product itself: every factor is <= 1, and no thread multiplies more than 15 of them one after the other.
+struct CsDecay {
+    float sa[kCsC], pre[kCsC], suf[kCsC], end[kCsC];    // end: j to the chunk's end
+    float whole;
+};
+// between two barriers of the caller: sa is there before, the tables are there behind the next one
+__device__ __forceinline__ void cs_decay_tables(CsDecay& d) {
+    const int t = threadIdx.x;
+    if (t >= kCsC) return;
+    const int b0 = t & ~15;
+    float p = 1.f, q = 1.f, e = 1.f;
+    for (int i = b0; i <= t; ++i) p *= d.sa[i];
+    for (int i = t + 1; i < b0 + 16; ++i) q *= d.sa[i];
+    for (int i = b0 + 16; i < kCsC; ++i) e *= d.sa[i];
+    d.pre[t] = p;
+    d.suf[t] = q;
+    d.end[t] = q * e;
+    if (t == 0) d.whole = p * q * e;
+}
+// factors of the thread's results: zero above the diagonal (and on it unless `diagonal`)
+__device__ __forceinline__ void cs_decay_factors(float (&f)[4][4], const CsDecay& d, int ty, int tx, bool diagonal) {
+    float in = 1.f, blk[4];
+#pragma unroll
+    for (int b = 0; b < 4; ++b) blk[b] = d.pre[16 * b + 15];
+#pragma unroll
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+            if (c > r) { f[r][c] = 0.f; continue; }
+            if (c == r) {
+                in = 1.f;
+                for (int i = tx + 1; i <= ty; ++i) in *= d.sa[16 * r + i];
+                f[r][c] = tx < ty || (diagonal && tx == ty) ? in : 0.f;
+                continue;
+            }
+            float x = d.pre[16 * r + ty] * d.suf[16 * c + tx];
+#pragma unroll
+            for (int b = 1; b < 3; ++b)
+                if (b > c && b < r) x *= blk[b];
+            f[r][c] = x;
+        }
 }
 
 // ---- lightning attention, Mamba-2: one decay per head and token ---------------------------------------------------------------------
-template <int DP>
+// HB neighbouring heads that read the same q and k (Mamba-2's groups) share a block: their scores differ by the decays alone.
+template <int DP, int HB>
 static __global__ void __launch_bounds__(256, 2) ly_chunk_in_kernel(ChunkArgs a) {
     pdl_chain();
     extern __shared__ __align__(16) float sm[];
     constexpr int LD = DP + kCsPad;
     float *sQ = sm, *sK = sQ + kCsC * LD, *sA = sK + kCsC * LD;        // the value slab takes the queries' place once they are used
-    __shared__ float sa[kCsC], sb[kCsC], se[kCsC];
-    const int hd = blockIdx.y, g = hd / (a.H / a.G), tid = threadIdx.x;
+    __shared__ CsDecay dec;
+    __shared__ float sb[kCsC];
+    const int h0 = blockIdx.y * HB, g = h0 / (a.H / a.G), tid = threadIdx.x;
     int row, len, ty, tx;
     if (!cs_find(a, blockIdx.x, row, len)) return;
     cs_thread(ty, tx);
     const float* src = a.src + (size_t)row * a.ld;
     cs_load<DP>(sQ, LD, src + a.off_q + g * a.D, a.ld, len, a.D, 1.f);
     cs_load<DP>(sK, LD, src + a.off_k + g * a.D, a.ld, len, a.D, 1.f);
-    if (tid < kCsC) {
-        sa[tid] = tid < len ? a.ab[((size_t)(row + tid) * a.H + hd) * 2] : 1.f;
-        sb[tid] = tid < len ? a.ab[((size_t)(row + tid) * a.H + hd) * 2 + 1] : 0.f;
-    }
     __syncthreads();
-    float acc[4][4];
-    cs_zero(acc);
-    cs_mm_nt<DP>(acc, sQ, LD, sK, LD, ty, tx);
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) sA[(ty + 16 * r) * kCsLdA + tx + 16 * c] = acc[r][c];
-    __syncthreads();
-    cs_decay_columns(sA, sa, se, true);
-    __syncthreads();
-    for (int i = tid; i < kCsC * DP; i += 256) sK[i / DP * LD + i % DP] *= se[i / DP];
-    if (tid == 0) a.dec[(size_t)blockIdx.x * a.H + hd] = se[0] * sa[0];
-    const float dsk = a.dskip ? a.dskip[hd] : 0.f;
-    float* us = a.us + ((size_t)blockIdx.x * a.H + hd) * a.D * a.Dv;
-    for (int v0 = 0; v0 < a.Dv; v0 += kCsSlab) {
-        cs_load_slab(sQ, src + a.off_v + hd * a.Dv, a.ld, len, v0, a.Dv, sb);
+    float qk[4][4];
+    cs_zero(qk);
+    cs_mm_nt<DP>(qk, sQ, LD, sK, LD, ty, tx);
+#pragma unroll 1
+    for (int hd = h0; hd < h0 + HB; ++hd) {
+        __syncthreads();                // everybody is done with the head before
+        if (tid < kCsC) {
+            const float2 v = tid < len ? *reinterpret_cast<const float2*>(a.ab + ((size_t)(row + tid) * a.H + hd) * 2) : make_float2(1.f, 0.f);
+            dec.sa[tid] = v.x;
+            sb[tid] = v.y;
+        }
         __syncthreads();
-        cs_slab_products<DP>(a, sA, sK, LD, sQ, row, len, hd, v0, dsk, us, ty, tx);
+        cs_decay_tables(dec);
         __syncthreads();
+        {
+            float f[4][4];
+            cs_decay_factors(f, dec, ty, tx, true);
+#pragma unroll
+            for (int r = 0; r < 4; ++r)
+#pragma unroll
+                for (int c = 0; c < 4; ++c) sA[(ty + 16 * r) * kCsLdA + tx + 16 * c] = qk[r][c] * f[r][c];
+        }
+        if (tid == 0) a.dec[(size_t)blockIdx.x * a.H + hd] = dec.whole;
+        const float dsk = a.dskip ? a.dskip[hd] : 0.f;
+        float* us = a.us + ((size_t)blockIdx.x * a.H + hd) * a.D * a.Dv;
+        for (int v0 = 0; v0 < a.Dv; v0 += kCsSlab) {
+            if (v0 > 0) __syncthreads();
+            cs_load_slab(sQ, src + a.off_v + hd * a.Dv, a.ld, len, v0, a.Dv, sb);
+            __syncthreads();
+            cs_slab_products<DP>(a, sA, sK, LD, sQ, row, len, hd, v0, dsk, us, ty, tx, dec.end);
+        }
     }
 }
 
@@ -323,7 +371,7 @@ static __global__ void __launch_bounds__(256) ly_chunk_gla_kernel(ChunkArgs a) {
     for (int v0 = 0; v0 < a.Dv; v0 += kCsSlab) {
         cs_load_slab(sF, src + a.off_v + hd * a.Dv, a.ld, len, v0, a.Dv, nullptr);
         __syncthreads();
-        cs_slab_products<DP>(a, sA, sK, LD, sF, row, len, hd, v0, 0.f, us, ty, tx);
+        cs_slab_products<DP>(a, sA, sK, LD, sF, row, len, hd, v0, 0.f, us, ty, tx, nullptr);
         __syncthreads();
     }
 }
@@ -442,7 +490,8 @@ static __global__ void __launch_bounds__(256) ly_chunk_delta_kernel(ChunkArgs a)
     extern __shared__ __align__(16) float sm[];
     constexpr int LD = DP + kCsPad, B = 16, NB = kCsC / B;
     float *sQ = sm, *sK = sQ + kCsC * LD, *sM = sK + kCsC * LD, *sT = sM + kCsC * kCsLdA;       // the value slab takes the queries' place
-    __shared__ float sa[kCsC], sb[kCsC], se[kCsC], sp[kCsC];
+    __shared__ CsDecay dec;
+    __shared__ float sb[kCsC], sp[kCsC];
     const int hd = blockIdx.y, g = hd / (a.H / a.G), tid = threadIdx.x;
     int row, len, ty, tx;
     if (!cs_find(a, blockIdx.x, row, len)) return;
@@ -451,41 +500,33 @@ static __global__ void __launch_bounds__(256) ly_chunk_delta_kernel(ChunkArgs a)
     cs_load<DP>(sQ, LD, src + a.off_q + g * a.D, a.ld, len, a.D, 1.f);
     cs_load<DP>(sK, LD, src + a.off_k + g * a.D, a.ld, len, a.D, 1.f);
     if (tid < kCsC) {
-        sa[tid] = tid < len ? a.ab[((size_t)(row + tid) * a.H + hd) * 2] : 1.f;
+        dec.sa[tid] = tid < len ? a.ab[((size_t)(row + tid) * a.H + hd) * 2] : 1.f;
         sb[tid] = tid < len ? a.ab[((size_t)(row + tid) * a.H + hd) * 2 + 1] : 0.f;
     }
     __syncthreads();
-    float acc[4][4];
-    auto store = [&](float* s) {
-#pragma unroll
-        for (int r = 0; r < 4; ++r)
-#pragma unroll
-            for (int c = 0; c < 4; ++c) s[(ty + 16 * r) * kCsLdA + tx + 16 * c] = acc[r][c];
-    };
+    cs_decay_tables(dec);
+    for (int i = tid; i < kCsC * kCsLdA; i += 256) sT[i] = 0.f;
+    float acc[4][4], kk[4][4], f[4][4];
     cs_zero(acc);
     cs_mm_nt<DP>(acc, sQ, LD, sK, LD, ty, tx);
-    store(sM);
-    if (tid < kCsC) {
-        float p = 1.f;
-        for (int i = 0; i <= tid; ++i) p *= sa[i];
+    cs_zero(kk);
+    cs_mm_nt<DP>(kk, sK, LD, sK, LD, ty, tx);
+    __syncthreads();
+    if (tid < kCsC) {                   // decay from the chunk's start
+        float p = dec.pre[tid];
+        for (int b = 0; b < tid / 16; ++b) p *= dec.pre[16 * b + 15];
         sp[tid] = p;
     }
-    __syncthreads();
-    cs_decay_columns(sM, sa, se, true);
-    __syncthreads();
+    cs_decay_factors(f, dec, ty, tx, true);
     float* aq = a.aq + ((size_t)blockIdx.x * a.H + hd) * kCsC * kCsC;
-    for (int i = tid; i < kCsC * kCsC; i += 256) aq[i] = sM[i / kCsC * kCsLdA + i % kCsC];
-    __syncthreads();
-    cs_zero(acc);
-    cs_mm_nt<DP>(acc, sK, LD, sK, LD, ty, tx);
 #pragma unroll
     for (int r = 0; r < 4; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] *= sb[ty + 16 * r];
-    store(sM);
-    for (int i = tid; i < kCsC * kCsLdA; i += 256) sT[i] = 0.f;
-    __syncthreads();
-    cs_decay_columns(sM, sa, se, false);
+        for (int c = 0; c < 4; ++c) {
+            const int i = ty + 16 * r, j = tx + 16 * c;
+            aq[i * kCsC + j] = acc[r][c] * f[r][c];
+            sM[i * kCsLdA + j] = i > j ? kk[r][c] * sb[i] * f[r][c] : 0.f;
+        }
     __syncthreads();
     // diagonal blocks of T: one thread per column, x_i = [i == c] - sum_{j < i} M_ij x_j
     if (tid < kCsC) {

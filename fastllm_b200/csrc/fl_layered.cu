@@ -1107,7 +1107,7 @@ static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurr
     static bool attr_set = false;
     if (!attr_set) {
         auto room = [](auto kern, size_t smem) { FL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); };
-        room(ly_chunk_in_kernel<DP>, sm_in); room(ly_chunk_gla_kernel<DP>, sm_gla); room(ly_chunk_delta_kernel<DP>, sm_delta);
+        room(ly_chunk_in_kernel<DP, 1>, sm_in); room(ly_chunk_in_kernel<DP, 4>, sm_in); room(ly_chunk_gla_kernel<DP>, sm_gla); room(ly_chunk_delta_kernel<DP>, sm_delta);
         room(ly_chunk_delta_state_kernel<DP>, sm_dstate);
         room(ly_chunk_out_kernel<DP, 0>, sm_out); room(ly_chunk_out_kernel<DP, 1>, sm_out); room(ly_chunk_out_kernel<DP, 2>, sm_out2);
         attr_set = true;
@@ -1135,7 +1135,8 @@ static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurr
         }
         const bool gla = kind == Recurrence::gla;
         if (gla) launch(lc, "gla_chunks", 0, ly_chunk_gla_kernel<DP>, grid, b, sm_gla, a);
-        else launch(lc, "ssm_chunks", 0, ly_chunk_in_kernel<DP>, grid, b, sm_in, a);
+        else if (a.H / a.G % 4 == 0) launch(lc, "ssm_chunks", 0, ly_chunk_in_kernel<DP, 4>, dim3(chunks, a.H / 4), b, sm_in, a);
+        else launch(lc, "ssm_chunks", 0, ly_chunk_in_kernel<DP, 1>, grid, b, sm_in, a);
         launch(lc, gla ? "gla_states" : "ssm_states", 0, ly_chunk_state_kernel, dim3((unsigned)((per / 4 + 255) / 256), n), b, 0, a, gla ? 1 : 0);
         if (gla) launch(lc, "gla_chunks_out", 0, ly_chunk_out_kernel<DP, 1>, grid, b, sm_out, a);
         else launch(lc, "ssm_chunks_out", 0, ly_chunk_out_kernel<DP, 0>, grid, b, sm_out, a);
