@@ -696,10 +696,6 @@ void layered_finalize(LayeredModel& m) {
                 lw.tc_moe = true;
                 lw.tm_gu = make_tmap_bf16(lw.w_gu, (uint64_t)d.experts * GF, (uint64_t)m.W, (uint64_t)m.W, 128);
                 lw.tm_down = make_tmap_bf16(lw.w_down, (uint64_t)d.experts * m.W, (uint64_t)d.ff, (uint64_t)d.ff, 128);
-                for (int e = 0; e < d.experts; ++e) {
-                    lw.tm_egu.push_back(make_tmap_bf16(lw.w_gu + (size_t)e * GF * m.W, (uint64_t)GF, (uint64_t)m.W, (uint64_t)m.W, 128));
-                    lw.tm_edown.push_back(make_tmap_bf16(lw.w_down + (size_t)e * m.W * d.ff, (uint64_t)m.W, (uint64_t)d.ff, (uint64_t)d.ff, 128));
-                }
             }
         }
         map(m.head, m.V, m.W, m.tm_head, m.tc_head);
@@ -861,7 +857,8 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
             y.qp_hi.alloc(R * m.max_hp); y.qp_lo.alloc(R * m.max_hp); y.qo_hi.alloc(R * m.max_hq); y.qo_lo.alloc(R * m.max_hq);
             y.ol_hi.alloc(R * m.max_hc); y.ol_lo.alloc(R * m.max_hc);
         }
-        y.gu.alloc(P * 2 * std::max(m.max_ff, 1)); y.act.alloc(P * std::max(m.max_ff, 1)); y.eo.alloc(std::max(P, run_rows) * W);
+        y.gu.alloc(std::max(P * 2, run_rows) * std::max(m.max_ff, 1));     // (run_rows: experts without a gate)
+        y.act.alloc(P * std::max(m.max_ff, 1)); y.eo.alloc(std::max(P, run_rows) * W);
         y.sh_gu.alloc(R * 2 * std::max(m.max_ff, 1)); y.sh_act.alloc(R * std::max(m.max_ff, 1)); y.sh_o.alloc(R * W);
         y.route_w.alloc(P); y.route_sel.alloc(P); y.sgate.alloc(R);
         y.pair_row.alloc(P); y.pair_of.alloc(P); y.grp_off.alloc((size_t)m.max_experts + 2); y.tile_off.alloc((size_t)m.max_experts + 2);

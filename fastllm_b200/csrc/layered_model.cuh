@@ -70,8 +70,7 @@ struct LayeredLayerW {
     // serving precision: TMA descriptors of the matrices whose shapes admit the tensor-core GEMM (tc_* says which)
     CUtensorMap tm_in{}, tm_o{}, tm_gu{}, tm_down{}, tm_sgu{}, tm_sdown{};
     bool tc_in = false, tc_o = false, tc_gu = false, tc_down = false, tc_sgu = false, tc_sdown = false;
-    bool tc_moe = false;                               // experts: tm_gu / tm_down cover the stacked matrices (grouped GEMM, few rows),
-    std::vector<CUtensorMap> tm_egu, tm_edown;         //   these one expert each (every expert over all rows, many rows)
+    bool tc_moe = false;                               // experts: tm_gu / tm_down cover the stacked matrices (grouped GEMMs)
     float* route_corr = nullptr;        // sigmoid router: [experts] added to the scores for the choice only
     // a second mixer beside this one: its rows follow this mixer's inside w_in (its offsets are absolute), it has its own w_o,
     // cache / state indices and side tables; nothing but the mixer fields of it is used
