@@ -37,8 +37,7 @@ struct BertModel {
     DevBuf<uint32_t> ids, mask;
     PinnedBuf<uint32_t> h_ids;
     PinnedBuf<float> h_out;
-    DevBuf<uint8_t> small_layers;           // the layers' pointers for the one-launch kernel (empty: other sizes than it is built for)
-    int small_clusters = -1;                // clusters of it that are resident at a time (-1: not asked yet)
+    void* small_layers = nullptr;           // in the slab: the layers' pointers for the one-launch kernel (null: other sizes than it is built for)
     ~BertModel();
 };
 

@@ -136,8 +136,11 @@ void bert_build(BertModel& m) {
         l.bqkv = take(3 * H * 4); l.bo = take(H * 4); l.bi = take(I * 4); l.bo2 = take(H * 4);
         l.l1w = take(H * 4); l.l1b = take(H * 4); l.l2w = take(H * 4); l.l2b = take(H * 4);
     }
+    const bool small = m.H == kBsH && m.I == kBsI && m.nh == kBsHeads;
+    const size_t o_small = small ? take(m.L * sizeof(BertSmallLayer)) : 0;
     m.slab.alloc(off, true);
     uint8_t* b = m.slab.p;
+    if (small) m.small_layers = b + o_small;
     m.wemb = (uint16_t*)(b + o_w); m.pemb = (uint16_t*)(b + o_p); m.lnw = (float*)(b + o_lw); m.lnb = (float*)(b + o_lb);
     m.layers.resize(m.L);
     for (int i = 0; i < m.L; ++i) {
@@ -265,11 +268,10 @@ void bert_finalize(BertModel& m) {
         w.tm_wi = make_tmap_bf16(w.wi, m.I, m.H, m.H, kBertBN);
         w.tm_wo2 = make_tmap_bf16(w.wo2, m.H, m.I, m.I, kBertBN);
     }
-    if (m.H == kBsH && m.I == kBsI && m.nh == kBsHeads) {
+    if (m.small_layers != nullptr) {
         std::vector<BertSmallLayer> tab;
         for (const BertLayerW& w : m.layers) tab.push_back({w.wqkv, w.wo, w.wi, w.wo2, w.bqkv, w.bo, w.bi, w.bo2, w.ln1w, w.ln1b, w.ln2w, w.ln2b});
-        m.small_layers.alloc(tab.size() * sizeof(BertSmallLayer));
-        FL_CUDA(cudaMemcpy(m.small_layers.p, tab.data(), tab.size() * sizeof(BertSmallLayer), cudaMemcpyHostToDevice));
+        FL_CUDA(cudaMemcpy(m.small_layers, tab.data(), tab.size() * sizeof(BertSmallLayer), cudaMemcpyHostToDevice));
     }
     m.finalized = true;
 }
@@ -291,7 +293,7 @@ static void bert_reserve(BertModel& m, int b, int t) {
 // the chain does (0.26 ms, whatever it has below some hundred tokens).
 constexpr int kBsCluster = 16;
 template <int MT>
-static bool bert_small_launch(BertModel& m, const BertSmallArgs& a, int clusters, bool ask) {
+static int bert_small_launch(BertModel& m, const BertSmallArgs& a, int clusters, bool ask) {      // ask: -> clusters that are resident at a time
     auto kern = bert_small_kernel<MT, kBsCluster>;
     static bool attr_set = false;
     if (!attr_set) {
@@ -313,28 +315,28 @@ static bool bert_small_launch(BertModel& m, const BertSmallArgs& a, int clusters
     if (ask) {
         int n = 0;
         if (cudaOccupancyMaxActiveClusters(&n, kern, &cfg) != cudaSuccess) { cudaGetLastError(); n = 0; }
-        m.small_clusters = n;
-        return true;
+        return n;
     }
     FL_CUDA(cudaLaunchKernelEx(&cfg, kern, a));
     g_launches.fetch_add(1, std::memory_order_relaxed);
-    return true;
+    return clusters;
 }
 static bool bert_enqueue_small(BertModel& m, int b, int t, bool has_mask) {
-    if (m.small_layers.n == 0 || t > kBsTokens) return false;
-    if (m.small_clusters < 0) bert_small_launch<kBsTokens / 16>(m, BertSmallArgs{}, 1, true);
-    if (m.small_clusters < 1) return false;
+    if (m.small_layers == nullptr || t > kBsTokens) return false;
+    static const int resident = bert_small_launch<kBsTokens / 16>(m, BertSmallArgs{}, 1, true);       // a property of the device
+    if (resident < 1) return false;
     // as many clusters as fit at a time, each with as few sentences as that leaves: up to 64 tokens per cluster
-    const int spc = (b + m.small_clusters - 1) / m.small_clusters, clusters = (b + spc - 1) / spc, rows = spc * t;
+    const int spc = (b + resident - 1) / resident, clusters = (b + spc - 1) / spc, rows = spc * t;
     if (rows > kBsTokens) return false;
-    const BertSmallArgs a{reinterpret_cast<const BertSmallLayer*>(m.small_layers.p), m.wemb, m.pemb, m.lnw, m.lnb, m.ids.p, has_mask ? m.mask.p : nullptr,
+    const BertSmallArgs a{static_cast<const BertSmallLayer*>(m.small_layers), m.wemb, m.pemb, m.lnw, m.lnb, m.ids.p, has_mask ? m.mask.p : nullptr,
                           m.L, b, t, m.V, m.maxpos, spc, m.cfg.norm_eps, (float)(1.0 / std::sqrt((double)m.d)), m.qkv.p, m.ctx.p, m.hbuf.p, m.pre.p, m.out.p};
     switch ((rows + 15) / 16) {
-        case 1: return bert_small_launch<1>(m, a, clusters, false);
-        case 2: return bert_small_launch<2>(m, a, clusters, false);
-        case 3: return bert_small_launch<3>(m, a, clusters, false);
-        default: return bert_small_launch<4>(m, a, clusters, false);
+        case 1: bert_small_launch<1>(m, a, clusters, false); break;
+        case 2: bert_small_launch<2>(m, a, clusters, false); break;
+        case 3: bert_small_launch<3>(m, a, clusters, false); break;
+        default: bert_small_launch<4>(m, a, clusters, false);
     }
+    return true;
 }
 
 // Enqueue the encoder on m.stream: B1 -> 6 x (B2..B7) -> B8
