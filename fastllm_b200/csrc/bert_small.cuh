@@ -227,7 +227,8 @@ static __global__ void __launch_bounds__(kBsThreads, 1) bert_small_kernel(const 
         wo.load(w.wo, rank, warp, lane);
         bs_wait();
         {   // attention: the cluster's warps share the (sentence, head) pairs, several warps of a pair its query rows
-            const int pairs = ns * kBsHeads, warps = CL * (kBsThreads / 32), split = max(1, min(a.t, warps / pairs)), per = (a.t + split - 1) / split;
+            // (whole stretches of `per` rows only: the first row of every item is one of the sentence)
+            const int pairs = ns * kBsHeads, warps = CL * (kBsThreads / 32), most = max(1, min(a.t, warps / pairs)), per = (a.t + most - 1) / most, split = (a.t + per - 1) / per;
             for (int it = warp * CL + rank; it < pairs * split; it += warps) {
                 const int pr = it % pairs, sent = pr / kBsHeads, head = pr % kBsHeads, first = it / pairs * per, last = min(a.t, first + per);
                 const uint16_t* base = qkv + (size_t)sent * a.t * 3 * kBsH + head * kBertD;
