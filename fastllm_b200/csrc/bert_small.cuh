@@ -3,14 +3,15 @@
 // A query of a dozen tokens through the launch chain is 44 kernels, each of them a few microseconds of latency around almost no work (the
 // 24 GEMMs fill 2 to 8 of 148 SMs and walk K one 64-column block after the other).  Here the blocks of a cluster split every projection's
 // output columns; phases are separated by the cluster's hardware barrier instead of a kernel boundary, and the weights of a phase -- which
-// depend on nothing -- travel into registers while the cluster waits for the phase before.
-//   per layer: x -> q|k|v | attention, one warp per (sentence, head, rows) | x + W_o ctx | LayerNorm (every block for itself) -> gelu(W_i x1) |
-//   x1 + W_o2 h | LayerNorm
-// A warp multiplies a quarter of K (mma.sync m16n8k16, f32 accumulation) for half of the block's columns; the four quarters meet in shared
-// memory in a fixed order.  Roundings are the chain's: q|k|v, ctx, x, h in bf16, sums, residuals and LayerNorm in f32 (and the
-// probabilities, which the chain rounds).
-// Bound: latency -- 5 phases x 6 layers of about 4 us (cluster barrier, L2 round trips of activations and weights, a few MMAs).
-// One sentence of 19 tokens, whole call: 257 -> 161 us.
+// depend on nothing -- travel into shared memory while the cluster waits for the phase before.
+//   per layer: x -> q|k|v | attention, one warp per (sentence, head, 16 query rows) | x + W_o ctx | LayerNorm (every block for itself) ->
+//   gelu(W_i x1) | x1 + W_o2 h | LayerNorm
+// The results are the chain's, bit for bit: an output's products go into its f32 accumulator 16 columns of K at a time in ascending order, as
+// tcgen05.mma takes them (mma.sync m16n8k16 sums the same 16 products to the same bits, in whatever order they stand inside the 16), so K is
+// not split over warps; attention, roundings and the order of every other sum are those of bert.cuh.
+// Bound: latency -- 5 phases x 6 layers of about 6 us (cluster barrier, L2 round trips of activations and weights, a chain of 24 to 96 MMAs).
+// One sentence of 19 tokens, whole call: 262 us as 44 launches, 180 us here.  (Four warps to a quarter of K each took 162, but their sums are
+// not the chain's, and 16-bit activations carry that to 3e-3 in the embedding.)
 #pragma once
 #include "bert.cuh"
 #include "gemm_tc.cuh"
@@ -18,7 +19,10 @@
 namespace fl {
 
 constexpr int kBsTokens = 64, kBsThreads = 256, kBsH = 384, kBsI = 1536, kBsHeads = 12;     // all-MiniLM-L6-v2's sizes
-constexpr int kBsLdX = kBsH + 8;            // bf16 row of the x tile: neighbouring rows start four banks apart
+// Operand rows in shared memory: bf16, 32 columns as four 16-byte pieces, piece q = columns 4 q .. 4 q + 3 of the first 16 and of the second 16.
+// One 16-byte load is then a lane's share of two MMAs, both inside their own 16 columns of K.  h and ctx lie in global memory the same way.
+__host__ __device__ constexpr int bs_at(int c) { return (c & ~31) | ((c >> 2 & 3) << 3) | ((c >> 4 & 1) << 2) | (c & 3); }
+__host__ __device__ constexpr int bs_ld(int k) { return k + 32; }       // the eight lanes of a quarter-warp's 16-byte load on different banks
 
 struct BertSmallLayer {
     const uint16_t *wqkv, *wo, *wi, *wo2;
@@ -33,85 +37,81 @@ struct BertSmallArgs {
     uint16_t *qkv, *ctx, *h; float* pre;    // workspace rows as the launch chain has them
     float* out;
 };
+// Shared memory of a block, in bytes: a layer's vectors twice | x | W_o or W_o2 | W_qkv, W_i or the gathered rows of ctx or h
+template <int MT, int CL>
+struct BsSmem {
+    static constexpr int NQ = 3 * kBsH / 8 / CL, NO = kBsH / 8 / CL, NI = kBsI / 8 / CL;        // column tiles per block of the three widths
+    static_assert(NQ * CL * 8 == 3 * kBsH && NO * CL * 8 == kBsH && NI * CL * 8 == kBsI, "whole tiles per block");
+    static constexpr int NV = 4 * kBsH + (NQ + 2 * NO + NI) * 8;
+    static constexpr int kPieces = MT <= 2 ? 1 : MT - 1;                                         // h arrives in so many pieces of its columns
+    static constexpr int kHPiece = kBsI / kPieces;
+    static constexpr size_t max2(size_t a, size_t b) { return a > b ? a : b; }
+    static constexpr size_t kX = (size_t)2 * NV * 4, kWo = kX + (size_t)MT * 16 * bs_ld(kBsH) * 2, kR = kWo + (size_t)NO * 8 * bs_ld(kBsI) * 2;
+    static constexpr size_t kBytes = kR + max2((size_t)(NQ > NI ? NQ : NI) * 8 * bs_ld(kBsH) * 2, max2((size_t)MT * 16 * bs_ld(kBsH) * 2, (size_t)MT * 16 * bs_ld(kHPiece) * 2));
+    static_assert(kHPiece % 32 == 0 && kX % 16 == 0 && kBytes <= 232448, "");
+};
 
 __device__ __forceinline__ void bs_arrive() { __syncwarp(); asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
 __device__ __forceinline__ void bs_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
 
-// One projection.  Output columns of the cluster: NT tiles of eight per block, block `rank` has columns [rank NT 8, ...); warp = (K quarter ks,
-// column half tg).  Within 32 columns of K a lane holds eight neighbouring ones of its row (16-byte loads); weights and activations are
-// permuted alike, so the sum does not change.
-template <int NT, int K>
-struct BsWeights {
-    static constexpr int HT = (NT + 1) / 2, STEPS = K / 4 / 32;
-    uint4 w[HT][STEPS];
-    __device__ __forceinline__ void load(const uint16_t* W, int rank, int warp, int lane) {
-        const int ks = warp & 3, tg = warp >> 2;
+// rows [0, ROWS) of a weight matrix [.., K], on their way
+template <int ROWS, int K>
+__device__ __forceinline__ void bs_bring_weights(uint16_t* dst, const uint16_t* W) {
+    for (int i = threadIdx.x; i < ROWS * (K / 4); i += kBsThreads) {
+        const int r = i / (K / 4), c = i % (K / 4) * 4;
+        cp_async8(dst + r * bs_ld(K) + bs_at(c), W + (size_t)r * K + c);
+    }
+}
+// columns [k0, k0 + KP) of the cluster's rows of an activation that the cluster wrote
+template <int KP>
+__device__ __forceinline__ void bs_bring_rows(uint16_t* dst, const uint16_t* src, int ld, int k0, int rows) {
+    for (int i = threadIdx.x; i < rows * (KP / 8); i += kBsThreads) {
+        const int r = i / (KP / 8), c = i % (KP / 8) * 8;
+        cp_async16(dst + r * bs_ld(KP) + c, src + (size_t)r * ld + k0 + c);
+    }
+}
+// One projection's NT x MT tiles of 8 columns x 16 rows, dealt to the warps: warp w has tiles w, w + 8, ... (column tiles first).
+template <int MT, int NT>
+struct BsTiles {
+    static constexpr int IT = (NT * MT + 7) / 8;
+    float acc[IT][4];
+    __device__ __forceinline__ void zero() {
 #pragma unroll
-        for (int i = 0; i < HT; ++i) {
-            const int tile = tg * HT + i;
-            if (tile < NT) {
-                const uint16_t* p = W + (size_t)((rank * NT + tile) * 8 + (lane >> 2)) * K + ks * (K / 4) + (lane & 3) * 8;
+        for (int i = 0; i < IT; ++i) acc[i][0] = acc[i][1] = acc[i][2] = acc[i][3] = 0.f;
+    }
+    // += A [.., KP] . columns [k0, k0 + KP) of W
+    template <int KP>
+    __device__ __forceinline__ void add(const uint16_t* A, const uint16_t* W, int ldw, int k0, int warp, int lane) {
+        const int g = lane >> 2, q = lane & 3;
+#pragma unroll 4
+        for (int s = 0; s < KP / 32; ++s)
 #pragma unroll
-                for (int s = 0; s < STEPS; ++s) w[i][s] = *reinterpret_cast<const uint4*>(p + s * 32);
+            for (int i = 0; i < IT; ++i) {
+                const int tile = warp + 8 * i;
+                if (tile < NT * MT) {
+                    const uint16_t* a = A + (tile / NT * 16 + g) * bs_ld(KP) + s * 32 + q * 8;
+                    const uint4 x0 = *reinterpret_cast<const uint4*>(a), x1 = *reinterpret_cast<const uint4*>(a + 8 * bs_ld(KP));
+                    const uint4 w = *reinterpret_cast<const uint4*>(W + (tile % NT * 8 + g) * ldw + k0 + s * 32 + q * 8);
+                    const uint32_t a0[4] = {x0.x, x1.x, x0.y, x1.y}, a1[4] = {x0.z, x1.z, x0.w, x1.w};
+                    mma_bf16_16816(acc[i], a0, w.x, w.y);
+                    mma_bf16_16816(acc[i], a1, w.z, w.w);
+                }
+            }
+    }
+    // out(row, column pair inside the block, sums)
+    template <typename Fn>
+    __device__ __forceinline__ void store(int rows, int warp, int lane, Fn&& out) const {
+#pragma unroll
+        for (int i = 0; i < IT; ++i) {
+            const int tile = warp + 8 * i;
+            if (tile < NT * MT) {
+                const int r = tile / NT * 16 + (lane >> 2), c = tile % NT * 8 + (lane & 3) * 2;
+                if (r < rows) out(r, c, make_float2(acc[i][0], acc[i][1]));
+                if (r + 8 < rows) out(r + 8, c, make_float2(acc[i][2], acc[i][3]));
             }
         }
     }
 };
-// red [4 quarters][MT 16 rows][NT 8 + 4] += A . W^T; row(r): pointer to row r's K activations (shared or global), r < MT 16
-template <int MT, int NT, int K, typename RowFn>
-__device__ __forceinline__ void bs_gemm(const BsWeights<NT, K>& bw, RowFn&& rows16, float* red, int warp, int lane) {
-    constexpr int LDR = NT * 8 + 4;
-    const int ks = warp & 3, tg = warp >> 2, g = lane >> 2, q = lane & 3;
-    using W = BsWeights<NT, K>;
-    float acc[MT][W::HT][4];
-#pragma unroll
-    for (int m = 0; m < MT; ++m)
-#pragma unroll
-        for (int i = 0; i < W::HT; ++i) acc[m][i][0] = acc[m][i][1] = acc[m][i][2] = acc[m][i][3] = 0.f;
-#pragma unroll
-    for (int s = 0; s < W::STEPS; ++s) {
-        const int k = ks * (K / 4) + s * 32 + q * 8;
-#pragma unroll
-        for (int m = 0; m < MT; ++m) {
-            const uint4 x0 = rows16(m * 16 + g, k), x1 = rows16(m * 16 + g + 8, k);
-            const uint32_t a0[4] = {x0.x, x1.x, x0.y, x1.y}, a1[4] = {x0.z, x1.z, x0.w, x1.w};
-#pragma unroll
-            for (int i = 0; i < W::HT; ++i)
-                if (tg * W::HT + i < NT) {
-                    const uint32_t b0[2] = {bw.w[i][s].x, bw.w[i][s].y}, b1[2] = {bw.w[i][s].z, bw.w[i][s].w};
-                    mma_bf16_16816(acc[m][i], a0, b0);
-                    mma_bf16_16816(acc[m][i], a1, b1);
-                }
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < MT; ++m)
-#pragma unroll
-        for (int i = 0; i < W::HT; ++i)
-            if (tg * W::HT + i < NT) {
-                float* r = red + (size_t)(ks * MT * 16 + m * 16 + g) * LDR + (tg * W::HT + i) * 8 + q * 2;
-                r[0] = acc[m][i][0]; r[1] = acc[m][i][1];
-                r[8 * LDR] = acc[m][i][2]; r[8 * LDR + 1] = acc[m][i][3];
-            }
-}
-// columns of the block, two at a time: out(row, column pair inside the block, sums of the four quarters)
-template <int MT, int NT, typename Fn>
-__device__ __forceinline__ void bs_fold(const float* red, int rows, Fn&& out) {
-    constexpr int LDR = NT * 8 + 4, HALF = NT * 4, Q = MT * 16 * LDR;
-    for (int i = threadIdx.x; i < rows * HALF; i += kBsThreads) {
-        const int r = i / HALF, c = i % HALF * 2;
-        const float* p = red + r * LDR + c;
-        float2 s = *reinterpret_cast<const float2*>(p);
-#pragma unroll
-        for (int k = 1; k < 4; ++k) {
-            const float2 v = *reinterpret_cast<const float2*>(p + k * Q);
-            s.x += v.x; s.y += v.y;
-        }
-        out(r, c, s);
-    }
-}
-
-__device__ __forceinline__ uint32_t bs_word(const uint4& v, int e) { return e == 0 ? v.x : (e == 1 ? v.y : (e == 2 ? v.z : v.w)); }
 
 // LayerNorm of the rows of pre (f32, global, written by the whole cluster) into the x tile; a warp has four rows on their way at a time
 // (w, b: shared memory)
@@ -142,29 +142,123 @@ __device__ __forceinline__ void bs_layernorm(const float* pre, int rows, const f
             for (int j = 0; j < 3; ++j) {
                 const int c = lane + 32 * j;
                 const float4 x = v[u][j], w4 = reinterpret_cast<const float4*>(w)[c], b4 = reinterpret_cast<const float4*>(b)[c];
-                *reinterpret_cast<uint2*>(sx + r * kBsLdX + 4 * c) = make_uint2(pack_bf16x2((x.x - mean) * inv * w4.x + b4.x, (x.y - mean) * inv * w4.y + b4.y),
-                                                                                pack_bf16x2((x.z - mean) * inv * w4.z + b4.z, (x.w - mean) * inv * w4.w + b4.w));
+                *reinterpret_cast<uint2*>(sx + r * bs_ld(kBsH) + bs_at(4 * c)) =
+                    make_uint2(pack_bf16x2((x.x - mean) * inv * w4.x + b4.x, (x.y - mean) * inv * w4.y + b4.y),
+                               pack_bf16x2((x.z - mean) * inv * w4.z + b4.z, (x.w - mean) * inv * w4.w + b4.w));
             }
         }
+    }
+}
+
+// bert_attn_kernel for 16 query rows of a head, operands straight from global memory (its key tiles behind the sentence add zeros; here there
+// are KT tiles of eight keys).  base: q columns of the head in the sentence's first row of q|k|v; ctx: the sentence's first row, permuted.
+template <int KT>
+__device__ __forceinline__ void bs_attention(const uint16_t* base, int t, int m0, float inv_scale, uint16_t* ctx, int lane) {
+    constexpr int LD = 3 * kBsH;
+    const int g = lane >> 2, q = lane & 3;
+    const uint2 zero2 = make_uint2(0u, 0u);
+    auto ld8 = [&](const uint16_t* p, int row) { return row < t ? __ldcg(reinterpret_cast<const uint2*>(p + (size_t)row * LD)) : zero2; };
+    uint32_t qa[2][4], vv[KT][4];
+    uint2 kk[KT][2];
+#pragma unroll
+    for (int ks = 0; ks < 2; ++ks) {
+        const uint2 x0 = ld8(base + ks * 16 + q * 4, m0 + g), x1 = ld8(base + ks * 16 + q * 4, m0 + g + 8);
+        qa[ks][0] = x0.x; qa[ks][1] = x1.x; qa[ks][2] = x0.y; qa[ks][3] = x1.y;
+    }
+#pragma unroll
+    for (int nt = 0; nt < KT; ++nt) {
+        const int key = nt * 8 + g;
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) kk[nt][ks] = ld8(base + kBsH + ks * 16 + q * 4, key);
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (key < t) v = __ldcg(reinterpret_cast<const uint4*>(base + 2 * kBsH + (size_t)key * LD + q * 8));
+        vv[nt][0] = v.x; vv[nt][1] = v.y; vv[nt][2] = v.z; vv[nt][3] = v.w;
+    }
+    float s[KT][4];
+#pragma unroll
+    for (int nt = 0; nt < KT; ++nt) {
+        s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+#pragma unroll
+        for (int ks = 0; ks < 2; ++ks) mma_bf16_16816(s[nt], qa[ks], kk[nt][ks].x, kk[nt][ks].y);
+    }
+    float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+    for (int nt = 0; nt < KT; ++nt) {
+#pragma unroll
+        for (int e = 0; e < 4; ++e) s[nt][e] = nt * 8 + q * 2 + (e & 1) < t ? s[nt][e] * inv_scale : -INFINITY;
+        mx0 = fmaxf(mx0, fmaxf(s[nt][0], s[nt][1]));
+        mx1 = fmaxf(mx1, fmaxf(s[nt][2], s[nt][3]));
+    }
+    mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, 2));
+    mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 2));
+    float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+    for (int nt = 0; nt < KT; ++nt) {
+        s[nt][0] = __expf(s[nt][0] - mx0); s[nt][1] = __expf(s[nt][1] - mx0);
+        s[nt][2] = __expf(s[nt][2] - mx1); s[nt][3] = __expf(s[nt][3] - mx1);
+        sum0 += s[nt][0] + s[nt][1];
+        sum1 += s[nt][2] + s[nt][3];
+    }
+    sum0 += __shfl_xor_sync(0xFFFFFFFFu, sum0, 1); sum0 += __shfl_xor_sync(0xFFFFFFFFu, sum0, 2);
+    sum1 += __shfl_xor_sync(0xFFFFFFFFu, sum1, 1); sum1 += __shfl_xor_sync(0xFFFFFFFFu, sum1, 2);
+    // A lane's 16 bytes of a key are channels 8 q .. 8 q + 7; transposing register j of eight keys gives the operand of the channels
+    // {8 q' + 2 j, 8 q' + 2 j + 1: q' < 4}, and the sums o[j] of this lane are those of its own q: eight neighbouring channels per row.
+    float o[4][4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) o[j][0] = o[j][1] = o[j][2] = o[j][3] = 0.f;
+#pragma unroll
+    for (int ks = 0; ks < KT / 2; ++ks) {
+        const uint32_t pa[4] = {pack_bf16(s[2 * ks][0], s[2 * ks][1]), pack_bf16(s[2 * ks][2], s[2 * ks][3]), pack_bf16(s[2 * ks + 1][0], s[2 * ks + 1][1]),
+                                pack_bf16(s[2 * ks + 1][2], s[2 * ks + 1][3])};
+#pragma unroll
+        for (int j = 0; j < 4; ++j) mma_bf16_16816(o[j], pa, movmatrix_trans(vv[2 * ks][j]), movmatrix_trans(vv[2 * ks + 1][j]));
+    }
+    const float i0 = 1.f / sum0, i1 = 1.f / sum1;
+#pragma unroll
+    for (int hf = 0; hf < 2; ++hf) {        // channels 8 q + 4 hf ..
+        uint16_t* p = ctx + bs_at(q * 8 + hf * 4);
+        const float *a = o[2 * hf], *b = o[2 * hf + 1];
+        if (m0 + g < t) *reinterpret_cast<uint2*>(p + (size_t)(m0 + g) * kBsH) = make_uint2(pack_bf16(a[0] * i0, a[1] * i0), pack_bf16(b[0] * i0, b[1] * i0));
+        if (m0 + g + 8 < t) *reinterpret_cast<uint2*>(p + (size_t)(m0 + g + 8) * kBsH) = make_uint2(pack_bf16(a[2] * i1, a[3] * i1), pack_bf16(b[2] * i1, b[3] * i1));
     }
 }
 
 // MT: row tiles of 16 (the cluster's tokens, rounded up); CL: blocks per cluster.  grid clusters * CL.
 template <int MT, int CL>
 static __global__ void __launch_bounds__(kBsThreads, 1) bert_small_kernel(const BertSmallArgs a) {
-    constexpr int NQ = 3 * kBsH / 8 / CL, NO = kBsH / 8 / CL, NI = kBsI / 8 / CL;        // column tiles per block of the three widths
-    static_assert(NQ * CL * 8 == 3 * kBsH && NO * CL * 8 == kBsH && NI * CL * 8 == kBsI, "whole tiles per block");
+    using M = BsSmem<MT, CL>;
+    constexpr int NQ = M::NQ, NO = M::NO, NI = M::NI, LDX = bs_ld(kBsH);
     extern __shared__ __align__(16) uint8_t bs_smem[];
-    uint16_t* sx = reinterpret_cast<uint16_t*>(bs_smem);                                // [MT 16][kBsLdX]
-    float* red = reinterpret_cast<float*>(bs_smem + (size_t)MT * 16 * kBsLdX * 2);      // [4][MT 16][NI 8 + 4]
+    float* sv = reinterpret_cast<float*>(bs_smem);                          // a layer's vectors, two layers
+    uint16_t* sx = reinterpret_cast<uint16_t*>(bs_smem + M::kX);            // x
+    uint16_t* swo = reinterpret_cast<uint16_t*>(bs_smem + M::kWo);          // W_o, W_o2
+    uint16_t* sr = reinterpret_cast<uint16_t*>(bs_smem + M::kR);            // W_qkv | ctx | W_i | h, one after the other
     const int rank = blockIdx.x % CL, cl = blockIdx.x / CL, tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const int s0 = cl * a.spc, ns = min(a.spc, a.b - s0), rows = ns * a.t;
     const size_t row0 = (size_t)s0 * a.t;
     uint16_t *qkv = a.qkv + row0 * 3 * kBsH, *ctx = a.ctx + row0 * kBsH, *hb = a.h + row0 * kBsI;
     float* pre = a.pre + row0 * kBsH;
 
+    // the block's biases and the LayerNorm vectors of a layer: [2][ln1w | ln1b | ln2w | ln2b | bqkv | bo | bi | bo2]; its rows of W_qkv
+    auto bring_layer = [&](int l) {
+        const BertSmallLayer& w = a.layers[l];
+        float* d = sv + (l & 1) * M::NV;
+        for (int i = tid; i < kBsH; i += kBsThreads) {
+            cp_async_f32(d + i, w.ln1w + i); cp_async_f32(d + kBsH + i, w.ln1b + i);
+            cp_async_f32(d + 2 * kBsH + i, w.ln2w + i); cp_async_f32(d + 3 * kBsH + i, w.ln2b + i);
+        }
+        d += 4 * kBsH;
+        if (tid < NQ * 8) cp_async_f32(d + tid, w.bqkv + rank * NQ * 8 + tid);
+        if (tid < NO * 8) { cp_async_f32(d + NQ * 8 + tid, w.bo + rank * NO * 8 + tid); cp_async_f32(d + (NQ + NO + NI) * 8 + tid, w.bo2 + rank * NO * 8 + tid); }
+        if (tid < NI * 8) cp_async_f32(d + (NQ + NO) * 8 + tid, w.bi + rank * NI * 8 + tid);
+        bs_bring_weights<NQ * 8, kBsH>(sr, w.wqkv + (size_t)rank * NQ * 8 * kBsH);
+        bs_bring_weights<NO * 8, kBsH>(swo, w.wo + (size_t)rank * NO * 8 * kBsH);
+        cp_async_commit();
+    };
+    bring_layer(0);
+
     // word + position embedding, LayerNorm (eps 1e-12): every block for itself; rows behind the sentences are zero
-    for (int i = tid; i < (MT * 16 - rows) * kBsLdX; i += kBsThreads) sx[(size_t)rows * kBsLdX + i] = 0;
+    for (int i = tid; i < (MT * 16 - rows) * LDX; i += kBsThreads) sx[(size_t)rows * LDX + i] = 0;
     for (int r = warp; r < rows; r += kBsThreads / 32) {
         const uint32_t id = min(a.ids[row0 + r], (uint32_t)(a.V - 1));
         const int pos = min(r % a.t, a.maxpos - 1);
@@ -184,150 +278,96 @@ static __global__ void __launch_bounds__(kBsThreads, 1) bert_small_kernel(const 
 #pragma unroll
         for (int j = 0; j < 12; ++j) {
             const int c = lane + 32 * j;
-            sx[r * kBsLdX + c] = f32_to_bf16_rne((v[j] - mean) * inv * a.lnw[c] + a.lnb[c]);
+            sx[r * LDX + bs_at(c)] = f32_to_bf16_rne((v[j] - mean) * inv * a.lnw[c] + a.lnb[c]);
         }
     }
-    auto from_x = [&](int r, int k) { return *reinterpret_cast<const uint4*>(sx + r * kBsLdX + k); };
-    const uint4 zero4 = make_uint4(0u, 0u, 0u, 0u);
-    // the block's biases and the LayerNorm vectors of a layer, on their way a layer ahead: [2][ln1w | ln1b | ln2w | ln2b | bqkv | bo | bi | bo2]
-    constexpr int NB = (NQ + 2 * NO + NI) * 8, NV = 4 * kBsH + NB;
-    float* sv = red + (size_t)4 * MT * 16 * (NI * 8 + 4);
-    auto bring_vectors = [&](int l) {
-        const BertSmallLayer& w = a.layers[l];
-        float* d = sv + (l & 1) * NV;
-        for (int i = tid; i < kBsH; i += kBsThreads) {
-            cp_async_f32(d + i, w.ln1w + i); cp_async_f32(d + kBsH + i, w.ln1b + i);
-            cp_async_f32(d + 2 * kBsH + i, w.ln2w + i); cp_async_f32(d + 3 * kBsH + i, w.ln2b + i);
-        }
-        d += 4 * kBsH;
-        if (tid < NQ * 8) cp_async_f32(d + tid, w.bqkv + rank * NQ * 8 + tid);
-        if (tid < NO * 8) { cp_async_f32(d + NQ * 8 + tid, w.bo + rank * NO * 8 + tid); cp_async_f32(d + (NQ + NO + NI) * 8 + tid, w.bo2 + rank * NO * 8 + tid); }
-        if (tid < NI * 8) cp_async_f32(d + (NQ + NO) * 8 + tid, w.bi + rank * NI * 8 + tid);
-        cp_async_commit();
-    };
-    bring_vectors(0);
 
-    BsWeights<NQ, kBsH> wq;
-    wq.load(a.layers[0].wqkv, rank, warp, lane);
 #pragma unroll 1
     for (int l = 0; l < a.L; ++l) {
         const BertSmallLayer& w = a.layers[l];
         cp_async_wait<0>();
-        __syncthreads();                    // the x tile and the layer's vectors are complete
-        const float *ln1w = sv + (l & 1) * NV, *ln1b = ln1w + kBsH, *ln2w = ln1b + kBsH, *ln2b = ln2w + kBsH, *bqkv = ln2b + kBsH, *bo = bqkv + NQ * 8, *bi = bo + NO * 8,
+        __syncthreads();                    // the x tile, the layer's vectors, W_qkv and W_o are complete
+        const float *ln1w = sv + (l & 1) * M::NV, *ln1b = ln1w + kBsH, *ln2w = ln1b + kBsH, *ln2b = ln2w + kBsH, *bqkv = ln2b + kBsH, *bo = bqkv + NQ * 8, *bi = bo + NO * 8,
                     *bo2 = bi + NI * 8;
-        bs_gemm<MT, NQ, kBsH>(wq, from_x, red, warp, lane);
-        __syncthreads();
-        bs_fold<MT, NQ>(red, rows, [&](int r, int c, float2 s) {
-            const int col = rank * NQ * 8 + c;
-            *reinterpret_cast<uint32_t*>(qkv + (size_t)r * 3 * kBsH + col) = pack_bf16x2(s.x + bqkv[c], s.y + bqkv[c + 1]);
-        });
-        BsWeights<NO, kBsH> wo;
+        {
+            BsTiles<MT, NQ> y;
+            y.zero();
+            y.template add<kBsH>(sx, sr, bs_ld(kBsH), 0, warp, lane);
+            y.store(rows, warp, lane, [&](int r, int c, float2 s) {
+                *reinterpret_cast<uint32_t*>(qkv + (size_t)r * 3 * kBsH + rank * NQ * 8 + c) = pack_bf16x2(s.x + bqkv[c], s.y + bqkv[c + 1]);
+            });
+        }
         bs_arrive();
-        wo.load(w.wo, rank, warp, lane);
         bs_wait();
-        {   // attention: the cluster's warps share the (sentence, head) pairs, several warps of a pair its query rows
-            // (whole stretches of `per` rows only: the first row of every item is one of the sentence)
-            const int pairs = ns * kBsHeads, warps = CL * (kBsThreads / 32), most = max(1, min(a.t, warps / pairs)), per = (a.t + most - 1) / most, split = (a.t + per - 1) / per;
-            for (int it = warp * CL + rank; it < pairs * split; it += warps) {
-                const int pr = it % pairs, sent = pr / kBsHeads, head = pr % kBsHeads, first = it / pairs * per, last = min(a.t, first + per);
-                const uint16_t* base = qkv + (size_t)sent * a.t * 3 * kBsH + head * kBertD;
-                uint4 kk[2][4], vv[2][4];   // this lane's keys and values: lane, lane + 32
-#pragma unroll
-                for (int u = 0; u < 2; ++u)
-#pragma unroll
-                    for (int c = 0; c < 4; ++c) {
-                        const uint4* p = reinterpret_cast<const uint4*>(base + (size_t)(lane + 32 * u) * 3 * kBsH + kBsH) + c;
-                        kk[u][c] = lane + 32 * u < a.t ? __ldcg(p) : zero4;
-                        vv[u][c] = lane + 32 * u < a.t ? __ldcg(p + kBsH / 8) : zero4;
-                    }
-                uint16_t qn = __ldcg(base + (size_t)first * 3 * kBsH + lane);
-                for (int i = first; i < last; ++i) {
-                    const float qv = __uint_as_float((uint32_t)qn << 16) * a.inv_scale;
-                    if (i + 1 < last) qn = __ldcg(base + (size_t)(i + 1) * 3 * kBsH + lane);
-                    float sc[2] = {0.f, 0.f};
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const float q0 = __shfl_sync(0xFFFFFFFFu, qv, c * 8 + e * 2), q1 = __shfl_sync(0xFFFFFFFFu, qv, c * 8 + e * 2 + 1);
-#pragma unroll
-                            for (int u = 0; u < 2; ++u) {
-                                const uint32_t kv = bs_word(kk[u][c], e);
-                                sc[u] = fmaf(q0, bf16lo(kv), fmaf(q1, bf16hi(kv), sc[u]));
-                            }
-                        }
-                    if (lane >= a.t) sc[0] = -INFINITY;
-                    if (lane + 32 >= a.t) sc[1] = -INFINITY;
-                    const float m = warp_max(fmaxf(sc[0], sc[1]));
-                    sc[0] = __expf(sc[0] - m);
-                    sc[1] = __expf(sc[1] - m);
-                    const float inv = 1.f / warp_sum(sc[0] + sc[1]);
-                    // 32 sums over the lanes: halves of them are exchanged, lane c ends with channel c's
-                    float o[32];
-#pragma unroll
-                    for (int c = 0; c < 4; ++c)
-#pragma unroll
-                        for (int e = 0; e < 4; ++e) {
-                            const uint32_t v0 = bs_word(vv[0][c], e), v1 = bs_word(vv[1][c], e);
-                            o[c * 8 + e * 2] = fmaf(sc[0], bf16lo(v0), sc[1] * bf16lo(v1));
-                            o[c * 8 + e * 2 + 1] = fmaf(sc[0], bf16hi(v0), sc[1] * bf16hi(v1));
-                        }
-#pragma unroll
-                    for (int n = 16; n >= 1; n >>= 1) {
-                        const bool up = lane & n;
-#pragma unroll
-                        for (int j = 0; j < n; ++j) {
-                            const float give = up ? o[j] : o[j + n], keep = up ? o[j + n] : o[j];
-                            o[j] = keep + __shfl_xor_sync(0xFFFFFFFFu, give, n);
-                        }
-                    }
-                    ctx[(size_t)(sent * a.t + i) * kBsH + head * kBertD + lane] = f32_to_bf16_rne(o[0] * inv);
-                }
+        {   // attention: the cluster's warps share the (sentence, head, 16 query rows)
+            const int pairs = ns * kBsHeads, per = 16, split = (a.t + per - 1) / per;
+            for (int it = warp * CL + rank; it < pairs * split; it += CL * (kBsThreads / 32)) {
+                const int pr = it % pairs, sent = pr / kBsHeads, head = pr % kBsHeads;
+                bs_attention<2 * MT>(qkv + (size_t)sent * a.t * 3 * kBsH + head * kBertD, a.t, it / pairs * per, a.inv_scale, ctx + (size_t)sent * a.t * kBsH + head * kBertD, lane);
             }
         }
         bs_arrive();
         bs_wait();
-        auto from_ctx = [&](int r, int k) { return r < rows ? __ldcg(reinterpret_cast<const uint4*>(ctx + (size_t)r * kBsH + k)) : zero4; };
-        bs_gemm<MT, NO, kBsH>(wo, from_ctx, red, warp, lane);
-        __syncthreads();
         auto residual = [&](const float* bias) {
             return [&, bias](int r, int c, float2 s) {
                 const int col = rank * NO * 8 + c;
-                const uint32_t x = *reinterpret_cast<const uint32_t*>(sx + r * kBsLdX + col);
+                const uint32_t x = *reinterpret_cast<const uint32_t*>(sx + r * LDX + bs_at(col));
                 *reinterpret_cast<float2*>(pre + (size_t)r * kBsH + col) = make_float2(s.x + bias[c] + bf16lo(x), s.y + bias[c + 1] + bf16hi(x));
             };
         };
-        bs_fold<MT, NO>(red, rows, residual(bo));
-        BsWeights<NI, kBsH> wi;
+        bs_bring_rows<kBsH>(sr, ctx, kBsH, 0, rows);
+        cp_async_commit();
+        cp_async_wait<0>();
+        __syncthreads();
+        {
+            BsTiles<MT, NO> y;
+            y.zero();
+            y.template add<kBsH>(sr, swo, bs_ld(kBsH), 0, warp, lane);
+            y.store(rows, warp, lane, residual(bo));
+        }
         bs_arrive();
-        wi.load(w.wi, rank, warp, lane);
+        __syncthreads();                    // ctx and W_o have been read
+        bs_bring_weights<NI * 8, kBsH>(sr, w.wi + (size_t)rank * NI * 8 * kBsH);
+        cp_async_commit();
+        bs_bring_weights<NO * 8, kBsI>(swo, w.wo2 + (size_t)rank * NO * 8 * kBsI);
+        cp_async_commit();
         bs_wait();
         bs_layernorm(pre, rows, ln1w, ln1b, a.eps, sx, warp, lane);
+        cp_async_wait<1>();
         __syncthreads();
-        bs_gemm<MT, NI, kBsH>(wi, from_x, red, warp, lane);
-        __syncthreads();
-        bs_fold<MT, NI>(red, rows, [&](int r, int c, float2 s) {
-            const int col = rank * NI * 8 + c;
-            *reinterpret_cast<uint32_t*>(hb + (size_t)r * kBsI + col) = pack_bf16x2(gelu_tanh_f(s.x + bi[c]), gelu_tanh_f(s.y + bi[c + 1]));
-        });
-        BsWeights<NO, kBsI> wd;
+        {
+            BsTiles<MT, NI> y;
+            y.zero();
+            y.template add<kBsH>(sx, sr, bs_ld(kBsH), 0, warp, lane);
+            y.store(rows, warp, lane, [&](int r, int c, float2 s) {
+                *reinterpret_cast<uint32_t*>(hb + (size_t)r * kBsI + bs_at(rank * NI * 8 + c)) = pack_bf16x2(gelu_tanh_f(s.x + bi[c]), gelu_tanh_f(s.y + bi[c + 1]));
+            });
+        }
         bs_arrive();
-        wd.load(w.wo2, rank, warp, lane);
-        if (l + 1 < a.L) bring_vectors(l + 1);
         bs_wait();
-        auto from_h = [&](int r, int k) { return r < rows ? __ldcg(reinterpret_cast<const uint4*>(hb + (size_t)r * kBsI + k)) : zero4; };
-        bs_gemm<MT, NO, kBsI>(wd, from_h, red, warp, lane);
-        __syncthreads();
-        bs_fold<MT, NO>(red, rows, residual(bo2));
+        {
+            BsTiles<MT, NO> y;
+            y.zero();
+#pragma unroll 1
+            for (int p = 0; p < M::kPieces; ++p) {
+                if (p > 0) __syncthreads();                 // the piece before has been read (the first: W_i, by everybody in front of the barrier)
+                bs_bring_rows<M::kHPiece>(sr, hb, kBsI, p * M::kHPiece, rows);
+                cp_async_commit();
+                cp_async_wait<0>();
+                __syncthreads();
+                y.template add<M::kHPiece>(sr, swo, bs_ld(kBsI), p * M::kHPiece, warp, lane);
+            }
+            y.store(rows, warp, lane, residual(bo2));
+        }
         bs_arrive();
-        if (l + 1 < a.L) wq.load(a.layers[l + 1].wqkv, rank, warp, lane);
+        __syncthreads();                    // h and W_o2 have been read
+        if (l + 1 < a.L) bring_layer(l + 1);
         bs_wait();
         bs_layernorm(pre, rows, ln2w, ln2b, a.eps, sx, warp, lane);
     }
     __syncthreads();
-    // masked mean pooling and L2 norm: a block takes every CL-th sentence, a thread up to two columns
-    __shared__ float tot[kBsThreads / 32];
+    // masked mean pooling and L2 norm: a block takes every CL-th sentence, a thread up to two columns; tot[w]: squares of columns 32 w ..
+    __shared__ float tot[kBsH / 32];
     for (int s = rank; s < ns; s += CL) {
         float acc[2] = {0.f, 0.f}, cnt = 0.f;
         for (int r = 0; r < a.t; ++r) {
@@ -336,16 +376,18 @@ static __global__ void __launch_bounds__(kBsThreads, 1) bert_small_kernel(const 
 #pragma unroll
             for (int u = 0; u < 2; ++u) {
                 const int c = tid + u * kBsThreads;
-                if (c < kBsH) acc[u] = fmaf(__uint_as_float((uint32_t)sx[(s * a.t + r) * kBsLdX + c] << 16), m, acc[u]);
+                if (c < kBsH) acc[u] = fmaf(__uint_as_float((uint32_t)sx[(s * a.t + r) * LDX + bs_at(c)] << 16), m, acc[u]);
             }
         }
-        acc[0] /= cnt * (float)kBsH;
-        acc[1] /= cnt * (float)kBsH;
-        const float sq = warp_sum(acc[0] * acc[0] + acc[1] * acc[1]);
-        if (lane == 0) tot[warp] = sq;
+#pragma unroll
+        for (int u = 0; u < 2; ++u) {
+            acc[u] /= cnt * (float)kBsH;
+            const float sq = warp_sum(acc[u] * acc[u]);
+            if (lane == 0 && warp + 8 * u < kBsH / 32) tot[warp + 8 * u] = sq;
+        }
         __syncthreads();
         float sum = 0.f;
-        for (int k = 0; k < kBsThreads / 32; ++k) sum += tot[k];
+        for (int k = 0; k < kBsH / 32; ++k) sum += tot[k];
         __syncthreads();
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
@@ -355,6 +397,6 @@ static __global__ void __launch_bounds__(kBsThreads, 1) bert_small_kernel(const 
     }
 }
 template <int MT, int CL>
-constexpr size_t bert_small_smem() { return (size_t)MT * 16 * kBsLdX * 2 + (size_t)4 * MT * 16 * (kBsI / CL + 4) * 4 + (size_t)2 * (4 * kBsH + (5 * kBsH + kBsI) / CL) * 4; }
+constexpr size_t bert_small_smem() { return BsSmem<MT, CL>::kBytes; }
 
 }  // namespace fl

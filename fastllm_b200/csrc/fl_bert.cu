@@ -329,7 +329,7 @@ static bool bert_enqueue_small(BertModel& m, int b, int t, bool has_mask) {
     const int spc = (b + resident - 1) / resident, clusters = (b + spc - 1) / spc, rows = spc * t;
     if (rows > kBsTokens) return false;
     const BertSmallArgs a{static_cast<const BertSmallLayer*>(m.small_layers), m.wemb, m.pemb, m.lnw, m.lnb, m.ids.p, has_mask ? m.mask.p : nullptr,
-                          m.L, b, t, m.V, m.maxpos, spc, m.cfg.norm_eps, (float)(1.0 / std::sqrt((double)m.d)), m.qkv.p, m.ctx.p, m.hbuf.p, m.pre.p, m.out.p};
+                          m.L, b, t, m.V, m.maxpos, spc, m.cfg.norm_eps, 1.f / (float)std::sqrt((double)m.d), m.qkv.p, m.ctx.p, m.hbuf.p, m.pre.p, m.out.p};
     switch ((rows + 15) / 16) {
         case 1: bert_small_launch<1>(m, a, clusters, false); break;
         case 2: bert_small_launch<2>(m, a, clusters, false); break;

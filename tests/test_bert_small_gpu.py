@@ -26,3 +26,21 @@ def test_short_sentences(b, t):
     # a sentence's embedding is that of the sentence alone, beyond the order of sums
     alone = m.embed_ids(ids[-1:])
     assert B._cos(alone, m.embed_ids(ids)[-1:]).min() >= B.COS_TOL
+
+
+@pytest.mark.parametrize("t", [1, 2, 5, 15, 16, 17, 19, 32, 33, 48, 49, 64])
+def test_same_bits_as_the_launch_chain(t):
+    """a sentence comes out the same whether it is embedded with few others (one launch) or in a batch that takes the chain: every sum of the
+    one-launch kernel runs in the chain's order"""
+    cfg = obert.MINILM_L6
+    w = obert.synth_weights(cfg, 0, 0.02)
+    m = B._product(cfg, w)
+    b = 16 * (64 // t + 1)              # more than 64 tokens for each of up to 16 clusters (148 SMs hold nine)
+    ids = synth.token_ids(700 + t, cfg.vocab_size, (b, t))
+    mask = np.ones((b, t), dtype=np.uint32)
+    mask[1::3, -(t // 3):] = 0 if t >= 3 else 1
+    for k in (None, mask):
+        whole = m.embed_ids(ids, k)
+        for few in (1, 2, 9, min(b, 9 * (64 // t))):
+            assert np.array_equal(m.embed_ids(ids[:few], None if k is None else k[:few]), whole[:few])
+            assert np.array_equal(m.embed_ids(ids[-few:], None if k is None else k[-few:]), whole[-few:])
