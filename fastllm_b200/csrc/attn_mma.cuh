@@ -632,7 +632,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const __
     constexpr uint32_t kKOff = kPOff + 65536, kVOff = kKOff + NK * kTile;
     extern __shared__ __align__(1024) uint8_t tcsm_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(tcsm_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t k_full[NK], k_empty[NK], v_full[NV], v_empty[NV], s_full[kTcSBufs], s_free[kTcSBufs], p_ready[2], p_free[2], o_done, q_ready;
+    __shared__ __align__(8) uint64_t k_full[NK], k_empty[NK], v_full[NV], v_empty[NV], s_full[kTcSBufs], s_free[kTcSBufs], p_ready[2], p_free[2], q_ready;
     __shared__ uint32_t s_tmem;
     __shared__ float xmax[2][2][kTcQ];      // [page parity][column half][row]: page maxima of the two halves of a row
     __shared__ float xsum[2][kTcQ];         // their row sums (epilogue)
@@ -650,7 +650,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const __
         for (int i = 0; i < NV; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
         for (int i = 0; i < kTcSBufs; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 8); }
         for (int i = 0; i < 2; ++i) { mbar_init(&p_ready[i], 8); mbar_init(&p_free[i], 1); }
-        mbar_init(&o_done, 1);
         mbar_init(&q_ready, 8);
         mbar_fence_init();
     }
@@ -708,7 +707,6 @@ __global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const __
                     }
                     umma_commit(&v_empty[pi % NV]);
                     umma_commit(&p_free[b]);
-                    umma_commit(&o_done);
                     ++pi;
                 } else if (qi < nkt && mbar_test(&k_full[qi % NK], (qi / NK) & 1) &&
                            mbar_test(&s_free[qi % kTcSBufs], ((qi / kTcSBufs) & 1) ^ 1)) {
@@ -807,8 +805,11 @@ __global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const __
             }
             l = l * alpha + ps;
             if (j > 0 && __any_sync(0xFFFFFFFFu, bump)) {
-                // O may be touched only when the previous P.V has completed; the warp rescales its half of the columns of its 32 lanes
-                mbar_wait(&o_done, (j - 1) & 1);
+                // O may be touched only when the previous P.V has completed; the warp rescales its half of the columns of its 32 lanes.
+                // (A parity names one phase only while the phase before it is known to be over: on this P buffer that is P.V of page
+                // j - 3, which page j - 1 waited for below.  One barrier with a phase per page would not do: P.V of page j - 2 may
+                // still be in flight here, and then the parity of page j - 1 is that of page j - 3.)
+                mbar_wait(&p_free[b ^ 1], ((j - 1) >> 1) & 1);
                 tc_fence_after();
 #pragma unroll 1
                 for (int c4 = 0; c4 < D / 64; ++c4) {
@@ -843,7 +844,7 @@ __global__ void __launch_bounds__(kTcThreads, 1) attn_prefill_tc_kernel(const __
         xsum[grp][r] = l;
         gsync();
         const float inv = 1.f / (l + xsum[grp ^ 1][r]);
-        mbar_wait(&o_done, (nkt - 1) & 1);
+        mbar_wait(&p_free[(nkt - 1) & 1], ((nkt - 1) >> 1) & 1);       // the last P.V, and with it all before
         tc_fence_after();
         const size_t obase = (((size_t)seq * a.t + irow) * a.nh + head) * D + grp * (D / 2);
 #pragma unroll 1

@@ -104,7 +104,7 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
     constexpr uint32_t kQBytes = HALF * 16384, kPOff = 2 * kQBytes, kKTile = DK * 128, kVTile = DV * 128, kKOff = kPOff + 65536, kVOff = kKOff + NK * kKTile;
     extern __shared__ __align__(1024) uint8_t gtsm_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gtsm_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t k_full[NK], k_empty[NK], v_full[NV], v_empty[NV], s_full[NS], s_free[NS], p_ready[2], p_free[2], o_done, q_ready;
+    __shared__ __align__(8) uint64_t k_full[NK], k_empty[NK], v_full[NV], v_empty[NV], s_full[NS], s_free[NS], p_ready[2], p_free[2], q_ready;
     __shared__ uint32_t s_tmem;
     __shared__ float xmax[2][2][kGtQ], xsum[2][kGtQ];
 
@@ -122,7 +122,6 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
         for (int i = 0; i < NV; ++i) { mbar_init(&v_full[i], 1); mbar_init(&v_empty[i], 1); }
         for (int i = 0; i < NS; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 8); }
         for (int i = 0; i < 2; ++i) { mbar_init(&p_ready[i], 8); mbar_init(&p_free[i], 1); }
-        mbar_init(&o_done, 1);
         mbar_init(&q_ready, 8);
         mbar_fence_init();
     }
@@ -176,7 +175,6 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
                     }
                     umma_commit(&v_empty[pi % NV]);
                     umma_commit(&p_free[b]);
-                    umma_commit(&o_done);
                     ++pi;
                     spin = 0;
                 } else if (qi < np && mbar_test(&k_full[qi % NK], (qi / NK) & 1) && mbar_test(&s_free[qi % NS], ((qi / NS) & 1) ^ 1)) {
@@ -276,7 +274,7 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
             }
             l = l * alpha + ps;
             if (j > 0 && __any_sync(0xFFFFFFFFu, bump)) {
-                ok &= gt_wait(&o_done, (j - 1) & 1);
+                ok &= gt_wait(&p_free[b ^ 1], ((j - 1) >> 1) & 1);      // the P.V before has completed (which barrier: see attn_prefill_tc_kernel)
                 tc_fence_after();
 #pragma unroll 1
                 for (int c4 = 0; c4 < DV / 64; ++c4) {
@@ -311,7 +309,7 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
         gsync();
         float sum = l + xsum[half ^ 1][r];
         if (a.sink) sum += ex2_approx(fmaf(a.sinkv ? a.sinkv[head] : 0.f, kLog2e, -m));
-        ok &= gt_wait(&o_done, (np - 1) & 1);
+        ok &= gt_wait(&p_free[(np - 1) & 1], ((np - 1) >> 1) & 1);      // the last P.V, and with it all before
         tc_fence_after();
         const float inv = ok ? 1.f / sum : __int_as_float(0x7FC00000);
         const int row = a.row0 + lrow;
