@@ -202,13 +202,16 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
         const int lrow = min(q0 + r, a.Ts - 1), irow = a.pos0 + lrow;          // rows past the portion are clamped: computed, never stored
         const uint32_t lane_addr = (uint32_t)(quarter * 32) << 16;
         auto gsync = [] { asm volatile("bar.sync 2, 256;" ::: "memory"); };
-        {   // q row -> hi | lo halves, swizzled operand layout
+        {   // q row times the score scale -> hi | lo halves, swizzled operand layout.  (Scaled here and not with the scores: a masked score is
+            // -inf, which a scale of zero or below would turn into NaN or +inf, and the maximum would be that of the unscaled scores.)
             const float* qsrc = a.proj + (size_t)(a.row0 + lrow) * a.ldp + a.off_q + (size_t)head * a.D;
 #pragma unroll
             for (int cc = 0; cc < DK / 16; ++cc) {
                 const int c = half * (DK / 16) + cc;
                 float4 x = make_float4(0.f, 0.f, 0.f, 0.f), y = x;
                 if (c * 8 < a.D) { x = *reinterpret_cast<const float4*>(qsrc + c * 8); y = *reinterpret_cast<const float4*>(qsrc + c * 8 + 4); }
+                x.x *= a.scale; x.y *= a.scale; x.z *= a.scale; x.w *= a.scale;
+                y.x *= a.scale; y.y *= a.scale; y.z *= a.scale; y.w *= a.scale;
                 uint4 h, l;
                 h.x = pack_bf16x2(x.x, x.y); h.y = pack_bf16x2(x.z, x.w); h.z = pack_bf16x2(y.x, y.y); h.w = pack_bf16x2(y.z, y.w);
                 l.x = pack_bf16x2(x.x - bf16lo(h.x), x.y - bf16hi(h.x)); l.y = pack_bf16x2(x.z - bf16lo(h.y), x.w - bf16hi(h.y));
@@ -223,7 +226,7 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
         }
         constexpr float kLog2e = 1.4426950408889634f;
         const bool cap = a.softcap > 0.f;
-        const float in_cap = cap ? a.scale / a.softcap : 0.f, c2 = cap ? kLog2e : a.scale * kLog2e;       // scores are carried in the exp2 domain
+        const float in_cap = cap ? 1.f / a.softcap : 0.f;
         const int w_lo = a.window > 0 ? irow - a.window + 1 : 0, c_lo = a.chunk > 0 ? irow / a.chunk * a.chunk : 0;
         float m = -INFINITY, l = 0.f;
         bool ok = true;
@@ -259,7 +262,7 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
             }
             xmax[b][half][r] = mx;
             gsync();
-            mx = fmaxf(mx, xmax[b][half ^ 1][r]) * c2;
+            mx = fmaxf(mx, xmax[b][half ^ 1][r]) * kLog2e;           // offsets and exponents in the exp2 domain
             // the offset m follows the maximum lazily (see attn_prefill_tc_kernel)
             const bool bump = mx > m + a.tau;
             const float mn = bump ? mx : m;
@@ -269,7 +272,7 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
             float ps = 0.f;
 #pragma unroll
             for (int e = 0; e < 32; ++e) {
-                sc[e] = ex2_approx(fmaf(sc[e], c2, -mu));
+                sc[e] = ex2_approx(fmaf(sc[e], kLog2e, -mu));
                 ps += sc[e];
             }
             l = l * alpha + ps;

@@ -169,3 +169,11 @@ def test_sliding_convolution(layer):
 def test_expert_lists_of_many_picks(n, experts, top):
     """more than one round of 256 picks per list, lists that end on its border"""
     check(N, N.config([N.gla(heads=2, dim=16, vdim=16, mlp=N.moe(ff=24, experts=experts, top=top, shared=(24, 0.75)))], vocab=64, width=64), n, 91)
+
+
+@pytest.mark.parametrize("scale", [-0.3, 0.0])
+@pytest.mark.parametrize("softcap", [None, 4.0])
+def test_attention_scale_of_any_sign(scale, softcap):
+    """a scale of zero or below: masked scores stay masked, the maximum is that of the scaled scores"""
+    both_ways(R, R.config([R.att(heads=2, kv_heads=1, dim=32, vdim=32, rot_dims=8, scale=scale, softcap=softcap)], width=64), 200, [130, 64], 73)
+    both_ways(M, M.config([M.par_layer(M.windowed(dim=16, vdim=16, window=257, keep=2, scale=scale), M.lightning(heads=2, dim=8, vdim=8))], width=64), 400, [70, 201, 100], 74)
