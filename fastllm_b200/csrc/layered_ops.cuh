@@ -2401,6 +2401,10 @@ static __global__ void ly_router_kernel(const float* __restrict__ h, int W, cons
             float bv = -1.f;
             for (int e = 0; e < E; ++e)
                 if (z[e] > bv) { bv = z[e]; best = e; }
+            if (best < 0) {                     // only scores that are not numbers are left: the first of them (every choice is an expert)
+                for (best = 0; z[best] == -2.f;) ++best;
+                bv = z[best];
+            }
             sel[row * top + k] = best;
             wt[row * top + k] = bv * inv;
             psum += bv * inv;

@@ -31,6 +31,23 @@ def test_expert_runs(n, experts, top, ff, width):
     check(N, cfg, n, 31)
 
 
+@pytest.mark.parametrize("n", [60, 150])
+def test_rows_that_are_not_numbers(n):
+    """a token whose embedding overflows: its row's scores are no numbers, yet its choices are experts (they index the row
+    lists); the other sequence does not notice"""
+    def overflow(w):
+        w["embed"][5, :] = np.inf
+    cfg = N.config([N.gla(heads=2, dim=16, vdim=16, mlp=N.moe(ff=24, experts=5, top=3))], vocab=64, width=64)
+    _, model = N.build(cfg, seed=97, dtype="bf16", tweak=overflow)
+    good = [6 + t % 58 for t in N.tokens(cfg, n, seed=98)]
+    bad = good[:n - 20] + [5] * 20
+    cache = model.new_device_cache(2, 256)
+    got = cache.forward_ragged([0, 1], [good, bad], [list(range(n)), list(range(n))])
+    alone = N.run_cut(model, good, [100, 100], cache=model.new_device_cache(1, 256))
+    assert N.relerr(got[:n], np.asarray(alone, dtype=np.float64)) < CHUNK_TOL
+    assert np.isfinite(got[n:n + min(64, n - 20)]).all()
+
+
 @pytest.mark.parametrize("n,ff", [(129, 24), (260, 136)])
 def test_expert_runs_without_a_gate(n, ff):
     check(T, T.config([T.layer(mlp=T.moe(experts=8, top=2, ff=ff))], width=64), n, 33)
