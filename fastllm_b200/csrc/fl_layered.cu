@@ -1270,7 +1270,7 @@ static bool gqa_attn_fused(fl_cache& c, LaunchCtx& lc, const GqaAttnArgs& a, int
     auto need = [&](auto& buf, size_t n) { if (buf.n < n) { FL_CUDA(cudaStreamSynchronize(c.stream)); buf.alloc(n + n / 4); } };
     need(y.at_kc, keys * dk); need(y.at_kct, keys * dv);
     const GqaTcArgs t{a.proj, a.ldp, a.off_q, r0, Ts, pos0, a.H, a.G, a.D, a.Dv, pg, a.window, a.keep_first, a.chunk, a.scale, a.softcap, a.sink, a.sinkv,
-                      a.ohi, a.olo, a.ldo, a.gate, 8.f};
+                      a.ohi, a.olo, a.ldo, a.gate, 8.f, y.at_failed.p};
     const int* page_row = y.page_table.p + (size_t)slot * c.pages_per_seq;
     if (dk == 64 && dv == 64) launch_gqa_tc<64, 64>(y, lc, a, t, page_row);
     else if (dk == 64) launch_gqa_tc<64, 128>(y, lc, a, t, page_row);
@@ -1340,6 +1340,13 @@ static void gqa_attn_tc(fl_cache& c, LaunchCtx& lc, const GqaAttnArgs& a, int r0
 static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const int* slots, const int* counts, int n, const int* h_row0,
                          const int* h_pos0);
 
+void layered_finish(fl_cache& c) {
+    FL_CUDA(cudaStreamSynchronize(c.stream));
+    if (*c.ly->at_failed.p == 0) return;
+    c.poisoned = true;
+    throw Error(FL_ERR_CUDA, "attention of a portion: a wait inside the kernel ran out, the step's results are not valid");
+}
+
 void layered_forward(fl_cache& c, const int* slots, const int* counts, int n, const uint32_t* ids, const int* want, int n_want) {
     const LayeredModel& m = *c.lm;
     LayeredCache& y = *c.ly;
@@ -1365,6 +1372,7 @@ void layered_forward(fl_cache& c, const int* slots, const int* counts, int n, co
     for (long long i = 0; i < T; ++i) FL_CHECK(ids[i] < (uint32_t)m.V, FL_ERR_INVALID, "token id out of range");
     for (int k = 0; k < n_want; ++k) FL_CHECK(want[k] >= 0 && want[k] < T, FL_ERR_INVALID, "wanted row out of range");
     ensure_ws(c, (size_t)T, (size_t)n_want);
+    if (y.at_failed.n == 0) { y.at_failed.alloc(1); *y.at_failed.p = 0; }
     const size_t tab_ints = (size_t)4 * T + 3 * (size_t)n + 1 + (size_t)n_want;
     if (tab_ints > y.tab_cap) {
         FL_CUDA(cudaStreamSynchronize(c.stream));

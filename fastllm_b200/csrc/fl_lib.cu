@@ -1810,7 +1810,7 @@ static void layered_uniform(fl_cache& c, const int* slots, const uint32_t* ids, 
         want[i] = i * t + t - 1;
     }
     layered_forward(c, sl.data(), cnt.data(), n, ids, want.data(), n);
-    FL_CUDA(cudaStreamSynchronize(c.stream));
+    layered_finish(c);
     std::memcpy(logits_host, c.ly->h_logits.p, (size_t)n * c.lm->V * 4);
 }
 
@@ -2180,7 +2180,7 @@ FL_EXPORT int fl_forward_ragged(fl_model* m, fl_cache* c, const int* slots, cons
     use_device();
     try {
         layered_forward(*c, slots, counts, n, ids, want, n_want);
-        FL_CUDA(cudaStreamSynchronize(c->stream));
+        layered_finish(*c);
         if (n_want > 0) std::memcpy(logits_host, c->ly->h_logits.p, (size_t)n_want * m->lay->V * 4);
     } catch (const fl::Error& e) {
         if (e.code == FL_ERR_CUDA) c->poisoned = true;

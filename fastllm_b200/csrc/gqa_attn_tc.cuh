@@ -23,21 +23,27 @@ __host__ __device__ constexpr size_t gqa_tc_smem(int dk, int dv) {
     return (size_t)2 * (dk / 64) * 16384 + 65536 + (size_t)kGtKStages * dk * 128 + (size_t)gqa_tc_vstages(dv) * dv * 128 + 1024;
 }
 
-// mbar_wait that gives up after some seconds: the block then ends with NaN results instead of never
+// mbar_wait that gives up after about two seconds.  A block whose wait ran out stops at one page for all its softmax threads, lets its own copies
+// and products land, frees its TMEM and leaves a mark that the host reads behind the step (GqaTcArgs.failed): the call then returns an error.
+__device__ __forceinline__ bool gt_try(uint64_t* bar, uint32_t parity) {
+    uint32_t done;
+    asm volatile(
+        "{\n"
+        ".reg .pred p;\n"
+        "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
+        "selp.u32 %0, 1, 0, p;\n"
+        "}\n"
+        : "=r"(done)
+        : "r"(smem_u32(bar)), "r"(parity)
+        : "memory");
+    return done != 0;
+}
 __device__ __forceinline__ bool gt_wait(uint64_t* bar, uint32_t parity) {
-    for (uint32_t n = 0; n < (1u << 24); ++n) {
-        uint32_t done;
-        asm volatile(
-            "{\n"
-            ".reg .pred p;\n"
-            "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n"
-            "selp.u32 %0, 1, 0, p;\n"
-            "}\n"
-            : "=r"(done)
-            : "r"(smem_u32(bar)), "r"(parity)
-            : "memory");
-        if (done) return true;
-    }
+    if (gt_try(bar, parity)) return true;
+    const long long t0 = clock64();
+    do {
+        if (gt_try(bar, parity)) return true;
+    } while (clock64() - t0 < (1ll << 32));
     return false;
 }
 
@@ -58,6 +64,7 @@ struct GqaTcArgs {
     uint16_t *ohi, *olo; int ldo;
     OutGate gate;
     float tau;
+    int* failed;                            // pinned host memory: set by a block that gave up
 };
 
 // kc [G][64 pages][DK] and vt [G][DV][64 pages] of the pages a portion reads; keys at or behind `end` and channels behind D / Dv are zero.
@@ -104,7 +111,8 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
     constexpr uint32_t kQBytes = HALF * 16384, kPOff = 2 * kQBytes, kKTile = DK * 128, kVTile = DV * 128, kKOff = kPOff + 65536, kVOff = kKOff + NK * kKTile;
     extern __shared__ __align__(1024) uint8_t gtsm_raw[];
     uint8_t* sm = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(gtsm_raw) + 1023) & ~(uintptr_t)1023);
-    __shared__ __align__(8) uint64_t k_full[NK], k_empty[NK], v_full[NV], v_empty[NV], s_full[NS], s_free[NS], p_ready[2], p_free[2], q_ready;
+    __shared__ __align__(8) uint64_t k_full[NK], k_empty[NK], v_full[NV], v_empty[NV], s_full[NS], s_free[NS], p_ready[2], p_free[2], q_ready, drained;
+    __shared__ int gave_up[2];
     __shared__ uint32_t s_tmem;
     __shared__ float xmax[2][2][kGtQ], xsum[2][kGtQ];
 
@@ -123,6 +131,8 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
         for (int i = 0; i < NS; ++i) { mbar_init(&s_full[i], 1); mbar_init(&s_free[i], 8); }
         for (int i = 0; i < 2; ++i) { mbar_init(&p_ready[i], 8); mbar_init(&p_free[i], 1); }
         mbar_init(&q_ready, 8);
+        mbar_init(&drained, 1);
+        gave_up[0] = gave_up[1] = 0;
         mbar_fence_init();
     }
     if (warp == 1) tmem_alloc(&s_tmem, 512);
@@ -137,32 +147,42 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
     if (warp == 0) {
         if (lane == 0) {
             asm volatile("fence.proxy.async;" ::: "memory");
-            for (int j = 0; j < np; ++j) {
+            int j = 0;
+            for (; j < np; ++j) {
                 const int st = j % NK, row = grp * nkp + a.pg.at(page_of(j)) * kKvPage;
                 if (!gt_wait(&k_empty[st], ((j / NK) & 1) ^ 1)) break;
                 mbar_expect_tx(&k_full[st], kKTile);
 #pragma unroll
                 for (int hf = 0; hf < HALF; ++hf) tma_load_2d(sm + kKOff + st * kKTile + hf * 8192, &tmk, hf * 64, row, &k_full[st]);
             }
+            if (j < np) {
+                for (int i = j > NK ? j - NK : 0; i < j; ++i) gt_wait(&k_full[i % NK], (i / NK) & 1);
+                *a.failed = 1;
+            }
         }
     } else if (warp == 10) {
         if (lane == 0) {
             asm volatile("fence.proxy.async;" ::: "memory");
-            for (int j = 0; j < np; ++j) {
+            int j = 0;
+            for (; j < np; ++j) {
                 const int st = j % NV;
                 if (!gt_wait(&v_empty[st], ((j / NV) & 1) ^ 1)) break;
                 mbar_expect_tx(&v_full[st], kVTile);
                 tma_load_2d(sm + kVOff + st * kVTile, &tmv, a.pg.at(page_of(j)) * kKvPage, grp * DV, &v_full[st]);
+            }
+            if (j < np) {
+                for (int i = j > NV ? j - NV : 0; i < j; ++i) gt_wait(&v_full[i % NV], (i / NV) & 1);
+                *a.failed = 1;
             }
         }
     } else if (warp == 1) {
         if (lane == 0) {
             constexpr uint32_t idesc_s = umma_idesc_bf16(128, 64), idesc_o = umma_idesc_bf16(128, DV);
             int qi = 0, pi = 0;
-            gt_wait(&q_ready, 0);
+            const bool q_ok = gt_wait(&q_ready, 0);
             tc_fence_after();
             // whichever is ready next: neither product waits for the other
-            for (uint32_t spin = 0; pi < np && spin < (1u << 27); ++spin) {
+            for (uint32_t spin = 0; q_ok && pi < np && spin < (1u << 26); ++spin) {
                 if (pi < qi && mbar_test(&p_ready[pi & 1], (pi >> 1) & 1) && mbar_test(&v_full[pi % NV], (pi / NV) & 1)) {
                     const int b = pi & 1;
                     tc_fence_after();
@@ -195,6 +215,11 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
                     ++qi;
                     spin = 0;
                 }
+            }
+            if (pi < np) {
+                umma_commit(&drained);
+                gt_wait(&drained, 0);
+                *a.failed = 1;
             }
         }
     } else {
@@ -230,7 +255,7 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
         const int w_lo = a.window > 0 ? irow - a.window + 1 : 0, c_lo = a.chunk > 0 ? irow / a.chunk * a.chunk : 0;
         float m = -INFINITY, l = 0.f;
         bool ok = true;
-        for (int j = 0; j < np && ok; ++j) {
+        for (int j = 0; j < np; ++j) {
             const int b = j & 1, sb = j % NS, key0 = page_of(j) * kKvPage + half * 32;
             ok &= gt_wait(&s_full[sb], (j / NS) & 1);
             tc_fence_after();
@@ -261,7 +286,9 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
                 }
             }
             xmax[b][half][r] = mx;
+            if (!ok) gave_up[b] = 1;
             gsync();
+            if (gave_up[b]) { ok = false; break; }       // one decision for the 256 threads (this page's word is next written behind the next page's barrier)
             mx = fmaxf(mx, xmax[b][half ^ 1][r]) * kLog2e;           // offsets and exponents in the exp2 domain
             // the offset m follows the maximum lazily (see attn_prefill_tc_kernel)
             const bool bump = mx > m + a.tau;
@@ -312,7 +339,8 @@ static __global__ void __launch_bounds__(kGtThreads, 1) ly_gqa_tc_kernel(const _
         gsync();
         float sum = l + xsum[half ^ 1][r];
         if (a.sink) sum += ex2_approx(fmaf(a.sinkv ? a.sinkv[head] : 0.f, kLog2e, -m));
-        ok &= gt_wait(&p_free[(np - 1) & 1], ((np - 1) >> 1) & 1);      // the last P.V, and with it all before
+        ok = ok && gt_wait(&p_free[(np - 1) & 1], ((np - 1) >> 1) & 1);      // the last P.V, and with it all before
+        if (!ok) *a.failed = 1;
         tc_fence_after();
         const float inv = ok ? 1.f / sum : __int_as_float(0x7FC00000);
         const int row = a.row0 + lrow;
