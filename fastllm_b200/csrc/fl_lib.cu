@@ -8,6 +8,7 @@
 #include "attn_mma.cuh"
 #include "comm.cuh"
 #include "decode_persistent.cuh"
+#include "deliver.hpp"
 #include "dense_ops.cuh"
 #include "gemm_tc.cuh"
 #include "elementwise.cuh"
@@ -1914,35 +1915,28 @@ FL_EXPORT int fl_cache_destroy(fl_cache* c) {
     FL_API_END
 }
 
-// A step's logits to the caller's buffer, through the pinned one; returns when they are there.  From 4 MB on the caller's pages are touched
-// while the device still computes (new ones cost a fault each) and the transfer goes in parts, each copied on while the next arrives.
-// 64 rows of 32000 logits behind a device step of 0.6 ms, whole call: 1.25 -> 1.15 ms (copying with helper threads: no faster here, they wake up late).
-static void deliver_logits(cudaStream_t stream, const float* dev, float* pinned, float* host, size_t n) {
-    constexpr size_t kPart = 512 * 1024;                // floats
-    constexpr int kMaxParts = 16;
-    const int parts = (int)std::min<size_t>(kMaxParts, n / kPart);
-    if (parts < 2) {
-        FL_CUDA(cudaMemcpyAsync(pinned, dev, n * 4, cudaMemcpyDeviceToHost, stream));
-        FL_CUDA(cudaStreamSynchronize(stream));
-        std::memcpy(host, pinned, n * 4);
-        return;
+// deliver_logits' device side
+struct LogitsTransfer {
+    static constexpr int kMaxParts = 16;
+    cudaStream_t stream; const float* dev; float* pinned;
+    int parts = 0;
+    cudaEvent_t e[kMaxParts] = {};
+    LogitsTransfer(cudaStream_t s, const float* d, float* p) : stream(s), dev(d), pinned(p) {}
+    LogitsTransfer(const LogitsTransfer&) = delete;
+    ~LogitsTransfer() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
+    void begin(int n) { parts = n; }
+    void fetch(int p, size_t at, size_t count) {
+        FL_CUDA(cudaMemcpyAsync(pinned + at, dev + at, count * 4, cudaMemcpyDeviceToHost, stream));
+        if (parts == 1) return;
+        FL_CUDA(cudaEventCreateWithFlags(&e[p], cudaEventDisableTiming));
+        FL_CUDA(cudaEventRecord(e[p], stream));
     }
-    struct Events {
-        cudaEvent_t e[kMaxParts] = {};
-        ~Events() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
-    } ev;
-    auto at = [&](int p) { return n * (size_t)p / parts; };
-    for (int p = 0; p < parts; ++p) {
-        FL_CUDA(cudaMemcpyAsync(pinned + at(p), dev + at(p), (at(p + 1) - at(p)) * 4, cudaMemcpyDeviceToHost, stream));
-        FL_CUDA(cudaEventCreateWithFlags(&ev.e[p], cudaEventDisableTiming));
-        FL_CUDA(cudaEventRecord(ev.e[p], stream));
-    }
-    volatile char* page = reinterpret_cast<volatile char*>(host);
-    for (size_t i = 0; i < n * 4; i += 4096) page[i] = 0;
-    for (int p = 0; p < parts; ++p) {
-        FL_CUDA(cudaEventSynchronize(ev.e[p]));
-        std::memcpy(host + at(p), pinned + at(p), (at(p + 1) - at(p)) * 4);
-    }
+    void wait(int p) { FL_CUDA(parts == 1 ? cudaStreamSynchronize(stream) : cudaEventSynchronize(e[p])); }
+    void check() { check_peer_error(); }
+};
+static void logits_to_host(fl_cache& c, float* host, size_t n) {
+    LogitsTransfer t(c.stream, c.logits.p, c.h_logits.p);
+    deliver_logits(t, c.h_logits.p, host, n);
 }
 
 FL_EXPORT int fl_forward(fl_model* m, fl_cache* c, const uint32_t* ids, int b, int t, size_t rope_offset, float* logits_host) {
@@ -1964,8 +1958,7 @@ FL_EXPORT int fl_forward(fl_model* m, fl_cache* c, const uint32_t* ids, int b, i
     try {
         run_forward(*c, ids, b, t, rope_offset);
         const size_t n = (size_t)b * c->w->Vfull;
-        deliver_logits(c->stream, c->logits.p, c->h_logits.p, logits_host, n);
-        check_peer_error();
+        logits_to_host(*c, logits_host, n);
     } catch (const fl::Error& e) {
         if (e.code == FL_ERR_CUDA || e.code == FL_ERR_NCCL) c->poisoned = true;   // a missed peer leaves kv_len / exchange epochs out of step
         throw;
@@ -2161,8 +2154,7 @@ FL_EXPORT int fl_forward_slots(fl_model* m, fl_cache* c, const int* slots, const
     try {
         run_forward_slots(*c, slots, ids, n, t, rope_offsets);
         const size_t cnt = (size_t)n * c->w->Vfull;
-        deliver_logits(c->stream, c->logits.p, c->h_logits.p, logits_host, cnt);
-        check_peer_error();
+        logits_to_host(*c, logits_host, cnt);
     } catch (const fl::Error& e) {
         if (e.code == FL_ERR_CUDA || e.code == FL_ERR_NCCL) c->poisoned = true;
         throw;

@@ -316,7 +316,8 @@ FL_EXPORT int fl_cache_destroy(fl_cache* c);
 
 /* ---- forward (causal LMs) ---------------------------------------------------------------------- */
 /* ids: host u32 [b, t] row-major.  rope_offset: RoPE position of ids[:,0] (explicit so the Mistral/Qwen2 adapter's
- * +1-per-call rule survives unchanged; the KV length is tracked inside the cache).  logits_host: f32 [b, vocab]. */
+ * +1-per-call rule survives unchanged; the KV length is tracked inside the cache).  logits_host: f32 [b, vocab], written once the
+ * step is known to be good: a call that fails before that leaves it as it was. */
 FL_EXPORT int fl_forward(fl_model* m, fl_cache* c, const uint32_t* ids, int b, int t, size_t rope_offset, float* logits_host);
 /* Same forward, arg-max on device (last index wins ties); next_ids: host u32 [b]. */
 FL_EXPORT int fl_forward_greedy(fl_model* m, fl_cache* c, const uint32_t* ids, int b, int t, size_t rope_offset, uint32_t* next_ids);
