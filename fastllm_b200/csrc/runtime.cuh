@@ -105,10 +105,13 @@ struct DevBuf {
     ~DevBuf() { release(); }
     void alloc(size_t count, bool zero = false) {
         release();
-        n = count;
         if (count == 0) return;
         FL_CUDA(cudaMalloc(&p, count * sizeof(T)));
-        if (zero) FL_CUDA(cudaMemset(p, 0, count * sizeof(T)));
+        if (zero) {                             // the streams of models and caches do not wait for the default one
+            FL_CUDA(cudaMemset(p, 0, count * sizeof(T)));
+            FL_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+        }
+        n = count;
     }
     void release() {
         if (p) cudaFree(p);
