@@ -829,6 +829,50 @@ static void drop_graphs(fl_cache& c) {
     c.graphs.clear();
 }
 
+// The first matrix of a gated feed-forward and its activation, as the hi | lo halves the second one reads.  More than 128 rows whose
+// tiles fill the chip take the activation in the GEMM's epilogue: the [rows, 2 F] f32 result (235 MB at 2048 rows of F = 14336) is neither
+// written nor read back (three such layers of width 4096, whole prefill: 8.29 -> 8.07 ms).  Few tiles keep the GEMM that cuts K; the
+// epilogue cannot see a sum in slices.
+static bool ff_in_fused(int R, int F, int K, int act, bool tc_in, bool tc_out, bool f32) {
+    const int tiles = (R + 127) / 128 * ((F + 127) / 128);
+    return tc_in && tc_out && !f32 && R > 128 && act != FL_ACT_RELU2 && F % 8 == 0 && (2 * tiles > kNumSMs || (K + 63) / 64 < 16);
+}
+// f32 scratch of the feed-forwards in steps of up to R rows, in floats: only the rows whose path leaves gate | up, the activation or the
+// experts' results there (run_rows: the experts' runs in a step of more than 128 rows).
+// A new cache's first step of 2048 rows through three 4096 x 14336 layers takes 937 instead of 1694 MB and, with the scratch of its portions
+// reserved up front (reserve_portions), 15.1 instead of 16.9 ms.
+struct FfScratch { size_t gu = 0, act = 0, eo = 0, sh_gu = 0, sh_act = 0, sh_o = 0; };
+static FfScratch ff_scratch(const LayeredModel& m, size_t R, size_t run_rows) {
+    FfScratch s;
+    const size_t W = m.W;
+    auto up = [](size_t& a, size_t b) { a = std::max(a, b); };
+    // rows of the largest step up to R whose gate | up is not fused: a step of fewer rows has fewer tiles
+    auto unfused = [&](int F, int act, bool tc_in, bool tc_out) {
+        size_t r = R;
+        while (r > 128 && ff_in_fused((int)r, F, m.W, act, tc_in, tc_out, m.f32)) r = (r - 1) / 128 * 128;
+        return r;
+    };
+    for (const LayeredLayerW& lw : m.layers) {
+        const fl_layer_desc& d = lw.d;
+        const size_t F = d.ff, GF = d.ffn_act == FL_ACT_RELU2 ? F : 2 * F, Fs = d.shared_ff;
+        if (d.ffn == FL_FFN_DENSE) {
+            up(s.gu, unfused(d.ff, d.ffn_act, lw.tc_gu, lw.tc_down) * GF);
+            if (!lw.tc_down) up(s.act, R * F);
+        } else if (d.ffn == FL_FFN_MOE) {
+            const size_t P = R * d.top;
+            if (!lw.tc_moe) { up(s.gu, P * GF); up(s.act, P * F); up(s.eo, P * W); }
+            else { up(s.eo, run_rows * W); if (d.ffn_act == FL_ACT_RELU2) up(s.gu, run_rows * F); }
+            if (d.shared_ff > 0 && !m.cfg.parallel_sub) {
+                up(s.sh_gu, unfused(d.shared_ff, d.ffn_act, lw.tc_sgu, lw.tc_sdown) * 2 * Fs);
+                if (!lw.tc_sdown) up(s.sh_act, R * Fs);
+                up(s.sh_o, R * W);
+            }
+        }
+    }
+    return s;
+}
+
+
 static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
     const LayeredModel& m = *c.lm;
     LayeredCache& y = *c.ly;
@@ -857,9 +901,8 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
             y.qp_hi.alloc(R * m.max_hp); y.qp_lo.alloc(R * m.max_hp); y.qo_hi.alloc(R * m.max_hq); y.qo_lo.alloc(R * m.max_hq);
             y.ol_hi.alloc(R * m.max_hc); y.ol_lo.alloc(R * m.max_hc);
         }
-        y.gu.alloc(std::max(P * 2, run_rows) * std::max(m.max_ff, 1));     // (run_rows: experts without a gate)
-        y.act.alloc(P * std::max(m.max_ff, 1)); y.eo.alloc(std::max(P, run_rows) * W);
-        y.sh_gu.alloc(R * 2 * std::max(m.max_ff, 1)); y.sh_act.alloc(R * std::max(m.max_ff, 1)); y.sh_o.alloc(R * W);
+        const FfScratch ff = ff_scratch(m, R, run_rows);
+        y.gu.alloc(ff.gu); y.act.alloc(ff.act); y.eo.alloc(ff.eo); y.sh_gu.alloc(ff.sh_gu); y.sh_act.alloc(ff.sh_act); y.sh_o.alloc(ff.sh_o);
         y.route_w.alloc(P); y.route_sel.alloc(P); y.sgate.alloc(R);
         y.pair_row.alloc(P); y.pair_of.alloc(P); y.grp_off.alloc((size_t)m.max_experts + 2); y.tile_off.alloc((size_t)m.max_experts + 2);
         if (!m.f32) {
@@ -883,10 +926,10 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
             }
             if (y.gemm_out.n < need) y.gemm_out.alloc(need);
             if (gx_rows > 0) gx_rows = std::max(gx_rows, run_rows);
-            if (y.gx_hi.n < gx_rows * W) {
-                y.gx_hi.alloc(gx_rows * W, true); y.gx_lo.alloc(gx_rows * W, true);
-                y.ga_hi.alloc(gx_rows * std::max(m.max_ff, 1), true); y.ga_lo.alloc(gx_rows * std::max(m.max_ff, 1), true);
-                y.grp_cnt.alloc((size_t)m.max_experts + 1, true);
+            if (y.gx_hi.n < gx_rows * W) {      // (not cleared: what a row behind an expert's list holds reaches that row's products alone, and nobody reads those)
+                y.gx_hi.alloc(gx_rows * W); y.gx_lo.alloc(gx_rows * W);
+                y.ga_hi.alloc(gx_rows * std::max(m.max_ff, 1)); y.ga_lo.alloc(gx_rows * std::max(m.max_ff, 1));
+                y.grp_cnt.alloc((size_t)m.max_experts + 1);
             }
         }
         y.rows = R;
@@ -965,15 +1008,6 @@ static void launch_glu(LaunchCtx& lc, const Slices& gu, int rows, int F, float l
         launch(lc, "glu", 0, ly_glu_kernel<4>, dim3(rows, (F + 1023) / 1024), dim3(256), 0, gu, ldg, ldo, F, limit, act, bias, out, hi, lo);
     else
         launch(lc, "glu", 0, ly_glu_kernel<1>, dim3(rows, (F + 255) / 256), dim3(256), 0, gu, ldg, ldo, F, limit, act, bias, out, hi, lo);
-}
-
-// The first matrix of a gated feed-forward and its activation, as the hi | lo halves the second one reads.  More than 128 rows whose
-// tiles fill the chip take the activation in the GEMM's epilogue: the [rows, 2 F] f32 result (235 MB at 2048 rows of F = 14336) is neither
-// written nor read back (three such layers of width 4096, whole prefill: 8.29 -> 8.07 ms).  Few tiles keep the GEMM that cuts K; the
-// epilogue cannot see a sum in slices.
-static bool ff_in_fused(int R, int F, int K, int act, bool tc_in, bool tc_out, const uint16_t* hhi) {
-    const int tiles = (R + 127) / 128 * ((F + 127) / 128);
-    return tc_in && tc_out && hhi != nullptr && R > 128 && act != FL_ACT_RELU2 && F % 8 == 0 && (2 * tiles > kNumSMs || (K + 63) / 64 < 16);
 }
 
 static void gemm_groups(LaunchCtx& lc, const char* tag, const LyGemm& g, int groups, int max_rows) {
@@ -1095,8 +1129,27 @@ static bool chunks_fit(const ChunkArgs& a, bool f32, const int* counts, int n) {
         if (counts[i] >= kCsMinTokens) return true;
     return false;
 }
+// How a step's long portions go through the chunked kernels: `span` chunks of each at a time, `most` chunks in the longest, states of `held` chunks.
+struct ChunkPlan { int span = 0, most = 0; size_t held = 0; };
+static ChunkPlan chunk_plan(const int* counts, int n) {
+    ChunkPlan p;
+    int longs = 0;
+    for (int i = 0; i < n; ++i)
+        if (counts[i] >= kCsMinTokens) { ++longs; p.most = std::max(p.most, (counts[i] + kCsC - 1) / kCsC); }
+    if (longs == 0) return p;
+    p.span = std::max(1, kCsChunks / longs);
+    p.held = (size_t)std::min(p.span, p.most) * longs;
+    return p;
+}
+struct ChunkScratch { size_t us = 0, dec = 0, qd = 0, aq = 0, wk = 0; };        // floats of the cs_ buffers
+static ChunkScratch chunk_scratch(Recurrence kind, int H, int D, int Dv, const ChunkPlan& p, size_t rows) {
+    ChunkScratch s{p.held * H * D * Dv, p.held * H * (kind == Recurrence::gla ? D : 1)};
+    if (kind == Recurrence::gla) s.qd = rows * H * D;
+    if (kind == Recurrence::delta) { s.aq = p.held * H * kCsC * kCsC; s.wk = p.held * H * kCsC * D; }
+    return s;
+}
 template <int DP>
-static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurrence kind, const int* counts, int n, cudaStream_t stream) {
+static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurrence kind, const int* counts, int n) {
     constexpr size_t row = DP + kCsPad, tile = kCsC * row, sq = kCsC * kCsLdA;
     constexpr size_t sm_in = (2 * tile + sq) * 4, sm_gla = (3 * tile + sq + kCsC / 16 * DP) * 4, sm_delta = (2 * tile + 2 * sq) * 4;
     constexpr size_t sm_dstate = (DP * (kCsCols + kCsPad) + 2 * (2 * tile + kCsC * (kCsCols + kCsPad) + kCsC)) * 4;
@@ -1109,16 +1162,14 @@ static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurr
         room(ly_chunk_out_kernel<DP, 0>, sm_out); room(ly_chunk_out_kernel<DP, 1>, sm_out); room(ly_chunk_out_kernel<DP, 2>, sm_out2);
         attr_set = true;
     }
-    int longs = 0, most = 0;
-    for (int i = 0; i < n; ++i)
-        if (counts[i] >= kCsMinTokens) { ++longs; most = std::max(most, (counts[i] + kCsC - 1) / kCsC); }
-    a.span = std::max(1, kCsChunks / longs);
-    const size_t held = (size_t)std::min(a.span, most) * longs, per = (size_t)a.H * a.D * a.Dv;
-    auto need = [&](auto& buf, size_t k) { if (buf.n < k) { FL_CUDA(cudaStreamSynchronize(stream)); buf.alloc(k); } };
-    need(y.cs_us, held * per); need(y.cs_dec, held * a.H * (kind == Recurrence::gla ? a.D : 1));
-    a.us = y.cs_us.p; a.dec = y.cs_dec.p;
-    if (kind == Recurrence::gla) { need(y.cs_qd, y.rows * a.H * a.D); a.qd = y.cs_qd.p; }
-    if (kind == Recurrence::delta) { need(y.cs_aq, held * a.H * kCsC * kCsC); need(y.cs_wk, held * a.H * kCsC * a.D); a.aq = y.cs_aq.p; a.wk = y.cs_wk.p; }
+    const ChunkPlan pl = chunk_plan(counts, n);
+    const ChunkScratch need = chunk_scratch(kind, a.H, a.D, a.Dv, pl, y.rows);
+    FL_CHECK(y.cs_us.n >= need.us && y.cs_dec.n >= need.dec && y.cs_qd.n >= need.qd && y.cs_aq.n >= need.aq && y.cs_wk.n >= need.wk, FL_ERR_STATE,
+             "internal: scratch of the chunked recurrences too small");
+    a.us = y.cs_us.p; a.dec = y.cs_dec.p; a.qd = y.cs_qd.p; a.aq = y.cs_aq.p; a.wk = y.cs_wk.p;
+    a.span = pl.span;
+    const int most = pl.most;
+    const size_t per = (size_t)a.H * a.D * a.Dv;
     for (a.span0 = 0; a.span0 < most; a.span0 += a.span) {
         int chunks = 0;
         for (int i = 0; i < n; ++i)
@@ -1141,8 +1192,8 @@ static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurr
 }
 // -> whether the token-serial kernel has sequences left
 static bool launch_chunks(fl_cache& c, LaunchCtx& lc, const ChunkArgs& a, Recurrence kind, const int* counts, int n) {
-    if (a.D <= 64) launch_chunks_dp<64>(*c.ly, lc, a, kind, counts, n, c.stream);
-    else launch_chunks_dp<128>(*c.ly, lc, a, kind, counts, n, c.stream);
+    if (a.D <= 64) launch_chunks_dp<64>(*c.ly, lc, a, kind, counts, n);
+    else launch_chunks_dp<128>(*c.ly, lc, a, kind, counts, n);
     for (int i = 0; i < n; ++i)
         if (counts[i] < kCsMinTokens) return true;
     return false;
@@ -1243,7 +1294,7 @@ static void latent_attn_tc(fl_cache& c, LaunchCtx& lc, const LatentAttnArgs& a, 
 }
 
 // Grouped-query attention of rows [r0, r0 + Ts) -- one sequence's portion, positions pos0.. -- in one kernel (gqa_attn_tc.cuh): heads of up
-// to 128 channels whose results go to the output projection as halves.  -> false: this shape is gqa_attn_tc's
+// to 128 channels whose results go to the output projection as halves (gqa_fusable; other shapes are gqa_attn_tc's).
 template <int DK, int DV>
 static void launch_gqa_tc(LayeredCache& y, LaunchCtx& lc, const GqaAttnArgs& a, GqaTcArgs t, const int* page_row) {
     static bool attr_set = false;
@@ -1257,18 +1308,24 @@ static void launch_gqa_tc(LayeredCache& y, LaunchCtx& lc, const GqaAttnArgs& a, 
     const CUtensorMap tk = make_tmap_bf16(y.at_kc.p, a.G * nkp, DK, DK, kKvPage), tv = make_tmap_bf16(y.at_kct.p, (uint64_t)a.G * DV, nkp, nkp, DV);
     launch(lc, "gqa_attn_tc", 0, ly_gqa_tc_kernel<DK, DV>, dim3((t.Ts + kGtQ - 1) / kGtQ, a.H), dim3(kGtThreads), gqa_tc_smem(DK, DV), tk, tv, t);
 }
-static bool gqa_attn_fused(fl_cache& c, LaunchCtx& lc, const GqaAttnArgs& a, int r0, int Ts, int pos0, int slot) {
-    if (a.D > 128 || a.Dv > 128 || ((a.D | a.Dv | a.ldo) & 7) != 0 || ((a.ldp | a.off_q) & 3) != 0 || a.ohi == nullptr) return false;
-    LayeredCache& y = *c.ly;
-    const int lo = std::max(a.window > 0 ? std::max(pos0 - a.window + 1, 0) : 0, a.chunk > 0 ? pos0 / a.chunk * a.chunk : 0);
+static bool gqa_fusable(const LayeredLayerW& lw, bool f32) {
+    const fl_layer_desc& d = lw.d;
+    return !f32 && lw.tc_o && d.dim <= 128 && d.vdim <= 128 && ((d.dim | d.vdim | lw.u_ld) & 7) == 0 && ((lw.n_in | lw.off_q) & 3) == 0;
+}
+static GqaPages gqa_pages(int window, int keep_first, int chunk, int pos0, int Ts) {
+    const int lo = std::max(window > 0 ? std::max(pos0 - window + 1, 0) : 0, chunk > 0 ? pos0 / chunk * chunk : 0);
     GqaPages pg;
     pg.base = lo / kKvPage;
-    pg.first = (a.window > 0 && a.keep_first > 0) ? std::min((a.keep_first + kKvPage - 1) / kKvPage, pg.base) : 0;
+    pg.first = (window > 0 && keep_first > 0) ? std::min((keep_first + kKvPage - 1) / kKvPage, pg.base) : 0;
     pg.pages = pg.first + (pos0 + Ts - 1) / kKvPage - pg.base + 1;
+    return pg;
+}
+static void gqa_attn_fused(fl_cache& c, LaunchCtx& lc, const GqaAttnArgs& a, int r0, int Ts, int pos0, int slot) {
+    LayeredCache& y = *c.ly;
+    const GqaPages pg = gqa_pages(a.window, a.keep_first, a.chunk, pos0, Ts);
     const int dk = a.D <= 64 ? 64 : 128, dv = a.Dv <= 64 ? 64 : 128;
     const size_t keys = (size_t)a.G * pg.pages * kKvPage;
-    auto need = [&](auto& buf, size_t n) { if (buf.n < n) { FL_CUDA(cudaStreamSynchronize(c.stream)); buf.alloc(n + n / 4); } };
-    need(y.at_kc, keys * dk); need(y.at_kct, keys * dv);
+    FL_CHECK(y.at_kc.n >= keys * dk && y.at_kct.n >= keys * dv, FL_ERR_STATE, "internal: scratch of the fused attention too small");
     const GqaTcArgs t{a.proj, a.ldp, a.off_q, r0, Ts, pos0, a.H, a.G, a.D, a.Dv, pg, a.window, a.keep_first, a.chunk, a.scale, a.softcap, a.sink, a.sinkv,
                       a.ohi, a.olo, a.ldo, a.gate, 8.f, y.at_failed.p};
     const int* page_row = y.page_table.p + (size_t)slot * c.pages_per_seq;
@@ -1276,7 +1333,6 @@ static bool gqa_attn_fused(fl_cache& c, LaunchCtx& lc, const GqaAttnArgs& a, int
     else if (dk == 64) launch_gqa_tc<64, 128>(y, lc, a, t, page_row);
     else if (dv == 64) launch_gqa_tc<128, 64>(y, lc, a, t, page_row);
     else launch_gqa_tc<128, 128>(y, lc, a, t, page_row);
-    return true;
 }
 
 // Grouped-query attention of rows [r0, r0 + Ts) -- one sequence's portion, positions pos0.. -- on the tensor-core GEMM: per block of
@@ -1340,6 +1396,49 @@ static void gqa_attn_tc(fl_cache& c, LaunchCtx& lc, const GqaAttnArgs& a, int r0
 static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const int* slots, const int* counts, int n, const int* h_row0,
                          const int* h_pos0);
 
+// Long portions (serving precision) run their scores and weighted sums on the tensor cores; decoded tokens, short portions and the exact mode
+// on the per-(row, head) kernel, and so do masks that leave a row few keys: that kernel reads just those.
+static bool gqa_portion_tc(const LayeredModel& m, const fl_layer_desc& d, int Ts) {
+    static const bool off = env_flag("FL_LAYERED_NO_TC_ATTN");
+    const bool few_keys = (d.window > 0 && d.window + d.keep_first <= 256) || (d.mask_chunk > 0 && d.mask_chunk <= 256);
+    return !(m.f32 || off || few_keys || d.vdim % 8 != 0 || Ts < 64 || (long long)Ts * (d.heads / d.kv_heads) <= 128);
+}
+// Scratch that depends on how long this step's portions are, taken before its first launch: growing it between launches would wait for the
+// device and allocate while it idles.
+static void reserve_portions(fl_cache& c, const int* slots, const int* counts, int n) {
+    const LayeredModel& m = *c.lm;
+    LayeredCache& y = *c.ly;
+    if (m.f32) return;
+    const ChunkPlan pl = chunk_plan(counts, n);
+    ChunkScratch cs;
+    size_t kc = 0, kct = 0;
+    auto up = [](size_t& a, size_t b) { a = std::max(a, b); };
+    auto mixer = [&](const LayeredLayerW& lw) {
+        const fl_layer_desc& d = lw.d;
+        if (d.mixer == FL_MIXER_ATTN) {
+            if (!gqa_fusable(lw, m.f32)) return;
+            for (int i = 0; i < n; ++i) {
+                if (!gqa_portion_tc(m, d, counts[i])) continue;
+                const size_t keys = (size_t)d.kv_heads * kKvPage * gqa_pages(d.window, d.keep_first, d.mask_chunk, c.slot_len[slots[i]], counts[i]).pages;
+                up(kc, keys * (d.dim <= 64 ? 64 : 128)); up(kct, keys * (d.vdim <= 64 ? 64 : 128));
+            }
+        } else if (d.mixer == FL_MIXER_GLA || d.mixer == FL_MIXER_DELTA || d.mixer == FL_MIXER_MAMBA2 || d.mixer == FL_MIXER_LIGHTNING) {
+            const int D = d.mixer == FL_MIXER_MAMBA2 ? d.state : d.dim;
+            if (pl.held == 0 || D > 128) return;
+            const Recurrence kind = d.mixer == FL_MIXER_GLA ? Recurrence::gla : (d.mixer == FL_MIXER_DELTA ? Recurrence::delta : Recurrence::scalar);
+            const ChunkScratch s = chunk_scratch(kind, d.heads, D, d.vdim, pl, y.rows);
+            up(cs.us, s.us); up(cs.dec, s.dec); up(cs.qd, s.qd); up(cs.aq, s.aq); up(cs.wk, s.wk);
+        }
+    };
+    for (const LayeredLayerW& lw : m.layers) {
+        mixer(lw);
+        if (lw.side) mixer(*lw.side);
+    }
+    auto need = [&](auto& buf, size_t k, size_t spare) { if (buf.n < k) { FL_CUDA(cudaStreamSynchronize(c.stream)); buf.alloc(k + spare); } };
+    need(y.cs_us, cs.us, 0); need(y.cs_dec, cs.dec, 0); need(y.cs_qd, cs.qd, 0); need(y.cs_aq, cs.aq, 0); need(y.cs_wk, cs.wk, 0);
+    need(y.at_kc, kc, kc / 4); need(y.at_kct, kct, kct / 4);
+}
+
 void layered_finish(fl_cache& c) {
     FL_CUDA(cudaStreamSynchronize(c.stream));
     if (*c.ly->at_failed.p == 0) return;
@@ -1372,6 +1471,7 @@ void layered_forward(fl_cache& c, const int* slots, const int* counts, int n, co
     for (long long i = 0; i < T; ++i) FL_CHECK(ids[i] < (uint32_t)m.V, FL_ERR_INVALID, "token id out of range");
     for (int k = 0; k < n_want; ++k) FL_CHECK(want[k] >= 0 && want[k] < T, FL_ERR_INVALID, "wanted row out of range");
     ensure_ws(c, (size_t)T, (size_t)n_want);
+    reserve_portions(c, slots, counts, n);
     if (y.at_failed.n == 0) { y.at_failed.alloc(1); *y.at_failed.p = 0; }
     const size_t tab_ints = (size_t)4 * T + 3 * (size_t)n + 1 + (size_t)n_want;
     if (tab_ints > y.tab_cap) {
@@ -1496,20 +1596,16 @@ static void run_mixer(fl_cache& c, LaunchCtx& lc, const StepTab& st, const Layer
         }
         if (d.window > 0) max_keys = std::min(max_keys, d.window + d.keep_first);
         if (d.mask_chunk > 0) max_keys = std::min(max_keys, d.mask_chunk);
-        // masks that leave a row few keys: the per-row kernel reads just those, the GEMM path would compute a block's whole rectangle
-        const bool few_keys = (d.window > 0 && d.window + d.keep_first <= 256) || (d.mask_chunk > 0 && d.mask_chunk <= 256);
-        // long portions (serving precision): scores and weighted sums as tensor-core GEMMs; decoded tokens, short portions and
-        // the exact mode on the per-(row, head) kernel.  Rows are taken in order.
-        static const bool tc_attn_off = env_flag("FL_LAYERED_NO_TC_ATTN");
-        int done = 0;
+        int done = 0;           // rows are taken in order
         for (int si = 0; si < n; ++si) {
             const int r0 = h_row0[si], Ts = counts[si];
-            if (m.f32 || tc_attn_off || few_keys || Dv % 8 != 0 || Ts < 64 || (long long)Ts * (H / G) <= 128) continue;
+            if (!gqa_portion_tc(m, d, Ts)) continue;
             if (r0 > done) {
                 at.row_base = done;
                 launch_gqa_attn<uint16_t>(lc, at, r0 - done, max_keys, true);
             }
-            if (!gqa_attn_fused(c, lc, at, r0, Ts, h_pos0[si], slots[si])) gqa_attn_tc(c, lc, at, r0, Ts, h_pos0[si], slots[si]);
+            if (gqa_fusable(lw, m.f32)) gqa_attn_fused(c, lc, at, r0, Ts, h_pos0[si], slots[si]);
+            else gqa_attn_tc(c, lc, at, r0, Ts, h_pos0[si], slots[si]);
             done = r0 + Ts;
         }
         if (done < Ti) {
@@ -1768,6 +1864,7 @@ static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const in
                    s.stride, y.y.p);
         s = Slices{y.y.p, 1, 0};
     };
+    auto room = [](const auto& buf, size_t floats) { FL_CHECK(buf.n >= floats, FL_ERR_STATE, "internal: feed-forward scratch too small"); };
     // the experts of a layer over all rows: out[row] = sum of the chosen ones' weighted outputs (+ the shared one)
     auto experts = [&](const LayeredLayerW& lw, float* out) {
         const fl_layer_desc& d = lw.d;
@@ -1790,12 +1887,14 @@ static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const in
         const float* sh = nullptr;
         if (d.shared_ff > 0 && !par) {  // the always-on expert first (parallel sublayers hold it in the mixer's matrices): its split-K scratch is free again before the routed experts run
             const int Fs = d.shared_ff;
-            if (ff_in_fused(Ti, Fs, W, act, lw.tc_sgu, lw.tc_sdown, hhi)) {
+            if (ff_in_fused(Ti, Fs, W, act, lw.tc_sgu, lw.tc_sdown, m.f32)) {
                 dense_gemm_glu(c, lc, "gemm_shared_in", Ti, Fs, W, lw.tm_sgu, hhi, hlo, nullptr, act, d.shared_limit, ahi, alo);
             } else {
+                room(y.sh_gu, (size_t)Ti * 2 * Fs); room(y.sh_act, lw.tc_sdown ? 0 : (size_t)Ti * Fs);
                 const Slices gu = gemm_slices(c, lc, "gemm_shared_in", sub_in, hhi, hlo, lw.s_gu, lw.tm_sgu, lw.tc_sgu, 2 * Fs, W, y.sh_gu.p, Ti);
                 launch_glu(lc, gu, Ti, Fs, d.shared_limit, act, nullptr, lw.tc_sdown ? (float*)nullptr : y.sh_act.p, lw.tc_sdown ? ahi : (uint16_t*)nullptr, alo);
             }
+            room(y.sh_o, (size_t)Ti * W);
             gemm_tc_or_exact(c, lc, "gemm_shared_out", y.sh_act.p, ahi, alo, lw.s_down, lw.tm_sdown, lw.tc_sdown, W, Fs, y.sh_o.p, Ti);
             sh = y.sh_o.p;
         }
@@ -1814,6 +1913,7 @@ static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const in
             // whole prefill; 340 rows of 2816-wide experts: 2.37 -> 1.41 ms.)
             const size_t cap = 128 * ((size_t)P / 128 + std::min(P, E));
             const RowRuns runs{E, y.tile_off.p};
+            room(y.eo, cap * W); room(y.gu, act == FL_ACT_RELU2 ? cap * F : 0); room(y.gx_lo, cap * W); room(y.ga_lo, cap * F);
             launch(lc, "moe_lists", 0, ly_moe_lists_kernel, dim3(E), dim3(256), 0, (const int*)y.route_sel.p, Ti, top, E, y.grp_off.p, y.pair_row.p,
                    y.pair_of.p);
             launch(lc, "moe_gather", 0, ly_moe_gather_runs_kernel, dim3(P), dim3(256), 0, (const uint16_t*)hhi, (const uint16_t*)hlo, W, (const int*)y.route_sel.p, top, E,
@@ -1845,6 +1945,7 @@ static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const in
                        (const int*)y.route_sel.p, (const int*)y.pair_of.p, (const int*)y.grp_off.p, cap, (const float*)y.route_w.p, top, sh,
                        sg, W, out);
             } else {
+                room(y.gu, (size_t)P * GF); room(y.act, (size_t)P * F); room(y.eo, (size_t)P * W);
                 LyGemm g1{sub_in, 0, W, y.pair_row.p, lw.w_gu, (long long)GF * W, GF, W, y.gu.p, 0, GF, y.grp_off.p, P};
                 gemm_groups(lc, "gemm_moe_in", g1, E, P);
                 launch_glu(lc, Slices{y.gu.p, 1, 0}, P, F, d.limit, act, nullptr, y.act.p, nullptr, nullptr);
@@ -1928,9 +2029,10 @@ static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const in
         sublayer_front(lw, run, 1);
         const int F = d.ff, act = d.ffn_act, GF = act == FL_ACT_RELU2 ? F : 2 * F;
         if (d.ffn == FL_FFN_DENSE) {
-            if (ff_in_fused(Ti, F, W, act, lw.tc_gu, lw.tc_down, hhi)) {
+            if (ff_in_fused(Ti, F, W, act, lw.tc_gu, lw.tc_down, m.f32)) {
                 dense_gemm_glu(c, lc, "gemm_ff_in", Ti, F, W, lw.tm_gu, hhi, hlo, lw.b_gu, act, d.limit, ahi, alo);
             } else {
+                room(y.gu, (size_t)Ti * GF); room(y.act, lw.tc_down ? 0 : (size_t)Ti * F);
                 const Slices gu = gemm_slices(c, lc, "gemm_ff_in", sub_in, hhi, hlo, lw.w_gu, lw.tm_gu, lw.tc_gu, GF, W, y.gu.p, Ti);
                 launch_glu(lc, gu, Ti, F, d.limit, act, lw.b_gu, lw.tc_down ? (float*)nullptr : y.act.p, lw.tc_down ? ahi : (uint16_t*)nullptr, alo);
             }

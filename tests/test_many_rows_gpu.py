@@ -194,3 +194,20 @@ def test_attention_scale_of_any_sign(scale, softcap):
     """a scale of zero or below: masked scores stay masked, the maximum is that of the scaled scores"""
     both_ways(R, R.config([R.att(heads=2, kv_heads=1, dim=32, vdim=32, rot_dims=8, scale=scale, softcap=softcap)], width=64), 200, [130, 64], 73)
     both_ways(M, M.config([M.par_layer(M.windowed(dim=16, vdim=16, window=257, keep=2, scale=scale), M.lightning(heads=2, dim=8, vdim=8))], width=64), 400, [70, 201, 100], 74)
+
+
+# ---- workspace: only what a step's path reads, grown between steps -----------------------------------------------------------------------------
+@pytest.mark.parametrize("mod,cfg", [
+    (N, N.config([N.gla(heads=2, dim=16, vdim=16, mlp=N.moe(ff=136, experts=5, top=2)), N.lat(mlp=N.dense(ff=1040))], vocab=64, width=64)),
+    (N, N.config([N.gla(heads=2, dim=16, vdim=16, mlp=N.dense(ff=30)), N.gla(heads=2, dim=16, vdim=16, mlp=N.moe(ff=20, experts=5, top=2, shared=(30, 0.75)))], vocab=64, width=66)),
+    (R, R.config([R.att(heads=4, kv_heads=2, dim=16, vdim=16, rot_dims=8, mlp=R.dense(ff=520)), R.delta(heads=4, kv_heads=2, dim=32, vdim=24, conv=4)], vocab=64, width=1024)),
+    (T, T.config([T.layer(mlp=T.moe(experts=8, top=2, ff=136))], width=64, max_positions=1024))])
+def test_steps_that_grow(mod, cfg):
+    """a cache whose steps grow from one row to hundreds gives what a new one gives"""
+    _, model = mod.build(cfg, seed=99, dtype="bf16")
+    toks = mod.tokens(cfg, 700, seed=100)
+    cache = model.new_device_cache(1, 1024)
+    for n in (1, 40, 129, 300, 129, 700):
+        cache.slot_reset(0)
+        want = model.new_device_cache(1, 1024).forward_ragged([0], [toks[:n]], [[0, n - 1]])
+        assert mod.relerr(cache.forward_ragged([0], [toks[:n]], [[0, n - 1]]), np.asarray(want, dtype=np.float64)) < CHUNK_TOL
