@@ -10,8 +10,8 @@
 // tcgen05.mma takes them (mma.sync m16n8k16 sums the same 16 products to the same bits, in whatever order they stand inside the 16), so K is
 // not split over warps; attention, roundings and the order of every other sum are those of bert.cuh.
 // Bound: latency -- 5 phases x 6 layers of about 6 us (cluster barrier, L2 round trips of activations and weights, a chain of 24 to 96 MMAs).
-// One sentence of 19 tokens, whole call: 262 us as 44 launches, 180 us here.  (Four warps to a quarter of K each took 162, but their sums are
-// not the chain's, and 16-bit activations carry that to 3e-3 in the embedding.)
+// One sentence of 4 / 19 / 48 / 64 tokens, whole call: 243 / 254 / 268 / 277 us as 44 launches, 120 / 160 / 224 / 269 us here.  (K in quarters over
+// the warps is no faster, and its sums are not the chain's: 16-bit activations carry that to 3e-3 in the embedding.)
 #pragma once
 #include "bert.cuh"
 #include "gemm_tc.cuh"
@@ -43,11 +43,12 @@ struct BsSmem {
     static constexpr int NQ = 3 * kBsH / 8 / CL, NO = kBsH / 8 / CL, NI = kBsI / 8 / CL;        // column tiles per block of the three widths
     static_assert(NQ * CL * 8 == 3 * kBsH && NO * CL * 8 == kBsH && NI * CL * 8 == kBsI, "whole tiles per block");
     static constexpr int NV = 4 * kBsH + (NQ + 2 * NO + NI) * 8;
-    static constexpr int kPieces = MT <= 2 ? 1 : MT - 1;                                         // h arrives in so many pieces of its columns
-    static constexpr int kHPiece = kBsI / kPieces;
+    // h arrives whole, or (rows that would not fit) in pieces of its columns, one multiplied while the next is on its way
+    static constexpr int kHPiece = MT <= 2 ? kBsI : (MT == 3 ? kBsI / 4 : kBsI / 6), kPieces = kBsI / kHPiece, kHBufs = kPieces > 1 ? 2 : 1;
+    static constexpr int kHBuf = MT * 16 * bs_ld(kHPiece);                                       // elements
     static constexpr size_t max2(size_t a, size_t b) { return a > b ? a : b; }
     static constexpr size_t kX = (size_t)2 * NV * 4, kWo = kX + (size_t)MT * 16 * bs_ld(kBsH) * 2, kR = kWo + (size_t)NO * 8 * bs_ld(kBsI) * 2;
-    static constexpr size_t kBytes = kR + max2((size_t)(NQ > NI ? NQ : NI) * 8 * bs_ld(kBsH) * 2, max2((size_t)MT * 16 * bs_ld(kBsH) * 2, (size_t)MT * 16 * bs_ld(kHPiece) * 2));
+    static constexpr size_t kBytes = kR + max2((size_t)(NQ > NI ? NQ : NI) * 8 * bs_ld(kBsH) * 2, max2((size_t)MT * 16 * bs_ld(kBsH) * 2, (size_t)kHBufs * kHBuf * 2));
     static_assert(kHPiece % 32 == 0 && kX % 16 == 0 && kBytes <= 232448, "");
 };
 
@@ -83,7 +84,7 @@ struct BsTiles {
     template <int KP>
     __device__ __forceinline__ void add(const uint16_t* A, const uint16_t* W, int ldw, int k0, int warp, int lane) {
         const int g = lane >> 2, q = lane & 3;
-#pragma unroll 4
+#pragma unroll 12
         for (int s = 0; s < KP / 32; ++s)
 #pragma unroll
             for (int i = 0; i < IT; ++i) {
@@ -348,14 +349,16 @@ static __global__ void __launch_bounds__(kBsThreads, 1) bert_small_kernel(const 
         {
             BsTiles<MT, NO> y;
             y.zero();
+            bs_bring_rows<M::kHPiece>(sr, hb, kBsI, 0, rows);
+            cp_async_commit();
 #pragma unroll 1
             for (int p = 0; p < M::kPieces; ++p) {
-                if (p > 0) __syncthreads();                 // the piece before has been read (the first: W_i, by everybody in front of the barrier)
-                bs_bring_rows<M::kHPiece>(sr, hb, kBsI, p * M::kHPiece, rows);
+                if (p > 0) __syncthreads();                 // the piece before has been read
+                if (p + 1 < M::kPieces) bs_bring_rows<M::kHPiece>(sr + ((p + 1) & 1) * M::kHBuf, hb, kBsI, (p + 1) * M::kHPiece, rows);
                 cp_async_commit();
-                cp_async_wait<0>();
+                cp_async_wait<1>();
                 __syncthreads();
-                y.template add<M::kHPiece>(sr, swo, bs_ld(kBsI), p * M::kHPiece, warp, lane);
+                y.template add<M::kHPiece>(sr + (p & 1) * M::kHBuf, swo, bs_ld(kBsI), p * M::kHPiece, warp, lane);
             }
             y.store(rows, warp, lane, residual(bo2));
         }

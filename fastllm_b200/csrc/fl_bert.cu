@@ -289,8 +289,9 @@ static void bert_reserve(BertModel& m, int b, int t) {
 }
 
 // Few short sentences: the whole encoder in one launch of clusters (bert_small.cuh).  -> false: the launch chain takes the call.
-// The line lies where the clusters (about nine of 16 blocks) are all resident and none has more than 64 tokens: a second wave would cost what
-// the chain does (0.26 ms, whatever it has below some hundred tokens).
+// The line lies where the clusters (about nine of 16 blocks) are all resident and none has more than 64 tokens: there both take the same (sentences
+// x tokens, chain / one launch, us: 16 x 19 315 / 256, 9 x 48 323 / 324, 18 x 31 319 / 323, 9 x 64 328 / 333, 36 x 16 319 / 315), and a second wave
+// would cost a whole pass more.
 constexpr int kBsCluster = 16;
 template <int MT>
 static int bert_small_launch(BertModel& m, const BertSmallArgs& a, int clusters, bool ask) {      // ask: -> clusters that are resident at a time
