@@ -958,8 +958,10 @@ static void launch_ly_gemm(LaunchCtx& lc, const char* tag, const LyGemm& g, int 
         FL_CUDA(cudaFuncSetAttribute(ly_gemm64_kernel<8, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ly_gemm64_smem<8, 64>()));
         attr_set = true;
     }
-    // up to 16 rows a tile of 32 would mostly multiply nothing (two tiles of eight: half the f64 work)
-    if (max_rows <= 16)
+    // Experts of few rows each: a tile of 32 would mostly multiply nothing.  8 experts of 5632, width 2048, whole decode step of 4 / 8 / 16 rows (8 /
+    // 16 / 32 picks): 3.02 / 3.29 / 3.50 ms with 32 x 32 tiles, 2.55 / 2.80 / 2.94 with 8 x 64; at 1 row 2.02 and 2.14, at 48 rows 3.61 and 4.09
+    // (experts of 2816, width 1024: 1.08 / 1.24 / 1.36 and 1.11 / 1.26 / 1.39).  One matrix is short of blocks instead: 1 / 8 / 16 rows of width 1024 take 0.85 / 0.94 / 1.07 ms with 32 x 32 tiles, 1.06 / 1.15 / 1.31 with 8 x 64.
+    if (groups > 1 && max_rows >= 8 && max_rows <= 32)
         launch(lc, tag, bytes, ly_gemm64_kernel<8, 64>, dim3((g.N + 63) / 64, (max_rows + 7) / 8, groups), dim3(256), ly_gemm64_smem<8, 64>(), g);
     else
         launch(lc, tag, bytes, ly_gemm64_kernel<32, 32>, dim3((g.N + 31) / 32, (max_rows + 31) / 32, groups), dim3(256), ly_gemm64_smem<32, 32>(), g);

@@ -165,6 +165,17 @@ def test_exact_gemm_rows_stand_alone(width, ff):
     assert np.array_equal(whole, R.run_cut(model, toks, [1, 8, 9, 16, 17, 32, 2], cache=model.new_device_cache(2, 128)))
 
 
+@pytest.mark.parametrize("width,ff", [(64, 72), (50, 34)])
+def test_exact_expert_rows_stand_alone(width, ff):
+    """the same for experts: 2, 8, 10, 16, 32, 34 and 128 picks in a step"""
+    cfg = N.config([N.gla(heads=2, dim=6, vdim=10, mlp=N.moe(ff=ff, experts=5, top=2))], vocab=101, width=width)
+    oracle, model = N.build(cfg, seed=75)
+    toks = N.tokens(cfg, 64, seed=76)
+    whole = N.run_whole(model, toks, cache=model.new_device_cache(2, 128))
+    assert N.relerr(whole, oracle.run(toks)) < N.TOL["f32"]
+    assert np.array_equal(whole, N.run_cut(model, toks, [1, 4, 5, 8, 16, 17], cache=model.new_device_cache(2, 128)))
+
+
 # ---- convolutions in front of the recurrences, rows with a sliding window (256 rows and more, four taps) -----------------------------------
 @pytest.mark.parametrize("layer", [R.delta(heads=4, kv_heads=2, dim=32, vdim=24, conv=4), R.delta(heads=2, kv_heads=2, dim=128, vdim=132, conv=4),
                                    R.delta(heads=6, kv_heads=3, dim=64, vdim=8, conv=4), R.mamba(heads=4, vdim=12, state=20, groups=2, conv=4),
