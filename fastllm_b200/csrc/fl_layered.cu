@@ -1623,8 +1623,11 @@ static void run_mixer(fl_cache& c, LaunchCtx& lc, const StepTab& st, const Layer
         // channel chunks per row: whole q / k heads for the delta rule (they are normalised inside one block)
         const int chunk = delta ? D * std::max(1, 512 / D) : 512, nchunk = (lw.conv_ch + chunk - 1) / chunk;
         // many rows, four taps, whole heads within a warp: a sliding window per thread (the exact mode keeps one order of sums for every step).
-        // 2048 rows: Mamba-2's 10240 channels 189 -> 66 us, the delta rule's 8192 133 -> 56 us
-        const bool slide = !m.f32 && Ti >= 256 && d.conv == 4 && ((lw.n_in | lw.conv_off | lw.conv_ch) & 3) == 0 && (!delta || D == 32 || D == 64 || D == 128);
+        // 2048 rows: Mamba-2's 10240 channels 189 -> 66 us, the delta rule's 8192 133 -> 56 us.  Its blocks of 16 rows x 1024 channels have to fill the
+        // chip: whole prefill of width 2048 (4096 and 5120 channels), per row -> sliding: 256 rows 655 -> 681 us, 448 rows 815 -> 827, 512 rows 848 ->
+        // 831; of width 4096: 224 rows 1147 -> 1154, 256 rows 1166 -> 1150.
+        constexpr int kSlideBlocks = 128;
+        const bool slide = !m.f32 && (Ti + kConvRows - 1) / kConvRows * ((lw.conv_ch + 1023) / 1024) >= kSlideBlocks && d.conv == 4 && ((lw.n_in | lw.conv_off | lw.conv_ch) & 3) == 0 && (!delta || D == 32 || D == 64 || D == 128);
         if (slide) {
             const ConvHeads hd{delta ? G * D : 0, D, (float)(1.0 / std::sqrt((double)D)), delta ? lw.off_a : lw.off_dt, delta ? lw.off_b : -1, lw.dt_bias, lw.a_log, H, y.rs.p};
             launch(lc, delta ? "delta_prep" : "ssm_prep", 0, ly_conv4_rows_kernel, dim3((Ti + kConvRows - 1) / kConvRows, (lw.conv_ch + 1023) / 1024), dim3(256), 0, ca, hd, Ti);

@@ -176,19 +176,21 @@ def test_exact_expert_rows_stand_alone(width, ff):
     assert np.array_equal(whole, N.run_cut(model, toks, [1, 4, 5, 8, 16, 17], cache=model.new_device_cache(2, 128)))
 
 
-# ---- convolutions in front of the recurrences, rows with a sliding window (256 rows and more, four taps) -----------------------------------
+# ---- convolutions in front of the recurrences, rows with a sliding window (blocks of 16 rows that fill the chip, four taps) -----------------------------------
 @pytest.mark.parametrize("layer", [R.delta(heads=4, kv_heads=2, dim=32, vdim=24, conv=4), R.delta(heads=2, kv_heads=2, dim=128, vdim=132, conv=4),
                                    R.delta(heads=6, kv_heads=3, dim=64, vdim=8, conv=4), R.mamba(heads=4, vdim=12, state=20, groups=2, conv=4),
                                    R.mamba(heads=8, vdim=128, state=16, groups=1, conv=4)])
-def test_sliding_convolution(layer):
-    """against the same model in portions that stay with the per-row kernel; several sequences per block, one that goes on, one of one token"""
+@pytest.mark.parametrize("long", [270, 2050])
+def test_sliding_convolution(layer, long):
+    """against the same model in portions that stay with the per-row kernel; several sequences per block, one that goes on, one of one token
+    (270: the per-row kernel takes the mixed step too)"""
     cfg = R.config([layer], width=64)
     _, model = R.build(cfg, seed=81, dtype="bf16")
-    reqs = [R.tokens(cfg, k, seed=82 + i) for i, k in enumerate((270, 5, 1, 33))]
-    alone = [R.run_cut(model, r, [100, 100, 70], cache=model.new_device_cache(1, 512)) for r in reqs]
-    cache = model.new_device_cache(4, 512)
+    reqs = [R.tokens(cfg, k, seed=82 + i) for i, k in enumerate((long, 5, 1, 33))]
+    alone = [R.run_cut(model, r, [100] * 21, cache=model.new_device_cache(1, 2112)) for r in reqs]
+    cache = model.new_device_cache(4, 2112)
     cache.forward_ragged([0], [reqs[0][:7]], [[]])
-    got = cache.forward_ragged([3, 0, 2, 1], [reqs[1], reqs[0][7:], reqs[2], reqs[3]], [list(range(5)), list(range(263)), [0], list(range(33))])
+    got = cache.forward_ragged([3, 0, 2, 1], [reqs[1], reqs[0][7:], reqs[2], reqs[3]], [list(range(5)), list(range(long - 7)), [0], list(range(33))])
     want = np.concatenate([alone[1], alone[0][7:], alone[2], alone[3]])
     assert R.relerr(got, np.asarray(want, dtype=np.float64)) < CHUNK_TOL
 
