@@ -26,7 +26,10 @@ constexpr int kCsSlab = 64;             // value columns at a time
 constexpr int kCsPad = 4;               // floats behind a row in shared memory: neighbouring rows start four banks apart
 constexpr int kCsLdA = kCsC + kCsPad;   // row stride of a [64][64] operand
 constexpr int kCsChunks = 32;           // chunks whose states are held at a time (32 heads of 128 x 128: 67 MB), over all sequences of a step
-constexpr int kCsMinTokens = 128;       // portions from this length on
+// Portions from this length on.  Whole prefill token by token -> in chunks, 96 / 128 / 160 / 192 tokens: gated linear attention, width 2048, 728 -> 722,
+// 771 -> 732, 847 -> 780, 881 -> 783 us; lightning 607 -> 577, 605 -> 590, 683 -> 657, 706 -> 661; delta rule and Mamba-2 543 -> 551, 550 -> 550,
+// 623 -> 617, 665 -> 622, of width 4096 838 -> 877, 889 -> 898, 1105 -> 1099, 1160 -> 1110.  (64 tokens are slower in chunks everywhere.)
+constexpr int kCsMinTokens = 128;
 
 struct ChunkArgs {
     const float* src; int ld, off_q, off_k, off_v;      // q, k [G][D], v [H][Dv] per row

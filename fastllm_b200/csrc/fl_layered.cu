@@ -832,7 +832,8 @@ static void drop_graphs(fl_cache& c) {
 // The first matrix of a gated feed-forward and its activation, as the hi | lo halves the second one reads.  More than 128 rows whose
 // tiles fill the chip take the activation in the GEMM's epilogue: the [rows, 2 F] f32 result (235 MB at 2048 rows of F = 14336) is neither
 // written nor read back (three such layers of width 4096, whole prefill: 8.29 -> 8.07 ms).  Few tiles keep the GEMM that cuts K; the
-// epilogue cannot see a sum in slices.
+// epilogue cannot see a sum in slices.  Hidden width 2816, whole prefill of width 2048, GEMM that cuts K -> fused: 384 rows (66 tiles) 711 -> 725 us,
+// 512 rows (88 tiles) 764 -> 763, 1024 rows 1130 -> 1116; of width 1024: 384 rows 587 -> 594, 512 rows 645 -> 636.
 static bool ff_in_fused(int R, int F, int K, int act, bool tc_in, bool tc_out, bool f32) {
     const int tiles = (R + 127) / 128 * ((F + 127) / 128);
     return tc_in && tc_out && !f32 && R > 128 && act != FL_ACT_RELU2 && F % 8 == 0 && (2 * tiles > kNumSMs || (K + 63) / 64 < 16);
@@ -944,8 +945,8 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
     }
 }
 
-// The FMA-chain GEMM: f32 accumulators where it stands in for the tensor-core GEMM on shapes outside its tiles (serving precision),
-// f64 accumulators in the exact mode.
+// GEMMs that are not gemm_tc_kernel's: f32 FMA where they stand in for it on shapes outside its tiles (serving precision), the f64 tensor pipe in
+// the exact mode.
 static void launch_ly_gemm(LaunchCtx& lc, const char* tag, const LyGemm& g, int groups, int max_rows) {
     const uint64_t bytes = (uint64_t)groups * g.N * g.K * 2;
     if (!lc.exact) {
@@ -1509,9 +1510,9 @@ void layered_forward(fl_cache& c, const int* slots, const int* counts, int n, co
     // ---- device: layer by layer over all rows of the step ----
     LaunchCtx lc;
     lc.stream = c.stream;
-    // Programmatic dependent launch where the kernels are short enough for their set-up to count: a mixed step of 340 rows of width 2048 runs
-    // in 0.87 instead of 0.99 ms, 1531 rows in 2.14 instead of 2.17 ms.  Where a kernel fills the chip for long, the next one's waiting blocks
-    // only take its room: 2048 rows of width 4096 lose 1.5 %, the exact mode (two blocks of 70 KB per SM) 5 %.
+    // Programmatic dependent launch where the kernels are short enough for their set-up to count: steps of 256 to 2048 rows of width 2048 gain 4 to
+    // 12 % (340 mixed rows 0.99 -> 0.87 ms, 1531 rows 2.05 -> 1.95), 1024 rows of width 4096 2 %.  Beyond, 1536 and 2048 rows of width 4096 were
+    // between 1.5 % slower and 0.7 % faster; the exact mode (two blocks of 70 KB per SM, which the next kernel's waiting blocks crowd) loses 5 %.
     static const bool no_pdl = env_flag("FL_NO_PDL");
     lc.pdl = !no_pdl && !m.f32 && (size_t)T * m.W <= ((size_t)4 << 20);
     lc.exact = m.f32;
