@@ -2,6 +2,10 @@
 
 Bars as in the design's own test files: the serving precision differs from the oracle (which rounds what it caches to bf16) by cached
 elements that land on the other side of a rounding boundary, and a near-tied router may pick another expert after one (`allow`)."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 
@@ -109,6 +113,13 @@ def test_chunks_of_several_sequences(kind):
             cache.slot_reset(s)
 
 
+@pytest.mark.parametrize("kind", ["gla", "gla_fast_decay", "mamba", "delta"])
+@pytest.mark.parametrize("dim,vdim,n", [(64, 64, 333), (100, 36, 200)])
+def test_chunks_against_the_oracle(kind, dim, vdim, n):
+    mod, cfg = recurrent(kind, dim, vdim)
+    check(mod, cfg, n, 47, 0.0)
+
+
 @pytest.mark.parametrize("dim,vdim,n", [(16, 24, 128), (128, 128, 200), (64, 72, 333)])
 def test_lightning_chunks(dim, vdim, n):
     check(M, M.config([M.par_layer(b=M.lightning(heads=2, dim=dim, vdim=vdim))], width=64), n, 45, 0.0)
@@ -207,6 +218,56 @@ def test_attention_scale_of_any_sign(scale, softcap):
     """a scale of zero or below: masked scores stay masked, the maximum is that of the scaled scores"""
     both_ways(R, R.config([R.att(heads=2, kv_heads=1, dim=32, vdim=32, rot_dims=8, scale=scale, softcap=softcap)], width=64), 200, [130, 64], 73)
     both_ways(M, M.config([M.par_layer(M.windowed(dim=16, vdim=16, window=257, keep=2, scale=scale), M.lightning(heads=2, dim=8, vdim=8))], width=64), 400, [70, 201, 100], 74)
+
+
+# ---- steps of single tokens, more than 128 of them: row runs inside a captured graph -----------------------------------------------------
+def test_expert_runs_of_single_tokens():
+    """run eagerly, captured, replayed and replayed with other tokens and routes; some sequences against the model alone"""
+    n, cfg = 150, N.config([N.gla(heads=2, dim=16, vdim=16, mlp=N.moe(ff=24, experts=5, top=2))], vocab=64, width=64)
+    _, model = N.build(cfg, seed=93, dtype="bf16")
+    toks = [N.tokens(cfg, 5, seed=200 + i) for i in range(n)]
+    cache = model.new_device_cache(n, 64)
+    got = np.stack([cache.forward_ragged(list(range(n)), [t[k:k + 1] for t in toks], [[0]] * n) for k in range(5)], axis=1)
+    for i in (0, 1, 77, 127, 128, 149):
+        alone = N.run_cut(model, toks[i], [5], cache=model.new_device_cache(1, 64))
+        assert N.relerr(got[i], np.asarray(alone, dtype=np.float64)) < CHUNK_TOL
+
+
+# ---- dependent launch ------------------------------------------------------------------------------------------------------------------------
+DEPENDENT_LAUNCH = r"""
+import sys
+import numpy as np
+import test_many_rows_gpu as S
+out = []
+for mod, cfg in S.dependent_launch_cases():
+    _, model = mod.build(cfg, seed=95, dtype="bf16")
+    toks = [mod.tokens(cfg, k, seed=300 + k) for k in (1, 140, 30)]
+    cache = model.new_device_cache(3, 256)
+    out.append(cache.forward_ragged([0, 1, 2], toks, [[0], list(range(0, 140, 7)), [29]]).ravel())
+    for k in range(4):                      # eager, captured, replayed
+        out.append(cache.forward_ragged([2, 0, 1], [t[-1:] for t in toks], [[0]] * 3).ravel())
+np.save(sys.argv[1], np.concatenate(out))
+"""
+
+
+def dependent_launch_cases():
+    return [(N, N.hybrid_cfg()), (R, R.config([R.delta(heads=4, kv_heads=2, dim=32, vdim=24, conv=4, mlp=R.dense(ff=40)), R.att(heads=4, kv_heads=2, dim=16, vdim=16, rot_dims=8),
+                                               R.mamba(heads=4, vdim=12, state=20, groups=2, conv=4)], width=64)),
+            (T, T.config([T.layer(mlp=T.moe(experts=8, top=2, ff=24))], width=64)),
+            (M, M.config([M.par_layer(M.windowed(dim=16, vdim=16, window=257, keep=2), M.lightning(heads=2, dim=8, vdim=8))], width=64)),
+            (U, U.bare([U.alayer(U.grouped(dim=16, dims=8))], width=64))]
+
+
+def test_dependent_launch_changes_nothing(tmp_path):
+    """every kernel of a layered step waits for the one before: the same bits with and without dependent launch"""
+    here = os.path.dirname(os.path.abspath(__file__))
+    res = []
+    for off in ("0", "1"):
+        path = str(tmp_path / f"{off}.npy")
+        env = {**os.environ, "FL_NO_PDL": off, "PYTHONPATH": os.pathsep.join([os.path.dirname(here), here])}
+        subprocess.run([sys.executable, "-c", DEPENDENT_LAUNCH, path], check=True, env=env, cwd=here, timeout=300)
+        res.append(np.load(path))
+    assert np.isfinite(res[0]).all() and np.array_equal(res[0], res[1])
 
 
 # ---- workspace: only what a step's path reads, grown between steps -----------------------------------------------------------------------------
