@@ -12,7 +12,8 @@
 //   1. ly_chunk_in_kernel / ly_chunk_gla_kernel / ly_chunk_delta_kernel   one block per (chunk, head): everything that needs no state
 //   2. ly_chunk_state_kernel / ly_chunk_delta_state_kernel                 the states at the chunks' starts, chunk by chunk
 //   3. ly_chunk_out_kernel                                                 one block per (chunk, head): what the starting state adds
-// Bound: f32 FMA issue in 1 and 3 (operands in shared memory, 4 x 4 results per thread: 64 FMA per 8 16-byte loads), HBM in 2.
+// Bound: 1 and 3 by latency -- operands in shared memory, 4 x 4 results per thread (64 FMA per 8 16-byte loads), 16 warps per SM (8 in the gated
+// one): at 1024 tokens ncu has the FMA pipe at 31 to 34 % (gated 14 %), issue slots at 45 to 47 % (25 %), shared memory at 47 to 50 % (24 %).  2: HBM.
 // Measured per layer, token by token -> chunks: gated linear attention, 1531 tokens, 16 heads of 128 x 128: 1160 -> 260 us; Mamba-2, 2048
 // tokens, 128 heads of 128 x 64: 1186 -> 668 us (four heads per block: their scores are multiplied once); delta rule, 2048 tokens, 32 heads of 128 x 128: 1022 -> 626 us; lightning attention, 333
 // tokens, 16 heads: 246 -> 65 us.  Same model, same tokens: the logits agree to 1e-5 .. 4e-5, their error against 64 bits is unchanged.

@@ -243,7 +243,7 @@ def test_batched_decode_graph_captured_at_a_short_context_stays_correct():
     # Tolerance of a LONG dense-path decode: the tensor-core path carries activations as hi + lo bf16 pairs (2^-17 residue), which
     # flips the bf16 rounding of a freshly cached K / V element ~100x more often than the f32 GEMV path's summation-order noise;
     # every flip moves later logits by ~1e-3 and this config shares ONE kv head between 8 query heads.  Measured over 150 steps:
-    # 1e-3 .. 8e-3, not growing with the step index; the bar is the north_star's 1e-2 (tools/diag_batch3.py; the batch-1 path against the same oracle: 3e-4 .. 1e-3).
+    # 1e-3 .. 8e-3, not growing with the step index; the bar is 1e-2 (the batch-1 path against the same oracle: 3e-4 .. 1e-3).
     assert worst <= 1e-2
 
 
