@@ -961,7 +961,8 @@ static void launch_ly_gemm(LaunchCtx& lc, const char* tag, const LyGemm& g, int 
     }
     // Experts of few rows each: a tile of 32 would mostly multiply nothing.  8 experts of 5632, width 2048, whole decode step of 4 / 8 / 16 rows (8 /
     // 16 / 32 picks): 3.02 / 3.29 / 3.50 ms with 32 x 32 tiles, 2.55 / 2.80 / 2.94 with 8 x 64; at 1 row 2.02 and 2.14, at 48 rows 3.61 and 4.09
-    // (experts of 2816, width 1024: 1.08 / 1.24 / 1.36 and 1.11 / 1.26 / 1.39).  One matrix is short of blocks instead: 1 / 8 / 16 rows of width 1024 take 0.85 / 0.94 / 1.07 ms with 32 x 32 tiles, 1.06 / 1.15 / 1.31 with 8 x 64.
+    // (experts of 2816, width 1024: 1.08 / 1.24 / 1.36 and 1.11 / 1.26 / 1.39).  One matrix is short of blocks instead: 1 / 8 / 16 rows of width
+    // 1024 take 0.85 / 0.94 / 1.07 ms with 32 x 32 tiles, 1.06 / 1.15 / 1.31 with 8 x 64.
     if (groups > 1 && max_rows >= 8 && max_rows <= 32)
         launch(lc, tag, bytes, ly_gemm64_kernel<8, 64>, dim3((g.N + 63) / 64, (max_rows + 7) / 8, groups), dim3(256), ly_gemm64_smem<8, 64>(), g);
     else
@@ -1411,7 +1412,7 @@ static bool gqa_portion_tc(const LayeredModel& m, const fl_layer_desc& d, int Ts
 static void reserve_portions(fl_cache& c, const int* slots, const int* counts, int n) {
     const LayeredModel& m = *c.lm;
     LayeredCache& y = *c.ly;
-    if (m.f32) return;
+    if (m.f32 || *std::max_element(counts, counts + n) < 64) return;        // (decoded tokens and short portions need none of it)
     const ChunkPlan pl = chunk_plan(counts, n);
     ChunkScratch cs;
     size_t kc = 0, kct = 0;
@@ -1628,7 +1629,8 @@ static void run_mixer(fl_cache& c, LaunchCtx& lc, const StepTab& st, const Layer
         // chip: whole prefill of width 2048 (4096 and 5120 channels), per row -> sliding: 256 rows 655 -> 681 us, 448 rows 815 -> 827, 512 rows 848 ->
         // 831; of width 4096: 224 rows 1147 -> 1154, 256 rows 1166 -> 1150.
         constexpr int kSlideBlocks = 128;
-        const bool slide = !m.f32 && (Ti + kConvRows - 1) / kConvRows * ((lw.conv_ch + 1023) / 1024) >= kSlideBlocks && d.conv == 4 && ((lw.n_in | lw.conv_off | lw.conv_ch) & 3) == 0 && (!delta || D == 32 || D == 64 || D == 128);
+        const bool slide = !m.f32 && (Ti + kConvRows - 1) / kConvRows * ((lw.conv_ch + 1023) / 1024) >= kSlideBlocks && d.conv == 4 &&
+                           ((lw.n_in | lw.conv_off | lw.conv_ch) & 3) == 0 && (!delta || D == 32 || D == 64 || D == 128);
         if (slide) {
             const ConvHeads hd{delta ? G * D : 0, D, (float)(1.0 / std::sqrt((double)D)), delta ? lw.off_a : lw.off_dt, delta ? lw.off_b : -1, lw.dt_bias, lw.a_log, H, y.rs.p};
             launch(lc, delta ? "delta_prep" : "ssm_prep", 0, ly_conv4_rows_kernel, dim3((Ti + kConvRows - 1) / kConvRows, (lw.conv_ch + 1023) / 1024), dim3(256), 0, ca, hd, Ti);

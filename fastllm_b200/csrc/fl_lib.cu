@@ -1917,10 +1917,9 @@ FL_EXPORT int fl_cache_destroy(fl_cache* c) {
 
 // deliver_logits' device side
 struct LogitsTransfer {
-    static constexpr int kMaxParts = 16;
     cudaStream_t stream; const float* dev; float* pinned;
     int parts = 0;
-    cudaEvent_t e[kMaxParts] = {};
+    cudaEvent_t e[kLogitsParts] = {};
     LogitsTransfer(cudaStream_t s, const float* d, float* p) : stream(s), dev(d), pinned(p) {}
     LogitsTransfer(const LogitsTransfer&) = delete;
     ~LogitsTransfer() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
