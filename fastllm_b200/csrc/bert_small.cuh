@@ -9,7 +9,7 @@
 // The results are the chain's, bit for bit: an output's products go into its f32 accumulator 16 columns of K at a time in ascending order, as
 // tcgen05.mma takes them (mma.sync m16n8k16 sums the same 16 products to the same bits, in whatever order they stand inside the 16), so K is
 // not split over warps; attention, roundings and the order of every other sum are those of bert.cuh.
-// Bound: latency -- 5 phases x 6 layers of about 6 us (cluster barrier, L2 round trips of activations and weights, a chain of 24 to 96 MMAs).
+// Bound: latency -- 5 phases x 6 layers of about 5 us (cluster barrier, L2 round trips of activations and weights, a chain of 24 to 96 MMAs).
 // One sentence of 4 / 19 / 48 / 64 tokens, whole call: 243 / 254 / 268 / 277 us as 44 launches, 120 / 160 / 224 / 269 us here.  (K in quarters over
 // the warps is no faster, and its sums are not the chain's: 16-bit activations carry that to 3e-3 in the embedding.)
 #pragma once

@@ -959,11 +959,14 @@ static void launch_ly_gemm(LaunchCtx& lc, const char* tag, const LyGemm& g, int 
         FL_CUDA(cudaFuncSetAttribute(ly_gemm64_kernel<8, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ly_gemm64_smem<8, 64>()));
         attr_set = true;
     }
-    // Experts of few rows each: a tile of 32 would mostly multiply nothing.  8 experts of 5632, width 2048, whole decode step of 4 / 8 / 16 rows (8 /
-    // 16 / 32 picks): 3.02 / 3.29 / 3.50 ms with 32 x 32 tiles, 2.55 / 2.80 / 2.94 with 8 x 64; at 1 row 2.02 and 2.14, at 48 rows 3.61 and 4.09
-    // (experts of 2816, width 1024: 1.08 / 1.24 / 1.36 and 1.11 / 1.26 / 1.39).  One matrix is short of blocks instead: 1 / 8 / 16 rows of width
-    // 1024 take 0.85 / 0.94 / 1.07 ms with 32 x 32 tiles, 1.06 / 1.15 / 1.31 with 8 x 64.
-    if (groups > 1 && max_rows >= 8 && max_rows <= 32)
+    // Few rows: a tile of 32 would mostly multiply nothing, tiles of 8 x 64 do a quarter of its work (up to eight rows; every further eight read the
+    // weights again) but are half as many.  One matrix whose 8 x 64 tiles nearly fill the chip takes them: whole decode step, 32 x 32 tiles
+    // everywhere -> 8 x 64 from 8000 columns on, 1 / 4 / 8 rows of width 1024: 835 / 859 / 923 -> 799 / 825 / 894 us, of width 4096: 4.54 / 4.58 / 4.68 ->
+    // 3.92 / 3.96 / 4.06 ms; from 4000 columns on: 838 / 871 / 932 us and 4.78 / 4.83 / 4.94 ms.  Experts of few rows each: 8 of 5632, width 2048,
+    // 4 / 8 / 16 rows (8 / 16 / 32 picks) 3.02 / 3.29 / 3.50 -> 2.55 / 2.80 / 2.94 ms, but 1 row 2.02 -> 2.14 and 48 rows 3.61 -> 4.09 (of 2816, width
+    // 1024: 1.08 / 1.24 / 1.36 -> 1.11 / 1.26 / 1.39).
+    const bool small_tiles = groups > 1 ? max_rows >= 8 && max_rows <= 32 : max_rows <= 8 && 6 * ((g.N + 63) / 64) >= 5 * kNumSMs;
+    if (small_tiles)
         launch(lc, tag, bytes, ly_gemm64_kernel<8, 64>, dim3((g.N + 63) / 64, (max_rows + 7) / 8, groups), dim3(256), ly_gemm64_smem<8, 64>(), g);
     else
         launch(lc, tag, bytes, ly_gemm64_kernel<32, 32>, dim3((g.N + 31) / 32, (max_rows + 31) / 32, groups), dim3(256), ly_gemm64_smem<32, 32>(), g);

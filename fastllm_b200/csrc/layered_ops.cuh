@@ -538,7 +538,7 @@ static __global__ void __launch_bounds__(256) ly_gemm_kernel(LyGemm g) {
 // Bound: the f64 pipe (64 FMA per clock and SM).  One thread per 4 x 4 outputs of a 64 x 64 tile, widening its operands at every use, left
 // half of the chip without a block; 4 x 4 outputs per thread over widened operands are bound by shared memory (16-byte loads of f64: ncu had
 // it at 83 %, the f64 pipe at 22 %).  203 x 1024 x 2816: 310 -> 83 us (33 at the pipe's rate); 203 x 5632 x 1024: 283 -> 134 us (65);
-// whole decode step of one row, width 1024, vocabulary 32000: 2.48 -> 0.85 ms.  Results bit-identical.
+// whole decode step of one row, width 1024, vocabulary 32000: 2.48 -> 0.80 ms.  Results bit-identical.
 __device__ __forceinline__ void mma_f64_884(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
 }

@@ -187,6 +187,16 @@ def test_exact_expert_rows_stand_alone(width, ff):
     assert np.array_equal(whole, N.run_cut(model, toks, [1, 4, 5, 8, 16, 17], cache=model.new_device_cache(2, 128)))
 
 
+def test_exact_head_rows_stand_alone():
+    """the same for a matrix of so many columns that up to eight rows take other tiles than more"""
+    cfg = R.config([R.delta(heads=4, kv_heads=2, dim=6, vdim=10)], vocab=8101, width=50)
+    oracle, model = R.build(cfg, seed=77)
+    toks = R.tokens(cfg, 40, seed=78)
+    whole = R.run_whole(model, toks, cache=model.new_device_cache(2, 64))
+    assert R.relerr(whole, oracle.run(toks)) < R.TOL["f32"]
+    assert np.array_equal(whole, R.run_cut(model, toks, [1, 8, 9, 7, 14], cache=model.new_device_cache(2, 64)))
+
+
 # ---- convolutions in front of the recurrences, rows with a sliding window (blocks of 16 rows that fill the chip, four taps) -----------------------------------
 @pytest.mark.parametrize("layer", [R.delta(heads=4, kv_heads=2, dim=32, vdim=24, conv=4), R.delta(heads=2, kv_heads=2, dim=128, vdim=132, conv=4),
                                    R.delta(heads=6, kv_heads=3, dim=64, vdim=8, conv=4), R.mamba(heads=4, vdim=12, state=20, groups=2, conv=4),
