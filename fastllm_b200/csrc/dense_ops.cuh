@@ -59,9 +59,8 @@ struct PrepArgs {
     int ldd;
     int nsl;                    // split-K slices of delta (>= 1), summed in order: deterministic
     long long sl_stride;
-    const float* norm_w;        // non-null: x = rms_norm(resid) * norm_w, else x = src row
+    const float* norm_w;        // x = rms_norm(resid) * norm_w
     float eps;
-    const float* src;           // plain split source [R, K] (norm_w == null, embed == null)
     int K;
     int t;                      // last_only: output row j takes input row (j + 1) * t - 1
     int last_only;
@@ -69,7 +68,8 @@ struct PrepArgs {
     uint16_t* xlo;
 };
 
-// one CTA per output row, float4-vectorised (K % 4 == 0); up to 1024 threads so a 4096-wide row is one load per thread
+// one CTA per output row, float4-vectorised (K % 4 == 0); up to 1024 threads.  Rows of any width: those that fit a block's registers take
+// dense_prep_rows_kernel.
 static __global__ void __launch_bounds__(1024) dense_prep_kernel(const PrepArgs a) {
     pdl_launch_dependents();
     pdl_wait();
@@ -85,11 +85,6 @@ static __global__ void __launch_bounds__(1024) dense_prep_kernel(const PrepArgs 
         xh[i] = make_uint2((uint32_t)h0 | ((uint32_t)h1 << 16), (uint32_t)h2 | ((uint32_t)h3 << 16));
         xl[i] = make_uint2((uint32_t)l0 | ((uint32_t)l1 << 16), (uint32_t)l2 | ((uint32_t)l3 << 16));
     };
-    if (a.norm_w == nullptr && a.embed == nullptr) {      // plain hi/lo split of an f32 row
-        const float4* s = reinterpret_cast<const float4*>(a.src + (size_t)row * K);
-        for (int i = threadIdx.x; i < K4; i += blockDim.x) emit(i, s[i]);
-        return;
-    }
     float4* r = reinterpret_cast<float4*>(a.resid + (size_t)row * K);
     float ss = 0.f;
     for (int i = threadIdx.x; i < K4; i += blockDim.x) {
@@ -134,14 +129,13 @@ static __global__ void __launch_bounds__(1024) dense_prep_kernel(const PrepArgs 
     }
 }
 
-// Many-row variant (prefill): 256 threads per row with the row held in registers between the sum-of-squares and the scaling pass
-// (NV float4 per thread: K <= 1024 NV), so a row is read once and more rows are resident per SM.  Same arithmetic as
-// dense_prep_kernel (slices summed in order, then added to the residual); only the residual-add + RMSNorm form.
-constexpr int kPrepRowsThreads = 256;
-template <int NV>
-static __global__ void __launch_bounds__(kPrepRowsThreads) dense_prep_rows_kernel(const PrepArgs a) {
+// The same with the row in registers between the two passes (THREADS threads, NV float4 each: K <= 4 NV THREADS), so a row is read once.
+// Calls of few rows take 512 threads per row, many-row calls 256 (four rows resident per SM).  The norm's weights do not depend on the
+// kernels before this one and are fetched ahead of the wait.  A block of 1024 threads x 58 registers left no room for the next GEMM's
+// block on its SM, which then started only behind this kernel; and it read the row back from L2 in the second pass.
+template <int NV, int THREADS>
+static __global__ void __launch_bounds__(THREADS) dense_prep_rows_kernel(const PrepArgs a) {
     pdl_launch_dependents();
-    pdl_wait();
     __shared__ float red[32];
     const int orow = blockIdx.x;
     const int row = a.last_only ? (orow + 1) * a.t - 1 : orow;
@@ -149,30 +143,70 @@ static __global__ void __launch_bounds__(kPrepRowsThreads) dense_prep_rows_kerne
     uint2* xh = reinterpret_cast<uint2*>(a.xhi + (size_t)orow * K);
     uint2* xl = reinterpret_cast<uint2*>(a.xlo + (size_t)orow * K);
     float4* r = reinterpret_cast<float4*>(a.resid + (size_t)row * K);
-    float4 v[NV];
+    constexpr bool kAhead = NV <= 2;               // (more would cost registers that many resident rows need)
+    float4 w[kAhead ? NV : 1];
+    if (kAhead) {
 #pragma unroll
-    for (int j = 0; j < NV; ++j) {
-        const int i = threadIdx.x + j * kPrepRowsThreads;
-        v[j] = i < K4 ? r[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        for (int j = 0; j < NV; ++j) {
+            const int i = threadIdx.x + j * THREADS;
+            w[kAhead ? j : 0] = i < K4 ? __ldg(reinterpret_cast<const float4*>(a.norm_w) + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+    }
+    pdl_wait();
+    float4 v[NV];
+    if (a.embed != nullptr) {
+        uint32_t id = a.ids[row];
+        if (id >= (uint32_t)a.vocab) id = a.vocab - 1;
+        const uint2* e = reinterpret_cast<const uint2*>(a.embed + (size_t)id * K);
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int i = threadIdx.x + j * THREADS;
+            const uint2 x = i < K4 ? e[i] : make_uint2(0u, 0u);
+            v[j] = make_float4(bf16lo(x.x), bf16hi(x.x), bf16lo(x.y), bf16hi(x.y));
+            if (i < K4) r[i] = v[j];
+        }
+    } else {
+#pragma unroll
+        for (int j = 0; j < NV; ++j) {
+            const int i = threadIdx.x + j * THREADS;
+            v[j] = i < K4 ? r[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
     }
     if (a.delta) {
         float4 ds[NV];
 #pragma unroll
         for (int j = 0; j < NV; ++j) ds[j] = make_float4(0.f, 0.f, 0.f, 0.f);
-        for (int s = 0; s < a.nsl; ++s) {         // fixed order: deterministic split-K reduction
-            const float4* dp = reinterpret_cast<const float4*>(a.delta + (size_t)s * a.sl_stride + (size_t)row * a.ldd);
+        const float4* dp = reinterpret_cast<const float4*>(a.delta + (size_t)row * a.ldd);
+        const size_t st4 = (size_t)a.sl_stride / 4;
+        constexpr int U = NV <= 2 ? 4 : 1;         // slices in flight
+        int s = 0;
+        for (; s + U <= a.nsl; s += U) {           // fixed order: deterministic split-K reduction
+            float4 p[U][NV];
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int j = 0; j < NV; ++j) {
+                    const int i = threadIdx.x + j * THREADS;
+                    p[u][j] = i < K4 ? dp[(size_t)(s + u) * st4 + i] : make_float4(0.f, 0.f, 0.f, 0.f);
+                }
+#pragma unroll
+            for (int u = 0; u < U; ++u)
+#pragma unroll
+                for (int j = 0; j < NV; ++j) { ds[j].x += p[u][j].x; ds[j].y += p[u][j].y; ds[j].z += p[u][j].z; ds[j].w += p[u][j].w; }
+        }
+        for (; s < a.nsl; ++s) {
 #pragma unroll
             for (int j = 0; j < NV; ++j) {
-                const int i = threadIdx.x + j * kPrepRowsThreads;
+                const int i = threadIdx.x + j * THREADS;
                 if (i < K4) {
-                    const float4 p = dp[i];
+                    const float4 p = dp[(size_t)s * st4 + i];
                     ds[j].x += p.x; ds[j].y += p.y; ds[j].z += p.z; ds[j].w += p.w;
                 }
             }
         }
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
-            const int i = threadIdx.x + j * kPrepRowsThreads;
+            const int i = threadIdx.x + j * THREADS;
             v[j].x += ds[j].x; v[j].y += ds[j].y; v[j].z += ds[j].z; v[j].w += ds[j].w;
             if (i < K4) r[i] = v[j];
         }
@@ -186,9 +220,9 @@ static __global__ void __launch_bounds__(kPrepRowsThreads) dense_prep_rows_kerne
     const float m = sqrtf(tot / (float)K + a.eps);       // candle rms_norm: x / sqrt(mean(x^2) + eps) * w
 #pragma unroll
     for (int j = 0; j < NV; ++j) {
-        const int i = threadIdx.x + j * kPrepRowsThreads;
+        const int i = threadIdx.x + j * THREADS;
         if (i < K4) {
-            const float4 wv = __ldg(reinterpret_cast<const float4*>(a.norm_w) + i);
+            const float4 wv = kAhead ? w[kAhead ? j : 0] : __ldg(reinterpret_cast<const float4*>(a.norm_w) + i);
             const float4 x = make_float4(v[j].x / m * wv.x, v[j].y / m * wv.y, v[j].z / m * wv.z, v[j].w / m * wv.w);
             uint16_t h0, l0, h1, l1, h2, l2, h3, l3;
             split_hi_lo(x.x, h0, l0); split_hi_lo(x.y, h1, l1); split_hi_lo(x.z, h2, l2); split_hi_lo(x.w, h3, l3);
@@ -343,27 +377,40 @@ static __global__ void __launch_bounds__(256) dense_qkv_epi_rows_kernel(const Qk
     }
 }
 
-// act = silu(gate) * up from the interleaved gate|up GEMM output, written directly as the hi/lo split the down GEMM reads
-// (grouped expert GEMMs: rows are blocks of `grp_cap` per expert, of which grp_cnt[block] are valid; the rest is skipped)
-static __global__ void dense_silu_split_kernel(const float* __restrict__ y, int nsl, long long sl_stride, int I, uint16_t* __restrict__ xhi,
-                                               uint16_t* __restrict__ xlo, const int* __restrict__ grp_cnt = nullptr, int grp_cap = 0) {
+// act = silu(gate) * up from the interleaved gate|up GEMM output, written directly as the hi/lo split the down GEMM reads; a thread takes four
+// outputs (I % 4 == 0).  Grouped expert GEMMs: rows are blocks of `grp_cap` per expert, of which grp_cnt[block] are valid; grid.y is then
+// kSiluGroupRows per expert, each of which walks its share of the valid rows (a block per row of every expert was 14336 blocks for 64 rows).
+constexpr int kSiluGroupRows = 16;
+static __global__ void __launch_bounds__(256) dense_silu_split_kernel(const float* __restrict__ y, int nsl, long long sl_stride, int I, uint16_t* __restrict__ xhi,
+                                                                     uint16_t* __restrict__ xlo, const int* __restrict__ grp_cnt = nullptr, int grp_cap = 0) {
     pdl_launch_dependents();
     pdl_wait();
-    const int row = blockIdx.y;
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
+    const int j = 4 * (blockIdx.x * blockDim.x + threadIdx.x);
     if (j >= I) return;
-    if (grp_cnt != nullptr && (row % grp_cap) >= grp_cnt[row / grp_cap]) return;
-    float2 gu = make_float2(0.f, 0.f);
-    for (int s = 0; s < nsl; ++s) {
-        const float2 p = *reinterpret_cast<const float2*>(y + (size_t)s * sl_stride + (size_t)row * 2 * I + 2 * j);
-        gu.x += p.x;
-        gu.y += p.y;
+    int row = blockIdx.y, step = 1, end = row + 1;
+    if (grp_cnt != nullptr) {
+        const int grp = blockIdx.y / kSiluGroupRows;
+        step = kSiluGroupRows;
+        row = grp * grp_cap + blockIdx.y % kSiluGroupRows;
+        end = grp * grp_cap + grp_cnt[grp];
     }
-    const float act = gu.x / (1.f + expf(-gu.x)) * gu.y;
-    uint16_t h, l;
-    split_hi_lo(act, h, l);
-    xhi[(size_t)row * I + j] = h;
-    xlo[(size_t)row * I + j] = l;
+    for (; row < end; row += step) {
+        const float* yr = y + (size_t)row * 2 * I + 2 * j;
+        float4 a = make_float4(0.f, 0.f, 0.f, 0.f), b = a;
+#pragma unroll 4
+        for (int s = 0; s < nsl; ++s) {
+            const float4 p = *reinterpret_cast<const float4*>(yr + (size_t)s * sl_stride), q = *reinterpret_cast<const float4*>(yr + (size_t)s * sl_stride + 4);
+            a.x += p.x; a.y += p.y; a.z += p.z; a.w += p.w;
+            b.x += q.x; b.y += q.y; b.z += q.z; b.w += q.w;
+        }
+        uint16_t h[4], l[4];
+        split_hi_lo(a.x / (1.f + expf(-a.x)) * a.y, h[0], l[0]);
+        split_hi_lo(a.z / (1.f + expf(-a.z)) * a.w, h[1], l[1]);
+        split_hi_lo(b.x / (1.f + expf(-b.x)) * b.y, h[2], l[2]);
+        split_hi_lo(b.z / (1.f + expf(-b.z)) * b.w, h[3], l[3]);
+        *reinterpret_cast<uint2*>(xhi + (size_t)row * I + j) = make_uint2((uint32_t)h[0] | ((uint32_t)h[1] << 16), (uint32_t)h[2] | ((uint32_t)h[3] << 16));
+        *reinterpret_cast<uint2*>(xlo + (size_t)row * I + j) = make_uint2((uint32_t)l[0] | ((uint32_t)l[1] << 16), (uint32_t)l[2] | ((uint32_t)l[3] << 16));
+    }
 }
 
 // ---- Mixtral sparse-MoE (candle-transformers models::mixtral::SparseMoeBlock) ----------------

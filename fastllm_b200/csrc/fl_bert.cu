@@ -114,7 +114,7 @@ static void launch_gemm(cudaStream_t st, const CUtensorMap& tmA, const CUtensorM
         attr_set = true;
     }
     const int tiles = ((g.M + kGemmBM - 1) / kGemmBM) * ((g.N + BN - 1) / BN);
-    blaunch(st, gemm_tc_kernel<BN, EPI>, dim3(std::min(tiles, kNumSMs)), dim3(kGemmThreads), smem, tmA, tmA, tmB, g);
+    blaunch(st, gemm_tc_kernel<BN, EPI>, dim3(std::min(tiles, kNumSMs)), dim3(gemm_threads(BN, DUAL_NONE)), smem, tmA, tmA, tmB, g);
 }
 
 // ---- weights -------------------------------------------------------------------------------------------------------------

@@ -6,6 +6,7 @@
 #include "layered_model.cuh"
 #include "layered_ops.cuh"
 #include "chunk_scan.cuh"
+#include "gemm_dec.cuh"
 #include "gqa_attn_tc.cuh"
 #include "model.cuh"
 #include "synth.cuh"
@@ -912,9 +913,9 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
             y.u_hi.alloc(R * std::max(m.max_u, 1)); y.u_lo.alloc(R * std::max(m.max_u, 1));
             if (m.cfg.token_side > 0) { y.ta_hi.alloc(R * m.cfg.token_side); y.ta_lo.alloc(R * m.cfg.token_side); }
             y.act_hi.alloc(R * std::max(m.max_ff, 1)); y.act_lo.alloc(R * std::max(m.max_ff, 1));
-            // split-K slices of a tensor-core GEMM with <= 128 rows: ks * rows <= 256 (see pick_ksplit)
+            // slices of a tensor-core GEMM with <= 128 rows
             const size_t nmax = std::max<size_t>(std::max<size_t>(std::max(m.max_in, m.max_q), W), std::max<size_t>(std::max<size_t>(2 * (size_t)m.max_ff, m.cfg.token_side), m.V));
-            size_t need = 256 * nmax;
+            size_t need = dec_scratch(128, nmax);
             size_t gx_rows = 0;
             for (const LayeredLayerW& lw : m.layers) {          // grouped expert GEMMs: [slices][experts * cap rows][2 ff | W]
                 if (!lw.tc_moe) continue;
@@ -983,7 +984,7 @@ static Slices gemm_slices(fl_cache& c, LaunchCtx& lc, const char* tag, const flo
     if (R <= 0) return Slices{Y, 1, 0};
     if (!tc || ahi == nullptr) { gemm(lc, tag, A, K, Wt, N, K, Y, N, R); return Slices{Y, 1, 0}; }
     LayeredCache& y = *c.ly;
-    int ks_plan = R <= 128 ? pick_ksplit((N + 127) / 128, (K + 63) / 64, R) : 1;
+    int ks_plan = R <= 128 ? dec_plan(N, K, R).slices : 1;
     if (R > 128) {              // many rows but few output tiles (a narrow matrix): cut K as long as the slices fit the scratch
         const int tiles = ((R + 127) / 128) * ((N + 255) / 256), nk = (K + 63) / 64;
         // (up to eight slices of at least eight k blocks: none of them is empty)

@@ -10,6 +10,7 @@
 #include "decode_persistent.cuh"
 #include "deliver.hpp"
 #include "dense_ops.cuh"
+#include "gemm_dec.cuh"
 #include "gemm_tc.cuh"
 #include "elementwise.cuh"
 #include "gemv.cuh"
@@ -1025,14 +1026,12 @@ static void ensure_dense_ws(fl_cache& c, int rows) {
     d.xhi.alloc(R * kmax); d.xlo.alloc(R * kmax);
     const size_t Rm = w.ep_dp ? R * (size_t)w.ep : R;        // rows the expert GEMMs see
     d.moe_rows = Rm;
-    {   // GEMM output: [ks][rows, N] for the largest N * ks over the model's GEMM shapes at this row count
+    {   // GEMM output: [slices][rows, N] for the largest of the model's GEMM shapes at this row count and those below
         size_t need = Rm * nmax;
-        auto consider = [&](size_t rows, size_t N, size_t K) {
-            const int ks = rows <= 128 ? pick_ksplit((int)((N + 127) / 128), (int)((K + kGemmBK - 1) / kGemmBK), (int)rows) : 1;
-            need = std::max(need, rows * N * (size_t)ks);
+        auto consider = [&](size_t rows, size_t N) {
+            need = std::max(need, std::max(rows * N, dec_scratch(std::min<size_t>(rows, 128), N)));
         };
-        consider(R, w.nqkv, w.H); consider(R, w.H, nq); consider(R, w.V, w.H);
-        consider(Rm, 2 * (size_t)w.I, w.H); consider(Rm, w.H, w.I);
+        consider(R, w.nqkv); consider(R, w.H); consider(R, w.V); consider(Rm, 2 * (size_t)w.I); consider(Rm, w.H);
         if (w.cfg.arch == FL_ARCH_MIXTRAL) {      // grouped expert GEMMs: E_local stacked matrices x one block of `cap` rows each
             for (size_t cap = 16; cap <= (size_t)moe_group_cap((int)std::min<size_t>(Rm, 128)); cap *= 2) {
                 const size_t Rg = (size_t)w.E_local * cap;
@@ -1043,7 +1042,6 @@ static void ensure_dense_ws(fl_cache& c, int rows) {
                 }
             }
         }
-        for (size_t r = 1; r <= std::min<size_t>(R, kMaxBatch); ++r) consider(r, w.V, w.H);     // the lm_head runs on one row per sequence
         d.y.alloc(need);
     }
     d.resid.alloc(R * w.H); d.q.alloc(R * nq);      // the attention output goes straight into xhi / xlo (hi/lo operand of o_proj)
@@ -1086,7 +1084,7 @@ static void launch_gemm_tc(cudaStream_t st, bool pdl, int items, const CUtensorM
     }
     cudaLaunchConfig_t cfg{};
     cfg.gridDim = dim3(std::min(items, kNumSMs));
-    cfg.blockDim = dim3(kGemmThreads);
+    cfg.blockDim = dim3(gemm_threads(BN, DUAL));
     cfg.dynamicSmemBytes = smem;
     cfg.stream = st;
     cudaLaunchAttribute attr[1];
@@ -1099,7 +1097,29 @@ static void launch_gemm_tc(cudaStream_t st, bool pdl, int items, const CUtensorM
     FL_CUDA(cudaLaunchKernelEx(&cfg, gemm_tc_kernel<BN, EPI, DUAL>, a, a2, b, g));
 }
 
-// Split-K factor of a swap-AB (decode) GEMM: the one whose work items (output tiles x k slices) fill whole waves of the 148
+template <int BN>
+static void launch_gemm_dec(cudaStream_t st, bool pdl, int ctas, const CUtensorMap& w, const CUtensorMap& hi, const CUtensorMap& lo, const DecArgs& g) {
+    static bool attr_set = false;
+    if (!attr_set) {
+        FL_CUDA(cudaFuncSetAttribute(gemm_dec_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)DecShape<BN>::kSmem));
+        attr_set = true;
+    }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(ctas);
+    cfg.blockDim = dim3(DecShape<BN>::kThreads);
+    cfg.dynamicSmemBytes = DecShape<BN>::kSmem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    if (pdl) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    FL_CUDA(cudaLaunchKernelEx(&cfg, gemm_dec_kernel<BN>, w, hi, lo, g));
+}
+
+// Split-K factor of a grouped swap-AB (decode) GEMM: the one whose work items (output tiles x k slices) fill whole waves of the 148
 // persistent CTAs best, counting the padding of the last k slice; fewer, longer items win ties (pipeline fill / epilogue per item).
 // The consumer sums the slices in a fixed order, so a row's bytes read grow with ks: capped by the row count.
 int pick_ksplit(int tiles, int nk, int R) {
@@ -1118,20 +1138,19 @@ int pick_ksplit(int tiles, int nk, int R) {
 
 // out[ks][R, N] (f32, row stride N, slice stride R*N) = (xhi + xlo)[R, K] . W[N, K]^T; returns the number of split-K slices,
 // which the consumer kernel sums in a fixed order (deterministic, no atomics, no memset).
-//   R <= 128 (decode batches, short prefills): swap-AB -- the weights are the 128-row MMA operand, the activations a tiny
-//             N = R tile, the result is stored transposed; the only large shared-memory traffic is the weight stream.
+//   R <= 128 (decode batches, short prefills): gemm_dec_kernel.  W has to be constant: it is read ahead of the kernels before this one.
 //   R  > 128 (prefill): tokens are the M dimension, 128 x 128 output tiles.
 int dense_gemm(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int N, int K, const CUtensorMap& tmW, float* out,
                const uint16_t* xhi, const uint16_t* xlo, uint16_t* silu_hi, uint16_t* silu_lo, int prefill_ks) {
     if (!xhi) { xhi = c.dw.xhi.p; xlo = c.dw.xlo.p; }
-    const int nk = (K + kGemmBK - 1) / kGemmBK;
     const bool swap = R <= 128;
     // prefill: 128 tokens x 256 weight rows per tile.  The hi/lo activation pair makes a k-block 2 x 16 KB of A next to the weight
     // tile, and the GEMM is bound by the shared-memory fill rate (L2 -> SM), not by the tensor pipe: a 256-row weight tile is
     // 64 KB per 2 x 128 x 256 x 64 MACs where the 128-row one is 48 KB per half of that -- 1.5x the arithmetic per staged byte.
     static const int prefill_bn = env_flag("FL_PREFILL_BN128") ? 128 : 256;      // dev knob: the 128-row tile of round 1
-    const int tiles = swap ? (N + 127) / 128 : ((R + kGemmBM - 1) / kGemmBM) * ((N + prefill_bn - 1) / prefill_bn);
-    const int ks = swap ? pick_ksplit(tiles, nk, R) : (silu_hi != nullptr ? 1 : prefill_ks);
+    const int tiles = ((R + kGemmBM - 1) / kGemmBM) * ((N + prefill_bn - 1) / prefill_bn);
+    const DecPlan dec = swap ? dec_plan(N, K, R) : DecPlan{};
+    const int ks = swap ? dec.slices : (silu_hi != nullptr ? 1 : prefill_ks);
     ProfEntry pe;
     const bool prof = g_prof.on && !lc.capturing;
     const bool pdl = lc.pdl && !prof;
@@ -1143,16 +1162,14 @@ int dense_gemm(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int N, int K,
         FL_CUDA(cudaEventRecord(pe.e0, lc.stream));
     }
     if (swap) {
-        const int bn = R <= 16 ? 16 : (R <= 32 ? 32 : (R <= 64 ? 64 : 128));
+        const int bn = dec_bn(R);
         const CUtensorMap hi = make_tmap_bf16(xhi, R, K, K, bn), lo = make_tmap_bf16(xlo, R, K, K, bn);
-        GemmArgs g{N, R, K, nullptr, nullptr, 0, out, N, ks, (long long)R * N};     // M = weight rows, N = activation rows
-        static const bool w_prefetch = env_flag("FL_GEMM_WPREFETCH");     // experimental: not yet measured on a GPU
-        g.w_prefetch = (w_prefetch && pdl) ? 1 : 0;
+        const DecArgs g{N, R, K, out, (long long)R * N, dec.nks, dec.L, dec.slices};
         switch (bn) {
-            case 16: launch_gemm_tc<16, GEPI_F32_T, DUAL_B>(lc.stream, pdl, tiles * ks, tmW, hi, lo, g); break;
-            case 32: launch_gemm_tc<32, GEPI_F32_T, DUAL_B>(lc.stream, pdl, tiles * ks, tmW, hi, lo, g); break;
-            case 64: launch_gemm_tc<64, GEPI_F32_T, DUAL_B>(lc.stream, pdl, tiles * ks, tmW, hi, lo, g); break;
-            default: launch_gemm_tc<128, GEPI_F32_T, DUAL_B>(lc.stream, pdl, tiles * ks, tmW, hi, lo, g); break;
+            case 16: launch_gemm_dec<16>(lc.stream, pdl, dec.ctas, tmW, hi, lo, g); break;
+            case 32: launch_gemm_dec<32>(lc.stream, pdl, dec.ctas, tmW, hi, lo, g); break;
+            case 64: launch_gemm_dec<64>(lc.stream, pdl, dec.ctas, tmW, hi, lo, g); break;
+            default: launch_gemm_dec<128>(lc.stream, pdl, dec.ctas, tmW, hi, lo, g); break;
         }
     } else {
         const CUtensorMap hi = make_tmap_bf16(xhi, R, K, K, kGemmBM), lo = make_tmap_bf16(xlo, R, K, K, kGemmBM);
@@ -1237,6 +1254,7 @@ void dense_gemm_blocks(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int b
     if (swap) {
         const int bn = R <= 16 ? 16 : (R <= 32 ? 32 : (R <= 64 ? 64 : 128)), tiles = blocks * ((N + 127) / 128);
         const CUtensorMap hi = make_tmap_bf16(xhi, R, KX, KX, bn), lo = make_tmap_bf16(xlo, R, KX, KX, bn);
+        g.w_prefetch = pdl ? 1 : 0;
         switch (bn) {
             case 16: launch_gemm_tc<16, GEPI_HL_T, DUAL_B>(lc.stream, pdl, tiles, tmW, hi, lo, g); break;
             case 32: launch_gemm_tc<32, GEPI_HL_T, DUAL_B>(lc.stream, pdl, tiles, tmW, hi, lo, g); break;
@@ -1309,17 +1327,14 @@ static void enqueue_forward_dense(fl_cache& c, LaunchCtx& lc, int b, int t, bool
 
     auto prep = [&](const char* tag, PrepArgs pa, int rows_out) {
         pa.xhi = d.xhi.p; pa.xlo = d.xlo.p; pa.eps = w.cfg.norm_eps; pa.t = t;
-        // many rows (prefill): the register-resident 256-thread kernel (dense_prep_rows_kernel); FL_PREP_ROWS=0 keeps the one-CTA-per-row kernel
+        // rows that fit a block's registers: one pass over memory (dense_prep_rows_kernel); FL_PREP_ROWS=0 keeps the loop kernel
         static const bool rows_kernel = !std::getenv("FL_PREP_ROWS") || std::atoi(std::getenv("FL_PREP_ROWS")) != 0;
-        if (rows_kernel && rows_out >= 512 && pa.norm_w != nullptr && pa.embed == nullptr && pa.K <= 8192 && pa.K % 4 == 0) {
-            if (pa.K <= 4096)
-                launch(lc, tag, 0, dense_prep_rows_kernel<4>, dim3(rows_out), dim3(kPrepRowsThreads), 0, pa);
-            else
-                launch(lc, tag, 0, dense_prep_rows_kernel<8>, dim3(rows_out), dim3(kPrepRowsThreads), 0, pa);
-            return;
-        }
-        const int threads = std::min(1024, std::max(32, (pa.K / 4 + 31) / 32 * 32));
-        launch(lc, tag, 0, dense_prep_kernel, dim3(rows_out), dim3(threads), 0, pa);
+        auto go = [&](auto kern, int threads) { launch(lc, tag, 0, kern, dim3(rows_out), dim3(threads), 0, pa); };
+        if (!rows_kernel || pa.K > 8192 || pa.K % 4 != 0) go(dense_prep_kernel, std::min(1024, std::max(32, (pa.K / 4 + 31) / 32 * 32)));
+        else if (rows_out >= 512) { if (pa.K <= 4096) go(dense_prep_rows_kernel<4, 256>, 256); else go(dense_prep_rows_kernel<8, 256>, 256); }
+        else if (pa.K <= 2048) go(dense_prep_rows_kernel<1, 512>, 512);
+        else if (pa.K <= 4096) go(dense_prep_rows_kernel<2, 512>, 512);
+        else go(dense_prep_rows_kernel<4, 512>, 512);
     };
     {   // K1 + K2 of layer 0
         PrepArgs pa{};
@@ -1413,7 +1428,7 @@ static void enqueue_forward_dense(fl_cache& c, LaunchCtx& lc, int b, int t, bool
                 launch(lc, "moe_gather", 0, moe_gather_kernel, dim3(w.E_local, std::max(1, std::min(Rm, 2 * kNumSMs / w.E_local))), dim3(256), 0, ga);
                 int ke = dense_gemm_grouped(c, lc, "gemm_tc_moe_w13", w.E_local, cap, 2 * w.I, w.H, lw.tm_ewgu_all, d.y.p, d.gx_hi.p, d.gx_lo.p,
                                             d.grp_cnt.p);
-                launch(lc, "dense_silu_split", 0, dense_silu_split_kernel, dim3((w.I + 255) / 256, Rg), dim3(256), 0, (const float*)d.y.p, ke,
+                launch(lc, "dense_silu_split", 0, dense_silu_split_kernel, dim3((w.I + 1023) / 1024, w.E_local * kSiluGroupRows), dim3(256), 0, (const float*)d.y.p, ke,
                        (long long)Rg * 2 * w.I, w.I, d.xhi2.p, d.xlo2.p, (const int*)d.grp_cnt.p, cap);
                 ke = dense_gemm_grouped(c, lc, "gemm_tc_moe_w2", w.E_local, cap, w.H, w.I, lw.tm_ewdown_all, d.y.p, d.xhi2.p, d.xlo2.p, d.grp_cnt.p);
                 launch(lc, "moe_combine", 0, moe_combine_kernel, dim3((w.H + 255) / 256, Rm), dim3(256), 0, (const float*)d.y.p, ke,
@@ -1422,7 +1437,7 @@ static void enqueue_forward_dense(fl_cache& c, LaunchCtx& lc, int b, int t, bool
             for (int j = 0; j < w.E_local; ++j) {
                 const int e = w.rank * w.E_local + j;
                 int ke = dense_gemm(c, lc, "gemm_tc_moe_w13", Rm, 2 * w.I, w.H, lw.tm_ewgu[j], d.y.p, ex_hi, ex_lo);
-                launch(lc, "dense_silu_split", 0, dense_silu_split_kernel, dim3((w.I + 255) / 256, Rm), dim3(256), 0, (const float*)d.y.p, ke,
+                launch(lc, "dense_silu_split", 0, dense_silu_split_kernel, dim3((w.I + 1023) / 1024, Rm), dim3(256), 0, (const float*)d.y.p, ke,
                        (long long)Rm * 2 * w.I, w.I, d.xhi2.p, d.xlo2.p, (const int*)nullptr, 0);
                 ke = dense_gemm(c, lc, "gemm_tc_moe_w2", Rm, w.H, w.I, lw.tm_ewdown[j], d.y.p, d.xhi2.p, d.xlo2.p);
                 launch(lc, "moe_accum", 0, moe_accum_kernel, dim3((w.H + 255) / 256, Rm), dim3(256), 0, (const float*)d.y.p, ke,
@@ -1446,7 +1461,7 @@ static void enqueue_forward_dense(fl_cache& c, LaunchCtx& lc, int b, int t, bool
                 ks = dense_gemm(c, lc, "gemm_tc_down", R, w.H, w.I, lw.tm_wdown, d.y.p, d.xhi2.p, d.xlo2.p);
             } else {
                 ks = dense_gemm(c, lc, "gemm_tc_gateup", R, 2 * w.I, w.H, lw.tm_wgu, d.y.p);
-                launch(lc, "dense_silu_split", 0, dense_silu_split_kernel, dim3((w.I + 255) / 256, R), dim3(256), 0, (const float*)d.y.p, ks,
+                launch(lc, "dense_silu_split", 0, dense_silu_split_kernel, dim3((w.I + 1023) / 1024, R), dim3(256), 0, (const float*)d.y.p, ks,
                        (long long)R * 2 * w.I, w.I, d.xhi.p, d.xlo.p, (const int*)nullptr, 0);
                 ks = dense_gemm(c, lc, "gemm_tc_down", R, w.H, w.I, lw.tm_wdown, d.y.p);
             }

@@ -25,7 +25,11 @@ enum : int { DUAL_NONE = 0, DUAL_A = 1, DUAL_B = 2 };
 constexpr int kGemmBM = 128;
 constexpr int kGemmBK = 64;          // 64 bf16 = 128 bytes = one swizzle row
 constexpr int kGemmEpiWarps = 16;      // four per TMEM lane quarter; each takes BN/4 columns of the tile
-constexpr int kGemmThreads = 64 + 32 * kGemmEpiWarps;
+// Epilogue warps of a kernel: the swap-AB tiles are BN columns of 32-column chunks, and warps without a chunk would only hold registers that
+// the blocks of the neighbouring kernels could use (576 threads x 72..96 registers left no room for an element-wise block of 1024 threads, nor
+// for the next GEMM beside one: the SMs under such blocks entered every GEMM late and nothing could be fetched ahead, see w_prefetch).
+__host__ __device__ constexpr int gemm_epi_warps(int BN, int dual) { return dual != 2 ? kGemmEpiWarps : BN <= 32 ? 4 : BN <= 64 ? 8 : 16; }
+__host__ __device__ constexpr int gemm_threads(int BN, int dual) { return 64 + 32 * gemm_epi_warps(BN, dual); }
 
 // Row tiles that share a weight tile in the tile walk of the many-row GEMMs (GemmArgs.raster_m).  148 CTAs then work on about 16 row tiles
 // x 9 weight tiles at a time: 25 x 512 K bytes of operands (128 hi | lo rows weigh what 256 weight rows do), close to the least a wave can
@@ -206,10 +210,11 @@ __device__ __forceinline__ float gelu_tanh_f(float x) {
 //           large tile), B = activations [rows <= BN, K] (hi, lo); D[out, rows] is stored transposed (GEPI_F32_T) so that
 //           a warp writes 32 consecutive floats of one activation row.
 template <int BN, int EPI, int DUAL = DUAL_NONE>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(gemm_threads(BN, DUAL), 1)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmA2, const __grid_constant__ CUtensorMap tmB,
                const GemmArgs g) {
     static_assert(BN % 16 == 0 && BN >= 16 && BN <= 256, "UMMA N for M=128 must be a multiple of 16 in [16, 256]");
+    constexpr int kEpiWarps = gemm_epi_warps(BN, DUAL);
     constexpr uint32_t kABytes = kGemmBM * kGemmBK * 2;   // 16 KB
     constexpr uint32_t kBBytes = BN * kGemmBK * 2;
     constexpr uint32_t kStageBytes = (DUAL == DUAL_A ? 2 : 1) * kABytes + (DUAL == DUAL_B ? 2 : 1) * kBBytes;
@@ -294,7 +299,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         }
         for (int s = 0; s < 2; ++s) {
             mbar_init(&acc_full[s], 1);
-            mbar_init(&acc_empty[s], kGemmEpiWarps);      // one arrive per epilogue warp
+            mbar_init(&acc_empty[s], kEpiWarps);      // one arrive per epilogue warp
         }
         mbar_fence_init();
         tma_prefetch_desc(&tmA);
@@ -320,7 +325,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             if (DUAL == DUAL_B && g.w_prefetch) {
                 for (int item = blockIdx.x; item < nitems && pre < (uint32_t)kStages; item += gridDim.x) {
                     const int tile = item / ksplit, ks = item % ksplit;
-                    const int m0 = (tile / nt) * kGemmBM;
+                    int m0, n0, grp, mrow0;
+                    coords(tile, m0, n0, grp, mrow0);
                     const int kb1 = min((ks + 1) * nkps, nk);
                     for (int kb = ks * nkps; kb < kb1 && pre < (uint32_t)kStages; ++kb, ++pre) {
                         mbar_expect_tx(&full[pre], kStageBytes);
@@ -343,8 +349,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     const int st = c % kStages;
                     uint8_t* sa = gsm + (size_t)st * kStageBytes;
                     if (DUAL == DUAL_B && c < pre) {       // weight tile already on its way; complete the stage with the activations
-                        tma_load_2d(sa + kBOff, &tmA2, kb * kGemmBK, n0, &full[st]);
-                        tma_load_2d(sa + kBOff + kBBytes, &tmB, kb * kGemmBK, n0, &full[st]);
+                        tma_load_2d(sa + kBOff, &tmA2, ax + kb * kGemmBK, n0, &full[st]);
+                        tma_load_2d(sa + kBOff + kBBytes, &tmB, ax + kb * kGemmBK, n0, &full[st]);
                         continue;
                     }
                     mbar_wait(&empty[st], ((c / kStages) & 1) ^ 1);
@@ -401,7 +407,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
         }
     } else {
-        // ===== epilogue: warps 2..17; TMEM lane quarter = warp % 4 (hardware rule), column slice = (warp - 2) / 4; thread == output row =====
+        // ===== epilogue: the other warps; TMEM lane quarter = warp % 4 (hardware rule), column slice = (warp - 2) / 4; thread == output row =====
         const int q = warp & 3;
         const int cslice = (warp - 2) >> 2;
         uint32_t ti = 0;
@@ -424,7 +430,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             mbar_wait(&acc_full[as], (ti_now >> 1) & 1);
             tc_fence_after();
 #pragma unroll 1
-            for (int c0 = cslice * 32; c0 < kBNOut; c0 += 128) {  // 32-column chunks dealt round-robin to the 4 warps of a lane quarter
+            for (int c0 = cslice * 32; c0 < kBNOut; c0 += 8 * kEpiWarps) {  // 32-column chunks dealt round-robin to the warps of a lane quarter
                 if constexpr (EPI == GEPI_GLU_HL) {
                     // 16 columns at a time: accumulator columns [0, 128) hold gate rows, [128, 256) the up rows of the same outputs
 #pragma unroll 1

@@ -169,7 +169,8 @@ struct fl_cache {
 namespace fl {
 // The dense tensor-core GEMM of fl_lib.cu (tcgen05 / TMEM / TMA, hi|lo activation halves), shared with the layered decoder:
 // out[ks][R, N] (f32, row stride N, slice stride R * N) = (xhi + xlo)[R, K] . W[N, K]^T; returns the number of split-K slices
-// (R <= 128: pick_ksplit of the weight tiles; R > 128: prefill_ks, one unless the caller asks for more), which the consumer sums in a fixed order.
+// (R <= 128: dec_plan's, and W is constant: it is read ahead of the kernels before; R > 128: prefill_ks, one unless the caller asks for more), which
+// the consumer sums in a fixed order.
 int pick_ksplit(int tiles, int nk, int R);
 int dense_gemm(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int N, int K, const CUtensorMap& tmW, float* out,
                const uint16_t* xhi = nullptr, const uint16_t* xlo = nullptr, uint16_t* silu_hi = nullptr, uint16_t* silu_lo = nullptr,
