@@ -102,7 +102,11 @@ struct SkArgs {
     int layer_row0;       // row of this layer's page 0 / kv head 0 in the pool-wide tensor maps
 };
 
-template <int D>
+// PAIR (query groups of up to 8 heads): the hi halves of the heads are rows 0-7 of the products' 16, the lo halves rows 8-15, of q and of the
+// probabilities alike, so one MMA multiplies both and a thread holds a head's two sums in one fragment.  With the halves as two tiles, of which
+// the heads above the group were zeros, the warps' MMAs and exponentials were the limit, not HBM: 64 sequences of 512 to 2048 tokens, 8 key/value
+// heads of 128 channels (335 MB per layer): 81 -> 74 us.
+template <int D, bool PAIR>
 __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constant__ CUtensorMap tmv,
                                                                     const SkArgs k) {
     const AttnArgs& a = k.a;
@@ -119,10 +123,10 @@ __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid
     uint16_t* ring = reinterpret_cast<uint16_t*>(sksm + ((front + 1023) & ~1023));
     __shared__ __align__(8) uint64_t full[kSkMaxStages];
     __shared__ __align__(8) uint64_t empty[kSkMaxStages];
-    __shared__ float red_m[NW][16], red_l[NW][16], mrg_w[NW][16], mrg_den[16], mrg_star[16];
+    __shared__ float red_m[NW][16], red_l[NW][16], mrg_w[NW][16], mrg_den[16];
     __shared__ int prefix[kMaxBatch + 1];        // pages of the sequences before s
     __shared__ int s_len[kMaxBatch], s_slot[kMaxBatch];
-    __shared__ int s_last, s_i0, s_i1;
+    __shared__ int s_last[2], s_i0[2], s_i1[2];
 
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, g = lane >> 2, tq = lane & 3;
     const int NST = k.nstages;
@@ -235,6 +239,7 @@ __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid
     float o[D / 8][4];
     float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
     bool open = false, from_start = false;
+    int end_s = -1, end_h = 0, on_s = -1, on_h = 0;        // pairs of which this CTA holds a part: the one that ends here, the one that goes on
     unsigned int c = 0;
     for (long long n = flat0; n < flat1; ++n, ++c) {
         const int np = prefix[s + 1] - prefix[s], len = s_len[s];
@@ -242,8 +247,16 @@ __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid
             csync();       // the previous pair's readers of the merge scratch are done
             for (int i = tid; i < 16 * D; i += kSkConsumers) {
                 const int hh = i / D, dd = i % D;
-                const float q = hh < n_rep ? a.q[((size_t)s * a.nh + h * n_rep + hh) * D + dd] : 0.f;
-                store_hi_lo(qhi, qlo, swz<D>(hh, dd), q);
+                if constexpr (PAIR) {
+                    if (hh >= 8) break;
+                    const float q = hh < n_rep ? a.q[((size_t)s * a.nh + h * n_rep + hh) * D + dd] : 0.f;
+                    const uint16_t hi = f32_to_bf16_rne(q);
+                    qhi[swz<D>(hh, dd)] = hi;
+                    qhi[swz<D>(hh + 8, dd)] = f32_to_bf16_rne(q - __uint_as_float((uint32_t)hi << 16));
+                } else {
+                    const float q = hh < n_rep ? a.q[((size_t)s * a.nh + h * n_rep + hh) * D + dd] : 0.f;
+                    store_hi_lo(qhi, qlo, swz<D>(hh, dd), q);
+                }
             }
             csync();
 #pragma unroll
@@ -264,44 +277,64 @@ __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid
             for (int ks = 0; ks < D / 16; ++ks) {
                 uint32_t ah[4], al[4], kb[4];
                 ldmatrix_x4(ah, qhi + swz<D>(lane & 15, ks * 16 + (lane >> 4) * 8));
-                ldmatrix_x4(al, qlo + swz<D>(lane & 15, ks * 16 + (lane >> 4) * 8));
+                if (!PAIR) ldmatrix_x4(al, qlo + swz<D>(lane & 15, ks * 16 + (lane >> 4) * 8));
                 ldmatrix_x4(kb, kt + kv_off<D>(warp * 16 + (lane & 7) + ((lane >> 4) << 3), ks * 16 + ((lane >> 3) & 1) * 8));
                 mma_bf16_16816(sc[0], ah, kb[0], kb[1]);
-                mma_bf16_16816(sc[0], al, kb[0], kb[1]);
+                if (!PAIR) mma_bf16_16816(sc[0], al, kb[0], kb[1]);
                 mma_bf16_16816(sc[1], ah, kb[2], kb[3]);
-                mma_bf16_16816(sc[1], al, kb[2], kb[3]);
+                if (!PAIR) mma_bf16_16816(sc[1], al, kb[2], kb[3]);
+            }
+            constexpr int EV = PAIR ? 2 : 4;       // scores of a fragment
+            if constexpr (PAIR) {
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) { sc[nt][0] += sc[nt][2]; sc[nt][1] += sc[nt][3]; }
             }
             float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-                for (int e = 0; e < 4; ++e) {
+                for (int e = 0; e < EV; ++e) {
                     const int key = key0 + nt * 8 + tq * 2 + (e & 1);
                     sc[nt][e] = key < len ? sc[nt][e] * a.qscale : -INFINITY;
                     if (e < 2) mx0 = fmaxf(mx0, sc[nt][e]); else mx1 = fmaxf(mx1, sc[nt][e]);
                 }
             mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, 2));
-            mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 2));
-            const float mn0 = fmaxf(m0, mx0), mn1 = fmaxf(m1, mx1);       // finite: key0 < len is valid for every row
-            const float al0 = expf(m0 - mn0), al1 = expf(m1 - mn1);
-            m0 = mn0; m1 = mn1;
-            float ps0 = 0.f, ps1 = 0.f;
-#pragma unroll
-            for (int nt = 0; nt < 2; ++nt) {
-                sc[nt][0] = expf(sc[nt][0] - mn0); sc[nt][1] = expf(sc[nt][1] - mn0);
-                sc[nt][2] = expf(sc[nt][2] - mn1); sc[nt][3] = expf(sc[nt][3] - mn1);
-                ps0 += sc[nt][0] + sc[nt][1];
-                ps1 += sc[nt][2] + sc[nt][3];
-            }
-            l0 = l0 * al0 + ps0;       // per-thread partial row sums; the quad is reduced when the pair is emitted
-            l1 = l1 * al1 + ps1;
+            const float mn0 = fmaxf(m0, mx0);       // finite: key0 < len is valid for every row
+            const float al0 = expf(m0 - mn0);
+            m0 = mn0;
+            float al1 = al0, ps0 = 0.f;
             uint32_t ph[4], pl[4];
-            ph[0] = pack_bf16x2(sc[0][0], sc[0][1]); ph[1] = pack_bf16x2(sc[0][2], sc[0][3]);
-            ph[2] = pack_bf16x2(sc[1][0], sc[1][1]); ph[3] = pack_bf16x2(sc[1][2], sc[1][3]);
-            pl[0] = pack_bf16x2(sc[0][0] - bf16lo(ph[0]), sc[0][1] - bf16hi(ph[0]));
-            pl[1] = pack_bf16x2(sc[0][2] - bf16lo(ph[1]), sc[0][3] - bf16hi(ph[1]));
-            pl[2] = pack_bf16x2(sc[1][0] - bf16lo(ph[2]), sc[1][1] - bf16hi(ph[2]));
-            pl[3] = pack_bf16x2(sc[1][2] - bf16lo(ph[3]), sc[1][3] - bf16hi(ph[3]));
+            if constexpr (PAIR) {
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+                    sc[nt][0] = expf(sc[nt][0] - mn0); sc[nt][1] = expf(sc[nt][1] - mn0);
+                    ps0 += sc[nt][0] + sc[nt][1];
+                    ph[2 * nt] = pack_bf16x2(sc[nt][0], sc[nt][1]);
+                    ph[2 * nt + 1] = pack_bf16x2(sc[nt][0] - bf16lo(ph[2 * nt]), sc[nt][1] - bf16hi(ph[2 * nt]));
+                }
+                l0 = l0 * al0 + ps0;       // per-thread partial row sums; the quad is reduced when the pair is emitted
+            } else {
+                mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 2));
+                const float mn1 = fmaxf(m1, mx1);
+                al1 = expf(m1 - mn1);
+                m1 = mn1;
+                float ps1 = 0.f;
+#pragma unroll
+                for (int nt = 0; nt < 2; ++nt) {
+                    sc[nt][0] = expf(sc[nt][0] - mn0); sc[nt][1] = expf(sc[nt][1] - mn0);
+                    sc[nt][2] = expf(sc[nt][2] - mn1); sc[nt][3] = expf(sc[nt][3] - mn1);
+                    ps0 += sc[nt][0] + sc[nt][1];
+                    ps1 += sc[nt][2] + sc[nt][3];
+                }
+                l0 = l0 * al0 + ps0;
+                l1 = l1 * al1 + ps1;
+                ph[0] = pack_bf16x2(sc[0][0], sc[0][1]); ph[1] = pack_bf16x2(sc[0][2], sc[0][3]);
+                ph[2] = pack_bf16x2(sc[1][0], sc[1][1]); ph[3] = pack_bf16x2(sc[1][2], sc[1][3]);
+                pl[0] = pack_bf16x2(sc[0][0] - bf16lo(ph[0]), sc[0][1] - bf16hi(ph[0]));
+                pl[1] = pack_bf16x2(sc[0][2] - bf16lo(ph[1]), sc[0][3] - bf16hi(ph[1]));
+                pl[2] = pack_bf16x2(sc[1][0] - bf16lo(ph[2]), sc[1][1] - bf16hi(ph[2]));
+                pl[3] = pack_bf16x2(sc[1][2] - bf16lo(ph[3]), sc[1][3] - bf16hi(ph[3]));
+            }
 #pragma unroll
             for (int dt = 0; dt < D / 16; ++dt) {
                 uint32_t vb[4];
@@ -311,9 +344,9 @@ __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid
                 oa[0] *= al0; oa[1] *= al0; oa[2] *= al1; oa[3] *= al1;
                 ob[0] *= al0; ob[1] *= al0; ob[2] *= al1; ob[3] *= al1;
                 mma_bf16_16816(oa, ph, vb[0], vb[1]);
-                mma_bf16_16816(oa, pl, vb[0], vb[1]);
+                if (!PAIR) mma_bf16_16816(oa, pl, vb[0], vb[1]);
                 mma_bf16_16816(ob, ph, vb[2], vb[3]);
-                mma_bf16_16816(ob, pl, vb[2], vb[3]);
+                if (!PAIR) mma_bf16_16816(ob, pl, vb[2], vb[3]);
             }
         }
         __syncwarp();
@@ -324,20 +357,23 @@ __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid
             // ---- emit: merge the 4 warps (each saw a different quarter of every page) ----
             const bool whole = from_start && pair_done;       // nobody else holds a piece of this pair
             l0 += __shfl_xor_sync(0xFFFFFFFFu, l0, 1); l0 += __shfl_xor_sync(0xFFFFFFFFu, l0, 2);
-            l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, 1); l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, 2);
+            if (!PAIR) { l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, 1); l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, 2); }
             csync();       // every warp is past its last read of the q tiles (the scratch overlays them)
             if (tq == 0) {
-                red_m[warp][g] = m0; red_m[warp][g + 8] = m1;
-                red_l[warp][g] = l0; red_l[warp][g + 8] = l1;
+                red_m[warp][g] = m0;
+                red_l[warp][g] = l0;
+                if (!PAIR) { red_m[warp][g + 8] = m1; red_l[warp][g + 8] = l1; }
             }
 #pragma unroll
             for (int nt = 0; nt < D / 8; ++nt) {
-                if (g < n_rep) *reinterpret_cast<float2*>(red_o + ((size_t)warp * n_rep + g) * D + nt * 8 + tq * 2) = make_float2(o[nt][0], o[nt][1]);
-                if (g + 8 < n_rep) *reinterpret_cast<float2*>(red_o + ((size_t)warp * n_rep + g + 8) * D + nt * 8 + tq * 2) = make_float2(o[nt][2], o[nt][3]);
+                if (g < n_rep)
+                    *reinterpret_cast<float2*>(red_o + ((size_t)warp * n_rep + g) * D + nt * 8 + tq * 2) =
+                        PAIR ? make_float2(o[nt][0] + o[nt][2], o[nt][1] + o[nt][3]) : make_float2(o[nt][0], o[nt][1]);
+                if (!PAIR && g + 8 < n_rep) *reinterpret_cast<float2*>(red_o + ((size_t)warp * n_rep + g + 8) * D + nt * 8 + tq * 2) = make_float2(o[nt][2], o[nt][3]);
             }
             csync();
             const int part = cta * 2 + (from_start ? 1 : 0);      // this CTA's partial slot for the pair
-            if (tid < 16) {
+            if (tid < (PAIR ? 8 : 16)) {
                 float ms = -INFINITY;
 #pragma unroll
                 for (int w = 0; w < NW; ++w) ms = fmaxf(ms, red_m[w][tid]);
@@ -372,59 +408,74 @@ __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid
                     *reinterpret_cast<float2*>(k.sk_acc + ((size_t)part * n_rep + hh) * D + cc) = make_float2(x0, x1);
                 }
             }
-            if (!whole) {
-                // ---- the pair straddles ranges: the last CTA to arrive merges the partials in CTA order ----
-                __threadfence();
-                csync();
-                if (tid == 0) {
-                    const long long ps = (long long)a.nkv * prefix[s] + (long long)h * np, pe = ps + np;
-                    const int i0 = (int)(((ps + 1) * G - 1) / P), i1 = (int)((pe * G - 1) / P);      // CTAs holding the first / last page
-                    const int ticket = atomicAdd(&a.counters[s * a.nkv + h], 1);
-                    s_last = (ticket == i1 - i0);
-                    s_i0 = i0;
-                    s_i1 = i1;
-                }
-                csync();
-                if (s_last) {
-                    __threadfence();
-                    const int i0 = s_i0, i1 = s_i1;
-                    // partial of CTA j: slot 1 in the CTA where the pair starts (i0), slot 0 in the others
-                    for (int hh = warp; hh < n_rep; hh += NW) {
-                        float mstar = -INFINITY;
-                        for (int j = i0 + lane; j <= i1; j += 32)
-                            mstar = fmaxf(mstar, __ldcg(k.sk_ml + ((size_t)(j * 2 + (j == i0)) * n_rep + hh) * 2));
-                        mstar = warp_max(mstar);
-                        float den = 0.f;
-                        for (int j = i0 + lane; j <= i1; j += 32) {
-                            const float* ml = k.sk_ml + ((size_t)(j * 2 + (j == i0)) * n_rep + hh) * 2;
-                            den = fmaf(expf(__ldcg(ml) - mstar), __ldcg(ml + 1), den);
-                        }
-                        den = warp_sum(den);
-                        if (lane == 0) { mrg_star[hh] = mstar; mrg_den[hh] = den; }
-                    }
-                    csync();
-                    for (int i = tid; i < n_rep * (D / 2); i += kSkConsumers) {
-                        const int hh = i / (D / 2), cc = (i % (D / 2)) * 2;
-                        float x0 = 0.f, x1 = 0.f;
-                        for (int j = i0; j <= i1; ++j) {
-                            const size_t pj = (size_t)(j * 2 + (j == i0)) * n_rep + hh;
-                            const float w = expf(__ldcg(k.sk_ml + pj * 2) - mrg_star[hh]);
-                            const float2 v = __ldcg(reinterpret_cast<const float2*>(k.sk_acc + pj * D + cc));
-                            x0 = fmaf(w, v.x, x0);
-                            x1 = fmaf(w, v.y, x1);
-                        }
-                        const float den = mrg_den[hh];
-                        store_out2(a, (size_t)s * a.nh * D + (size_t)(h * n_rep + hh) * D + cc, x0 / den, x1 / den);
-                    }
-                    if (tid == 0) a.counters[s * a.nkv + h] = 0;
-                }
-            }
+            if (!whole && pair_done) { end_s = s; end_h = h; }
+            if (!whole && !pair_done) { on_s = s; on_h = h; }
             open = false;
         }
         if (++p == np) {
             p = 0;
             if (++h == a.nkv) { h = 0; ++s; }
         }
+    }
+
+    // ---- pairs that straddle ranges (at most this CTA's first and its last): the last CTA to arrive merges the partials in CTA order.  Both
+    // wait for the end of the range: a ticket costs 2 us of round trips, which held up the pages behind it (8 sequences of 2048 tokens: the
+    // last page came 4 us after the median block's). ----
+    if (end_s < 0 && on_s < 0) return;
+    csync();                                       // every partial is written
+    if (lane == 0 && warp < 2 && (warp == 0 ? end_s : on_s) >= 0) {
+        const int ss = warp == 0 ? end_s : on_s, sh = warp == 0 ? end_h : on_h, np = prefix[ss + 1] - prefix[ss];
+        const long long ps = (long long)a.nkv * prefix[ss] + (long long)sh * np, pe = ps + np;
+        const int i0 = (int)(((ps + 1) * G - 1) / P), i1 = (int)((pe * G - 1) / P);      // CTAs holding the first / last page
+        __threadfence();
+        const int ticket = atomicAdd(&a.counters[ss * a.nkv + sh], 1);
+        s_last[warp] = (ticket == i1 - i0);
+        s_i0[warp] = i0;
+        s_i1[warp] = i1;
+        __threadfence();
+    }
+    csync();
+#pragma unroll 1
+    for (int w2 = 0; w2 < 2; ++w2) {
+        const int ss = w2 == 0 ? end_s : on_s, sh = w2 == 0 ? end_h : on_h;
+        if (ss < 0 || !s_last[w2]) continue;
+        const int i0 = s_i0[w2], i1 = s_i1[w2];
+        // partial of CTA j: slot 1 in the CTA where the pair starts (i0), slot 0 in the others.  Eight partials' sums and columns are loaded
+        // together, so a merge is one round trip to L2 (as passes over the maxima, the weights and the columns it was 4 us, twice in some
+        // blocks)
+        for (int i = tid; i < n_rep * (D / 4); i += kSkConsumers) {
+            const int hh = i / (D / 4), cc = (i % (D / 4)) * 4;
+            float mx = -INFINITY, den = 0.f;
+            float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (int j0 = i0; j0 <= i1; j0 += 8) {
+                float2 ml[8];
+                float4 v[8];
+#pragma unroll
+                for (int u = 0; u < 8; ++u) {
+                    const int j = min(j0 + u, i1);
+                    const size_t pj = (size_t)(j * 2 + (j == i0)) * n_rep + hh;
+                    ml[u] = __ldcg(reinterpret_cast<const float2*>(k.sk_ml + pj * 2));
+                    v[u] = __ldcg(reinterpret_cast<const float4*>(k.sk_acc + pj * D + cc));
+                }
+                float mn = mx;
+#pragma unroll
+                for (int u = 0; u < 8; ++u) mn = fmaxf(mn, ml[u].x);       // (the clamped ones repeat the last)
+                const float old = expf(mx - mn);                           // a part has a visible key: its maximum is finite
+                den *= old; x.x *= old; x.y *= old; x.z *= old; x.w *= old;
+                mx = mn;
+#pragma unroll
+                for (int u = 0; u < 8; ++u)
+                    if (j0 + u <= i1) {
+                        const float w = expf(ml[u].x - mn);
+                        den = fmaf(w, ml[u].y, den);
+                        x.x = fmaf(w, v[u].x, x.x); x.y = fmaf(w, v[u].y, x.y); x.z = fmaf(w, v[u].z, x.z); x.w = fmaf(w, v[u].w, x.w);
+                    }
+            }
+            const size_t o = (size_t)ss * a.nh * D + (size_t)(sh * n_rep + hh) * D + cc;
+            store_out2(a, o, x.x / den, x.y / den);
+            store_out2(a, o + 2, x.z / den, x.w / den);
+        }
+        if (tid == 0) a.counters[ss * a.nkv + sh] = 0;
     }
 }
 

@@ -145,7 +145,9 @@ static SkPlan attn_sk_plan_d(int n_rep) {
     if (it != memo.end()) return it->second;
     auto fit = [&](int st) {
         int n = 0;
-        FL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_sk_decode_kernel<D>, kSkThreads, attn_sk_smem_bytes(D, n_rep, st)));
+        const size_t smem = attn_sk_smem_bytes(D, n_rep, st);
+        if (n_rep <= 8) FL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_sk_decode_kernel<D, true>, kSkThreads, smem));
+        else FL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_sk_decode_kernel<D, false>, kSkThreads, smem));
         return n;
     };
     SkPlan p;
@@ -168,17 +170,22 @@ static SkPlan attn_sk_plan(int d, int n_rep) {
 }
 static void launch_attn_sk(LaunchCtx& lc, int d, const SkPlan& pl, uint64_t bytes, const CUtensorMap& tmk, const CUtensorMap& tmv, const SkArgs& k) {
     const dim3 g(pl.ctas * kNumSMs), b(kSkThreads);
-    switch (d) {
-        case 16: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<16>, g, b, pl.smem, tmk, tmv, k); break;
-        case 32: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<32>, g, b, pl.smem, tmk, tmv, k); break;
-        case 64: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<64>, g, b, pl.smem, tmk, tmv, k); break;
-        default: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<128>, g, b, pl.smem, tmk, tmv, k); break;
-    }
+    auto go = [&](auto pair) {
+        constexpr bool P = decltype(pair)::value;
+        switch (d) {
+            case 16: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<16, P>, g, b, pl.smem, tmk, tmv, k); break;
+            case 32: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<32, P>, g, b, pl.smem, tmk, tmv, k); break;
+            case 64: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<64, P>, g, b, pl.smem, tmk, tmv, k); break;
+            default: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<128, P>, g, b, pl.smem, tmk, tmv, k); break;
+        }
+    };
+    if (k.a.nh / k.a.nkv <= 8) go(std::true_type{}); else go(std::false_type{});
 }
 
 template <int D>
 static void attn_mma_set_attrs() {
-    FL_CUDA(cudaFuncSetAttribute(attn_sk_decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    FL_CUDA(cudaFuncSetAttribute(attn_sk_decode_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    FL_CUDA(cudaFuncSetAttribute(attn_sk_decode_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     if constexpr (D == 64 || D == 128)
         FL_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_prefill_tc_smem_bytes(D)));
     FL_CUDA(cudaFuncSetAttribute(attn_prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_prefill_smem_bytes(D)));
