@@ -254,7 +254,8 @@ struct QkvEpiArgs {
 static __global__ void dense_qkv_epi_kernel(const QkvEpiArgs a) {
     // the dependent (attention) kernel is released only AFTER this kernel's own wait: when it starts, the q|k|v GEMM -- and by
     // induction every earlier kernel of the stream -- has completed, so its preamble may read the step state, the page table and
-    // every K/V page except the rows appended here before its own griddepcontrol.wait (attn_sk_decode_kernel streams them early)
+    // every K/V page except the rows appended here before its own griddepcontrol.wait (attn_sk_decode_kernel streams them early).
+    // (Released at entry its blocks took the SMs as the GEMM's blocks left them, three on some and one on others: 24.1 -> 25.2 us.)
     pdl_wait();
     pdl_launch_dependents();
     const int row = blockIdx.y;
@@ -429,6 +430,7 @@ static __global__ void __launch_bounds__(256) moe_router_kernel(const uint16_t* 
     for (int e = warp; e < E; e += 8) {
         const float4* wg = reinterpret_cast<const float4*>(wgate + (size_t)e * H);
         float acc = 0.f;
+#pragma unroll 8          // (the loads of eight steps together: one after the other they cost 18 us at H = 4096, all of it latency)
         for (int i = lane; i < H / 4; i += 32) {
             const uint2 a = h4[i], b = l4[i];
             const float4 w = wg[i];
@@ -569,14 +571,29 @@ static __global__ void __launch_bounds__(256) dense_argmax_kernel(const float* _
     __shared__ float sv[8];
     __shared__ int si[8];
     const size_t row = blockIdx.y, base = row * V;
-    const int per = (V + gridDim.x - 1) / gridDim.x, c0 = blockIdx.x * per, c1 = min(V, c0 + per);
+    const int per = ((V + gridDim.x - 1) / gridDim.x + 3) & ~3, c0 = blockIdx.x * per, c1 = min(V, c0 + per);
+    const bool vec = (V & 3) == 0;           // (rows of any other length come from sharded vocabularies alone)
     float v = -INFINITY;
     int idx = -1;
-    for (int i = c0 + threadIdx.x; i < c1; i += 256) {
+#pragma unroll 2
+    for (int i = c0 + 4 * threadIdx.x; vec && i < c1; i += 1024) {
+        float4 x = make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll 2
+        for (int s = 0; s < nsl; ++s) {
+            const float4 p = *reinterpret_cast<const float4*>(y + (size_t)s * sl_stride + base + i);
+            x.x += p.x; x.y += p.y; x.z += p.z; x.w += p.w;
+        }
+        *reinterpret_cast<float4*>(logits + base + i) = x;
+        if (x.x >= v) { v = x.x; idx = i; }      // i ascends per thread: >= keeps the last
+        if (x.y >= v) { v = x.y; idx = i + 1; }
+        if (x.z >= v) { v = x.z; idx = i + 2; }
+        if (x.w >= v) { v = x.w; idx = i + 3; }
+    }
+    for (int i = c0 + threadIdx.x; !vec && i < c1; i += 256) {
         float x = 0.f;
         for (int s = 0; s < nsl; ++s) x += y[(size_t)s * sl_stride + base + i];
         logits[base + i] = x;
-        if (x >= v) { v = x; idx = i; }      // i ascends per thread: >= keeps the last
+        if (x >= v) { v = x; idx = i; }
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
