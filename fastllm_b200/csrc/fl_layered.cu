@@ -940,7 +940,7 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
         FL_CUDA(cudaStreamSynchronize(c.stream));
         drop_graphs(c);
         const size_t N = std::max<size_t>(n_want, 2 * y.want_cap);
-        y.hf.alloc(N * m.W); y.logits.alloc(N * m.V); y.h_logits.alloc(N * m.V);
+        y.hf.alloc(N * m.W); y.logits.alloc(N * m.V);
         if (!m.f32) { y.hf_hi.alloc(N * m.W); y.hf_lo.alloc(N * m.W); }
         y.want_cap = N;
     }
@@ -1330,6 +1330,7 @@ static GqaPages gqa_pages(int window, int keep_first, int chunk, int pos0, int T
 }
 static void gqa_attn_fused(fl_cache& c, LaunchCtx& lc, const GqaAttnArgs& a, int r0, int Ts, int pos0, int slot) {
     LayeredCache& y = *c.ly;
+    y.may_fail = true;
     const GqaPages pg = gqa_pages(a.window, a.keep_first, a.chunk, pos0, Ts);
     const int dk = a.D <= 64 ? 64 : 128, dv = a.Dv <= 64 ? 64 : 128;
     const size_t keys = (size_t)a.G * pg.pages * kKvPage;
@@ -1449,6 +1450,9 @@ static void reserve_portions(fl_cache& c, const int* slots, const int* counts, i
 
 void layered_finish(fl_cache& c) {
     FL_CUDA(cudaStreamSynchronize(c.stream));
+    layered_check(c);
+}
+void layered_check(fl_cache& c) {
     if (*c.ly->at_failed.p == 0) return;
     c.poisoned = true;
     throw Error(FL_ERR_CUDA, "attention of a portion: a wait inside the kernel ran out, the step's results are not valid");
@@ -1481,6 +1485,7 @@ void layered_forward(fl_cache& c, const int* slots, const int* counts, int n, co
     ensure_ws(c, (size_t)T, (size_t)n_want);
     reserve_portions(c, slots, counts, n);
     if (y.at_failed.n == 0) { y.at_failed.alloc(1); *y.at_failed.p = 0; }
+    y.may_fail = false;
     const size_t tab_ints = (size_t)4 * T + 3 * (size_t)n + 1 + (size_t)n_want;
     if (tab_ints > y.tab_cap) {
         FL_CUDA(cudaStreamSynchronize(c.stream));
@@ -1556,8 +1561,6 @@ void layered_forward(fl_cache& c, const int* slots, const int* counts, int n, co
     } else {
         enqueue_step(c, lc, st, slots, counts, n, h_row0, h_pos0);
     }
-    if (n_want > 0)
-        FL_CUDA(cudaMemcpyAsync(y.h_logits.p, y.logits.p, (size_t)n_want * m.V * 4, cudaMemcpyDeviceToHost, c.stream));
     for (int i = 0, r = 0; i < n; ++i) {
         c.slot_len[slots[i]] += counts[i];
         r += counts[i];

@@ -850,7 +850,6 @@ static void cache_create(fl_cache& c, int max_batch, int max_seq) {
     c.amax_idx.alloc((size_t)kPassRows * c.amax_parts);
     c.am_val.alloc((size_t)max_batch * kArgmaxParts); c.am_idx.alloc((size_t)max_batch * kArgmaxParts);
     c.h_ids.alloc((size_t)max_batch * max_seq);
-    c.h_logits.alloc((size_t)max_batch * w.Vfull);
     c.slot_len.assign(max_batch, 0);
     c.slot_tab.alloc(2 * (size_t)max_batch);
     c.h_slot_tab.alloc(2 * (size_t)max_batch);
@@ -1675,6 +1674,23 @@ FL_EXPORT int fl_init(int device) {
     FL_API_END
 }
 
+FL_EXPORT int fl_host_alloc(size_t bytes, void** out) {
+    FL_API_BEGIN
+    FL_CHECK(out && bytes > 0, FL_ERR_INVALID, "bad argument");
+    use_device();
+    FL_CUDA(cudaMallocHost(out, bytes));
+    FL_API_END
+}
+
+FL_EXPORT int fl_host_free(void* p) {
+    FL_API_BEGIN
+    if (p) {
+        use_device();
+        FL_CUDA(cudaFreeHost(p));
+    }
+    FL_API_END
+}
+
 FL_EXPORT int fl_device_synchronize(void) {
     FL_API_BEGIN
     use_device();
@@ -1819,6 +1835,52 @@ FL_EXPORT int fl_cache_pool_stats(fl_cache* c, int* pages_total, int* pages_free
     FL_API_END
 }
 
+// deliver_logits' device side
+struct LogitsTransfer {
+    fl_cache& c; const float* dev; float* pinned;
+    int parts = 0;
+    cudaEvent_t e[kLogitsParts] = {};
+    LogitsTransfer(fl_cache& cache, const float* d, float* p) : c(cache), dev(d), pinned(p) {}
+    LogitsTransfer(const LogitsTransfer&) = delete;
+    ~LogitsTransfer() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
+    void begin(int n) { parts = n; }
+    void fetch(int p, size_t at, size_t count) {
+        FL_CUDA(cudaMemcpyAsync(pinned + at, dev + at, count * 4, cudaMemcpyDeviceToHost, c.stream));
+        if (parts == 1) return;
+        FL_CUDA(cudaEventCreateWithFlags(&e[p], cudaEventDisableTiming));
+        FL_CUDA(cudaEventRecord(e[p], c.stream));
+    }
+    void wait(int p) { FL_CUDA(parts == 1 ? cudaStreamSynchronize(c.stream) : cudaEventSynchronize(e[p])); }
+    void check() { if (c.ly) layered_check(c); else check_peer_error(); }
+};
+// page-locked from its first byte to its last
+static bool page_locked(const float* p, size_t n) {
+    for (const void* q : {(const void*)p, (const void*)(reinterpret_cast<const char*>(p + n) - 1)}) {
+        cudaPointerAttributes at;
+        if (cudaPointerGetAttributes(&at, q) != cudaSuccess) { cudaGetLastError(); return false; }
+        if (at.type != cudaMemoryTypeHost) return false;
+    }
+    return true;
+}
+// The step's logits (n floats) in the caller's buffer.  Page-locked buffers (fl_host_alloc) are written by the device itself; others get them
+// through a page-locked one.  Either way nothing there changes unless the step was good.
+static void logits_to_host(fl_cache& c, float* host, size_t n) {
+    const float* dev = c.ly ? c.ly->logits.p : c.logits.p;
+    if (page_locked(host, n)) {
+        if (c.ly ? c.ly->may_fail : g_peer.ready) {        // a step that may have failed without a CUDA error is waited for first
+            FL_CUDA(cudaStreamSynchronize(c.stream));
+            LogitsTransfer(c, dev, host).check();
+        }
+        FL_CUDA(cudaMemcpyAsync(host, dev, n * 4, cudaMemcpyDeviceToHost, c.stream));
+        FL_CUDA(cudaStreamSynchronize(c.stream));
+        return;
+    }
+    PinnedBuf<float>& stage = c.ly ? c.ly->h_logits : c.h_logits;
+    if (stage.n < n) stage.alloc(c.ly ? c.ly->logits.n : (size_t)c.max_batch * c.w->Vfull);
+    LogitsTransfer t(c, dev, stage.p);
+    deliver_logits(t, stage.p, host, n);
+}
+
 // Layered models behind the uniform entry points: b sequences in slots 0..b-1 (or the given slots), t tokens each, logits of every
 // sequence's last token.  Positions follow from what a slot holds, so the caller's offset must agree with it.
 static void layered_uniform(fl_cache& c, const int* slots, const uint32_t* ids, int n, int t, const size_t* offsets, size_t offset_all,
@@ -1833,8 +1895,7 @@ static void layered_uniform(fl_cache& c, const int* slots, const uint32_t* ids, 
         want[i] = i * t + t - 1;
     }
     layered_forward(c, sl.data(), cnt.data(), n, ids, want.data(), n);
-    layered_finish(c);
-    std::memcpy(logits_host, c.ly->h_logits.p, (size_t)n * c.lm->V * 4);
+    logits_to_host(c, logits_host, (size_t)n * c.lm->V);
 }
 
 FL_EXPORT int fl_cache_create(fl_model* m, int max_batch, int max_seq, fl_cache** out) {
@@ -1935,29 +1996,6 @@ FL_EXPORT int fl_cache_destroy(fl_cache* c) {
         delete c;
     }
     FL_API_END
-}
-
-// deliver_logits' device side
-struct LogitsTransfer {
-    cudaStream_t stream; const float* dev; float* pinned;
-    int parts = 0;
-    cudaEvent_t e[kLogitsParts] = {};
-    LogitsTransfer(cudaStream_t s, const float* d, float* p) : stream(s), dev(d), pinned(p) {}
-    LogitsTransfer(const LogitsTransfer&) = delete;
-    ~LogitsTransfer() { for (cudaEvent_t x : e) if (x) cudaEventDestroy(x); }
-    void begin(int n) { parts = n; }
-    void fetch(int p, size_t at, size_t count) {
-        FL_CUDA(cudaMemcpyAsync(pinned + at, dev + at, count * 4, cudaMemcpyDeviceToHost, stream));
-        if (parts == 1) return;
-        FL_CUDA(cudaEventCreateWithFlags(&e[p], cudaEventDisableTiming));
-        FL_CUDA(cudaEventRecord(e[p], stream));
-    }
-    void wait(int p) { FL_CUDA(parts == 1 ? cudaStreamSynchronize(stream) : cudaEventSynchronize(e[p])); }
-    void check() { check_peer_error(); }
-};
-static void logits_to_host(fl_cache& c, float* host, size_t n) {
-    LogitsTransfer t(c.stream, c.logits.p, c.h_logits.p);
-    deliver_logits(t, c.h_logits.p, host, n);
 }
 
 FL_EXPORT int fl_forward(fl_model* m, fl_cache* c, const uint32_t* ids, int b, int t, size_t rope_offset, float* logits_host) {
@@ -2139,6 +2177,7 @@ FL_EXPORT int fl_forward_sample(fl_model* m, fl_cache* c, const uint32_t* ids, i
         run_forward(*c, ids, b, t, rope_offset);
         // only row 0 is sampled (logits.get(0)?.flatten_all()?, models/mod.rs:421): one V*4-byte read-back into the pinned staging row
         const size_t n = c->w->Vfull;
+        if (c->h_logits.n < n) c->h_logits.alloc((size_t)c->max_batch * n);
         FL_CUDA(cudaMemcpyAsync(c->h_logits.p, c->logits.p, n * 4, cudaMemcpyDeviceToHost, c->stream));
         FL_CUDA(cudaStreamSynchronize(c->stream));
         check_peer_error();
@@ -2193,8 +2232,8 @@ FL_EXPORT int fl_forward_ragged(fl_model* m, fl_cache* c, const int* slots, cons
     use_device();
     try {
         layered_forward(*c, slots, counts, n, ids, want, n_want);
-        layered_finish(*c);
-        if (n_want > 0) std::memcpy(logits_host, c->ly->h_logits.p, (size_t)n_want * m->lay->V * 4);
+        if (n_want > 0) logits_to_host(*c, logits_host, (size_t)n_want * m->lay->V);
+        else layered_finish(*c);
     } catch (const fl::Error& e) {
         if (e.code == FL_ERR_CUDA) c->poisoned = true;
         throw;

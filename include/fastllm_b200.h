@@ -283,6 +283,10 @@ FL_EXPORT int fl_init(int device);                               /* cudaSetDevic
 FL_EXPORT const char* fl_last_error(void);                       /* thread-local, never NULL */
 FL_EXPORT int fl_version(void);
 FL_EXPORT int fl_device_synchronize(void);
+/* Page-locked host memory.  A logits_host buffer from here is written by the device itself; any other buffer costs a copy by the calling
+ * thread (and its page faults, when it is new).  Freeing memory that a call is still writing to is undefined. */
+FL_EXPORT int fl_host_alloc(size_t bytes, void** out);
+FL_EXPORT int fl_host_free(void* p);
 
 /* ---- model (weights) --------------------------------------------------------------------------- */
 FL_EXPORT int fl_model_create(const fl_config* cfg, fl_model** out);

@@ -1,0 +1,72 @@
+"""The page-locked memory under a cache's result arrays: bounded, reused only when no array is left over it, freed in the end."""
+import ctypes
+import gc
+
+import numpy as np
+
+from fastllm_b200 import models
+
+
+class FakeLib:
+    def __init__(self, refuse=False):
+        self.live, self.refuse = {}, refuse
+
+    def fl_host_alloc(self, size, out):
+        if self.refuse:
+            return -2
+        buf = ctypes.create_string_buffer(size)
+        out._obj.value = ctypes.addressof(buf)
+        self.live[out._obj.value] = buf
+        return 0
+
+    def fl_host_free(self, p):
+        del self.live[p.value]
+        return 0
+
+
+SHAPE = (4, 8192)
+
+
+def at(a):
+    return a.__array_interface__["data"][0]
+
+
+def test_blocks_are_reused_only_when_free():
+    lib = FakeLib()
+    pool = models._ResultPool(lib)
+    a = pool.empty(SHAPE)
+    a[:] = 1.0
+    row, where = a[2], at(a)
+    del a
+    b = pool.empty(SHAPE)                       # a row of the first result is still held
+    assert at(b) != where and len(lib.live) == 2
+    c = pool.empty(SHAPE)                       # both blocks are taken: plain memory
+    assert at(c) not in lib.live and (row == 1.0).all()
+    del row
+    gc.collect()
+    d = pool.empty((3, 8192))
+    assert at(d) == where and d.shape == (3, 8192) and d.dtype == np.float32 and d.flags.writeable and len(lib.live) == 2
+
+
+def test_sizes_and_refusals():
+    lib = FakeLib()
+    pool = models._ResultPool(lib)
+    assert at(pool.empty((1, 16))) not in lib.live                # small results: a copy is as good
+    a = pool.empty(SHAPE)
+    del a
+    b = pool.empty((8, 8192))                                     # the free block is too small: exchanged, not added to
+    assert at(b) in lib.live and len(lib.live) == 1
+    assert models._ResultPool(FakeLib(refuse=True)).empty(SHAPE).shape == SHAPE
+
+
+def test_freed_with_the_pool_or_the_last_array():
+    lib = FakeLib()
+    pool = models._ResultPool(lib)
+    a, b = pool.empty(SHAPE), pool.empty(SHAPE)
+    del b
+    pool.close()
+    assert len(lib.live) == 1
+    a[:] = 2.0
+    del a
+    gc.collect()
+    assert not lib.live
