@@ -382,7 +382,7 @@ static __global__ void __launch_bounds__(256) dense_qkv_epi_rows_kernel(const Qk
 // outputs (I % 4 == 0).  Grouped expert GEMMs: rows are blocks of `grp_cap` per expert, of which grp_cnt[block] are valid; grid.y is then
 // kSiluGroupRows per expert, each of which walks its share of the valid rows (a block per row of every expert was 14336 blocks for 64 rows).
 constexpr int kSiluGroupRows = 16;
-static __global__ void __launch_bounds__(256) dense_silu_split_kernel(const float* __restrict__ y, int nsl, long long sl_stride, int I, uint16_t* __restrict__ xhi,
+static __global__ void __launch_bounds__(256, 4) dense_silu_split_kernel(const float* __restrict__ y, int nsl, long long sl_stride, int I, uint16_t* __restrict__ xhi,
                                                                      uint16_t* __restrict__ xlo, const int* __restrict__ grp_cnt = nullptr, int grp_cap = 0) {
     pdl_launch_dependents();
     pdl_wait();
@@ -418,7 +418,7 @@ static __global__ void __launch_bounds__(256) dense_silu_split_kernel(const floa
 // router: logits = x . W_gate^T, softmax over ALL experts (f32), stable descending sort (ties keep the LOWER expert index),
 // take top_k, renormalise by their sum; route_w[row][e] = weight or 0.  One CTA per row, one WARP per expert (128-bit loads,
 // one shuffle reduction each): the eight dot products of a Mixtral row run side by side instead of as eight block reductions.
-static __global__ void __launch_bounds__(256) moe_router_kernel(const uint16_t* __restrict__ xhi, const uint16_t* __restrict__ xlo, int H,
+static __global__ void __launch_bounds__(256, 1) moe_router_kernel(const uint16_t* __restrict__ xhi, const uint16_t* __restrict__ xlo, int H,
                                                                 const float* __restrict__ wgate, int E, int top_k, float* __restrict__ route_w,
                                                                 int* __restrict__ sel_log, float* __restrict__ margin_log) {
     pdl_launch_dependents();

@@ -123,6 +123,7 @@ struct Slices {
 template <int V>
 __device__ __forceinline__ void ld_slices(const Slices& s, size_t i, float (&o)[V]) {
     ld_vec<V>(s.p + i, o);
+#pragma unroll 4
     for (int k = 1; k < s.n; ++k) {
         float t[V];
         ld_vec<V>(s.p + (size_t)k * s.stride + i, t);
@@ -187,12 +188,24 @@ static __global__ void ly_embed_norm_kernel(const uint16_t* __restrict__ embed, 
         for (int c = threadIdx.x; c < W; c += blockDim.x) { const float v = __uint_as_float((uint32_t)e[c] << 16); es += v * v; }
         er = 1.f / sqrtf(block_sum(es, red) / (float)W + eps);
     }
-    for (int c = threadIdx.x; c < W; c += blockDim.x) {
-        float v = __uint_as_float((uint32_t)e[c] << 16);
+    for (int c0 = threadIdx.x; c0 < W; c0 += 4 * blockDim.x) {
+      float ev[4], pv[4], bv[4];               // four channels' loads together (the stores between them would hold them apart)
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+          const int c = c0 + k * blockDim.x;
+          ev[k] = c < W ? __uint_as_float((uint32_t)e[c] << 16) : 0.f;
+          pv[k] = pe && c < W ? __uint_as_float((uint32_t)pe[c] << 16) : 0.f;
+          bv[k] = be && c < W ? __uint_as_float((uint32_t)be[c] << 16) : 0.f;
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int c = c0 + k * blockDim.x;
+        if (c >= W) break;
+        float v = ev[k];
         if (en != nullptr) v *= er * norm_scale(en, c, plain);
         if (escale != 0.f) v *= escale;
-        if (pe) v += __uint_as_float((uint32_t)pe[c] << 16);
-        if (be) v += __uint_as_float((uint32_t)be[c] << 16);
+        if (pe) v += pv[k];
+        if (be) v += bv[k];
         if (x0) x0[(size_t)row * W + c] = v;
         if (step) v += step[c];
         xr[c] = v;
@@ -203,6 +216,7 @@ static __global__ void ly_embed_norm_kernel(const uint16_t* __restrict__ embed, 
             if (h) h[(size_t)row * W + c] = v;
             split_store(hhi, hlo, (size_t)row * W + c, v);
         }
+      }
     }
     if (nw.w == nullptr || nw.alpha != nullptr) return;
     const float r = 1.f / sqrtf(block_sum(ss, red) / (float)W + eps);
@@ -822,7 +836,7 @@ struct LatentAppendArgs {
 // Both norms' sums of squares are taken in one pass.  With a query latent the projected row may still lie in split-K slices (`in`):
 // they are folded as the columns are read, and the gate's columns are folded into proj for the kernel that reads them later.
 template <typename CT>
-static __global__ void __launch_bounds__(1024) ly_latent_append_kernel(LatentAppendArgs a) {
+static __global__ void __launch_bounds__(1024, 1) ly_latent_append_kernel(LatentAppendArgs a) {
     pdl_chain();
     __shared__ float2 red[33];
     const int row = blockIdx.x, pos = a.row_pos[row], tid = threadIdx.x, nt = blockDim.x;
@@ -832,15 +846,35 @@ static __global__ void __launch_bounds__(1024) ly_latent_append_kernel(LatentApp
     const float* sn = a.sinb + (size_t)pos * (a.rdims / 2);
     auto in = [&](int c) { float v[1]; ld_slices<1>(a.in, rb + c, v); return v[0]; };
     const bool own = a.off_dkv >= 0;
+    // everything that does not wait for the sums is fetched first, and what the sums are taken of stays in registers (two latents of up to
+    // 2 nt channels; wider ones are read again): as loads behind one another a row was 16 us, of a block per row
+    CT* dst = nullptr;
+    if (own) {
+        const int slot = a.seq_slot[a.row_seq[row]];
+        const int page = a.page_table[(size_t)slot * a.pps + pos / kKvPage];
+        dst = (CT*)a.pool + ((size_t)page * kKvPage + pos % kKvPage) * (a.C + a.R);
+    }
+    constexpr int KEEP = 2;
+    float kq[KEEP], kc[KEEP], wq[KEEP], wc[KEEP];
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) {
+        const int c = tid + k * nt;
+        kq[k] = c < a.Q ? in(a.off_dq + c) : 0.f;
+        kc[k] = own && c < a.C ? in(a.off_dkv + c) : 0.f;
+        wq[k] = c < a.Q ? a.dq_norm[c] : 0.f;
+        wc[k] = own && c < a.C ? a.dkv_norm[c] : 0.f;
+    }
     float2 ss = make_float2(0.f, 0.f);
-    for (int c = tid; c < a.Q; c += nt) { const float v = in(a.off_dq + c); ss.x += v * v; }
+#pragma unroll
+    for (int k = 0; k < KEEP; ++k) { ss.x += kq[k] * kq[k]; ss.y += kc[k] * kc[k]; }
+    for (int c = tid + KEEP * nt; c < a.Q; c += nt) { const float v = in(a.off_dq + c); ss.x += v * v; }
     if (own)
-        for (int c = tid; c < a.C; c += nt) { const float v = in(a.off_dkv + c); ss.y += v * v; }
+        for (int c = tid + KEEP * nt; c < a.C; c += nt) { const float v = in(a.off_dkv + c); ss.y += v * v; }
     ss = block_sum2(ss, red);
     if (a.Q > 0) {
         const float rq = 1.f / sqrtf(ss.x / (float)a.Q + a.eps);
-        for (int c = tid; c < a.Q; c += nt) {
-            const float v = in(a.off_dq + c) * rq * a.dq_norm[c];
+        for (int c = tid, k = 0; c < a.Q; c += nt, ++k) {
+            const float v = k == 0 ? kq[0] * rq * wq[0] : k == 1 ? kq[1] * rq * wq[1] : in(a.off_dq + c) * rq * a.dq_norm[c];
             if (a.cq != nullptr) a.cq[(size_t)row * a.Q + c] = v;
             split_store(a.cqhi, a.cqlo, (size_t)row * a.Q + c, v);
         }
@@ -850,11 +884,8 @@ static __global__ void __launch_bounds__(1024) ly_latent_append_kernel(LatentApp
         for (int i = tid; i < a.H * (a.rdims / 2); i += nt) turn_pair(pr + a.off_q, a.D, a.R, a.rdims / 2, i, cs, sn);
     }
     if (!own) return;
-    const int slot = a.seq_slot[a.row_seq[row]];
-    const int page = a.page_table[(size_t)slot * a.pps + pos / kKvPage];
-    CT* dst = (CT*)a.pool + ((size_t)page * kKvPage + pos % kKvPage) * (a.C + a.R);
     const float r = 1.f / sqrtf(ss.y / (float)a.C + a.eps);
-    for (int c = tid; c < a.C; c += nt) st_c(dst + c, in(a.off_dkv + c) * r * a.dkv_norm[c]);
+    for (int c = tid, k = 0; c < a.C; c += nt, ++k) st_c(dst + c, k == 0 ? kc[0] * r * wc[0] : k == 1 ? kc[1] * r * wc[1] : in(a.off_dkv + c) * r * a.dkv_norm[c]);
     for (int i = tid; i < a.R; i += nt) {
         float val;
         if (i < a.rdims) {
@@ -1577,9 +1608,16 @@ static __global__ void __launch_bounds__(256) ly_attn_prep_kernel(AttnPrepArgs a
     float* pr = a.proj + rb;
     auto in = [&](int c) { float v[1]; ld_slices<1>(a.in, rb + c, v); return v[0]; };
     const bool own = a.off_k >= 0, shared_v = a.off_v < 0;
+    CT* dst = nullptr;
+    if (own) {
+        const int slot = a.seq_slot[a.row_seq[row]];
+        const int page = a.page_table[(size_t)slot * a.pps + pos / kKvPage];
+        dst = (CT*)a.pool + ((size_t)page * kKvPage + pos % kKvPage) * (size_t)a.kv.E;
+    }
     float rq = 0.f, rk = 0.f;
     if (a.whole && a.qnorm != nullptr) {
         float ss = 0.f;
+#pragma unroll 8
         for (int c = threadIdx.x; c < a.H * a.D; c += blockDim.x) { const float v = in(a.off_q + c) + (a.bq ? a.bq[c] : 0.f); ss += v * v; }
         rq = 1.f / sqrtf(block_sum(ss, red) / (float)(a.H * a.D) + a.eps);
         if (own) {
@@ -1592,14 +1630,81 @@ static __global__ void __launch_bounds__(256) ly_attn_prep_kernel(AttnPrepArgs a
     const float* cs = a.cosb + (size_t)pos * half;
     const float* sn = a.sinb + (size_t)pos * half;
     float* buf = sm + wid * a.D;
-    CT* dst = nullptr;
-    if (own) {
-        const int slot = a.seq_slot[a.row_seq[row]];
-        const int page = a.page_table[(size_t)slot * a.pps + pos / kKvPage];
-        dst = (CT*)a.pool + ((size_t)page * kKvPage + pos % kKvPage) * (size_t)a.kv.E;
-    }
     const int items = a.H + (own ? a.G : 0);
-    for (int it = blockIdx.y * nw + wid; it < items; it += gridDim.y * nw) {
+    // heads of up to 128 channels: a lane's channels, weights and turns in registers, the next head's values on their way while this one is
+    // turned (one dependent load after the other -- values, weights, turns, of every head -- a row of 20 heads was 18 us)
+    constexpr int NC = 4;
+    const bool narrow = a.D <= 32 * NC;
+    float cj[NC], sj[NC];
+    auto place = [&](int c, int& pi) { if (a.halves) { pi = c >= half ? c - half : c; return c >= half; } pi = c >> 1; return (c & 1) != 0; };
+    auto fetch = [&](int it, float (&v)[NC], float (&w)[NC]) {
+        const bool isq = it < a.H;
+        const int hd = isq ? it : it - a.H, src = (isq ? a.off_q : a.off_k) + hd * a.D;
+        const float* bias = isq ? a.bq : a.bk;
+        const float* wn = isq ? a.qnorm : a.knorm;
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+            const int c = lane + 32 * j;
+            v[j] = c < a.D ? in(src + c) + (bias ? bias[(size_t)hd * a.D + c] : 0.f) : 0.f;
+            w[j] = wn != nullptr && c < a.D ? wn[a.whole ? (size_t)hd * a.D + c : (size_t)c] : 0.f;
+        }
+    };
+    if (narrow) {
+#pragma unroll
+        for (int j = 0; j < NC; ++j) {
+            const int c = lane + 32 * j;
+            int pi = 0;
+            place(c, pi);
+            cj[j] = c < a.rdims ? cs[pi] : 0.f;
+            sj[j] = c < a.rdims ? sn[pi] : 0.f;
+        }
+        float v[NC], w[NC], nv[NC], nwt[NC];
+        const int step = gridDim.y * nw;
+        int it = blockIdx.y * nw + wid;
+        if (it < items) fetch(it, v, w);
+        for (; it < items; it += step) {
+            if (it + step < items) fetch(it + step, nv, nwt);
+            const bool isq = it < a.H;
+            const int hd = isq ? it : it - a.H, src = (isq ? a.off_q : a.off_k) + hd * a.D;
+            if ((isq ? a.qnorm : a.knorm) != nullptr) {
+                float r;
+                if (a.whole) {
+                    r = isq ? rq : rk;
+                } else {
+                    float ss = 0.f;
+#pragma unroll
+                    for (int j = 0; j < NC; ++j) ss += v[j] * v[j];      // (channels behind the head are zeros)
+                    r = 1.f / sqrtf(warp_sum(ss) / (float)a.D + a.eps);
+                }
+#pragma unroll
+                for (int j = 0; j < NC; ++j) v[j] = v[j] * r * w[j];
+            }
+            __syncwarp();
+#pragma unroll
+            for (int j = 0; j < NC; ++j)
+                if (lane + 32 * j < a.D) buf[lane + 32 * j] = v[j];
+            __syncwarp();
+            CT* kd = isq ? nullptr : dst + (size_t)hd * a.kv.ks;
+#pragma unroll
+            for (int j = 0; j < NC; ++j) {
+                const int c = lane + 32 * j;
+                if (c >= a.D) break;
+                float val = v[j];
+                if (c < a.rdims) {
+                    int pi;
+                    const bool second = place(c, pi);
+                    const float x = buf[a.halves ? pi : 2 * pi], y = buf[a.halves ? pi + half : 2 * pi + 1];
+                    val = second ? y * cj[j] + x * sj[j] : x * cj[j] - y * sj[j];
+                }
+                if (isq) { pr[src + c] = val; continue; }
+                st_c(kd + c, val);
+                if (shared_v && c < a.rdims) st_c(kd + a.D + c, v[j]);
+            }
+#pragma unroll
+            for (int j = 0; j < NC; ++j) { v[j] = nv[j]; w[j] = nwt[j]; }
+        }
+    }
+    for (int it = blockIdx.y * nw + wid; !narrow && it < items; it += gridDim.y * nw) {
         const bool isq = it < a.H;
         const int hd = isq ? it : it - a.H;
         const int src = (isq ? a.off_q : a.off_k) + hd * a.D;
@@ -1817,26 +1922,34 @@ static __global__ void __launch_bounds__(kGqaWarps * 32) ly_gqa_attn_kernel(GqaA
 }
 // Folds the key splits of ly_gqa_attn_kernel (or ly_latent_mma_kernel) in split order (and the sink): one block per (row, head).
 // out == nullptr: only the halves are wanted.  roll: element i of a partial is channel (i + roll) mod Dv (see KvLayout).
+constexpr int kMergeSplits = 16;       // at most
 static __global__ void ly_gqa_merge_kernel(const float* __restrict__ part, int S, int H, int Dv, int sink, const float* __restrict__ sinkv, int row_base,
                                            int ldo, int roll, OutGate gate, float* __restrict__ out, uint16_t* __restrict__ ohi, uint16_t* __restrict__ olo) {
     pdl_chain();
     const int row = row_base + blockIdx.x, hd = blockIdx.y;
     const float* pp = part + ((size_t)blockIdx.x * H + hd) * S * (Dv + 2);
+    // the splits' maxima and sums are read once, their weights computed once (a pass over them per use was 20 us at 16 splits of 512 channels)
+    __shared__ float pm[kMergeSplits], pl[kMergeSplits], pf[kMergeSplits];
     const float sv = sinkv ? sinkv[hd] : 0.f;
+    for (int s = threadIdx.x; s < S; s += blockDim.x) { pm[s] = pp[(size_t)s * (Dv + 2)]; pl[s] = pp[(size_t)s * (Dv + 2) + 1]; }
+    __syncthreads();
     float M = sink ? sv : -INFINITY;
-    for (int s = 0; s < S; ++s) M = fmaxf(M, pp[(size_t)s * (Dv + 2)]);
+    for (int s = 0; s < S; ++s) M = fmaxf(M, pm[s]);
+    for (int s = threadIdx.x; s < S; s += blockDim.x) pf[s] = pm[s] == -INFINITY ? 0.f : expf(pm[s] - M);
+    __syncthreads();
     float L = sink ? expf(sv - M) : 0.f;
-    for (int s = 0; s < S; ++s) {
-        const float ms = pp[(size_t)s * (Dv + 2)];
-        L += ms == -INFINITY ? 0.f : pp[(size_t)s * (Dv + 2) + 1] * expf(ms - M);
-    }
+    for (int s = 0; s < S; ++s) L += pm[s] == -INFINITY ? 0.f : pl[s] * pf[s];
     const float inv = 1.f / L;
     const size_t ob = (size_t)row * ldo + (size_t)hd * Dv;
     for (int i = threadIdx.x; i < Dv; i += blockDim.x) {
         float t = 0.f;
-        for (int s = 0; s < S; ++s) {
-            const float ms = pp[(size_t)s * (Dv + 2)];
-            if (ms != -INFINITY) t += pp[(size_t)s * (Dv + 2) + 2 + i] * expf(ms - M);
+        for (int s0 = 0; s0 < S; s0 += 8) {
+            float v[8];
+#pragma unroll
+            for (int k = 0; k < 8; ++k) v[k] = s0 + k < S ? pp[(size_t)(s0 + k) * (Dv + 2) + 2 + i] : 0.f;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+                if (s0 + k < S && pm[s0 + k] != -INFINITY) t += v[k] * pf[s0 + k];
         }
         t *= inv;
         const int c = i + roll < Dv ? i + roll : i + roll - Dv;
@@ -2376,6 +2489,7 @@ static __global__ void ly_router_kernel(const float* __restrict__ h, int W, cons
         if ((W & 3) == 0) {         // 16-byte rows: four channels per load
             const float4* w4 = reinterpret_cast<const float4*>(w);
             const float4* h4 = reinterpret_cast<const float4*>(hr);
+#pragma unroll 8
             for (int c = lane; c < W / 4; c += 32) {
                 const float4 a = w4[c], b = h4[c];
                 d = fmaf(a.x, b.x, d); d = fmaf(a.y, b.y, d); d = fmaf(a.z, b.z, d); d = fmaf(a.w, b.w, d);
@@ -2423,7 +2537,7 @@ static __global__ void ly_router_kernel(const float* __restrict__ h, int W, cons
 // One block per RB rows (many rows: an expert's weights are read once per RB of them), one warp per expert in turn, then one warp per row;
 // shared memory: RB (2 E + groups) floats.  A row's sums are taken in the same order whatever RB.
 template <int RB>
-static __global__ void __launch_bounds__(256) ly_router_groups_kernel(const float* __restrict__ h, int W, const float* __restrict__ wr, int E, int top, int softmax,
+static __global__ void __launch_bounds__(256, 1) ly_router_groups_kernel(const float* __restrict__ h, int W, const float* __restrict__ wr, int E, int top, int softmax,
                                                const float* __restrict__ corr, int groups, int keep, int mark2, int renorm, int T, int* __restrict__ sel,
                                                float* __restrict__ wt) {
     pdl_chain();
@@ -2438,7 +2552,8 @@ static __global__ void __launch_bounds__(256) ly_router_groups_kernel(const floa
         for (int r = 0; r < RB; ++r) d[r] = 0.f;
         if ((W & 3) == 0) {
             const float4* w4 = reinterpret_cast<const float4*>(w);
-#pragma unroll 2
+            constexpr int U = RB == 1 ? 8 : 2;
+#pragma unroll U
             for (int c = lane; c < W / 4; c += 32) {
                 const float4 a = w4[c];
 #pragma unroll
@@ -2584,14 +2699,18 @@ static __global__ void ly_moe_gather_kernel(const uint16_t* __restrict__ hhi, co
 }
 // The activation over the grouped GEMM's output: gu[slice][e * cap + i][2F] (F columns for the ungated act 2) summed over slices, rows
 // i < cnt[e] only -> hi | lo.
+constexpr int kGluGroupRows = 16;
 static __global__ void ly_glu_grouped_kernel(const float* __restrict__ gu, int nsl, size_t sl_stride, int F, float limit, int act_kind,
                                              const int* __restrict__ cnt, int cap, uint16_t* __restrict__ ahi, uint16_t* __restrict__ alo) {
     pdl_chain();
-    const int r = blockIdx.y;                   // row e * cap + i
-    if (r % cap >= cnt[r / cap]) return;
-    for (int f = blockIdx.x * blockDim.x + threadIdx.x; f < F; f += gridDim.x * blockDim.x) {
+    // kGluGroupRows blocks per expert and 256 columns walk the expert's valid rows (a block per row of every expert's capacity: most had nothing to do)
+    const int e = blockIdx.y / kGluGroupRows, end = e * cap + cnt[e];
+    const int f = blockIdx.x * blockDim.x + threadIdx.x;
+    if (f >= F) return;
+    const size_t gs = act_kind == 2 ? (size_t)F : (size_t)2 * F;
+    for (int r = e * cap + blockIdx.y % kGluGroupRows; r < end; r += kGluGroupRows) {
         float g = 0.f, u = 0.f;
-        const size_t gs = act_kind == 2 ? (size_t)F : (size_t)2 * F;
+#pragma unroll 4
         for (int k = 0; k < nsl; ++k) {
             g += gu[k * sl_stride + (size_t)r * gs + f];
             if (act_kind != 2) u += gu[k * sl_stride + (size_t)r * gs + F + f];
