@@ -760,6 +760,8 @@ void layered_cache_create(fl_cache& c, int max_slots, int max_seq, int pool_toke
     FL_CHECK(m.finalized, FL_ERR_STATE, "model not finalized");
     FL_CHECK(max_slots >= 1 && max_slots <= kMaxBatch && max_seq >= 1 && pool_tokens >= 1, FL_ERR_INVALID, "bad cache dimensions");
     c.max_batch = max_slots; c.max_seq = max_seq;
+    c.step_failed.alloc(1);
+    *c.step_failed.p = 0;
     c.pages_per_seq = (max_seq + kKvPage - 1) / kKvPage;
     FL_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
     c.ly.reset(new LayeredCache);
@@ -934,6 +936,7 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
                 y.grp_cnt.alloc((size_t)m.max_experts + 1);
             }
         }
+        if (!m.f32) ensure_pairs(c, R);
         y.rows = R;
     }
     if (n_want > y.want_cap) {
@@ -1330,13 +1333,13 @@ static GqaPages gqa_pages(int window, int keep_first, int chunk, int pos0, int T
 }
 static void gqa_attn_fused(fl_cache& c, LaunchCtx& lc, const GqaAttnArgs& a, int r0, int Ts, int pos0, int slot) {
     LayeredCache& y = *c.ly;
-    y.may_fail = true;
+    c.may_fail = true;
     const GqaPages pg = gqa_pages(a.window, a.keep_first, a.chunk, pos0, Ts);
     const int dk = a.D <= 64 ? 64 : 128, dv = a.Dv <= 64 ? 64 : 128;
     const size_t keys = (size_t)a.G * pg.pages * kKvPage;
     FL_CHECK(y.at_kc.n >= keys * dk && y.at_kct.n >= keys * dv, FL_ERR_STATE, "internal: scratch of the fused attention too small");
     const GqaTcArgs t{a.proj, a.ldp, a.off_q, r0, Ts, pos0, a.H, a.G, a.D, a.Dv, pg, a.window, a.keep_first, a.chunk, a.scale, a.softcap, a.sink, a.sinkv,
-                      a.ohi, a.olo, a.ldo, a.gate, 8.f, y.at_failed.p};
+                      a.ohi, a.olo, a.ldo, a.gate, 8.f, c.step_failed.p};
     const int* page_row = y.page_table.p + (size_t)slot * c.pages_per_seq;
     if (dk == 64 && dv == 64) launch_gqa_tc<64, 64>(y, lc, a, t, page_row);
     else if (dk == 64) launch_gqa_tc<64, 128>(y, lc, a, t, page_row);
@@ -1450,12 +1453,7 @@ static void reserve_portions(fl_cache& c, const int* slots, const int* counts, i
 
 void layered_finish(fl_cache& c) {
     FL_CUDA(cudaStreamSynchronize(c.stream));
-    layered_check(c);
-}
-void layered_check(fl_cache& c) {
-    if (*c.ly->at_failed.p == 0) return;
-    c.poisoned = true;
-    throw Error(FL_ERR_CUDA, "attention of a portion: a wait inside the kernel ran out, the step's results are not valid");
+    step_check(c);
 }
 
 void layered_forward(fl_cache& c, const int* slots, const int* counts, int n, const uint32_t* ids, const int* want, int n_want) {
@@ -1484,8 +1482,7 @@ void layered_forward(fl_cache& c, const int* slots, const int* counts, int n, co
     for (int k = 0; k < n_want; ++k) FL_CHECK(want[k] >= 0 && want[k] < T, FL_ERR_INVALID, "wanted row out of range");
     ensure_ws(c, (size_t)T, (size_t)n_want);
     reserve_portions(c, slots, counts, n);
-    if (y.at_failed.n == 0) { y.at_failed.alloc(1); *y.at_failed.p = 0; }
-    y.may_fail = false;
+    c.may_fail = false;
     const size_t tab_ints = (size_t)4 * T + 3 * (size_t)n + 1 + (size_t)n_want;
     if (tab_ints > y.tab_cap) {
         FL_CUDA(cudaStreamSynchronize(c.stream));

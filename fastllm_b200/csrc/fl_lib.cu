@@ -11,6 +11,7 @@
 #include "deliver.hpp"
 #include "dense_ops.cuh"
 #include "gemm_dec.cuh"
+#include "gemm_pair.cuh"
 #include "gemm_tc.cuh"
 #include "elementwise.cuh"
 #include "gemv.cuh"
@@ -804,6 +805,8 @@ static void cache_create(fl_cache& c, int max_batch, int max_seq) {
     FL_CHECK(w.finalized, FL_ERR_STATE, "model not finalized");
     FL_CHECK(max_batch >= 1 && max_batch <= kMaxBatch && max_seq >= 1, FL_ERR_INVALID, "bad cache dimensions");
     c.max_batch = max_batch;
+    c.step_failed.alloc(1);
+    *c.step_failed.p = 0;
     c.max_seq = max_seq;
     c.pages_per_seq = (max_seq + kKvPage - 1) / kKvPage;
     FL_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
@@ -1077,6 +1080,7 @@ static void ensure_dense_ws(fl_cache& c, int rows) {
         d.vt.alloc(d.vt_pages_cap * w.nkv * w.d * kKvPage, true);        // zero: the last page's tail multiplies P = 0 and must stay finite
         d.tm_vt = make_tmap_bf16(d.vt.p, d.vt_pages_cap * w.nkv * w.d, kKvPage, kKvPage, (uint32_t)w.d);
     }
+    ensure_pairs(c, R);
     d.rows = R;
 }
 
@@ -1123,6 +1127,54 @@ static void launch_gemm_dec(cudaStream_t st, bool pdl, int ctas, const CUtensorM
         cfg.numAttrs = 1;
     }
     FL_CUDA(cudaLaunchKernelEx(&cfg, gemm_dec_kernel<BN>, w, hi, lo, g));
+}
+
+// Pairs of SMs that can be resident at once (the driver's answer; 74 on a whole chip)
+static int pair_clusters() {
+    static const int n = [] {
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(2 * kPairMaxClusters); cfg.blockDim = dim3(kPairThreads); cfg.dynamicSmemBytes = kPairSmem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        for (auto kern : {gemm_pair_kernel<GEPI_F32>, gemm_pair_kernel<GEPI_SILU_HL>, gemm_pair_kernel<GEPI_GLU_HL>})
+            FL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kPairSmem));
+        int k = 0;
+        FL_CUDA(cudaOccupancyMaxActiveClusters(&k, gemm_pair_kernel<GEPI_F32>, &cfg));
+        return std::min(k, kPairMaxClusters);
+    }();
+    return n;
+}
+void ensure_pairs(fl_cache& c, size_t rows) {
+    if (rows < (size_t)kPairMinRows || c.pair_ws.n > 0) return;
+    c.pair_tickets.alloc(2 * kPairMaxClusters, true);
+    c.pair_ws.alloc(kPairWsFloats);
+}
+// -> whether the GEMM went to pairs of SMs
+template <int EPI>
+static bool launch_gemm_pair(fl_cache& c, cudaStream_t st, bool pdl, const CUtensorMap& hi, const CUtensorMap& lo, const CUtensorMap& w, const GemmArgs& g) {
+    if (c.pair_ws.n == 0 || g.M < kPairMinRows) return false;
+    const int most = pair_clusters();
+    if (most < 1) return false;
+    const PairPlan pl = pair_plan(g.M, g.N, g.K, EPI == GEPI_GLU_HL, most);
+    if (!pair_wins(pl, g.M, most)) return false;
+    const PairArgs p{g, pl.nk, pl.mp, pl.nt, pl.full, pl.L, c.pair_ws.p, c.pair_tickets.p, c.step_failed.p};
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(2 * pl.clusters);
+    cfg.blockDim = dim3(kPairThreads);
+    cfg.dynamicSmemBytes = kPairSmem;
+    cfg.stream = st;
+    cudaLaunchAttribute attr[1];
+    if (pdl) {
+        attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+        attr[0].val.programmaticStreamSerializationAllowed = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+    }
+    FL_CUDA(cudaLaunchKernelEx(&cfg, gemm_pair_kernel<EPI>, hi, lo, w, p));
+    c.may_fail = true;
+    return true;
 }
 
 // Split-K factor of a grouped swap-AB (decode) GEMM: the one whose work items (output tiles x k slices) fill whole waves of the 148
@@ -1182,12 +1234,14 @@ int dense_gemm(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int N, int K,
         if (silu_hi != nullptr) {       // prefill gate|up: SiLU(gate) * up + hi/lo split fused into the epilogue
             GemmArgs g{R, N, K, nullptr, nullptr, 0, silu_hi, N / 2, 1, 0, silu_lo};
             g.raster_m = kGemmRasterRows;
-            if (prefill_bn == 256) launch_gemm_tc<256, GEPI_SILU_HL, DUAL_A>(lc.stream, pdl, tiles, hi, lo, tmW, g);
+            if (prefill_bn == 256 && launch_gemm_pair<GEPI_SILU_HL>(c, lc.stream, pdl, hi, lo, tmW, g)) {}
+            else if (prefill_bn == 256) launch_gemm_tc<256, GEPI_SILU_HL, DUAL_A>(lc.stream, pdl, tiles, hi, lo, tmW, g);
             else launch_gemm_tc<128, GEPI_SILU_HL, DUAL_A>(lc.stream, pdl, tiles, hi, lo, tmW, g);
         } else {
             GemmArgs g{R, N, K, nullptr, nullptr, 0, out, N, ks, (long long)R * N};
             g.raster_m = kGemmRasterRows;
-            if (prefill_bn == 256) launch_gemm_tc<256, GEPI_F32, DUAL_A>(lc.stream, pdl, tiles * ks, hi, lo, tmW, g);
+            if (prefill_bn == 256 && ks == 1 && launch_gemm_pair<GEPI_F32>(c, lc.stream, pdl, hi, lo, tmW, g)) {}
+            else if (prefill_bn == 256) launch_gemm_tc<256, GEPI_F32, DUAL_A>(lc.stream, pdl, tiles * ks, hi, lo, tmW, g);
             else launch_gemm_tc<128, GEPI_F32, DUAL_A>(lc.stream, pdl, tiles * ks, hi, lo, tmW, g);
         }
     }
@@ -1214,7 +1268,8 @@ static void launch_rows_gemm(fl_cache& c, LaunchCtx& lc, const char* tag, const 
         FL_CUDA(cudaEventRecord(pe.e0, lc.stream));
     }
     const CUtensorMap hi = make_tmap_bf16(xhi, g.M, g.K, g.K, kGemmBM), lo = make_tmap_bf16(xlo, g.M, g.K, g.K, kGemmBM);
-    if (glu) launch_gemm_tc<256, GEPI_GLU_HL, DUAL_A>(lc.stream, pdl, tiles, hi, lo, tmW, g);
+    if (glu && g.groups == 0 && launch_gemm_pair<GEPI_GLU_HL>(c, lc.stream, pdl, hi, lo, tmW, g)) {}
+    else if (glu) launch_gemm_tc<256, GEPI_GLU_HL, DUAL_A>(lc.stream, pdl, tiles, hi, lo, tmW, g);
     else launch_gemm_tc<256, GEPI_F32, DUAL_A>(lc.stream, pdl, tiles, hi, lo, tmW, g);
     if (prof) {
         FL_CUDA(cudaEventRecord(pe.e1, lc.stream));
@@ -1545,6 +1600,7 @@ static void check_call(fl_cache& c, const uint32_t* ids, int b, int t, size_t ro
 
 static void run_forward(fl_cache& c, const uint32_t* ids, int b, int t, size_t rope_offset) {
     check_call(c, ids, b, t, rope_offset, 0);
+    c.may_fail = false;
     if ((b * t >= 3 || c.w->cfg.arch == FL_ARCH_MIXTRAL) && c.w->dense_ok) ensure_dense_ws(c, b * t);
     std::memcpy(c.h_ids.p, ids, (size_t)b * t * 4);
     FL_CUDA(cudaMemcpyAsync(c.ids.p, c.h_ids.p, (size_t)b * t * 4, cudaMemcpyHostToDevice, c.stream));
@@ -1590,6 +1646,7 @@ static void run_forward_slots(fl_cache& c, const int* slots, const uint32_t* ids
                  "Llama: multi-token forward needs an empty cache (candle builds a t x t mask)");
     }
     for (int i = 0; i < n * t; ++i) FL_CHECK(ids[i] < (uint32_t)w.Vfull, FL_ERR_INVALID, "token id out of range");
+    c.may_fail = false;
     ensure_dense_ws(c, n * t);
     c.dw.route_rows = n * t;
     c.fresh_call = true;
@@ -1643,6 +1700,15 @@ static void check_peer_error() {
     FL_CUDA(cudaMemcpy(&err, (uint8_t*)g_peer.local + PeerComm::kErrOff, 4, cudaMemcpyDeviceToHost));
     FL_CHECK(err == 0, FL_ERR_NCCL, "tensor-parallel exchange timed out: a peer rank did not reach the same decode step");
 }
+
+namespace fl {
+void step_check(fl_cache& c) {
+    check_peer_error();
+    if (*c.step_failed.p == 0) return;
+    c.poisoned = true;
+    throw Error(FL_ERR_CUDA, "a wait inside a kernel ran out, the step's results are not valid");
+}
+}  // namespace fl
 
 static void use_device() {
     const int dev = g_device.load();
@@ -1851,7 +1917,7 @@ struct LogitsTransfer {
         FL_CUDA(cudaEventRecord(e[p], c.stream));
     }
     void wait(int p) { FL_CUDA(parts == 1 ? cudaStreamSynchronize(c.stream) : cudaEventSynchronize(e[p])); }
-    void check() { if (c.ly) layered_check(c); else check_peer_error(); }
+    void check() { step_check(c); }
 };
 // page-locked from its first byte to its last
 static bool page_locked(const float* p, size_t n) {
@@ -1867,7 +1933,7 @@ static bool page_locked(const float* p, size_t n) {
 static void logits_to_host(fl_cache& c, float* host, size_t n) {
     const float* dev = c.ly ? c.ly->logits.p : c.logits.p;
     if (page_locked(host, n)) {
-        if (c.ly ? c.ly->may_fail : g_peer.ready) {        // a step that may have failed without a CUDA error is waited for first
+        if (c.may_fail || g_peer.ready) {        // a step that may have failed without a CUDA error is waited for first
             FL_CUDA(cudaStreamSynchronize(c.stream));
             LogitsTransfer(c, dev, host).check();
         }
@@ -2034,7 +2100,7 @@ FL_EXPORT int fl_forward_greedy(fl_model* m, fl_cache* c, const uint32_t* ids, i
         run_forward(*c, ids, b, t, rope_offset);
         FL_CUDA(cudaMemcpyAsync(c->h_ids.p, c->next_ids.p, (size_t)b * 4, cudaMemcpyDeviceToHost, c->stream));
         FL_CUDA(cudaStreamSynchronize(c->stream));
-        check_peer_error();
+        step_check(*c);
         std::memcpy(next_ids, c->h_ids.p, (size_t)b * 4);
     } catch (const fl::Error& e) {
         if (e.code == FL_ERR_CUDA || e.code == FL_ERR_NCCL) c->poisoned = true;   // a missed peer leaves kv_len / exchange epochs out of step
@@ -2086,7 +2152,7 @@ FL_EXPORT int fl_decode_greedy_loop(fl_model* m, fl_cache* c, const uint32_t* fi
         }
         FL_CUDA(cudaEventRecord(ev.e1, c->stream));
         FL_CUDA(cudaStreamSynchronize(c->stream));
-        check_peer_error();
+        step_check(*c);
         float ms = 0.f;
         FL_CUDA(cudaEventElapsedTime(&ms, ev.e0, ev.e1));
         if (elapsed_ms) *elapsed_ms = ms;
@@ -2180,7 +2246,7 @@ FL_EXPORT int fl_forward_sample(fl_model* m, fl_cache* c, const uint32_t* ids, i
         if (c->h_logits.n < n) c->h_logits.alloc((size_t)c->max_batch * n);
         FL_CUDA(cudaMemcpyAsync(c->h_logits.p, c->logits.p, n * 4, cudaMemcpyDeviceToHost, c->stream));
         FL_CUDA(cudaStreamSynchronize(c->stream));
-        check_peer_error();
+        step_check(*c);
         try {
             *next_id = s->lp.sample(c->h_logits.p, n);
         } catch (const fl::SamplerError& e) {
@@ -2259,7 +2325,7 @@ FL_EXPORT int fl_forward_sample_device(fl_model* m, fl_cache* c, const uint32_t*
         }
         FL_CUDA(cudaMemcpyAsync(c->h_ids.p, src, 4, cudaMemcpyDeviceToHost, c->stream));
         FL_CUDA(cudaStreamSynchronize(c->stream));
-        check_peer_error();
+        step_check(*c);
         *next_id = c->h_ids.p[0];
     } catch (const fl::Error& e) {
         if (e.code == FL_ERR_CUDA || e.code == FL_ERR_NCCL) c->poisoned = true;

@@ -160,6 +160,71 @@ __device__ __forceinline__ void st_global_32b(void* p, const uint32_t (&v)[8]) {
                  : "memory");
 }
 
+// ---- 16 output columns of one row (column col on), shared by the kernels of many rows ------------------------------------------------------
+// glu(gate, up) as hi | lo halves; N is a multiple of 8
+__device__ __forceinline__ void glu_store16(const GemmArgs& g, int row, int col, const float (&rg)[16], const float (&ru)[16]) {
+    const bool second = col + 8 < g.N;
+    uint32_t ph[8], pl[8];
+#pragma unroll
+    for (int e = 0; e < 8; ++e) {
+        float a[2];
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+            const int j = 2 * e + i;
+            float gv = rg[j], uv = ru[j];
+            if (g.bias != nullptr && (e < 4 || second)) { gv += g.bias[col + j]; uv += g.bias[g.N + col + j]; }
+            a[i] = glu_value(gv, uv, g.act, g.act_limit);
+        }
+        ph[e] = pack_bf16x2(a[0], a[1]);
+        pl[e] = pack_bf16x2(a[0] - bf16lo(ph[e]), a[1] - bf16hi(ph[e]));
+    }
+    uint16_t* oh = reinterpret_cast<uint16_t*>(g.out) + (size_t)row * g.ldo + col;
+    uint16_t* ol = reinterpret_cast<uint16_t*>(g.out2) + (size_t)row * g.ldo + col;
+    if (((g.ldo | g.N) & 15) == 0) {
+        st_global_32b(oh, ph);
+        st_global_32b(ol, pl);
+    } else {
+        *reinterpret_cast<uint4*>(oh) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+        *reinterpret_cast<uint4*>(ol) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+        if (second) {
+            *reinterpret_cast<uint4*>(oh + 8) = make_uint4(ph[4], ph[5], ph[6], ph[7]);
+            *reinterpret_cast<uint4*>(ol + 8) = make_uint4(pl[4], pl[5], pl[6], pl[7]);
+        }
+    }
+}
+// gate|up GEMM of the prefill: columns interleave gate_j (even) and up_j (odd); act_j = silu(gate_j) * up_j is written straight as the hi/lo bf16
+// operand of the down_proj GEMM ([M, N/2] each)
+__device__ __forceinline__ void silu_store16(const GemmArgs& g, int row, int col, const float (&r)[16]) {
+    uint32_t ph[4], pl[4];
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+        const float g0 = r[4 * e], u0 = r[4 * e + 1], g1 = r[4 * e + 2], u1 = r[4 * e + 3];
+        const float a0 = g0 / (1.f + expf(-g0)) * u0, a1 = g1 / (1.f + expf(-g1)) * u1;
+        ph[e] = pack_bf16x2(a0, a1);
+        pl[e] = pack_bf16x2(a0 - bf16lo(ph[e]), a1 - bf16hi(ph[e]));
+    }
+    const size_t o = (size_t)row * g.ldo + (col >> 1);
+    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(g.out) + o) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
+    *reinterpret_cast<uint4*>(reinterpret_cast<uint16_t*>(g.out2) + o) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
+}
+// N is a multiple of 4
+__device__ __forceinline__ void f32_store16(const GemmArgs& g, int row, int col, const float (&r)[16]) {
+    float* o = reinterpret_cast<float*>(g.out) + (size_t)row * g.ldo + col;
+    if (((g.ldo | g.N) & 7) == 0 && (reinterpret_cast<uintptr_t>(g.out) & 31) == 0) {
+#pragma unroll
+        for (int j = 0; j < 16; j += 8)
+            if (col + j < g.N) {
+                const uint32_t v[8] = {__float_as_uint(r[j]), __float_as_uint(r[j + 1]), __float_as_uint(r[j + 2]), __float_as_uint(r[j + 3]),
+                                       __float_as_uint(r[j + 4]), __float_as_uint(r[j + 5]), __float_as_uint(r[j + 6]), __float_as_uint(r[j + 7])};
+                st_global_32b(o + j, v);
+            }
+        return;
+    }
+#pragma unroll
+    for (int j = 0; j < 16; j += 4)
+        if (col + j < g.N) *reinterpret_cast<float4*>(o + j) = make_float4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+}
+
 // Shared-memory matrix descriptor for a K-major bf16 tile stored as rows of 128 bytes with the 128-byte swizzle
 // (exactly what TMA SWIZZLE_128B writes): start address >> 4, LBO = 1 (ignored for swizzled K-major), SBO = 1024 B >> 4
 // (stride between 8-row groups), version = 1 (Blackwell), layout type 2 = SWIZZLE_128B.
@@ -439,36 +504,11 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                         const uint32_t at = tmem_base + as * kAccCols + ((uint32_t)(q * 32) << 16) + (uint32_t)(c0 + h);
                         tmem_ld16(at, rg);
                         tmem_ld16(at + 128u, ru);
-                        const int col = n0 + c0 + h;
-                        if (row < row_lim && col < g.N) {
-                            const bool second = col + 8 < g.N;             // N is a multiple of 8
-                            uint32_t ph[8], pl[8];
+                        if (row < row_lim && n0 + c0 + h < g.N) {
+                            float a[16], b[16];
 #pragma unroll
-                            for (int e = 0; e < 8; ++e) {
-                                float a[2];
-#pragma unroll
-                                for (int i = 0; i < 2; ++i) {
-                                    const int j = 2 * e + i;
-                                    float gv = __uint_as_float(rg[j]), uv = __uint_as_float(ru[j]);
-                                    if (g.bias != nullptr && (e < 4 || second)) { gv += g.bias[col + j]; uv += g.bias[g.N + col + j]; }
-                                    a[i] = glu_value(gv, uv, g.act, g.act_limit);
-                                }
-                                ph[e] = pack_bf16x2(a[0], a[1]);
-                                pl[e] = pack_bf16x2(a[0] - bf16lo(ph[e]), a[1] - bf16hi(ph[e]));
-                            }
-                            uint16_t* oh = reinterpret_cast<uint16_t*>(g.out) + (size_t)row * g.ldo + col;
-                            uint16_t* ol = reinterpret_cast<uint16_t*>(g.out2) + (size_t)row * g.ldo + col;
-                            if (((g.ldo | g.N) & 15) == 0) {
-                                st_global_32b(oh, ph);
-                                st_global_32b(ol, pl);
-                            } else {
-                                *reinterpret_cast<uint4*>(oh) = make_uint4(ph[0], ph[1], ph[2], ph[3]);
-                                *reinterpret_cast<uint4*>(ol) = make_uint4(pl[0], pl[1], pl[2], pl[3]);
-                                if (second) {
-                                    *reinterpret_cast<uint4*>(oh + 8) = make_uint4(ph[4], ph[5], ph[6], ph[7]);
-                                    *reinterpret_cast<uint4*>(ol + 8) = make_uint4(pl[4], pl[5], pl[6], pl[7]);
-                                }
-                            }
+                            for (int j = 0; j < 16; ++j) { a[j] = __uint_as_float(rg[j]); b[j] = __uint_as_float(ru[j]); }
+                            glu_store16(g, row, n0 + c0 + h, a, b);
                         }
                         __syncwarp();
                     }

@@ -172,8 +172,6 @@ struct LayeredCache {
     // tensor-core latent attention of long portions: gathered keys, their transpose, Q / P operand halves, the score block
     DevBuf<uint16_t> at_kc, at_kct, at_qhi, at_qlo, at_phi, at_plo;
     DevBuf<float> at_part;              // attention with key splits: partial (max, sum, values) per (row, head, split)
-    bool may_fail = false;              // the step launched kernels that report failures in at_failed
-    PinnedBuf<int> at_failed;           // one word: a block of the fused attention kernel gave up (read by layered_finish)
     DevBuf<float> at_s, at_o;           // at_o: grouped-query attention, the value GEMMs' outputs per key/value head before they are interleaved
 };
 
@@ -190,7 +188,6 @@ void layered_cache_create(fl_cache& c, int max_slots, int max_seq, int pool_toke
 // one step of a mixed batch; logits of the wanted rows land in c.ly->logits (device)
 void layered_forward(fl_cache& c, const int* slots, const int* counts, int n, const uint32_t* ids, const int* want, int n_want);
 void layered_finish(fl_cache& c);        // waits for the step; throws when one of its kernels reported a failure
-void layered_check(fl_cache& c);         // the same behind a step that is waited for
 void layered_slot_reset(fl_cache& c, int slot);
 void layered_cache_reset(fl_cache& c);
 }  // namespace fl

@@ -295,3 +295,31 @@ def test_steps_that_grow(mod, cfg):
         cache.slot_reset(0)
         want = model.new_device_cache(1, 1024).forward_ragged([0], [toks[:n]], [[0, n - 1]])
         assert mod.relerr(cache.forward_ragged([0], [toks[:n]], [[0, n - 1]]), np.asarray(want, dtype=np.float64)) < CHUNK_TOL
+
+
+# ---- GEMMs on pairs of SMs (gemm_pair.cuh): from 1024 rows on, where whole waves of pair tiles leave a few that are cut along K ------------------
+def test_pairs_llama():
+    """1290 rows: the last pair row ends inside its second half; o and gate|up leave 16 tiles to cut, which end inside a k block's run"""
+    from fastllm_b200 import models
+    from helpers import product_model
+    from oracle import causal_lm as ocl
+    from oracle import synth
+    cfg = ocl.CausalLMConfig("llama", 3840, 1920, 1000, 1, 30, 5, 1e-5, 1e4, 1536)
+    w = ocl.synth_weights(cfg, 0, 0.5 * 3840 ** -0.5)
+    model = product_model(cfg, w)[0]
+    ids = synth.token_ids(9, 1000, (1, 1290))
+    cache = models.DeviceCache(model.dev, 1, 1536)
+    want = ocl.CausalLM(cfg, w, kv_dtype="bf16").forward(ids, 0)
+    for _ in range(2):                          # (the tiles' tickets are back at zero after a call)
+        cache.reset()
+        assert np.abs(cache.forward(ids, 0) - want).max() <= 3e-3
+
+
+def test_pairs_gated_epilogue():
+    """the gated epilogue on pairs (1290 rows) against the same tokens in portions that stay on single tiles"""
+    cfg = R.config([R.mamba(heads=4, vdim=32, state=32, groups=2, mlp=R.dense(ff=1920))], vocab=64, width=3072)
+    _, model = R.build(cfg, seed=71, dtype="bf16")
+    toks = R.tokens(cfg, 1290, seed=72)
+    cut = R.run_cut(model, toks, [650, 640], cache=model.new_device_cache(1, 1536))
+    whole = R.run_whole(model, toks, cache=model.new_device_cache(1, 1536))
+    assert R.relerr(whole, np.asarray(cut, dtype=np.float64)) < CHUNK_TOL
