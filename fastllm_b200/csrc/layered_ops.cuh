@@ -188,24 +188,12 @@ static __global__ void ly_embed_norm_kernel(const uint16_t* __restrict__ embed, 
         for (int c = threadIdx.x; c < W; c += blockDim.x) { const float v = __uint_as_float((uint32_t)e[c] << 16); es += v * v; }
         er = 1.f / sqrtf(block_sum(es, red) / (float)W + eps);
     }
-    for (int c0 = threadIdx.x; c0 < W; c0 += 4 * blockDim.x) {
-      float ev[4], pv[4], bv[4];               // four channels' loads together (the stores between them would hold them apart)
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-          const int c = c0 + k * blockDim.x;
-          ev[k] = c < W ? __uint_as_float((uint32_t)e[c] << 16) : 0.f;
-          pv[k] = pe && c < W ? __uint_as_float((uint32_t)pe[c] << 16) : 0.f;
-          bv[k] = be && c < W ? __uint_as_float((uint32_t)be[c] << 16) : 0.f;
-      }
-#pragma unroll
-      for (int k = 0; k < 4; ++k) {
-        const int c = c0 + k * blockDim.x;
-        if (c >= W) break;
-        float v = ev[k];
+    for (int c = threadIdx.x; c < W; c += blockDim.x) {
+        float v = __uint_as_float((uint32_t)e[c] << 16);
         if (en != nullptr) v *= er * norm_scale(en, c, plain);
         if (escale != 0.f) v *= escale;
-        if (pe) v += pv[k];
-        if (be) v += bv[k];
+        if (pe) v += __uint_as_float((uint32_t)pe[c] << 16);
+        if (be) v += __uint_as_float((uint32_t)be[c] << 16);
         if (x0) x0[(size_t)row * W + c] = v;
         if (step) v += step[c];
         xr[c] = v;
@@ -216,7 +204,6 @@ static __global__ void ly_embed_norm_kernel(const uint16_t* __restrict__ embed, 
             if (h) h[(size_t)row * W + c] = v;
             split_store(hhi, hlo, (size_t)row * W + c, v);
         }
-      }
     }
     if (nw.w == nullptr || nw.alpha != nullptr) return;
     const float r = 1.f / sqrtf(block_sum(ss, red) / (float)W + eps);
@@ -1579,6 +1566,7 @@ static __global__ void __launch_bounds__(256) ly_attn_softmax_warp_kernel(const 
 struct KvLayout {
     int E, ks, vo, vs, roll;
 };
+constexpr int kPrepAheadDim = 128, kPrepAheadRows = 512;
 struct AttnPrepArgs {
     float* proj; int ldp, off_q, off_k, off_v;  // off_k < 0: the layer reads another layer's cache (queries are still prepared)
     const float *qnorm, *knorm; float eps;       // [dim] each ([H * dim], [G * dim] when `whole`)
@@ -1598,7 +1586,8 @@ struct AttnPrepArgs {
 // take the heads in turn.  Biases, when the projections have them, are added as the values are read; with `whole` the mean square is
 // taken over all heads of q (of k) before any head is rewritten (one block per row then: gridDim.y = 1) and the weight is indexed by
 // the channel inside the whole projection.
-template <typename CT>
+// AHEAD (steps of few rows, heads of up to 128 channels): see below.
+template <typename CT, bool AHEAD>
 static __global__ void __launch_bounds__(256) ly_attn_prep_kernel(AttnPrepArgs a) {
     pdl_chain();
     extern __shared__ float sm[];               // [warps][D]
@@ -1631,10 +1620,10 @@ static __global__ void __launch_bounds__(256) ly_attn_prep_kernel(AttnPrepArgs a
     const float* sn = a.sinb + (size_t)pos * half;
     float* buf = sm + wid * a.D;
     const int items = a.H + (own ? a.G : 0);
-    // heads of up to 128 channels: a lane's channels, weights and turns in registers, the next head's values on their way while this one is
-    // turned (one dependent load after the other -- values, weights, turns, of every head -- a row of 20 heads was 18 us)
-    constexpr int NC = 4;
-    const bool narrow = a.D <= 32 * NC;
+    // a lane's channels, weights and turns in registers, the next head's values on their way while this one is turned: one dependent load after
+    // the other -- values, weights, turns, of every head -- 8 rows of 40 heads were 9.8 us (7.0 now), 340 rows of 20 heads 24 (20).  Where rows
+    // fill the chip the registers cost more blocks than that is worth (2048 rows of 40 heads: 56 us without, 84 with).
+    constexpr int NC = kPrepAheadDim / 32;
     float cj[NC], sj[NC];
     auto place = [&](int c, int& pi) { if (a.halves) { pi = c >= half ? c - half : c; return c >= half; } pi = c >> 1; return (c & 1) != 0; };
     auto fetch = [&](int it, float (&v)[NC], float (&w)[NC]) {
@@ -1649,7 +1638,7 @@ static __global__ void __launch_bounds__(256) ly_attn_prep_kernel(AttnPrepArgs a
             w[j] = wn != nullptr && c < a.D ? wn[a.whole ? (size_t)hd * a.D + c : (size_t)c] : 0.f;
         }
     };
-    if (narrow) {
+    if constexpr (AHEAD) {
 #pragma unroll
         for (int j = 0; j < NC; ++j) {
             const int c = lane + 32 * j;
@@ -1704,7 +1693,7 @@ static __global__ void __launch_bounds__(256) ly_attn_prep_kernel(AttnPrepArgs a
             for (int j = 0; j < NC; ++j) { v[j] = nv[j]; w[j] = nwt[j]; }
         }
     }
-    for (int it = blockIdx.y * nw + wid; !narrow && it < items; it += gridDim.y * nw) {
+    for (int it = blockIdx.y * nw + wid; !AHEAD && it < items; it += gridDim.y * nw) {
         const bool isq = it < a.H;
         const int hd = isq ? it : it - a.H;
         const int src = (isq ? a.off_q : a.off_k) + hd * a.D;
