@@ -17,6 +17,7 @@ struct BertLayerW {
     float *bqkv = nullptr, *bo = nullptr, *bi = nullptr, *bo2 = nullptr;
     float *ln1w = nullptr, *ln1b = nullptr, *ln2w = nullptr, *ln2b = nullptr;
     CUtensorMap tm_wqkv, tm_wo, tm_wi, tm_wo2;
+    CUtensorMap tb_wo, tb_wi, tb_wo2;       // the boxes of bert_block_kernel
 };
 
 struct BertModel {
@@ -31,12 +32,13 @@ struct BertModel {
     cudaStream_t stream = nullptr;
     std::mutex mu;
     // workspace (grown on demand)
-    size_t cap_tokens = 0, cap_batch = 0;
+    size_t cap_tokens = 0, cap_batch = 0, cap_chain = 0;
     DevBuf<uint16_t> x, x1, ctx, qkv, hbuf;
     DevBuf<float> pre, out;
     DevBuf<uint32_t> ids, mask;
     PinnedBuf<uint32_t> h_ids;
     PinnedBuf<float> h_out;
+    PinnedBuf<int> failed;                  // one word: a wait inside a kernel ran out
     void* small_layers = nullptr;           // in the slab: the layers' pointers for the one-launch kernel (null: other sizes than it is built for)
     ~BertModel();
 };

@@ -4,6 +4,7 @@
 #include <memory>
 
 #include "bert.cuh"
+#include "bert_block.cuh"
 #include "bert_small.cuh"
 #include "bert_model.cuh"
 #include "gemm_tc.cuh"
@@ -151,6 +152,8 @@ void bert_build(BertModel& m) {
         w.ln1w = (float*)(b + l.l1w); w.ln1b = (float*)(b + l.l1b); w.ln2w = (float*)(b + l.l2w); w.ln2b = (float*)(b + l.l2b);
     }
     FL_CUDA(cudaStreamCreateWithFlags(&m.stream, cudaStreamNonBlocking));
+    m.failed.alloc(1);
+    *m.failed.p = 0;
 }
 
 struct BertRoute {
@@ -267,6 +270,9 @@ void bert_finalize(BertModel& m) {
         w.tm_wo = make_tmap_bf16(w.wo, m.H, m.H, m.H, kBertBN);
         w.tm_wi = make_tmap_bf16(w.wi, m.I, m.H, m.H, kBertBN);
         w.tm_wo2 = make_tmap_bf16(w.wo2, m.H, m.I, m.I, kBertBN);
+        w.tb_wo = make_tmap_bf16(w.wo, m.H, m.H, m.H, 96);
+        w.tb_wi = make_tmap_bf16(w.wi, m.I, m.H, m.H, 64);
+        w.tb_wo2 = make_tmap_bf16(w.wo2, m.H, m.I, m.I, 96);
     }
     if (m.small_layers != nullptr) {
         std::vector<BertSmallLayer> tab;
@@ -276,14 +282,41 @@ void bert_finalize(BertModel& m) {
     m.finalized = true;
 }
 
+static int bert_block_clusters() {       // pairs of SMs that can be resident at once (the driver's answer)
+    static const int n = [] {
+        if (cudaFuncSetAttribute(bert_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBbSmem) != cudaSuccess) { cudaGetLastError(); return 0; }
+        cudaLaunchConfig_t cfg{};
+        cfg.gridDim = dim3(kNumSMs); cfg.blockDim = dim3(kBbThreads); cfg.dynamicSmemBytes = kBbSmem;
+        cudaLaunchAttribute at[1];
+        at[0].id = cudaLaunchAttributeClusterDimension;
+        at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+        cfg.attrs = at; cfg.numAttrs = 1;
+        int k = 0;
+        if (cudaOccupancyMaxActiveClusters(&k, bert_block_kernel, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+        return std::min(k, kNumSMs / 2);
+    }();
+    return n;
+}
+// A pair of SMs takes about 65 us for 256 tokens however many tiles there are, the chain's kernels grow with the tokens: whole encoder, chain ->
+// blocks, us, by tiles of 256 tokens: 32 (64 x 128) 576 -> 605, 46 (154 x 76) 781 -> 673, 64 930 -> 764, 74 999 -> 807, 80 (two waves) 1159 ->
+// 1199, 128 1719 -> 1437.
+static bool bert_blocks(const BertModel& m, int T) {
+    if (m.H != kBbH || m.I != kBbI) return false;
+    const int n = bert_block_clusters(), tiles = (T + 255) / 256;
+    return n > 0 && 5 * tiles >= 3 * n * ((tiles + n - 1) / n);
+}
 static void bert_reserve(BertModel& m, int b, int t) {
     const size_t T = (size_t)b * t;
-    if (T <= m.cap_tokens && (size_t)b <= m.cap_batch) return;
     const size_t H = m.H, I = m.I;
+    if (!bert_blocks(m, (int)T) && T > m.cap_chain) {       // what the launch chain alone reads
+        m.cap_chain = T;
+        m.x1.alloc(T * H); m.hbuf.alloc(T * I); m.pre.alloc(T * H);
+    }
+    if (T <= m.cap_tokens && (size_t)b <= m.cap_batch) return;
     m.cap_tokens = std::max(T, m.cap_tokens);
     m.cap_batch = std::max((size_t)b, m.cap_batch);
     const size_t Tc = m.cap_tokens;
-    m.x.alloc(Tc * H); m.x1.alloc(Tc * H); m.ctx.alloc(Tc * H); m.qkv.alloc(Tc * 3 * H); m.hbuf.alloc(Tc * I); m.pre.alloc(Tc * H);
+    m.x.alloc(Tc * H); m.ctx.alloc(Tc * H); m.qkv.alloc(Tc * 3 * H);
     m.ids.alloc(Tc); m.mask.alloc(Tc); m.out.alloc(m.cap_batch * H);
     m.h_ids.alloc(2 * Tc); m.h_out.alloc(m.cap_batch * H);
 }
@@ -340,6 +373,14 @@ static bool bert_enqueue_small(BertModel& m, int b, int t, bool has_mask) {
     return true;
 }
 
+static void launch_bert_block(BertModel& m, const CUtensorMap& tm_ctx, const CUtensorMap& tm_x, const BertLayerW& w, int T, float eps) {
+    const BertBlockArgs a{T, m.x.p, w.bo, w.bi, w.bo2, w.ln1w, w.ln1b, w.ln2w, w.ln2b, eps, m.failed.p};
+    blaunch(m.stream, bert_block_kernel, dim3(2 * std::min((T + 255) / 256, bert_block_clusters())), dim3(kBbThreads), kBbSmem, tm_ctx, w.tb_wo, w.tb_wi, w.tb_wo2, tm_x, a);
+}
+static void bert_check(const BertModel& m) {
+    FL_CHECK(*m.failed.p == 0, FL_ERR_CUDA, "a wait inside a kernel ran out, the results are not valid");
+}
+
 // Enqueue the encoder on m.stream: B1 -> 6 x (B2..B7) -> B8
 static void bert_enqueue(BertModel& m, int b, int t, bool has_mask) {
     if (bert_enqueue_small(m, b, t, has_mask)) return;
@@ -349,8 +390,10 @@ static void bert_enqueue(BertModel& m, int b, int t, bool has_mask) {
     const dim3 row_grid((T + rows_per_cta - 1) / rows_per_cta), row_block(rows_per_cta * 32);
     blaunch(st, embed_ln_kernel, row_grid, row_block, 0, (const uint16_t*)m.wemb, (const uint16_t*)m.pemb, (const float*)m.lnw, (const float*)m.lnb,
             (const uint32_t*)m.ids.p, T, t, H, m.V, m.maxpos, 1e-12f, m.x.p);
-    const CUtensorMap tm_x = make_tmap_bf16(m.x.p, T, H, H, kGemmBM), tm_x1 = make_tmap_bf16(m.x1.p, T, H, H, kGemmBM),
-                      tm_ctx = make_tmap_bf16(m.ctx.p, T, H, H, kGemmBM), tm_h = make_tmap_bf16(m.hbuf.p, T, I, I, kGemmBM);
+    const bool blocks = bert_blocks(m, T);
+    const CUtensorMap tm_x = make_tmap_bf16(m.x.p, T, H, H, kGemmBM), tm_x1 = blocks ? tm_x : make_tmap_bf16(m.x1.p, T, H, H, kGemmBM),
+                      tm_ctx = make_tmap_bf16(m.ctx.p, T, H, H, kGemmBM);
+    const CUtensorMap tm_h = blocks ? tm_x : make_tmap_bf16(m.hbuf.p, T, I, I, kGemmBM);
     const float eps = m.cfg.norm_eps;
     const float scale = (float)std::sqrt((double)m.d);
     for (int l = 0; l < m.L; ++l) {
@@ -362,6 +405,10 @@ static void bert_enqueue(BertModel& m, int b, int t, bool has_mask) {
             blaunch(st, bert_attn_kernel, dim3(m.nh, b), dim3(128), 0, (const uint16_t*)m.qkv.p, t, H, scale, m.ctx.p);
         else
             blaunch(st, bert_attn_long_kernel, dim3(m.nh, b, (t + kBertS - 1) / kBertS), dim3(128), 0, (const uint16_t*)m.qkv.p, t, H, scale, m.ctx.p);
+        if (blocks) {       // B5 to B7 in one kernel
+            launch_bert_block(m, tm_ctx, tm_x, w, T, eps);
+            continue;
+        }
         // B5: attention output dense + bias + residual -> f32, then LayerNorm -> bf16
         launch_gemm<GEPI_BIAS_RESID_F32>(st, tm_ctx, w.tm_wo, GemmArgs{T, H, H, w.bo, m.x.p, H, m.pre.p, H, 1, 0});
         blaunch(st, layernorm_kernel, row_grid, row_block, 0, (const float*)m.pre.p, (const float*)w.ln1w, (const float*)w.ln1b, T, H, eps, m.x1.p);
@@ -402,6 +449,7 @@ void bert_embed(BertModel& m, const uint32_t* ids, const uint32_t* mask, int b, 
     FL_CUDA(cudaGetLastError());
     FL_CUDA(cudaMemcpyAsync(m.h_out.p, m.out.p, (size_t)b * m.H * 4, cudaMemcpyDeviceToHost, m.stream));
     FL_CUDA(cudaStreamSynchronize(m.stream));
+    bert_check(m);
     std::memcpy(out, m.h_out.p, (size_t)b * m.H * 4);
     if (device_ms) FL_CUDA(cudaEventElapsedTime(device_ms, ev->e0, ev->e1));
 }
@@ -416,6 +464,7 @@ void bert_repeat(BertModel& m, int b, int t, int iters, float* elapsed_ms) {
     FL_CUDA(cudaEventRecord(ev.e1, m.stream));
     FL_CUDA(cudaStreamSynchronize(m.stream));
     FL_CUDA(cudaGetLastError());
+    bert_check(m);
     FL_CUDA(cudaEventElapsedTime(elapsed_ms, ev.e0, ev.e1));
 }
 

@@ -88,11 +88,11 @@ __device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
                  : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // false when the wait ran out (seconds): the caller leaves its loop
 __device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity) {
-    for (int i = 0; i < (1 << 22); ++i) {
+    for (int i = 0; i < (1 << 20); ++i) {
         uint32_t done;
         asm volatile(
             "{\n"
