@@ -6,10 +6,9 @@
 // and half of every weight tile.  The 1536-wide activations exist 128 columns at a time: S (128 TMEM columns) -> GELU -> shared memory -> O (384
 // columns).  The tensor core alternates between the next columns' S and the last columns' O while the epilogue warps turn S into operands.
 // As five launches every layer moved 100 to 200 MB of activations between kernels that each waited for HBM and for their epilogues' stores
-// (256 x 128 tokens, whole encoder: 1.72 ms; 1.44 in this form).  What bounds it: 3.4 us per 128 intermediate columns, where the products alone take
-// 1.6 (measured by themselves: 3090 clocks) and the GELUs 1.0; the weight stages are there in time, so what slows the products is the shared memory that
-// they read (256 KB per 128 columns and CTA) while the stages (96 KB) and the operands (32 KB) are written.  8 epilogue warps: 16 were no faster
-// (the tanh unit is the limit of both).
+// (256 x 128 tokens, whole encoder: 1.76 ms; 1.28 in this form).  What bounds it: per 128 intermediate columns the products take 1.6 us (3090 clocks,
+// measured by themselves) and the GELUs 1.0 (the tanh unit), one epilogue warp of them waiting for the other now and then; 5 us in front and 6 behind for
+// the two norms.  8 epilogue warps: 16 were no faster.
 #pragma once
 #include "gemm_pair.cuh"
 
@@ -45,7 +44,7 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
     uint8_t* sW = sH + kBbHid;
     __shared__ __align__(8) uint64_t w_full[kBbStages], w_empty[kBbStages], a_full, x_ready, x_free, s_full, s_free, h_ready, h_free, o_full;
     __shared__ uint32_t tmem_base_s;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int cl = blockIdx.x >> 1, G = gridDim.x >> 1, tiles = (g.T + 255) / 256;
 
@@ -114,63 +113,58 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {             // (the whole warp, see uniform_warp; a wait that ran out ends the waiting, not the walk)
             constexpr uint32_t id1 = umma_idesc_bf16(256, 128), id2 = umma_idesc_bf16(256, 192);
             const uint64_t dX = umma_smem_desc_sw128(sX), dH = umma_smem_desc_sw128(sH), dW = umma_smem_desc_sw128(sW);
-            int st = 0;
-            uint32_t ph = 0;
-            auto acquire = [&]() {
-                if (ok) ok = pair_wait(&w_full[st], ph);
+            uint32_t n = 0;                         // stages so far
+            auto wait = [&](uint64_t* bar, uint32_t parity) {
+                if (ok) ok = pair_wait(bar, parity);
+                __syncwarp();
                 tc_fence_after();
-                return dW + (uint64_t)(st * (kBbStage >> 4));
             };
-            auto release = [&]() {
-                umma_commit_pair(&w_empty[st]);
-                if (++st == kBbStages) { st = 0; ph ^= 1; }
-            };
-            // O (two halves of 192 columns) += A (one k block) . the stage
+            // O (two halves of 192 columns) += A (one k block) . the next stage
             auto out = [&](uint64_t a, uint32_t acc) {
-                const uint64_t b = acquire();
-                if (!ok) return;
+                const uint32_t st = n % kBbStages;
+                const uint64_t b = dW + (uint64_t)(st * (kBbStage >> 4));
+                wait(&w_full[st], (n / kBbStages) & 1);
 #pragma unroll
-                for (int n = 0; n < 2; ++n)
+                for (int h = 0; h < 2; ++h)
 #pragma unroll
-                    for (int q = 0; q < 4; ++q) umma_bf16_pair(tmem + n * 192, a + 2 * q, b + (uint64_t)(n * (12288 >> 4) + 2 * q), id2, q ? 1u : acc);
-                release();
+                    for (int q = 0; q < 4; ++q) umma_bf16_pair_warp(tmem + h * 192, a + 2 * q, b + (uint64_t)(h * (12288 >> 4) + 2 * q), id2, q ? 1u : acc);
+                umma_commit_pair_warp(&w_empty[st]);
+                ++n;
             };
             uint32_t chunk = 0;                     // over all tiles
             int it = 0;
-            for (int tile = cl; ok && tile < tiles; tile += G, ++it) {
-                if (!(ok = pair_wait(&a_full, it & 1))) break;
-                tc_fence_after();
-                for (int k = 0; ok && k < kBbKb; ++k) out(dX + (uint64_t)(k * 1024), k ? 1u : 0u);
-                umma_commit_pair(&o_full);
-                if (!ok || !(ok = pair_wait(&x_ready, it & 1))) break;
-                tc_fence_after();
-                for (int j = 0; ok && j <= kBbChunks; ++j) {
+            for (int tile = cl; tile < tiles; tile += G, ++it) {
+                wait(&a_full, it & 1);
+                for (int k = 0; k < kBbKb; ++k) out(dX + (uint64_t)(k * 1024), k ? 1u : 0u);
+                umma_commit_pair_warp(&o_full);
+                wait(&x_ready, it & 1);
+                for (int j = 0; j <= kBbChunks; ++j) {
                     if (j < kBbChunks) {
-                        if (!(ok = pair_wait(&s_free, ((chunk + j) & 1) ^ 1))) break;
-                        tc_fence_after();
-                        for (int p = 0; ok && p < 2; ++p) {
-                            const uint64_t b = acquire();
-                            if (!ok) break;
+                        wait(&s_free, ((chunk + j) & 1) ^ 1);
+                        for (int p = 0; p < 2; ++p) {
+                            const uint32_t st = n % kBbStages;
+                            const uint64_t b = dW + (uint64_t)(st * (kBbStage >> 4)), a = dX + (uint64_t)(p * 3 * 1024);
+                            wait(&w_full[st], (n / kBbStages) & 1);
 #pragma unroll
                             for (int k = 0; k < 3; ++k)
 #pragma unroll
                                 for (int q = 0; q < 4; ++q)
-                                    umma_bf16_pair(tS, dX + (uint64_t)((p * 3 + k) * 1024 + 2 * q), b + (uint64_t)(k * (8192 >> 4) + 2 * q), id1, (p | k | q) ? 1u : 0u);
-                            release();
+                                    umma_bf16_pair_warp(tS, a + (uint64_t)(k * 1024 + 2 * q), b + (uint64_t)(k * (8192 >> 4) + 2 * q), id1, (k | q) ? 1u : (uint32_t)p);
+                            umma_commit_pair_warp(&w_empty[st]);
+                            ++n;
                         }
-                        umma_commit_pair(&s_full);
+                        umma_commit_pair_warp(&s_full);
                     }
-                    if (j > 0 && ok) {
-                        if (!(ok = pair_wait(&h_ready, (chunk + j - 1) & 1))) break;
-                        tc_fence_after();
-                        for (int k = 0; ok && k < 2; ++k) out(dH + (uint64_t)(k * 1024), (j > 1 || k) ? 1u : 0u);
-                        umma_commit_pair(&h_free);
+                    if (j > 0) {
+                        wait(&h_ready, (chunk + j - 1) & 1);
+                        for (int k = 0; k < 2; ++k) out(dH + (uint64_t)(k * 1024), (j > 1 || k) ? 1u : 0u);
+                        umma_commit_pair_warp(&h_free);
                     }
                 }
-                umma_commit_pair(&o_full);
+                umma_commit_pair_warp(&o_full);
                 chunk += kBbChunks;
             }
         }

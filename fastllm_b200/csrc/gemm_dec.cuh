@@ -71,7 +71,7 @@ gemm_dec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
     uint8_t* gsm = gsm_raw + ((1024u - (smem_u32(gsm_raw) & 1023u)) & 1023u);
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base_s;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int nks = g.nks;
     const int tiles = (g.N + kGemmBM - 1) / kGemmBM;
     const int u0 = blockIdx.x * g.L, u1 = min(u0 + g.L, tiles * nks);       // this block's stages of the flattened (tile, k) walk
@@ -123,7 +123,7 @@ gemm_dec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
             }
         }
     } else if (warp == 1) {
-        if (lane == 0) {
+        {                                                         // the whole warp, one elected lane issues (see uniform_warp)
             constexpr uint32_t idesc = umma_idesc_bf16(kGemmBM, 2 * BN);
             const uint64_t base = umma_smem_desc_sw128(gsm);
             int st = 0;
@@ -142,13 +142,13 @@ gemm_dec_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__
                     for (int k = 0; k < KS; ++k) {
                         const uint64_t a = sd + (uint64_t)((k * S::kW) >> 4), b = sd + (uint64_t)((KS * S::kW + 2 * k * S::kX) >> 4);
 #pragma unroll
-                        for (int q = 0; q < kGemmBK / 16; ++q) umma_bf16(tacc, a + 2 * q, b + 2 * q, idesc, (k | q) ? 1u : acc);
+                        for (int q = 0; q < kGemmBK / 16; ++q) umma_bf16_warp(tacc, a + 2 * q, b + 2 * q, idesc, (k | q) ? 1u : acc);
                     }
                     acc = 1;
-                    umma_commit(&empty[st]);
+                    umma_commit_warp(&empty[st]);
                     if (++st == kStages) { st = 0; ph ^= 1; }
                 }
-                umma_commit(&acc_full[as]);
+                umma_commit_warp(&acc_full[as]);
             }
         }
     } else {

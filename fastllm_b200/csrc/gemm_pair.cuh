@@ -72,20 +72,28 @@ __device__ __forceinline__ void tma_load_2d_pair(uint32_t dst, const CUtensorMap
                  "r"(c0), "r"(c1), "r"(mbar)
                  : "memory");
 }
-__device__ __forceinline__ void umma_bf16_pair(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+// a whole warp: one elected lane issues
+__device__ __forceinline__ void umma_bf16_pair_warp(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
     asm volatile(
         "{\n"
-        ".reg .pred p;\n"
+        ".reg .pred p, e;\n"
         "setp.ne.b32 p, %4, 0;\n"
-        "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
+        "elect.sync _|e, 0xFFFFFFFF;\n"
+        "@e tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n"
         "}\n" ::"r"(tmem_d),
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-// arrives on the barrier of both CTAs when all previously issued products of this thread have completed
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;" ::"r"(smem_u32(bar)), "h"((uint16_t)3)
-                 : "memory");
+// arrives on the barrier of both CTAs when all products issued so far have completed
+__device__ __forceinline__ void umma_commit_pair_warp(uint64_t* bar) {
+    asm volatile(
+        "{\n"
+        ".reg .pred e;\n"
+        "elect.sync _|e, 0xFFFFFFFF;\n"
+        "@e tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n"
+        "}\n" ::"r"(smem_u32(bar)),
+        "h"((uint16_t)3)
+        : "memory");
 }
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
     asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
@@ -119,7 +127,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant_
     __shared__ __align__(8) uint64_t full[kPairStages], empty[kPairStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base_s;
     __shared__ int s_last;
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int cl = blockIdx.x >> 1, G = gridDim.x >> 1, nk = p.nk, T = p.mp * p.nt;
     const int left0 = p.full * G, units = (T - left0) * nk;
@@ -191,28 +199,31 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmH, const __grid_constant_
             }
         }
     } else if (warp == 1) {
-        if (lane == 0 && rank == 0) {
+        if (rank == 0) {             // the whole warp, one elected lane issues (see uniform_warp); a wait that ran out ends the waiting, not the walk
             constexpr uint32_t idesc = umma_idesc_bf16(256, 256);
             const uint64_t base = umma_smem_desc_sw128(gsm);
             Walk w;
             int tile, kb0, kb1, st = 0;
             uint32_t ph = 0, seg = 0;
-            while (ok && next(w, tile, kb0, kb1)) {
-                const uint32_t as = seg & 1, tacc = tmem_base + as * 256;
-                if (!(ok = pair_wait(&acc_empty[as], ((seg >> 1) & 1) ^ 1))) break;
+            auto wait = [&](uint64_t* bar, uint32_t parity) {
+                if (ok) ok = pair_wait(bar, parity);
+                __syncwarp();
                 tc_fence_after();
+            };
+            while (next(w, tile, kb0, kb1)) {
+                const uint32_t as = seg & 1, tacc = tmem_base + as * 256;
+                wait(&acc_empty[as], ((seg >> 1) & 1) ^ 1);
                 for (int kb = kb0; kb < kb1; ++kb) {
-                    if (!(ok = pair_wait(&full[st], ph))) break;
-                    tc_fence_after();
+                    wait(&full[st], ph);
                     const uint64_t ah = base + (uint64_t)(st * (kPairStage >> 4)), al = ah + (kPairABytes >> 4), b = al + (kPairABytes >> 4);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) umma_bf16_pair(tacc, ah + 2 * k, b + 2 * k, idesc, ((kb - kb0) | k) ? 1u : 0u);
+                    for (int k = 0; k < 4; ++k) umma_bf16_pair_warp(tacc, ah + 2 * k, b + 2 * k, idesc, ((kb - kb0) | k) ? 1u : 0u);
 #pragma unroll
-                    for (int k = 0; k < 4; ++k) umma_bf16_pair(tacc, al + 2 * k, b + 2 * k, idesc, 1u);
-                    umma_commit_pair(&empty[st]);
+                    for (int k = 0; k < 4; ++k) umma_bf16_pair_warp(tacc, al + 2 * k, b + 2 * k, idesc, 1u);
+                    umma_commit_pair_warp(&empty[st]);
                     if (++st == kPairStages) { st = 0; ph ^= 1; }
                 }
-                umma_commit_pair(&acc_full[as]);
+                umma_commit_pair_warp(&acc_full[as]);
                 ++seg;
             }
         }

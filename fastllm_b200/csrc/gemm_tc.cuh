@@ -108,6 +108,30 @@ __device__ __forceinline__ void umma_bf16(uint32_t tmem_d, uint64_t adesc, uint6
         "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// A role's warp index that the compiler knows to be the same in all lanes.  The issuing warps walk their loops with all 32 lanes and one elected
+// lane issues: descriptors then stay in uniform registers, which the instruction wants; in a branch of one lane every descriptor is moved there
+// first, and products of 64 to 96 clocks were issued 110 apart.
+__device__ __forceinline__ int uniform_warp() { return __shfl_sync(0xFFFFFFFFu, (int)(threadIdx.x >> 5), 0); }
+__device__ __forceinline__ void umma_bf16_warp(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+    asm volatile(
+        "{\n"
+        ".reg .pred p, e;\n"
+        "setp.ne.b32 p, %4, 0;\n"
+        "elect.sync _|e, 0xFFFFFFFF;\n"
+        "@e tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n"
+        "}\n" ::"r"(tmem_d),
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void umma_commit_warp(uint64_t* bar) {
+    asm volatile(
+        "{\n"
+        ".reg .pred e;\n"
+        "elect.sync _|e, 0xFFFFFFFF;\n"
+        "@e tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n"
+        "}\n" ::"r"(smem_u32(bar))
+        : "memory");
+}
 // arrives on the mbarrier when all previously issued tcgen05.mma of this thread have completed
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
@@ -300,7 +324,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
     __shared__ __align__(8) uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2];
     __shared__ uint32_t tmem_base_s;
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const int nk = (g.K + kGemmBK - 1) / kGemmBK;
     const bool grouped = (DUAL == DUAL_B) && g.grp_m > 0;
     const int mt_e = grouped ? (g.grp_m + kGemmBM - 1) / kGemmBM : 0;      // m tiles per group
@@ -437,8 +461,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
         }
     } else if (warp == 1) {
-        // ===== MMA issuer (single thread) =====
-        if (lane == 0) {
+        // ===== MMA issuer (one elected lane issues) =====
+        {
             constexpr uint32_t idesc = umma_idesc_bf16(kGemmBM, kMmaN);
             uint32_t c = 0, ti = 0;
             if (grouped || runs) pdl_wait();      // grp_cnt / tile_off is written by a preceding kernel
@@ -460,15 +484,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
                     const uint64_t adesc = umma_smem_desc_sw128(sa), bdesc = umma_smem_desc_sw128(sa + kBOff);
 #pragma unroll
                     for (int k = 0; k < kGemmBK / 16; ++k)   // advance 16 elements = 32 bytes inside the swizzle row: +2 in the (>>4) address field
-                        umma_bf16(tacc, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, ((kb - kb0) | k) ? 1u : 0u);
+                        umma_bf16_warp(tacc, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, ((kb - kb0) | k) ? 1u : 0u);
                     if (DUAL == DUAL_A) {
                         const uint64_t a2desc = umma_smem_desc_sw128(sa + kABytes);
 #pragma unroll
-                        for (int k = 0; k < kGemmBK / 16; ++k) umma_bf16(tacc, a2desc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, 1u);
+                        for (int k = 0; k < kGemmBK / 16; ++k) umma_bf16_warp(tacc, a2desc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc, 1u);
                     }       // DUAL_B: the first loop already covered hi | lo (N = 2 BN)
-                    umma_commit(&empty[st]);                 // slot reusable once these MMAs have read it
+                    umma_commit_warp(&empty[st]);            // slot reusable once these MMAs have read it
                 }
-                umma_commit(&acc_full[as]);                  // accumulator of this tile complete
+                umma_commit_warp(&acc_full[as]);             // accumulator of this tile complete
             }
         }
     } else {
