@@ -298,8 +298,8 @@ static int bert_block_clusters() {       // pairs of SMs that can be resident at
     return n;
 }
 // A pair of SMs takes about as long for 256 tokens however many tiles there are, the chain's kernels grow with the tokens: whole encoder, chain ->
-// blocks, us, by tiles of 256 tokens: 32 (64 x 128) 576 -> 530, 50 (100 x 128) 810 -> 609, 64 930 -> 699, 74 999 -> 738, 80 (two waves) 1159 -> 1090,
-// 128 1719 -> 1283.
+// blocks, us, by tiles of 256 tokens: 46 781 -> 591, 64 930 -> 699, 74 999 -> 738, 128 (two waves) 1719 -> 1283. The line was drawn with blocks that
+// took 12 % longer than today's: 32 tiles 576 -> 605, 80 (two waves) 1159 -> 1199.
 static bool bert_blocks(const BertModel& m, int T) {
     if (m.H != kBbH || m.I != kBbI) return false;
     const int n = bert_block_clusters(), tiles = (T + 255) / 256;
