@@ -95,8 +95,10 @@ __device__ __forceinline__ void umma_commit_pair_warp(uint64_t* bar) {
         "h"((uint16_t)3)
         : "memory");
 }
+// Release at cluster scope: the waits of the pair acquire there, and the default scope, the CTA, would order nothing for the other CTA.  In
+// bert_block_kernel these arrives are what stands between the second CTA's operand stores and the products that the first one issues over them.
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
-    asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 // false when the wait ran out (seconds): the caller leaves its loop
 __device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity) {
