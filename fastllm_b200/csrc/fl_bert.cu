@@ -7,6 +7,7 @@
 #include "bert_block.cuh"
 #include "bert_small.cuh"
 #include "bert_model.cuh"
+#include "grow.hpp"
 #include "gemm_tc.cuh"
 #include "synth.cuh"
 
@@ -306,19 +307,14 @@ static bool bert_blocks(const BertModel& m, int T) {
     return n > 0 && 5 * tiles >= 3 * n * ((tiles + n - 1) / n);
 }
 static void bert_reserve(BertModel& m, int b, int t) {
-    const size_t T = (size_t)b * t;
-    const size_t H = m.H, I = m.I;
-    if (!bert_blocks(m, (int)T) && T > m.cap_chain) {       // what the launch chain alone reads
-        m.cap_chain = T;
-        m.x1.alloc(T * H); m.hbuf.alloc(T * I); m.pre.alloc(T * H);
-    }
-    if (T <= m.cap_tokens && (size_t)b <= m.cap_batch) return;
-    m.cap_tokens = std::max(T, m.cap_tokens);
-    m.cap_batch = std::max((size_t)b, m.cap_batch);
-    const size_t Tc = m.cap_tokens;
-    m.x.alloc(Tc * H); m.ctx.alloc(Tc * H); m.qkv.alloc(Tc * 3 * H);
-    m.ids.alloc(Tc); m.mask.alloc(Tc); m.out.alloc(m.cap_batch * H);
-    m.h_ids.alloc(2 * Tc); m.h_out.alloc(m.cap_batch * H);
+    const size_t T = (size_t)b * t, B = b, H = m.H, I = m.I;
+    if (!bert_blocks(m, (int)T))            // what the launch chain alone reads
+        grow(m.cap_chain, T, [&] { m.x1.alloc(T * H); m.hbuf.alloc(T * I); m.pre.alloc(T * H); });
+    grow(m.cap_tokens, T, [&] {
+        m.x.alloc(T * H); m.ctx.alloc(T * H); m.qkv.alloc(T * 3 * H);
+        m.ids.alloc(T); m.mask.alloc(T); m.h_ids.alloc(2 * T);
+    });
+    grow(m.cap_batch, B, [&] { m.out.alloc(B * H); m.h_out.alloc(B * H); });
 }
 
 // Few short sentences: the whole encoder in one launch of clusters (bert_small.cuh).  -> false: the launch chain takes the call.

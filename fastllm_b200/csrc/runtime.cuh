@@ -133,8 +133,9 @@ struct PinnedBuf {
     void alloc(size_t count) {
         if (p) cudaFreeHost(p);
         p = nullptr;
-        n = count;
+        n = 0;
         if (count) FL_CUDA(cudaMallocHost(&p, count * sizeof(T)));
+        n = count;
     }
 };
 
