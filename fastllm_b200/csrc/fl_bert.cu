@@ -306,18 +306,8 @@ static bool bert_blocks(const BertModel& m, int T) {
     const int n = bert_block_clusters(), tiles = (T + 255) / 256;
     return n > 0 && 5 * tiles >= 3 * n * ((tiles + n - 1) / n);
 }
-static void bert_reserve(BertModel& m, int b, int t) {
-    const size_t T = (size_t)b * t, B = b, H = m.H, I = m.I;
-    if (!bert_blocks(m, (int)T))            // what the launch chain alone reads
-        grow(m.cap_chain, T, [&] { m.x1.alloc(T * H); m.hbuf.alloc(T * I); m.pre.alloc(T * H); });
-    grow(m.cap_tokens, T, [&] {
-        m.x.alloc(T * H); m.ctx.alloc(T * H); m.qkv.alloc(T * 3 * H);
-        m.ids.alloc(T); m.mask.alloc(T); m.h_ids.alloc(2 * T);
-    });
-    grow(m.cap_batch, B, [&] { m.out.alloc(B * H); m.h_out.alloc(B * H); });
-}
 
-// Few short sentences: the whole encoder in one launch of clusters (bert_small.cuh).  -> false: the launch chain takes the call.
+// Few short sentences: the whole encoder in one launch of clusters (bert_small.cuh).
 // The line lies where the clusters (about nine of 16 blocks) are all resident and none has more than 64 tokens: there both take the same (sentences
 // x tokens, chain / one launch, us: 16 x 19 315 / 256, 9 x 48 323 / 324, 18 x 31 319 / 323, 9 x 64 328 / 333, 36 x 16 319 / 315), and a second wave
 // would cost a whole pass more.
@@ -351,13 +341,34 @@ static int bert_small_launch(BertModel& m, const BertSmallArgs& a, int clusters,
     g_launches.fetch_add(1, std::memory_order_relaxed);
     return clusters;
 }
-static bool bert_enqueue_small(BertModel& m, int b, int t, bool has_mask) {
-    if (m.small_layers == nullptr || t > kBsTokens) return false;
-    static const int resident = bert_small_launch<kBsTokens / 16>(m, BertSmallArgs{}, 1, true);       // a property of the device
-    if (resident < 1) return false;
-    // as many clusters as fit at a time, each with as few sentences as that leaves: up to 64 tokens per cluster
-    const int spc = (b + resident - 1) / resident, clusters = (b + spc - 1) / spc, rows = spc * t;
-    if (rows > kBsTokens) return false;
+
+// What takes a call; which buffers are reserved and what is launched both follow from it.
+enum class BertPath { small, blocks, chain };
+struct BertRun { BertPath path; int spc, clusters; };       // small: sentences per cluster, clusters
+static BertRun bert_run(BertModel& m, int b, int t) {
+    if (m.small_layers != nullptr && t <= kBsTokens) {
+        static const int resident = bert_small_launch<kBsTokens / 16>(m, BertSmallArgs{}, 1, true);       // a property of the device
+        if (resident >= 1) {
+            // as many clusters as fit at a time, each with as few sentences as that leaves: up to 64 tokens per cluster
+            const int spc = (b + resident - 1) / resident;
+            if (spc * t <= kBsTokens) return {BertPath::small, spc, (b + spc - 1) / spc};
+        }
+    }
+    return {bert_blocks(m, b * t) ? BertPath::blocks : BertPath::chain, 0, 0};
+}
+static void bert_reserve(BertModel& m, const BertRun& run, int b, int t) {
+    const size_t T = (size_t)b * t, B = b, H = m.H, I = m.I;
+    if (run.path != BertPath::blocks)
+        grow(m.cap_chain, T, [&] { m.x1.alloc(T * H); m.hbuf.alloc(T * I); m.pre.alloc(T * H); });
+    grow(m.cap_tokens, T, [&] {
+        m.x.alloc(T * H); m.ctx.alloc(T * H); m.qkv.alloc(T * 3 * H);
+        m.ids.alloc(T); m.mask.alloc(T); m.h_ids.alloc(2 * T);
+    });
+    grow(m.cap_batch, B, [&] { m.out.alloc(B * H); m.h_out.alloc(B * H); });
+}
+
+static void bert_enqueue_small(BertModel& m, const BertRun& run, int b, int t, bool has_mask) {
+    const int spc = run.spc, clusters = run.clusters, rows = spc * t;
     const BertSmallArgs a{static_cast<const BertSmallLayer*>(m.small_layers), m.wemb, m.pemb, m.lnw, m.lnb, m.ids.p, has_mask ? m.mask.p : nullptr,
                           m.L, b, t, m.V, m.maxpos, spc, m.cfg.norm_eps, 1.f / (float)std::sqrt((double)m.d), m.qkv.p, m.ctx.p, m.hbuf.p, m.pre.p, m.out.p};
     switch ((rows + 15) / 16) {
@@ -366,7 +377,6 @@ static bool bert_enqueue_small(BertModel& m, int b, int t, bool has_mask) {
         case 3: bert_small_launch<3>(m, a, clusters, false); break;
         default: bert_small_launch<4>(m, a, clusters, false);
     }
-    return true;
 }
 
 static void launch_bert_block(BertModel& m, const CUtensorMap& tm_ctx, const CUtensorMap& tm_x, const BertLayerW& w, int T, float eps) {
@@ -378,15 +388,18 @@ static void bert_check(const BertModel& m) {
 }
 
 // Enqueue the encoder on m.stream: B1 -> 6 x (B2..B7) -> B8
-static void bert_enqueue(BertModel& m, int b, int t, bool has_mask) {
-    if (bert_enqueue_small(m, b, t, has_mask)) return;
+static void bert_enqueue(BertModel& m, const BertRun& run, int b, int t, bool has_mask) {
+    if (run.path == BertPath::small) {
+        bert_enqueue_small(m, run, b, t, has_mask);
+        return;
+    }
     const int T = b * t, H = m.H, I = m.I;
     cudaStream_t st = m.stream;
     const int rows_per_cta = 8;
     const dim3 row_grid((T + rows_per_cta - 1) / rows_per_cta), row_block(rows_per_cta * 32);
     blaunch(st, embed_ln_kernel, row_grid, row_block, 0, (const uint16_t*)m.wemb, (const uint16_t*)m.pemb, (const float*)m.lnw, (const float*)m.lnb,
             (const uint32_t*)m.ids.p, T, t, H, m.V, m.maxpos, 1e-12f, m.x.p);
-    const bool blocks = bert_blocks(m, T);
+    const bool blocks = run.path == BertPath::blocks;
     const CUtensorMap tm_x = make_tmap_bf16(m.x.p, T, H, H, kGemmBM), tm_x1 = blocks ? tm_x : make_tmap_bf16(m.x1.p, T, H, H, kGemmBM),
                       tm_ctx = make_tmap_bf16(m.ctx.p, T, H, H, kGemmBM);
     const CUtensorMap tm_h = blocks ? tm_x : make_tmap_bf16(m.hbuf.p, T, I, I, kGemmBM);
@@ -427,7 +440,8 @@ void bert_embed(BertModel& m, const uint32_t* ids, const uint32_t* mask, int b, 
     FL_CHECK(t <= m.maxpos, FL_ERR_INVALID, "sentence longer than max_position_embeddings (the position-embedding lookup fails in the reference too)");
     for (int i = 0; i < b * t; ++i) FL_CHECK(ids[i] < (uint32_t)m.V, FL_ERR_INVALID, "token id out of range");
     std::lock_guard<std::mutex> lock(m.mu);      // embed(&self) may be called from several threads: one workspace
-    bert_reserve(m, b, t);
+    const BertRun run = bert_run(m, b, t);
+    bert_reserve(m, run, b, t);
     const size_t T = (size_t)b * t;
     std::memcpy(m.h_ids.p, ids, T * 4);
     FL_CUDA(cudaMemcpyAsync(m.ids.p, m.h_ids.p, T * 4, cudaMemcpyHostToDevice, m.stream));
@@ -440,7 +454,7 @@ void bert_embed(BertModel& m, const uint32_t* ids, const uint32_t* mask, int b, 
         ev.reset(new EventPair);
         FL_CUDA(cudaEventRecord(ev->e0, m.stream));
     }
-    bert_enqueue(m, b, t, mask != nullptr);
+    bert_enqueue(m, run, b, t, mask != nullptr);
     if (device_ms) FL_CUDA(cudaEventRecord(ev->e1, m.stream));
     FL_CUDA(cudaGetLastError());
     FL_CUDA(cudaMemcpyAsync(m.h_out.p, m.out.p, (size_t)b * m.H * 4, cudaMemcpyDeviceToHost, m.stream));
@@ -456,7 +470,8 @@ void bert_repeat(BertModel& m, int b, int t, int iters, float* elapsed_ms) {
     FL_CHECK((size_t)b * t <= m.cap_tokens, FL_ERR_STATE, "call fl_embed with this shape first");
     EventPair ev;
     FL_CUDA(cudaEventRecord(ev.e0, m.stream));
-    for (int i = 0; i < iters; ++i) bert_enqueue(m, b, t, false);
+    const BertRun run = bert_run(m, b, t);
+    for (int i = 0; i < iters; ++i) bert_enqueue(m, run, b, t, false);
     FL_CUDA(cudaEventRecord(ev.e1, m.stream));
     FL_CUDA(cudaStreamSynchronize(m.stream));
     FL_CUDA(cudaGetLastError());

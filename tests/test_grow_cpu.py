@@ -46,3 +46,10 @@ def test_the_encoder_reserves_through_it():
     body = (CSRC / "fl_bert.cu").read_text().split("static void bert_reserve(", 1)[1].split("\n}\n", 1)[0]
     for cap in ("cap_chain", "cap_tokens", "cap_batch"):
         assert f"grow(m.{cap}, " in body and f"m.{cap} =" not in body
+
+
+def test_one_decision_for_buffers_and_launches():
+    """bert_run alone asks which kernels take a call: reserving and launching on answers of their own could differ"""
+    source = (CSRC / "fl_bert.cu").read_text()
+    calls = source.count("bert_blocks(m,")
+    assert calls == 1 and "bert_blocks(m, b * t)" in source.split("static BertRun bert_run(", 1)[1].split("\n}\n", 1)[0]
