@@ -175,7 +175,16 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
         float2* part = reinterpret_cast<float2*>(sH);                             // [slice][128] row sums (the operand is not there yet, or done with)
         auto esync = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * kBbEpiWarps) : "memory"); };
         auto wait = [&](uint64_t* bar, uint32_t parity) { if (ok) ok = __all_sync(0xFFFFFFFFu, pair_wait(bar, parity)); tc_fence_after(); };
-        auto arrive = [&](uint64_t* bar) { __syncwarp(); if (lane == 0) mbar_arrive_cluster(mapa_u32(smem_u32(bar), 0)); };
+        // Arrives on the first CTA's barriers.  Operands in shared memory are released at the scope that the first CTA's products need: its own warps
+        // within the CTA, the second one's warps at cluster scope, which takes 0.25 us that the products wait for.  s_free hands over no
+        // memory -- what was loaded from S is in registers -- and needs no release (256 x 128 tokens, us: everything released at cluster scope by
+        // both CTAs 1405, by the second one alone 1381, this 1348; one release behind a barrier of the eight warps 1355).
+        auto arrive = [&](uint64_t* bar) {
+            __syncwarp();
+            if (lane != 0) return;
+            if (rank == 0) mbar_arrive(bar); else mbar_arrive_cluster(mapa_u32(smem_u32(bar), 0));
+        };
+        auto free_s = [&] { __syncwarp(); if (lane == 0) mbar_arrive_cluster_relaxed(mapa_u32(smem_u32(&s_free), 0)); };
         // 16-byte chunk c of the row inside a tile of 64-column blocks
         auto at = [&](int c) { return (uint32_t)(c >> 3) * 16384u + (uint32_t)lrow * 128u + (uint32_t)(((c & 7) ^ (lrow & 7)) << 4); };
         // this thread's columns of O: + bias + add(32-column step), kept in TMEM; -> mean and 1 / deviation of the row
@@ -255,7 +264,7 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
 #pragma unroll
                 for (int h = 0; h < kSC; h += 32) tmem_ld32(tS + lane_at + (uint32_t)(cs * kSC + h), reinterpret_cast<uint32_t(&)[32]>(v[h]));
                 tc_fence_before();
-                arrive(&s_free);
+                free_s();
 #pragma unroll
                 for (int i = 0; i < kSC; i += 4) {
                     const float4 b = __ldg(reinterpret_cast<const float4*>(g.b1 + j * 128 + cs * kSC + i));

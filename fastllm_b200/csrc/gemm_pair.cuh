@@ -100,6 +100,10 @@ __device__ __forceinline__ void umma_commit_pair_warp(uint64_t* bar) {
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
     asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
+// orders nothing but itself: for what is no memory
+__device__ __forceinline__ void mbar_arrive_cluster_relaxed(uint32_t bar) {
+    asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
 // false when the wait ran out (seconds): the caller leaves its loop
 __device__ __forceinline__ bool pair_wait(uint64_t* bar, uint32_t parity) {
     for (int i = 0; i < (1 << 20); ++i) {
