@@ -284,7 +284,8 @@ FL_EXPORT const char* fl_last_error(void);                       /* thread-local
 FL_EXPORT int fl_version(void);
 FL_EXPORT int fl_device_synchronize(void);
 /* Page-locked host memory.  A logits_host buffer from here is written by the device itself; any other buffer costs a copy by the calling
- * thread (and its page faults, when it is new).  Freeing memory that a call is still writing to is undefined. */
+ * thread (and its page faults, when it is new).  The memory is the process's own: a forked child keeps what it held at the fork.  Freeing
+ * memory that a call is still writing to is undefined. */
 FL_EXPORT int fl_host_alloc(size_t bytes, void** out);
 FL_EXPORT int fl_host_free(void* p);
 
