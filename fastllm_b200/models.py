@@ -104,40 +104,54 @@ class _Block:
 class _ResultPool:
     """Page-locked memory for a cache's results, which the device then writes by itself (64 x 32000 logits behind a 0.5 ms step: 1.1 -> 0.7 ms
     a call; into new pageable memory one thread copies them and takes a page fault for every 4 KB).  A caller who drops or overwrites a
-    result before asking for the one after the next needs two blocks; whoever keeps more gets plain arrays.  Blocks are freed with the pool or, when
-    an array outlives it, with that array.  Lists are only appended to and popped from (arrays may go in any thread, in the middle of
-    a collection)."""
-    BLOCKS, LEAST = 2, 1 << 16          # blocks; bytes below which a copy is as good
-    AHEAD = 64 << 20                    # bytes of the first block that are taken when the cache is made (page-locking takes 1 ms per MB)
+    result before asking for the one after the next needs two blocks; whoever keeps more gets plain arrays, and so does whoever asks for more
+    than MOST.  Page-locking takes 0.4 ms per MB: both blocks are taken with the cache, for one row per sequence, and a block that has become
+    too small is exchanged for one of at least twice its size.  Blocks are freed with the pool or, when an array outlives it, with that array.
+    Lists are only appended to and popped from (arrays may go in any thread, in the middle of a collection)."""
+    BLOCKS, LEAST, MOST = 2, 1 << 16, 64 << 20      # blocks; bytes below which a copy is as good; bytes of a block, at most
 
     def __init__(self, lib):
         self.lib, self.free, self.tickets, self.closed = lib, [], [None] * self.BLOCKS, False
 
     def empty(self, shape) -> np.ndarray:
         room = 4 * shape[0] * shape[1]
-        if room < self.LEAST:
+        if not self.LEAST <= room <= self.MOST:
             return np.empty(shape, dtype=np.float32)
-        try:
-            ptr, have = self.free.pop()
-        except IndexError:
-            ptr, have = None, 0
-        if have < room:
-            if ptr is not None:
-                self.drop(ptr)
-            try:
-                self.tickets.pop()
-            except IndexError:
-                return np.empty(shape, dtype=np.float32)
-            p = C.c_void_p()
-            if self.lib.fl_host_alloc(room, C.byref(p)) != 0:
-                self.tickets.append(None)
-                return np.empty(shape, dtype=np.float32)
-            ptr, have = p.value, room
+        ptr, have = self.take(room)
+        if ptr is None:
+            return np.empty(shape, dtype=np.float32)
         return np.asarray(_Block(self, ptr, have, tuple(shape)))
 
+    def take(self, room):
+        """-> (address, bytes) of a block with at least that room; (None, 0): there is none to be had"""
+        blocks = []
+        try:
+            while True:
+                blocks.append(self.free.pop())
+        except IndexError:
+            pass
+        blocks.sort(key=lambda b: b[1])
+        fits = [i for i, (_, have) in enumerate(blocks) if have >= room]
+        chosen = blocks.pop(fits[0]) if fits else (blocks.pop(0) if blocks else None)       # the smallest that fits, else the smallest
+        self.free.extend(blocks)
+        if fits:
+            return chosen
+        if chosen is not None:
+            self.drop(chosen[0])
+            room = max(room, min(2 * chosen[1], self.MOST))
+        try:
+            self.tickets.pop()
+        except IndexError:
+            return None, 0
+        p = C.c_void_p()
+        if self.lib.fl_host_alloc(room, C.byref(p)) != 0:
+            self.tickets.append(None)
+            return None, 0
+        return p.value, room
+
     def reserve(self, shape):
-        if 4 * shape[0] * shape[1] <= self.AHEAD:
-            self.empty(shape)           # (dropped at once: its block is free)
+        arrays = [self.empty(shape) for _ in range(self.BLOCKS)]
+        del arrays                      # (their blocks are free again)
 
     def drop(self, ptr):
         self.lib.fl_host_free(C.c_void_p(ptr))

@@ -70,3 +70,49 @@ def test_freed_with_the_pool_or_the_last_array():
     del a
     gc.collect()
     assert not lib.live
+
+
+class CountingLib(FakeLib):
+    def __init__(self):
+        super().__init__()
+        self.taken = []
+
+    def fl_host_alloc(self, size, out):
+        self.taken.append(size)
+        return super().fl_host_alloc(size, out)
+
+
+def test_growing_calls_hardly_ever_page_lock():
+    """page-locking a block takes milliseconds: a batch that grows finds its blocks there, and longer and longer results exchange them a few times"""
+    lib = CountingLib()
+    pool = models._ResultPool(lib)
+    pool.reserve((64, 8192))
+    assert lib.taken == [64 * 8192 * 4] * 2
+    for b in range(1, 65):
+        keep = pool.empty((b, 8192))                            # noqa: F841  (held until the next one is there, as by a program's loop)
+    assert len(lib.taken) == 2
+    for rows in range(100, 301):
+        keep = pool.empty((rows, 8192))                         # noqa: F841
+    assert len(lib.taken) <= 2 + 2 * 3 and len(lib.live) == 2
+
+
+def test_a_block_that_fits_is_taken_before_one_is_exchanged():
+    lib = CountingLib()
+    pool = models._ResultPool(lib)
+    large, small = pool.empty((16, 8192)), pool.empty((4, 8192))
+    where = at(large)
+    del large
+    del small                                                   # (in this order: the small one was given back last)
+    assert at(pool.empty((16, 8192))) == where and len(lib.taken) == 2
+
+
+def test_results_beyond_a_limit_are_plain():
+    lib = CountingLib()
+    pool = models._ResultPool(lib)
+    rows = pool.MOST // (4 * 8192)
+    pool.reserve((rows + 1, 8192))
+    assert not lib.taken and at(pool.empty((rows + 1, 8192))) not in lib.live
+    a = pool.empty((rows // 2 + 1, 8192))
+    del a
+    b = pool.empty((rows, 8192))                                # an exchanged block stays inside the limit
+    assert at(b) in lib.live and max(lib.taken) == pool.MOST
