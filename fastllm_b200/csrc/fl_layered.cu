@@ -943,7 +943,7 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
         FL_CUDA(cudaStreamSynchronize(c.stream));
         drop_graphs(c);
         const size_t N = std::max<size_t>(n_want, 2 * y.want_cap);
-        y.hf.alloc(N * m.W); y.logits.alloc(N * m.V);
+        y.hf.alloc(N * m.W); y.logits.alloc(N * m.V); y.h_logits.alloc(N * m.V);
         if (!m.f32) { y.hf_hi.alloc(N * m.W); y.hf_lo.alloc(N * m.W); }
         y.want_cap = N;
     }

@@ -857,6 +857,7 @@ static void cache_create(fl_cache& c, int max_batch, int max_seq) {
     c.amax_idx.alloc((size_t)kPassRows * c.amax_parts);
     c.am_val.alloc((size_t)max_batch * kArgmaxParts); c.am_idx.alloc((size_t)max_batch * kArgmaxParts);
     c.h_ids.alloc((size_t)max_batch * max_seq);
+    c.h_logits.alloc((size_t)max_batch * w.Vfull);
     c.slot_len.assign(max_batch, 0);
     c.slot_tab.alloc(2 * (size_t)max_batch);
     c.h_slot_tab.alloc(2 * (size_t)max_batch);
@@ -1954,10 +1955,9 @@ static void logits_to_host(fl_cache& c, float* host, size_t n) {
         FL_CUDA(cudaStreamSynchronize(c.stream));
         return;
     }
-    PinnedBuf<float>& stage = c.ly ? c.ly->h_logits : c.h_logits;
-    if (stage.n < n) stage.alloc(c.ly ? c.ly->logits.n : (size_t)c.max_batch * c.w->Vfull);
-    LogitsTransfer t(c, dev, stage.p);
-    deliver_logits(t, stage.p, host, n);
+    float* stage = c.ly ? c.ly->h_logits.p : c.h_logits.p;
+    LogitsTransfer t(c, dev, stage);
+    deliver_logits(t, stage, host, n);
 }
 
 // Layered models behind the uniform entry points: b sequences in slots 0..b-1 (or the given slots), t tokens each, logits of every
@@ -2256,7 +2256,6 @@ FL_EXPORT int fl_forward_sample(fl_model* m, fl_cache* c, const uint32_t* ids, i
         run_forward(*c, ids, b, t, rope_offset);
         // only row 0 is sampled (logits.get(0)?.flatten_all()?, models/mod.rs:421): one V*4-byte read-back into the pinned staging row
         const size_t n = c->w->Vfull;
-        if (c->h_logits.n < n) c->h_logits.alloc((size_t)c->max_batch * n);
         FL_CUDA(cudaMemcpyAsync(c->h_logits.p, c->logits.p, n * 4, cudaMemcpyDeviceToHost, c->stream));
         FL_CUDA(cudaStreamSynchronize(c->stream));
         step_check(*c);

@@ -53,3 +53,14 @@ def test_one_decision_for_buffers_and_launches():
     source = (CSRC / "fl_bert.cu").read_text()
     calls = source.count("bert_blocks(m,")
     assert calls == 1 and "bert_blocks(m, b * t)" in source.split("static BertRun bert_run(", 1)[1].split("\n}\n", 1)[0]
+
+
+def test_nothing_is_taken_between_a_step_and_its_logits():
+    """a step that has run has moved the cache on: memory for its delivery that cannot be had then would cost the cache, and page-locking takes
+    milliseconds of the call"""
+    source = (CSRC / "fl_lib.cu").read_text()
+    deliver = source.split("static void logits_to_host(", 1)[1].split("\n}\n", 1)[0]
+    sample = source.split("FL_EXPORT int fl_forward_sample(", 1)[1].split("FL_API_END", 1)[0]
+    assert ".alloc(" not in deliver and ".alloc(" not in sample
+    assert "c.h_logits.alloc(" in source.split("static void cache_create(", 1)[1].split("\n}\n", 1)[0]
+    assert "y.h_logits.alloc(" in (CSRC / "fl_layered.cu").read_text().split("static void ensure_ws(", 1)[1].split("\n}\n", 1)[0]
