@@ -23,9 +23,11 @@ struct Error : std::runtime_error {
 #define FL_CUDA(expr)                                                                                  \
     do {                                                                                               \
         cudaError_t _e = (expr);                                                                       \
-        if (_e != cudaSuccess)                                                                         \
+        if (_e != cudaSuccess) {                                                                       \
+            cudaGetLastError(); /* reported here; a later look at the launches of this thread starts anew */ \
             throw ::fl::Error(-2, std::string(#expr) + ": " + cudaGetErrorString(_e) + " (" + __FILE__ + \
                                       ":" + std::to_string(__LINE__) + ")");                           \
+        }                                                                                              \
     } while (0)
 
 #define FL_CHECK(cond, code, msg)                       \

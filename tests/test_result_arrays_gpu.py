@@ -53,3 +53,15 @@ def test_a_forked_child_keeps_the_result_it_holds():
     assert reused and not (reused[0] == before).all()           # the device has written over the block the child looked at
     assert status == 0
     assert (again == kept[0]).all() and (others == kept[1]).all()
+
+
+def test_a_refused_allocation_fails_one_call():
+    """memory that cannot be had is reported by the call that asked for it, not once more by the next one of the thread"""
+    from fastllm_b200 import _lib, models
+    encoder = models.MiniLMModel(models.BertConfig(), None, 0, random_seed=5)
+    ids = np.full((2, 7), 100, dtype=np.uint32)
+    want = encoder.embed_ids(ids)
+    cf = models.ConfigFile(8192, 8192, 1 << 30, 1, 64, 64, 1e-5, 1e4, 64, None)      # an embedding table of 16 TB
+    with pytest.raises(_lib.FastllmError, match="out of memory"):
+        models.LlamaWithConfig.initialize_model(cf, None, random_seed=0)
+    assert (encoder.embed_ids(ids) == want).all()
