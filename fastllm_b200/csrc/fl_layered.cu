@@ -936,7 +936,6 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
                 y.grp_cnt.alloc((size_t)m.max_experts + 1);
             }
         }
-        if (!m.f32) ensure_pairs(c, R);
         y.rows = R;
     }
     if (n_want > y.want_cap) {
@@ -1483,6 +1482,7 @@ void layered_forward(fl_cache& c, const int* slots, const int* counts, int n, co
     ensure_ws(c, (size_t)T, (size_t)n_want);
     reserve_portions(c, slots, counts, n);
     c.may_fail = false;
+    step_pairs(c, m.f32 ? 0 : (size_t)T);
     const size_t tab_ints = (size_t)4 * T + 3 * (size_t)n + 1 + (size_t)n_want;
     if (tab_ints > y.tab_cap) {
         FL_CUDA(cudaStreamSynchronize(c.stream));

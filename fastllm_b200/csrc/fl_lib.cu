@@ -1085,7 +1085,6 @@ static void ensure_dense_ws(fl_cache& c, int rows) {
         d.vt.alloc(d.vt_pages_cap * w.nkv * w.d * kKvPage, true);        // zero: the last page's tail multiplies P = 0 and must stay finite
         d.tm_vt = make_tmap_bf16(d.vt.p, d.vt_pages_cap * w.nkv * w.d, kKvPage, kKvPage, (uint32_t)w.d);
     }
-    ensure_pairs(c, R);
     d.rows = R;
 }
 
@@ -1151,15 +1150,25 @@ static int pair_clusters() {
     }();
     return n;
 }
-void ensure_pairs(fl_cache& c, size_t rows) {
-    if (rows < (size_t)kPairMinRows || c.pair_ws.n > 0) return;
-    c.pair_tickets.alloc(2 * kPairMaxClusters, true);
-    c.pair_ws.alloc(kPairWsFloats);
+// Whether the GEMMs of a step of `rows` rows may go to pairs follows from the step, not from what the cache has seen before: a GEMM of more rows than
+// the step has (query heads beside one another) takes the same way on every cache.  The workspace is taken by the first step that needs it; where it
+// cannot be had, the cache goes on without pairs.
+void step_pairs(fl_cache& c, size_t rows) {
+    c.pairs = rows >= (size_t)kPairMinRows && !c.pairs_refused;
+    if (!c.pairs || c.pair_ws.n > 0) return;
+    try {
+        c.pair_tickets.alloc(2 * kPairMaxClusters, true);
+        c.pair_ws.alloc(kPairWsFloats);
+    } catch (const Error&) {
+        c.pair_tickets.release();
+        c.pairs = false;
+        c.pairs_refused = true;
+    }
 }
 // -> whether the GEMM went to pairs of SMs
 template <int EPI>
 static bool launch_gemm_pair(fl_cache& c, cudaStream_t st, bool pdl, const CUtensorMap& hi, const CUtensorMap& lo, const CUtensorMap& w, const GemmArgs& g) {
-    if (c.pair_ws.n == 0 || g.M < kPairMinRows) return false;
+    if (!c.pairs || g.M < kPairMinRows) return false;
     const int most = pair_clusters();
     if (most < 1) return false;
     const PairPlan pl = pair_plan(g.M, g.N, g.K, EPI == GEPI_GLU_HL, most);
@@ -1606,6 +1615,7 @@ static void check_call(fl_cache& c, const uint32_t* ids, int b, int t, size_t ro
 static void run_forward(fl_cache& c, const uint32_t* ids, int b, int t, size_t rope_offset) {
     check_call(c, ids, b, t, rope_offset, 0);
     c.may_fail = false;
+    step_pairs(c, c.w->dense_ok ? (size_t)b * t : 0);
     if ((b * t >= 3 || c.w->cfg.arch == FL_ARCH_MIXTRAL) && c.w->dense_ok) ensure_dense_ws(c, b * t);
     std::memcpy(c.h_ids.p, ids, (size_t)b * t * 4);
     FL_CUDA(cudaMemcpyAsync(c.ids.p, c.h_ids.p, (size_t)b * t * 4, cudaMemcpyHostToDevice, c.stream));
@@ -1652,6 +1662,7 @@ static void run_forward_slots(fl_cache& c, const int* slots, const uint32_t* ids
     }
     for (int i = 0; i < n * t; ++i) FL_CHECK(ids[i] < (uint32_t)w.Vfull, FL_ERR_INVALID, "token id out of range");
     c.may_fail = false;
+    step_pairs(c, (size_t)n * t);
     ensure_dense_ws(c, n * t);
     c.dw.route_rows = n * t;
     c.fresh_call = true;
@@ -2131,6 +2142,7 @@ FL_EXPORT int fl_decode_greedy_loop(fl_model* m, fl_cache* c, const uint32_t* fi
     use_device();
     try {
         check_call(*c, first_ids, b, 1, rope_offset, steps - 1);
+        step_pairs(*c, c->w->dense_ok ? (size_t)b : 0);
         if ((b >= 3 || c->w->cfg.arch == FL_ARCH_MIXTRAL) && c->w->dense_ok) ensure_dense_ws(*c, b);
         if (c->trace_cap < (size_t)steps * b) {
             c->trace.alloc((size_t)steps * b);

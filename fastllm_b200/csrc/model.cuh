@@ -163,9 +163,11 @@ struct fl_cache {
     fl::DevBuf<float> tp_buf;        // [rows, H] partial o_proj / down_proj outputs awaiting the all-reduce (tp > 1)
     fl::DevBuf<float> tp_gather;     // [tp, max_batch, V] vocab-parallel logits gathered from all ranks
     fl::DevBuf<float> tp_local;      // [max_batch, V] this rank's logits slice
-    // shared tiles of the many-row GEMMs (gemm_pair.cuh): their parts and tickets, taken for calls of kPairMinRows rows and more
+    // shared tiles of the many-row GEMMs (gemm_pair.cuh): their parts and tickets, taken for calls of kPairMinRows rows and more; whether the step at
+    // hand may use them (step_pairs); that they could not be had
     fl::DevBuf<float> pair_ws;
     fl::DevBuf<int> pair_tickets;
+    bool pairs = false, pairs_refused = false;
     fl::PinnedBuf<int> step_failed;  // one word: a wait inside a kernel ran out (see step_check)
     bool may_fail = false;           // the step launched kernels that report there
     bool poisoned = false;
@@ -173,7 +175,7 @@ struct fl_cache {
 
 namespace fl {
 void step_check(fl_cache& c);            // behind a step that is waited for: throws when one of its kernels reported a failure
-void ensure_pairs(fl_cache& c, size_t rows);
+void step_pairs(fl_cache& c, size_t rows);        // ahead of a step's launches
 // The dense tensor-core GEMM of fl_lib.cu (tcgen05 / TMEM / TMA, hi|lo activation halves), shared with the layered decoder:
 // out[ks][R, N] (f32, row stride N, slice stride R * N) = (xhi + xlo)[R, K] . W[N, K]^T; returns the number of split-K slices
 // (R <= 128: dec_plan's, and W is constant: it is read ahead of the kernels before; R > 128: prefill_ks, one unless the caller asks for more), which

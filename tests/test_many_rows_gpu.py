@@ -323,3 +323,20 @@ def test_pairs_gated_epilogue():
     cut = R.run_cut(model, toks, [650, 640], cache=model.new_device_cache(1, 1536))
     whole = R.run_whole(model, toks, cache=model.new_device_cache(1, 1536))
     assert R.relerr(whole, np.asarray(cut, dtype=np.float64)) < CHUNK_TOL
+
+
+def test_a_step_does_not_depend_on_what_the_cache_has_seen():
+    """heads above 128 channels: the value GEMM of a 1000-token portion has 19000 rows and K = 2560, a shape for pairs, in a step of fewer than 1024
+    rows: the same kernels, hence the same bits, on a new cache and on one that has read a longer portion"""
+    cfg = R.config([R.att(heads=19, kv_heads=1, dim=192, vdim=64, rot_dims=32, softcap=None)], vocab=64, width=64)
+    _, model = R.build(cfg, seed=81, dtype="bf16")
+    toks = R.tokens(cfg, 2540, seed=82)
+    rows = []
+    for used in (False, True):
+        cache = model.new_device_cache(2, 2560)
+        if used:
+            cache.forward_ragged([1], [toks[:1100]], [[1099]])
+        for a, b in ((0, 1000), (1000, 1540), (1540, 2540)):
+            got = cache.forward_ragged([0], [toks[a:b]], [list(range(b - a))])
+        rows.append(got)
+    assert np.array_equal(*rows)
