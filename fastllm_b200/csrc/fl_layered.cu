@@ -1591,10 +1591,10 @@ static void run_mixer(fl_cache& c, LaunchCtx& lc, const StepTab& st, const Layer
         // norm over the whole projection: its sums read every head before any is rewritten in place, which one block orders)
         const size_t psm = (size_t)8 * D * 4;
         const int heads_all = H + (lw.off_k >= 0 ? G : 0), py = (Ti <= 64 && !d.qk_norm_whole) ? std::max(1, std::min(8, std::max((heads_all + 7) / 8, n_gate / 512))) : 1;
-        const bool ahead = D <= kPrepAheadDim && Ti <= kPrepAheadRows;
+        // (the exact mode has one form whatever the rows: two would round differently wherever the compiler fuses their multiply-adds differently)
         auto prep = [&](auto kern) { launch(lc, "attn_prep", 0, kern, dim3(Ti, py), dim3(256), psm, pa); };
-        if (m.f32) { if (ahead) prep(ly_attn_prep_kernel<float, true>); else prep(ly_attn_prep_kernel<float, false>); }
-        else if (ahead) prep(ly_attn_prep_kernel<uint16_t, true>);
+        if (m.f32) prep(ly_attn_prep_kernel<float, false>);
+        else if (D <= kPrepAheadDim && Ti <= kPrepAheadRows) prep(ly_attn_prep_kernel<uint16_t, true>);
         else prep(ly_attn_prep_kernel<uint16_t, false>);
         GqaAttnArgs at{y.proj.p, lw.n_in, lw.off_q, y.kv_pool[kv_index], y.page_table.p, c.pages_per_seq, st.row_seq, st.row_pos, st.seq_slot,
                        y.u.p, lw.tc_o ? uhi : (uint16_t*)nullptr, ulo, H, G, D, Dv, d.window, d.scale, d.softcap, d.sink, 0, y.at_part.p,

@@ -197,6 +197,17 @@ def test_exact_head_rows_stand_alone():
     assert np.array_equal(whole, R.run_cut(model, toks, [1, 8, 9, 7, 14], cache=model.new_device_cache(2, 64)))
 
 
+@pytest.mark.parametrize("dim", [8, 96])
+def test_exact_attention_rows_stand_alone(dim):
+    """the same for the preparation of heads (norm, rotation, cache append), in steps of more than 512 rows and of fewer"""
+    cfg = R.config([R.att(heads=4, kv_heads=2, dim=dim, vdim=16, rot_dims=dim // 2)], vocab=64, width=64)
+    oracle, model = R.build(cfg, seed=79)
+    toks = R.tokens(cfg, 700, seed=80)
+    whole = R.run_whole(model, toks, cache=model.new_device_cache(2, 768))
+    assert R.relerr(whole, oracle.run(toks)) < R.TOL["f32"]
+    assert np.array_equal(whole, R.run_cut(model, toks, [512, 3, 185], cache=model.new_device_cache(2, 768)))
+
+
 # ---- convolutions in front of the recurrences, rows with a sliding window (blocks of 16 rows that fill the chip, four taps) -----------------------------------
 @pytest.mark.parametrize("layer", [R.delta(heads=4, kv_heads=2, dim=32, vdim=24, conv=4), R.delta(heads=2, kv_heads=2, dim=128, vdim=132, conv=4),
                                    R.delta(heads=6, kv_heads=3, dim=64, vdim=8, conv=4), R.mamba(heads=4, vdim=12, state=20, groups=2, conv=4),
