@@ -102,11 +102,11 @@ struct SkArgs {
     int layer_row0;       // row of this layer's page 0 / kv head 0 in the pool-wide tensor maps
 };
 
-// PAIR (query groups of up to 8 heads): the hi halves of the heads are rows 0-7 of the products' 16, the lo halves rows 8-15, of q and of the
+// Query groups have up to 8 heads (kAttnMaxRep): the hi halves of the heads are rows 0-7 of the products' 16, the lo halves rows 8-15, of q and of the
 // probabilities alike, so one MMA multiplies both and a thread holds a head's two sums in one fragment.  With the halves as two tiles, of which
 // the heads above the group were zeros, the warps' MMAs and exponentials were the limit, not HBM: 64 sequences of 512 to 2048 tokens, 8 key/value
 // heads of 128 channels (335 MB per layer): 81 -> 74 us.
-template <int D, bool PAIR>
+template <int D>
 __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid_constant__ CUtensorMap tmk, const __grid_constant__ CUtensorMap tmv,
                                                                     const SkArgs k) {
     const AttnArgs& a = k.a;
@@ -114,16 +114,15 @@ __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid
     constexpr int NW = kSkConsumerWarps;
     extern __shared__ __align__(1024) uint8_t sksm[];
     const int n_rep = a.nh / a.nkv;
-    // q tiles (hi | lo, [16][D] each) and the cross-warp merge scratch ([NW][n_rep][D] f32) share the front region: the scratch is
-    // written when a pair's last page is done, the q tiles are rewritten before the next pair starts
-    const int front = max(2 * 16 * D * 2, NW * n_rep * D * 4);
-    uint16_t* qhi = reinterpret_cast<uint16_t*>(sksm);
-    uint16_t* qlo = qhi + 16 * D;
+    // the q tile ([16][D]: the heads' hi halves, then their lo halves) and the cross-warp merge scratch ([NW][n_rep][D] f32) share the front
+    // region: the scratch is written when a pair's last page is done, the q tile is rewritten before the next pair starts
+    const int front = max(16 * D * 2, NW * n_rep * D * 4);
+    uint16_t* qt = reinterpret_cast<uint16_t*>(sksm);
     float* red_o = reinterpret_cast<float*>(sksm);
     uint16_t* ring = reinterpret_cast<uint16_t*>(sksm + ((front + 1023) & ~1023));
     __shared__ __align__(8) uint64_t full[kSkMaxStages];
     __shared__ __align__(8) uint64_t empty[kSkMaxStages];
-    __shared__ float red_m[NW][16], red_l[NW][16], mrg_w[NW][16], mrg_den[16];
+    __shared__ float red_m[NW][8], red_l[NW][8], mrg_w[NW][8], mrg_den[8];
     __shared__ int prefix[kMaxBatch + 1];        // pages of the sequences before s
     __shared__ int s_len[kMaxBatch], s_slot[kMaxBatch];
     __shared__ int s_last[2], s_i0[2], s_i1[2];
@@ -237,7 +236,7 @@ __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid
     int s, h, p;
     locate(flat0, s, h, p);
     float o[D / 8][4];
-    float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+    float m0 = -INFINITY, l0 = 0.f;
     bool open = false, from_start = false;
     int end_s = -1, end_h = 0, on_s = -1, on_h = 0;        // pairs of which this CTA holds a part: the one that ends here, the one that goes on
     unsigned int c = 0;
@@ -245,24 +244,18 @@ __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid
         const int np = prefix[s + 1] - prefix[s], len = s_len[s];
         if (!open) {       // first page of this CTA's share of pair (s, h): stage q, reset the running softmax
             csync();       // the previous pair's readers of the merge scratch are done
-            for (int i = tid; i < 16 * D; i += kSkConsumers) {
+            for (int i = tid; i < 8 * D; i += kSkConsumers) {
                 const int hh = i / D, dd = i % D;
-                if constexpr (PAIR) {
-                    if (hh >= 8) break;
-                    const float q = hh < n_rep ? a.q[((size_t)s * a.nh + h * n_rep + hh) * D + dd] : 0.f;
-                    const uint16_t hi = f32_to_bf16_rne(q);
-                    qhi[swz<D>(hh, dd)] = hi;
-                    qhi[swz<D>(hh + 8, dd)] = f32_to_bf16_rne(q - __uint_as_float((uint32_t)hi << 16));
-                } else {
-                    const float q = hh < n_rep ? a.q[((size_t)s * a.nh + h * n_rep + hh) * D + dd] : 0.f;
-                    store_hi_lo(qhi, qlo, swz<D>(hh, dd), q);
-                }
+                const float q = hh < n_rep ? a.q[((size_t)s * a.nh + h * n_rep + hh) * D + dd] : 0.f;
+                const uint16_t hi = f32_to_bf16_rne(q);
+                qt[swz<D>(hh, dd)] = hi;
+                qt[swz<D>(hh + 8, dd)] = f32_to_bf16_rne(q - __uint_as_float((uint32_t)hi << 16));
             }
             csync();
 #pragma unroll
             for (int i = 0; i < D / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
-            m0 = m1 = -INFINITY;
-            l0 = l1 = 0.f;
+            m0 = -INFINITY;
+            l0 = 0.f;
             open = true;
             from_start = (p == 0);
         }
@@ -275,78 +268,45 @@ __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid
             float sc[2][4] = {{0.f, 0.f, 0.f, 0.f}, {0.f, 0.f, 0.f, 0.f}};
 #pragma unroll
             for (int ks = 0; ks < D / 16; ++ks) {
-                uint32_t ah[4], al[4], kb[4];
-                ldmatrix_x4(ah, qhi + swz<D>(lane & 15, ks * 16 + (lane >> 4) * 8));
-                if (!PAIR) ldmatrix_x4(al, qlo + swz<D>(lane & 15, ks * 16 + (lane >> 4) * 8));
+                uint32_t qf[4], kb[4];
+                ldmatrix_x4(qf, qt + swz<D>(lane & 15, ks * 16 + (lane >> 4) * 8));
                 ldmatrix_x4(kb, kt + kv_off<D>(warp * 16 + (lane & 7) + ((lane >> 4) << 3), ks * 16 + ((lane >> 3) & 1) * 8));
-                mma_bf16_16816(sc[0], ah, kb[0], kb[1]);
-                if (!PAIR) mma_bf16_16816(sc[0], al, kb[0], kb[1]);
-                mma_bf16_16816(sc[1], ah, kb[2], kb[3]);
-                if (!PAIR) mma_bf16_16816(sc[1], al, kb[2], kb[3]);
+                mma_bf16_16816(sc[0], qf, kb[0], kb[1]);
+                mma_bf16_16816(sc[1], qf, kb[2], kb[3]);
             }
-            constexpr int EV = PAIR ? 2 : 4;       // scores of a fragment
-            if constexpr (PAIR) {
-#pragma unroll
-                for (int nt = 0; nt < 2; ++nt) { sc[nt][0] += sc[nt][2]; sc[nt][1] += sc[nt][3]; }
-            }
-            float mx0 = -INFINITY, mx1 = -INFINITY;
+            float mx = -INFINITY;
 #pragma unroll
             for (int nt = 0; nt < 2; ++nt)
 #pragma unroll
-                for (int e = 0; e < EV; ++e) {
-                    const int key = key0 + nt * 8 + tq * 2 + (e & 1);
-                    sc[nt][e] = key < len ? sc[nt][e] * a.qscale : -INFINITY;
-                    if (e < 2) mx0 = fmaxf(mx0, sc[nt][e]); else mx1 = fmaxf(mx1, sc[nt][e]);
+                for (int e = 0; e < 2; ++e) {
+                    const int key = key0 + nt * 8 + tq * 2 + e;
+                    sc[nt][e] = key < len ? (sc[nt][e] + sc[nt][e + 2]) * a.qscale : -INFINITY;
+                    mx = fmaxf(mx, sc[nt][e]);
                 }
-            mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, 1)); mx0 = fmaxf(mx0, __shfl_xor_sync(0xFFFFFFFFu, mx0, 2));
-            const float mn0 = fmaxf(m0, mx0);       // finite: key0 < len is valid for every row
-            const float al0 = expf(m0 - mn0);
-            m0 = mn0;
-            float al1 = al0, ps0 = 0.f;
-            uint32_t ph[4], pl[4];
-            if constexpr (PAIR) {
+            mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 1)); mx = fmaxf(mx, __shfl_xor_sync(0xFFFFFFFFu, mx, 2));
+            const float mn = fmaxf(m0, mx);       // finite: key0 < len is valid for every row
+            const float al = expf(m0 - mn);
+            m0 = mn;
+            float ps = 0.f;
+            uint32_t ph[4];
 #pragma unroll
-                for (int nt = 0; nt < 2; ++nt) {
-                    sc[nt][0] = expf(sc[nt][0] - mn0); sc[nt][1] = expf(sc[nt][1] - mn0);
-                    ps0 += sc[nt][0] + sc[nt][1];
-                    ph[2 * nt] = pack_bf16x2(sc[nt][0], sc[nt][1]);
-                    ph[2 * nt + 1] = pack_bf16x2(sc[nt][0] - bf16lo(ph[2 * nt]), sc[nt][1] - bf16hi(ph[2 * nt]));
-                }
-                l0 = l0 * al0 + ps0;       // per-thread partial row sums; the quad is reduced when the pair is emitted
-            } else {
-                mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 1)); mx1 = fmaxf(mx1, __shfl_xor_sync(0xFFFFFFFFu, mx1, 2));
-                const float mn1 = fmaxf(m1, mx1);
-                al1 = expf(m1 - mn1);
-                m1 = mn1;
-                float ps1 = 0.f;
-#pragma unroll
-                for (int nt = 0; nt < 2; ++nt) {
-                    sc[nt][0] = expf(sc[nt][0] - mn0); sc[nt][1] = expf(sc[nt][1] - mn0);
-                    sc[nt][2] = expf(sc[nt][2] - mn1); sc[nt][3] = expf(sc[nt][3] - mn1);
-                    ps0 += sc[nt][0] + sc[nt][1];
-                    ps1 += sc[nt][2] + sc[nt][3];
-                }
-                l0 = l0 * al0 + ps0;
-                l1 = l1 * al1 + ps1;
-                ph[0] = pack_bf16x2(sc[0][0], sc[0][1]); ph[1] = pack_bf16x2(sc[0][2], sc[0][3]);
-                ph[2] = pack_bf16x2(sc[1][0], sc[1][1]); ph[3] = pack_bf16x2(sc[1][2], sc[1][3]);
-                pl[0] = pack_bf16x2(sc[0][0] - bf16lo(ph[0]), sc[0][1] - bf16hi(ph[0]));
-                pl[1] = pack_bf16x2(sc[0][2] - bf16lo(ph[1]), sc[0][3] - bf16hi(ph[1]));
-                pl[2] = pack_bf16x2(sc[1][0] - bf16lo(ph[2]), sc[1][1] - bf16hi(ph[2]));
-                pl[3] = pack_bf16x2(sc[1][2] - bf16lo(ph[3]), sc[1][3] - bf16hi(ph[3]));
+            for (int nt = 0; nt < 2; ++nt) {
+                sc[nt][0] = expf(sc[nt][0] - mn); sc[nt][1] = expf(sc[nt][1] - mn);
+                ps += sc[nt][0] + sc[nt][1];
+                ph[2 * nt] = pack_bf16x2(sc[nt][0], sc[nt][1]);
+                ph[2 * nt + 1] = pack_bf16x2(sc[nt][0] - bf16lo(ph[2 * nt]), sc[nt][1] - bf16hi(ph[2 * nt]));
             }
+            l0 = l0 * al + ps;       // per-thread partial row sums; the quad is reduced when the pair is emitted
 #pragma unroll
             for (int dt = 0; dt < D / 16; ++dt) {
                 uint32_t vb[4];
                 ldmatrix_x4_trans(vb, vt + kv_off<D>(warp * 16 + (lane & 15), dt * 16 + (lane >> 4) * 8));
                 float(&oa)[4] = o[2 * dt];
                 float(&ob)[4] = o[2 * dt + 1];
-                oa[0] *= al0; oa[1] *= al0; oa[2] *= al1; oa[3] *= al1;
-                ob[0] *= al0; ob[1] *= al0; ob[2] *= al1; ob[3] *= al1;
+#pragma unroll
+                for (int e = 0; e < 4; ++e) { oa[e] *= al; ob[e] *= al; }
                 mma_bf16_16816(oa, ph, vb[0], vb[1]);
-                if (!PAIR) mma_bf16_16816(oa, pl, vb[0], vb[1]);
                 mma_bf16_16816(ob, ph, vb[2], vb[3]);
-                if (!PAIR) mma_bf16_16816(ob, pl, vb[2], vb[3]);
             }
         }
         __syncwarp();
@@ -357,23 +317,19 @@ __global__ void __launch_bounds__(kSkThreads) attn_sk_decode_kernel(const __grid
             // ---- emit: merge the 4 warps (each saw a different quarter of every page) ----
             const bool whole = from_start && pair_done;       // nobody else holds a piece of this pair
             l0 += __shfl_xor_sync(0xFFFFFFFFu, l0, 1); l0 += __shfl_xor_sync(0xFFFFFFFFu, l0, 2);
-            if (!PAIR) { l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, 1); l1 += __shfl_xor_sync(0xFFFFFFFFu, l1, 2); }
-            csync();       // every warp is past its last read of the q tiles (the scratch overlays them)
+            csync();       // every warp is past its last read of the q tile (the scratch overlays it)
             if (tq == 0) {
                 red_m[warp][g] = m0;
                 red_l[warp][g] = l0;
-                if (!PAIR) { red_m[warp][g + 8] = m1; red_l[warp][g + 8] = l1; }
             }
 #pragma unroll
             for (int nt = 0; nt < D / 8; ++nt) {
                 if (g < n_rep)
-                    *reinterpret_cast<float2*>(red_o + ((size_t)warp * n_rep + g) * D + nt * 8 + tq * 2) =
-                        PAIR ? make_float2(o[nt][0] + o[nt][2], o[nt][1] + o[nt][3]) : make_float2(o[nt][0], o[nt][1]);
-                if (!PAIR && g + 8 < n_rep) *reinterpret_cast<float2*>(red_o + ((size_t)warp * n_rep + g + 8) * D + nt * 8 + tq * 2) = make_float2(o[nt][2], o[nt][3]);
+                    *reinterpret_cast<float2*>(red_o + ((size_t)warp * n_rep + g) * D + nt * 8 + tq * 2) = make_float2(o[nt][0] + o[nt][2], o[nt][1] + o[nt][3]);
             }
             csync();
             const int part = cta * 2 + (from_start ? 1 : 0);      // this CTA's partial slot for the pair
-            if (tid < (PAIR ? 8 : 16)) {
+            if (tid < 8) {
                 float ms = -INFINITY;
 #pragma unroll
                 for (int w = 0; w < NW; ++w) ms = fmaxf(ms, red_m[w][tid]);

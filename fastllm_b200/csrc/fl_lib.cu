@@ -130,9 +130,9 @@ static size_t attn_prefill_smem_bytes(int d) {
     return (size_t)(2 * kPrefillBM + 4 * kKvPage) * d * 2;
 }
 
-// stream-K batched decode (attn_sk_decode_kernel): q tiles / merge scratch in front, then the K|V ring
+// stream-K batched decode (attn_sk_decode_kernel): q tile / merge scratch in front, then the K|V ring
 static size_t attn_sk_smem_bytes(int d, int n_rep, int stages) {
-    const size_t front = std::max<size_t>((size_t)2 * 16 * d * 2, (size_t)kSkConsumerWarps * n_rep * d * 4);
+    const size_t front = std::max<size_t>((size_t)16 * d * 2, (size_t)kSkConsumerWarps * n_rep * d * 4);
     return ((front + 1023) & ~(size_t)1023) + (size_t)stages * 2 * kKvPage * d * 2;
 }
 struct SkPlan { int stages = 0, ctas = 0; size_t smem = 0; };
@@ -150,9 +150,7 @@ static SkPlan attn_sk_plan_d(int n_rep) {
     if (it != memo.end()) return it->second;
     auto fit = [&](int st) {
         int n = 0;
-        const size_t smem = attn_sk_smem_bytes(D, n_rep, st);
-        if (n_rep <= 8) FL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_sk_decode_kernel<D, true>, kSkThreads, smem));
-        else FL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_sk_decode_kernel<D, false>, kSkThreads, smem));
+        FL_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, attn_sk_decode_kernel<D>, kSkThreads, attn_sk_smem_bytes(D, n_rep, st)));
         return n;
     };
     SkPlan p;
@@ -175,22 +173,17 @@ static SkPlan attn_sk_plan(int d, int n_rep) {
 }
 static void launch_attn_sk(LaunchCtx& lc, int d, const SkPlan& pl, uint64_t bytes, const CUtensorMap& tmk, const CUtensorMap& tmv, const SkArgs& k) {
     const dim3 g(pl.ctas * kNumSMs), b(kSkThreads);
-    auto go = [&](auto pair) {
-        constexpr bool P = decltype(pair)::value;
-        switch (d) {
-            case 16: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<16, P>, g, b, pl.smem, tmk, tmv, k); break;
-            case 32: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<32, P>, g, b, pl.smem, tmk, tmv, k); break;
-            case 64: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<64, P>, g, b, pl.smem, tmk, tmv, k); break;
-            default: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<128, P>, g, b, pl.smem, tmk, tmv, k); break;
-        }
-    };
-    if (k.a.nh / k.a.nkv <= 8) go(std::true_type{}); else go(std::false_type{});
+    switch (d) {
+        case 16: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<16>, g, b, pl.smem, tmk, tmv, k); break;
+        case 32: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<32>, g, b, pl.smem, tmk, tmv, k); break;
+        case 64: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<64>, g, b, pl.smem, tmk, tmv, k); break;
+        default: launch(lc, "attn_sk_decode", bytes, attn_sk_decode_kernel<128>, g, b, pl.smem, tmk, tmv, k); break;
+    }
 }
 
 template <int D>
 static void attn_mma_set_attrs() {
-    FL_CUDA(cudaFuncSetAttribute(attn_sk_decode_kernel<D, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    FL_CUDA(cudaFuncSetAttribute(attn_sk_decode_kernel<D, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    FL_CUDA(cudaFuncSetAttribute(attn_sk_decode_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
     if constexpr (D == 64 || D == 128)
         FL_CUDA(cudaFuncSetAttribute(attn_prefill_tc_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_prefill_tc_smem_bytes(D)));
     FL_CUDA(cudaFuncSetAttribute(attn_prefill_kernel<D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)attn_prefill_smem_bytes(D)));
@@ -1439,7 +1432,7 @@ static void enqueue_forward_dense(fl_cache& c, LaunchCtx& lc, int b, int t, bool
                 // stream-K: a fixed grid of resident CTAs, each an equal share of the step's page stream.  The grid does NOT depend
                 // on the KV length: this launch is captured into the step's CUDA graph, which is keyed by (batch, mode) only and
                 // replayed as the context grows.
-                FL_CHECK(c.kv_tmaps && w.nh / w.nkv <= 16, FL_ERR_UNSUPPORTED, "batched decode attention: GQA group > 16 heads or KV pool beyond 2^31 rows");
+                FL_CHECK(c.kv_tmaps && w.nh / w.nkv <= kAttnMaxRep, FL_ERR_UNSUPPORTED, "batched decode attention: GQA group > 8 heads or KV pool beyond 2^31 rows");
                 const SkPlan pl = attn_sk_plan(w.d, w.nh / w.nkv);
                 SkArgs sk{};
                 sk.a = at; sk.sk_acc = d.sk_acc.p; sk.sk_ml = d.sk_ml.p; sk.b = b; sk.nstages = pl.stages;

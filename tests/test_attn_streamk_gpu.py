@@ -65,3 +65,27 @@ def test_stream_k_decode_attention_over_more_pages_than_ctas(name, monkeypatch):
     print(f"{name}: {nseq} ragged sequences, {pages} K|V pages per layer: prefill err {prefill_err:.2e}, decode err {max(step_errs):.2e}")
     # long dense-path decode tolerance (tests/test_zz_widening_gpu.py): bf16 rounding flips of cached K / V under the hi + lo split
     assert prefill_err <= 1e-2 and max(step_errs) <= 1e-2
+
+
+@pytest.mark.parametrize("heads,dim", [(8, 64), (1, 128), (7, 32)])
+def test_pairs_over_many_ctas(heads, dim):
+    """few long sequences, fewer pages than CTAs: a (sequence, kv head) pair is spread a page per CTA, over up to 16 of them (the last CTA to arrive
+    takes the parts eight at a time: here 8, 9, 15 and 16), for query groups of one head, of an odd number and of the largest"""
+    from fastllm_b200 import models
+    cfg = ocl.CausalLMConfig("llama", heads * dim, 160, 256, 2, heads, 1, 1e-5, 1e4, 1024)
+    w = ocl.synth_weights(cfg, 31, 0.06)
+    model, _ = product_model(cfg, w)
+    lengths = [960 + 40, 511, 512, 940]                 # 16, 8, 9 and 15 pages with the step's own token
+    cache = models.DeviceCache(model.dev, len(lengths), 1024)
+    oracles, ids = [], []
+    for i, n in enumerate(lengths):
+        prompt = synth.token_ids(700 + i, cfg.vocab_size, (1, n))
+        oracles.append(ocl.CausalLM(cfg, w, kv_dtype="bf16"))
+        ids.append([models.sample_argmax(oracles[i].forward(prompt, 0)[0])])
+        cache.forward_slots([i], prompt, [0])
+    for step in range(2):
+        got = cache.forward_slots(list(range(len(lengths))), np.array(ids, dtype=np.uint32), [n + step for n in lengths])
+        for i, n in enumerate(lengths):
+            want = oracles[i].forward(np.array([ids[i]], dtype=np.uint32), n + step)[0]
+            assert np.abs(got[i] - want).max() <= 1e-2, (step, i)
+            ids[i] = [models.sample_argmax(want)]
