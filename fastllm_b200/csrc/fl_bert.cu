@@ -298,13 +298,14 @@ static int bert_block_clusters() {       // pairs of SMs that can be resident at
     }();
     return n;
 }
-// A pair of SMs takes about as long for 256 tokens however many tiles there are, the chain's kernels grow with the tokens: whole encoder, chain ->
-// blocks, us, by tiles of 256 tokens: 46 781 -> 591, 64 930 -> 699, 74 999 -> 738, 128 (two waves) 1719 -> 1283. The line was drawn with blocks that
-// took 12 % longer than today's: 32 tiles 576 -> 605, 80 (two waves) 1159 -> 1199.
+// A pair of SMs takes about as long for 256 tokens however many tiles there are, the chain's kernels grow with the tokens, in steps of their own waves.
+// Whole encoder, chain -> blocks, us, by tiles of 256 tokens (128-token sentences; 64 and 512 tokens a sentence cross at the same places): 28 506 -> 506,
+// 32 526 -> 522, 36 544 -> 532, 38 658 -> 550, 44 688 -> 576, 64 853 -> 674, 74 914 -> 702; two waves: 75 1034 -> 1036, 80 1070 -> 1058,
+// 88 1146 -> 1097, 128 1607 -> 1283.  Up to half a wave the two are within 2 % of each other; behind it, and in every later wave, the blocks are ahead.
 static bool bert_blocks(const BertModel& m, int T) {
     if (m.H != kBbH || m.I != kBbI) return false;
     const int n = bert_block_clusters(), tiles = (T + 255) / 256;
-    return n > 0 && 5 * tiles >= 3 * n * ((tiles + n - 1) / n);
+    return n > 0 && 2 * tiles >= n;
 }
 
 // Few short sentences: the whole encoder in one launch of clusters (bert_small.cuh).
