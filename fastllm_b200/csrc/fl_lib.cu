@@ -1241,13 +1241,13 @@ int dense_gemm(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int N, int K,
         if (silu_hi != nullptr) {       // prefill gate|up: SiLU(gate) * up + hi/lo split fused into the epilogue
             GemmArgs g{R, N, K, nullptr, nullptr, 0, silu_hi, N / 2, 1, 0, silu_lo};
             g.raster_m = kGemmRasterRows;
-            if (prefill_bn == 256 && launch_gemm_pair<GEPI_SILU_HL>(c, lc.stream, pdl, hi, lo, tmW, g)) {}
+            if (prefill_bn == 256 && launch_gemm_pair<GEPI_SILU_HL>(c, lc.stream, pdl, hi, lo, tmW, g)) pe.tag += "_pairs";
             else if (prefill_bn == 256) launch_gemm_tc<256, GEPI_SILU_HL, DUAL_A>(lc.stream, pdl, tiles, hi, lo, tmW, g);
             else launch_gemm_tc<128, GEPI_SILU_HL, DUAL_A>(lc.stream, pdl, tiles, hi, lo, tmW, g);
         } else {
             GemmArgs g{R, N, K, nullptr, nullptr, 0, out, N, ks, (long long)R * N};
             g.raster_m = kGemmRasterRows;
-            if (prefill_bn == 256 && ks == 1 && launch_gemm_pair<GEPI_F32>(c, lc.stream, pdl, hi, lo, tmW, g)) {}
+            if (prefill_bn == 256 && ks == 1 && launch_gemm_pair<GEPI_F32>(c, lc.stream, pdl, hi, lo, tmW, g)) pe.tag += "_pairs";
             else if (prefill_bn == 256) launch_gemm_tc<256, GEPI_F32, DUAL_A>(lc.stream, pdl, tiles * ks, hi, lo, tmW, g);
             else launch_gemm_tc<128, GEPI_F32, DUAL_A>(lc.stream, pdl, tiles * ks, hi, lo, tmW, g);
         }
@@ -1275,7 +1275,7 @@ static void launch_rows_gemm(fl_cache& c, LaunchCtx& lc, const char* tag, const 
         FL_CUDA(cudaEventRecord(pe.e0, lc.stream));
     }
     const CUtensorMap hi = make_tmap_bf16(xhi, g.M, g.K, g.K, kGemmBM), lo = make_tmap_bf16(xlo, g.M, g.K, g.K, kGemmBM);
-    if (glu && g.groups == 0 && launch_gemm_pair<GEPI_GLU_HL>(c, lc.stream, pdl, hi, lo, tmW, g)) {}
+    if (glu && g.groups == 0 && launch_gemm_pair<GEPI_GLU_HL>(c, lc.stream, pdl, hi, lo, tmW, g)) pe.tag += "_pairs";
     else if (glu) launch_gemm_tc<256, GEPI_GLU_HL, DUAL_A>(lc.stream, pdl, tiles, hi, lo, tmW, g);
     else launch_gemm_tc<256, GEPI_F32, DUAL_A>(lc.stream, pdl, tiles, hi, lo, tmW, g);
     if (prof) {

@@ -310,7 +310,7 @@ def test_steps_that_grow(mod, cfg):
 
 # ---- GEMMs on pairs of SMs (gemm_pair.cuh): from 1024 rows on, where whole waves of pair tiles leave a few that are cut along K ------------------
 def test_pairs_llama():
-    """1290 rows: the last pair row ends inside its second half; o and gate|up leave 16 tiles to cut, which end inside a k block's run"""
+    """1290 rows: the last pair row ends inside its first half; o and gate|up leave 16 tiles to cut, which end inside a k block's run"""
     from fastllm_b200 import models
     from helpers import product_model
     from oracle import causal_lm as ocl
@@ -351,3 +351,41 @@ def test_a_step_does_not_depend_on_what_the_cache_has_seen():
             got = cache.forward_ragged([0], [toks[a:b]], [list(range(b - a))])
         rows.append(got)
     assert np.array_equal(*rows)
+
+
+def tags_of(run):
+    """kernels that `run` launched, by the profiler's tags"""
+    from fastllm_b200 import models
+    models.prof_begin()
+    out = run()
+    return out, {p["kernel"] for p in models.prof_end()}
+
+
+# rows and the tiles of 256 x 256 over 74 pairs: the last pair row ends inside its second half, 1 whole tile each and 16 cut ones (o, gate|up); 2 and 6
+# (gate|up); 4 and none (gate|up).  Short sentences: a row of every tenth or eighth token is looked at
+@pytest.mark.parametrize("batch,tokens,hidden,inter,heads,kv,paired", [(144, 10, 3840, 1920, 30, 5, {"o", "gateup"}), (170, 10, 2560, 2816, 20, 4, {"gateup"}),
+                                                                       (250, 8, 512, 4736, 4, 2, {"gateup"})])
+def test_pairs_all_over_the_rows(batch, tokens, hidden, inter, heads, kv, paired):
+    from fastllm_b200 import models
+    from helpers import product_model
+    from oracle import causal_lm as ocl
+    from oracle import synth
+    cfg = ocl.CausalLMConfig("llama", hidden, inter, 500, 1, heads, kv, 1e-5, 1e4, 32)
+    w = ocl.synth_weights(cfg, 0, 0.5 * hidden ** -0.5)
+    model = product_model(cfg, w)[0]
+    ids = synth.token_ids(11, 500, (batch, tokens))
+    got, tags = tags_of(lambda: models.DeviceCache(model.dev, batch, 32).forward(ids, 0))
+    assert {t for t in tags if t.endswith("_pairs")} == {f"gemm_tc_{p}_pairs" for p in paired}
+    want = ocl.CausalLM(cfg, w, kv_dtype="bf16").forward(ids, 0)
+    assert np.abs(got - want).max() <= 3e-3
+
+
+def test_pairs_gated_rows():
+    """the gated epilogue, 1440 rows (the last pair row ends inside its second half), every row against the same tokens in portions on single tiles"""
+    cfg = R.config([R.mamba(heads=4, vdim=32, state=32, groups=2, mlp=R.dense(ff=1920))], vocab=64, width=3072)
+    _, model = R.build(cfg, seed=71, dtype="bf16")
+    toks = R.tokens(cfg, 1440, seed=73)
+    cut = R.run_cut(model, toks, [720, 720], cache=model.new_device_cache(1, 1536))
+    whole, tags = tags_of(lambda: R.run_whole(model, toks, cache=model.new_device_cache(1, 1536)))
+    assert "gemm_ff_in_pairs" in tags
+    assert R.relerr(whole, np.asarray(cut, dtype=np.float64)) < CHUNK_TOL
