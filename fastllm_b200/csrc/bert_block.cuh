@@ -6,9 +6,11 @@
 // and half of every weight tile.  The 1536-wide activations exist 128 columns at a time: S (128 TMEM columns) -> GELU -> shared memory -> O (384
 // columns).  The tensor core alternates between the next columns' S and the last columns' O while the epilogue warps turn S into operands.
 // As five launches every layer moved 100 to 200 MB of activations between kernels that each waited for HBM and for their epilogues' stores
-// (256 x 128 tokens, whole encoder: 1.76 ms; 1.28 in this form).  What bounds it: per 128 intermediate columns the products take 1.6 us (3090 clocks,
-// measured by themselves) and the GELUs 1.0 (the tanh unit), one epilogue warp of them waiting for the other now and then; 5 us in front and 6 behind for
-// the two norms.  8 epilogue warps: 16 were no faster.
+// (256 x 128 tokens, whole encoder: 1.76 ms; 1.35 in this form).  256 tokens take 56 us (74 -> 75 tiles, a second wave in each of six layers: 702 ->
+// 1036 us), of which the products are 22 (1.6 us per 128 intermediate columns, measured by themselves, 2.4 for the output projection) and the two norms 5
+// in front and 6 behind.  The rest, 3.4 us per 128 columns instead of 1.6, is the chain from S to the next operand that the products wait for: load,
+// GELU (1.0 us, the tanh unit), store, fence, release (0.25).  Tensor pipe 33 %, issue slots 21 %, DRAM 5 % at one wave.  8 epilogue warps: 16 were no
+// faster.
 #pragma once
 #include "gemm_pair.cuh"
 

@@ -255,7 +255,7 @@ static __global__ void dense_qkv_epi_kernel(const QkvEpiArgs a) {
     // the dependent (attention) kernel is released only AFTER this kernel's own wait: when it starts, the q|k|v GEMM -- and by
     // induction every earlier kernel of the stream -- has completed, so its preamble may read the step state, the page table and
     // every K/V page except the rows appended here before its own griddepcontrol.wait (attn_sk_decode_kernel streams them early).
-    // (Released at entry its blocks took the SMs as the GEMM's blocks left them, three on some and one on others: 24.1 -> 25.2 us.)
+    // (Released at entry: a step of 8 sequences of 2048 tokens 522 us instead of 526, of 64 the same.)
     pdl_wait();
     pdl_launch_dependents();
     const int row = blockIdx.y;

@@ -43,8 +43,12 @@ inline PairPlan pair_plan(int M, int N, int K, bool glu, int max_clusters) {
     return p;
 }
 // Whether pairs are the faster way, counted in k blocks of a tile: a single CTA's tiles fill whole waves of 148, pairs pay about 20 k blocks for
-// the parts of shared tiles (their way through the workspace).  A last wave that is more than a quarter full runs at a higher clock than the whole chip
-// does under the power limit: there is nothing to win then (2048 x 4096 x 14336, 1.73 waves: 311 us single, 314 in pairs).
+// the parts of shared tiles (their way through the workspace) and 12 for the rest.  Single -> pairs, us, by the pairs (of 74) that a last wave would
+// fill: 10 (1536 x 3584 x 18944) 400 -> 275, 12 (2560 x 4096 x 14336) 482 -> 379, 22 (1536 x 4096 x 14336) 295 -> 228, 38 (2048 x 3584 x 18944)
+// 410 -> 375, 48 (3584 x 3584 x 18944) 636 -> 602, 54 (2048 x 4096 x 14336) 314 -> 316, 66 (2560 x 3584 x 18944) 440 -> 454: a last wave that is nearly full
+// runs at a higher clock than the whole chip does under the power limit.  The line lies at a quarter of a wave and not at the two thirds up to which
+// single shapes gain, because cut tiles are sums in another order, and a whole prompt of 2048 rows and width 4096 with the line there took 6.43 ms instead of
+// 6.44 at a distance from 64 bits of 5.5e-4 instead of 5.4e-4.  K = 2048 is too short for any of it: 3072 x 11264 x 2048, 10: 193 -> 215.
 constexpr int kPairMinRows = 1024;
 inline bool pair_wins(const PairPlan& p, int M, int max_clusters) {
     const int T = p.mp * p.nt, left = T - p.full * max_clusters, single = ((M + 127) / 128 * p.nt + kNumSMs - 1) / kNumSMs * p.nk;
