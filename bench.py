@@ -1,5 +1,5 @@
 #!/usr/bin/env python
-"""Benchmark of the hot path (BASELINE.json): decode tok/s and % of the HBM roofline.
+"""Benchmark of the hot path: decode tok/s and % of the HBM roofline.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--workload NAME] [--impl ours|reference]
 
@@ -73,8 +73,8 @@ WORKLOADS = {
                            "silu experts) beside Latodra (latent attention, dense feed-forward) and Medulorn (grouped-query attention, experts with a "
                            "shared one) at equal width / layers: 2048-token prefill and batch-8 decode at 2k context, random weights"),
 }
-QWEN_PREFILL_TFLOP_4K = 56.83         # SURVEY.md section 8d: 53.46 linear + 3.37 causal attention
-MINILM_FLOP_PER_TOKEN = 22.41e6      # SURVEY.md section 8d: 2 x 10.617 M linear + 4 T H 6 attention at T = 128
+QWEN_PREFILL_TFLOP_4K = 56.83         # 53.46 linear + 3.37 causal attention
+MINILM_FLOP_PER_TOKEN = 22.41e6      # 2 x 10.617 M linear + 4 T H 6 attention at T = 128
 
 
 def oracle_config(key):
@@ -488,7 +488,7 @@ def compare_sharded(got, want, what, routing=None):
 
 
 def tinyllama_parity(local_rank):
-    """BASELINE.json config 1 against the committed f32-oracle golden (tests/golden/fulldepth_tinyllama.*, written by
+    """TinyLlama-1.1B at full depth against the committed f32-oracle golden (tests/golden/fulldepth_tinyllama.*, written by
     tests/golden/make_fulldepth_golden.py): TinyLlama-1.1B, all 22 layers, 128-token prompt + 64 greedy steps through the
     reference's generate loop.  No oracle code runs here: ids and three full logits rows are compared with the stored ones."""
     from fastllm_b200 import models, presets
@@ -518,7 +518,6 @@ def run_ours(args, rank, world, local_rank):
     # Mistral / Qwen2 shard with tensor parallelism (strong scaling; batch-1 decode all-reduces over NVLink peer memory inside the
     # persistent kernel, the dense path through NCCL); Mixtral shards its experts (expert parallelism, sequences data-parallel,
     # dispatch / combine all-to-all); TinyLlama runs as independent batch-data-parallel replicas (no collective, weak scaling)
-    # -- BASELINE.json configs / SURVEY.md section 8e.
     use_tp = world > 1 and arch in ("mistral7b", "qwen25_7b")
     use_ep = world > 1 and arch == "mixtral8x7b"
     dist = _setup_dist(world, local_rank)
@@ -793,7 +792,7 @@ def moe_leg(args, rank, world, local_rank, dist, peak):
 
 def run_prefill(args, rank, world, local_rank):
     """Qwen2.5-7B: a "step" is one 4096-token prefill from an empty cache (tensor-core bound); the 256 decode steps that follow
-    in BASELINE.json's config are timed once and reported beside it."""
+    the prompt are timed once and reported beside it."""
     import torch
     from dataclasses import replace
     from fastllm_b200 import models, presets, tp as fltp

@@ -1,6 +1,6 @@
 // Paged-KV decode attention, split-K over the sequence, bulk-copy (TMA engine) staging in shared memory, sm_100a.
 //
-// Replaces the reference's K6-K11 chain (SURVEY.md section 2.4): whole-cache `cat`, `repeat_kv` materialisation,
+// Replaces the reference's K6-K11 chain: whole-cache `cat`, `repeat_kv` materialisation,
 // q.k^T matmul, scale, mask, softmax_last_dim, att.v matmul, transpose.  Here:
 //   * the KV cache is paged ([page][kv_head][64 tokens][d] bf16) and appended in place by the QKV GEMV epilogue;
 //   * one CTA owns (split, kv_head, row): it streams its pages' K and V chunks (contiguous 64*d*2 bytes each) into a

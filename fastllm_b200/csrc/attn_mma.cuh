@@ -11,7 +11,7 @@
 // Precision: q and the softmax probabilities are f32 in the oracle.  Both are split hi + lo into two bf16 operands and
 // multiplied against the same K / V fragments (as the dense GEMMs do with their activations), K/V are bf16 in the cache
 // already, accumulation is f32: results stay inside the kernel tolerance of the f32 oracle.
-// Semantics (SURVEY.md section 8a rows 1, 3, 4): scores * 1/sqrt(d) after the matmul, causal rows for multi-token calls,
+// Semantics: scores * 1/sqrt(d) after the matmul, causal rows for multi-token calls,
 // Mistral/Qwen2 sliding-window rule inside the prefill only (key j banned when j + sw < i, new tokens only; cached keys stay visible), softmax max-subtract/exp/sum/div.
 #pragma once
 #include "attn_decode.cuh"

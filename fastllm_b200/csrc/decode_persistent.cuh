@@ -156,7 +156,7 @@ __device__ __forceinline__ uint4 ldcg_u4(const void* p) {
 // L2 eviction-priority hint of the weight stream: weights are read exactly once per step and are dead once they are in shared
 // memory, so the demand loads carry evict_first and leave the L2 to the KV cache and the activations.
 // Prefetching the NEXT phase's weights into the L2 while the consumers sit between two weight phases (HBM idles there, and the L2
-// feeds these boxes at 14.3 TB/s against 6.4-7.5 TB/s from HBM, tools/tma_stream_bench.cu) was built twice in round 2 -- a
+// feeds these boxes at 14.3 TB/s against 6.4-7.5 TB/s from HBM) was built twice -- a
 // prefetch warp walking the CTA's static share N chunks ahead of the producer, with `cp.async.bulk.prefetch.tensor` and with
 // plain `prefetch.global.L2`, all the time or only inside the gaps -- and measured SLOWER every time (N = 4: -4 %, 8: -10 %,
 // 16: -15 %; DRAM bytes +1.4 %, only a third of the demand sectors turned into L2 hits): profiles/r02_persistent_limits.md.

@@ -2,7 +2,7 @@
 // The GEMMs run on tcgen05 (gemm_tc.cuh) with bf16 operands; to stay within parity tolerance of the f32 oracle every f32
 // activation x is split as x = hi + lo (hi = bf16(x), lo = bf16(x - hi)) and BOTH halves are multiplied with the same
 // staged weight tile (DUAL mode), i.e. ~16 mantissa bits on the activation side at no extra weight traffic.
-// These kernels implement the same fused steps as the GEMV epilogues in gemv.cuh.
+// These kernels implement the same fused steps as the GEMV epilogues in gemv.cuh (K1-K18).
 #pragma once
 #include "common.cuh"
 #include "gemv.cuh"
@@ -414,7 +414,7 @@ static __global__ void __launch_bounds__(256, 4) dense_silu_split_kernel(const f
     }
 }
 
-// ---- Mixtral sparse-MoE (candle-transformers models::mixtral::SparseMoeBlock; SURVEY.md section 8a row 7) ----------------
+// ---- Mixtral sparse-MoE (candle-transformers models::mixtral::SparseMoeBlock) ----------------
 // router: logits = x . W_gate^T, softmax over ALL experts (f32), stable descending sort (ties keep the LOWER expert index),
 // take top_k, renormalise by their sum; route_w[row][e] = weight or 0.  One CTA per row, one WARP per expert (128-bit loads,
 // one shuffle reduction each): the eight dot products of a Mixtral row run side by side instead of as eight block reductions.

@@ -388,7 +388,7 @@ static void bert_check(const BertModel& m) {
     FL_CHECK(*m.failed.p == 0, FL_ERR_CUDA, "a wait inside a kernel ran out, the results are not valid");
 }
 
-// Enqueue the encoder on m.stream: B1 -> 6 x (B2..B7) -> B8 (SURVEY.md section 2.4)
+// Enqueue the encoder on m.stream: B1 -> 6 x (B2..B7) -> B8
 static void bert_enqueue(BertModel& m, const BertRun& run, int b, int t, bool has_mask) {
     if (run.path == BertPath::small) {
         bert_enqueue_small(m, run, b, t, has_mask);

@@ -321,7 +321,7 @@ static void build_weights(Weights& w) {
     }
     w.rope_cos = (float*)(base + o_cos);
     w.rope_sin = (float*)(base + o_sin);
-    // bytes one decode step must stream: every parameter except the embedding table (SURVEY.md section 8d)
+    // bytes one decode step must stream: every parameter except the embedding table
     const uint64_t mlp = moe ? (uint64_t)w.E_local * 3 * I * H : 3 * I * H;     // every local expert is streamed each step
     w.streamed_bytes = 2 * ((uint64_t)w.L * ((uint64_t)w.nqkv * H + H * nq + mlp) + V * H) +
                        4 * ((uint64_t)w.L * (2 * H + (c.qkv_bias ? w.nqkv : 0) + (moe ? (uint64_t)w.E * H : 0)) + H);
@@ -1212,7 +1212,7 @@ int dense_gemm(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int N, int K,
     // prefill: 128 tokens x 256 weight rows per tile.  The hi/lo activation pair makes a k-block 2 x 16 KB of A next to the weight
     // tile, and the GEMM is bound by the shared-memory fill rate (L2 -> SM), not by the tensor pipe: a 256-row weight tile is
     // 64 KB per 2 x 128 x 256 x 64 MACs where the 128-row one is 48 KB per half of that -- 1.5x the arithmetic per staged byte.
-    static const int prefill_bn = env_flag("FL_PREFILL_BN128") ? 128 : 256;      // dev knob: the 128-row tile of round 1
+    static const int prefill_bn = env_flag("FL_PREFILL_BN128") ? 128 : 256;      // dev knob: the 128-row tile
     const int tiles = ((R + kGemmBM - 1) / kGemmBM) * ((N + prefill_bn - 1) / prefill_bn);
     const DecPlan dec = swap ? dec_plan(N, K, R) : DecPlan{};
     const int ks = swap ? dec.slices : (silu_hi != nullptr ? 1 : prefill_ks);
@@ -1722,7 +1722,7 @@ void step_check(fl_cache& c) {
 static void use_device() {
     const int dev = g_device.load();
     FL_CHECK(dev >= 0, FL_ERR_STATE, "fl_init has not been called");
-    FL_CUDA(cudaSetDevice(dev));   // no thread-affine state: callers may hop OS threads between calls (SURVEY.md section 8b)
+    FL_CUDA(cudaSetDevice(dev));   // no thread-affine state: callers may hop OS threads between calls
 }
 
 extern "C" {
@@ -1740,7 +1740,7 @@ FL_EXPORT int fl_init(int device) {
     FL_CUDA(cudaGetDeviceProperties(&prop, device));
     FL_CHECK(prop.major == 10, FL_ERR_UNSUPPORTED,
              std::string("fastllm_b200 is built for sm_100a (B200) only; found ") + prop.name);
-    // one process drives ONE GPU (a process per GPU); per-process state -- the opt-in shared-memory
+    // one process drives ONE GPU; per-process state -- the opt-in shared-memory
     // attributes of the kernels, the exchange area, the communicator -- is bound to the first device
     const int cur = g_device.load();
     FL_CHECK(cur < 0 || cur == device, FL_ERR_STATE, "fl_init: this process is already bound to device " + std::to_string(cur));

@@ -7,7 +7,7 @@
 //     accumulating f32 in TMEM; tcgen05.commit releases ring slots / signals the epilogue through mbarriers;
 //   * warp roles: warp 0 = TMA producer, warp 1 = TMEM allocator + MMA issuer, warps 2-5 = epilogue (tcgen05.ld
 //     32x32b: thread == accumulator row), which applies bias / GELU-tanh / residual and stores bf16 or f32.
-// Replaces the reference's cuBLAS-through-candle matmuls + separate bias/activation kernels (SURVEY.md section 2.4 B2, B5,
+// Replaces the reference's cuBLAS-through-candle matmuls + separate bias/activation kernels (B2, B5,
 // B6, B7 and K3/K12/K15/K16 for prefill).
 #pragma once
 #include <cuda.h>

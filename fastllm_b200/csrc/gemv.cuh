@@ -1,11 +1,11 @@
 // HBM-bound bf16 weight-streaming GEMV family for decode (1-2 activation rows), sm_100a.
 //
 // Replaces, per decoder layer, the reference's cuBLAS-through-candle matmuls plus the element-wise kernels around
-// them (SURVEY.md section 2.4): K2+K3+K4+K5+K6 (RMSNorm -> q/k/v Linear(+bias) -> RoPE -> KV append) in ONE kernel,
+// them: K2+K3+K4+K5+K6 (RMSNorm -> q/k/v Linear(+bias) -> RoPE -> KV append) in ONE kernel,
 // K12+K13 (o_proj + residual), K14+K15 (RMSNorm -> gate/up -> SiLU*up), K16 (down_proj + residual) and
 // K17 (final RMSNorm -> lm_head -> f32 logits + arg-max partials).
 //
-// Design (DESIGN.md section "GEMV"):
+// Design:
 //   * y[n] = sum_k W[n,k] x[k];  W is bf16 [N,K] row-major and is read exactly once per step with 128-bit
 //     ld.global.nc.L1::no_allocate loads.  One CTA per SM (grid = 148 x ctas_per_sm), each owning a contiguous,
 //     even-aligned slice of rows, so every kernel is a single resident wave.

@@ -405,7 +405,7 @@ class _OffsetCache:
 
 class LlamaCache(_OffsetCache):
     """llama.rs:61-92.  In the reference this owns candle's KV `Cache`; here it owns the device KV cache, created lazily
-    on the first forward because initialize_cache(device, dtype) gets no model argument (SURVEY.md section 8b)."""
+    on the first forward because initialize_cache(device, dtype) gets no model argument."""
 
     def __init__(self):
         super().__init__()
@@ -1140,7 +1140,7 @@ class Model:
         return (out, trace) if return_logits else out
 
     def generate_batch(self, prompts, max_tokens: int, temperature: float = 0.0, max_batch: int = 64):
-        """Request batching at the API boundary (SURVEY.md section 8f-3; the reference serialises requests at batch 1 under a
+        """Request batching at the API boundary (the reference serialises requests at batch 1 under a
         mutex, chat.rs:206-208).  Exact by construction: only prompts of EQUAL token length share a batch, so the sequences of
         a group advance in lock-step through one [b, t] forward per step (no padding, one KV length), every sequence has its
         own LogitsProcessor seeded 0 like every request of the reference, and a sequence that hit EOS keeps its row (fed its
@@ -1188,7 +1188,7 @@ class Model:
 
 
 class ContinuousBatcher:
-    """Continuous batching above fl_forward_slots (SURVEY.md section 8f-3).  The reference serialises chat requests at batch 1
+    """Continuous batching above fl_forward_slots.  The reference serialises chat requests at batch 1
     under one mutex (api/chat.rs:206-208); here up to `max_batch` requests of ANY lengths share the decode steps: a request is
     admitted into a free sequence slot as soon as one exists (its prompt is prefilled alone, [1, T]), every step then advances all
     running requests by one token in ONE ragged forward ([n, 1], per-slot KV lengths and RoPE positions), and a request that
@@ -1376,7 +1376,7 @@ class MiniLMModel:
         return out
 
     def embed_many(self, sentences, max_batch: int = 256) -> np.ndarray:
-        """`input: [String]` batching (SURVEY.md section 8f-3; the reference takes one string per request, api/embeddings.rs:11-15).
+        """`input: [String]` batching (the reference takes one string per request, api/embeddings.rs:11-15).
         Exact by construction: the reference's attention applies NO mask (embeddings.rs:155-159) and a lone sentence has an
         all-ones mask, so padding would change results; sentences of EQUAL token length are therefore grouped into one [b, t]
         call each (no padding) and the rows scattered back in request order.  Returns f32 [len(sentences), hidden]."""

@@ -1,4 +1,4 @@
-"""config.json presets of the BASELINE.json models (sizes only), as the adapters' ConfigFile (llama.rs:17-29 etc.)."""
+"""config.json presets of the headline models (sizes only), as the adapters' ConfigFile (llama.rs:17-29 etc.)."""
 from .models import ConfigFile, LlamaWithConfig, MistralWithConfig, MixtralWithConfig, QwenWithConfig
 
 # TinyLlama-1.1B-Chat: the shape llama.rs:125-145 hard-codes for its cache

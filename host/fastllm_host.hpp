@@ -212,7 +212,7 @@ struct Model {
     }
 };
 
-// ---- continuous batching above fl_forward_slots (SURVEY.md section 8f-3; the reference serialises requests at batch 1 under one
+// ---- continuous batching above fl_forward_slots (the reference serialises requests at batch 1 under one
 // mutex, api/chat.rs:206-208).  Transliteration of fastllm_b200/models.py ContinuousBatcher: a request is admitted into a free
 // sequence slot (its prompt prefilled alone), every step advances all running requests by one token in ONE ragged forward, a
 // finished request frees its slot.  Per request: its own LogitsProcessor seeded 0, EOS break before emitting, the adapter's
@@ -456,7 +456,7 @@ struct MiniLMModel {
         for (size_t i = 0; i < va.size(); ++i) { dot += (double)va[i] * vb[i]; na += (double)va[i] * va[i]; nb += (double)vb[i] * vb[i]; }
         return (float)(dot / (std::sqrt(na) * std::sqrt(nb)));
     }
-    // `input: [String]` batching (SURVEY.md section 8f-3), exact: only sentences of EQUAL token length share a [b, t] call (the
+    // `input: [String]` batching, exact: only sentences of EQUAL token length share a [b, t] call (the
     // reference's attention has no mask, so padding would change results); rows come back in request order
     std::vector<std::vector<float>> embed_many(const std::vector<std::vector<uint32_t>>& sentences, int max_batch = 256) const {
         std::vector<std::vector<float>> out(sentences.size());

@@ -1,5 +1,5 @@
 /* fastllm_b200 — C ABI of the B200-native transformer forward pass that slots in under fastllm's
- * trait-based model API (the L2->L0 boundary of SURVEY.md section 1 / section 8b).
+ * trait-based model API.
  *
  * Every entry point is `extern "C"`, takes plain pointers/sizes, returns 0 on success and a negative
  * fl_status on failure; the message for the calling thread's last failure is fl_last_error().  Nothing
@@ -297,7 +297,7 @@ FL_EXPORT int fl_model_create(const fl_config* cfg, fl_model** out);
 FL_EXPORT int fl_model_create_layered(const fl_stack_config* cfg, const fl_layer_desc* layers, fl_model** out);
 /* Upload one tensor by its HuggingFace name (same names VarBuilder asks for).  f32/f16 inputs are rounded to
  * bf16 (round-to-nearest-even), as VarBuilder::from_tensors(.., DType::BF16, ..) does (main.rs:120).  The host
- * buffer may be freed on return.  q/k/v and gate/up are fused and row-permuted on upload (DESIGN.md). */
+ * buffer may be freed on return.  q/k/v and gate/up are fused and row-permuted on upload. */
 FL_EXPORT int fl_model_put_tensor(fl_model* m, const char* name, int dtype, const int64_t* shape, int rank, const void* host_ptr);
 /* Deterministic synthetic weights generated on the device (rule: oracle/synth.py; N(0,std^2)-like -> bf16,
  * norm weights 1.0).  Used by the benchmark instead of shipping 14-93 GB of tensors. */
@@ -332,7 +332,7 @@ FL_EXPORT int fl_forward_greedy(fl_model* m, fl_cache* c, const uint32_t* ids, i
 FL_EXPORT int fl_decode_greedy_loop(fl_model* m, fl_cache* c, const uint32_t* first_ids, int b, size_t rope_offset, int steps,
                           uint32_t* out_ids, float* elapsed_ms);
 
-/* ---- continuous batching: sequence slots with their own lengths (SURVEY.md section 8f-3) -------------------------------------
+/* ---- continuous batching: sequence slots with their own lengths -------------------------------------
  * The reference serialises requests at batch 1 under a mutex (api/chat.rs:206-208) and runs streams concurrently at batch 1 each
  * (models/mod.rs:151-175).  A cache created with max_batch > 1 holds max_batch independent sequence SLOTS; fl_forward_slots feeds
  * t new tokens to each of n distinct slots in ONE forward -- a new request's prompt (n = 1, t = prompt length) or one decode step

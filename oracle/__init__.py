@@ -1,8 +1,7 @@
 """CPU oracle for the fastllm transformer forward pass.  TEST INFRASTRUCTURE ONLY.
 
 This package is a CPU *restatement* (numpy, f32) of the arithmetic the
-reference issues through candle 0.8.x for the hot path named in
-BASELINE.json / SURVEY.md section 8:
+reference issues through candle 0.8.x for the hot path:
 
   * Llama / Mistral / Qwen2 causal-LM forward (prefill + decode)
       reference adapters: src/models/llama.rs:147-149, src/models/mistral.rs:206-236,
@@ -12,7 +11,7 @@ BASELINE.json / SURVEY.md section 8:
   * the Mixtral sparse-MoE block (candle-transformers models::mixtral; not wired in the reference)
 
 PARITY STATUS: **parity unpinned by the reference**.  The reference holds no
-golden vectors or known-answer tests for this path (SURVEY.md section 4), its
+golden vectors or known-answer tests for this path, its
 arithmetic lives in the un-vendored crates candle-core/candle-nn/
 candle-transformers "^0.8.2" (Cargo.toml:19-21, no Cargo.lock), and there is no
 Rust toolchain in the image, so the reference itself cannot be run here.  The

@@ -7,7 +7,7 @@ What follows which reference line:
   * QwenAdapter.forward       -> src/models/qwen.rs:129-145    (same rule as Mistral)
   * generate()                -> src/models/mod.rs:363-463     (prefill at pos 0, arg-max, EOS break before emit)
   * sample_argmax()           -> candle_transformers::generation::LogitsProcessor (ties -> LAST index)
-  * CausalLM.forward          -> candle-transformers 0.8.x models::{llama,mistral,qwen2} (un-vendored; SURVEY.md section 8a rows 1,3,4)
+  * CausalLM.forward          -> candle-transformers 0.8.x models::{llama,mistral,qwen2} (un-vendored)
 """
 from __future__ import annotations
 
@@ -129,7 +129,7 @@ class CausalLM:
         j = np.arange(t)[None, :]
         if self.cfg.arch == ARCH_LLAMA:
             # candle llama.rs Cache::mask: mask[i][j] = (j > i); masked_fill(att, mask, -inf).  t x t only,
-            # so a Llama prefill must start from an empty cache (SURVEY.md section 8a row 1).
+            # so a Llama prefill must start from an empty cache.
             assert offset == 0, "candle Llama cannot prefill t>1 on a non-empty cache (t x t mask)"
             banned = j > i
         else:
@@ -205,7 +205,7 @@ class CausalLM:
         return ops.linear(last, w["lm_head.weight"])
 
 
-# ---- reference adapters (the L2 layer of SURVEY.md section 1) -------------------------------------
+# ---- reference adapters -------------------------------------
 
 @dataclass
 class OffsetCache:

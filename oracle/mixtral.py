@@ -2,7 +2,7 @@
 
 The reference does not wire Mixtral at all (src/models/model_registry.rs:169-182 has no key that
 "MixtralForCausalLM" contains; src/models/mistral.rs:244-246 accepts only MistralForCausalLM), so this follows
-candle-transformers 0.8.x models::mixtral::SparseMoeBlock::forward (un-vendored; SURVEY.md section 8a row 7):
+candle-transformers 0.8.x models::mixtral::SparseMoeBlock::forward (un-vendored):
 
     router_logits = x . W_gate^T                      [n, E]
     routing       = softmax_last_dim(router_logits)   over ALL experts, f32

@@ -1,7 +1,6 @@
 """Deterministic synthetic weights / token ids (TEST INFRASTRUCTURE, see oracle/__init__.py).
 
-The benchmark models are random-init (no network, no checkpoints; SURVEY.md
-section 8d "Synthetic inputs").  Host and device must produce *bit-identical*
+The benchmark models are random-init (no network, no checkpoints).  Host and device must produce *bit-identical*
 bf16 weights without shipping 14-93 GB of tensors, so the generator is
 counter-based and uses integer arithmetic plus ONE IEEE f32 multiply chain (no
 transcendental functions whose last-ulp behaviour differs between libm and CUDA):

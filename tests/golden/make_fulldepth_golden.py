@@ -1,12 +1,11 @@
-"""Generates tests/golden/fulldepth_tinyllama.json: BASELINE.json config 1 at FULL depth on the f32 oracle.
+"""Generates tests/golden/fulldepth_tinyllama.json: TinyLlama-1.1B at FULL depth on the f32 oracle.
 
     TinyLlama-1.1B (22 layers, llama.rs:125-145 shape), synthetic weights (oracle/synth.py, seed 0, std 0.02),
     prompt = 128 synthetic ids, 64 greedy steps through the reference's generate loop (models/mod.rs:411-453).
 
 Prompt seed.  Random-init logits over 32000 tokens have top-1/top-2 gaps that are exponentially distributed with mean ~0.28: in
 64 steps some gap is almost always < 1e-2, and a step like that says nothing about a kernel (the product's bf16 KV cache alone
-moves logits by ~1e-2 against the f32 oracle; SURVEY.md section 7, hard part 1 asks to "choose/record seeds whose margins exceed
-the measured error").  `--search N` runs seeds 1..N and prints, per seed, the smallest margin over the first 32 and over all 64
+moves logits by ~1e-2 against the f32 oracle): the seed has to be one whose margins exceed the measured error.  `--search N` runs seeds 1..N and prints, per seed, the smallest margin over the first 32 and over all 64
 steps; the committed golden uses PROMPT_SEED = the seed with the largest 32-step minimum among 1..300 (ties: larger 64-step
 minimum).  Nothing else about the run is selected.
 

@@ -2,7 +2,7 @@
 
 Run here (authoring container, no GPU):   python tests/golden/make_golden.py
 
-The reference has no golden vectors for the forward pass (SURVEY.md section 4 / 8c) and cannot be built (no Rust
+The reference has no golden vectors for the forward pass and cannot be built (no Rust
 toolchain), so the pins are: (1) the oracle, which restates candle 0.8.x; (2) an independent implementation, HF
 transformers, with the known deltas neutralised (BERT: token-type embedding zeroed, tanh-GELU, all-ones mask;
 Mistral/Qwen2: compared in POSITION-CORRECT mode because HF does not have the adapters' +1-per-call offset quirk).
@@ -117,7 +117,7 @@ def make_causal(name: str, cfg: ocl.CausalLMConfig, check_hf: bool = True):
         key = "faithful" if cfg.arch == "llama" else "poscorrect"
         if cfg.sliding_window < PROMPT + NEW:
             # candle applies the window only inside the PREFILL mask and never trims the KV cache, so decode attends the
-            # full history (SURVEY.md section 5 "Long context"); HF windows decode too.  Only the prefill logits compare.
+            # full history; HF windows decode too.  Only the prefill logits compare.
             htoks, hlogits = list(res[f"{key}_ids"]), hlogits[:1]
         err = max(float(np.abs(a - b).max()) for a, b in zip(hlogits, res[f"{key}_logits"]))
         assert htoks == list(res[f"{key}_ids"]), (name, htoks, res[f"{key}_ids"])

@@ -3,7 +3,7 @@ stream into equal ranges, so a (sequence, kv head) pair may lie inside one CTA's
 many.  These cases need MORE pages than resident CTAs (296-444), which the tiny parity configs never reach: here 96-192 ragged
 sequences of 1 .. 15 pages decode together, at head dims 32 (unswizzled box), 64 and 128 (one / two swizzled TMA boxes per page).
 The prompts (up to 960 tokens, prefilled on empty slots) also run the tcgen05 prefill attention (attn_prefill_tc_kernel: head dims 64 /
-128, several 128-query tiles, a 100-token sliding window in one case).  Every row against a per-sequence oracle with the same bf16 KV rounding (8f-3)."""
+128, several 128-query tiles, a 100-token sliding window in one case).  Every row against a per-sequence oracle with the same bf16 KV rounding."""
 import numpy as np
 import pytest
 

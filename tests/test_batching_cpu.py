@@ -1,4 +1,4 @@
-"""Request batching at the API boundary (SURVEY.md section 8f-3): host logic, tested on CPU against a stand-in model.
+"""Request batching at the API boundary: host logic, tested on CPU against a stand-in model.
 
 The batcher is exact by construction -- only requests of equal token length share a [b, t] call -- so the property under test is
 generate_batch(prompts) == [generate(p) for p in prompts] and embed_many(sentences)[i] == embed(sentences[i]), in request order,

@@ -1,4 +1,4 @@
-"""CPU checks of the measurement contract pieces that do not need a GPU: workloads cover BASELINE.json's configs, the committed
+"""CPU checks of the measurement contract pieces that do not need a GPU: workloads cover the headline models, the committed
 ncu capture feeds `roofline.traffic`, the reference arm answers for every workload, the default flags finish within minutes."""
 import json
 import os
@@ -20,7 +20,7 @@ def test_workloads_cover_baseline_configs():
 
 def test_ncu_traffic_matches_algorithmic_bytes():
     """profiles/rNN_persistent*_full_raw.csv (newest round): DRAM bytes per decode step of the persistent kernel == weights once +
-    KV once (Mistral-7B b=1, KV 2048: 14.490 GB, SURVEY.md section 8d) within 1 %, and the line names the file it comes from."""
+    KV once (Mistral-7B b=1, KV 2048: 14.490 GB) within 1 %, and the line names the file it comes from."""
     import bench
     t, src = bench.ncu_traffic_per_step()
     assert t is not None and abs(t / 14.490e9 - 1.0) < 0.01, t

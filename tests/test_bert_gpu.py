@@ -1,6 +1,6 @@
 """GPU parity of the BERT/MiniLM encoder path (tcgen05 GEMMs + fused attention) against the oracle.
 
-Tolerance (north_star): cosine >= 0.999 per embedding; the path runs bf16 tensor-core inputs with f32 accumulation, so
+Tolerance: cosine >= 0.999 per embedding; the path runs bf16 tensor-core inputs with f32 accumulation, so
 max-abs on the unit-norm embedding components is also held to 2e-2.
 """
 import os

@@ -1,5 +1,5 @@
-"""Full-depth parity on the BASELINE.json configurations (SURVEY.md section 8c "full TinyLlama 128+64 ids"; north_star: "greedy
-token ids must be identical for the first 32 generated tokens, logits within a stated tolerance").
+"""Full-depth parity on the headline configurations: greedy token ids identical for the first 32 generated tokens, logits within a
+stated tolerance.
 
 Config 1: TinyLlama-1.1B, ALL 22 layers, a real 128-token prefill and 64 greedy decode steps through the reference's generate
 loop (models/mod.rs:411-453), against
@@ -12,7 +12,7 @@ Tolerances at full depth (stated here, measured values are printed by the test):
   KERNEL_TOL_FULL = 1.5e-2 max-abs logits vs the oracle with the same bf16 KV rounding
 The prompt seed is the one of 1..300 whose f32-oracle top-1/top-2 margin over the first 32 steps is largest (selection rule in
 tests/golden/make_fulldepth_golden.py, margins in the golden file): random-init logits have top-2 gaps down to 1e-3, and an id
-flip on such a step says nothing about the kernels (hard part 1).  So: the first 32 free-running ids must be
+flip on such a step says nothing about the kernels.  So: the first 32 free-running ids must be
 IDENTICAL; past them, and for every teacher-forced step, an arg-max may differ only where the oracle's gap is within 2x the
 measured logits error of that step.
 """
@@ -79,7 +79,7 @@ def test_tinyllama_full_depth_prompt128_greedy64():
     print(f"TinyLlama 22L 128+64 (teacher-forced): max-abs logits err vs f32 oracle {err:.3e} (tol {LOGIT_TOL_FULL}), vs bf16-KV oracle "
           f"{kerr:.3e} (tol {KERNEL_TOL_FULL}); arg-max == oracle id on {64 - len(flips)}/64 steps, differs at {flips}")
     assert err <= LOGIT_TOL_FULL and kerr <= KERNEL_TOL_FULL
-    # north_star: the first 32 generated ids are identical to the reference CPU path's
+    # the first 32 generated ids are identical to the reference CPU path's
     assert ids[:32] == g["ids"][:32], f"greedy ids diverge from the f32 oracle at step {n_same}"
     if n_same < 64:
         assert g["margins"][n_same] <= 2 * errs[n_same]
@@ -248,8 +248,8 @@ def test_batched_decode_graph_captured_at_a_short_context_stays_correct():
 
 
 def test_minilm_baseline_batch_256x128():
-    """BASELINE.json config 2 at its full size: all-MiniLM-L6-v2 shapes, 256 sentences x 128 tokens, against the f32 oracle
-    (north_star: cosine >= 0.999 per embedding; max-abs on the unit-norm components reported and held to 2e-2)."""
+    """The headline encoder at its full size: all-MiniLM-L6-v2 shapes, 256 sentences x 128 tokens, against the f32 oracle
+    (cosine >= 0.999 per embedding; max-abs on the unit-norm components reported and held to 2e-2)."""
     from oracle import bert as obert
     from fastllm_b200 import models
     cfg = obert.MINILM_L6

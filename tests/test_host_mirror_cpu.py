@@ -1,4 +1,4 @@
-"""The reference's own unit tests (SURVEY.md section 4), re-stated against the product's host-side mirror (fastllm_b200/models.py)
+"""The reference's own unit tests, re-stated against the product's host-side mirror (fastllm_b200/models.py)
 and the C ABI's config failure points.  No GPU: config validation is host logic and runs before the library touches a device.
 
 Reference tests mirrored (paths under /root/reference/src/models):

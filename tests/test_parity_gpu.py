@@ -6,7 +6,7 @@ So every case is checked twice:
   * against the oracle run with kv_dtype="bf16" (same cache rounding): logits max-abs <= KERNEL_TOL = 3e-3 (a 1e-7
     summation-order difference, or the 2^-17 residue of the hi/lo bf16 split on the tensor-core path, can flip the bf16
     rounding of a cached K/V element, which then moves logits by ~1e-3; without a flip the measured gap is 1e-6..3e-4)
-    -- this pins the kernels themselves; at the BASELINE models' true widths (more cached elements, more flips) the bar is
+    -- this pins the kernels themselves; at the headline models' true widths (more cached elements, more flips) the bar is
     KERNEL_TOL_WIDE = 6e-3 (measured 1e-4 .. 3.3e-3);
   * against the pure-f32 oracle / golden vectors: greedy ids IDENTICAL, and logits max-abs <= LOGIT_TOL = 5e-2
     (measured: 0.6e-2 .. 3.2e-2 over 32000 x 5 logits of std 1.3, i.e. ~0.5 % rms -- the bf16 KV rounding, nothing else).
@@ -153,7 +153,7 @@ def test_device_random_init_matches_host_generator():
 
 @pytest.mark.parametrize("arch", ["tinyllama", "mistral7b", "qwen25_7b"])
 def test_true_width_two_layers(arch):
-    """True per-layer shapes of the BASELINE models (2 layers; reduced vocab for Qwen to keep the CPU side small):
+    """True per-layer shapes of the headline models (2 layers; reduced vocab for Qwen to keep the CPU side small):
     prefill + 4 greedy steps against the oracle on the same synthetic weights."""
     from dataclasses import replace
     base = {"tinyllama": ocl.TINYLLAMA, "mistral7b": ocl.MISTRAL_7B, "qwen25_7b": replace(ocl.QWEN25_7B, vocab_size=32064)}[arch]

@@ -1,4 +1,4 @@
-"""Sampling step of the generate loop (SURVEY.md section 8f-1): candle's LogitsProcessor over rand 0.8's StdRng.
+"""Sampling step of the generate loop: candle's LogitsProcessor over rand 0.8's StdRng.
 
 CPU tests: the generator is pinned by published known-answer vectors (the ChaCha key stream for the all-zero key, and rand
 0.8's own value-stability vector for StdRng); the product's sampler (host code inside libfastllm_b200.so, reached through the

@@ -35,7 +35,7 @@ def _ngpu():
 
 
 @pytest.mark.gpu
-@pytest.mark.skipif(_ngpu() < 2, reason="needs 2 GPUs (gpurun --gpus 2)")
+@pytest.mark.skipif(_ngpu() < 2, reason="needs 2 GPUs")
 def test_tp2_matches_tp1(tmp_path):
     r1 = _run("gpu", 1, str(tmp_path / "tp1.json"), 29641)
     r2 = _run("gpu", 2, str(tmp_path / "tp2.json"), 29642)
@@ -67,7 +67,7 @@ def test_tpN_matches_tp1_at_true_widths(n, tmp_path):
     (1 layer, 8 experts).  Teacher-forced with fixed tokens; logits within the true-width kernel tolerance (the split changes the
     summation order), arg-max identical wherever the single-GPU top-2 gap exceeds that noise."""
     if _ngpu() < n:
-        pytest.skip(f"needs {n} GPUs (gpurun --gpus {n})")
+        pytest.skip(f"needs {n} GPUs")
     r1 = _run("gpu_wide", 1, str(tmp_path / "w1.json"), 29651)
     rn = _run("gpu_wide", n, str(tmp_path / f"w{n}.json"), 29652 + n)
     for tag in ("mistral7b", "qwen25_7b"):

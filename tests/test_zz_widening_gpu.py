@@ -1,5 +1,4 @@
-"""GPU tests of the SURVEY.md section 8f widening rows -- sampling (8f-1) and equal-length request batching (8f-3).  Written after the
-round's GPU budget was spent, so the file name sorts after the parity suites: they run last.
+"""GPU tests of sampling and of equal-length request batching.  The file name sorts after the parity suites: they run last.
 
 fl_forward_sample = fl_forward + the library's LogitsProcessor on row 0.  The kernels are deterministic, so a second cache fed
 the same ids produces the same logits; sampling those with the ORACLE's LogitsProcessor (same seed) must give the same ids."""
