@@ -192,7 +192,7 @@ def run_minilm(args, rank, world, local_rank):
             "e2e": {"value": B / e2e_s, "unit": "emb/s", "h2d_bytes_per_step": int(b * T * 4), "d2h_bytes_per_step": int(b * 384 * 4)},
             "gpu_launches": int(launches),
             "roofline": {"bound": "tensor", "achieved": tflops, "peak": peak, "unit": "TFLOP/s", "frac": tflops / peak, "traffic": None,
-                         "kernel": "gemm_tc_kernel<128,EPI> (tcgen05/TMEM/TMA) x 24 + bert_attn_kernel x 6 per batch: whole-encoder algorithmic FLOPs / device time",
+                         "kernel": "bert_block_kernel x 6 (tcgen05 on SM pairs) + gemm_tc_kernel<128, BIAS_BF16> x 6 + bert_attn_kernel x 6 per batch: whole-encoder algorithmic FLOPs / device time",
                          "peak_source": src},
             "cpu_baseline": cpu}
     print(json.dumps(line), flush=True)
@@ -656,9 +656,9 @@ def run_ours(args, rank, world, local_rank):
     pk = [p for p in prof if p["kernel"] == "decode_persistent"]
     if pk:      # batch-1: the whole step is ONE persistent kernel; its algorithmic bytes = streamed weights + KV read
         dom, dom_name = pk, "decode_persistent_kernel<D> (whole decode step: weight stream + attention + arg-max, 4 steps per launch here)"
-    elif any(p["kernel"].startswith("gemm_tc_") for p in prof):   # dense path: tcgen05 swap-AB weight-streaming GEMMs
+    elif any(p["kernel"].startswith("gemm_tc_") for p in prof):   # dense path: tcgen05 weight-streaming GEMMs
         dom = [p for p in prof if p["kernel"].startswith("gemm_tc_")]
-        dom_name = "gemm_tc_kernel<BN, F32_T, DUAL_B> family (tcgen05 swap-AB split-K weight streaming: qkv, o, gate|up / experts, down, lm_head)"
+        dom_name = "gemm_dec_kernel<BN> (tcgen05 weight streaming: qkv, o, gate|up, down, lm_head), gemm_tc_kernel<BN, F32_T, DUAL_B> (experts)"
     else:       # multi-kernel path: the GEMV family dominates
         dom = [p for p in prof if p["kernel"].startswith("gemv_")]
         dom_name = "gemv_kernel<M,CPT,PRO,EPI> family (qkv+rope, o+resid, gate/up+silu, down+resid, lm_head)"
@@ -853,7 +853,7 @@ def run_prefill(args, rank, world, local_rank):
             "gpu_launches": int(launches),
             "roofline": {"bound": "tensor", "achieved": lin_tflop / world / (gemm_ms / 1e3), "peak": peak, "unit": "TFLOP/s",
                          "frac": lin_tflop / world / (gemm_ms / 1e3) / peak, "traffic": None,
-                         "kernel": "gemm_tc_kernel<128, F32, DUAL_A> (tcgen05 prefill GEMMs; algorithmic linear FLOPs per GPU / their CUDA-event time; "
+                         "kernel": "gemm_pair_kernel<EPI> and gemm_tc_kernel<256, EPI, DUAL_A> (tcgen05 prefill GEMMs; algorithmic linear FLOPs per GPU / their CUDA-event time; "
                                    "the hi/lo activation split issues 2x these FLOPs on the tensor pipe)",
                          "peak_source": src, "kernel_share_of_step": gemm_ms / dev_ms if dev_ms else None,
                          "whole_step": {"algorithmic_tflop": tflop, "achieved_tflops_per_gpu": tflop / world / dt, "frac": tflop / world / dt / peak},

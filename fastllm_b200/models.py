@@ -173,7 +173,9 @@ class _ResultPool:
 
 
 class DeviceCache:
-    """fl_cache*: paged KV cache + per-cache stream/workspaces."""
+    """fl_cache*: paged KV cache + per-cache stream/workspaces.  The logits arrays that its calls return may lie over page-locked memory of the
+    cache's pool (see _ResultPool): they are the caller's like any array and outlive the cache, but do not own their memory, so that
+    `ndarray.resize` refuses them (`np.resize` and `copy` do not)."""
 
     def __init__(self, model: DeviceModel, max_batch: int, max_seq: int, pool_tokens: int | None = None):
         """pool_tokens (layered models): the cache's pages are a pool of that many tokens shared by the max_batch sequence slots,
