@@ -766,6 +766,7 @@ void layered_cache_create(fl_cache& c, int max_slots, int max_seq, int pool_toke
     FL_CUDA(cudaStreamCreateWithFlags(&c.stream, cudaStreamNonBlocking));
     c.ly.reset(new LayeredCache);
     LayeredCache& y = *c.ly;
+    y.h_logits.alloc((size_t)max_slots * m.V);          // a row per sequence; steps that want more take it then (ensure_ws)
     y.f32 = m.f32;
     const int pages = (pool_tokens + kKvPage - 1) / kKvPage;
     y.pool = PagePool(pages, max_slots, c.pages_per_seq, kKvPage);
@@ -942,7 +943,8 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
         FL_CUDA(cudaStreamSynchronize(c.stream));
         drop_graphs(c);
         const size_t N = std::max<size_t>(n_want, 2 * y.want_cap);
-        y.hf.alloc(N * m.W); y.logits.alloc(N * m.V); y.h_logits.alloc(N * m.V);
+        y.hf.alloc(N * m.W); y.logits.alloc(N * m.V);
+        if (y.h_logits.n < N * m.V) y.h_logits.alloc(N * m.V);
         if (!m.f32) { y.hf_hi.alloc(N * m.W); y.hf_lo.alloc(N * m.W); }
         y.want_cap = N;
     }

@@ -1,10 +1,6 @@
 // fastllm_b200: C-ABI entry points + causal-LM decode/prefill orchestration (sm_100a).
 // See include/fastllm_b200.h for the reference interface each entry point replaces.
-#include <unistd.h>
-
 #include <cmath>
-#include <cstdlib>
-#include <memory>
 #include <sstream>
 #include <thread>
 
@@ -1753,15 +1749,7 @@ FL_EXPORT int fl_host_alloc(size_t bytes, void** out) {
     FL_API_BEGIN
     FL_CHECK(out && bytes > 0, FL_ERR_INVALID, "bad argument");
     use_device();
-    // The process's own memory, page-locked: cudaMallocHost hands out a shared mapping, through which a forked child would see every later result
-    // in the place of the one that it holds (registered pages are copied at a fork like any others).  Whole pages: no neighbour shares one.
-    const size_t page = (size_t)sysconf(_SC_PAGESIZE);
-    FL_CHECK(bytes <= SIZE_MAX - page, FL_ERR_INVALID, "bad argument");
-    const size_t size = (bytes + page - 1) / page * page;
-    std::unique_ptr<void, decltype(&std::free)> p(std::aligned_alloc(page, size), &std::free);
-    FL_CHECK(p != nullptr, FL_ERR_INVALID, "out of host memory");
-    FL_CUDA(cudaHostRegister(p.get(), size, cudaHostRegisterDefault));
-    *out = p.release();
+    *out = lock_host(bytes);
     FL_API_END
 }
 
@@ -1769,8 +1757,7 @@ FL_EXPORT int fl_host_free(void* p) {
     FL_API_BEGIN
     if (p) {
         use_device();
-        FL_CUDA(cudaHostUnregister(p));
-        std::free(p);
+        unlock_host(p);
     }
     FL_API_END
 }

@@ -162,7 +162,7 @@ struct LayeredCache {
     DevBuf<float> cq, qx;               // query latents [rows, max_qr], the queries expanded from them [rows, max_q]
     DevBuf<float> cv, rs;               // recurrent mixers: convolved + activated columns [rows, max_cv]; per-head (decay, strength) [rows, 2 heads]
     DevBuf<int> route_sel, pair_row, pair_of, grp_off, tile_off;
-    PinnedBuf<float> h_logits;
+    HostBuf<float> h_logits;
     // serving precision: hi/lo halves of the activations that feed tensor-core GEMMs, and the split-K slices of their outputs
     DevBuf<uint16_t> h_hi, h_lo, cq_hi, cq_lo, qp_hi, qp_lo, qo_hi, qo_lo, ol_hi, ol_lo, u_hi, u_lo, act_hi, act_lo, hf_hi, hf_lo;
     DevBuf<float> gemm_out;

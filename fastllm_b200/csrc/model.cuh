@@ -150,7 +150,7 @@ struct fl_cache {
     fl::DevBuf<float> am_val;             // arg-max partials of the dense path [row][kArgmaxParts]
     fl::DevBuf<int> am_idx;
     fl::PinnedBuf<uint32_t> h_ids;
-    fl::PinnedBuf<float> h_logits;
+    fl::HostBuf<float> h_logits;
     size_t trace_cap = 0;
     int amax_parts = 0;
     std::map<fl::GraphKey, fl::GraphEntry> graphs;

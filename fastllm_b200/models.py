@@ -87,16 +87,29 @@ class DeviceModel:
             pass
 
 
-class _Block:
-    """one page-locked piece of host memory under a result array; goes back to its pool when the last array over it is gone"""
+class _Memory:
+    """page-locked host memory, freed with the last reference"""
 
-    def __init__(self, pool, ptr, room, shape):
-        self.pool, self.ptr, self.room = pool, ptr, room
-        self.__array_interface__ = {"shape": shape, "typestr": "<f4", "data": (ptr, False), "version": 3}
+    def __init__(self, lib, ptr):
+        self.lib, self.ptr = lib, ptr
 
     def __del__(self):
         try:
-            self.pool.give_back(self.ptr, self.room)
+            self.lib.fl_host_free(C.c_void_p(self.ptr))
+        except Exception:
+            pass
+
+
+class _Block:
+    """one piece of page-locked memory under a result array; goes back to its pool when the last array over it is gone"""
+
+    def __init__(self, pool, piece, shape):
+        self.pool, self.piece = pool, piece
+        self.__array_interface__ = {"shape": shape, "typestr": "<f4", "data": (piece[0], False), "version": 3}
+
+    def __del__(self):
+        try:
+            self.pool.give_back(self.piece)
         except Exception:
             pass
 
@@ -104,72 +117,76 @@ class _Block:
 class _ResultPool:
     """Page-locked memory for a cache's results, which the device then writes by itself (64 x 32000 logits behind a 0.5 ms step: 1.1 -> 0.7 ms
     a call; into new pageable memory one thread copies them and takes a page fault for every 4 KB).  A caller who drops or overwrites a
-    result before asking for the one after the next needs two blocks; whoever keeps more gets plain arrays, and so does whoever asks for more
-    than MOST.  Page-locking takes 0.4 ms per MB: both blocks are taken with the cache, for one row per sequence, and a block that has become
-    too small is exchanged for one of at least twice its size.  Blocks are freed with the pool or, when an array outlives it, with that array.
-    Lists are only appended to and popped from (arrays may go in any thread, in the middle of a collection)."""
-    BLOCKS, LEAST, MOST = 2, 1 << 16, 64 << 20      # blocks; bytes below which a copy is as good; bytes of a block, at most
+    result before asking for the one after the next needs two pieces; whoever keeps more gets plain arrays, and so does whoever asks for more
+    than MOST.  Page-locking takes 0.5 to 1 ms, and 0.13 per MB: both pieces are taken at once with the cache, for one row per sequence, and a
+    piece that has become too small is exchanged for one of at least twice its size.  Memory is freed with the pool or, when an array
+    outlives it, with that array.  Lists are only appended to and popped from (arrays may go in any thread, in the middle of a collection)."""
+    PIECES, LEAST, MOST = 2, 1 << 16, 64 << 20      # pieces; bytes below which a copy is as good; bytes of a piece, at most
 
     def __init__(self, lib):
-        self.lib, self.free, self.tickets, self.closed = lib, [], [None] * self.BLOCKS, False
+        self.lib, self.free, self.tickets, self.closed = lib, [], [None] * self.PIECES, False       # free: (address, bytes, memory)
 
     def empty(self, shape) -> np.ndarray:
         room = 4 * shape[0] * shape[1]
-        if not self.LEAST <= room <= self.MOST:
-            return np.empty(shape, dtype=np.float32)
-        ptr, have = self.take(room)
-        if ptr is None:
-            return np.empty(shape, dtype=np.float32)
-        return np.asarray(_Block(self, ptr, have, tuple(shape)))
+        piece = self.take(room) if self.LEAST <= room <= self.MOST else None
+        return np.empty(shape, dtype=np.float32) if piece is None else np.asarray(_Block(self, piece, tuple(shape)))
 
     def take(self, room):
-        """-> (address, bytes) of a block with at least that room; (None, 0): there is none to be had"""
-        blocks = []
+        """-> a piece with at least that room, None: there is none to be had"""
+        pieces = []
         try:
             while True:
-                blocks.append(self.free.pop())
+                pieces.append(self.free.pop())
+                if len(pieces) == 1 and pieces[0][1] == room:       # (as nearly always: the same call again)
+                    return pieces[0]
         except IndexError:
             pass
-        blocks.sort(key=lambda b: b[1])
-        fits = [i for i, (_, have) in enumerate(blocks) if have >= room]
-        chosen = blocks.pop(fits[0]) if fits else (blocks.pop(0) if blocks else None)       # the smallest that fits, else the smallest
-        self.free.extend(blocks)
+        pieces.sort(key=lambda p: p[1])
+        fits = [i for i, p in enumerate(pieces) if p[1] >= room]
+        chosen = pieces.pop(fits[0] if fits else 0) if pieces else None         # the smallest that fits, else the smallest
+        self.free.extend(pieces)
         if fits:
             return chosen
         if chosen is not None:
-            self.drop(chosen[0])
             room = max(room, min(2 * chosen[1], self.MOST))
+            self.tickets.append(None)
+            del chosen, pieces                  # (its memory is freed before the new one is taken)
         try:
             self.tickets.pop()
         except IndexError:
-            return None, 0
-        p = C.c_void_p()
-        if self.lib.fl_host_alloc(room, C.byref(p)) != 0:
+            return None
+        memory = self.lock(room)
+        if memory is None:
             self.tickets.append(None)
-            return None, 0
-        return p.value, room
+            return None
+        return memory.ptr, room, memory
+
+    def lock(self, size):
+        p = C.c_void_p()
+        return _Memory(self.lib, p.value) if self.lib.fl_host_alloc(size, C.byref(p)) == 0 else None
 
     def reserve(self, shape):
-        arrays = [self.empty(shape) for _ in range(self.BLOCKS)]
-        del arrays                      # (their blocks are free again)
+        """the first pieces, before anything else is asked of the pool"""
+        room = 4 * shape[0] * shape[1]
+        if not self.LEAST <= room <= self.MOST:
+            return
+        step = (room + 4095) // 4096 * 4096
+        memory = self.lock(self.PIECES * step)
+        if memory is not None:
+            self.tickets.clear()
+            self.free.extend((memory.ptr + i * step, room, memory) for i in range(self.PIECES))
 
-    def drop(self, ptr):
-        self.lib.fl_host_free(C.c_void_p(ptr))
-        self.tickets.append(None)
-
-    def give_back(self, ptr, room):
-        self.free.append((ptr, room))
+    def give_back(self, piece):
         if self.closed:
-            self.close()
+            self.tickets.append(None)
+        else:
+            self.free.append(piece)
+            if self.closed:
+                self.close()
 
     def close(self):
         self.closed = True
-        while True:
-            try:
-                ptr, _ = self.free.pop()
-            except IndexError:
-                return
-            self.drop(ptr)
+        self.free.clear()
 
 
 class DeviceCache:

@@ -12,20 +12,21 @@ from oracle import synth
 from helpers import product_model
 
 pytestmark = pytest.mark.gpu
-VOCAB = 4096                # 8 rows: 128 KB, enough for a page-locked array
 
 
-def _cache():
+def _cache(vocab):
     from fastllm_b200 import models
-    cfg = ocl.CausalLMConfig("llama", 64, 96, VOCAB, 1, 4, 2, 1e-5, 1e4, 64)
+    cfg = ocl.CausalLMConfig("llama", 64, 96, vocab, 1, 4, 2, 1e-5, 1e4, 64)
     model = product_model(cfg, ocl.synth_weights(cfg, 0, 0.05))[0]
     return models.DeviceCache(model.dev, 8, 32)
 
 
-def test_a_forked_child_keeps_the_result_it_holds():
+# eight rows: 128 KB, enough for a page-locked array, and 1.25 MB, which lies in huge pages
+@pytest.mark.parametrize("vocab", [4096, 40000])
+def test_a_forked_child_keeps_the_result_it_holds(vocab):
     from fastllm_b200 import models
-    cache = _cache()
-    out = cache.forward(synth.token_ids(1, VOCAB, (8, 1)), 0)
+    cache = _cache(vocab)
+    out = cache.forward(synth.token_ids(1, vocab, (8, 1)), 0)
     assert isinstance(out.base, models._Block)                  # page-locked
     before, where = out.copy(), out.__array_interface__["data"][0]
     go, told = os.pipe()
@@ -36,8 +37,8 @@ def test_a_forked_child_keeps_the_result_it_holds():
         out[:] = -1.0       # and its writes are its own
         os._exit(0 if same else 3)
     del out
-    again = cache.forward(synth.token_ids(2, VOCAB, (8, 1)), 1)
-    others = cache.forward(synth.token_ids(3, VOCAB, (8, 1)), 2)
+    again = cache.forward(synth.token_ids(2, vocab, (8, 1)), 1)
+    others = cache.forward(synth.token_ids(3, vocab, (8, 1)), 2)
     reused = [a for a in (again, others) if a.__array_interface__["data"][0] == where]
     kept = [a.copy() for a in (again, others)]
     os.write(told, b"x")

@@ -87,13 +87,13 @@ def test_growing_calls_hardly_ever_page_lock():
     lib = CountingLib()
     pool = models._ResultPool(lib)
     pool.reserve((64, 8192))
-    assert lib.taken == [64 * 8192 * 4] * 2
+    assert lib.taken == [2 * 64 * 8192 * 4]                     # both pieces at once
     for b in range(1, 65):
         keep = pool.empty((b, 8192))                            # noqa: F841  (held until the next one is there, as by a program's loop)
-    assert len(lib.taken) == 2
+    assert len(lib.taken) == 1
     for rows in range(100, 301):
         keep = pool.empty((rows, 8192))                         # noqa: F841
-    assert len(lib.taken) <= 2 + 2 * 3 and len(lib.live) == 2
+    assert len(lib.taken) <= 1 + 2 * 3 and len(lib.live) == 2
 
 
 def test_a_block_that_fits_is_taken_before_one_is_exchanged():
@@ -116,3 +116,25 @@ def test_results_beyond_a_limit_are_plain():
     del a
     b = pool.empty((rows, 8192))                                # an exchanged block stays inside the limit
     assert at(b) in lib.live and max(lib.taken) == pool.MOST
+
+
+def test_pieces_of_one_memory():
+    """the pieces that are taken together do not overlap, and their memory goes with the last of them"""
+    lib = CountingLib()
+    pool = models._ResultPool(lib)
+    pool.reserve((5, 8191))
+    a, b = pool.empty((5, 8191)), pool.empty((5, 8191))
+    a[:], b[:] = 1.0, 2.0
+    assert abs(at(a) - at(b)) >= a.nbytes and (a == 1.0).all() and (b == 2.0).all() and len(lib.live) == 1
+    assert at(pool.empty((5, 8191))) not in (at(a), at(b))      # both are held
+    del a
+    c = pool.empty((50, 8191))                                  # the free piece is exchanged, the other one's memory stays
+    c[:] = 3.0
+    assert len(lib.live) == 2 and (b == 2.0).all()
+    pool.close()
+    del b
+    gc.collect()
+    assert len(lib.live) == 1 and (c == 3.0).all()
+    del c
+    gc.collect()
+    assert not lib.live
