@@ -468,10 +468,11 @@ void bert_embed(BertModel& m, const uint32_t* ids, const uint32_t* mask, int b, 
 // Device-resident repeat of the encoder on the ids already uploaded by the last bert_embed (benchmark `value`).
 void bert_repeat(BertModel& m, int b, int t, int iters, float* elapsed_ms) {
     std::lock_guard<std::mutex> lock(m.mu);
-    FL_CHECK((size_t)b * t <= m.cap_tokens, FL_ERR_STATE, "call fl_embed with this shape first");
+    const BertRun run = bert_run(m, b, t);
+    const size_t T = (size_t)b * t;
+    FL_CHECK(T <= m.cap_tokens && (size_t)b <= m.cap_batch && (run.path == BertPath::blocks || T <= m.cap_chain), FL_ERR_STATE, "call fl_embed with this shape first");
     EventPair ev;
     FL_CUDA(cudaEventRecord(ev.e0, m.stream));
-    const BertRun run = bert_run(m, b, t);
     for (int i = 0; i < iters; ++i) bert_enqueue(m, run, b, t, false);
     FL_CUDA(cudaEventRecord(ev.e1, m.stream));
     FL_CUDA(cudaStreamSynchronize(m.stream));

@@ -64,3 +64,9 @@ def test_nothing_is_taken_between_a_step_and_its_logits():
     assert ".alloc(" not in deliver and ".alloc(" not in sample
     assert "c.h_logits.alloc(" in source.split("static void cache_create(", 1)[1].split("\n}\n", 1)[0]
     assert "y.h_logits.alloc(" in (CSRC / "fl_layered.cu").read_text().split("static void ensure_ws(", 1)[1].split("\n}\n", 1)[0]
+
+
+def test_repeats_ask_for_every_buffer():
+    """an embedding in another thread may have failed to grow the workspace in between: a repeat looks at all three sizes"""
+    body = (CSRC / "fl_bert.cu").read_text().split("void bert_repeat(", 1)[1].split("\n}\n", 1)[0]
+    assert all(f"<= m.{cap}" in body for cap in ("cap_tokens", "cap_batch", "cap_chain"))
