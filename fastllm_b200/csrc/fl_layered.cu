@@ -7,6 +7,7 @@
 #include "layered_ops.cuh"
 #include "chunk_scan.cuh"
 #include "gemm_dec.cuh"
+#include "gemm_f64.cuh"
 #include "gqa_attn_tc.cuh"
 #include "model.cuh"
 #include "synth.cuh"
@@ -958,23 +959,19 @@ static void launch_ly_gemm(LaunchCtx& lc, const char* tag, const LyGemm& g, int 
         launch(lc, tag, bytes, ly_gemm_kernel, dim3((g.N + kLyBN - 1) / kLyBN, (max_rows + kLyBM - 1) / kLyBM, groups), dim3(256), 0, g);
         return;
     }
-    static bool attr_set = false;
-    if (!attr_set) {
-        FL_CUDA(cudaFuncSetAttribute(ly_gemm64_kernel<32, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ly_gemm64_smem<32, 32>()));
-        FL_CUDA(cudaFuncSetAttribute(ly_gemm64_kernel<8, 64>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)ly_gemm64_smem<8, 64>()));
-        attr_set = true;
-    }
-    // Few rows: a tile of 32 would mostly multiply nothing, tiles of 8 x 64 do a quarter of its work (up to eight rows; every further eight read the
-    // weights again) but are half as many.  One matrix whose 8 x 64 tiles nearly fill the chip takes them: whole decode step, 32 x 32 tiles
-    // everywhere -> 8 x 64 from 8000 columns on, 1 / 4 / 8 rows of width 1024: 835 / 859 / 923 -> 799 / 825 / 894 us, of width 4096: 4.54 / 4.58 / 4.68 ->
-    // 3.92 / 3.96 / 4.06 ms; from 4000 columns on: 838 / 871 / 932 us and 4.78 / 4.83 / 4.94 ms.  Experts of few rows each: 8 of 5632, width 2048,
-    // 4 / 8 / 16 rows (8 / 16 / 32 picks) 3.02 / 3.29 / 3.50 -> 2.55 / 2.80 / 2.94 ms, but 1 row 2.02 -> 2.14 and 48 rows 3.61 -> 4.09 (of 2816, width
-    // 1024: 1.08 / 1.24 / 1.36 -> 1.11 / 1.26 / 1.39).
-    const bool small_tiles = groups > 1 ? max_rows >= 8 && max_rows <= 32 : max_rows <= 8 && 6 * ((g.N + 63) / 64) >= 5 * kNumSMs;
-    if (small_tiles)
-        launch(lc, tag, bytes, ly_gemm64_kernel<8, 64>, dim3((g.N + 63) / 64, (max_rows + 7) / 8, groups), dim3(256), ly_gemm64_smem<8, 64>(), g);
-    else
-        launch(lc, tag, bytes, ly_gemm64_kernel<32, 32>, dim3((g.N + 31) / 32, (max_rows + 31) / 32, groups), dim3(256), ly_gemm64_smem<32, 32>(), g);
+    auto go = [&](auto rows_per_tile) {
+        constexpr int BM = decltype(rows_per_tile)::value;
+        static bool attr_set = false;
+        if (!attr_set) {
+            FL_CUDA(cudaFuncSetAttribute(ly_gemm64_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, F64Form<BM>::kSmem));
+            attr_set = true;
+        }
+        launch(lc, tag, bytes, ly_gemm64_kernel<BM>, dim3((g.N + kF64BN - 1) / kF64BN, (max_rows + BM - 1) / BM, groups), dim3(32 * kF64Sums), F64Form<BM>::kSmem, g);
+    };
+    // (experts share max_rows picks between them)
+    const bool known = g.grp_off == nullptr;
+    if (f64_rows_per_tile(known ? max_rows : (double)max_rows / groups, g.N, groups, known) == 16) go(std::integral_constant<int, 16>{});
+    else go(std::integral_constant<int, 8>{});
 }
 static void gemm(LaunchCtx& lc, const char* tag, const float* A, int lda, const uint16_t* Wt, int N, int K, float* Y, int ldy, int R) {
     if (R <= 0) return;

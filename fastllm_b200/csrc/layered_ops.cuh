@@ -531,137 +531,6 @@ static __global__ void __launch_bounds__(256) ly_gemm_kernel(LyGemm g) {
     }
 }
 
-// The exact mode: f64 accumulators, every output is the correctly rounded f32 of its dot product, whatever K.
-// A block of eight warps owns BM x BN outputs; of every 64 columns of K a warp multiplies eight on the f64 tensor pipe (mma.m8n8k4), and the
-// warps' sums meet in warp order at the end -- an order that depends on K alone, so a row's result is bitwise the same whatever rows stand
-// beside it and whichever BM was taken.  Operands are widened once, on their way into shared memory; a row of 68 doubles puts the four rows
-// of a half-warp's fragment on different banks.
-// Bound: the f64 pipe (64 FMA per clock and SM).  One thread per 4 x 4 outputs of a 64 x 64 tile, widening its operands at every use, left
-// half of the chip without a block; 4 x 4 outputs per thread over widened operands are bound by shared memory (16-byte loads of f64: ncu had
-// it at 83 %, the f64 pipe at 22 %).  203 x 1024 x 2816: 310 -> 83 us (33 at the pipe's rate); 203 x 5632 x 1024: 283 -> 134 us (65);
-// whole decode step of one row, width 1024, vocabulary 32000: 2.48 -> 0.80 ms.  Results bit-identical.
-__device__ __forceinline__ void mma_f64_884(double (&d)[2], double a, double b) {
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
-}
-template <int BM, int BN>
-static __global__ void __launch_bounds__(256, 2) ly_gemm64_kernel(LyGemm g) {
-    pdl_chain();
-    constexpr int KT = 64, LD = KT + 4, STAGE = (BM + BN) * LD, MT = BM / 8, NT = BN / 8;
-    constexpr int PA = BM * KT / 4, PW = BN * KT / 4, NA = (PA + 255) / 256, NWT = (PW + 255) / 256;      // 4-element pieces per stage / per thread
-    extern __shared__ __align__(16) double sm64[];           // two stages of [BM][LD] | [BN][LD], then the warps' sums
-    const int grp = blockIdx.z;
-    int p_lo = 0, p_hi = g.R;
-    if (g.grp_off != nullptr) { p_lo = g.grp_off[grp]; p_hi = g.grp_off[grp + 1]; }
-    const int p0 = p_lo + blockIdx.y * BM;
-    if (p0 >= p_hi) return;
-    const int n0 = blockIdx.x * BN, tid = threadIdx.x, w = tid >> 5, lane = tid & 31;
-    const float* A = g.A + (size_t)grp * g.a_gs;
-    const uint16_t* Wm = g.W + (size_t)grp * g.w_gs;
-    float* Y = g.Y + (size_t)grp * g.y_gs;
-    const bool va = ((g.K | g.lda) & 3) == 0 && (reinterpret_cast<uintptr_t>(A) & 15) == 0, vw = (g.K & 3) == 0 && (reinterpret_cast<uintptr_t>(Wm) & 7) == 0;
-    // piece i of a stage: row i / 16, columns 4 (i % 16) ..
-    const float* arow[NA];
-    const uint16_t* wrow[NWT];
-    const int kq = tid % 16 * 4;
-#pragma unroll
-    for (int t = 0; t < NA; ++t) {
-        const int i = tid + t * 256, ap = p0 + i / 16;
-        arow[t] = ap < p_hi && i < PA ? A + (size_t)(g.a_idx ? g.a_idx[ap] : ap) * g.lda : nullptr;
-    }
-#pragma unroll
-    for (int t = 0; t < NWT; ++t) {
-        const int i = tid + t * 256, n = n0 + i / 16;
-        wrow[t] = n < g.N && i < PW ? Wm + (size_t)n * g.K : nullptr;
-    }
-    float4 ra[NA];
-    ushort4 rw[NWT];
-    auto fetch = [&](int k) {
-        k += kq;
-#pragma unroll
-        for (int t = 0; t < NA; ++t) {
-            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (arow[t] != nullptr) {
-                if (va) { if (k < g.K) v = *reinterpret_cast<const float4*>(arow[t] + k); }
-                else {
-                    if (k < g.K) v.x = arow[t][k];
-                    if (k + 1 < g.K) v.y = arow[t][k + 1];
-                    if (k + 2 < g.K) v.z = arow[t][k + 2];
-                    if (k + 3 < g.K) v.w = arow[t][k + 3];
-                }
-            }
-            ra[t] = v;
-        }
-#pragma unroll
-        for (int t = 0; t < NWT; ++t) {
-            ushort4 v = make_ushort4(0, 0, 0, 0);
-            if (wrow[t] != nullptr) {
-                if (vw) { if (k < g.K) v = *reinterpret_cast<const ushort4*>(wrow[t] + k); }
-                else {
-                    if (k < g.K) v.x = wrow[t][k];
-                    if (k + 1 < g.K) v.y = wrow[t][k + 1];
-                    if (k + 2 < g.K) v.z = wrow[t][k + 2];
-                    if (k + 3 < g.K) v.w = wrow[t][k + 3];
-                }
-            }
-            rw[t] = v;
-        }
-    };
-    auto wide = [](uint16_t b) { return (double)__uint_as_float((uint32_t)b << 16); };
-    auto stage = [&](double* s) {
-#pragma unroll
-        for (int t = 0; t < NA; ++t) {
-            const int i = tid + t * 256;
-            double2* d = reinterpret_cast<double2*>(s + i / 16 * LD + kq);
-            if (i < PA) { d[0] = make_double2(ra[t].x, ra[t].y); d[1] = make_double2(ra[t].z, ra[t].w); }
-        }
-#pragma unroll
-        for (int t = 0; t < NWT; ++t) {
-            const int i = tid + t * 256;
-            double2* d = reinterpret_cast<double2*>(s + (BM + i / 16) * LD + kq);
-            if (i < PW) { d[0] = make_double2(wide(rw[t].x), wide(rw[t].y)); d[1] = make_double2(wide(rw[t].z), wide(rw[t].w)); }
-        }
-    };
-    double acc[MT][NT][2] = {};
-    fetch(0);
-    int b = 0;
-    for (int k0 = 0; k0 < g.K; k0 += KT, b ^= 1) {
-        double* s = sm64 + b * STAGE;
-        stage(s);
-        __syncthreads();            // (the other stage was last read before the previous barrier)
-        if (k0 + KT < g.K) fetch(k0 + KT);
-        const double *sa = s + (lane >> 2) * LD + w * 8 + (lane & 3), *sw = sa + BM * LD;
-#pragma unroll
-        for (int kk = 0; kk < 8; kk += 4) {
-            double av[MT], bv[NT];
-#pragma unroll
-            for (int i = 0; i < MT; ++i) av[i] = sa[i * 8 * LD + kk];
-#pragma unroll
-            for (int j = 0; j < NT; ++j) bv[j] = sw[j * 8 * LD + kk];
-#pragma unroll
-            for (int i = 0; i < MT; ++i)
-#pragma unroll
-                for (int j = 0; j < NT; ++j) mma_f64_884(acc[i][j], av[i], bv[j]);
-        }
-    }
-    __syncthreads();
-    double* part = sm64 + (size_t)w * BM * BN + (lane >> 2) * BN + (lane & 3) * 2;
-#pragma unroll
-    for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int j = 0; j < NT; ++j) *reinterpret_cast<double2*>(part + i * 8 * BN + j * 8) = make_double2(acc[i][j][0], acc[i][j][1]);
-    __syncthreads();
-    for (int o = tid; o < BM * BN; o += 256) {
-        const int p = p0 + o / BN, n = n0 + o % BN;
-        if (p >= p_hi || n >= g.N) continue;
-        double t = 0.0;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) t += sm64[(size_t)q * BM * BN + o];
-        Y[(size_t)p * g.ldy + n] = (float)t;
-    }
-}
-template <int BM, int BN>
-constexpr size_t ly_gemm64_smem() { return std::max<size_t>((size_t)2 * 68 * (BM + BN), (size_t)8 * BM * BN) * 8; }
-
 // ---- gated linear attention ------------------------------------------------------------------------------------------------
 struct GlaArgs {
     const float* proj; int ldp, off_q, off_k, off_v;

@@ -176,6 +176,18 @@ def test_exact_gemm_rows_stand_alone(width, ff):
     assert np.array_equal(whole, R.run_cut(model, toks, [1, 8, 9, 16, 17, 32, 2], cache=model.new_device_cache(2, 128)))
 
 
+@pytest.mark.parametrize("width,ff", [(1032, 1544), (1028, 770), (550, 2050)])
+def test_exact_gemm_long_sums(width, ff):
+    """sums of more chunks than a warp keeps on their way (above 512 columns), the last chunk a half or less, rows aligned for 16-byte copies or not;
+    tiles of 8 and of 16 rows"""
+    cfg = R.config([R.delta(heads=4, kv_heads=2, dim=6, vdim=10, mlp=R.dense(ff=ff))], vocab=101, width=width)
+    oracle, model = R.build(cfg, seed=73)
+    toks = R.tokens(cfg, 48, seed=74)
+    whole = R.run_whole(model, toks, cache=model.new_device_cache(2, 64))
+    assert R.relerr(whole, oracle.run(toks)) < R.TOL["f32"]
+    assert np.array_equal(whole, R.run_cut(model, toks, [1, 8, 16, 17, 6], cache=model.new_device_cache(2, 64)))
+
+
 @pytest.mark.parametrize("width,ff", [(64, 72), (50, 34)])
 def test_exact_expert_rows_stand_alone(width, ff):
     """the same for experts: 2, 8, 10, 16, 32, 34 and 128 picks in a step"""
