@@ -5,12 +5,12 @@
 // Two CTAs of a cluster take 256 tokens (tcgen05.mma.cta_group::2, see gemm_pair.cuh): each holds its 128 rows of ctx, then x1, in shared memory
 // and half of every weight tile.  The 1536-wide activations exist 128 columns at a time: S (128 TMEM columns) -> GELU -> shared memory -> O (384
 // columns).  The tensor core alternates between the next columns' S and the last columns' O while the epilogue warps turn S into operands.
-// As five launches every layer moved 100 to 200 MB of activations between kernels that each waited for HBM and for their epilogues' stores
-// (256 x 128 tokens, whole encoder: 1.76 ms; 1.35 in this form).  256 tokens take 56 us (74 -> 75 tiles, a second wave in each of six layers: 702 ->
-// 1036 us), of which the products are 22 (1.6 us per 128 intermediate columns, measured by themselves, 2.4 for the output projection) and the two norms 5
-// in front and 6 behind.  The rest, 3.4 us per 128 columns instead of 1.6, is the chain from S to the next operand that the products wait for: load,
-// GELU (1.0 us, the tanh unit), store, fence, release (0.25).  Tensor pipe 33 %, issue slots 21 %, DRAM 5 % at one wave.  8 epilogue warps: 16 were no
-// faster.
+// As five launches every layer moved 100 to 200 MB of activations between kernels that each waited for HBM and for their epilogues' stores.  256 tokens
+// take 51 us, of which the products are 22 (1.6 us per 128 intermediate columns, measured by themselves, 2.4 for the output projection).  The rest is the
+// chain from S to the next operand that the products wait for (2.3 us per 128 columns instead of 1.6: load, GELU (1.0 us, the tanh unit), store, fence,
+// release (0.25)), the two norms, and the first loads.  Beside 225 KB of shared memory an SM has a few KB of L1: the norms' parameters are brought into the
+// operand's place, which is free while they run, and the residual comes 128 bytes of a row per eight lanes; read through L1 by every thread for its own
+// row both took 9 us more (256 x 128 tokens: 112 -> 102 us a layer).  8 epilogue warps: 16 were no faster.
 #pragma once
 #include "gemm_pair.cuh"
 
@@ -44,7 +44,7 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
     uint8_t* sX = gsm_raw + ((1024u - (smem_u32(gsm_raw) & 1023u)) & 1023u);
     uint8_t* sH = sX + kBbX;
     uint8_t* sW = sH + kBbHid;
-    __shared__ __align__(8) uint64_t w_full[kBbStages], w_empty[kBbStages], a_full, x_ready, x_free, s_full, s_free, h_ready, h_free, o_full;
+    __shared__ __align__(8) uint64_t w_full[kBbStages], w_empty[kBbStages], a_full[kBbKb / 2], x_ready, x_free, s_full, s_free, h_ready, h_free, o_full;
     __shared__ uint32_t tmem_base_s;
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
@@ -53,7 +53,7 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < kBbStages; ++s) { mbar_init(&w_full[s], 1); mbar_init(&w_empty[s], 1); }
-        mbar_init(&a_full, 1);
+        for (int k = 0; k < kBbKb / 2; ++k) mbar_init(&a_full[k], 1);
         mbar_init(&x_ready, 2 * kBbEpiWarps);
         mbar_init(&x_free, 1);
         mbar_init(&s_full, 1);
@@ -104,9 +104,10 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
                     asm volatile("fence.proxy.async;" ::: "memory");
                 }
                 if (it > 0 && !(ok = pair_wait(&x_free, (it - 1) & 1))) break;
-                if (rank == 0) mbar_expect_tx(&a_full, 2 * kBbX);
-                const uint32_t bar = mapa_u32(smem_u32(&a_full), 0);
-                for (int k = 0; k < kBbKb; ++k) tma_load_2d_pair(smem_u32(sX) + k * 16384, &tmC, k * 64, tile * 256 + (int)rank * 128, bar);
+                for (int k = 0; k < kBbKb; ++k) {       // (the products start with the first two blocks)
+                    if (rank == 0 && k % 2 == 0) mbar_expect_tx(&a_full[k / 2], 4 * 16384);
+                    tma_load_2d_pair(smem_u32(sX) + k * 16384, &tmC, k * 64, tile * 256 + (int)rank * 128, mapa_u32(smem_u32(&a_full[k / 2]), 0));
+                }
                 for (; first < kBbKb; ++first) stage(0, 0, first);
                 for (int j = 0; j <= kBbChunks; ++j) {
                     if (j < kBbChunks) { stage(1, j, 0); stage(1, j, 1); }
@@ -139,8 +140,10 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
             uint32_t chunk = 0;                     // over all tiles
             int it = 0;
             for (int tile = cl; tile < tiles; tile += G, ++it) {
-                wait(&a_full, it & 1);
-                for (int k = 0; k < kBbKb; ++k) out(dX + (uint64_t)(k * 1024), k ? 1u : 0u);
+                for (int k = 0; k < kBbKb; ++k) {
+                    if (k % 2 == 0) wait(&a_full[k / 2], it & 1);
+                    out(dX + (uint64_t)(k * 1024), k ? 1u : 0u);
+                }
                 umma_commit_pair_warp(&o_full);
                 wait(&x_ready, it & 1);
                 for (int j = 0; j <= kBbChunks; ++j) {
@@ -174,7 +177,9 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
         const int q = warp & 3, cs = (warp - 2) >> 2, lrow = q * 32 + lane;      // row of the CTA; slice of the columns
         constexpr int kOC = kBbH / kBbSlices, kSC = 128 / kBbSlices;              // columns of O and of S per warp
         const uint32_t lane_at = (uint32_t)(q * 32) << 16;
-        float2* part = reinterpret_cast<float2*>(sH);                             // [slice][128] row sums (the operand is not there yet, or done with)
+        // while the norms run the operand is not there yet, or done with: [slice][128] row sums; bias | weight | bias of the norm
+        float2* part = reinterpret_cast<float2*>(sH);
+        float* par = reinterpret_cast<float*>(sH + kBbSlices * 128 * 8);
         auto esync = [] { asm volatile("bar.sync 1, %0;" ::"n"(32 * kBbEpiWarps) : "memory"); };
         auto wait = [&](uint64_t* bar, uint32_t parity) { if (ok) ok = __all_sync(0xFFFFFFFFu, pair_wait(bar, parity)); tc_fence_after(); };
         // Arrives on the first CTA's barriers.  Operands in shared memory are released at the scope that the first CTA's products need: its own warps
@@ -189,18 +194,38 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
         auto free_s = [&] { __syncwarp(); if (lane == 0) mbar_arrive_cluster_relaxed(mapa_u32(smem_u32(&s_free), 0)); };
         // 16-byte chunk c of the row inside a tile of 64-column blocks
         auto at = [&](int c) { return (uint32_t)(c >> 3) * 16384u + (uint32_t)lrow * 128u + (uint32_t)(((c & 7) ^ (lrow & 7)) << 4); };
-        // this thread's columns of O: + bias + add(32-column step), kept in TMEM; -> mean and 1 / deviation of the row
-        auto row_sums = [&](const float* bias, auto add, float& mean, float& inv) {
+        // a norm's parameters, 288 pieces of 16 bytes: on their way, and into shared memory once the operand's place is free
+        const int pi = threadIdx.x - 64;
+        auto request = [&](const float* b, const float* w, const float* lb, float4 (&v)[2]) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int i = pi + k * 32 * kBbEpiWarps;
+                if (i < 3 * (kBbH / 4)) v[k] = __ldg(reinterpret_cast<const float4*>(i < kBbH / 4 ? b : i < kBbH / 2 ? w : lb) + i % (kBbH / 4));
+            }
+        };
+        auto put = [&](const float4 (&v)[2]) {
+#pragma unroll
+            for (int k = 0; k < 2; ++k) {
+                const int i = pi + k * 32 * kBbEpiWarps;
+                if (i < 3 * (kBbH / 4)) reinterpret_cast<float4*>(par)[i] = v[k];
+            }
+        };
+        // this thread's columns of O: + bias + the row of sX, kept in TMEM; -> mean and 1 / deviation of the row
+        auto row_sums = [&](float& mean, float& inv) {
             float s = 0.f, s2 = 0.f;
 #pragma unroll
             for (int i = 0; i < kOC / 32; ++i) {
                 const int c = cs * kOC + 32 * i;
                 uint32_t v[32], r[16];
+#pragma unroll
+                for (int k = 0; k < 4; ++k) {
+                    const uint4 z = *reinterpret_cast<const uint4*>(sX + at(c / 8 + k));
+                    r[4 * k] = z.x; r[4 * k + 1] = z.y; r[4 * k + 2] = z.z; r[4 * k + 3] = z.w;
+                }
                 tmem_ld32(tmem + lane_at + (uint32_t)c, v);
-                add(i, r);
 #pragma unroll
                 for (int j = 0; j < 32; j += 4) {
-                    const float4 b = __ldg(reinterpret_cast<const float4*>(bias + c + j));
+                    const float4 b = *reinterpret_cast<const float4*>(par + c + j);
                     const float y[4] = {__uint_as_float(v[j]) + b.x + bf16lo(r[j >> 1]), __uint_as_float(v[j + 1]) + b.y + bf16hi(r[j >> 1]),
                                         __uint_as_float(v[j + 2]) + b.z + bf16lo(r[(j >> 1) + 1]), __uint_as_float(v[j + 3]) + b.w + bf16hi(r[(j >> 1) + 1])};
 #pragma unroll
@@ -217,43 +242,49 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
             inv = 1.f / sqrtf(s2 / (float)kBbH - mean * mean + g.eps);
         };
         // 32 normalised columns as bf16 pairs
-        auto normed = [&](int c, const float* lw, const float* lb, float mean, float inv, uint32_t (&o)[16]) {
+        auto normed = [&](int c, float mean, float inv, uint32_t (&o)[16]) {
             uint32_t v[32];
             tmem_ld32(tmem + lane_at + (uint32_t)c, v);
 #pragma unroll
             for (int j = 0; j < 32; j += 4) {
-                const float4 w = __ldg(reinterpret_cast<const float4*>(lw + c + j)), b = __ldg(reinterpret_cast<const float4*>(lb + c + j));
+                const float4 w = *reinterpret_cast<const float4*>(par + kBbH + c + j), b = *reinterpret_cast<const float4*>(par + 2 * kBbH + c + j);
                 o[j >> 1] = pack_bf16x2((__uint_as_float(v[j]) - mean) * inv * w.x + b.x, (__uint_as_float(v[j + 1]) - mean) * inv * w.y + b.y);
                 o[(j >> 1) + 1] = pack_bf16x2((__uint_as_float(v[j + 2]) - mean) * inv * w.z + b.z, (__uint_as_float(v[j + 3]) - mean) * inv * w.w + b.w);
             }
         };
-        // the parameters into L1, where the epilogues find them (384 and 1536 floats: lines of 32)
-        for (int i = threadIdx.x - 64; i < 6 * 12 + 48; i += 32 * kBbEpiWarps) {
-            const float* const v[6] = {g.bo, g.ln1w, g.ln1b, g.b2, g.ln2w, g.ln2b};
-            const float* p = i < 48 ? g.b1 + 32 * i : nullptr;
-#pragma unroll
-            for (int k = 0; k < 6; ++k)
-                if (i >= 48 + 12 * k && i < 60 + 12 * k) p = v[k] + 32 * (i - 48 - 12 * k);
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(p));
-        }
+        if (pi < kBbI / 32) asm volatile("prefetch.global.L1 [%0];" ::"l"(g.b1 + 32 * pi));
+        float4 p1[2], p2[2];
+        request(g.bo, g.ln1w, g.ln1b, p1);
         pdl_wait();
         uint32_t chunk = 0, of = 0;
         for (int tile = cl; tile < tiles; tile += G) {            // (to the end even behind a wait that ran out: the warps meet at barriers)
-            const int row = tile * 256 + (int)rank * 128 + lrow;
-            const uint16_t* xr = g.x + (size_t)row * kBbH;
+            // The residual, on its way while the first products run: this warp's 32 rows and half of the columns, 128 bytes of a row per eight lanes (thread ==
+            // row would take 32 lines a load), into the places of sX that the warp itself fills with x1.
+            const int row0 = tile * 256 + (int)rank * 128;
             float mean, inv;
-            uint4 res[kOC / 8];                                        // the residual's columns, on their way while the first products run
+            uint4 res[kOC / 8];
+            auto place = [&](int k, int& r) { r = q * 32 + k % 8 * 4 + (lane >> 3); return (uint32_t)(cs * (kOC / 64) + k / 8) * 16384u + (uint32_t)r * 128u + (uint32_t)(((lane & 7) ^ (r & 7)) << 4); };
 #pragma unroll
-            for (int k = 0; k < kOC / 8; ++k) res[k] = row < g.T ? *reinterpret_cast<const uint4*>(xr + cs * kOC + 8 * k) : make_uint4(0u, 0u, 0u, 0u);
+            for (int k = 0; k < kOC / 8; ++k) {
+                int r;
+                place(k, r);
+                res[k] = row0 + r < g.T ? *reinterpret_cast<const uint4*>(g.x + (size_t)(row0 + r) * kBbH + cs * kOC + k / 8 * 64 + (lane & 7) * 8) : make_uint4(0u, 0u, 0u, 0u);
+            }
+            put(p1);
+            request(g.b2, g.ln2w, g.ln2b, p2);
             wait(&o_full, of++ & 1);
-            row_sums(g.bo, [&](int i, uint32_t (&r)[16]) {
 #pragma unroll
-                for (int k = 0; k < 4; ++k) { const uint4 z = res[4 * i + k]; r[4 * k] = z.x; r[4 * k + 1] = z.y; r[4 * k + 2] = z.z; r[4 * k + 3] = z.w; }
-            }, mean, inv);
+            for (int k = 0; k < kOC / 8; ++k) {
+                int r;
+                const uint32_t to = place(k, r);
+                *reinterpret_cast<uint4*>(sX + to) = res[k];
+            }
+            esync();
+            row_sums(mean, inv);
 #pragma unroll 1
             for (int c = cs * kOC; c < cs * kOC + kOC; c += 32) {
                 uint32_t o[16];
-                normed(c, g.ln1w, g.ln1b, mean, inv, o);
+                normed(c, mean, inv, o);                          // (over the residual's values that this thread alone reads)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(sX + at(c / 8 + k)) = make_uint4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
             }
@@ -280,17 +311,14 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
                 arrive(&h_ready);
             }
             wait(&o_full, of++ & 1);
-            row_sums(g.b2, [&](int i, uint32_t (&r)[16]) {
-#pragma unroll
-                for (int k = 0; k < 4; ++k) {
-                    const uint4 z = *reinterpret_cast<const uint4*>(sX + at(cs * (kOC / 8) + 4 * i + k));
-                    r[4 * k] = z.x; r[4 * k + 1] = z.y; r[4 * k + 2] = z.z; r[4 * k + 3] = z.w;
-                }
-            }, mean, inv);
+            put(p2);
+            request(g.bo, g.ln1w, g.ln1b, p1);
+            esync();
+            row_sums(mean, inv);
 #pragma unroll 1
             for (int c = cs * kOC; c < cs * kOC + kOC; c += 32) {
                 uint32_t o[16];
-                normed(c, g.ln2w, g.ln2b, mean, inv, o);          // (over the x1 values that this thread alone reads)
+                normed(c, mean, inv, o);          // (over the x1 values that this thread alone reads)
 #pragma unroll
                 for (int k = 0; k < 4; ++k) *reinterpret_cast<uint4*>(sX + at(c / 8 + k)) = make_uint4(o[4 * k], o[4 * k + 1], o[4 * k + 2], o[4 * k + 3]);
             }
@@ -298,7 +326,6 @@ bert_block_kernel(const __grid_constant__ CUtensorMap tmC, const __grid_constant
             tc_fence_before();
             esync();
             if (threadIdx.x == 64) {
-                const int row0 = tile * 256 + (int)rank * 128;
                 for (int k = 0; ok && row0 < g.T && k < kBbKb; ++k) tma_store_2d(&tmX, sX + k * 16384, k * 64, row0);
                 asm volatile("cp.async.bulk.commit_group;" ::: "memory");
                 asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
