@@ -17,7 +17,7 @@ struct BertLayerW {
     float *bqkv = nullptr, *bo = nullptr, *bi = nullptr, *bo2 = nullptr;
     float *ln1w = nullptr, *ln1b = nullptr, *ln2w = nullptr, *ln2b = nullptr;
     CUtensorMap tm_wqkv, tm_wo, tm_wi, tm_wo2;
-    CUtensorMap tb_wo, tb_wi, tb_wo2;       // the boxes of bert_block_kernel
+    CUtensorMap tb_wqkv, tb_wo, tb_wi, tb_wo2;       // the boxes of bert_qkv_attn_kernel and bert_block_kernel
 };
 
 struct BertModel {

@@ -5,6 +5,7 @@
 
 #include "bert.cuh"
 #include "bert_block.cuh"
+#include "bert_qkv.cuh"
 #include "bert_small.cuh"
 #include "bert_model.cuh"
 #include "grow.hpp"
@@ -271,6 +272,7 @@ void bert_finalize(BertModel& m) {
         w.tm_wo = make_tmap_bf16(w.wo, m.H, m.H, m.H, kBertBN);
         w.tm_wi = make_tmap_bf16(w.wi, m.I, m.H, m.H, kBertBN);
         w.tm_wo2 = make_tmap_bf16(w.wo2, m.H, m.I, m.I, kBertBN);
+        w.tb_wqkv = make_tmap_bf16(w.wqkv, 3 * m.H, m.H, m.H, kBqCols / 2);
         w.tb_wo = make_tmap_bf16(w.wo, m.H, m.H, m.H, 96);
         w.tb_wi = make_tmap_bf16(w.wi, m.I, m.H, m.H, 64);
         w.tb_wo2 = make_tmap_bf16(w.wo2, m.H, m.I, m.I, 96);
@@ -283,21 +285,29 @@ void bert_finalize(BertModel& m) {
     m.finalized = true;
 }
 
-static int bert_block_clusters() {       // pairs of SMs that can be resident at once (the driver's answer)
-    static const int n = [] {
-        if (cudaFuncSetAttribute(bert_block_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kBbSmem) != cudaSuccess) { cudaGetLastError(); return 0; }
-        cudaLaunchConfig_t cfg{};
-        cfg.gridDim = dim3(kNumSMs); cfg.blockDim = dim3(kBbThreads); cfg.dynamicSmemBytes = kBbSmem;
-        cudaLaunchAttribute at[1];
-        at[0].id = cudaLaunchAttributeClusterDimension;
-        at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
-        cfg.attrs = at; cfg.numAttrs = 1;
-        int k = 0;
-        if (cudaOccupancyMaxActiveClusters(&k, bert_block_kernel, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
-        return std::min(k, kNumSMs / 2);
-    }();
+// pairs of SMs that can be resident at once (the driver's answer)
+template <typename K>
+static int pairs_resident(K kern, int threads, size_t smem) {
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess) { cudaGetLastError(); return 0; }
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3(kNumSMs); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 2; at[0].val.clusterDim.y = 1; at[0].val.clusterDim.z = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    int k = 0;
+    if (cudaOccupancyMaxActiveClusters(&k, kern, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+    return std::min(k, kNumSMs / 2);
+}
+static int bert_block_clusters() {
+    static const int n = pairs_resident(bert_block_kernel, kBbThreads, kBbSmem);
     return n;
 }
+static int bert_qkv_clusters() {
+    static const int n = pairs_resident(bert_qkv_attn_kernel, kBqThreads, kBqSmem);
+    return n;
+}
+static bool bert_qkv_attn(const BertModel& m, int t) { return m.H == kBbH && m.nh == kBsHeads && t <= kBertS && bert_qkv_clusters() > 0; }
 // A pair of SMs takes about as long for 256 tokens however many tiles there are, the chain's kernels grow with the tokens, in steps of their own waves.
 // Whole encoder, chain -> blocks, us, by tiles of 256 tokens (128-token sentences; 64 and 512 tokens a sentence cross at the same places): 28 506 -> 506,
 // 32 526 -> 522, 36 544 -> 532, 38 658 -> 550, 44 688 -> 576, 64 853 -> 674, 74 914 -> 702; two waves: 75 1034 -> 1036, 80 1070 -> 1058,
@@ -384,6 +394,19 @@ static void launch_bert_block(BertModel& m, const CUtensorMap& tm_ctx, const CUt
     const BertBlockArgs a{T, m.x.p, w.bo, w.bi, w.bo2, w.ln1w, w.ln1b, w.ln2w, w.ln2b, eps, m.failed.p};
     blaunch(m.stream, bert_block_kernel, dim3(2 * std::min((T + 255) / 256, bert_block_clusters())), dim3(kBbThreads), kBbSmem, tm_ctx, w.tb_wo, w.tb_wi, w.tb_wo2, tm_x, a);
 }
+// Heads per unit: units go round the resident pairs in whole numbers, and one costs about 0.7 of a head whatever its heads (37 x 127 tokens: 19 pairs, 76
+// units of three heads for 74 clusters 449 us, 114 of two 430; 256 x 128: three; 4 x 128: one, 307 -> 302).
+static void launch_bert_qkv(BertModel& m, const CUtensorMap& tm_x, const BertLayerW& w, int b, int t, float scale) {
+    const int spc = kBertS / t, pairs = ((b + spc - 1) / spc + 1) / 2, G = bert_qkv_clusters();
+    int hpu = kBqHeads;
+    double best = 1e30;
+    for (int h = kBqHeads; h >= 1; --h) {
+        const double cost = ((pairs * (kBqAllHeads / h) + G - 1) / G) * (0.7 + h);
+        if (cost < best) { best = cost; hpu = h; }
+    }
+    const BertQkvArgs a{b, t, spc, hpu, w.bqkv, 1.4426950408889634f / scale, m.ctx.p, m.failed.p};
+    blaunch(m.stream, bert_qkv_attn_kernel, dim3(2 * std::min(pairs * (kBqAllHeads / hpu), G)), dim3(kBqThreads), kBqSmem, tm_x, w.tb_wqkv, a);
+}
 static void bert_check(const BertModel& m) {
     FL_CHECK(*m.failed.p == 0, FL_ERR_CUDA, "a wait inside a kernel ran out, the results are not valid");
 }
@@ -400,7 +423,7 @@ static void bert_enqueue(BertModel& m, const BertRun& run, int b, int t, bool ha
     const dim3 row_grid((T + rows_per_cta - 1) / rows_per_cta), row_block(rows_per_cta * 32);
     blaunch(st, embed_ln_kernel, row_grid, row_block, 0, (const uint16_t*)m.wemb, (const uint16_t*)m.pemb, (const float*)m.lnw, (const float*)m.lnb,
             (const uint32_t*)m.ids.p, T, t, H, m.V, m.maxpos, 1e-12f, m.x.p);
-    const bool blocks = run.path == BertPath::blocks;
+    const bool blocks = run.path == BertPath::blocks, qkv_attn = bert_qkv_attn(m, t);
     const CUtensorMap tm_x = make_tmap_bf16(m.x.p, T, H, H, kGemmBM), tm_x1 = blocks ? tm_x : make_tmap_bf16(m.x1.p, T, H, H, kGemmBM),
                       tm_ctx = make_tmap_bf16(m.ctx.p, T, H, H, kGemmBM);
     const CUtensorMap tm_h = blocks ? tm_x : make_tmap_bf16(m.hbuf.p, T, I, I, kGemmBM);
@@ -408,13 +431,17 @@ static void bert_enqueue(BertModel& m, const BertRun& run, int b, int t, bool ha
     const float scale = (float)std::sqrt((double)m.d);
     for (int l = 0; l < m.L; ++l) {
         const BertLayerW& w = m.layers[l];
-        // B2: fused q|k|v projection + bias -> bf16 [T, 3H]
-        launch_gemm<GEPI_BIAS_BF16>(st, tm_x, w.tm_wqkv, GemmArgs{T, 3 * H, H, w.bqkv, nullptr, 0, m.qkv.p, 3 * H, 1, 0});
-        // B3+B4: per (sentence, head) softmax(QK^T / sqrt(d)) V, no mask
-        if (t <= kBertS)
-            blaunch(st, bert_attn_kernel, dim3(m.nh, b), dim3(128), 0, (const uint16_t*)m.qkv.p, t, H, scale, m.ctx.p);
-        else
-            blaunch(st, bert_attn_long_kernel, dim3(m.nh, b, (t + kBertS - 1) / kBertS), dim3(128), 0, (const uint16_t*)m.qkv.p, t, H, scale, m.ctx.p);
+        if (qkv_attn) {     // B2 to B4 in one kernel
+            launch_bert_qkv(m, tm_x, w, b, t, scale);
+        } else {
+            // B2: fused q|k|v projection + bias -> bf16 [T, 3H]
+            launch_gemm<GEPI_BIAS_BF16>(st, tm_x, w.tm_wqkv, GemmArgs{T, 3 * H, H, w.bqkv, nullptr, 0, m.qkv.p, 3 * H, 1, 0});
+            // B3+B4: per (sentence, head) softmax(QK^T / sqrt(d)) V, no mask
+            if (t <= kBertS)
+                blaunch(st, bert_attn_kernel, dim3(m.nh, b), dim3(128), 0, (const uint16_t*)m.qkv.p, t, H, scale, m.ctx.p);
+            else
+                blaunch(st, bert_attn_long_kernel, dim3(m.nh, b, (t + kBertS - 1) / kBertS), dim3(128), 0, (const uint16_t*)m.qkv.p, t, H, scale, m.ctx.p);
+        }
         if (blocks) {       // B5 to B7 in one kernel
             launch_bert_block(m, tm_ctx, tm_x, w, T, eps);
             continue;

@@ -1,0 +1,42 @@
+"""The kernel of q|k|v and attention (bert_qkv.cuh), which sentences of up to 128 tokens take, at the edges of its groups of sentences, of its 16-row and
+16-key tiles and of its pairs of SMs, against the oracle."""
+import numpy as np
+import pytest
+
+from oracle import bert as obert
+from oracle import synth
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def encoder():
+    from fastllm_b200 import models
+    cfg = obert.BertConfig(384, 12, 2, 1536, 128, 1e-12, 512)
+    w = obert.synth_weights(cfg, 11, 0.06)
+    return cfg, obert.MiniLM(cfg, w), models.MiniLMModel(models.BertConfig(384, 12, 2, 1536, 128, 1e-12, 512), w, 0)
+
+
+# a whole tile, one row less; two sentences a group and one; rows of a tile left over (43: 42 of 128; 25: three); sentences within a 16-row tile; an odd
+# number of groups; fewer units than pairs of SMs, more, runs that begin inside a pair's heads
+@pytest.mark.parametrize("b,t", [(1, 128), (2, 127), (37, 128), (9, 64), (10, 65), (31, 43), (33, 25), (70, 17), (75, 16), (150, 8), (223, 5), (700, 1), (300, 113)])
+def test_against_the_oracle(encoder, b, t):
+    """bf16 operands: 2^-9 of a value per rounding, four roundings between sums of hundreds per layer; a misplaced row, head or key is a cosine below 0.9"""
+    cfg, oracle, model = encoder
+    ids = synth.token_ids(1000 + b * 131 + t, cfg.vocab_size, (b, t))
+    picked = sorted({0, 1 % b, b // 2, b - 2 if b > 1 else 0, b - 1})
+    got, want = model.embed_ids(ids)[picked], oracle.embed_ids(ids[picked])
+    cos = (got * want).sum(1) / (np.linalg.norm(got, axis=1) * np.linalg.norm(want, axis=1))
+    assert cos.min() >= 0.999 and np.abs(got - want).max() <= 2e-2
+
+
+@pytest.mark.parametrize("b,t", [(60, 20), (200, 7), (41, 50), (10, 127)])
+def test_sentences_do_not_see_each_other(encoder, b, t):
+    """another sentence in its place leaves the neighbours in its tile as they are, to the bit"""
+    cfg, _, model = encoder
+    ids = synth.token_ids(7, cfg.vocab_size, (b, t))
+    before = model.embed_ids(ids)
+    ids[b // 2] = synth.token_ids(8, cfg.vocab_size, (t,))
+    after = model.embed_ids(ids)
+    others = np.arange(b) != b // 2
+    assert np.array_equal(after[others], before[others]) and not np.array_equal(after[b // 2], before[b // 2])
