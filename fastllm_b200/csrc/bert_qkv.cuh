@@ -46,21 +46,21 @@ __device__ __forceinline__ float2 add_f32x2(float2 x, float2 y) {
     return d;
 }
 // 16 query rows (m0 on) of a sentence's head: sq, sk, sv at the sentence's first row.  The rows of o take the place of the q rows that this warp alone reads.
-// KT: 16-key steps of the sentence's t tokens; rows behind it read as its last one, as queries nobody uses what they give, as keys their weight is zero.
-template <int KT>
+// LD: elements of a row.  KT: 16-key steps of the sentence's t tokens; rows behind it read as its last one, as queries nobody uses what they give, as keys their weight is zero.
+template <int KT, int LD>
 __device__ __forceinline__ void bq_attention(uint16_t* sq, const uint16_t* sk, const uint16_t* sv, int t, int m0, float qscale, uint16_t* ctx, int lane) {
     const int g = lane >> 2, tq = lane & 3;
     uint32_t qa[2][4];
     float2 s[2 * KT][2];
 #pragma unroll
-    for (int ks = 0; ks < 2; ++ks) ldmatrix_x4(qa[ks], sq + min(m0 + (lane & 15), t - 1) * kBqLd + ks * 16 + (lane >> 4) * 8);
+    for (int ks = 0; ks < 2; ++ks) ldmatrix_x4(qa[ks], sq + min(m0 + (lane & 15), t - 1) * LD + ks * 16 + (lane >> 4) * 8);
     // two key tiles a step, the next step's keys requested before this one's products
     uint32_t kb[2][2][4];
     auto keys = [&](int i) {
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             const int r = (2 * i + u) * 8 + (lane & 7);
-            ldmatrix_x4(kb[i & 1][u], sk + (i + 1 < KT ? r : min(r, t - 1)) * kBqLd + (lane >> 3) * 8);
+            ldmatrix_x4(kb[i & 1][u], sk + (i + 1 < KT ? r : min(r, t - 1)) * LD + (lane >> 3) * 8);
         }
     };
     keys(0);
@@ -104,7 +104,7 @@ __device__ __forceinline__ void bq_attention(uint16_t* sq, const uint16_t* sk, c
         uint32_t pa[4], vb[2][4];
         const int vr = ks * 16 + (lane & 15);
 #pragma unroll
-        for (int d = 0; d < 2; ++d) ldmatrix_x4_trans(vb[d], sv + (ks + 1 < KT ? vr : min(vr, t - 1)) * kBqLd + d * 16 + (lane >> 4) * 8);
+        for (int d = 0; d < 2; ++d) ldmatrix_x4_trans(vb[d], sv + (ks + 1 < KT ? vr : min(vr, t - 1)) * LD + d * 16 + (lane >> 4) * 8);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             float2 x = fma_f32x2(s[2 * ks + h][0], qs, b0), y = fma_f32x2(s[2 * ks + h][1], qs, b1);
@@ -132,13 +132,13 @@ __device__ __forceinline__ void bq_attention(uint16_t* sq, const uint16_t* sk, c
     __syncwarp();
 #pragma unroll
     for (int dt = 0; dt < 4; ++dt) {
-        if (m0 + g < t) *reinterpret_cast<uint32_t*>(sq + (m0 + g) * kBqLd + dt * 8 + tq * 2) = pack_bf16(o[dt][0] * inv[0], o[dt][1] * inv[0]);
-        if (m0 + g + 8 < t) *reinterpret_cast<uint32_t*>(sq + (m0 + g + 8) * kBqLd + dt * 8 + tq * 2) = pack_bf16(o[dt][2] * inv[1], o[dt][3] * inv[1]);
+        if (m0 + g < t) *reinterpret_cast<uint32_t*>(sq + (m0 + g) * LD + dt * 8 + tq * 2) = pack_bf16(o[dt][0] * inv[0], o[dt][1] * inv[0]);
+        if (m0 + g + 8 < t) *reinterpret_cast<uint32_t*>(sq + (m0 + g + 8) * LD + dt * 8 + tq * 2) = pack_bf16(o[dt][2] * inv[1], o[dt][3] * inv[1]);
     }
     __syncwarp();
 #pragma unroll
     for (int r = m0 + g; r < m0 + 16; r += 8)           // whole 64-byte pieces of the rows
-        if (r < t) *reinterpret_cast<uint4*>(ctx + (size_t)r * kBbH + tq * 8) = *reinterpret_cast<const uint4*>(sq + r * kBqLd + tq * 8);
+        if (r < t) *reinterpret_cast<uint4*>(ctx + (size_t)r * kBbH + tq * 8) = *reinterpret_cast<const uint4*>(sq + r * LD + tq * 8);
 }
 // 32 columns on their way; tmem_arrived32: all that were requested are there
 __device__ __forceinline__ void tmem_request32(uint32_t taddr, uint32_t (&r)[32]) {
@@ -307,7 +307,7 @@ bert_qkv_attn_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             for (int it = aw; ok && it < ns * mts * g.hpu; it += kBqWarps) {
                 const int h = it % g.hpu, s = it / g.hpu / mts, m0 = it / g.hpu % mts * 16;
                 uint16_t *row = sQ + s * g.t * kBqLd + h * kBertD, *to = ctx + (size_t)s * g.t * kBbH + h * kBertD;
-                auto go = [&](auto kt) { bq_attention<decltype(kt)::value>(row, row + kBqCols, row + 2 * kBqCols, g.t, m0, g.qscale, to, lane); };
+                auto go = [&](auto kt) { bq_attention<decltype(kt)::value, kBqLd>(row, row + kBqCols, row + 2 * kBqCols, g.t, m0, g.qscale, to, lane); };
                 switch (mts) {
                     case 1: go(std::integral_constant<int, 1>{}); break;
                     case 2: go(std::integral_constant<int, 2>{}); break;

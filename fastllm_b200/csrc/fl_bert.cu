@@ -279,8 +279,16 @@ void bert_finalize(BertModel& m) {
     }
     if (m.small_layers != nullptr) {
         std::vector<BertSmallLayer> tab;
-        for (const BertLayerW& w : m.layers) tab.push_back({w.wqkv, w.wo, w.wi, w.wo2, w.bqkv, w.bo, w.bi, w.bo2, w.ln1w, w.ln1b, w.ln2w, w.ln2b});
+        m.small_pack.alloc(m.layers.size() * kBsCluster * kBsPack);
+        for (const BertLayerW& w : m.layers) {
+            uint16_t* pack = m.small_pack.p + tab.size() * kBsCluster * kBsPack;
+            bert_small_pack_kernel<<<dim3(32, kBsCluster), 256>>>(w.wqkv, w.wo, w.wi, w.wo2, pack);
+            g_launches.fetch_add(1);
+            tab.push_back({pack, w.bqkv, w.bo, w.bi, w.bo2, w.ln1w, w.ln1b, w.ln2w, w.ln2b});
+        }
+        FL_CUDA(cudaGetLastError());
         FL_CUDA(cudaMemcpy(m.small_layers, tab.data(), tab.size() * sizeof(BertSmallLayer), cudaMemcpyHostToDevice));
+        FL_CUDA(cudaStreamSynchronize(cudaStreamLegacy));       // (the model's stream does not wait for the default one)
     }
     m.finalized = true;
 }
@@ -322,7 +330,6 @@ static bool bert_blocks(const BertModel& m, int T) {
 // The line lies where the clusters (about nine of 16 blocks) are all resident and none has more than 64 tokens: there both take the same (sentences
 // x tokens, chain / one launch, us: 16 x 19 315 / 256, 9 x 48 323 / 324, 18 x 31 319 / 323, 9 x 64 328 / 333, 36 x 16 319 / 315), and a second wave
 // would cost a whole pass more.
-constexpr int kBsCluster = 16;
 template <int MT>
 static int bert_small_launch(BertModel& m, const BertSmallArgs& a, int clusters, bool ask) {      // ask: -> clusters that are resident at a time
     auto kern = bert_small_kernel<MT, kBsCluster>;
@@ -381,7 +388,8 @@ static void bert_reserve(BertModel& m, const BertRun& run, int b, int t) {
 static void bert_enqueue_small(BertModel& m, const BertRun& run, int b, int t, bool has_mask) {
     const int spc = run.spc, clusters = run.clusters, rows = spc * t;
     const BertSmallArgs a{static_cast<const BertSmallLayer*>(m.small_layers), m.wemb, m.pemb, m.lnw, m.lnb, m.ids.p, has_mask ? m.mask.p : nullptr,
-                          m.L, b, t, m.V, m.maxpos, spc, m.cfg.norm_eps, 1.f / (float)std::sqrt((double)m.d), m.qkv.p, m.ctx.p, m.hbuf.p, m.pre.p, m.out.p};
+                          m.L, b, t, m.V, m.maxpos, spc, m.cfg.norm_eps, 1.4426950408889634f / (float)std::sqrt((double)m.d), m.ctx.p, m.hbuf.p, m.pre.p,
+                          m.failed.p, m.out.p};
     switch ((rows + 15) / 16) {
         case 1: bert_small_launch<1>(m, a, clusters, false); break;
         case 2: bert_small_launch<2>(m, a, clusters, false); break;
