@@ -27,10 +27,11 @@ constexpr int kCsSlab = 64;             // value columns at a time
 constexpr int kCsPad = 4;               // floats behind a row in shared memory: neighbouring rows start four banks apart
 constexpr int kCsLdA = kCsC + kCsPad;   // row stride of a [64][64] operand
 constexpr int kCsChunks = 32;           // chunks whose states are held at a time (32 heads of 128 x 128: 67 MB), over all sequences of a step
-// Portions from this length on.  Whole prefill token by token -> in chunks, 96 / 128 / 160 / 192 tokens: gated linear attention, width 2048, 728 -> 722,
-// 771 -> 732, 847 -> 780, 881 -> 783 us; lightning 607 -> 577, 605 -> 590, 683 -> 657, 706 -> 661; delta rule and Mamba-2 543 -> 551, 550 -> 550,
-// 623 -> 617, 665 -> 622, of width 4096 838 -> 877, 889 -> 898, 1105 -> 1099, 1160 -> 1110.  (64 tokens are slower in chunks everywhere.)
-constexpr int kCsMinTokens = 128;
+// Portions from this length on.  Whole prefill token by token -> in chunks, us: gated linear attention, width 2048, 96 / 128 / 160 / 192 tokens: 728 -> 722,
+// 771 -> 732, 847 -> 780, 881 -> 783.  One decay per head (ly_rec_scan_kernel takes 0.25 to 0.3 us a token): delta rule and Mamba-2 128 / 192 / 256 / 327
+// tokens: width 1024 361 -> 424, 477 -> 505, 536 -> 527; 2048 449 -> 503, 575 -> 611, 629 -> 661, 697 -> 713; 4096 (192, 256) 1054 -> 1093, 1145 -> 1131;
+// lightning, width 2048, 128 / 192 / 256 / 333: 550 -> 568, 662 -> 665, 675 -> 678, 717 -> 692.
+constexpr int kCsMinTokensGla = 128, kCsMinTokens = 256;
 
 struct ChunkArgs {
     const float* src; int ld, off_q, off_k, off_v;      // q, k [G][D], v [H][Dv] per row
@@ -41,6 +42,7 @@ struct ChunkArgs {
     float* state;                   // [slots][H][D][Dv]
     const int *seq_row0, *seq_slot, *seq_pos0;
     int n, H, G, D, Dv;
+    int min_tokens;                 // of a portion that goes in chunks
     int span0, span;                // chunks [span0, span0 + span) of every sequence are handled by this round of launches
     float* us;                      // [chunk][H][D][Dv]: what a chunk adds to the state, then the state at its start
     float* dec;                     // [chunk][H]: decay over a chunk ([chunk][H][D] for the gated linear attention)
@@ -50,7 +52,7 @@ struct ChunkArgs {
 };
 // chunks of a sequence of `len` tokens in this span
 __device__ __forceinline__ int cs_count(const ChunkArgs& a, int len) {
-    return len < kCsMinTokens ? 0 : max(0, min(a.span, (len + kCsC - 1) / kCsC - a.span0));
+    return len < a.min_tokens ? 0 : max(0, min(a.span, (len + kCsC - 1) / kCsC - a.span0));
 }
 // chunk number of the launch -> sequence, first row, tokens; false: none
 __device__ __forceinline__ bool cs_find(const ChunkArgs& a, int chunk, int& row, int& len) {

@@ -1117,34 +1117,35 @@ static void launch_gqa_attn(LaunchCtx& lc, const GqaAttnArgs& a, int T, int max_
 template <bool DELTA>
 static void launch_rec_scan(LaunchCtx& lc, const RecArgs& a, int n) {
     const int rpt = (a.D + kRecParts - 1) / kRecParts;
-    auto go = [&](auto kern, int RPT) {
-        const size_t smem = (size_t)4 * (RPT >= 64 ? 4 : 8) * (2 * kRecParts * (RPT + 4) + 12) * 4;       // [4 warps][ring][slot] floats
-        launch(lc, DELTA ? "delta_scan" : "ssm_scan", 0, kern, dim3(n, a.H, (a.Dv + kRecCols - 1) / kRecCols), dim3(128), smem, a);
+    auto go = [&](auto rows) {
+        constexpr int RPT = decltype(rows)::value;
+        launch(lc, DELTA ? "delta_scan" : "ssm_scan", 0, ly_rec_scan_kernel<RPT, DELTA>, dim3(n, a.H, (a.Dv + kRecCols - 1) / kRecCols), dim3(160), ly_rec_smem<RPT>(), a);
     };
-    if (rpt <= 2) go(ly_rec_scan_kernel<2, DELTA>, 2);
-    else if (rpt <= 4) go(ly_rec_scan_kernel<4, DELTA>, 4);
-    else if (rpt <= 8) go(ly_rec_scan_kernel<8, DELTA>, 8);
-    else if (rpt <= 16) go(ly_rec_scan_kernel<16, DELTA>, 16);
-    else if (rpt <= 32) go(ly_rec_scan_kernel<32, DELTA>, 32);
-    else go(ly_rec_scan_kernel<64, DELTA>, 64);
+    if (rpt <= 2) go(std::integral_constant<int, 2>{});
+    else if (rpt <= 4) go(std::integral_constant<int, 4>{});
+    else if (rpt <= 8) go(std::integral_constant<int, 8>{});
+    else if (rpt <= 16) go(std::integral_constant<int, 16>{});
+    else if (rpt <= 32) go(std::integral_constant<int, 32>{});
+    else go(std::integral_constant<int, 64>{});
 }
 
 enum class Recurrence { scalar, gla, delta };
-// Portions of kCsMinTokens tokens and more take the chunked kernels (chunk_scan.cuh), in the serving precision: the exact mode's sums must
+static int chunk_min(Recurrence kind) { return kind == Recurrence::gla ? kCsMinTokensGla : kCsMinTokens; }
+// Portions of chunk_min tokens and more take the chunked kernels (chunk_scan.cuh), in the serving precision: the exact mode's sums must
 // not depend on how a prompt was cut.  The chunked kernels read 16 bytes at a time and hold at most 128 state rows.
-static bool chunks_fit(const ChunkArgs& a, bool f32, const int* counts, int n) {
+static bool chunks_fit(const ChunkArgs& a, Recurrence kind, bool f32, const int* counts, int n) {
     if (f32 || a.D > 128 || ((a.D | a.Dv | a.ld | a.off_q | a.off_k | a.off_v) & 3) != 0) return false;
     for (int i = 0; i < n; ++i)
-        if (counts[i] >= kCsMinTokens) return true;
+        if (counts[i] >= chunk_min(kind)) return true;
     return false;
 }
 // How a step's long portions go through the chunked kernels: `span` chunks of each at a time, `most` chunks in the longest, states of `held` chunks.
 struct ChunkPlan { int span = 0, most = 0; size_t held = 0; };
-static ChunkPlan chunk_plan(const int* counts, int n) {
+static ChunkPlan chunk_plan(Recurrence kind, const int* counts, int n) {
     ChunkPlan p;
     int longs = 0;
     for (int i = 0; i < n; ++i)
-        if (counts[i] >= kCsMinTokens) { ++longs; p.most = std::max(p.most, (counts[i] + kCsC - 1) / kCsC); }
+        if (counts[i] >= chunk_min(kind)) { ++longs; p.most = std::max(p.most, (counts[i] + kCsC - 1) / kCsC); }
     if (longs == 0) return p;
     p.span = std::max(1, kCsChunks / longs);
     p.held = (size_t)std::min(p.span, p.most) * longs;
@@ -1171,7 +1172,7 @@ static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurr
         room(ly_chunk_out_kernel<DP, 0>, sm_out); room(ly_chunk_out_kernel<DP, 1>, sm_out); room(ly_chunk_out_kernel<DP, 2>, sm_out2);
         attr_set = true;
     }
-    const ChunkPlan pl = chunk_plan(counts, n);
+    const ChunkPlan pl = chunk_plan(kind, counts, n);
     const ChunkScratch need = chunk_scratch(kind, a.H, a.D, a.Dv, pl, y.rows);
     FL_CHECK(y.cs_us.n >= need.us && y.cs_dec.n >= need.dec && y.cs_qd.n >= need.qd && y.cs_aq.n >= need.aq && y.cs_wk.n >= need.wk, FL_ERR_STATE,
              "internal: scratch of the chunked recurrences too small");
@@ -1182,7 +1183,7 @@ static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurr
     for (a.span0 = 0; a.span0 < most; a.span0 += a.span) {
         int chunks = 0;
         for (int i = 0; i < n; ++i)
-            if (counts[i] >= kCsMinTokens) chunks += std::max(0, std::min(a.span, (counts[i] + kCsC - 1) / kCsC - a.span0));
+            if (counts[i] >= a.min_tokens) chunks += std::max(0, std::min(a.span, (counts[i] + kCsC - 1) / kCsC - a.span0));
         const dim3 grid(chunks, a.H), b(256);
         if (kind == Recurrence::delta) {
             launch(lc, "delta_chunks", 0, ly_chunk_delta_kernel<DP>, grid, b, sm_delta, a);
@@ -1200,11 +1201,12 @@ static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurr
     }
 }
 // -> whether the token-serial kernel has sequences left
-static bool launch_chunks(fl_cache& c, LaunchCtx& lc, const ChunkArgs& a, Recurrence kind, const int* counts, int n) {
+static bool launch_chunks(fl_cache& c, LaunchCtx& lc, ChunkArgs a, Recurrence kind, const int* counts, int n) {
+    a.min_tokens = chunk_min(kind);
     if (a.D <= 64) launch_chunks_dp<64>(*c.ly, lc, a, kind, counts, n);
     else launch_chunks_dp<128>(*c.ly, lc, a, kind, counts, n);
     for (int i = 0; i < n; ++i)
-        if (counts[i] < kCsMinTokens) return true;
+        if (counts[i] < a.min_tokens) return true;
     return false;
 }
 // a recurrence with one decay per head and token
@@ -1214,9 +1216,10 @@ static void run_recurrence(fl_cache& c, LaunchCtx& lc, RecArgs ra, bool f32, con
     ca.src = ra.cv; ca.ld = ra.ldc; ca.off_q = ra.off_q; ca.off_k = ra.off_k; ca.off_v = ra.off_v; ca.ab = ra.ab; ca.dskip = ra.dskip;
     ca.o = ra.o; ca.state = ra.state; ca.seq_row0 = ra.seq_row0; ca.seq_slot = ra.seq_slot; ca.seq_pos0 = ra.seq_pos0;
     ca.n = n; ca.H = ra.H; ca.G = ra.G; ca.D = ra.D; ca.Dv = ra.Dv;
-    if (chunks_fit(ca, f32, counts, n)) {
-        ra.skip_from = kCsMinTokens;
-        if (!launch_chunks(c, lc, ca, DELTA ? Recurrence::delta : Recurrence::scalar, counts, n)) return;
+    constexpr Recurrence kind = DELTA ? Recurrence::delta : Recurrence::scalar;
+    if (chunks_fit(ca, kind, f32, counts, n)) {
+        ra.skip_from = chunk_min(kind);
+        if (!launch_chunks(c, lc, ca, kind, counts, n)) return;
     }
     launch_rec_scan<DELTA>(lc, ra, n);
 }
@@ -1419,7 +1422,6 @@ static void reserve_portions(fl_cache& c, const int* slots, const int* counts, i
     const LayeredModel& m = *c.lm;
     LayeredCache& y = *c.ly;
     if (m.f32 || *std::max_element(counts, counts + n) < 64) return;        // (decoded tokens and short portions need none of it)
-    const ChunkPlan pl = chunk_plan(counts, n);
     ChunkScratch cs;
     size_t kc = 0, kct = 0;
     auto up = [](size_t& a, size_t b) { a = std::max(a, b); };
@@ -1434,8 +1436,9 @@ static void reserve_portions(fl_cache& c, const int* slots, const int* counts, i
             }
         } else if (d.mixer == FL_MIXER_GLA || d.mixer == FL_MIXER_DELTA || d.mixer == FL_MIXER_MAMBA2 || d.mixer == FL_MIXER_LIGHTNING) {
             const int D = d.mixer == FL_MIXER_MAMBA2 ? d.state : d.dim;
-            if (pl.held == 0 || D > 128) return;
             const Recurrence kind = d.mixer == FL_MIXER_GLA ? Recurrence::gla : (d.mixer == FL_MIXER_DELTA ? Recurrence::delta : Recurrence::scalar);
+            const ChunkPlan pl = chunk_plan(kind, counts, n);
+            if (pl.held == 0 || D > 128) return;
             const ChunkScratch s = chunk_scratch(kind, d.heads, D, d.vdim, pl, y.rows);
             up(cs.us, s.us); up(cs.dec, s.dec); up(cs.qd, s.qd); up(cs.aq, s.aq); up(cs.wk, s.wk);
         }
@@ -1683,8 +1686,8 @@ static void run_mixer(fl_cache& c, LaunchCtx& lc, const StepTab& st, const Layer
         gc.qscale = ga.qscale; gc.o = ga.o; gc.state = ga.state; gc.seq_row0 = ga.seq_row0; gc.seq_slot = ga.seq_slot; gc.seq_pos0 = ga.seq_pos0;
         gc.n = n; gc.H = gc.G = H; gc.D = D; gc.Dv = Dv;
         bool rest = true;
-        if (chunks_fit(gc, m.f32, counts, n)) {
-            ga.skip_from = kCsMinTokens;
+        if (chunks_fit(gc, Recurrence::gla, m.f32, counts, n)) {
+            ga.skip_from = chunk_min(Recurrence::gla);
             rest = launch_chunks(c, lc, gc, Recurrence::gla, counts, n);
         }
         if (rest) launch_gla_scan(lc, ga, n);

@@ -2124,116 +2124,161 @@ struct RecArgs {
     int H, G, D, Dv;
     int skip_from = 0;          // as for the gated linear attention
 };
-constexpr int kRecCols = 32, kRecParts = 4;       // value columns per block; threads that share a column's rows
+constexpr int kRecCols = 32, kRecParts = 4;       // value columns per block; parts of a column's rows
 // Token by token, per head:  S <- a S;  u = b v   (DELTA: u = b (v - S^T k));  S <- S + k u^T;  o = S^T q (+ dskip v).
-// One block of four warps per (sequence, head, 32 value columns) -- columns of S never interact.  A column's rows are split over
-// four neighbouring lanes (lane part p keeps rows p RPT .. p RPT + RPT - 1 in registers), so the two reductions over rows are a
-// serial sum per lane and two shuffles: the warps of a block never wait for one another.  Each warp keeps a ring of the next
-// tokens' operands (k, q, its eight values, a, b) in its own shared memory, filled by asynchronous copies several tokens ahead,
-// so a token's step waits for no global load.  The order of operations per token does not depend on how a prompt was cut.
+// One block per (sequence, head, 32 value columns) -- columns of S never interact.  A column's rows are split over four neighbouring lanes of one of
+// four warps, in registers, so the two reductions over rows are two serial sums per lane and two shuffles: the warps never wait for one another.  A
+// fifth warp brings k, q and the block's values four tokens at a time, two groups ahead (bulk copies where rows are 16-byte pieces); decays and
+// strengths are loaded a group ahead, results stored a group at a time.  The order of operations per token does not depend on how a prompt was cut.
+// A lane's pieces of four rows begin with a piece of its own (`rot`), so that the four read different banks of unpadded rows.
+// Bound: the chain per token.  203 tokens, delta rule, 8 heads of 128 x 128: 99 -> 60 us; 95 -> 51 without the correction (every warp copying for itself, four
+// bytes a lane, the copies and stores held up the warp's own products: 0.5 us a token, of which 0.3 were those).  The rows over eight lanes: the same.
 template <int RPT, bool DELTA>
-static __global__ void __launch_bounds__(128) ly_rec_scan_kernel(RecArgs a) {
+static __global__ void __launch_bounds__(160) ly_rec_scan_kernel(RecArgs a) {
     pdl_chain();
-    extern __shared__ __align__(16) float sm[]; // [4 warps][NST tokens][k | q: 4 parts x (RPT + 4) each (the pad keeps the parts on different banks) | v x 8 | a | b | pad]
     constexpr int DP = RPT * kRecParts;         // rows, padded (rows >= D hold zeros and never change)
-    constexpr int PS = RPT + 4, DPS = kRecParts * PS;      // floats per part / per vector in shared memory
-    constexpr int NST = RPT >= 64 ? 4 : 8;      // tokens in the ring
-    constexpr int SLOT = 2 * DPS + 12;
-    constexpr int NL = (2 * DP + 31) / 32;      // k | q values a lane copies per token
+    constexpr int GT = 4, NG = 3;               // tokens of a group, groups in the ring
+    constexpr int BC = kRecCols, SLOT = 2 * DP + BC;                          // columns of the block; floats of a token: k | q | v
+    constexpr int LPC = kRecParts, CW = 32 / LPC, HALF = RPT / 2;             // lanes per column, columns per warp; a lane sums the halves of its rows
+    constexpr int NP = HALF / 4;                // pieces of four rows in half a part
+    extern __shared__ __align__(16) float sm[]; // [NG GT][SLOT]
+    __shared__ __align__(8) uint64_t full[NG], empty[NG];
     const int D = a.D, Dv = a.Dv;
-    const int seq = blockIdx.x, hd = blockIdx.y, g = hd / (a.H / a.G);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, p = lane & 3, cl = lane >> 2;
-    const int col0 = blockIdx.z * kRecCols + wid * 8, col = col0 + cl;
-    const bool vok = col < Dv;
-    float* wsm = sm + wid * (NST * SLOT);
+    const int seq = blockIdx.x, hd = blockIdx.y, g = hd / (a.H / a.G), v0 = blockIdx.z * BC;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int r0 = a.seq_row0[seq], r1 = a.seq_row0[seq + 1];
-    if (a.skip_from > 0 && r1 - r0 >= a.skip_from) return;
+    if (r0 >= r1 || (a.skip_from > 0 && r1 - r0 >= a.skip_from)) return;
+    if (threadIdx.x == 0) {
+        for (int i = 0; i < NG; ++i) { mbar_init(&full[i], 1); mbar_init(&empty[i], 4); }
+        mbar_fence_init();
+    }
+    for (int i = threadIdx.x; i < NG * GT * SLOT; i += 160) sm[i] = 0.f;       // what no copy ever writes (rows >= D, columns >= Dv) reads as zero
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncthreads();
+
+    if (wid == 4) {
+        const int nv = min(BC, Dv - v0);
+        const bool pieces = ((D | Dv | a.ldc | a.off_q | a.off_k | a.off_v) & 3) == 0 && (reinterpret_cast<uintptr_t>(a.cv) & 15) == 0;
+        int grp = 0;
+        uint32_t ph = 1;
+        for (int row = r0; row < r1; row += GT) {
+            const int n = min(GT, r1 - row);
+            mbar_wait(&empty[grp], ph);
+            if (pieces) {
+                if (lane == 0) mbar_expect_tx(&full[grp], (uint32_t)(n * (2 * D + nv) * 4));
+                __syncwarp();
+                if (lane < 3 * n) {             // a copy per lane: k, q or v of one of the tokens
+                    const int t = lane / 3, w = lane % 3;
+                    const float* pr = a.cv + (size_t)(row + t) * a.ldc;
+                    bulk_g2s(sm + (grp * GT + t) * SLOT + w * DP, pr + (w == 0 ? a.off_k + g * D : w == 1 ? a.off_q + g * D : a.off_v + hd * Dv + v0), (uint32_t)(w < 2 ? D : nv) * 4,
+                             &full[grp]);
+                }
+            } else {
+                for (int t = 0; t < n; ++t) {
+                    const float* pr = a.cv + (size_t)(row + t) * a.ldc;
+                    float* dst = sm + (grp * GT + t) * SLOT;
+                    for (int d = lane; d < D; d += 32) {
+                        dst[d] = pr[a.off_k + g * D + d];
+                        dst[DP + d] = pr[a.off_q + g * D + d];
+                    }
+                    for (int c = lane; c < nv; c += 32) dst[2 * DP + c] = pr[a.off_v + hd * Dv + v0 + c];
+                }
+                __syncwarp();
+                if (lane == 0) mbar_arrive(&full[grp]);
+            }
+            if (++grp == NG) { grp = 0; ph ^= 1; }
+        }
+        return;
+    }
+
+    const int p = lane % LPC, c0 = wid * CW + lane / LPC, col = v0 + c0;      // part, column
+    const bool vok = col < Dv;
+    // register i is row at(i) of the head: half i / HALF of part p, its pieces from piece rot on
+    auto at = [&](int i) {
+        const int h = i / HALF, j = i % HALF;
+        if (NP <= 1) return p * RPT + h * HALF + j;
+        const int rot = RPT >= 64 ? 2 * p + h : RPT == 32 ? p : p >> 1;
+        return p * RPT + h * HALF + (j / 4 + rot) % NP * 4 + j % 4;
+    };
     float* st = a.state + (((size_t)a.seq_slot[seq] * a.H + hd) * D) * Dv + col;
     float s[RPT];
     const bool fresh = a.seq_pos0[seq] == 0;
 #pragma unroll
     for (int i = 0; i < RPT; ++i) {
-        const int d = p * RPT + i;
+        const int d = at(i);
         s[i] = (!fresh && vok && d < D) ? st[(size_t)d * Dv] : 0.f;
     }
     const float dsk = a.dskip ? a.dskip[hd] : 0.f;
-    for (int i = lane; i < NST * SLOT; i += 32) wsm[i] = 0.f;       // what no copy ever writes (rows >= D, columns >= Dv) reads as zero
-    __syncwarp();
-    auto issue = [&](int row, int slot) {
-        const float* pr = a.cv + (size_t)row * a.ldc;
-        float* dst = wsm + slot * SLOT;
+    // over the column's rows
+    auto whole = [&](const float (&h)[2]) {
+        float t = h[0] + h[1];
 #pragma unroll
-        for (int t = 0; t < NL; ++t) {
-            const int idx = lane + 32 * t, isq = idx >= DP, d = idx - isq * DP;
-            if (idx < 2 * DP && d < D) cp_async_f32(dst + isq * DPS + (d / RPT) * PS + d % RPT, pr + (isq ? a.off_q : a.off_k) + g * D + d);
-        }
-        if (lane < 8) {
-            if (col0 + lane < Dv) cp_async_f32(dst + 2 * DPS + lane, pr + a.off_v + hd * Dv + col0 + lane);
-        } else if (lane < 10) {
-            cp_async_f32(dst + 2 * DPS + lane, a.ab + ((size_t)row * a.H + hd) * 2 + (lane - 8));
-        }
+        for (int o = 1; o < LPC; o <<= 1) t += __shfl_xor_sync(0xFFFFFFFFu, t, o);
+        return t;
     };
+    // lane t: decay and strength of token t of a group
+    auto decays = [&](int row) { return lane < GT && row + lane < r1 ? *reinterpret_cast<const float2*>(a.ab + ((size_t)(row + lane) * a.H + hd) * 2) : make_float2(1.f, 0.f); };
+    float2 ab = decays(r0);
+    int grp = 0;
+    uint32_t ph = 0;
+    for (int row = r0; row < r1; row += GT) {
+        const float2 now = ab;
+        ab = decays(row + GT);
+        mbar_wait(&full[grp], ph);
+        float mine = 0.f;
+        auto token = [&](int t) {
+            const float* cur = sm + (grp * GT + t) * SLOT;
+            const float v = cur[2 * DP + c0], da = __shfl_sync(0xFFFFFFFFu, now.x, t), db = __shfl_sync(0xFFFFFFFFu, now.y, t);
+            float kb[RPT], qb[RPT];                   // this lane's rows of k and q
+            if (HALF % 4 == 0) {
 #pragma unroll
-    for (int t = 0; t < NST - 1; ++t) {
-        if (r0 + t < r1) issue(r0 + t, t);
-        cp_async_commit();
-    }
-    int it = 0;
-    for (int row = r0; row < r1; ++row, ++it) {
-        if (row + NST - 1 < r1) issue(row + NST - 1, (it + NST - 1) % NST);
-        cp_async_commit();
-        cp_async_wait<NST - 1>();               // this token's copies have landed (one group per token, empty ones included)
-        __syncwarp();
-        const float* cur = wsm + (it % NST) * SLOT;
-        const float v = cur[2 * DPS + cl], da = cur[2 * DPS + 8], db = cur[2 * DPS + 9];
-        float kb[RPT], qb[RPT];                 // this lane's rows of k and q
-        {
-            const float* ks = cur + p * PS;
-            if (RPT % 4 == 0) {
-#pragma unroll
-                for (int i = 0; i < RPT / 4; ++i) {
-                    const float4 k4 = reinterpret_cast<const float4*>(ks)[i], q4 = reinterpret_cast<const float4*>(ks + DPS)[i];
-                    kb[4 * i] = k4.x; kb[4 * i + 1] = k4.y; kb[4 * i + 2] = k4.z; kb[4 * i + 3] = k4.w;
-                    qb[4 * i] = q4.x; qb[4 * i + 1] = q4.y; qb[4 * i + 2] = q4.z; qb[4 * i + 3] = q4.w;
+                for (int i = 0; i < RPT; i += 4) {
+                    const float4 k4 = *reinterpret_cast<const float4*>(cur + at(i)), q4 = *reinterpret_cast<const float4*>(cur + DP + at(i));
+                    kb[i] = k4.x; kb[i + 1] = k4.y; kb[i + 2] = k4.z; kb[i + 3] = k4.w;
+                    qb[i] = q4.x; qb[i + 1] = q4.y; qb[i + 2] = q4.z; qb[i + 3] = q4.w;
                 }
             } else {
 #pragma unroll
-                for (int i = 0; i < RPT; ++i) { kb[i] = ks[i]; qb[i] = ks[DPS + i]; }
+                for (int i = 0; i < RPT; ++i) { kb[i] = cur[at(i)]; qb[i] = cur[DP + at(i)]; }
             }
-        }
-        float u;
-        if (DELTA) {
-            float part = 0.f;
+            float u = db * v;
+            if (DELTA) {
+                float part[2] = {0.f, 0.f};
 #pragma unroll
-            for (int i = 0; i < RPT; ++i) { s[i] *= da; part = fmaf(s[i], kb[i], part); }
-            part += __shfl_xor_sync(0xFFFFFFFFu, part, 1);
-            part += __shfl_xor_sync(0xFFFFFFFFu, part, 2);
-            u = db * (v - part);
-        } else {
+                for (int i = 0; i < RPT; ++i) { s[i] *= da; part[i / HALF] = fmaf(s[i], kb[i], part[i / HALF]); }
+                u = db * (v - whole(part));
+            } else {
 #pragma unroll
-            for (int i = 0; i < RPT; ++i) s[i] *= da;
-            u = db * v;
-        }
-        float acc = 0.f;
+                for (int i = 0; i < RPT; ++i) s[i] *= da;
+            }
+            float acc[2] = {0.f, 0.f};
 #pragma unroll
-        for (int i = 0; i < RPT; ++i) {
-            s[i] = fmaf(kb[i], u, s[i]);
-            acc = fmaf(s[i], qb[i], acc);
-        }
-        acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 1);
-        acc += __shfl_xor_sync(0xFFFFFFFFu, acc, 2);
-        if (p == 0 && vok) a.o[(size_t)row * a.H * Dv + hd * Dv + col] = acc + dsk * v;
-        __syncwarp();                           // the slot may be refilled in the next iteration
+            for (int i = 0; i < RPT; ++i) {
+                s[i] = fmaf(kb[i], u, s[i]);
+                acc[i / HALF] = fmaf(s[i], qb[i], acc[i / HALF]);
+            }
+            const float o = whole(acc) + dsk * v;
+            mine = lane % LPC == t ? o : mine;
+        };
+        const int n = min(GT, r1 - row);
+#pragma unroll 2
+        for (int t = 0; t < n; ++t) token(t);       // (unrolled whole: slower, 0.38 us a token without the delta rule)
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&empty[grp]);
+        // every lane of a column has the sums: one store for the group's tokens
+        if (lane % LPC < GT && row + lane % LPC < r1 && vok) a.o[(size_t)(row + lane % LPC) * a.H * Dv + hd * Dv + col] = mine;
+        if (++grp == NG) { grp = 0; ph ^= 1; }
     }
-    cp_async_wait<0>();
     if (vok) {
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
-            const int d = p * RPT + i;
+            const int d = at(i);
             if (d < D) st[(size_t)d * Dv] = s[i];
         }
     }
 }
+template <int RPT>
+constexpr size_t ly_rec_smem() { return (size_t)12 * (2 * RPT * kRecParts + kRecCols) * 4; }
 
 // u[row, part] = v / sqrt(mean_part v^2 + eps) * w,  v = y * silu(z): the gated output of Mamba-2, normed in `parts` equal pieces of
 // the inner width.  z = proj[row, off_z ...].  One block per (row, part).

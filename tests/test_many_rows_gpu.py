@@ -94,6 +94,19 @@ def test_chunks_equal_token_by_token(kind, dim, vdim, n):
     assert mod.relerr(cut, np.asarray(serial, dtype=np.float64)) < CHUNK_TOL
 
 
+@pytest.mark.parametrize("kind", ["mamba", "delta"])
+@pytest.mark.parametrize("dim,vdim", [(128, 64), (64, 40), (20, 36), (6, 10), (256, 32)])
+def test_token_by_token_in_any_cut(kind, dim, vdim):
+    """the serial recurrences bring four tokens at a time, rows of 16-byte pieces or not, heads of one to several pieces a lane: portions of every
+    remainder give the bits of the whole prompt, in the exact mode, and the oracle's numbers"""
+    mod, cfg = recurrent(kind, dim, vdim)
+    oracle, model = mod.build(cfg, seed=57)
+    toks = mod.tokens(cfg, 41, seed=58)
+    whole = mod.run_whole(model, toks, cache=model.new_device_cache(2, 64))
+    assert mod.relerr(whole, oracle.run(toks)) < mod.TOL["f32"]
+    assert np.array_equal(whole, mod.run_cut(model, toks, [1, 2, 3, 4, 5, 12, 14], cache=model.new_device_cache(2, 64)))
+
+
 @pytest.mark.parametrize("kind", ["gla", "mamba", "delta"])
 def test_chunks_of_several_sequences(kind):
     """two prompts of more chunks than are held at a time beside a short one and a decoded token; a reused slot starts from zero"""
