@@ -12,9 +12,9 @@
 //   1. ly_chunk_in_kernel / ly_chunk_gla_kernel / ly_chunk_delta_kernel   one block per (chunk, head): everything that needs no state
 //   2. ly_chunk_state_kernel / ly_chunk_delta_state_kernel                 the states at the chunks' starts, chunk by chunk
 //   3. ly_chunk_out_kernel                                                 one block per (chunk, head): what the starting state adds
-// Bound: 1 and 3 by latency -- operands in shared memory, 4 x 4 results per thread (64 FMA per 8 16-byte loads), 16 warps per SM (8 in the gated
-// one): at 1024 tokens ncu has the FMA pipe at 31 to 34 % (gated 14 %), issue slots at 45 to 47 % (25 %), shared memory at 47 to 50 % (24 %).  2: HBM.
-// Measured per layer, token by token -> chunks: gated linear attention, 1531 tokens, 16 heads of 128 x 128: 1160 -> 260 us; Mamba-2, 2048
+// Bound: 1 and 3 by latency -- operands in shared memory, 4 x 4 results per thread (64 FMA per 8 16-byte loads), 16 warps per SM:
+// at 1024 tokens ncu has the FMA pipe at 31 to 34 %, issue slots at 45 to 47 %, shared memory at 47 to 50 %.  2: HBM.
+// Measured per layer, token by token -> chunks: gated linear attention, 1531 tokens, 16 heads of 128 x 128: 1160 -> 180 us; Mamba-2, 2048
 // tokens, 128 heads of 128 x 64: 1186 -> 668 us (four heads per block: their scores are multiplied once); delta rule, 2048 tokens, 32 heads of 128 x 128: 1022 -> 626 us; lightning attention, 333
 // tokens, 16 heads: 246 -> 65 us.  Same model, same tokens: the logits agree to 1e-5 .. 4e-5, their error against 64 bits is unchanged.
 #pragma once
@@ -27,11 +27,11 @@ constexpr int kCsSlab = 64;             // value columns at a time
 constexpr int kCsPad = 4;               // floats behind a row in shared memory: neighbouring rows start four banks apart
 constexpr int kCsLdA = kCsC + kCsPad;   // row stride of a [64][64] operand
 constexpr int kCsChunks = 32;           // chunks whose states are held at a time (32 heads of 128 x 128: 67 MB), over all sequences of a step
-// Portions from this length on.  Whole prefill token by token -> in chunks, us: gated linear attention, width 2048, 96 / 128 / 160 / 192 tokens: 728 -> 722,
-// 771 -> 732, 847 -> 780, 881 -> 783.  One decay per head (ly_rec_scan_kernel takes 0.25 to 0.3 us a token): delta rule and Mamba-2 128 / 192 / 256 / 327
+// Portions from this length on (at least a chunk).  Whole prefill token by token -> in chunks, us: gated linear attention 64 / 80 / 96 / 127 tokens: width
+// 1024 373 -> 366, 411 -> 396, 431 -> 397, 469 -> 407; 2048 557 -> 551, 628 -> 615, 650 -> 619, 694 -> 638.  One decay per head (ly_rec_scan_kernel takes 0.25 to 0.3 us a token): delta rule and Mamba-2 128 / 192 / 256 / 327
 // tokens: width 1024 361 -> 424, 477 -> 505, 536 -> 527; 2048 449 -> 503, 575 -> 611, 629 -> 661, 697 -> 713; 4096 (192, 256) 1054 -> 1093, 1145 -> 1131;
 // lightning, width 2048, 128 / 192 / 256 / 333: 550 -> 568, 662 -> 665, 675 -> 678, 717 -> 692.
-constexpr int kCsMinTokensGla = 128, kCsMinTokens = 256;
+constexpr int kCsMinTokensGla = 64, kCsMinTokens = 256;
 
 struct ChunkArgs {
     const float* src; int ld, off_q, off_k, off_v;      // q, k [G][D], v [H][Dv] per row
@@ -71,8 +71,8 @@ __device__ __forceinline__ bool cs_find(const ChunkArgs& a, int chunk, int& row,
 }
 
 // ---- products of operands in shared memory, 256 threads, a 64 x 64 result: thread (ty, tx) holds rows ty + 16 r, r < 4 ------------------
-__device__ __forceinline__ void cs_thread(int& ty, int& tx) {
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+__device__ __forceinline__ void cs_thread(int& ty, int& tx) {         // (of 256 threads; a block of 512 makes two results at a time)
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5 & 7;
     ty = (w & 1) * 8 + (lane >> 2);
     tx = (w >> 1) * 4 + (lane & 3);
 }
@@ -125,9 +125,9 @@ __device__ __forceinline__ void cs_zero(float (&acc)[4][4]) {
         for (int c = 0; c < 4; ++c) acc[r][c] = 0.f;
 }
 // rows [0, len) x columns [0, D) of src (row stride ld) into dst [64][ldd], times scale; what lies outside is zero
-template <int DP>
+template <int DP, int NT = 256>
 __device__ __forceinline__ void cs_load(float* dst, int ldd, const float* src, int ld, int len, int D, float scale) {
-    for (int i = threadIdx.x; i < kCsC * (DP / 4); i += 256) {
+    for (int i = threadIdx.x; i < kCsC * (DP / 4); i += NT) {
         const int r = i / (DP / 4), c = i % (DP / 4) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < len && c < D) v = *reinterpret_cast<const float4*>(src + (size_t)r * ld + c);
@@ -137,7 +137,7 @@ __device__ __forceinline__ void cs_load(float* dst, int ldd, const float* src, i
 }
 // value columns [v0, v0 + 64), row j times rows[j] (nullptr: 1)
 __device__ __forceinline__ void cs_load_slab(float* dst, const float* src, int ld, int len, int v0, int Dv, const float* rows) {
-    for (int i = threadIdx.x; i < kCsC * (kCsSlab / 4); i += 256) {
+    for (int i = threadIdx.x & 255; i < kCsC * (kCsSlab / 4); i += 256) {
         const int r = i / (kCsSlab / 4), c = i % (kCsSlab / 4) * 4;
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if (r < len && v0 + c < Dv) v = *reinterpret_cast<const float4*>(src + (size_t)r * ld + v0 + c);
@@ -282,20 +282,25 @@ static __global__ void __launch_bounds__(256, 2) ly_chunk_in_kernel(ChunkArgs a)
 // ---- gated linear attention: one decay per head, token and key channel ---------------------------------------------------------------
 // The chunk's score matrix in 16 x 16 blocks: on the diagonal each pair's decay is the running product itself; below it the query is
 // decayed from its block's start, the key to the end of the block before that, so every factor stays <= 1.
+// One block fits an SM: sixteen warps, each half of the block with a slab of values of its own.  (Eight warps, and a reduction over the warp per pair of
+// the diagonal blocks: 209 -> 125 us for 1531 tokens of 16 heads of 128 x 128.)
+constexpr int kCsGlaThreads = 512;
 template <int DP>
-static __global__ void __launch_bounds__(256) ly_chunk_gla_kernel(ChunkArgs a) {
+constexpr size_t cs_gla_smem() { return ((size_t)2 * kCsC * (DP + kCsPad) + (kCsC * (DP + kCsPad) > 2 * kCsC * kCsLdA ? kCsC * (DP + kCsPad) : 2 * kCsC * kCsLdA) + kCsC * kCsLdA + kCsC / 16 * DP) * 4; }
+template <int DP>
+static __global__ void __launch_bounds__(kCsGlaThreads, 1) ly_chunk_gla_kernel(ChunkArgs a) {
     pdl_chain();
     extern __shared__ __align__(16) float sm[];
-    constexpr int LD = DP + kCsPad, B = 16, NB = kCsC / B;
-    float *sQ = sm, *sK = sQ + kCsC * LD, *sF = sK + kCsC * LD, *sA = sF + kCsC * LD, *sB = sA + kCsC * kCsLdA;    // sF: the tokens' decays, then value slabs
+    constexpr int LD = DP + kCsPad, B = 16, NB = kCsC / B, NT = kCsGlaThreads, FREE = kCsC * LD > 2 * kCsC * kCsLdA ? kCsC * LD : 2 * kCsC * kCsLdA;
+    float *sQ = sm, *sK = sQ + kCsC * LD, *sF = sK + kCsC * LD, *sA = sF + FREE, *sB = sA + kCsC * kCsLdA;    // sF: the tokens' decays, then two value slabs
     const int hd = blockIdx.y, tid = threadIdx.x, lane = tid & 31, w = tid >> 5, D = a.D;
     int row, len, ty, tx;
     if (!cs_find(a, blockIdx.x, row, len)) return;
     cs_thread(ty, tx);
     const float* src = a.src + (size_t)row * a.ld;
-    cs_load<DP>(sQ, LD, src + a.off_q + hd * D, a.ld, len, D, a.qscale);
-    cs_load<DP>(sK, LD, src + a.off_k + hd * D, a.ld, len, D, 1.f);
-    for (int i = tid; i < kCsC * DP; i += 256) {
+    cs_load<DP, NT>(sQ, LD, src + a.off_q + hd * D, a.ld, len, D, a.qscale);
+    cs_load<DP, NT>(sK, LD, src + a.off_k + hd * D, a.ld, len, D, 1.f);
+    for (int i = tid; i < kCsC * DP; i += NT) {
         const int t = i / DP, d = i % DP;
         float f = 1.f;
         if (t < len && d < D) {         // alpha = sigmoid(z)^(1/tau), as the token-serial kernel evaluates it
@@ -304,51 +309,64 @@ static __global__ void __launch_bounds__(256) ly_chunk_gla_kernel(ChunkArgs a) {
         }
         sF[t * LD + d] = f;
     }
-    for (int i = tid; i < kCsC * kCsLdA; i += 256) sA[i] = 0.f;
+    for (int i = tid; i < kCsC * kCsLdA; i += NT) sA[i] = 0.f;
     __syncthreads();
-    // diagonal blocks: a warp takes a key, its lanes four channels each
-    for (int j = w; j < kCsC; j += 8) {
+    // diagonal blocks: a warp takes a key, its lanes four channels each; the sums over the lanes for all of the block's queries at once
+    for (int j = w; j < kCsC; j += NT / 32) {
         const bool on = lane * 4 < DP;
         const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
         float4 p = on ? *reinterpret_cast<const float4*>(sK + j * LD + lane * 4) : zero;
-        for (int i = j; i < (j / B + 1) * B; ++i) {
-            float s = 0.f;
-            if (on) {
+        const int b0 = j / B * B;
+        float s[B];
+#pragma unroll
+        for (int e = 0; e < B; ++e) {
+            const int i = b0 + e;
+            s[e] = 0.f;
+            if (i >= j && on) {
                 if (i > j) {
                     const float4 f = *reinterpret_cast<const float4*>(sF + i * LD + lane * 4);
                     p.x *= f.x; p.y *= f.y; p.z *= f.z; p.w *= f.w;
                 }
                 const float4 q = *reinterpret_cast<const float4*>(sQ + i * LD + lane * 4);
-                s = fmaf(q.x, p.x, fmaf(q.y, p.y, fmaf(q.z, p.z, q.w * p.w)));
+                s[e] = fmaf(q.x, p.x, fmaf(q.y, p.y, fmaf(q.z, p.z, q.w * p.w)));
             }
-            s = warp_sum(s);
-            if (lane == 0) sA[i * kCsLdA + j] = s;
         }
+#pragma unroll
+        for (int o = 16, n = B / 2; n > 0; o >>= 1, n >>= 1)        // a lane keeps half of its sums, sends the other half: sum lane / 2 is left
+#pragma unroll
+            for (int e = 0; e < n; ++e) {
+                const bool up = lane & o;
+                const float keep = up ? s[e + n] : s[e], send = up ? s[e] : s[e + n];
+                s[e] = keep + __shfl_xor_sync(0xFFFFFFFFu, send, o);
+            }
+        const float t = s[0] + __shfl_xor_sync(0xFFFFFFFFu, s[0], 1);
+        if ((lane & 1) == 0 && b0 + lane / 2 >= j) sA[(b0 + lane / 2) * kCsLdA + j] = t;
     }
     __syncthreads();
     // queries decayed from their block's start, keys to their block's end, the blocks' whole decays
-    for (int d = tid; d < 2 * DP; d += 256) {
-        if (d < DP) {
-            for (int b = 0; b < NB; ++b) {
-                float run = 1.f;
-                for (int i = b * B; i < (b + 1) * B; ++i) { run *= sF[i * LD + d]; sQ[i * LD + d] *= run; }
-                sB[b * DP + d] = run;
-            }
+    for (int r = tid; r < 2 * NB * DP; r += NT) {
+        const int d = r % DP, b = r / DP % NB;
+        float f[B], x[B];
+        float* v = (r < NB * DP ? sQ : sK) + b * B * LD + d;
+#pragma unroll
+        for (int i = 0; i < B; ++i) { f[i] = sF[(b * B + i) * LD + d]; x[i] = v[i * LD]; }
+        float run = 1.f;
+        if (r < NB * DP) {
+#pragma unroll
+            for (int i = 0; i < B; ++i) { run *= f[i]; v[i * LD] = x[i] * run; }
+            sB[b * DP + d] = run;
         } else {
-            const int c = d - DP;
-            for (int b = 0; b < NB; ++b) {
-                float run = 1.f;
-                for (int i = (b + 1) * B - 1; i >= b * B; --i) { sK[i * LD + c] *= run; run *= sF[i * LD + c]; }
-            }
+#pragma unroll
+            for (int i = B - 1; i >= 0; --i) { v[i * LD] = x[i] * run; run *= f[i]; }
         }
     }
     __syncthreads();
 #pragma unroll 1
     for (int b = 1; b <= NB; ++b) {     // keys of the blocks before b, decayed to the end of block b - 1
-        for (int i = tid; i < (b - 1) * B * DP; i += 256) sK[i / DP * LD + i % DP] *= sB[(b - 1) * DP + i % DP];
+        for (int i = tid; i < (b - 1) * B * DP; i += NT) sK[i / DP * LD + i % DP] *= sB[(b - 1) * DP + i % DP];
         __syncthreads();
         if (b == NB) break;
-        for (int p = tid; p < B * b * B; p += 256) {        // 16 queries x 16 b keys; a warp: 8 keys x 4 queries
+        for (int p = tid; p < B * b * B; p += NT) {        // 16 queries x 16 b keys; a warp: 8 keys x 4 queries
             const int i = b * B + (p / 32 % 4) * 4 + (p & 3), j = p / 128 * 8 + (p >> 2 & 7);
             float s = 0.f;
 #pragma unroll 4
@@ -361,23 +379,26 @@ static __global__ void __launch_bounds__(256) ly_chunk_gla_kernel(ChunkArgs a) {
         __syncthreads();
     }
     // queries decayed from the chunk's start, for the part that the starting state adds
-    for (int i = tid; i < kCsC * DP; i += 256) {
+    for (int i = tid; i < kCsC * DP; i += NT) {
         const int t = i / DP, d = i % DP;
         if (t >= len || d >= D) continue;
         float q = sQ[t * LD + d];
         for (int b = 0; b < t / B; ++b) q *= sB[b * DP + d];
         a.qd[(size_t)(row + t) * a.H * D + hd * D + d] = q;
     }
-    for (int d = tid; d < D; d += 256) {
+    for (int d = tid; d < D; d += NT) {
         float p = 1.f;
         for (int b = 0; b < NB; ++b) p *= sB[b * DP + d];
         a.dec[((size_t)blockIdx.x * a.H + hd) * D + d] = p;
     }
     float* us = a.us + ((size_t)blockIdx.x * a.H + hd) * D * a.Dv;
-    for (int v0 = 0; v0 < a.Dv; v0 += kCsSlab) {
-        cs_load_slab(sF, src + a.off_v + hd * a.Dv, a.ld, len, v0, a.Dv, nullptr);
+    const int half = tid >> 8;
+    float* sV = sF + half * kCsC * kCsLdA;
+    for (int vb = 0; vb < a.Dv; vb += 2 * kCsSlab) {
+        const int v0 = vb + half * kCsSlab;
+        if (v0 < a.Dv) cs_load_slab(sV, src + a.off_v + hd * a.Dv, a.ld, len, v0, a.Dv, nullptr);
         __syncthreads();
-        cs_slab_products<DP>(a, sA, sK, LD, sF, row, len, hd, v0, 0.f, us, ty, tx, nullptr);
+        if (v0 < a.Dv) cs_slab_products<DP>(a, sA, sK, LD, sV, row, len, hd, v0, 0.f, us, ty, tx, nullptr);
         __syncthreads();
     }
 }

@@ -1161,7 +1161,7 @@ static ChunkScratch chunk_scratch(Recurrence kind, int H, int D, int Dv, const C
 template <int DP>
 static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurrence kind, const int* counts, int n) {
     constexpr size_t row = DP + kCsPad, tile = kCsC * row, sq = kCsC * kCsLdA;
-    constexpr size_t sm_in = (2 * tile + sq) * 4, sm_gla = (3 * tile + sq + kCsC / 16 * DP) * 4, sm_delta = (2 * tile + 2 * sq) * 4;
+    constexpr size_t sm_in = (2 * tile + sq) * 4, sm_gla = cs_gla_smem<DP>(), sm_delta = (2 * tile + 2 * sq) * 4;
     constexpr size_t sm_dstate = (DP * (kCsCols + kCsPad) + 2 * (2 * tile + kCsC * (kCsCols + kCsPad) + kCsC)) * 4;
     constexpr size_t sm_out = (tile + DP * kCsLdA) * 4, sm_out2 = sm_out + 2 * sq * 4;
     static bool attr_set = false;
@@ -1192,7 +1192,7 @@ static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurr
             continue;
         }
         const bool gla = kind == Recurrence::gla;
-        if (gla) launch(lc, "gla_chunks", 0, ly_chunk_gla_kernel<DP>, grid, b, sm_gla, a);
+        if (gla) launch(lc, "gla_chunks", 0, ly_chunk_gla_kernel<DP>, grid, dim3(kCsGlaThreads), sm_gla, a);
         else if (a.H / a.G % 4 == 0) launch(lc, "ssm_chunks", 0, ly_chunk_in_kernel<DP, 4>, dim3(chunks, a.H / 4), b, sm_in, a);
         else launch(lc, "ssm_chunks", 0, ly_chunk_in_kernel<DP, 1>, grid, b, sm_in, a);
         launch(lc, gla ? "gla_states" : "ssm_states", 0, ly_chunk_state_kernel, dim3((unsigned)((per / 4 + 255) / 256), n), b, 0, a, gla ? 1 : 0);

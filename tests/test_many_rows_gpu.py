@@ -107,6 +107,19 @@ def test_token_by_token_in_any_cut(kind, dim, vdim):
     assert np.array_equal(whole, mod.run_cut(model, toks, [1, 2, 3, 4, 5, 12, 14], cache=model.new_device_cache(2, 64)))
 
 
+# the first lengths that go in chunks (64 tokens of gated linear attention, 256 of the others), a token more, a last chunk of one token to 63
+@pytest.mark.parametrize("kind,n", [("gla", 64), ("gla", 65), ("gla", 127), ("gla_fast_decay", 191), ("mamba", 256), ("mamba", 257), ("delta", 256), ("delta", 319)])
+@pytest.mark.parametrize("dim,vdim", [(128, 128), (68, 132), (16, 20)])
+def test_first_lengths_in_chunks(kind, n, dim, vdim):
+    """against portions of 60 tokens, which no recurrence takes in chunks"""
+    mod, cfg = recurrent(kind, dim, vdim)
+    _, model = mod.build(cfg, seed=81, dtype="bf16")
+    toks = mod.tokens(cfg, n, seed=82)
+    serial = mod.run_cut(model, toks, [60] * 6, cache=model.new_device_cache(2, 512))
+    whole = mod.run_whole(model, toks, cache=model.new_device_cache(2, 512))
+    assert mod.relerr(whole, np.asarray(serial, dtype=np.float64)) < CHUNK_TOL
+
+
 @pytest.mark.parametrize("kind", ["gla", "mamba", "delta"])
 def test_chunks_of_several_sequences(kind):
     """two prompts of more chunks than are held at a time beside a short one and a decoded token; a reused slot starts from zero"""
