@@ -39,7 +39,7 @@ struct BertModel {
     PinnedBuf<uint32_t> h_ids;
     PinnedBuf<float> h_out;
     PinnedBuf<int> failed;                  // one word: a wait inside a kernel ran out
-    DevBuf<uint16_t> small_pack;            // the matrices as the one-launch kernel's blocks take them (23 MB; made when the model is finalized)
+    uint16_t* small_pack = nullptr;         // in the slab: the matrices as that kernel's blocks take them (23 MB; made when the model is finalized)
     void* small_layers = nullptr;           // in the slab: the layers' pointers for the one-launch kernel (null: other sizes than it is built for)
     ~BertModel();
 };

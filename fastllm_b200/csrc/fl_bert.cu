@@ -140,10 +140,10 @@ void bert_build(BertModel& m) {
         l.l1w = take(H * 4); l.l1b = take(H * 4); l.l2w = take(H * 4); l.l2b = take(H * 4);
     }
     const bool small = m.H == kBsH && m.I == kBsI && m.nh == kBsHeads;
-    const size_t o_small = small ? take(m.L * sizeof(BertSmallLayer)) : 0;
+    const size_t o_small = small ? take(m.L * sizeof(BertSmallLayer)) : 0, o_pack = small ? take((size_t)m.L * kBsCluster * kBsPack * 2) : 0;
     m.slab.alloc(off, true);
     uint8_t* b = m.slab.p;
-    if (small) m.small_layers = b + o_small;
+    if (small) { m.small_layers = b + o_small; m.small_pack = (uint16_t*)(b + o_pack); }
     m.wemb = (uint16_t*)(b + o_w); m.pemb = (uint16_t*)(b + o_p); m.lnw = (float*)(b + o_lw); m.lnb = (float*)(b + o_lb);
     m.layers.resize(m.L);
     for (int i = 0; i < m.L; ++i) {
@@ -279,9 +279,8 @@ void bert_finalize(BertModel& m) {
     }
     if (m.small_layers != nullptr) {
         std::vector<BertSmallLayer> tab;
-        m.small_pack.alloc(m.layers.size() * kBsCluster * kBsPack);
         for (const BertLayerW& w : m.layers) {
-            uint16_t* pack = m.small_pack.p + tab.size() * kBsCluster * kBsPack;
+            uint16_t* pack = m.small_pack + tab.size() * kBsCluster * kBsPack;
             bert_small_pack_kernel<<<dim3(32, kBsCluster), 256>>>(w.wqkv, w.wo, w.wi, w.wo2, pack);
             g_launches.fetch_add(1);
             tab.push_back({pack, w.bqkv, w.bo, w.bi, w.bo2, w.ln1w, w.ln1b, w.ln2w, w.ln2b});
