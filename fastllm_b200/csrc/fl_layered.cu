@@ -847,6 +847,8 @@ static bool ff_in_fused(int R, int F, int K, int act, bool tc_in, bool tc_out, b
 // experts' results there (run_rows: the experts' runs in a step of more than 128 rows).
 // A new cache's first step of 2048 rows through three 4096 x 14336 layers takes 937 instead of 1694 MB and, with the scratch of its portions
 // reserved up front (reserve_portions), 15.1 instead of 16.9 ms.
+// rows of the experts' runs: whole 128-row tiles per expert that any row picked
+static size_t run_capacity(size_t picks, size_t experts) { return 128 * (picks / 128 + std::min(picks, experts)); }
 struct FfScratch { size_t gu = 0, act = 0, eo = 0, sh_gu = 0, sh_act = 0, sh_o = 0; };
 static FfScratch ff_scratch(const LayeredModel& m, size_t R, size_t run_rows) {
     FfScratch s;
@@ -867,7 +869,13 @@ static FfScratch ff_scratch(const LayeredModel& m, size_t R, size_t run_rows) {
         } else if (d.ffn == FL_FFN_MOE) {
             const size_t P = R * d.top;
             if (!lw.tc_moe) { up(s.gu, P * GF); up(s.act, P * F); up(s.eo, P * W); }
-            else { up(s.eo, run_rows * W); if (d.ffn_act == FL_ACT_RELU2) up(s.gu, run_rows * F); }
+            else {
+                for (size_t T = 129; T <= R; ++T) {         // (a step of fewer rows may be cut along K more often)
+                    const int picks = (int)T * d.top;
+                    up(s.eo, runs_ksplit(picks, d.experts, m.W, d.ff) * run_capacity(picks, d.experts) * W);
+                }
+                if (d.ffn_act == FL_ACT_RELU2) up(s.gu, run_rows * F);
+            }
             if (d.shared_ff > 0 && !m.cfg.parallel_sub) {
                 up(s.sh_gu, unfused(d.shared_ff, d.ffn_act, lw.tc_sgu, lw.tc_sdown) * 2 * Fs);
                 if (!lw.tc_sdown) up(s.sh_act, R * Fs);
@@ -886,8 +894,7 @@ static void ensure_ws(fl_cache& c, size_t T, size_t n_want) {
         FL_CUDA(cudaStreamSynchronize(c.stream));
         drop_graphs(c);
         const size_t R = std::max<size_t>(T, 2 * y.rows), W = m.W, P = R * std::max(m.max_top, 1);
-        // rows of the experts' runs in a step of many rows (whole 128-row tiles per expert that any row picked)
-        const size_t run_rows = R > 128 && m.max_experts > 0 ? 128 * (P / 128 + std::min<size_t>(P, m.max_experts)) : 0;
+        const size_t run_rows = R > 128 && m.max_experts > 0 ? run_capacity(P, m.max_experts) : 0;
         y.x.alloc(R * W); y.h.alloc(R * W); y.y.alloc(R * W);
         y.proj.alloc(R * m.max_in); y.u.alloc(R * std::max(m.max_u, 1)); y.go.alloc(R * std::max(m.max_hv, 1));
         y.la.alloc(R * std::max(m.max_hd, 1));
@@ -1916,21 +1923,22 @@ static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const in
             sh = y.sh_o.p;
         }
         const dim3 gw((W + 255) / 256, Ti);
-        auto combine = [&] {            // the picked rows of eo, weighted, and the shared expert
+        auto combine = [&](int nsl, size_t stride) {            // the picked rows of eo (its slices added), weighted, and the shared expert
             if (W % 4 == 0)
-                launch(lc, "moe_combine", 0, ly_moe_combine_kernel<4>, dim3((W + 1023) / 1024, Ti), dim3(256), 0, (const float*)y.eo.p, (const int*)y.pair_of.p,
+                launch(lc, "moe_combine", 0, ly_moe_combine_kernel<4>, dim3((W + 1023) / 1024, Ti), dim3(256), 0, (const float*)y.eo.p, nsl, stride, (const int*)y.pair_of.p,
                        (const float*)y.route_w.p, top, sh, sg, W, out);
             else
-                launch(lc, "moe_combine", 0, ly_moe_combine_kernel<1>, gw, dim3(256), 0, (const float*)y.eo.p, (const int*)y.pair_of.p, (const float*)y.route_w.p, top,
-                       sh, sg, W, out);
+                launch(lc, "moe_combine", 0, ly_moe_combine_kernel<1>, gw, dim3(256), 0, (const float*)y.eo.p, nsl, stride, (const int*)y.pair_of.p,
+                       (const float*)y.route_w.p, top, sh, sg, W, out);
         };
         if (lw.tc_moe && Ti > 128) {
             // many rows: each expert's rows gathered into a run of whole 128-row tiles, ONE grouped GEMM pair over all runs.  (Every expert over
             // all rows, kept where picked, did E / top times the work: 1531 tokens, 8 experts of 5632, top 2, two layers: 5.43 -> 3.02 ms for the
             // whole prefill; 340 rows of 2816-wide experts: 2.37 -> 1.41 ms.)
-            const size_t cap = 128 * ((size_t)P / 128 + std::min(P, E));
+            const size_t cap = run_capacity(P, E);
             const RowRuns runs{E, y.tile_off.p};
-            room(y.eo, cap * W); room(y.gu, act == FL_ACT_RELU2 ? cap * F : 0); room(y.gx_lo, cap * W); room(y.ga_lo, cap * F);
+            const int kso = runs_ksplit(P, E, W, F);
+            room(y.eo, kso * cap * W); room(y.gu, act == FL_ACT_RELU2 ? cap * F : 0); room(y.gx_lo, cap * W); room(y.ga_lo, cap * F);
             launch(lc, "moe_lists", 0, ly_moe_lists_kernel, dim3(E), dim3(256), 0, (const int*)y.route_sel.p, Ti, top, E, y.grp_off.p, y.pair_row.p,
                    y.pair_of.p);
             launch(lc, "moe_gather", 0, ly_moe_gather_runs_kernel, dim3(P), dim3(256), 0, (const uint16_t*)hhi, (const uint16_t*)hlo, W, (const int*)y.route_sel.p, top, E,
@@ -1942,8 +1950,8 @@ static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const in
                 launch(lc, "glu", 0, ly_relu2_runs_kernel, dim3((F + 1023) / 1024, (unsigned)(cap / 128)), dim3(256), 0, (const float*)y.gu.p, F, E, (const int*)y.tile_off.p,
                        y.ga_hi.p, y.ga_lo.p);
             }
-            dense_gemm_runs(c, lc, "gemm_tc_moe_out", (int)cap, W, F, lw.tm_down, y.eo.p, y.ga_hi.p, y.ga_lo.p, runs);
-            combine();
+            dense_gemm_runs(c, lc, "gemm_tc_moe_out", (int)cap, W, F, lw.tm_down, y.eo.p, y.ga_hi.p, y.ga_lo.p, runs, kso);
+            combine(kso, cap * W);
         } else {
             launch(lc, "moe_lists", 0, ly_moe_lists_kernel, dim3(E), dim3(256), 0, (const int*)y.route_sel.p, Ti, top, E, y.grp_off.p, y.pair_row.p,
                    y.pair_of.p);
@@ -1968,7 +1976,7 @@ static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const in
                 launch_glu(lc, Slices{y.gu.p, 1, 0}, P, F, d.limit, act, nullptr, y.act.p, nullptr, nullptr);
                 LyGemm g2{y.act.p, 0, F, nullptr, lw.w_down, (long long)W * F, W, F, y.eo.p, 0, W, y.grp_off.p, P};
                 gemm_groups(lc, "gemm_moe_out", g2, E, P);
-                combine();
+                combine(1, 0);
             }
         }
     };

@@ -425,7 +425,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             }
             pdl_wait();
             asm volatile("fence.proxy.async;" ::: "memory");      // the previous kernel's generic-proxy stores -> TMA reads
-            const int ntiles = runs ? g.tile_off[g.groups] * nt : nitems;
+            const int ntiles = runs ? g.tile_off[g.groups] * nt * ksplit : nitems;
             uint32_t c = 0;
             for (int item = blockIdx.x; item < ntiles; item += gridDim.x) {
                 const int tile = item / ksplit, ks = item % ksplit;
@@ -466,7 +466,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
             constexpr uint32_t idesc = umma_idesc_bf16(kGemmBM, kMmaN);
             uint32_t c = 0, ti = 0;
             if (grouped || runs) pdl_wait();      // grp_cnt / tile_off is written by a preceding kernel
-            const int ntiles = runs ? g.tile_off[g.groups] * nt : nitems;
+            const int ntiles = runs ? g.tile_off[g.groups] * nt * ksplit : nitems;
             for (int item = blockIdx.x; item < ntiles; item += gridDim.x) {
                 if (grouped && g.grp_cnt[(item / ksplit) / mt_e] == 0) continue;
                 const uint32_t ti_now = ti++;
@@ -501,7 +501,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ 
         const int cslice = (warp - 2) >> 2;
         uint32_t ti = 0;
         if (grouped || runs) pdl_wait();          // grp_cnt / tile_off is written by a preceding kernel
-        const int ntiles = runs ? g.tile_off[g.groups] * nt : nitems;
+        const int ntiles = runs ? g.tile_off[g.groups] * nt * ksplit : nitems;
         for (int item = blockIdx.x; item < ntiles; item += gridDim.x) {
             const int tile = item / ksplit, ksi = item % ksplit;
             int m0, n0, grp, mrow0;

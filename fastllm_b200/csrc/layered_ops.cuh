@@ -2693,7 +2693,7 @@ static __global__ void __launch_bounds__(256) ly_relu2_runs_kernel(const float* 
 // y[row, c] = sum_k wt[row, k] * eo[pair_of[row, k], c]  (pick order)  + sgate[row] * sh[row, c];  V channels per thread (V = 4: W a multiple
 // of 4).  grid (channel blocks of 256 V, rows)
 template <int V>
-static __global__ void __launch_bounds__(256) ly_moe_combine_kernel(const float* __restrict__ eo, const int* __restrict__ pair_of, const float* __restrict__ wt, int top,
+static __global__ void __launch_bounds__(256) ly_moe_combine_kernel(const float* __restrict__ eo, int nsl, size_t sl_stride, const int* __restrict__ pair_of, const float* __restrict__ wt, int top,
                                                                     const float* __restrict__ sh, const float* __restrict__ sgate, int W, float* __restrict__ y) {
     pdl_chain();
     const int row = blockIdx.y, c = (blockIdx.x * 256 + threadIdx.x) * V;
@@ -2701,7 +2701,14 @@ static __global__ void __launch_bounds__(256) ly_moe_combine_kernel(const float*
     float t[V] = {}, v[V];
     for (int k = 0; k < top; ++k) {
         const float wk = wt[row * top + k];
-        ld_vec<V>(eo + (size_t)pair_of[row * top + k] * W + c, v);
+        const float* p = eo + (size_t)pair_of[row * top + k] * W + c;
+        ld_vec<V>(p, v);
+        for (int s = 1; s < nsl; ++s) {
+            float x[V];
+            ld_vec<V>(p + s * sl_stride, x);
+#pragma unroll
+            for (int i = 0; i < V; ++i) v[i] += x[i];
+        }
 #pragma unroll
         for (int i = 0; i < V; ++i) t[i] = fmaf(wk, v[i], t[i]);
     }

@@ -52,6 +52,13 @@ def test_rows_that_are_not_numbers(n):
     assert np.isfinite(got[n:n + min(64, n - 20)]).all()
 
 
+# expert results of one to four slices of K (hidden widths of 8 to 44 k blocks), k blocks that do not go evenly into them
+@pytest.mark.parametrize("n,ff,experts", [(129, 520, 5), (129, 1030 * 2, 8), (300, 1536, 3), (140, 2824, 2)])
+def test_expert_results_in_slices(n, ff, experts):
+    cfg = N.config([N.gla(heads=2, dim=16, vdim=16, mlp=N.moe(ff=ff, experts=experts, top=2))], vocab=64, width=64)
+    check(N, cfg, n, 37, 0.0)
+
+
 @pytest.mark.parametrize("n,ff", [(129, 24), (260, 136)])
 def test_expert_runs_without_a_gate(n, ff):
     check(T, T.config([T.layer(mlp=T.moe(experts=8, top=2, ff=ff))], width=64), n, 33)
