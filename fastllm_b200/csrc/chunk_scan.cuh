@@ -11,11 +11,11 @@
 // own factors (each <= 1: nothing is divided and nothing can overflow).
 //   1. ly_chunk_in_kernel / ly_chunk_gla_kernel / ly_chunk_delta_kernel   one block per (chunk, head): everything that needs no state
 //   2. ly_chunk_state_kernel / ly_chunk_delta_state_kernel                 the states at the chunks' starts, chunk by chunk
-//   3. ly_chunk_out_kernel                                                 one block per (chunk, head): what the starting state adds
+//   3. ly_chunk_out_kernel / ly_chunk_out_heads_kernel                     one block per (chunk, head): what the starting state adds
 // Bound: 1 and 3 by latency -- operands in shared memory, 4 x 4 results per thread (64 FMA per 8 16-byte loads), 16 warps per SM:
 // at 1024 tokens ncu has the FMA pipe at 31 to 34 %, issue slots at 45 to 47 %, shared memory at 47 to 50 %.  2: HBM.
 // Measured per layer, token by token -> chunks: gated linear attention, 1531 tokens, 16 heads of 128 x 128: 1160 -> 180 us; Mamba-2, 2048
-// tokens, 128 heads of 128 x 64: 1186 -> 668 us (four heads per block: their scores are multiplied once); delta rule, 2048 tokens, 32 heads of 128 x 128: 1022 -> 626 us; lightning attention, 333
+// tokens, 128 heads of 128 x 64: 1186 -> 440 us (four heads per block: their scores are multiplied once); delta rule, 2048 tokens, 32 heads of 128 x 128: 1022 -> 626 us; lightning attention, 333
 // tokens, 16 heads: 246 -> 65 us.  Same model, same tokens: the logits agree to 1e-5 .. 4e-5, their error against 64 bits is unchanged.
 #pragma once
 #include "layered_ops.cuh"
@@ -145,10 +145,9 @@ __device__ __forceinline__ void cs_load_slab(float* dst, const float* src, int l
         *reinterpret_cast<float4*>(dst + r * kCsLdA + c) = v;
     }
 }
-// o (rows [0, len) of the head, columns [v0, v0 + 64)) = A V (+ dskip v);  us [D][Dv] = K^T V, V's rows times `rows` first (nullptr: as they are)
+// o (rows [0, len) of the head, columns [v0, v0 + 64)) = A V;  us [D][Dv] = K^T V
 template <int DP>
-__device__ __forceinline__ void cs_slab_products(const ChunkArgs& a, const float* sA, const float* sK, int ldk, float* sV, int row, int len, int hd, int v0, float dsk,
-                                                 float* us, int ty, int tx, const float* rows) {
+__device__ __forceinline__ void cs_slab_products(const ChunkArgs& a, const float* sA, const float* sK, int ldk, const float* sV, int row, int len, int hd, int v0, float* us, int ty, int tx) {
     float acc[4][4];
     cs_zero(acc);
     cs_mm_nn<kCsC>(acc, sA, kCsLdA, sV, kCsLdA, ty, tx);
@@ -157,19 +156,8 @@ __device__ __forceinline__ void cs_slab_products(const ChunkArgs& a, const float
 #pragma unroll
         for (int r = 0; r < 4; ++r) {
             const int i = ty + 16 * r;
-            if (i >= len) continue;
-            float4 v = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
-            if (dsk != 0.f) {
-                const float4 x = *reinterpret_cast<const float4*>(a.src + (size_t)(row + i) * a.ld + a.off_v + hd * a.Dv + col);
-                v.x = fmaf(dsk, x.x, v.x); v.y = fmaf(dsk, x.y, v.y); v.z = fmaf(dsk, x.z, v.z); v.w = fmaf(dsk, x.w, v.w);
-            }
-            *reinterpret_cast<float4*>(a.o + (size_t)(row + i) * a.H * a.Dv + hd * a.Dv + col) = v;
+            if (i < len) *reinterpret_cast<float4*>(a.o + (size_t)(row + i) * a.H * a.Dv + hd * a.Dv + col) = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
         }
-    }
-    if (rows != nullptr) {
-        __syncthreads();
-        for (int i = threadIdx.x; i < kCsC * kCsSlab; i += 256) sV[i / kCsSlab * kCsLdA + i % kCsSlab] *= rows[i / kCsSlab];
-        __syncthreads();
     }
 #pragma unroll 1
     for (int m0 = 0; m0 < DP; m0 += 64) {
@@ -190,9 +178,7 @@ struct CsDecay {
     float whole;
 };
 // between two barriers of the caller: sa is there before, the tables are there behind the next one
-__device__ __forceinline__ void cs_decay_tables(CsDecay& d) {
-    const int t = threadIdx.x;
-    if (t >= kCsC) return;
+__device__ __forceinline__ void cs_decay_tables(CsDecay& d, int t) {       // t: token of the thread
     const int b0 = t & ~15;
     float p = 1.f, q = 1.f, e = 1.f;
     for (int i = b0; i <= t; ++i) p *= d.sa[i];
@@ -228,15 +214,20 @@ __device__ __forceinline__ void cs_decay_factors(float (&f)[4][4], const CsDecay
 }
 
 // ---- lightning attention, Mamba-2: one decay per head and token ---------------------------------------------------------------------
-// HB neighbouring heads that read the same q and k (Mamba-2's groups) share a block: their scores differ by the decays alone.
+// HB neighbouring heads that read the same q and k (Mamba-2's groups) share a block: their scores differ by the decays alone.  The decays' products of all
+// of them are made at the start; a head's values (a slab of 64 columns at a time) are on their way while the slab before is multiplied.
+// (Heads one after the other, each with its tables, its loads and two passes over its values: 338 -> 233 us for 2048 tokens of 128 heads of 128 x 64,
+// four heads a block; 34 -> 26 for 333 tokens of 16 heads of 128 x 128.)
+template <int DP>
+constexpr size_t cs_in_smem() { return ((size_t)(kCsC * (DP + kCsPad) > 2 * kCsC * kCsLdA ? kCsC * (DP + kCsPad) : 2 * kCsC * kCsLdA) + kCsC * (DP + kCsPad) + kCsC * kCsLdA) * 4; }
 template <int DP, int HB>
 static __global__ void __launch_bounds__(256, 2) ly_chunk_in_kernel(ChunkArgs a) {
     pdl_chain();
     extern __shared__ __align__(16) float sm[];
-    constexpr int LD = DP + kCsPad;
-    float *sQ = sm, *sK = sQ + kCsC * LD, *sA = sK + kCsC * LD;        // the value slab takes the queries' place once they are used
-    __shared__ CsDecay dec;
-    __shared__ float sb[kCsC];
+    constexpr int LD = DP + kCsPad, FREE = kCsC * LD > 2 * kCsC * kCsLdA ? kCsC * LD : 2 * kCsC * kCsLdA, B = 16;
+    float *sQ = sm, *sK = sQ + FREE, *sA = sK + kCsC * LD;             // two value slabs take the queries' place once they are used
+    __shared__ CsDecay dec[HB];
+    __shared__ float sb[HB][kCsC], sw[HB][kCsC], sin[HB][kCsC][B];       // strength, strength x decay to the chunk's end, decays inside a 16-token block: [to][from]
     const int h0 = blockIdx.y * HB, g = h0 / (a.H / a.G), tid = threadIdx.x;
     int row, len, ty, tx;
     if (!cs_find(a, blockIdx.x, row, len)) return;
@@ -244,38 +235,115 @@ static __global__ void __launch_bounds__(256, 2) ly_chunk_in_kernel(ChunkArgs a)
     const float* src = a.src + (size_t)row * a.ld;
     cs_load<DP>(sQ, LD, src + a.off_q + g * a.D, a.ld, len, a.D, 1.f);
     cs_load<DP>(sK, LD, src + a.off_k + g * a.D, a.ld, len, a.D, 1.f);
+    const int th = tid / kCsC, tt = tid % kCsC;         // the tables: a head per 64 threads
+    if (th < HB) {
+        const float2 v = tt < len ? *reinterpret_cast<const float2*>(a.ab + ((size_t)(row + tt) * a.H + h0 + th) * 2) : make_float2(1.f, 0.f);
+        dec[th].sa[tt] = v.x;
+        sb[th][tt] = v.y;
+    }
     __syncthreads();
+    if (th < HB) {
+        cs_decay_tables(dec[th], tt);
+        sw[th][tt] = sb[th][tt] * dec[th].end[tt];
+        if (tt == 0) a.dec[(size_t)blockIdx.x * a.H + h0 + th] = dec[th].whole;
+        float f[B], p = 1.f;
+#pragma unroll
+        for (int j = 0; j < B; ++j) f[j] = dec[th].sa[(tt & ~15) + j];
+#pragma unroll
+        for (int j = B - 1; j >= 0; --j) {
+            sin[th][tt][j] = j <= (tt & 15) ? p : 0.f;
+            if (j <= (tt & 15)) p *= f[j];
+        }
+    }
     float qk[4][4];
     cs_zero(qk);
     cs_mm_nt<DP>(qk, sQ, LD, sK, LD, ty, tx);
-#pragma unroll 1
-    for (int hd = h0; hd < h0 + HB; ++hd) {
-        __syncthreads();                // everybody is done with the head before
-        if (tid < kCsC) {
-            const float2 v = tid < len ? *reinterpret_cast<const float2*>(a.ab + ((size_t)(row + tid) * a.H + hd) * 2) : make_float2(1.f, 0.f);
-            dec.sa[tid] = v.x;
-            sb[tid] = v.y;
+    __syncthreads();                    // the queries are done with, the tables are there
+    const int slabs = (a.Dv + kCsSlab - 1) / kCsSlab, items = HB * slabs;
+    auto bring = [&](int item) {        // values of rows behind the portion and of columns behind the head are zero
+        float* dst = sQ + (item & 1) * kCsC * kCsLdA;
+        const float* v = src + a.off_v + (h0 + item / slabs) * a.Dv;
+        const int v0 = item % slabs * kCsSlab;
+        for (int i = tid; i < kCsC * (kCsSlab / 4); i += 256) {
+            const int r = i / (kCsSlab / 4), c = i % (kCsSlab / 4) * 4;
+            if (r < len && v0 + c < a.Dv) cp_async16(dst + r * kCsLdA + c, v + (size_t)r * a.ld + v0 + c);
+            else *reinterpret_cast<float4*>(dst + r * kCsLdA + c) = make_float4(0.f, 0.f, 0.f, 0.f);
         }
-        __syncthreads();
-        cs_decay_tables(dec);
-        __syncthreads();
-        {
-            float f[4][4];
-            cs_decay_factors(f, dec, ty, tx, true);
+        cp_async_commit();
+    };
+    bring(0);
+#pragma unroll 1
+    for (int item = 0; item < items; ++item) {
+        const int hh = item / slabs, hd = h0 + hh, v0 = item % slabs * kCsSlab;
+        if (item + 1 < items) bring(item + 1);
+        else cp_async_commit();
+        if (v0 == 0) {                  // scores of the head: decayed, times the keys' strengths
+            const CsDecay& d = dec[hh];
+            float blk[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) blk[k] = d.pre[16 * k + 15];
 #pragma unroll
             for (int r = 0; r < 4; ++r)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) sA[(ty + 16 * r) * kCsLdA + tx + 16 * c] = qk[r][c] * f[r][c];
+                for (int c = 0; c < 4; ++c) {
+                    float f = 0.f;
+                    if (c == r) f = sin[hh][16 * r + ty][tx];
+                    if (c < r) {
+                        f = d.pre[16 * r + ty] * d.suf[16 * c + tx];
+#pragma unroll
+                        for (int k = 1; k < 3; ++k)
+                            if (k > c && k < r) f *= blk[k];
+                    }
+                    sA[(ty + 16 * r) * kCsLdA + tx + 16 * c] = qk[r][c] * f * sb[hh][tx + 16 * c];
+                }
         }
-        if (tid == 0) a.dec[(size_t)blockIdx.x * a.H + hd] = dec.whole;
+        cp_async_wait<1>();
+        __syncthreads();
+        const float* sV = sQ + (item & 1) * kCsC * kCsLdA;
         const float dsk = a.dskip ? a.dskip[hd] : 0.f;
         float* us = a.us + ((size_t)blockIdx.x * a.H + hd) * a.D * a.Dv;
-        for (int v0 = 0; v0 < a.Dv; v0 += kCsSlab) {
-            if (v0 > 0) __syncthreads();
-            cs_load_slab(sQ, src + a.off_v + hd * a.Dv, a.ld, len, v0, a.Dv, sb);
-            __syncthreads();
-            cs_slab_products<DP>(a, sA, sK, LD, sQ, row, len, hd, v0, dsk, us, ty, tx, dec.end);
+        const int col = v0 + 4 * tx;
+        {
+            float acc[4][4];
+            cs_zero(acc);
+            cs_mm_nn<kCsC>(acc, sA, kCsLdA, sV, kCsLdA, ty, tx);
+            if (col < a.Dv) {
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int i = ty + 16 * r;
+                    if (i >= len) continue;
+                    const float4 x = *reinterpret_cast<const float4*>(sV + i * kCsLdA + 4 * tx);
+                    *reinterpret_cast<float4*>(a.o + (size_t)(row + i) * a.H * a.Dv + hd * a.Dv + col) =
+                        dsk != 0.f ? make_float4(fmaf(dsk, x.x, acc[r][0]), fmaf(dsk, x.y, acc[r][1]), fmaf(dsk, x.z, acc[r][2]), fmaf(dsk, x.w, acc[r][3]))
+                                   : make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
+                }
+            }
         }
+        {   // what the chunk adds to the state: K^T (strength x decay x V), all key channels in one walk over the tokens
+            constexpr int MB = DP / 64;
+            float acc[MB][4][4];
+#pragma unroll
+            for (int m = 0; m < MB; ++m) cs_zero(acc[m]);
+#pragma unroll 4
+            for (int k = 0; k < kCsC; ++k) {
+                const float s = sw[hh][k];
+                float4 y = *reinterpret_cast<const float4*>(sV + k * kCsLdA + 4 * tx);
+                y.x *= s; y.y *= s; y.z *= s; y.w *= s;
+#pragma unroll
+                for (int m = 0; m < MB; ++m) {
+                    const float4 x = *reinterpret_cast<const float4*>(sK + k * LD + 64 * m + 4 * ty);
+                    cs_fma4(acc[m][0], x.x, y); cs_fma4(acc[m][1], x.y, y); cs_fma4(acc[m][2], x.z, y); cs_fma4(acc[m][3], x.w, y);
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < MB; ++m)
+#pragma unroll
+                for (int r = 0; r < 4; ++r) {
+                    const int d = 64 * m + 4 * ty + r;
+                    if (d < a.D && col < a.Dv) *reinterpret_cast<float4*>(us + (size_t)d * a.Dv + col) = make_float4(acc[m][r][0], acc[m][r][1], acc[m][r][2], acc[m][r][3]);
+                }
+        }
+        __syncthreads();                // the slab and the scores have been read
     }
 }
 
@@ -398,7 +466,7 @@ static __global__ void __launch_bounds__(kCsGlaThreads, 1) ly_chunk_gla_kernel(C
         const int v0 = vb + half * kCsSlab;
         if (v0 < a.Dv) cs_load_slab(sV, src + a.off_v + hd * a.Dv, a.ld, len, v0, a.Dv, nullptr);
         __syncthreads();
-        if (v0 < a.Dv) cs_slab_products<DP>(a, sA, sK, LD, sV, row, len, hd, v0, 0.f, us, ty, tx, nullptr);
+        if (v0 < a.Dv) cs_slab_products<DP>(a, sA, sK, LD, sV, row, len, hd, v0, us, ty, tx);
         __syncthreads();
     }
 }
@@ -439,8 +507,76 @@ static __global__ void __launch_bounds__(256) ly_chunk_state_kernel(ChunkArgs a,
 }
 
 // ---- what the starting state adds: o += (decayed q) S ----------------------------------------------------------------------------------
-// MODE 0: one decay per head (q from src, decayed here); 1: gated linear attention (q from qd); 2: delta rule -- o holds u on entry,
-// o = A u + (decayed q) S with A from aq.
+// One decay per head, HB heads of a block that read the same q: their states (64 columns at a time) and what o holds are on their way while the ones
+// before are multiplied: 206 -> 152 us for 2048 tokens of 128 heads of
+// 128 x 64, four heads a block.
+template <int DP>
+constexpr size_t cs_out_smem() { return ((size_t)kCsC * (DP + kCsPad) + 2 * DP * kCsLdA) * 4; }
+template <int DP, int HB>
+static __global__ void __launch_bounds__(256, 2) ly_chunk_out_heads_kernel(ChunkArgs a) {
+    pdl_chain();
+    extern __shared__ __align__(16) float sm[];
+    constexpr int LD = DP + kCsPad;
+    float *sQ = sm, *sS = sQ + kCsC * LD;               // two state slabs
+    __shared__ float sa[HB][kCsC], pre[HB][kCsC], sp[HB][kCsC];          // decays; their products from the start of 16 tokens, of the chunk
+    const int h0 = blockIdx.y * HB, g = h0 / (a.H / a.G), tid = threadIdx.x;
+    int row, len, ty, tx;
+    if (!cs_find(a, blockIdx.x, row, len)) return;
+    cs_thread(ty, tx);
+    const int slabs = (a.Dv + kCsSlab - 1) / kCsSlab, items = HB * slabs;
+    auto bring = [&](int item) {
+        float* dst = sS + (item & 1) * DP * kCsLdA;
+        const float* S = a.us + ((size_t)blockIdx.x * a.H + h0 + item / slabs) * a.D * a.Dv;
+        const int v0 = item % slabs * kCsSlab;
+        for (int i = tid; i < DP * (kCsSlab / 4); i += 256) {
+            const int d = i / (kCsSlab / 4), c = i % (kCsSlab / 4) * 4;
+            if (d < a.D && v0 + c < a.Dv) cp_async16(dst + d * kCsLdA + c, S + (size_t)d * a.Dv + v0 + c);
+            else *reinterpret_cast<float4*>(dst + d * kCsLdA + c) = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+        cp_async_commit();
+    };
+    bring(0);
+    cs_load<DP>(sQ, LD, a.src + (size_t)row * a.ld + a.off_q + g * a.D, a.ld, len, a.D, 1.f);
+    const int th = tid / kCsC, tt = tid % kCsC;
+    if (th < HB) sa[th][tt] = tt < len ? a.ab[((size_t)(row + tt) * a.H + h0 + th) * 2] : 1.f;
+    __syncthreads();
+    if (th < HB) {
+        float p = 1.f;
+        for (int i = tt & ~15; i <= tt; ++i) p *= sa[th][i];
+        pre[th][tt] = p;
+    }
+    __syncthreads();
+    if (th < HB) {
+        float p = pre[th][tt];
+        for (int k = 0; k < tt / 16; ++k) p *= pre[th][16 * k + 15];
+        sp[th][tt] = p;
+    }
+#pragma unroll 1
+    for (int item = 0; item < items; ++item) {
+        const int hh = item / slabs, col = item % slabs * kCsSlab + 4 * tx;
+        float* op = a.o + (size_t)row * a.H * a.Dv + (h0 + hh) * a.Dv + col;
+        if (item + 1 < items) bring(item + 1);
+        else cp_async_commit();
+        float4 x[4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) x[r] = col < a.Dv && ty + 16 * r < len ? *reinterpret_cast<const float4*>(op + (size_t)(ty + 16 * r) * a.H * a.Dv) : make_float4(0.f, 0.f, 0.f, 0.f);
+        cp_async_wait<1>();
+        __syncthreads();
+        float acc[4][4];
+        cs_zero(acc);
+        cs_mm_nn<DP>(acc, sQ, LD, sS + (item & 1) * DP * kCsLdA, kCsLdA, ty, tx);
+        if (col < a.Dv) {
+#pragma unroll
+            for (int r = 0; r < 4; ++r) {
+                const int i = ty + 16 * r;
+                const float p = sp[hh][i];
+                if (i < len) *reinterpret_cast<float4*>(op + (size_t)i * a.H * a.Dv) = make_float4(acc[r][0] * p + x[r].x, acc[r][1] * p + x[r].y, acc[r][2] * p + x[r].z, acc[r][3] * p + x[r].w);
+            }
+        }
+        __syncthreads();                // the slab has been read
+    }
+}
+// MODE 1: gated linear attention (q from qd); 2: delta rule (q from src, decayed here) -- o holds u on entry, o = A u + (decayed q) S with A from aq.
 template <int DP, int MODE>
 static __global__ void __launch_bounds__(256, 2) ly_chunk_out_kernel(ChunkArgs a) {
     pdl_chain();
@@ -483,7 +619,7 @@ static __global__ void __launch_bounds__(256, 2) ly_chunk_out_kernel(ChunkArgs a
         float acc[4][4];
         cs_zero(acc);
         cs_mm_nn<DP>(acc, sQ, LD, sS, kCsLdA, ty, tx);
-        if (MODE != 1) {
+        if (MODE == 2) {
 #pragma unroll
             for (int r = 0; r < 4; ++r) {
                 const float p = sp[ty + 16 * r];
@@ -500,7 +636,7 @@ static __global__ void __launch_bounds__(256, 2) ly_chunk_out_kernel(ChunkArgs a
                 if (i >= len) continue;
                 float4* op = reinterpret_cast<float4*>(a.o + (size_t)(row + i) * a.H * a.Dv + hd * a.Dv + col);
                 float4 v = make_float4(acc[r][0], acc[r][1], acc[r][2], acc[r][3]);
-                if (MODE != 2) { const float4 x = *op; v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w; }
+                if (MODE == 1) { const float4 x = *op; v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w; }
                 *op = v;
             }
         }
@@ -531,7 +667,7 @@ static __global__ void __launch_bounds__(256) ly_chunk_delta_kernel(ChunkArgs a)
         sb[tid] = tid < len ? a.ab[((size_t)(row + tid) * a.H + hd) * 2 + 1] : 0.f;
     }
     __syncthreads();
-    cs_decay_tables(dec);
+    if (tid < kCsC) cs_decay_tables(dec, tid);
     for (int i = tid; i < kCsC * kCsLdA; i += 256) sT[i] = 0.f;
     float acc[4][4], kk[4][4], f[4][4];
     cs_zero(acc);

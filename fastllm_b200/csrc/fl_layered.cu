@@ -1168,7 +1168,7 @@ static ChunkScratch chunk_scratch(Recurrence kind, int H, int D, int Dv, const C
 template <int DP>
 static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurrence kind, const int* counts, int n) {
     constexpr size_t row = DP + kCsPad, tile = kCsC * row, sq = kCsC * kCsLdA;
-    constexpr size_t sm_in = (2 * tile + sq) * 4, sm_gla = cs_gla_smem<DP>(), sm_delta = (2 * tile + 2 * sq) * 4;
+    constexpr size_t sm_in = cs_in_smem<DP>(), sm_gla = cs_gla_smem<DP>(), sm_delta = (2 * tile + 2 * sq) * 4;
     constexpr size_t sm_dstate = (DP * (kCsCols + kCsPad) + 2 * (2 * tile + kCsC * (kCsCols + kCsPad) + kCsC)) * 4;
     constexpr size_t sm_out = (tile + DP * kCsLdA) * 4, sm_out2 = sm_out + 2 * sq * 4;
     static bool attr_set = false;
@@ -1176,7 +1176,7 @@ static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurr
         auto room = [](auto kern, size_t smem) { FL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem)); };
         room(ly_chunk_in_kernel<DP, 1>, sm_in); room(ly_chunk_in_kernel<DP, 4>, sm_in); room(ly_chunk_gla_kernel<DP>, sm_gla); room(ly_chunk_delta_kernel<DP>, sm_delta);
         room(ly_chunk_delta_state_kernel<DP>, sm_dstate);
-        room(ly_chunk_out_kernel<DP, 0>, sm_out); room(ly_chunk_out_kernel<DP, 1>, sm_out); room(ly_chunk_out_kernel<DP, 2>, sm_out2);
+        room(ly_chunk_out_heads_kernel<DP, 1>, cs_out_smem<DP>()); room(ly_chunk_out_heads_kernel<DP, 4>, cs_out_smem<DP>()); room(ly_chunk_out_kernel<DP, 1>, sm_out); room(ly_chunk_out_kernel<DP, 2>, sm_out2);
         attr_set = true;
     }
     const ChunkPlan pl = chunk_plan(kind, counts, n);
@@ -1204,7 +1204,9 @@ static void launch_chunks_dp(LayeredCache& y, LaunchCtx& lc, ChunkArgs a, Recurr
         else launch(lc, "ssm_chunks", 0, ly_chunk_in_kernel<DP, 1>, grid, b, sm_in, a);
         launch(lc, gla ? "gla_states" : "ssm_states", 0, ly_chunk_state_kernel, dim3((unsigned)((per / 4 + 255) / 256), n), b, 0, a, gla ? 1 : 0);
         if (gla) launch(lc, "gla_chunks_out", 0, ly_chunk_out_kernel<DP, 1>, grid, b, sm_out, a);
-        else launch(lc, "ssm_chunks_out", 0, ly_chunk_out_kernel<DP, 0>, grid, b, sm_out, a);
+        // (four heads a block where that still gives every SM one: 327 tokens of 64 heads, 96 blocks, whole prompt 711 -> 725 us)
+        else if (a.H / a.G % 4 == 0 && chunks * (a.H / 4) >= kNumSMs) launch(lc, "ssm_chunks_out", 0, ly_chunk_out_heads_kernel<DP, 4>, dim3(chunks, a.H / 4), b, cs_out_smem<DP>(), a);
+        else launch(lc, "ssm_chunks_out", 0, ly_chunk_out_heads_kernel<DP, 1>, grid, b, cs_out_smem<DP>(), a);
     }
 }
 // -> whether the token-serial kernel has sequences left
