@@ -5,13 +5,13 @@
 // Two CTAs of a cluster take two groups of whole sentences of up to 128 rows each (tcgen05.mma.cta_group::2, see gemm_pair.cuh: a single CTA would read
 // every weight from L2 for 128 tokens, 18 TB/s at the tensor cores' rate).  A unit of work is up to three heads of such a pair: 288 columns of q|k|v in TMEM,
 // rounded into shared memory by twelve warps, which then are the attention's (mma.sync, a sentence's 16 query rows of a head at a time) while the tensor
-// core makes the next unit's columns.  The clusters take equal runs of units; x stays in shared memory over the units of a pair.
+// core makes the next unit's columns.  The clusters take equal runs of heads; x stays in shared memory over the units of a pair.
 // q, k and v never leave the SM: the GEMM and the attention moved 75 MB each way between them at 256 x 128 tokens.
-// Whole encoder, GEMM and attention -> this kernel, us (with the block kernel as it is): 256 x 128 tokens 1280 -> 1087, 76 x 128 572 -> 564, 500 x 64 1360 ->
-// 1035, 1500 x 20 1690 -> 1170, 3000 x 8 2150 -> 1300, 60 x 43 378 -> 356; a layer of 256 x 128: 87 -> 64.  A unit of 128-token sentences takes about 14500
-// clocks: 2200 to bring q|k|v into shared memory, 12000 of attention in which the tensor core's 3700 for the next unit run -- the warps' products (3300),
-// ex2 (3100) and shared memory (3300 and the operands of the other products) would overlap better with more warps than the registers allow (eight warps
-// of 168 registers: 17800; two row tiles a warp and an online softmax: no gain).
+// Whole encoder, GEMM and attention -> this kernel, us (with the block kernel as it is): 256 x 128 tokens 1280 -> 1087, 76 x 128 552 -> 511, 400 x 43 788 ->
+// 649, 1500 x 20 1690 -> 1170, 3000 x 8 2150 -> 1300, 60 x 43 378 -> 368; a layer of 256 x 128: 87 -> 64.  (Runs of whole units of three heads: 76 x 128 567.)
+// A unit of 128-token sentences takes about 14500 clocks: 2200 to bring q|k|v into shared memory, 12000 of attention in which the tensor core's 3700 for
+// the next unit run -- the warps' products (3300), ex2 (3100) and shared memory (3300 and the operands of the other products) would overlap better with
+// more warps than the registers allow (eight warps of 168 registers: 17800; two row tiles a warp and an online softmax: no gain).
 #pragma once
 #include "bert.cuh"
 #include "bert_block.cuh"
@@ -27,7 +27,6 @@ static_assert(kBqAllHeads * kBertD == kBbH && kBqSmem <= 232448, "");
 
 struct BertQkvArgs {
     int b, t, spc;              // sentences, tokens of each, sentences per CTA: 128 / t
-    int hpu;                    // heads per unit: 1, 2 or 3
     const float* bias;          // [1152]
     float qscale;               // log2(e) / sqrt(d)
     uint16_t* ctx;              // [b t, 384]
@@ -175,8 +174,10 @@ bert_qkv_attn_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     const int warp = uniform_warp(), lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
     const int cl = blockIdx.x >> 1, G = gridDim.x >> 1;
-    const int groups = (g.b + g.spc - 1) / g.spc, upp = kBqAllHeads / g.hpu, units = (groups + 1) / 2 * upp;        // units per pair
-    const int u0 = (int)((long long)units * cl / G), u1 = (int)((long long)units * (cl + 1) / G);
+    const int groups = (g.b + g.spc - 1) / g.spc, heads = (groups + 1) / 2 * kBqAllHeads;      // of all pairs, in a row
+    const int h0 = (int)((long long)heads * cl / G), h1 = (int)((long long)heads * (cl + 1) / G);
+    // the unit that begins at a head: how many heads
+    auto unit = [&](int h) { return min(kBqHeads, min(h1 - h, kBqAllHeads - h % kBqAllHeads)); };
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {
@@ -204,55 +205,57 @@ bert_qkv_attn_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             int st = 0;
             uint32_t ph = 1;
             // stage i of a unit: two k blocks of its heads' rows of q (i < 3), k, v (48 rows whatever the heads: the box's; what lies behind is not used)
-            auto stage = [&](int unit, int i) {
+            auto stage = [&](int h, int n, int i) {
                 if (!ok || !(ok = pair_wait(&w_empty[st], ph))) return;
                 if (rank == 0) mbar_expect_tx(&w_full[st], 2 * kBqStage);
                 const uint32_t bar = mapa_u32(smem_u32(&w_full[st]), 0), sa = smem_u32(sW) + st * kBqStage;
-                const int row = i / 3 * kBbH + (unit % upp * 2 + (int)rank) * g.hpu * (kBertD / 2);
+                const int row = i / 3 * kBbH + h % kBqAllHeads * kBertD + (int)rank * n * (kBertD / 2);
 #pragma unroll
                 for (int k = 0; k < 2; ++k) tma_load_2d_pair(sa + k * kBqPart, &tmW, (i % 3 * 2 + k) * 64, row, bar);
                 if (++st == kBqStages) { st = 0; ph ^= 1; }
             };
             int tiles = 0;
-            for (int u = u0; ok && u < u1; ++u) {
+            for (int h = h0, n; ok && h < h1; h += n) {
+                n = unit(h);
                 int first = 0;
-                if (u == u0) {                      // the first ring of weights does not wait for the kernels before
-                    for (; first < kBqStages; ++first) stage(u, first);
+                if (h == h0) {                      // the first ring of weights does not wait for the kernels before
+                    for (; first < kBqStages; ++first) stage(h, n, first);
                     pdl_wait();
                     asm volatile("fence.proxy.async;" ::: "memory");
                 }
-                if (u == u0 || u % upp == 0) {
+                if (h == h0 || h % kBqAllHeads == 0) {
                     if (tiles > 0 && !(ok = pair_wait(&x_free, (tiles - 1) & 1))) break;
-                    const int row = (u / upp * 2 + (int)rank) * g.spc * g.t;
+                    const int row = (h / kBqAllHeads * 2 + (int)rank) * g.spc * g.t;
                     for (int k = 0; k < kBbKb; ++k) {       // (the products start with the first two blocks)
                         if (rank == 0 && k % 2 == 0) mbar_expect_tx(&x_full[k / 2], 4 * 16384);
                         tma_load_2d_pair(smem_u32(sX) + k * 16384, &tmX, k * 64, row, mapa_u32(smem_u32(&x_full[k / 2]), 0));
                     }
                     ++tiles;
                 }
-                for (; first < 9; ++first) stage(u, first);
+                for (; first < 9; ++first) stage(h, n, first);
             }
         }
     } else if (warp == 1) {
         if (rank == 0) {             // (the whole warp, see uniform_warp; a wait that ran out ends the waiting, not the walk)
-            const uint32_t idesc = umma_idesc_bf16(256, g.hpu * kBertD);
             const uint64_t dX = umma_smem_desc_sw128(sX), dW = umma_smem_desc_sw128(sW);
-            uint32_t n = 0;                         // stages so far
-            int tiles = 0;
+            uint32_t c = 0;                         // stages so far
+            int tiles = 0, units = 0;
             auto wait = [&](uint64_t* bar, uint32_t parity) {
                 if (ok) ok = pair_wait(bar, parity);
                 __syncwarp();
                 tc_fence_after();
             };
-            for (int u = u0; u < u1; ++u) {
-                wait(&acc_free, ((u - u0) & 1) ^ 1);
-                const bool fresh = u == u0 || u % upp == 0;
+            for (int h = h0, n; h < h1; h += n, ++units) {
+                n = unit(h);
+                const uint32_t idesc = umma_idesc_bf16(256, n * kBertD);
+                wait(&acc_free, (units & 1) ^ 1);
+                const bool fresh = h == h0 || h % kBqAllHeads == 0;
 #pragma unroll 1
-                for (int i = 0; i < 9; ++i, ++n) {
+                for (int i = 0; i < 9; ++i, ++c) {
                     if (fresh && i < 3) wait(&x_full[i], tiles & 1);
-                    const uint32_t st = n % kBqStages, col = i / 3 * kBqCols;
+                    const uint32_t st = c % kBqStages, col = i / 3 * kBqCols;
                     const uint64_t a = dX + (uint64_t)(i % 3 * 2048), b = dW + (uint64_t)(st * (kBqStage >> 4));
-                    wait(&w_full[st], (n / kBqStages) & 1);
+                    wait(&w_full[st], (c / kBqStages) & 1);
 #pragma unroll
                     for (int k = 0; k < 2; ++k)
 #pragma unroll
@@ -262,7 +265,7 @@ bert_qkv_attn_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
                 }
                 umma_commit_pair_warp(&acc_full);
                 tiles += fresh;
-                if (u + 1 < u1 && (u + 1) % upp == 0) umma_commit_pair_warp(&x_free);
+                if (h + n < h1 && (h + n) % kBqAllHeads == 0) umma_commit_pair_warp(&x_free);
             }
         }
     } else {
@@ -274,10 +277,11 @@ bert_qkv_attn_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
         for (int i = threadIdx.x - 64; i < 3 * kBbH; i += 32 * kBqWarps) sB[i] = g.bias[i];
         esync();
         pdl_wait();
-        for (int u = u0; u < u1; ++u) {             // (to the end even behind a wait that ran out: the warps meet at barriers)
-            if (ok) ok = __all_sync(0xFFFFFFFFu, pair_wait(&acc_full, (u - u0) & 1));
+        for (int hd = h0, n, units = 0; hd < h1; hd += n, ++units) {             // (to the end even behind a wait that ran out: the warps meet at barriers)
+            n = unit(hd);
+            if (ok) ok = __all_sync(0xFFFFFFFFu, pair_wait(&acc_full, units & 1));
             tc_fence_after();
-            const int head0 = u % upp * g.hpu;
+            const int head0 = hd % kBqAllHeads;
             uint8_t* dst = reinterpret_cast<uint8_t*>(sQ + lrow * kBqLd + part * kBqCols);
             const float* bias = sB + part * kBbH + head0 * kBertD;
             uint32_t v[kBqHeads][32];
@@ -287,7 +291,7 @@ bert_qkv_attn_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             for (int c = 0; c < kBqHeads; ++c) tmem_arrived32(v[c]);
 #pragma unroll
             for (int c = 0; c < kBqHeads; ++c) {
-                if (c >= g.hpu) continue;           // (a unit of fewer heads)
+                if (c >= n) continue;           // (a unit of fewer heads)
 #pragma unroll
                 for (int j = 0; j < 32; j += 8) {
                     const float4 x = *reinterpret_cast<const float4*>(bias + c * 32 + j), y = *reinterpret_cast<const float4*>(bias + c * 32 + j + 4);
@@ -301,11 +305,11 @@ bert_qkv_attn_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             __syncwarp();
             if (lane == 0) mbar_arrive_cluster_relaxed(mapa_u32(smem_u32(&acc_free), 0));      // (loaded into registers: no memory changes hands)
             esync();                                // q, k, v of three heads are there
-            const int grp = u / upp * 2 + (int)rank, ns = min(g.spc, g.b - grp * g.spc);
+            const int grp = hd / kBqAllHeads * 2 + (int)rank, ns = min(g.spc, g.b - grp * g.spc);
             uint16_t* ctx = g.ctx + (size_t)grp * g.spc * g.t * kBbH + head0 * kBertD;
             // (a rejected wait leaves nothing to store)
-            for (int it = aw; ok && it < ns * mts * g.hpu; it += kBqWarps) {
-                const int h = it % g.hpu, s = it / g.hpu / mts, m0 = it / g.hpu % mts * 16;
+            for (int it = aw; ok && it < ns * mts * n; it += kBqWarps) {
+                const int h = it % n, s = it / n / mts, m0 = it / n % mts * 16;
                 uint16_t *row = sQ + s * g.t * kBqLd + h * kBertD, *to = ctx + (size_t)s * g.t * kBbH + h * kBertD;
                 auto go = [&](auto kt) { bq_attention<decltype(kt)::value, kBqLd>(row, row + kBqCols, row + 2 * kBqCols, g.t, m0, g.qscale, to, lane); };
                 switch (mts) {

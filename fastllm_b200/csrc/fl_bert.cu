@@ -314,7 +314,19 @@ static int bert_qkv_clusters() {
     static const int n = pairs_resident(bert_qkv_attn_kernel, kBqThreads, kBqSmem);
     return n;
 }
-static bool bert_qkv_attn(const BertModel& m, int t) { return m.H == kBbH && m.nh == kBsHeads && t <= kBertS && bert_qkv_clusters() > 0; }
+// pairs of groups of whole sentences, up to 128 rows a group
+static int bert_qkv_pairs(int b, int t) {
+    const int spc = kBertS / t;
+    return ((b + spc - 1) / spc + 1) / 2;
+}
+// One kernel for q|k|v and the attention, GEMM and attention kernel where most rows of its tiles would be padding and its heads go round badly: a group is
+// one sentence from 65 tokens on, and four heads a pair of SMs are two units.  Whole encoder, us, two kernels -> one: 38 / 46 x 65 359 -> 371, 371 -> 386,
+// 38 x 75 369 -> 383, but 36 x 65 (three heads a pair) 363 -> 362, 50 x 65 (five) 406 -> 392, 38 x 85 404 -> 396, 38 x 128 463 -> 439.
+static bool bert_qkv_attn(const BertModel& m, int b, int t) {
+    if (m.H != kBbH || m.nh != kBsHeads || t > kBertS || bert_qkv_clusters() == 0) return false;
+    const int heads = (bert_qkv_pairs(b, t) * kBqAllHeads + bert_qkv_clusters() - 1) / bert_qkv_clusters();
+    return !(t > kBertS / 2 && t <= 5 * kBertS / 8 && heads == 4);
+}
 // A pair of SMs takes about as long for 256 tokens however many tiles there are, the chain's kernels grow with the tokens, in steps of their own waves.
 // Whole encoder, chain -> blocks, us, by tiles of 256 tokens (128-token sentences; 64 and 512 tokens a sentence cross at the same places): 28 506 -> 506,
 // 32 526 -> 522, 36 544 -> 532, 38 658 -> 550, 44 688 -> 576, 64 853 -> 674, 74 914 -> 702; two waves: 75 1034 -> 1036, 80 1070 -> 1058,
@@ -401,18 +413,9 @@ static void launch_bert_block(BertModel& m, const CUtensorMap& tm_ctx, const CUt
     const BertBlockArgs a{T, m.x.p, w.bo, w.bi, w.bo2, w.ln1w, w.ln1b, w.ln2w, w.ln2b, eps, m.failed.p};
     blaunch(m.stream, bert_block_kernel, dim3(2 * std::min((T + 255) / 256, bert_block_clusters())), dim3(kBbThreads), kBbSmem, tm_ctx, w.tb_wo, w.tb_wi, w.tb_wo2, tm_x, a);
 }
-// Heads per unit: units go round the resident pairs in whole numbers, and one costs about 0.7 of a head whatever its heads (37 x 127 tokens: 19 pairs, 76
-// units of three heads for 74 clusters 449 us, 114 of two 430; 256 x 128: three; 4 x 128: one, 307 -> 302).
 static void launch_bert_qkv(BertModel& m, const CUtensorMap& tm_x, const BertLayerW& w, int b, int t, float scale) {
-    const int spc = kBertS / t, pairs = ((b + spc - 1) / spc + 1) / 2, G = bert_qkv_clusters();
-    int hpu = kBqHeads;
-    double best = 1e30;
-    for (int h = kBqHeads; h >= 1; --h) {
-        const double cost = ((pairs * (kBqAllHeads / h) + G - 1) / G) * (0.7 + h);
-        if (cost < best) { best = cost; hpu = h; }
-    }
-    const BertQkvArgs a{b, t, spc, hpu, w.bqkv, 1.4426950408889634f / scale, m.ctx.p, m.failed.p};
-    blaunch(m.stream, bert_qkv_attn_kernel, dim3(2 * std::min(pairs * (kBqAllHeads / hpu), G)), dim3(kBqThreads), kBqSmem, tm_x, w.tb_wqkv, a);
+    const BertQkvArgs a{b, t, kBertS / t, w.bqkv, 1.4426950408889634f / scale, m.ctx.p, m.failed.p};
+    blaunch(m.stream, bert_qkv_attn_kernel, dim3(2 * std::min(bert_qkv_pairs(b, t) * kBqAllHeads, bert_qkv_clusters())), dim3(kBqThreads), kBqSmem, tm_x, w.tb_wqkv, a);
 }
 static void bert_check(const BertModel& m) {
     FL_CHECK(*m.failed.p == 0, FL_ERR_CUDA, "a wait inside a kernel ran out, the results are not valid");
@@ -430,7 +433,7 @@ static void bert_enqueue(BertModel& m, const BertRun& run, int b, int t, bool ha
     const dim3 row_grid((T + rows_per_cta - 1) / rows_per_cta), row_block(rows_per_cta * 32);
     blaunch(st, embed_ln_kernel, row_grid, row_block, 0, (const uint16_t*)m.wemb, (const uint16_t*)m.pemb, (const float*)m.lnw, (const float*)m.lnb,
             (const uint32_t*)m.ids.p, T, t, H, m.V, m.maxpos, 1e-12f, m.x.p);
-    const bool blocks = run.path == BertPath::blocks, qkv_attn = bert_qkv_attn(m, t);
+    const bool blocks = run.path == BertPath::blocks, qkv_attn = bert_qkv_attn(m, b, t);
     const CUtensorMap tm_x = make_tmap_bf16(m.x.p, T, H, H, kGemmBM), tm_x1 = blocks ? tm_x : make_tmap_bf16(m.x1.p, T, H, H, kGemmBM),
                       tm_ctx = make_tmap_bf16(m.ctx.p, T, H, H, kGemmBM);
     const CUtensorMap tm_h = blocks ? tm_x : make_tmap_bf16(m.hbuf.p, T, I, I, kGemmBM);
