@@ -328,13 +328,13 @@ static bool bert_qkv_attn(const BertModel& m, int b, int t) {
     return !(t > kBertS / 2 && t <= 5 * kBertS / 8 && heads == 4);
 }
 // A pair of SMs takes about as long for 256 tokens however many tiles there are, the chain's kernels grow with the tokens, in steps of their own waves.
-// Whole encoder, chain -> blocks, us, by tiles of 256 tokens (128-token sentences; 64 and 512 tokens a sentence cross at the same places): 28 506 -> 506,
-// 32 526 -> 522, 36 544 -> 532, 38 658 -> 550, 44 688 -> 576, 64 853 -> 674, 74 914 -> 702; two waves: 75 1034 -> 1036, 80 1070 -> 1058,
-// 88 1146 -> 1097, 128 1607 -> 1283.  Up to half a wave the two are within 2 % of each other; behind it, and in every later wave, the blocks are ahead.
+// Whole encoder, chain -> blocks, us, by tiles of 256 tokens (128-token sentences): 20 451 -> 465, 24 459 -> 463, 28 513 -> 487, 32 533 -> 490, 36 558 -> 505,
+// 38 661 -> 517, 44 693 -> 535, 64 847 -> 612, 74 887 -> 629; two waves: 75 1020 -> 914, 88 1114 -> 965, 128 1519 -> 1104.  28 tiles of 64-token sentences 498 ->
+// 469, of 512 tokens 746 -> 718; 14 376 -> 414.  The line lies at three eighths of a wave, and in every later wave the blocks are ahead.
 static bool bert_blocks(const BertModel& m, int T) {
     if (m.H != kBbH || m.I != kBbI) return false;
     const int n = bert_block_clusters(), tiles = (T + 255) / 256;
-    return n > 0 && 2 * tiles >= n;
+    return n > 0 && 8 * tiles >= 3 * n;
 }
 
 // Few short sentences: the whole encoder in one launch of clusters (bert_small.cuh).

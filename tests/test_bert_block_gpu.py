@@ -31,6 +31,12 @@ def test_block_equals_chain(b, t):
     assert np.linalg.norm(got - want, axis=1).max() <= 5e-3
 
 
+@pytest.mark.parametrize("b,t", [(56, 128), (107, 67)])
+def test_fewest_tiles_of_the_block_kernel(b, t):
+    """28 tiles of 256 tokens, the last one full or with 257 rows less"""
+    test_block_equals_chain(b, t)
+
+
 def test_block_against_the_oracle():
     """norm weights between 1/2 and 3/2 and biases everywhere, so that no column may stand in another's place; sentences at the borders of the tiles"""
     cfg = obert.BertConfig(384, 12, 2, 1536, 96, 1e-12, 512)
