@@ -7,8 +7,8 @@
 // rounded into shared memory by twelve warps, which then are the attention's (mma.sync, a sentence's 16 query rows of a head at a time) while the tensor
 // core makes the next unit's columns.  The clusters take equal runs of heads; x stays in shared memory over the units of a pair.
 // q, k and v never leave the SM: the GEMM and the attention moved 75 MB each way between them at 256 x 128 tokens.
-// Whole encoder, GEMM and attention -> this kernel, us (with the block kernel as it is): 256 x 128 tokens 1280 -> 1087, 76 x 128 552 -> 511, 400 x 43 788 ->
-// 649, 1500 x 20 1690 -> 1170, 3000 x 8 2150 -> 1300, 60 x 43 378 -> 368; a layer of 256 x 128: 87 -> 64.  (Runs of whole units of three heads: 76 x 128 567.)
+// Whole encoder, GEMM and attention -> this kernel, us (with the block kernel as it is): 256 x 128 tokens 1280 -> 1102, 76 x 128 552 -> 517, 400 x 43 788 ->
+// 645, 1500 x 20 1690 -> 1177, 60 x 43 378 -> 368; a layer of 256 x 128: 87 -> 66.  (Runs of whole units of three heads: 76 x 128 567.)
 // A unit of 128-token sentences takes about 14500 clocks: 2200 to bring q|k|v into shared memory, 12000 of attention in which the tensor core's 3700 for
 // the next unit run -- the warps' products (3300), ex2 (3100) and shared memory (3300 and the operands of the other products) would overlap better with
 // more warps than the registers allow (eight warps of 168 registers: 17800; two row tiles a warp and an online softmax: no gain).
@@ -28,15 +28,15 @@ static_assert(kBqAllHeads * kBertD == kBbH && kBqSmem <= 232448, "");
 struct BertQkvArgs {
     int b, t, spc;              // sentences, tokens of each, sentences per CTA: 128 / t
     const float* bias;          // [1152]
-    float qscale;               // log2(e) / sqrt(d)
+    float inv_scale;            // 1 / sqrt(d)
     uint16_t* ctx;              // [b t, 384]
     int* failed;                // set when a wait ran out
 };
 
-// two f32 at a time: x * y + z, x + y
-__device__ __forceinline__ float2 fma_f32x2(float2 x, float2 y, float2 z) {
+// two f32 at a time: x * y, x + y
+__device__ __forceinline__ float2 mul_f32x2(float2 x, float2 y) {
     float2 d;
-    asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<const uint64_t&>(x)), "l"(reinterpret_cast<const uint64_t&>(y)), "l"(reinterpret_cast<const uint64_t&>(z)));
+    asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(reinterpret_cast<uint64_t&>(d)) : "l"(reinterpret_cast<const uint64_t&>(x)), "l"(reinterpret_cast<const uint64_t&>(y)));
     return d;
 }
 __device__ __forceinline__ float2 add_f32x2(float2 x, float2 y) {
@@ -45,10 +45,14 @@ __device__ __forceinline__ float2 add_f32x2(float2 x, float2 y) {
     return d;
 }
 // 16 query rows (m0 on) of a sentence's head: sq, sk, sv at the sentence's first row.  The rows of o take the place of the q rows that this warp alone reads.
+// Every operation on a score is bert_attn_kernel's, in its order, so that a sentence's embedding is the same to the bit whichever kernel takes it: score /
+// sqrt(d), minus the row's largest, e to that as 2^(x log2 e) (weights below 2^-126 are zero), a lane's sum a pair of neighbouring keys at a time.  (One fma
+// in front of ex2 and the sums two columns at a time: 256 x 128 tokens 1080 us instead of 1102, but weights on other sides of bf16 roundings, 1.2e-3 in an embedding.)
 // LD: elements of a row.  KT: 16-key steps of the sentence's t tokens; rows behind it read as its last one, as queries nobody uses what they give, as keys their weight is zero.
 template <int KT, int LD>
-__device__ __forceinline__ void bq_attention(uint16_t* sq, const uint16_t* sk, const uint16_t* sv, int t, int m0, float qscale, uint16_t* ctx, int lane) {
+__device__ __forceinline__ void bq_attention(uint16_t* sq, const uint16_t* sk, const uint16_t* sv, int t, int m0, float inv_scale, uint16_t* ctx, int lane) {
     const int g = lane >> 2, tq = lane & 3;
+    const float2 scale = make_float2(inv_scale, inv_scale), log2e = make_float2(1.4426950408889634f, 1.4426950408889634f);
     uint32_t qa[2][4];
     float2 s[2 * KT][2];
 #pragma unroll
@@ -74,13 +78,14 @@ __device__ __forceinline__ void bq_attention(uint16_t* sq, const uint16_t* sk, c
 #pragma unroll
         for (int u = 0; u < 2; ++u) {
             const int nt = 2 * i + u;
-            if (i + 1 == KT) {
 #pragma unroll
-                for (int e = 0; e < 4; ++e)
-                    if (nt * 8 + tq * 2 + (e & 1) >= t) c[u][e] = -INFINITY;
+            for (int h = 0; h < 2; ++h) {
+                s[nt][h] = mul_f32x2(make_float2(c[u][2 * h], c[u][2 * h + 1]), scale);
+                if (i + 1 == KT) {
+                    if (nt * 8 + tq * 2 >= t) s[nt][h].x = -INFINITY;
+                    if (nt * 8 + tq * 2 + 1 >= t) s[nt][h].y = -INFINITY;
+                }
             }
-            s[nt][0] = make_float2(c[u][0], c[u][1]);
-            s[nt][1] = make_float2(c[u][2], c[u][3]);
         }
     }
     float mx[2] = {-INFINITY, -INFINITY};
@@ -91,10 +96,10 @@ __device__ __forceinline__ void bq_attention(uint16_t* sq, const uint16_t* sk, c
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
         mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xFFFFFFFFu, mx[h], 1));
-        mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xFFFFFFFFu, mx[h], 2)) * -qscale;
+        mx[h] = fmaxf(mx[h], __shfl_xor_sync(0xFFFFFFFFu, mx[h], 2));
     }
-    const float2 qs = make_float2(qscale, qscale), b0 = make_float2(mx[0], mx[0]), b1 = make_float2(mx[1], mx[1]);
-    float2 sum[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    const float2 b0 = make_float2(-mx[0], -mx[0]), b1 = make_float2(-mx[1], -mx[1]);
+    float sum[2] = {0.f, 0.f};
     float o[4][4];
 #pragma unroll
     for (int dt = 0; dt < 4; ++dt) o[dt][0] = o[dt][1] = o[dt][2] = o[dt][3] = 0.f;
@@ -106,11 +111,11 @@ __device__ __forceinline__ void bq_attention(uint16_t* sq, const uint16_t* sk, c
         for (int d = 0; d < 2; ++d) ldmatrix_x4_trans(vb[d], sv + (ks + 1 < KT ? vr : min(vr, t - 1)) * LD + d * 16 + (lane >> 4) * 8);
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
-            float2 x = fma_f32x2(s[2 * ks + h][0], qs, b0), y = fma_f32x2(s[2 * ks + h][1], qs, b1);
+            float2 x = mul_f32x2(add_f32x2(s[2 * ks + h][0], b0), log2e), y = mul_f32x2(add_f32x2(s[2 * ks + h][1], b1), log2e);
             x.x = ex2_approx(x.x); x.y = ex2_approx(x.y);
             y.x = ex2_approx(y.x); y.y = ex2_approx(y.y);
-            sum[0] = add_f32x2(sum[0], x);
-            sum[1] = add_f32x2(sum[1], y);
+            sum[0] += x.x + x.y;
+            sum[1] += y.x + y.y;
             pa[2 * h] = pack_bf16(x.x, x.y);
             pa[2 * h + 1] = pack_bf16(y.x, y.y);
         }
@@ -123,7 +128,7 @@ __device__ __forceinline__ void bq_attention(uint16_t* sq, const uint16_t* sk, c
     float inv[2];
 #pragma unroll
     for (int h = 0; h < 2; ++h) {
-        float l = sum[h].x + sum[h].y;
+        float l = sum[h];
         l += __shfl_xor_sync(0xFFFFFFFFu, l, 1);
         l += __shfl_xor_sync(0xFFFFFFFFu, l, 2);
         inv[h] = 1.f / l;
@@ -311,7 +316,7 @@ bert_qkv_attn_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
             for (int it = aw; ok && it < ns * mts * n; it += kBqWarps) {
                 const int h = it % n, s = it / n / mts, m0 = it / n % mts * 16;
                 uint16_t *row = sQ + s * g.t * kBqLd + h * kBertD, *to = ctx + (size_t)s * g.t * kBbH + h * kBertD;
-                auto go = [&](auto kt) { bq_attention<decltype(kt)::value, kBqLd>(row, row + kBqCols, row + 2 * kBqCols, g.t, m0, g.qscale, to, lane); };
+                auto go = [&](auto kt) { bq_attention<decltype(kt)::value, kBqLd>(row, row + kBqCols, row + 2 * kBqCols, g.t, m0, g.inv_scale, to, lane); };
                 switch (mts) {
                     case 1: go(std::integral_constant<int, 1>{}); break;
                     case 2: go(std::integral_constant<int, 2>{}); break;

@@ -55,7 +55,7 @@ struct BertSmallArgs {
     const uint16_t *wemb, *pemb; const float *lnw, *lnb;
     const uint32_t *ids, *mask;             // [b t]; mask may be null
     int L, b, t, V, maxpos, spc;            // spc: sentences per cluster
-    float eps, qscale;                      // qscale: log2(e) / sqrt(d)
+    float eps, inv_scale;                   // inv_scale: 1 / sqrt(d)
     uint16_t *ctx, *h; float* pre;          // workspace rows as the launch chain has them
     int* failed;                            // set when a wait ran out
     float* out;
@@ -275,7 +275,7 @@ static __global__ void __launch_bounds__(kBsThreads, 1) bert_small_kernel(const 
             for (int it = warp; it < pairs * split; it += kBsThreads / 32) {
                 const int sent = it % pairs, m0 = it / pairs * per;
                 uint16_t *q = sqkv + sent * a.t * M::kQkvLd, *to = ctx + (size_t)sent * a.t * kBsH + rank * kBertD;
-                auto go = [&](auto kt) { bq_attention<decltype(kt)::value, M::kQkvLd>(q, q + kBertD, q + 2 * kBertD, a.t, m0, a.qscale, to, lane); };
+                auto go = [&](auto kt) { bq_attention<decltype(kt)::value, M::kQkvLd>(q, q + kBertD, q + 2 * kBertD, a.t, m0, a.inv_scale, to, lane); };
                 switch (split) {
                     case 1: go(std::integral_constant<int, 1>{}); break;
                     case 2: go(std::integral_constant<int, 2>{}); break;

@@ -399,7 +399,7 @@ static void bert_reserve(BertModel& m, const BertRun& run, int b, int t) {
 static void bert_enqueue_small(BertModel& m, const BertRun& run, int b, int t, bool has_mask) {
     const int spc = run.spc, clusters = run.clusters, rows = spc * t;
     const BertSmallArgs a{static_cast<const BertSmallLayer*>(m.small_layers), m.wemb, m.pemb, m.lnw, m.lnb, m.ids.p, has_mask ? m.mask.p : nullptr,
-                          m.L, b, t, m.V, m.maxpos, spc, m.cfg.norm_eps, 1.4426950408889634f / (float)std::sqrt((double)m.d), m.ctx.p, m.hbuf.p, m.pre.p,
+                          m.L, b, t, m.V, m.maxpos, spc, m.cfg.norm_eps, 1.f / (float)std::sqrt((double)m.d), m.ctx.p, m.hbuf.p, m.pre.p,
                           m.failed.p, m.out.p};
     switch ((rows + 15) / 16) {
         case 1: bert_small_launch<1>(m, a, clusters, false); break;
@@ -414,7 +414,7 @@ static void launch_bert_block(BertModel& m, const CUtensorMap& tm_ctx, const CUt
     blaunch(m.stream, bert_block_kernel, dim3(2 * std::min((T + 255) / 256, bert_block_clusters())), dim3(kBbThreads), kBbSmem, tm_ctx, w.tb_wo, w.tb_wi, w.tb_wo2, tm_x, a);
 }
 static void launch_bert_qkv(BertModel& m, const CUtensorMap& tm_x, const BertLayerW& w, int b, int t, float scale) {
-    const BertQkvArgs a{b, t, kBertS / t, w.bqkv, 1.4426950408889634f / scale, m.ctx.p, m.failed.p};
+    const BertQkvArgs a{b, t, kBertS / t, w.bqkv, 1.f / scale, m.ctx.p, m.failed.p};
     blaunch(m.stream, bert_qkv_attn_kernel, dim3(2 * std::min(bert_qkv_pairs(b, t) * kBqAllHeads, bert_qkv_clusters())), dim3(kBqThreads), kBqSmem, tm_x, w.tb_wqkv, a);
 }
 static void bert_check(const BertModel& m) {

@@ -1,5 +1,7 @@
 """The kernel of q|k|v and attention (bert_qkv.cuh), which sentences of up to 128 tokens take, at the edges of its groups of sentences, of its 16-row and
 16-key tiles and of its pairs of SMs, against the oracle."""
+from pathlib import Path
+
 import numpy as np
 import pytest
 
@@ -40,3 +42,13 @@ def test_sentences_do_not_see_each_other(encoder, b, t):
     after = model.embed_ids(ids)
     others = np.arange(b) != b // 2
     assert np.array_equal(after[others], before[others]) and not np.array_equal(after[b // 2], before[b // 2])
+
+
+@pytest.mark.parametrize("b,t", [(1, 64), (2, 127), (31, 43), (75, 16), (223, 5), (300, 113), (50, 70), (38, 70), (256, 128)])
+def test_same_bits_as_gemm_and_attention_kernel(encoder, b, t):
+    """golden/bert_attention_bits.npz holds what these sentences gave (first, middle, last) when the q|k|v GEMM and bert_attn_kernel took them: the kernels
+    that attend on the chip (one sentence of 64 tokens: the one-launch kernel) run every sum and every rounding in that order"""
+    cfg, _, model = encoder
+    ids = synth.token_ids(1000 + b * 131 + t, cfg.vocab_size, (b, t))
+    want = np.load(Path(__file__).parent / "golden" / "bert_attention_bits.npz")[f"{b}x{t}"]
+    assert np.array_equal(model.embed_ids(ids)[sorted({0, b // 2, b - 1})], want)
