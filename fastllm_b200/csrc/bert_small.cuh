@@ -257,7 +257,7 @@ static __global__ void __launch_bounds__(kBsThreads, 1) bert_small_kernel(const 
 #pragma unroll 1
     for (int l = 0; l < a.L; ++l) {
         const BertSmallLayer& w = a.layers[l];
-        ok = pair_wait(&front, l & 1) && ok;
+        ok = ok && pair_wait(&front, l & 1);
         __syncthreads();                    // the x tile, the layer's vectors, W_qkv and W_o are complete
         const float *ln1w = sv + (l & 1) * M::NV, *ln1b = ln1w + kBsH, *ln2w = ln1b + kBsH, *ln2b = ln2w + kBsH, *bqkv = ln2b + kBsH, *bo = bqkv + NQ * 8, *bi = bo + NO * 8,
                     *bo2 = bi + NI * 8;
@@ -314,7 +314,7 @@ static __global__ void __launch_bounds__(kBsThreads, 1) bert_small_kernel(const 
         }
         bs_wait();
         bs_layernorm(pre, rows, ln1w, ln1b, a.eps, sx, warp, lane);
-        ok = pair_wait(&wi, l & 1) && ok;
+        ok = ok && pair_wait(&wi, l & 1);
         __syncthreads();
         {
             BsTiles<MT, NI> y;
@@ -335,7 +335,7 @@ static __global__ void __launch_bounds__(kBsThreads, 1) bert_small_kernel(const 
                 bs_bring_rows<M::kHPiece>(sr + p * M::kHBuf, hb, kBsI, p * M::kHPiece, rows);
                 cp_async_commit();
             }
-            ok = pair_wait(&wo2, l & 1) && ok;
+            ok = ok && pair_wait(&wo2, l & 1);
             if constexpr (AHEAD == M::kPieces) {
                 auto piece = [&](auto at) {
                     constexpr int P = decltype(at)::value;
@@ -368,7 +368,10 @@ static __global__ void __launch_bounds__(kBsThreads, 1) bert_small_kernel(const 
         bs_wait();
         bs_layernorm(pre, rows, ln2w, ln2b, a.eps, sx, warp, lane);
     }
-    if (!ok && lane == 0 && a.failed != nullptr) *a.failed = 1;
+    if (!ok) {          // a wait ran out: report it, leave the copies in flight time to land, go on to the end
+        if (lane == 0 && a.failed != nullptr) *a.failed = 1;
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    }
     __syncthreads();
     // masked mean pooling and L2 norm: a block takes every CL-th sentence, a thread up to two columns; tot[w]: squares of columns 32 w ..
     __shared__ float tot[kBsH / 32];
