@@ -1225,6 +1225,7 @@ static void run_recurrence(fl_cache& c, LaunchCtx& lc, RecArgs ra, bool f32, con
     ca.src = ra.cv; ca.ld = ra.ldc; ca.off_q = ra.off_q; ca.off_k = ra.off_k; ca.off_v = ra.off_v; ca.ab = ra.ab; ca.dskip = ra.dskip;
     ca.o = ra.o; ca.state = ra.state; ca.seq_row0 = ra.seq_row0; ca.seq_slot = ra.seq_slot; ca.seq_pos0 = ra.seq_pos0;
     ca.n = n; ca.H = ra.H; ca.G = ra.G; ca.D = ra.D; ca.Dv = ra.Dv;
+    ra.failed = c.step_failed.p;
     constexpr Recurrence kind = DELTA ? Recurrence::delta : Recurrence::scalar;
     if (chunks_fit(ca, kind, f32, counts, n)) {
         ra.skip_from = chunk_min(kind);

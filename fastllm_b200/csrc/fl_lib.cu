@@ -1951,7 +1951,8 @@ static bool page_locked(const float* p, size_t n) {
     return true;
 }
 // The step's logits (n floats) in the caller's buffer.  Page-locked buffers (fl_host_alloc) are written by the device itself; others get them
-// through a page-locked one.  Either way nothing there changes unless the step was good.
+// through a page-locked one.  Either way nothing there changes unless the step was good -- or gave up on a copy of a block's own (the serial
+// recurrences): such a step is not waited for beforehand, its numbers may be there when the call returns the error.
 static void logits_to_host(fl_cache& c, float* host, size_t n) {
     const float* dev = c.ly ? c.ly->logits.p : c.logits.p;
     if (page_locked(host, n)) {
@@ -1961,6 +1962,7 @@ static void logits_to_host(fl_cache& c, float* host, size_t n) {
         }
         FL_CUDA(cudaMemcpyAsync(host, dev, n * 4, cudaMemcpyDeviceToHost, c.stream));
         FL_CUDA(cudaStreamSynchronize(c.stream));
+        LogitsTransfer(c, dev, host).check();
         return;
     }
     float* stage = c.ly ? c.ly->h_logits.p : c.h_logits.p;

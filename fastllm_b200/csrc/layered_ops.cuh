@@ -2123,6 +2123,7 @@ struct RecArgs {
     const int *seq_row0, *seq_slot, *seq_pos0;
     int H, G, D, Dv;
     int skip_from = 0;          // as for the gated linear attention
+    int* failed = nullptr;      // pinned host memory: set by a block whose wait ran out
 };
 constexpr int kRecCols = 32, kRecParts = 4;       // value columns per block; parts of a column's rows
 // Token by token, per head:  S <- a S;  u = b v   (DELTA: u = b (v - S^T k));  S <- S + k u^T;  o = S^T q (+ dskip v).
@@ -2155,6 +2156,12 @@ static __global__ void __launch_bounds__(160) ly_rec_scan_kernel(RecArgs a) {
     for (int i = threadIdx.x; i < NG * GT * SLOT; i += 160) sm[i] = 0.f;       // what no copy ever writes (rows >= D, columns >= Dv) reads as zero
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncthreads();
+    bool ok = true;
+    // a wait ran out: report it, leave the copies in flight time to land
+    auto give_up = [&] {
+        if (lane == 0 && a.failed != nullptr) *a.failed = 1;
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    };
 
     if (wid == 4) {
         const int nv = min(BC, Dv - v0);
@@ -2163,7 +2170,7 @@ static __global__ void __launch_bounds__(160) ly_rec_scan_kernel(RecArgs a) {
         uint32_t ph = 1;
         for (int row = r0; row < r1; row += GT) {
             const int n = min(GT, r1 - row);
-            mbar_wait(&empty[grp], ph);
+            if (!(ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&empty[grp], ph)))) break;
             if (pieces) {
                 if (lane == 0) mbar_expect_tx(&full[grp], (uint32_t)(n * (2 * D + nv) * 4));
                 __syncwarp();
@@ -2188,6 +2195,7 @@ static __global__ void __launch_bounds__(160) ly_rec_scan_kernel(RecArgs a) {
             }
             if (++grp == NG) { grp = 0; ph ^= 1; }
         }
+        if (!ok) give_up();
         return;
     }
 
@@ -2224,7 +2232,7 @@ static __global__ void __launch_bounds__(160) ly_rec_scan_kernel(RecArgs a) {
     for (int row = r0; row < r1; row += GT) {
         const float2 now = ab;
         ab = decays(row + GT);
-        mbar_wait(&full[grp], ph);
+        if (!(ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&full[grp], ph)))) break;
         float mine = 0.f;
         auto token = [&](int t) {
             const float* cur = sm + (grp * GT + t) * SLOT;
@@ -2269,7 +2277,8 @@ static __global__ void __launch_bounds__(160) ly_rec_scan_kernel(RecArgs a) {
         if (lane % LPC < GT && row + lane % LPC < r1 && vok) a.o[(size_t)(row + lane % LPC) * a.H * Dv + hd * Dv + col] = mine;
         if (++grp == NG) { grp = 0; ph ^= 1; }
     }
-    if (vok) {
+    if (!ok) give_up();
+    if (ok && vok) {
 #pragma unroll
         for (int i = 0; i < RPT; ++i) {
             const int d = at(i);

@@ -8,7 +8,8 @@ import pytest
 CSRC = Path(__file__).resolve().parent.parent / "fastllm_b200" / "csrc"
 
 
-@pytest.mark.parametrize("path,name", [("bert_small.cuh", ") bert_small_kernel"), ("bert_qkv.cuh", "\nbert_qkv_attn_kernel"), ("bert_block.cuh", "\nbert_block_kernel")])
+@pytest.mark.parametrize("path,name", [("bert_small.cuh", ") bert_small_kernel"), ("bert_qkv.cuh", "\nbert_qkv_attn_kernel"), ("bert_block.cuh", "\nbert_block_kernel"),
+                                       ("layered_ops.cuh", ") ly_rec_scan_kernel")])
 def test_a_wait_that_runs_out(path, name):
     body = (CSRC / path).read_text().split(f"{name}(", 1)[1].split("\n}\n", 1)[0]
     assert re.search(r"\bmbar_wait\(", body) is None, "a wait without a limit"
