@@ -966,14 +966,23 @@ static void launch_ly_gemm(LaunchCtx& lc, const char* tag, const LyGemm& g, int 
         launch(lc, tag, bytes, ly_gemm_kernel, dim3((g.N + kLyBN - 1) / kLyBN, (max_rows + kLyBM - 1) / kLyBM, groups), dim3(256), 0, g);
         return;
     }
-    auto go = [&](auto rows_per_tile) {
+    auto form = [&](auto rows_per_tile, auto unit) {
         constexpr int BM = decltype(rows_per_tile)::value;
+        auto kern = ly_gemm64_kernel<BM, decltype(unit)::value>;
         static bool attr_set = false;
         if (!attr_set) {
-            FL_CUDA(cudaFuncSetAttribute(ly_gemm64_kernel<BM>, cudaFuncAttributeMaxDynamicSharedMemorySize, F64Form<BM>::kSmem));
+            FL_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, F64Form<BM>::kSmem));
             attr_set = true;
         }
-        launch(lc, tag, bytes, ly_gemm64_kernel<BM>, dim3((g.N + kF64BN - 1) / kF64BN, (max_rows + BM - 1) / BM, groups), dim3(32 * kF64Sums), F64Form<BM>::kSmem, g);
+        launch(lc, tag, bytes, kern, dim3((g.N + kF64BN - 1) / kF64BN, (max_rows + BM - 1) / BM, groups), dim3(32 * kF64Sums), F64Form<BM>::kSmem, g);
+    };
+    auto go = [&](auto rows_per_tile) {
+        switch (f64_unit(g)) {
+            case 16: form(rows_per_tile, std::integral_constant<int, 16>{}); break;
+            case 8: form(rows_per_tile, std::integral_constant<int, 8>{}); break;
+            case 4: form(rows_per_tile, std::integral_constant<int, 4>{}); break;
+            default: form(rows_per_tile, std::integral_constant<int, 2>{});
+        }
     };
     // (experts share max_rows picks between them)
     const bool known = g.grp_off == nullptr;

@@ -34,12 +34,30 @@ inline int f64_rows_per_tile(double rows, int cols, int groups, bool known) {
 __device__ __forceinline__ void mma_f64_884(double (&d)[2], double a, double b) {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};" : "+d"(d[0]), "+d"(d[1]) : "d"(a), "d"(b));
 }
-// 16 bytes, of which the first `bytes` are read and the others are zero
-__device__ __forceinline__ void cp_async16_part(uint32_t smem_dst, const void* gsrc, int bytes) {
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_dst), "l"(gsrc), "r"(bytes) : "memory");
+// 16 bytes as copies of UNIT bytes (16, 8 or 4, which both addresses are multiples of): the first `bytes` are read, the others are zero
+template <int UNIT>
+__device__ __forceinline__ void cp_async_piece(uint32_t smem_dst, const void* gsrc, const void* any, int bytes) {
+#pragma unroll
+    for (int at = 0; at < 16; at += UNIT) {
+        const int n = UNIT == 16 ? bytes : max(0, min(UNIT, bytes - at));
+        const void* p = n > 0 ? static_cast<const char*>(gsrc) + at : any;
+        if (UNIT == 16) asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_dst), "l"(p), "r"(n) : "memory");
+        else if (UNIT == 8) asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(smem_dst + at), "l"(p), "r"(n) : "memory");
+        else asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(smem_dst + at), "l"(p), "r"(n) : "memory");
+    }
+}
+// Bytes that a copy of W takes at a time: what the rows' addresses are multiples of.  A's go twice as many at a time, up to 16.
+// Rows of 2-byte pieces alone (odd K) are read an element at a time, a chunk ahead of its place in the ring.  Prompts of 203 / 600 tokens, delta rule and
+// dense feed-forward, us, every row that is no multiple of 16 bytes an element at a time as it was needed -> this: width 1028 1000 -> 650, 2230 -> 1480; 1026
+// 1003 -> 720, 2240 -> 1620; 1023 1030 -> 905, 2340 -> 2060 (1024, by 16 bytes: 610, 1405).
+inline int f64_unit(const LyGemm& g) {
+    auto fits = [](const void* p, long long gs, long long row, int unit) { return ((reinterpret_cast<uintptr_t>(p) | (uintptr_t)gs | (uintptr_t)row) & (unit - 1)) == 0; };
+    for (int u = 16; u > 2; u /= 2)
+        if (fits(g.W, g.w_gs * 2, (long long)g.K * 2, u) && fits(g.A, g.a_gs * 4, (long long)g.lda * 4, std::min(16, 2 * u))) return u;
+    return 2;
 }
 
-template <int BM>
+template <int BM, int UNIT>
 static __global__ void __launch_bounds__(32 * kF64Sums, F64Form<BM>::kPerSM) ly_gemm64_kernel(LyGemm g) {
     pdl_chain();
     using F = F64Form<BM>;
@@ -54,7 +72,6 @@ static __global__ void __launch_bounds__(32 * kF64Sums, F64Form<BM>::kPerSM) ly_
     const float* A = g.A + (size_t)grp * g.a_gs;
     const uint16_t* Wm = g.W + (size_t)grp * g.w_gs;
     float* Y = g.Y + (size_t)grp * g.y_gs;
-    const bool whole = (g.lda & 3) == 0 && (g.K & 7) == 0 && ((reinterpret_cast<uintptr_t>(A) | reinterpret_cast<uintptr_t>(Wm)) & 15) == 0;
     // 16-byte pieces of a stage: piece i of A is row i / 4, columns 4 (i % 4) ..; piece i of W is row i / 2, columns 8 (i % 2) ..
     const float* arow[NA];
     const uint16_t* wrow[NB];
@@ -74,39 +91,44 @@ static __global__ void __launch_bounds__(32 * kF64Sums, F64Form<BM>::kPerSM) ly_
         if (j < mine) {
             uint8_t* s = ring + (j % kF64Ring) * F::kStage;
             const int ka = (sum + kF64Sums * j) * kF64Chunk + lane % 4 * 4, kw = (sum + kF64Sums * j) * kF64Chunk + lane % 2 * 8;
-            if (whole) {
-                const int ba = ka < g.K ? min(16, 4 * (g.K - ka)) : 0, bw = kw < g.K ? 16 : 0;
+            const int ba = ka < g.K ? (UNIT >= 8 ? 16 : 4 * min(4, g.K - ka)) : 0, bw = kw < g.K ? (UNIT == 16 ? 16 : 2 * min(8, g.K - kw)) : 0;     // (K is a multiple of UNIT / 2)
 #pragma unroll
-                for (int t = 0; t < NA; ++t) {
-                    const bool in = arow[t] != nullptr && ba > 0;
-                    cp_async16_part(smem_u32(s + (lane + 32 * t) * 16), in ? arow[t] + ka : A, in ? ba : 0);
-                }
+            for (int t = 0; t < NA; ++t) cp_async_piece<UNIT >= 8 ? 16 : 2 * UNIT>(smem_u32(s + (lane + 32 * t) * 16), arow[t] + ka, A, arow[t] != nullptr ? ba : 0);
+            if (UNIT > 2) {
 #pragma unroll
-                for (int t = 0; t < NB; ++t) {
-                    const bool in = wrow[t] != nullptr && bw > 0;
-                    cp_async16_part(smem_u32(s + BM * kF64Chunk * 4 + (lane + 32 * t) * 16), in ? wrow[t] + kw : Wm, in ? bw : 0);
-                }
-            } else {
-#pragma unroll
-                for (int t = 0; t < NA; ++t)
-                    for (int e = 0; e < 4; ++e)
-                        reinterpret_cast<float*>(s + (lane + 32 * t) * 16)[e] = arow[t] != nullptr && ka + e < g.K ? arow[t][ka + e] : 0.f;
-#pragma unroll
-                for (int t = 0; t < NB; ++t)
-                    for (int e = 0; e < 8; ++e)
-                        reinterpret_cast<uint16_t*>(s + BM * kF64Chunk * 4 + (lane + 32 * t) * 16)[e] = wrow[t] != nullptr && kw + e < g.K ? wrow[t][kw + e] : (uint16_t)0;
+                for (int t = 0; t < NB; ++t) cp_async_piece<UNIT>(smem_u32(s + BM * kF64Chunk * 4 + (lane + 32 * t) * 16), wrow[t] + kw, Wm, wrow[t] != nullptr ? bw : 0);
             }
         }
         cp_async_commit();
     };
+    // odd K: chunk j of W through registers
+    uint32_t held[NB][4];
+    auto load = [&](int j) {
+        if (UNIT > 2 || j >= mine) return;
+        const int kw = (sum + kF64Sums * j) * kF64Chunk + lane % 2 * 8;
+#pragma unroll
+        for (int t = 0; t < NB; ++t)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const uint32_t lo = wrow[t] != nullptr && kw + 2 * e < g.K ? wrow[t][kw + 2 * e] : 0u, hi = wrow[t] != nullptr && kw + 2 * e + 1 < g.K ? wrow[t][kw + 2 * e + 1] : 0u;
+                held[t][e] = lo | hi << 16;
+            }
+    };
+    auto put = [&](int j) {
+        if (UNIT > 2 || j >= mine) return;
+        uint8_t* s = ring + (j % kF64Ring) * F::kStage + BM * kF64Chunk * 4;
+#pragma unroll
+        for (int t = 0; t < NB; ++t) *reinterpret_cast<uint4*>(s + (lane + 32 * t) * 16) = make_uint4(held[t][0], held[t][1], held[t][2], held[t][3]);
+    };
     auto wide = [](uint32_t b) { return (double)__uint_as_float(b); };
     double acc[MT][NT][2] = {};
 #pragma unroll
-    for (int j = 0; j < kF64Ring - 1; ++j) fetch(j);
+    for (int j = 0; j < kF64Ring - 1; ++j) { fetch(j); load(j); put(j); }
     for (int j = 0; j < mine; ++j) {
         cp_async_wait<kF64Ring - 2>();
         __syncwarp();                   // chunk j is there; every lane has read chunk j - 1, whose place the next one takes
         fetch(j + kF64Ring - 1);
+        load(j + kF64Ring - 1);
         const uint8_t* s = ring + (j % kF64Ring) * F::kStage;
         float4 a[MT];
         uint2 b[NT];
@@ -126,6 +148,7 @@ static __global__ void __launch_bounds__(32 * kF64Sums, F64Form<BM>::kPerSM) ly_
 #pragma unroll
                 for (int n = 0; n < NT; ++n) mma_f64_884(acc[i][n], av[i], bv[n]);
         }
+        put(j + kF64Ring - 1);
     }
     cp_async_wait<0>();
     __syncthreads();

@@ -197,7 +197,7 @@ def test_attention_sharp_scores():
 
 
 # ---- the exact mode's GEMM -----------------------------------------------------------------------------------------------------------------
-@pytest.mark.parametrize("width,ff", [(64, 72), (50, 34), (36, 130)])
+@pytest.mark.parametrize("width,ff", [(64, 72), (50, 34), (36, 130), (33, 71)])
 def test_exact_gemm_rows_stand_alone(width, ff):
     """f64 sums whose order depends on K alone: bitwise the same logits whether a token's row shares its tile with 7, 15, 16, 31, 32 others or
     with none, aligned rows or not"""
@@ -209,10 +209,10 @@ def test_exact_gemm_rows_stand_alone(width, ff):
     assert np.array_equal(whole, R.run_cut(model, toks, [1, 8, 9, 16, 17, 32, 2], cache=model.new_device_cache(2, 128)))
 
 
-@pytest.mark.parametrize("width,ff", [(1032, 1544), (1028, 770), (550, 2050)])
+@pytest.mark.parametrize("width,ff", [(1032, 1544), (1028, 770), (550, 2050), (547, 1033), (1034, 1553)])
 def test_exact_gemm_long_sums(width, ff):
-    """sums of more chunks than a warp keeps on their way (above 512 columns), the last chunk a half or less, rows aligned for 16-byte copies or not;
-    tiles of 8 and of 16 rows"""
+    """sums of more chunks than a warp keeps on their way (above 512 columns), the last chunk a half or less, rows of W aligned for copies of 16, 8 or 4
+    bytes or for none; tiles of 8 and of 16 rows"""
     cfg = R.config([R.delta(heads=4, kv_heads=2, dim=6, vdim=10, mlp=R.dense(ff=ff))], vocab=101, width=width)
     oracle, model = R.build(cfg, seed=73)
     toks = R.tokens(cfg, 48, seed=74)
