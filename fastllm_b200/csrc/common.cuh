@@ -111,10 +111,11 @@ __device__ __forceinline__ void mbar_wait(uint64_t* bar, uint32_t parity) {
             : "memory");
     } while (!done);
 }
-// the same with a limit (a try sleeps for some time by itself): false when it ran out
-__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity) {
-    for (int i = 0; i < (1 << 20); ++i) {
-        uint32_t done;
+// the same with a limit: true when the phase is over, false when `tries` ran out (a try sleeps for some time by itself)
+constexpr int kMbarTries = 1 << 20;
+__device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity, int tries) {
+    uint32_t done;
+    do {
         asm volatile(
             "{\n"
             ".reg .pred p;\n"
@@ -124,9 +125,8 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
             : "=r"(done)
             : "r"(smem_u32(bar)), "r"(parity)
             : "memory");
-        if (done) return true;
-    }
-    return false;
+    } while (!done && --tries > 0);
+    return done != 0;
 }
 // non-blocking probe of the phase with the given parity
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {

@@ -2170,7 +2170,7 @@ static __global__ void __launch_bounds__(160) ly_rec_scan_kernel(RecArgs a) {
         uint32_t ph = 1;
         for (int row = r0; row < r1; row += GT) {
             const int n = min(GT, r1 - row);
-            if (!(ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&empty[grp], ph)))) break;
+            if (!(ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&empty[grp], ph, kMbarTries)))) break;
             if (pieces) {
                 if (lane == 0) mbar_expect_tx(&full[grp], (uint32_t)(n * (2 * D + nv) * 4));
                 __syncwarp();
@@ -2227,12 +2227,12 @@ static __global__ void __launch_bounds__(160) ly_rec_scan_kernel(RecArgs a) {
     // lane t: decay and strength of token t of a group
     auto decays = [&](int row) { return lane < GT && row + lane < r1 ? *reinterpret_cast<const float2*>(a.ab + ((size_t)(row + lane) * a.H + hd) * 2) : make_float2(1.f, 0.f); };
     float2 ab = decays(r0);
-    int grp = 0;
+    int grp = 0, tries = kMbarTries;
     uint32_t ph = 0;
     for (int row = r0; row < r1; row += GT) {
         const float2 now = ab;
         ab = decays(row + GT);
-        if (!(ok = __all_sync(0xFFFFFFFFu, mbar_wait_bounded(&full[grp], ph)))) break;
+        tries = mbar_wait_bounded(&full[grp], ph, tries) ? tries : 0;        // (to the end even behind one that ran out, which later ones then do at once: no branch on it here)
         float mine = 0.f;
         auto token = [&](int t) {
             const float* cur = sm + (grp * GT + t) * SLOT;
@@ -2277,6 +2277,7 @@ static __global__ void __launch_bounds__(160) ly_rec_scan_kernel(RecArgs a) {
         if (lane % LPC < GT && row + lane % LPC < r1 && vok) a.o[(size_t)(row + lane % LPC) * a.H * Dv + hd * Dv + col] = mine;
         if (++grp == NG) { grp = 0; ph ^= 1; }
     }
+    ok = __all_sync(0xFFFFFFFFu, tries > 0);
     if (!ok) give_up();
     if (ok && vok) {
 #pragma unroll
