@@ -27,11 +27,17 @@ constexpr int kCsSlab = 64;             // value columns at a time
 constexpr int kCsPad = 4;               // floats behind a row in shared memory: neighbouring rows start four banks apart
 constexpr int kCsLdA = kCsC + kCsPad;   // row stride of a [64][64] operand
 constexpr int kCsChunks = 32;           // chunks whose states are held at a time (32 heads of 128 x 128: 67 MB), over all sequences of a step
-// Portions from this length on (at least a chunk).  Whole prefill token by token -> in chunks, us: gated linear attention 64 / 80 / 96 / 127 tokens: width
-// 1024 373 -> 366, 411 -> 396, 431 -> 397, 469 -> 407; 2048 557 -> 551, 628 -> 615, 650 -> 619, 694 -> 638.  One decay per head (ly_rec_scan_kernel takes 0.25 to 0.3 us a token): delta rule and Mamba-2 128 / 192 / 256 / 327
-// tokens: width 1024 361 -> 424, 477 -> 505, 536 -> 527; 2048 449 -> 503, 575 -> 611, 629 -> 661, 697 -> 713; 4096 (192, 256) 1054 -> 1093, 1145 -> 1131;
-// lightning, width 2048, 128 / 192 / 256 / 333: 550 -> 568, 662 -> 665, 675 -> 678, 717 -> 692.
-constexpr int kCsMinTokensGla = 64, kCsMinTokens = 256;
+// Portions from this length on (at least a chunk).  Two layers of the kind alone, whole prefill, us, token by token -> in chunks:
+// gated linear attention, one / four portions of 64 and 127 tokens: width 1024 240 -> 231, 366 -> 245 / 322 -> 308, 443 -> 306; 2048 274 -> 268, 402 -> 290 / 382 ->
+// 345, 523 -> 367.
+// Mamba-2, 160 / 192 / 224 / 255 tokens: one portion of width 1024 301 -> 308, 261 -> 282, 327 -> 293, 410 -> 347; 2048 352 -> 380, 362 -> 361, 411 -> 381, 457 -> 402;
+// 4096 499 -> 538, 540 -> 532, 582 -> 562; four portions of 1024 370 -> 410, 410 -> 426, 455 -> 436, 429 -> 448; 2048 572 -> 578, 629 -> 590, 681 -> 603, 729 -> 605;
+// 4096 1068 -> 1076, 1163 -> 1109, 1330 -> 1279, 1436 -> 1324.  Lightning (beside attention): 2048 396 -> 418, 421 -> 426, 437 -> 431, 452 -> 437; four 720 -> 738,
+// 760 -> 756, 847 -> 820, 901 -> 854.
+// Delta rule, 192 / 224 / 255 / 320 tokens: one portion of 1024 364 -> 341, 292 -> 340, 304 -> 333, 389 -> 370; 2048 380 -> 409, 363 -> 403, 445 -> 442, 480 -> 453;
+// 4096 467 -> 492, 498 -> 539, 601 -> 556, 622 -> 594; four of 1024 407 -> 422, 446 -> 439, 497 -> 451, 501 -> 479; 2048 523 -> 582, 569 -> 610, 606 -> 618, 709 -> 772;
+// 4096 837 -> 1001, 976 -> 1186, 1036 -> 1200, 1377 -> 1632: where serial blocks fill the SMs more than once they stay ahead for longer.
+constexpr int kCsMinTokensGla = 64, kCsMinTokensOne = 192, kCsMinTokensDelta = 256;      // (One: one decay per head, no delta rule)
 
 struct ChunkArgs {
     const float* src; int ld, off_q, off_k, off_v;      // q, k [G][D], v [H][Dv] per row

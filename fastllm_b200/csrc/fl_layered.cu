@@ -1146,7 +1146,7 @@ static void launch_rec_scan(LaunchCtx& lc, const RecArgs& a, int n) {
 }
 
 enum class Recurrence { scalar, gla, delta };
-static int chunk_min(Recurrence kind) { return kind == Recurrence::gla ? kCsMinTokensGla : kCsMinTokens; }
+static int chunk_min(Recurrence kind) { return kind == Recurrence::gla ? kCsMinTokensGla : kind == Recurrence::delta ? kCsMinTokensDelta : kCsMinTokensOne; }
 // Portions of chunk_min tokens and more take the chunked kernels (chunk_scan.cuh), in the serving precision: the exact mode's sums must
 // not depend on how a prompt was cut.  The chunked kernels read 16 bytes at a time and hold at most 128 state rows.
 static bool chunks_fit(const ChunkArgs& a, Recurrence kind, bool f32, const int* counts, int n) {

@@ -3,8 +3,10 @@
 Bars as in the design's own test files: the serving precision differs from the oracle (which rounds what it caches to bf16) by cached
 elements that land on the other side of a rounding boundary, and a near-tied router may pick another expert after one (`allow`)."""
 import os
+import re
 import subprocess
 import sys
+from pathlib import Path
 
 import numpy as np
 import pytest
@@ -71,10 +73,35 @@ def test_gated_epilogue(n, ff, width):
     check(R, cfg, n, 35, 0.0)
 
 
-# ---- recurrences in chunks of 64 tokens (portions of at least 128) against the same model fed in portions that stay token by token ------
+# ---- recurrences in chunks of 64 tokens (portions from LINE on) against the same model fed in portions that stay token by token ------
+_LINE = {k: int(v) for k, v in re.findall(r"kCsMinTokens(\w+) = (\d+)", (Path(__file__).resolve().parent.parent / "fastllm_b200/csrc/chunk_scan.cuh").read_text())}
+LINE = {"gla": _LINE["Gla"], "gla_fast_decay": _LINE["Gla"], "mamba": _LINE["One"], "lightning": _LINE["One"], "delta": _LINE["Delta"]}
+SERIAL = 60                 # tokens of a portion that no recurrence takes in chunks
+assert SERIAL < min(LINE.values())
 # No cache is rounded in these models, so what is left between the two is the order of f32 sums in the recurrence and in the GEMMs around
 # it: a few 1e-7 per sum, some tens of sums and norms behind one another.
 CHUNK_TOL = 3e-5
+
+
+def tags_of(run):
+    """kernels that `run` launched, by the profiler's tags"""
+    from fastllm_b200 import models
+    models.prof_begin()
+    out = run()
+    return out, {p["kernel"] for p in models.prof_end()}
+
+
+def in_portions(mod, model, toks, size=SERIAL):
+    """token by token: portions below every line"""
+    out, tags = tags_of(lambda: mod.run_cut(model, toks, [size] * (len(toks) // size + 1), cache=model.new_device_cache(2, max(512, len(toks) + 8))))
+    assert not any("chunks" in t for t in tags)
+    return np.asarray(out, dtype=np.float64)
+
+
+def in_chunks(run):
+    out, tags = tags_of(run)
+    assert any("chunks" in t for t in tags)
+    return out
 
 
 def recurrent(kind, dim, vdim, heads=2):
@@ -87,18 +114,20 @@ def recurrent(kind, dim, vdim, heads=2):
     return R, R.config([R.delta(heads=2 * heads, kv_heads=heads, dim=dim, vdim=vdim)], width=64)
 
 
+# tokens behind the kind's line: whole chunks, a last one of 63 tokens, of one, of 57 to 9
 @pytest.mark.parametrize("kind", ["gla", "gla_fast_decay", "mamba", "delta"])
-@pytest.mark.parametrize("dim,vdim,n", [(16, 16, 128), (64, 64, 191), (68, 36, 129), (128, 68, 192), (100, 128, 321), (4, 132, 200)])
-def test_chunks_equal_token_by_token(kind, dim, vdim, n):
+@pytest.mark.parametrize("dim,vdim,more", [(16, 16, 0), (64, 64, 63), (68, 36, 1), (128, 68, 64), (100, 128, 121), (4, 132, 73)])
+def test_chunks_equal_token_by_token(kind, dim, vdim, more):
     mod, cfg = recurrent(kind, dim, vdim)
     _, model = mod.build(cfg, seed=41, dtype="bf16")
+    n = LINE[kind] + more
     toks = mod.tokens(cfg, n, seed=42)
-    serial = mod.run_cut(model, toks, [100] * 4, cache=model.new_device_cache(2, 512))
-    whole = mod.run_whole(model, toks, cache=model.new_device_cache(2, 512))
-    assert mod.relerr(whole, np.asarray(serial, dtype=np.float64)) < CHUNK_TOL
-    # a portion of chunks behind a short one, and a short one behind it: the state passes both borders
-    cut = mod.run_cut(model, toks, [30, n - 40] if n >= 168 else [n], cache=model.new_device_cache(2, 512))
-    assert mod.relerr(cut, np.asarray(serial, dtype=np.float64)) < CHUNK_TOL
+    serial = in_portions(mod, model, toks)
+    whole = in_chunks(lambda: mod.run_whole(model, toks, cache=model.new_device_cache(2, 512)))
+    assert mod.relerr(whole, serial) < CHUNK_TOL
+    if more >= 40:      # a portion of chunks behind a short one, and a short one behind it: the state passes both borders
+        cut = in_chunks(lambda: mod.run_cut(model, toks, [30, n - 40], cache=model.new_device_cache(2, 512)))
+        assert mod.relerr(cut, serial) < CHUNK_TOL
 
 
 @pytest.mark.parametrize("kind", ["mamba", "delta"])
@@ -114,17 +143,20 @@ def test_token_by_token_in_any_cut(kind, dim, vdim):
     assert np.array_equal(whole, mod.run_cut(model, toks, [1, 2, 3, 4, 5, 12, 14], cache=model.new_device_cache(2, 64)))
 
 
-# the first lengths that go in chunks (64 tokens of gated linear attention, 256 of the others), a token more, a last chunk of one token to 63
-@pytest.mark.parametrize("kind,n", [("gla", 64), ("gla", 65), ("gla", 127), ("gla_fast_decay", 191), ("mamba", 256), ("mamba", 257), ("delta", 256), ("delta", 319)])
+# the first lengths that go in chunks and a token more, a last chunk of 63 tokens
+@pytest.mark.parametrize("kind,more", [("gla", 0), ("gla", 1), ("gla", 63), ("gla_fast_decay", 127), ("mamba", 0), ("mamba", 1), ("delta", 0), ("delta", 63)])
 @pytest.mark.parametrize("dim,vdim", [(128, 128), (68, 132), (16, 20)])
-def test_first_lengths_in_chunks(kind, n, dim, vdim):
-    """against portions of 60 tokens, which no recurrence takes in chunks"""
+def test_first_lengths_in_chunks(kind, more, dim, vdim):
+    """against portions of 60 tokens, which no recurrence takes in chunks; a token less stays token by token"""
     mod, cfg = recurrent(kind, dim, vdim)
     _, model = mod.build(cfg, seed=81, dtype="bf16")
+    n = LINE[kind] + more
     toks = mod.tokens(cfg, n, seed=82)
-    serial = mod.run_cut(model, toks, [60] * 6, cache=model.new_device_cache(2, 512))
-    whole = mod.run_whole(model, toks, cache=model.new_device_cache(2, 512))
-    assert mod.relerr(whole, np.asarray(serial, dtype=np.float64)) < CHUNK_TOL
+    whole = in_chunks(lambda: mod.run_whole(model, toks, cache=model.new_device_cache(2, 512)))
+    assert mod.relerr(whole, in_portions(mod, model, toks)) < CHUNK_TOL
+    if more == 0:
+        _, tags = tags_of(lambda: mod.run_whole(model, toks[:-1], cache=model.new_device_cache(2, 512)))
+        assert not any("chunks" in t for t in tags)
 
 
 @pytest.mark.parametrize("kind", ["gla", "mamba", "delta"])
@@ -136,26 +168,25 @@ def test_chunks_of_several_sequences(kind):
     reqs = [mod.tokens(cfg, k, seed=50 + i) for i, k in enumerate(lens)]
     cache = model.new_device_cache(4, 1536)
     for round_ in range(2):
-        got = cache.forward_ragged([2, 0, 3, 1], reqs, [list(range(k)) for k in lens])
+        got = in_chunks(lambda: cache.forward_ragged([2, 0, 3, 1], reqs, [list(range(k)) for k in lens]))
         at = 0
         for r, k in zip(reqs, lens):
-            alone = mod.run_cut(model, r, [120] * 10, cache=model.new_device_cache(1, 1536))
-            assert mod.relerr(got[at:at + k], np.asarray(alone, dtype=np.float64)) < CHUNK_TOL
+            assert mod.relerr(got[at:at + k], in_portions(mod, model, r)) < CHUNK_TOL
             at += k
         for s in range(4):
             cache.slot_reset(s)
 
 
 @pytest.mark.parametrize("kind", ["gla", "gla_fast_decay", "mamba", "delta"])
-@pytest.mark.parametrize("dim,vdim,n", [(64, 64, 333), (100, 36, 200)])
-def test_chunks_against_the_oracle(kind, dim, vdim, n):
+@pytest.mark.parametrize("dim,vdim,more", [(64, 64, 77), (100, 36, 8)])
+def test_chunks_against_the_oracle(kind, dim, vdim, more):
     mod, cfg = recurrent(kind, dim, vdim)
-    check(mod, cfg, n, 47, 0.0)
+    in_chunks(lambda: check(mod, cfg, LINE[kind] + more, 47, 0.0))
 
 
-@pytest.mark.parametrize("dim,vdim,n", [(16, 24, 128), (128, 128, 200), (64, 72, 333)])
-def test_lightning_chunks(dim, vdim, n):
-    check(M, M.config([M.par_layer(b=M.lightning(heads=2, dim=dim, vdim=vdim))], width=64), n, 45, 0.0)
+@pytest.mark.parametrize("dim,vdim,more", [(16, 24, 0), (128, 128, 8), (64, 72, 141)])
+def test_lightning_chunks(dim, vdim, more):
+    in_chunks(lambda: check(M, M.config([M.par_layer(b=M.lightning(heads=2, dim=dim, vdim=vdim))], width=64), LINE["lightning"] + more, 45, 0.0))
 
 
 # ---- grouped-query attention of a portion in one kernel ----------------------------------------------------------------------------------
@@ -396,14 +427,6 @@ def test_a_step_does_not_depend_on_what_the_cache_has_seen():
             got = cache.forward_ragged([0], [toks[a:b]], [list(range(b - a))])
         rows.append(got)
     assert np.array_equal(*rows)
-
-
-def tags_of(run):
-    """kernels that `run` launched, by the profiler's tags"""
-    from fastllm_b200 import models
-    models.prof_begin()
-    out = run()
-    return out, {p["kernel"] for p in models.prof_end()}
 
 
 # rows and the tiles of 256 x 256 over 74 pairs: the last pair row ends inside its second half, 1 whole tile each and 16 cut ones (o, gate|up); 2 and 6
