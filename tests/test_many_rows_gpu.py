@@ -159,6 +159,17 @@ def test_first_lengths_in_chunks(kind, more, dim, vdim):
         assert not any("chunks" in t for t in tags)
 
 
+@pytest.mark.parametrize("groups,state,vdim", [(4, 128, 64), (1, 128, 68), (8, 64, 132), (4, 20, 36)])
+def test_chunks_of_four_heads(groups, state, vdim):
+    """heads that read the same queries and keys share a block by fours; 34 chunks: 32 at a time, whose 256 blocks of four heads go together in the last kernel too,
+    then two, whose 16 blocks would leave SMs idle there and take one head each"""
+    cfg = R.config([R.mamba(heads=32, vdim=vdim, state=state, groups=groups)], width=64)
+    _, model = R.build(cfg, seed=83, dtype="bf16")
+    toks = R.tokens(cfg, 2118, seed=84)
+    whole = in_chunks(lambda: R.run_whole(model, toks, cache=model.new_device_cache(1, 2176)))
+    assert R.relerr(whole, in_portions(R, model, toks)) < CHUNK_TOL
+
+
 @pytest.mark.parametrize("kind", ["gla", "mamba", "delta"])
 def test_chunks_of_several_sequences(kind):
     """two prompts of more chunks than are held at a time beside a short one and a decoded token; a reused slot starts from zero"""
