@@ -5,10 +5,11 @@
 // Two CTAs of a cluster take two groups of whole sentences of up to 128 rows each (tcgen05.mma.cta_group::2, see gemm_pair.cuh: a single CTA would read
 // every weight from L2 for 128 tokens, 18 TB/s at the tensor cores' rate).  A unit of work is up to three heads of such a pair: 288 columns of q|k|v in TMEM,
 // rounded into shared memory by twelve warps, which then are the attention's (mma.sync, a sentence's 16 query rows of a head at a time) while the tensor
-// core makes the next unit's columns.  The clusters take equal runs of heads; x stays in shared memory over the units of a pair.
+// core makes the next unit's columns.  The clusters take equal runs of heads (up to four heads a run none crosses from one pair of groups to the next: 60 x 43
+// tokens 366 -> 354 us, 36 x 65 354 -> 345); x stays in shared memory over the units of a pair.
 // q, k and v never leave the SM: the GEMM and the attention moved 75 MB each way between them at 256 x 128 tokens.
 // Whole encoder, GEMM and attention -> this kernel, us (with the block kernel as it is): 256 x 128 tokens 1280 -> 1102, 76 x 128 552 -> 517, 400 x 43 788 ->
-// 645, 1500 x 20 1690 -> 1177, 60 x 43 378 -> 368; a layer of 256 x 128: 87 -> 66.  (Runs of whole units of three heads: 76 x 128 567.)
+// 645, 1500 x 20 1690 -> 1177, 60 x 43 377 -> 354; a layer of 256 x 128: 87 -> 66.  (Runs of whole units of three heads: 76 x 128 567.)
 // A unit of 128-token sentences takes about 14500 clocks: 2200 to bring q|k|v into shared memory, 12000 of attention in which the tensor core's 3700 for
 // the next unit run -- the warps' products (3300), ex2 (3100) and shared memory (3300 and the operands of the other products) would overlap better with
 // more warps than the registers allow (eight warps of 168 registers: 17800; two row tiles a warp and an online softmax: no gain).
@@ -167,6 +168,12 @@ __device__ __forceinline__ void tmem_arrived32(uint32_t (&r)[32]) {
                      : "memory");
 }
 
+// Four heads, of `pieces` 16-row tiles each, as two units of two instead of three and one: the warps go round a unit's pieces in whole rounds.
+// (37 / 46 x 65 tokens 373 -> 368, 381 -> 378 us; units of two throughout, three rounds instead of four for twelve heads: 300 x 67 1034 -> 1055.)
+__host__ __device__ constexpr bool bq_halves(int pieces) {
+    auto rounds = [](int n) { return (n + kBqWarps - 1) / kBqWarps; };
+    return 2 * rounds(2 * pieces) < rounds(3 * pieces) + rounds(pieces);
+}
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kBqThreads, 1)
 bert_qkv_attn_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_constant__ CUtensorMap tmW, const BertQkvArgs g) {
     extern __shared__ uint8_t gsm_raw[];
@@ -182,7 +189,11 @@ bert_qkv_attn_kernel(const __grid_constant__ CUtensorMap tmX, const __grid_const
     const int groups = (g.b + g.spc - 1) / g.spc, heads = (groups + 1) / 2 * kBqAllHeads;      // of all pairs, in a row
     const int h0 = (int)((long long)heads * cl / G), h1 = (int)((long long)heads * (cl + 1) / G);
     // the unit that begins at a head: how many heads
-    auto unit = [&](int h) { return min(kBqHeads, min(h1 - h, kBqAllHeads - h % kBqAllHeads)); };
+    const bool halves = bq_halves(g.spc * ((g.t + 15) / 16));
+    auto unit = [&](int h) {
+        const int left = min(h1 - h, kBqAllHeads - h % kBqAllHeads);
+        return left == 4 && halves ? 2 : min(kBqHeads, left);
+    };
 
     pdl_launch_dependents();
     if (threadIdx.x == 0) {

@@ -319,13 +319,15 @@ static int bert_qkv_pairs(int b, int t) {
     const int spc = kBertS / t;
     return ((b + spc - 1) / spc + 1) / 2;
 }
-// One kernel for q|k|v and the attention, GEMM and attention kernel where most rows of its tiles would be padding and its heads go round badly: a group is
-// one sentence from 65 tokens on, and four heads a pair of SMs are two units.  Whole encoder, us, two kernels -> one: 38 / 46 x 65 359 -> 371, 371 -> 386,
-// 38 x 75 369 -> 383, but 36 x 65 (three heads a pair) 363 -> 362, 50 x 65 (five) 406 -> 392, 38 x 85 404 -> 396, 38 x 128 463 -> 439.
+// heads of the longest run that a pair of SMs takes
+static int bert_qkv_run(int b, int t) { return (bert_qkv_pairs(b, t) * kBqAllHeads + bert_qkv_clusters() - 1) / bert_qkv_clusters(); }
+// One kernel for q|k|v and the attention; GEMM and attention kernel where the longest run has four heads, which are two units however few rows the groups
+// hold, while the time of the two kernels goes with the rows.  Whole encoder, us, two kernels -> one, four heads a run: 37 x 65 358 -> 368, 38 x 75 370 -> 379, 38 x 80
+// (3040 rows) 373 -> 382, 37 x 83 (3071) 385 -> 388, 44 x 70 (3080) 380 -> 382, 48 x 65 (3120) 381 -> 381, 38 x 85 400 -> 390, 48 x 80 400 -> 389, 76 x 43 405 -> 379;
+// one to three heads: 12 x 65 331 -> 309, 25 x 65 338 -> 331, 36 x 65 359 -> 345; five: 50 x 65 408 -> 395.
 static bool bert_qkv_attn(const BertModel& m, int b, int t) {
     if (m.H != kBbH || m.nh != kBsHeads || t > kBertS || bert_qkv_clusters() == 0) return false;
-    const int heads = (bert_qkv_pairs(b, t) * kBqAllHeads + bert_qkv_clusters() - 1) / bert_qkv_clusters();
-    return !(t > kBertS / 2 && t <= 5 * kBertS / 8 && heads == 4);
+    return bert_qkv_run(b, t) != 4 || b * t > 24 * kGemmBM;
 }
 // A pair of SMs takes about as long for 256 tokens however many tiles there are, the chain's kernels grow with the tokens, in steps of their own waves.
 // Whole encoder, chain -> blocks, us, by tiles of 256 tokens (128-token sentences): 20 451 -> 465, 24 459 -> 463, 28 513 -> 487, 32 533 -> 490, 36 558 -> 505,
@@ -414,8 +416,10 @@ static void launch_bert_block(BertModel& m, const CUtensorMap& tm_ctx, const CUt
     blaunch(m.stream, bert_block_kernel, dim3(2 * std::min((T + 255) / 256, bert_block_clusters())), dim3(kBbThreads), kBbSmem, tm_ctx, w.tb_wo, w.tb_wi, w.tb_wo2, tm_x, a);
 }
 static void launch_bert_qkv(BertModel& m, const CUtensorMap& tm_x, const BertLayerW& w, int b, int t, float scale) {
+    // equal runs of heads; up to four heads a run none of them crosses from one pair of groups to the next
+    const int run = bert_qkv_run(b, t), clusters = run <= 4 ? bert_qkv_pairs(b, t) * kBqAllHeads / run : bert_qkv_clusters();
     const BertQkvArgs a{b, t, kBertS / t, w.bqkv, 1.f / scale, m.ctx.p, m.failed.p};
-    blaunch(m.stream, bert_qkv_attn_kernel, dim3(2 * std::min(bert_qkv_pairs(b, t) * kBqAllHeads, bert_qkv_clusters())), dim3(kBqThreads), kBqSmem, tm_x, w.tb_wqkv, a);
+    blaunch(m.stream, bert_qkv_attn_kernel, dim3(2 * clusters), dim3(kBqThreads), kBqSmem, tm_x, w.tb_wqkv, a);
 }
 static void bert_check(const BertModel& m) {
     FL_CHECK(*m.failed.p == 0, FL_ERR_CUDA, "a wait inside a kernel ran out, the results are not valid");

@@ -20,8 +20,10 @@ def encoder():
 
 
 # a whole tile, one row less; two sentences a group and one; rows of a tile left over (43: 42 of 128; 25: three); sentences within a 16-row tile; an odd
-# number of groups; fewer heads than pairs of SMs, runs of heads that begin and end inside a pair's; the two kernels' route (38 x 70)
-@pytest.mark.parametrize("b,t", [(1, 128), (2, 127), (37, 128), (9, 64), (10, 65), (31, 43), (33, 25), (70, 17), (75, 16), (150, 8), (223, 5), (700, 1), (300, 113), (152, 64), (41, 128), (38, 70)])
+# number of groups; runs of one to four heads, four as three and one (76 x 43: a pair of groups ends behind every third run; 41 x 128) or as two and two (38 x 85);
+# longer runs that begin and end inside a pair's; the two kernels' route (38 x 70)
+@pytest.mark.parametrize("b,t", [(1, 128), (2, 127), (37, 128), (19, 64), (21, 63), (10, 65), (36, 65), (31, 43), (33, 25), (70, 17), (75, 16), (150, 8), (223, 5), (700, 1), (300, 113),
+                                 (152, 64), (41, 128), (76, 43), (38, 85), (38, 70)])
 def test_against_the_oracle(encoder, b, t):
     """bf16 operands: 2^-9 of a value per rounding, four roundings between sums of hundreds per layer; a misplaced row, head or key is a cosine below 0.9"""
     cfg, oracle, model = encoder
