@@ -32,7 +32,7 @@ struct BertModel {
     cudaStream_t stream = nullptr;
     std::mutex mu;
     // workspace (grown on demand)
-    size_t cap_tokens = 0, cap_batch = 0, cap_chain = 0;
+    size_t cap_tokens = 0, cap_batch = 0, cap_chain = 0, cap_qkv = 0;
     DevBuf<uint16_t> x, x1, ctx, qkv, hbuf;
     DevBuf<float> pre, out;
     DevBuf<uint32_t> ids, mask;

@@ -375,24 +375,31 @@ static int bert_small_launch(BertModel& m, const BertSmallArgs& a, int clusters,
 
 // What takes a call; which buffers are reserved and what is launched both follow from it.
 enum class BertPath { small, blocks, chain };
-struct BertRun { BertPath path; int spc, clusters; };       // small: sentences per cluster, clusters
+struct BertRun {
+    BertPath path;
+    int spc, clusters;          // small: sentences per cluster, clusters
+    bool front;                 // blocks, chain: q|k|v and the attention in one kernel
+    bool chain() const { return path != BertPath::blocks; }                    // buffers x1, hbuf, pre
+    bool qkv() const { return path != BertPath::small && !front; }             // buffer qkv
+};
 static BertRun bert_run(BertModel& m, int b, int t) {
     if (m.small_layers != nullptr && t <= kBsTokens) {
         static const int resident = bert_small_launch<kBsTokens / 16>(m, BertSmallArgs{}, 1, true);       // a property of the device
         if (resident >= 1) {
             // as many clusters as fit at a time, each with as few sentences as that leaves: up to 64 tokens per cluster
             const int spc = (b + resident - 1) / resident;
-            if (spc * t <= kBsTokens) return {BertPath::small, spc, (b + spc - 1) / spc};
+            if (spc * t <= kBsTokens) return {BertPath::small, spc, (b + spc - 1) / spc, false};
         }
     }
-    return {bert_blocks(m, b * t) ? BertPath::blocks : BertPath::chain, 0, 0};
+    return {bert_blocks(m, b * t) ? BertPath::blocks : BertPath::chain, 0, 0, bert_qkv_attn(m, b, t)};
 }
 static void bert_reserve(BertModel& m, const BertRun& run, int b, int t) {
     const size_t T = (size_t)b * t, B = b, H = m.H, I = m.I;
-    if (run.path != BertPath::blocks)
+    if (run.chain())
         grow(m.cap_chain, T, [&] { m.x1.alloc(T * H); m.hbuf.alloc(T * I); m.pre.alloc(T * H); });
+    if (run.qkv()) grow(m.cap_qkv, T, [&] { m.qkv.alloc(T * 3 * H); });
     grow(m.cap_tokens, T, [&] {
-        m.x.alloc(T * H); m.ctx.alloc(T * H); m.qkv.alloc(T * 3 * H);
+        m.x.alloc(T * H); m.ctx.alloc(T * H);
         m.ids.alloc(T); m.mask.alloc(T); m.h_ids.alloc(2 * T);
     });
     grow(m.cap_batch, B, [&] { m.out.alloc(B * H); m.h_out.alloc(B * H); });
@@ -437,7 +444,7 @@ static void bert_enqueue(BertModel& m, const BertRun& run, int b, int t, bool ha
     const dim3 row_grid((T + rows_per_cta - 1) / rows_per_cta), row_block(rows_per_cta * 32);
     blaunch(st, embed_ln_kernel, row_grid, row_block, 0, (const uint16_t*)m.wemb, (const uint16_t*)m.pemb, (const float*)m.lnw, (const float*)m.lnb,
             (const uint32_t*)m.ids.p, T, t, H, m.V, m.maxpos, 1e-12f, m.x.p);
-    const bool blocks = run.path == BertPath::blocks, qkv_attn = bert_qkv_attn(m, b, t);
+    const bool blocks = run.path == BertPath::blocks;
     const CUtensorMap tm_x = make_tmap_bf16(m.x.p, T, H, H, kGemmBM), tm_x1 = blocks ? tm_x : make_tmap_bf16(m.x1.p, T, H, H, kGemmBM),
                       tm_ctx = make_tmap_bf16(m.ctx.p, T, H, H, kGemmBM);
     const CUtensorMap tm_h = blocks ? tm_x : make_tmap_bf16(m.hbuf.p, T, I, I, kGemmBM);
@@ -445,7 +452,7 @@ static void bert_enqueue(BertModel& m, const BertRun& run, int b, int t, bool ha
     const float scale = (float)std::sqrt((double)m.d);
     for (int l = 0; l < m.L; ++l) {
         const BertLayerW& w = m.layers[l];
-        if (qkv_attn) {     // B2 to B4 in one kernel
+        if (run.front) {    // B2 to B4 in one kernel
             launch_bert_qkv(m, tm_x, w, b, t, scale);
         } else {
             // B2: fused q|k|v projection + bias -> bf16 [T, 3H]
@@ -511,7 +518,7 @@ void bert_repeat(BertModel& m, int b, int t, int iters, float* elapsed_ms) {
     std::lock_guard<std::mutex> lock(m.mu);
     const BertRun run = bert_run(m, b, t);
     const size_t T = (size_t)b * t;
-    FL_CHECK(T <= m.cap_tokens && (size_t)b <= m.cap_batch && (run.path == BertPath::blocks || T <= m.cap_chain), FL_ERR_STATE, "call fl_embed with this shape first");
+    FL_CHECK(T <= m.cap_tokens && (size_t)b <= m.cap_batch && (!run.chain() || T <= m.cap_chain) && (!run.qkv() || T <= m.cap_qkv), FL_ERR_STATE, "call fl_embed with this shape first");
     EventPair ev;
     FL_CUDA(cudaEventRecord(ev.e0, m.stream));
     for (int i = 0; i < iters; ++i) bert_enqueue(m, run, b, t, false);

@@ -54,3 +54,16 @@ def test_same_bits_as_gemm_and_attention_kernel(encoder, b, t):
     ids = synth.token_ids(1000 + b * 131 + t, cfg.vocab_size, (b, t))
     want = np.load(Path(__file__).parent / "golden" / "bert_attention_bits.npz")[f"{b}x{t}"]
     assert np.array_equal(model.embed_ids(ids)[sorted({0, b // 2, b - 1})], want)
+
+
+def test_only_the_buffers_of_a_route():
+    """256 x 128 tokens: x and ctx are 25 MB each; q|k|v, which stay on the chip, would be 75 MB more.  A repeat finds every buffer of its route, whatever calls came before"""
+    import torch
+    from fastllm_b200 import models
+    model = models.MiniLMModel(models.BertConfig(), None, 0, random_seed=3)
+    ids = np.random.default_rng(1).integers(3, 30000, (256, 128)).astype(np.uint32)
+    free = torch.cuda.mem_get_info()[0]
+    model.embed_ids(ids)
+    assert free - torch.cuda.mem_get_info()[0] < 70 << 20
+    for b, t in ((38, 70), (256, 128), (1, 19), (30, 400)):        # GEMM and attention kernel; the front; one launch; long sentences
+        assert np.array_equal(model.embed_ids_timed(ids.reshape(-1)[:b * t].reshape(b, t), 2)[0], model.embed_ids(ids.reshape(-1)[:b * t].reshape(b, t)))
