@@ -28,22 +28,23 @@ constexpr int kBsCluster = 16;
 constexpr int kBsQkvRows = 3 * kBertD, kBsORows = kBsH / kBsCluster, kBsIRows = kBsI / kBsCluster;
 constexpr int kBsAtO = kBsQkvRows * bs_ld(kBsH), kBsAtI = kBsAtO + kBsORows * bs_ld(kBsH), kBsAtO2 = kBsAtI + kBsIRows * bs_ld(kBsH),
               kBsPack = kBsAtO2 + kBsORows * bs_ld(kBsI);                     // elements of a block
-static_assert(kBsAtO % 8 == 0 && kBsAtI % 8 == 0 && kBsAtO2 % 8 == 0 && kBsPack % 8 == 0, "16-byte pieces");
-static __global__ void bert_small_pack_kernel(const uint16_t* __restrict__ wqkv, const uint16_t* __restrict__ wo, const uint16_t* __restrict__ wi,
-                                              const uint16_t* __restrict__ wo2, uint16_t* __restrict__ out) {
-    const int rank = blockIdx.y;
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < kBsPack; i += gridDim.x * blockDim.x) {
-        const int ld = i < kBsAtO2 ? bs_ld(kBsH) : bs_ld(kBsI), k = i < kBsAtO2 ? kBsH : kBsI;
-        const int at = i < kBsAtO ? 0 : i < kBsAtI ? kBsAtO : i < kBsAtO2 ? kBsAtI : kBsAtO2, r = (i - at) / ld, c = (i - at) % ld;
-        uint16_t v = 0;
-        if (c < k) {
-            if (i < kBsAtO) v = rank < kBsHeads ? wqkv[(size_t)(r / kBertD * kBsH + rank * kBertD + r % kBertD) * kBsH + c] : (uint16_t)0;
-            else if (i < kBsAtI) v = wo[(size_t)(rank * kBsORows + r) * kBsH + c];
-            else if (i < kBsAtO2) v = wi[(size_t)(rank * kBsIRows + r) * kBsH + c];
-            else v = wo2[(size_t)(rank * kBsORows + r) * kBsI + c];
-        }
-        out[(size_t)rank * kBsPack + i] = v;
+static_assert(kBsAtO % 8 == 0 && kBsAtI % 8 == 0 && kBsAtO2 % 8 == 0 && kBsPack % 8 == 0 && kBsH % 8 == 0 && kBsI % 8 == 0, "16-byte pieces");
+// grid (pieces / 256, blocks of a cluster, layers); the layers' matrices lie `stride` elements apart.  16 bytes a thread: rows and their ends are whole pieces.
+static __global__ void __launch_bounds__(256) bert_small_pack_kernel(const uint16_t* __restrict__ wqkv, const uint16_t* __restrict__ wo, const uint16_t* __restrict__ wi,
+                                                                     const uint16_t* __restrict__ wo2, size_t stride, uint16_t* __restrict__ out) {
+    const int rank = blockIdx.y, i = (blockIdx.x * 256 + threadIdx.x) * 8;
+    if (i >= kBsPack) return;
+    const int ld = i < kBsAtO2 ? bs_ld(kBsH) : bs_ld(kBsI), k = i < kBsAtO2 ? kBsH : kBsI;
+    const int at = i < kBsAtO ? 0 : i < kBsAtI ? kBsAtO : i < kBsAtO2 ? kBsAtI : kBsAtO2, r = (i - at) / ld, c = (i - at) % ld;
+    const uint16_t* src = nullptr;
+    if (c < k) {
+        if (i >= kBsAtO2) src = wo2 + (size_t)(rank * kBsORows + r) * kBsI;
+        else if (i >= kBsAtI) src = wi + (size_t)(rank * kBsIRows + r) * kBsH;
+        else if (i >= kBsAtO) src = wo + (size_t)(rank * kBsORows + r) * kBsH;
+        else if (rank < kBsHeads) src = wqkv + (size_t)(r / kBertD * kBsH + rank * kBertD + r % kBertD) * kBsH;
     }
+    const uint4 v = src != nullptr ? *reinterpret_cast<const uint4*>(src + blockIdx.z * stride + c) : make_uint4(0u, 0u, 0u, 0u);
+    *reinterpret_cast<uint4*>(out + ((size_t)blockIdx.z * kBsCluster + rank) * kBsPack + i) = v;
 }
 
 struct BertSmallLayer {

@@ -279,12 +279,13 @@ void bert_finalize(BertModel& m) {
     }
     if (m.small_layers != nullptr) {
         std::vector<BertSmallLayer> tab;
-        for (const BertLayerW& w : m.layers) {
-            uint16_t* pack = m.small_pack + tab.size() * kBsCluster * kBsPack;
-            bert_small_pack_kernel<<<dim3(32, kBsCluster), 256>>>(w.wqkv, w.wo, w.wi, w.wo2, pack);
-            g_launches.fetch_add(1);
-            tab.push_back({pack, w.bqkv, w.bo, w.bi, w.bo2, w.ln1w, w.ln1b, w.ln2w, w.ln2b});
-        }
+        for (const BertLayerW& w : m.layers)
+            tab.push_back({m.small_pack + tab.size() * kBsCluster * kBsPack, w.bqkv, w.bo, w.bi, w.bo2, w.ln1w, w.ln1b, w.ln2w, w.ln2b});
+        // (every layer takes the same room in the slab)
+        const BertLayerW& w = m.layers[0];
+        const size_t stride = m.L > 1 ? (size_t)(m.layers[1].wqkv - w.wqkv) : 0;
+        bert_small_pack_kernel<<<dim3((kBsPack / 8 + 255) / 256, kBsCluster, m.L), 256>>>(w.wqkv, w.wo, w.wi, w.wo2, stride, m.small_pack);
+        g_launches.fetch_add(1);
         FL_CUDA(cudaGetLastError());
         FL_CUDA(cudaMemcpy(m.small_layers, tab.data(), tab.size() * sizeof(BertSmallLayer), cudaMemcpyHostToDevice));
         FL_CUDA(cudaStreamSynchronize(cudaStreamLegacy));       // (the model's stream does not wait for the default one)
