@@ -1,5 +1,6 @@
 // Layered decoders (FL_ARCH_NIFUNEX, FL_ARCH_ROFETAR, FL_ARCH_TOZARAX, FL_ARCH_MEDULORN, FL_ARCH_LATODRA, FL_ARCH_TUFAZEN): weight layout + ingest, pooled cache (pages of latents or keys | values +
 // recurrent-state slots), and the step function for mixed batches (portions of prompts beside single decoded tokens).
+#include <array>
 #include <cmath>
 #include <map>
 
@@ -10,6 +11,7 @@
 #include "gemm_f64.cuh"
 #include "gqa_attn_tc.cuh"
 #include "model.cuh"
+#include "runs.hpp"
 #include "synth.cuh"
 
 namespace fl {
@@ -847,12 +849,11 @@ static bool ff_in_fused(int R, int F, int K, int act, bool tc_in, bool tc_out, b
 // experts' results there (run_rows: the experts' runs in a step of more than 128 rows).
 // A new cache's first step of 2048 rows through three 4096 x 14336 layers takes 937 instead of 1694 MB and, with the scratch of its portions
 // reserved up front (reserve_portions), 15.1 instead of 16.9 ms.
-// rows of the experts' runs: whole 128-row tiles per expert that any row picked
-static size_t run_capacity(size_t picks, size_t experts) { return 128 * (picks / 128 + std::min(picks, experts)); }
 struct FfScratch { size_t gu = 0, act = 0, eo = 0, sh_gu = 0, sh_act = 0, sh_o = 0; };
 static FfScratch ff_scratch(const LayeredModel& m, size_t R, size_t run_rows) {
     FfScratch s;
     const size_t W = m.W;
+    std::map<std::array<int, 3>, size_t> runs;          // layers of equal sizes
     auto up = [](size_t& a, size_t b) { a = std::max(a, b); };
     // rows of the largest step up to R whose gate | up is not fused: a step of fewer rows has fewer tiles
     auto unfused = [&](int F, int act, bool tc_in, bool tc_out) {
@@ -870,10 +871,9 @@ static FfScratch ff_scratch(const LayeredModel& m, size_t R, size_t run_rows) {
             const size_t P = R * d.top;
             if (!lw.tc_moe) { up(s.gu, P * GF); up(s.act, P * F); up(s.eo, P * W); }
             else {
-                for (size_t T = 129; T <= R; ++T) {         // (a step of fewer rows may be cut along K more often)
-                    const int picks = (int)T * d.top;
-                    up(s.eo, runs_ksplit(picks, d.experts, m.W, d.ff) * run_capacity(picks, d.experts) * W);
-                }
+                const std::array<int, 3> key{d.top, d.experts, d.ff};
+                if (!runs.count(key)) runs[key] = runs_most_rows(d.top, d.experts, m.W, d.ff, kNumSMs, R);
+                up(s.eo, runs[key] * W);
                 if (d.ffn_act == FL_ACT_RELU2) up(s.gu, run_rows * F);
             }
             if (d.shared_ff > 0 && !m.cfg.parallel_sub) {
@@ -1949,7 +1949,7 @@ static void enqueue_step(fl_cache& c, LaunchCtx& lc, const StepTab& st, const in
             // whole prefill; 340 rows of 2816-wide experts: 2.37 -> 1.41 ms.)
             const size_t cap = run_capacity(P, E);
             const RowRuns runs{E, y.tile_off.p};
-            const int kso = runs_ksplit(P, E, W, F);
+            const int kso = runs_ksplit(P, E, W, F, kNumSMs);
             room(y.eo, kso * cap * W); room(y.gu, act == FL_ACT_RELU2 ? cap * F : 0); room(y.gx_lo, cap * W); room(y.ga_lo, cap * F);
             launch(lc, "moe_lists", 0, ly_moe_lists_kernel, dim3(E), dim3(256), 0, (const int*)y.route_sel.p, Ti, top, E, y.grp_off.p, y.pair_row.p,
                    y.pair_of.p);

@@ -1289,22 +1289,6 @@ void dense_gemm_glu(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int F, i
     if (runs != nullptr) { g.groups = mats = runs->groups; g.tile_off = runs->tile_off; g.grp_m = 2 * F; }
     launch_rows_gemm(c, lc, tag, g, (R + kGemmBM - 1) / kGemmBM * ((F + 127) / 128), mats * 2 * F, tmW, xhi, xlo, true);
 }
-// Slices of K for the runs' plain GEMM: few experts of few rows leave most of the chip idle (340 rows, 8 experts, 2048 columns: 64 tiles of 128 x 256).
-// An expert's rows are not known here; with its share of the picks and a tenth more, the slices whose waves are shortest, up to four of at least eight
-// k blocks; a slice costs its way to memory and back, about a twentieth of a tile's time for 64 tiles.  Whole prompt, one slice -> this, us: experts of
-// 2816, width 1024, 130 / 286 / 400 / 583 tokens 503 -> 477, 528 -> 499, 548 -> 528, 610 -> 589; of 5632, width 2048, 130 / 200 / 1000 tokens 734 -> 694,
-// 753 -> 711, 1417 -> 1377 (four slices of 256 tiles, at 1531 tokens: 1973 -> 1995).
-int runs_ksplit(int picks, int groups, int N, int K) {
-    const int per = (int)(1.1 * picks / groups) + 1, tiles = std::min(groups, picks) * ((per + 127) / 128) * ((N + 255) / 256), nk = (K + 63) / 64;
-    int best = 1;
-    double cost = 1e30;
-    for (int ks = 1; ks <= 4 && (ks == 1 || nk / ks >= 8); ++ks) {
-        const double t = (double)((tiles * ks + kNumSMs - 1) / kNumSMs) / ks + 0.05 / 64 * tiles * ks;
-        if (t < cost) { cost = t; best = ks; }
-    }
-    while (best > 1 && (nk + best - 1) / best * (best - 1) >= nk) --best;         // none of them is empty
-    return best;
-}
 // ksplit > 1: slice s goes to out + s * R * N
 void dense_gemm_runs(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int N, int K, const CUtensorMap& tmW, float* out, const uint16_t* xhi,
                      const uint16_t* xlo, const RowRuns& runs, int ksplit) {

@@ -192,7 +192,6 @@ int dense_gemm_grouped(fl_cache& c, LaunchCtx& lc, const char* tag, int groups, 
 struct RowRuns { int groups; const int* tile_off; };
 void dense_gemm_glu(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int F, int K, const CUtensorMap& tmW, const uint16_t* xhi, const uint16_t* xlo,
                     const float* bias, int act, float limit, uint16_t* ohi, uint16_t* olo, const RowRuns* runs = nullptr);
-int runs_ksplit(int picks, int groups, int N, int K);
 void dense_gemm_runs(fl_cache& c, LaunchCtx& lc, const char* tag, int R, int N, int K, const CUtensorMap& tmW, float* out, const uint16_t* xhi,
                      const uint16_t* xlo, const RowRuns& runs, int ksplit = 1);
 // Block-diagonal GEMM (one matrix per head, say): out[t * ldo + b * o_bs + n] = sum_k x[t, b K + k] W_b[n, k] for b < blocks, n < N,
