@@ -54,10 +54,11 @@ def test_rows_that_are_not_numbers(n):
     assert np.isfinite(got[n:n + min(64, n - 20)]).all()
 
 
-# expert results of one to four slices of K (hidden widths of 8 to 44 k blocks), k blocks that do not go evenly into them
-@pytest.mark.parametrize("n,ff,experts", [(129, 520, 5), (129, 1030 * 2, 8), (300, 1536, 3), (140, 2824, 2)])
-def test_expert_results_in_slices(n, ff, experts):
-    cfg = N.config([N.gla(heads=2, dim=16, vdim=16, mlp=N.moe(ff=ff, experts=experts, top=2))], vocab=64, width=64)
+# expert results of one to four slices of K (hidden widths of 8 to 44 k blocks), k blocks that do not go evenly into them; one column tile of 256, three whole
+# ones, two and a piece; runs of uneven length, an expert that few rows pick
+@pytest.mark.parametrize("n,ff,experts,width", [(129, 520, 5, 64), (129, 1030 * 2, 8, 64), (300, 1536, 3, 64), (140, 2824, 2, 64), (260, 1536, 5, 768), (131, 2056, 19, 520)])
+def test_expert_results_in_slices(n, ff, experts, width):
+    cfg = N.config([N.gla(heads=2, dim=16, vdim=16, mlp=N.moe(ff=ff, experts=experts, top=2))], vocab=64, width=width)
     check(N, cfg, n, 37, 0.0)
 
 
