@@ -195,8 +195,8 @@ __device__ __forceinline__ void cs_decay_tables(CsDecay& d, int t) {       // t:
     d.end[t] = q * e;
     if (t == 0) d.whole = p * q * e;
 }
-// factors of the thread's results: zero above the diagonal (and on it unless `diagonal`)
-__device__ __forceinline__ void cs_decay_factors(float (&f)[4][4], const CsDecay& d, int ty, int tx, bool diagonal) {
+// factors of the thread's results: zero above the diagonal
+__device__ __forceinline__ void cs_decay_factors(float (&f)[4][4], const CsDecay& d, int ty, int tx) {
     float in = 1.f, blk[4];
 #pragma unroll
     for (int b = 0; b < 4; ++b) blk[b] = d.pre[16 * b + 15];
@@ -208,7 +208,7 @@ __device__ __forceinline__ void cs_decay_factors(float (&f)[4][4], const CsDecay
             if (c == r) {
                 in = 1.f;
                 for (int i = tx + 1; i <= ty; ++i) in *= d.sa[16 * r + i];
-                f[r][c] = tx < ty || (diagonal && tx == ty) ? in : 0.f;
+                f[r][c] = tx <= ty ? in : 0.f;
                 continue;
             }
             float x = d.pre[16 * r + ty] * d.suf[16 * c + tx];
@@ -686,7 +686,7 @@ static __global__ void __launch_bounds__(256) ly_chunk_delta_kernel(ChunkArgs a)
         for (int b = 0; b < tid / 16; ++b) p *= dec.pre[16 * b + 15];
         sp[tid] = p;
     }
-    cs_decay_factors(f, dec, ty, tx, true);
+    cs_decay_factors(f, dec, ty, tx);
     float* aq = a.aq + ((size_t)blockIdx.x * a.H + hd) * kCsC * kCsC;
 #pragma unroll
     for (int r = 0; r < 4; ++r)
