@@ -19,7 +19,7 @@ def test_workloads_cover_baseline_configs():
 
 
 def test_ncu_traffic_matches_algorithmic_bytes():
-    """profiles/rNN_persistent*_full_raw.csv (newest round): DRAM bytes per decode step of the persistent kernel == weights once +
+    """profiles/persistent_<n>step_dram.csv: DRAM bytes per decode step of the persistent kernel == weights once +
     KV once (Mistral-7B b=1, KV 2048: 14.490 GB) within 1 %, and the line names the file it comes from."""
     import bench
     t, src = bench.ncu_traffic_per_step()
