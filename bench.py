@@ -88,7 +88,7 @@ def peaks(kind="hbm"):
     if os.path.exists(p):
         d = json.load(open(p))
         return float(d["hbm_gbs"] if kind == "hbm" else d["bf16_tflops_sustained"]), "measured (MEASURED_PEAKS.json)"
-    return (6650.0 if kind == "hbm" else 1400.0), "fallback (B200_PROFILING.md)"
+    return (6650.0 if kind == "hbm" else 1400.0), "fallback (an earlier measurement)"
 
 
 def ncu_traffic_per_step():

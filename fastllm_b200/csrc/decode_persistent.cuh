@@ -351,7 +351,7 @@ __global__ void __launch_bounds__(kPkThreads, 1) decode_persistent_kernel(const 
             const uint8_t* tile = ring + (size_t)st * kPkStageBytes + a_off;
             const int col0 = cc * kPkChunkCols;
             // all fragment loads of a half chunk first (independent, in flight together), then the MMAs (two accumulator chains).
-            // (Round 2 tried the whole chunk's 16 loads ahead of four chains, with the stage index kept incrementally instead of
+            // (The whole chunk's 16 loads ahead of four chains, with the stage index kept incrementally instead of
             // c % NS: faster with the weight traffic switched off, 0.8-3.6 % SLOWER in the real run on all three models: dropped.)
             constexpr int KPW = kPkChunkCols / 16 / kPkConsumerWarps;      // k-steps per warp per full chunk (8)
             const uint16_t* xcol = xrow + (col0 + bk + warp * 16);

@@ -5,7 +5,7 @@ The reference is Rust and there is no Rust toolchain in this image, so the drop-
   * this module -- the same interface in Python, used by tests/ and bench.py so the parity tests read like the
     reference's own tests (same names, same argument meaning, same offset rules, same error behaviour).
 
-Reference interfaces mirrored (paths under /root/reference/src/models):
+Reference interfaces mirrored (paths under src/models):
   ModelInitializer {initialize_model, initialize_cache, forward}     model_initializer.rs:6-22
   ModelCache {increment_offset, reset, get_offset}                   cache.rs:5-10
   LlamaWithConfig / LlamaCache                                       llama.rs:52-149

@@ -6,7 +6,7 @@
  * throws or aborts across this boundary.  The library owns all device memory (weights, paged KV cache,
  * workspaces), its own CUDA stream per cache, and the NCCL communicator.  There is no CPU fallback.
  *
- * Reference interface each group replaces (paths under /root/reference/src):
+ * Reference interface each group replaces (paths under src):
  *   fl_model_create / fl_model_put_tensor / fl_model_finalize
  *        <- ModelInitializer::initialize_model(&Config, HashMap<String,Tensor>, DType, &Device)
  *           models/model_initializer.rs:10-17; called from providers/huggingface/huggingface.rs:135;

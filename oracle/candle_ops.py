@@ -1,7 +1,7 @@
 """candle 0.8.x primitive-op semantics restated in numpy f32 (TEST INFRASTRUCTURE).
 
 candle-core / candle-nn are crates.io dependencies of the reference
-(/root/reference/Cargo.toml:19-21, "^0.8.2", un-vendored), so each function below
+(Cargo.toml:19-21, "^0.8.2", un-vendored), so each function below
 restates the published CPU algorithm of the named candle op; the reference call
 site that reaches it is cited.  All arithmetic is f32 (candle CPU F32 path, the
 only dtype the reference's CPU build can execute).

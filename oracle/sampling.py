@@ -1,6 +1,6 @@
 """CPU restatement of the sampling step of the reference's generate loop.  TEST INFRASTRUCTURE ONLY.
 
-Reference call sites (paths under /root/reference/src):
+Reference call sites (paths under src):
     LogitsProcessor::new(Default::default(), Some(temperature as f64), None)     models/mod.rs:157-158, 373-374
     logits_processor.sample(&last_logits)                                         models/mod.rs:308-310, 425-428
 

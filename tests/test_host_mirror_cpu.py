@@ -1,7 +1,7 @@
 """The reference's own unit tests, re-stated against the product's host-side mirror (fastllm_b200/models.py)
 and the C ABI's config failure points.  No GPU: config validation is host logic and runs before the library touches a device.
 
-Reference tests mirrored (paths under /root/reference/src/models):
+Reference tests mirrored (paths under src/models):
     cache.rs:49-65, llama.rs:168-205, mistral.rs:255-271, qwen.rs:192-208      cache offset +1 / reset
     cache.rs:68-79 (+ llama/mistral/qwen twins)                                 `Any` downcast -> isinstance here
     llama.rs:208-232, mistral.rs:274-300, qwen.rs:211-237                        config field copy-through (+ the unwrap_or defaults)
