@@ -190,7 +190,7 @@ def run_minilm(args, rank, world, local_rank):
             "e2e": {"value": B / e2e_s, "unit": "emb/s", "h2d_bytes_per_step": int(b * T * 4), "d2h_bytes_per_step": int(b * 384 * 4)},
             "gpu_launches": int(launches),
             "roofline": {"bound": "tensor", "achieved": tflops, "peak": peak, "unit": "TFLOP/s", "frac": tflops / peak, "traffic": None,
-                         "kernel": "bert_block_kernel x 6 (tcgen05 on SM pairs) + gemm_tc_kernel<128, BIAS_BF16> x 6 + bert_attn_kernel x 6 per batch: whole-encoder algorithmic FLOPs / device time",
+                         "kernel": "bert_qkv_attn_kernel x 6 + bert_block_kernel x 6 (tcgen05 on SM pairs) per batch: whole-encoder algorithmic FLOPs / device time",
                          "peak_source": src},
             "cpu_baseline": cpu}
     print(json.dumps(line), flush=True)
