@@ -1,8 +1,7 @@
 // The recurrences of the layered decoders over long portions of a prompt (serving precision), 64 tokens at a time.
 //
 // Token by token a state S of [D, Dv] floats per head is read and written once per token and nothing of token t + 1 can start before
-// token t: ly_rec_scan_kernel / ly_gla_scan_kernel take about 0.5 us per token whatever the chip has free (2048 tokens of 32 heads of
-// 128 x 128: 1.0 to 1.2 ms per layer).  Within a chunk of C = 64 tokens the same sums are products of small matrices, and only the state
+// token t: ly_rec_scan_kernel takes 0.25 to 0.3 us per token and ly_gla_scan_kernel 1 us, however much of the chip is free.  Within a chunk of C = 64 tokens the same sums are products of small matrices, and only the state
 // at the chunks' borders is serial:
 //   o_i = q_i^T (decay to i) S_0 + sum_{j <= i} (q_i . k_j decayed from j to i) u_j,     S_C = (decay to C) S_0 + sum_j (k_j decayed to C) u_j^T
 //   (Yang et al., "Gated linear attention transformers with hardware-efficient training", 2024; the delta rule's u by the WY form of
@@ -14,9 +13,10 @@
 //   3. ly_chunk_out_kernel / ly_chunk_out_heads_kernel                     one block per (chunk, head): what the starting state adds
 // Bound: 1 and 3 by latency -- operands in shared memory, 4 x 4 results per thread (64 FMA per 8 16-byte loads), 16 warps per SM:
 // at 1024 tokens ncu has the FMA pipe at 31 to 34 %, issue slots at 45 to 47 %, shared memory at 47 to 50 %.  2: HBM.
-// Measured per layer, token by token -> chunks: gated linear attention, 1531 tokens, 16 heads of 128 x 128: 1160 -> 180 us; Mamba-2, 2048
-// tokens, 128 heads of 128 x 64: 1186 -> 440 us (four heads per block: their scores are multiplied once); delta rule, 2048 tokens, 32 heads of 128 x 128: 1022 -> 626 us; lightning attention, 333
-// tokens, 16 heads: 246 -> 65 us.  Same model, same tokens: the logits agree to 1e-5 .. 4e-5, their error against 64 bits is unchanged.
+// Measured per layer, token by token -> chunks, kernel by kernel: gated linear attention, 1531 tokens, 16 heads of 128 x 128: 1575 -> 192 us; Mamba-2, 2048
+// tokens, 128 heads of 128 x 64: 772 -> 470 us (four heads per block: their scores are multiplied once); delta rule, 2048 tokens, 32 heads of 128 x 128: 596 -> 576 us,
+// 1024 tokens, 16 heads: 304 -> 204; lightning attention, 333 tokens, 16 heads: 89 -> 57 us.  Same model, same tokens: the logits agree to 1e-5 .. 4e-5, their
+// error against 64 bits is unchanged.
 #pragma once
 #include "layered_ops.cuh"
 

@@ -341,9 +341,9 @@ static bool bert_blocks(const BertModel& m, int T) {
 }
 
 // Few short sentences: the whole encoder in one launch of clusters (bert_small.cuh).
-// The line lies where the clusters (about nine of 16 blocks) are all resident and none has more than 64 tokens: there both take the same (sentences
-// x tokens, chain / one launch, us: 16 x 19 315 / 256, 9 x 48 323 / 324, 18 x 31 319 / 323, 9 x 64 328 / 333, 36 x 16 319 / 315), and a second wave
-// would cost a whole pass more.
+// The line lies where the clusters (as many of 16 blocks as the driver finds room for: seven on the devices measured) are all resident and none has more than
+// 64 tokens (sentences x tokens, chain / one launch, us: 1 x 4 224 / 93, 1 x 19 235 / 118, 1 x 64 252 / 192, 16 x 19 286 / 194, 8 x 31 284 / 192).  Behind it a second wave
+// would cost a whole pass more: 8 x 64 289 as a chain, 201 a wave of seven.
 template <int MT>
 static int bert_small_launch(BertModel& m, const BertSmallArgs& a, int clusters, bool ask) {      // ask: -> clusters that are resident at a time
     auto kern = bert_small_kernel<MT, kBsCluster>;
