@@ -8,7 +8,7 @@
 // core makes the next unit's columns.  The clusters take equal runs of heads (up to four heads a run none crosses from one pair of groups to the next: 60 x 43
 // tokens 366 -> 354 us, 36 x 65 354 -> 345); x stays in shared memory over the units of a pair.
 // q, k and v never leave the SM: the GEMM and the attention moved 75 MB each way between them at 256 x 128 tokens.
-// Whole encoder, GEMM and attention -> this kernel, us (with the block kernel as it is): 256 x 128 tokens 1280 -> 1102, 76 x 128 552 -> 517, 400 x 43 788 ->
+// Whole encoder, GEMM and attention -> this kernel, us (with the block kernel as it is): 256 x 128 tokens 1280 -> 1107, 76 x 128 552 -> 517, 400 x 43 788 ->
 // 645, 1500 x 20 1690 -> 1177, 60 x 43 377 -> 354; a layer of 256 x 128: 87 -> 66.  (Runs of whole units of three heads: 76 x 128 567.)
 // A unit of 128-token sentences takes about 14500 clocks: 2200 to bring q|k|v into shared memory, 12000 of attention in which the tensor core's 3700 for
 // the next unit run -- the warps' products (3300), ex2 (3100) and shared memory (3300 and the operands of the other products) would overlap better with
@@ -48,12 +48,13 @@ __device__ __forceinline__ float2 add_f32x2(float2 x, float2 y) {
 // 16 query rows (m0 on) of a sentence's head: sq, sk, sv at the sentence's first row.  The rows of o take the place of the q rows that this warp alone reads.
 // Every operation on a score is bert_attn_kernel's, in its order, so that a sentence's embedding is the same to the bit whichever kernel takes it: score /
 // sqrt(d), minus the row's largest, e to that as 2^(x log2 e) (weights below 2^-126 are zero), a lane's sum a pair of neighbouring keys at a time.  (One fma
-// in front of ex2 and the sums two columns at a time: 256 x 128 tokens 1080 us instead of 1102, but weights on other sides of bf16 roundings, 1.2e-3 in an embedding.)
+// in front of ex2 and the sums two columns at a time: 256 x 128 tokens 1080 us instead of 1107, but weights on other sides of bf16 roundings, 1.2e-3 in an embedding.  The products with 1 / sqrt(d) are
+// __fmul_rn: a packed product in front of the packed sum comes out of the assembler as one fma.)
 // LD: elements of a row.  KT: 16-key steps of the sentence's t tokens; rows behind it read as its last one, as queries nobody uses what they give, as keys their weight is zero.
 template <int KT, int LD>
 __device__ __forceinline__ void bq_attention(uint16_t* sq, const uint16_t* sk, const uint16_t* sv, int t, int m0, float inv_scale, uint16_t* ctx, int lane) {
     const int g = lane >> 2, tq = lane & 3;
-    const float2 scale = make_float2(inv_scale, inv_scale), log2e = make_float2(1.4426950408889634f, 1.4426950408889634f);
+    const float2 log2e = make_float2(1.4426950408889634f, 1.4426950408889634f);
     uint32_t qa[2][4];
     float2 s[2 * KT][2];
 #pragma unroll
@@ -81,7 +82,7 @@ __device__ __forceinline__ void bq_attention(uint16_t* sq, const uint16_t* sk, c
             const int nt = 2 * i + u;
 #pragma unroll
             for (int h = 0; h < 2; ++h) {
-                s[nt][h] = mul_f32x2(make_float2(c[u][2 * h], c[u][2 * h + 1]), scale);
+                s[nt][h] = make_float2(__fmul_rn(c[u][2 * h], inv_scale), __fmul_rn(c[u][2 * h + 1], inv_scale));
                 if (i + 1 == KT) {
                     if (nt * 8 + tq * 2 >= t) s[nt][h].x = -INFINITY;
                     if (nt * 8 + tq * 2 + 1 >= t) s[nt][h].y = -INFINITY;
