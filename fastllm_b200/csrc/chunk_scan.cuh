@@ -12,7 +12,7 @@
 //   2. ly_chunk_state_kernel / ly_chunk_delta_state_kernel                 the states at the chunks' starts, chunk by chunk
 //   3. ly_chunk_out_kernel / ly_chunk_out_heads_kernel                     one block per (chunk, head): what the starting state adds
 // Bound: 1 and 3 by latency -- operands in shared memory, 4 x 4 results per thread (64 FMA per 8 16-byte loads), 16 warps per SM:
-// at 1024 tokens ncu has the FMA pipe at 31 to 34 %, issue slots at 45 to 47 %, shared memory at 47 to 50 %.  2: HBM.
+// at 1024 tokens ncu has the FMA pipe at 24 to 47 %, issue slots at 42 to 60 %, shared memory at 37 to 52 %.  2: HBM.
 // Measured per layer, token by token -> chunks, kernel by kernel: gated linear attention, 1531 tokens, 16 heads of 128 x 128: 1575 -> 192 us; Mamba-2, 2048
 // tokens, 128 heads of 128 x 64: 772 -> 470 us (four heads per block: their scores are multiplied once); delta rule, 2048 tokens, 32 heads of 128 x 128: 596 -> 576 us,
 // 1024 tokens, 16 heads: 304 -> 204; lightning attention, 333 tokens, 16 heads: 89 -> 57 us.  Same model, same tokens: the logits agree to 1e-5 .. 4e-5, their
