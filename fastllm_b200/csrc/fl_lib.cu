@@ -1940,13 +1940,14 @@ static bool page_locked(const float* p, size_t n) {
 static void logits_to_host(fl_cache& c, float* host, size_t n) {
     const float* dev = c.ly ? c.ly->logits.p : c.logits.p;
     if (page_locked(host, n)) {
-        if (c.may_fail || g_peer.ready) {        // a step that may have failed without a CUDA error is waited for first
+        const bool before = c.may_fail || g_peer.ready;
+        if (before) {        // a step that may have failed without a CUDA error is waited for first
             FL_CUDA(cudaStreamSynchronize(c.stream));
             LogitsTransfer(c, dev, host).check();
         }
         FL_CUDA(cudaMemcpyAsync(host, dev, n * 4, cudaMemcpyDeviceToHost, c.stream));
         FL_CUDA(cudaStreamSynchronize(c.stream));
-        LogitsTransfer(c, dev, host).check();
+        if (!before) LogitsTransfer(c, dev, host).check();
         return;
     }
     float* stage = c.ly ? c.ly->h_logits.p : c.h_logits.p;
